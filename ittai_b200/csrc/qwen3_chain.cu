@@ -1,0 +1,1053 @@
+// Qwen3-0.6B greedy decode as a chain of small dependent kernels, one CUDA graph per token (batch 1, 2, 4 or 8).
+//
+// A decoded token is 28 x (QKV, attention, O-proj, gate/up, down) + head + finish: 142 launches whose only dependency is
+// one short vector.  With programmatic dependent launch every kernel is resident, and has fetched its weights, while its
+// predecessor still runs; what remains per hand-off is a kernel boundary, 1.1 us in a graph on a B200 (1.5 us with a
+// cluster barrier), against 1.4-2.9 us for a polled flag word that 148 CTAs read (qwen3_decode.cu).
+//
+// * GEMV kernels (gemv_kernel): 512 threads; a CTA's whole slice of a projection (32 to 96 KB) is on its way to
+//   shared memory BEFORE griddepcontrol.wait (weights do not depend on the token); after the wait it is multiplied with
+//   the activations of all sequences as mma.sync m16n8k16 tiles (the sequences are the N dimension), a warp taking 16 (or
+//   8) rows x one K chunk.  Two such CTAs fit an SM, so the next kernel's weights stream while this one waits.  The K chunks
+//   meet in shared memory, in fixed order.
+// * Attention (attn_kernel): a cluster of CS CTAs per (sequence, kv head) splits the cache; K/V tiles of 32 positions
+//   arrive by TMA (128-byte swizzle), the first six before the wait; scores and P V on mma.sync, the splits meet
+//   through distributed shared memory.  Probabilities enter P V as a high and a low bf16 part in separate N columns (the
+//   columns are idle anyway), so nothing is lost against fp32 probabilities.
+// * finish_kernel: argmax over the head's candidates, token feedback, positions, next token's embedding row.
+//
+// Rounding points are the eager modules' (the same as in qwen3_decode.cu).
+//
+// Measured on a B200, us per step, the persistent kernel of qwen3_decode.cu -> this chain: batch 1 at 47 / 4096 / 8100 cached
+// positions 558 -> 426, 579 -> 525, 658 -> 590; batch 4 at 47 / 1000 / 8100 792 -> 454, 813 -> 540, 1418 -> 1020; batch 8 at 1000 /
+// 8100 1009 -> 668, 2206 -> 1577.  A layer takes 13 us at a short cache: five boundaries of 0.7-0.9 us (last store of a kernel
+// to the release of the next), attention 2.6, gate/up 2.2, QKV 2.0, down 1.5, O-proj 1.1; the head 47 us at 6.6 TB/s.  What had
+// to go on the way (batch 1, 47 positions): weights through registers (800 us: a kernel's activation loads stand behind the
+// next kernel's weight loads in the load pipe), normalisation in every warp's fragments (509: issue-bound), constants
+// loaded ahead of the wait but scheduled behind it, the head through registers (93 us instead of 47).
+#include <mutex>
+
+#include "gemm2_common.cuh"
+#include "launch.h"
+#include "tcgen05.cuh"
+#include "tmap.h"
+
+namespace ittai {
+namespace chain {
+
+constexpr int D = ITTAI_Q3_D, HD = ITTAI_Q3_HD, NKV = ITTAI_Q3_NKV, DQ = ITTAI_Q3_DQ, DQKV = ITTAI_Q3_DQKV, DGU = ITTAI_Q3_DGU, FF = ITTAI_Q3_FF;
+constexpr int kGemvThreads = 512;
+constexpr int kMaxHeadCtas = 1024;
+constexpr uint32_t kSpin = 1u << 22;         // polls of a copy that does not land
+constexpr uint32_t kSpinParked = 1u << 18;   // the same where a poll parks the warp for up to 2 us
+
+// Device-side state of one decode call (in the caller's workspace).
+struct State {
+    int32_t step, n_steps, n_forced, abort;
+    int32_t* out_ids;
+    const int32_t* forced;
+    uint64_t* step_ns;
+    int32_t cur_pos[ITTAI_MAX_BATCH];    // cache row of the token being computed; -1 once the call has aborted
+};
+struct Buffers {
+    State* st;
+    bf16 *h, *hmid, *qkv, *attn, *act;   // [B, width]
+    float* cand_val;                     // [head CTAs, B]
+    int32_t* cand_idx;
+};
+inline size_t layout(int batch, char* base, Buffers* w) {
+    size_t off = 0;
+    auto take = [&](size_t n) { char* p = base + off; off += (n + 255) / 256 * 256; return p; };
+    w->st = reinterpret_cast<State*>(take(sizeof(State)));
+    w->h = reinterpret_cast<bf16*>(take((size_t)batch * D * 2));
+    w->hmid = reinterpret_cast<bf16*>(take((size_t)batch * D * 2));
+    w->qkv = reinterpret_cast<bf16*>(take((size_t)batch * DQKV * 2));
+    w->attn = reinterpret_cast<bf16*>(take((size_t)batch * DQ * 2));
+    w->act = reinterpret_cast<bf16*>(take((size_t)batch * FF * 2));
+    w->cand_val = reinterpret_cast<float*>(take((size_t)kMaxHeadCtas * batch * 4));
+    w->cand_idx = reinterpret_cast<int32_t*>(take((size_t)kMaxHeadCtas * batch * 4));
+    return off;
+}
+
+__device__ __forceinline__ void mma16816(float (&d)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0, uint32_t b1) {
+    asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, {%0, %1, %2, %3};"
+                 : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3]) : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
+}
+// Weights: read once per token.  Their L2 lines are the first to go, so that 1.2 GB of them per token do not push out what
+// every kernel needs again: its instructions, its parameters, the activation vectors.
+__device__ __forceinline__ uint64_t evict_first_policy() {
+    uint64_t pol;
+    asm volatile("createpolicy.fractional.L2::evict_first.b64 %0, 1.0;" : "=l"(pol));
+    return pol;
+}
+__device__ __forceinline__ uint4 ldg_weight(const void* p, uint64_t pol) {
+    uint4 v;
+    asm volatile("ld.global.nc.L1::no_allocate.L2::cache_hint.v4.u32 {%0,%1,%2,%3}, [%4], %5;"
+                 : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "l"(p), "l"(pol));
+    return v;
+}
+// bf16 pair of x -> bf16(bf16(x * rstd) * gain)
+__device__ __forceinline__ uint32_t norm_pair(uint32_t x, uint32_t g, float rstd) {
+    return pack_bf16x2(bf16r(bf_lo(x) * rstd) * bf_lo(g), bf16r(bf_hi(x) * rstd) * bf_hi(g));
+}
+// 1 / sqrt(v) to fp32 accuracy: the hardware approximation and one Newton step (1.0f / sqrtf(v) is two long dependent
+// sequences, and every kernel that normalises has one on its critical path).
+__device__ __forceinline__ float rsqrt_full(float v) {
+    const float r = rsqrtf(v);
+    return fmaf(r * 0.5f, fmaf(-v * r, r, 1.0f), r);
+}
+// RMSNorm of the NB rows of x (width D) into xs[b][..] (rows padded by 64 bytes, see the weight rows): the 512 threads share
+// the rows out, 2 NB values each, so that every value is normalised once per CTA.  Contains the two barriers after which xs
+// may be read.
+constexpr int kXsLd = D + 32;             // bf16 per row of xs
+__device__ __forceinline__ void gemv_sync() { asm volatile("bar.sync 1, %0;" ::"n"(kGemvThreads) : "memory"); }   // not the head's feeding warp
+template <int NB>
+__device__ __forceinline__ void norm_rows(const bf16* x, const bf16* gain_s, bf16* xs, float* ss_s, int tid, float eps) {
+    constexpr int W = 16 / NB, E = 2 * NB;             // warps per row, values per thread
+    const int warp = tid >> 5, b = warp / W, e0 = (tid - b * W * 32) * E;
+    uint32_t u[NB];
+    const bf16* src = x + (size_t)b * D + e0;
+    if constexpr (NB == 1) u[0] = ldcg32(src);
+    else if constexpr (NB == 2) asm volatile("ld.global.cg.v2.u32 {%0,%1}, [%2];" : "=r"(u[0]), "=r"(u[1]) : "l"(src));
+    else {
+#pragma unroll
+        for (int i = 0; i < NB / 4; ++i) {
+            const uint4 q = ldcg128(src + 8 * i);
+            u[4 * i] = q.x; u[4 * i + 1] = q.y; u[4 * i + 2] = q.z; u[4 * i + 3] = q.w;
+        }
+    }
+    float s = 0.f;
+#pragma unroll
+    for (int i = 0; i < NB; ++i) s = fmaf(bf_lo(u[i]), bf_lo(u[i]), fmaf(bf_hi(u[i]), bf_hi(u[i]), s));
+    s = warp_sum(s);
+    if ((tid & 31) == 0) ss_s[warp] = s;
+    gemv_sync();
+    float tot = 0.f;
+#pragma unroll
+    for (int i = 0; i < W; ++i) tot += ss_s[b * W + i];
+    const float rstd = rsqrt_full(tot * (1.0f / D) + eps);
+    const uint32_t* gw = reinterpret_cast<const uint32_t*>(gain_s + e0);
+    uint32_t* dst = reinterpret_cast<uint32_t*>(xs + b * kXsLd + e0);
+#pragma unroll
+    for (int i = 0; i < NB; ++i) dst[i] = norm_pair(u[i], gw[i], rstd);
+    gemv_sync();
+}
+
+enum { kPlain = 0, kSwiglu = 1, kResidual = 2 };
+
+struct GemvArgs {
+    const bf16* w;          // [rows][K]
+    const bf16* x;          // [B][K]
+    const bf16* gain;       // norm in front of the projection, or unused
+    const bf16* res;        // kResidual: [B][D]
+    bf16* out;              // [B][ld_out]
+    int ld_out;
+    float eps;
+    uint32_t* status;
+    const State* st;        // gate/up: the next layer's cache rows to bring into L2 (k_next [B * 8][kv_cap][128]); nullptr: none
+    const bf16 *k_next, *v_next;
+    int kv_cap;
+    const unsigned char* ahead;      // O-proj: weights to bring into L2, eight pieces of ahead_bytes per CTA (nullptr: none)
+    uint32_t ahead_bytes;
+    int late_trigger;       // first kernel of a token: dependents start only once everything before this kernel is complete
+};
+
+// out = epilogue(W x).  ROWS = 32 or 48: 16-row tiles; ROWS = 8: half a tile.  KC K chunks x (16 / KC) tile groups over the 16
+// warps.  QKV: 128 CTAs of 32 rows (64 KB), gate/up: 128 of 48 (96 KB), O-proj: 128 of 8 (32 KB), down: 128 of 8 (48 KB).
+// The weight rows come by bulk copies (they bypass the load pipe, in which the next kernel's weights would otherwise
+// stand in front of this one's activations) into rows padded by 64 bytes, so that the eight rows a warp reads at once fall
+// on different banks.  A lane reads 16-byte pieces of its rows: columns 32 j + 8 t .. + 7 of the chunk, which serve as the
+// k-indices of two MMAs (which column a k-index stands for is free as long as A and B agree).
+template <int K, int ROWS>
+constexpr uint32_t gemv_smem() { return (uint32_t)ROWS * (K * 2 + 64); }
+
+template <int NB, int K, int ROWS, int EPI>
+__global__ void __launch_bounds__(kGemvThreads, 2) gemv_kernel(const GemvArgs a) {
+    constexpr int KC = ROWS == 32 ? 8 : 16, KW = K / KC, NJ = KW / 32, NR = ROWS == 8 ? 1 : 2, NT = ROWS == 48 ? 3 : 1;
+    constexpr int LD = K * 2 + 64;                      // bytes per weight row in shared memory
+    constexpr bool kNorm = EPI != kResidual;
+    static_assert(KW % 32 == 0, "K chunk");
+    extern __shared__ __align__(128) unsigned char w_s[];
+    __shared__ float part[KC][NB][ROWS];
+    __shared__ float ss_s[16];
+    __shared__ __align__(16) bf16 gain_s[kNorm ? D : 8];
+    __shared__ __align__(16) bf16 xs[kNorm ? NB * kXsLd : 8];
+    __shared__ unsigned long long landed;
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, g = lane >> 2, t = lane & 3;
+    const int kc = ROWS == 32 ? warp & 7 : warp, tile = ROWS == 32 ? warp >> 3 : 0;
+    const int row0 = blockIdx.x * ROWS;
+    const int col = kc * KW + 8 * t;
+    if (tid == 0) { mbar_init(&landed, 1); fence_mbar_init(); mbar_expect_tx(&landed, ROWS * K * 2); }
+    __syncwarp();
+    if (warp == 0) {
+        for (int r = lane; r < ROWS; r += 32) bulk_g2s(w_s + r * LD, a.w + (size_t)(row0 + r) * K, K * 2, &landed);
+    }
+    if (!a.late_trigger) pdl_trigger();
+    if (EPI == kSwiglu && a.k_next != nullptr && warp == 1) {
+        // an even share of every sequence's cached rows; positions are stable here (see attn_kernel)
+        constexpr int kItems = NB * NKV, kParts = DGU / 48 / kItems;
+        const int item = blockIdx.x % kItems, piece = blockIdx.x / kItems;
+        int pos = (int)ld_relaxed(reinterpret_cast<const uint32_t*>(&a.st->cur_pos[item / NKV]));
+        if ((long long)NB * NKV * pos * HD * 4 > (24 << 20)) pos = 0;            // more than L2 keeps until it is read
+        const int q0 = (int)((long long)pos * piece / kParts), q1 = (int)((long long)pos * (piece + 1) / kParts);
+        for (int q = q0 + 32 * lane; q < q1; q += 32 * 32) {
+            const uint32_t n = (uint32_t)(q1 - q < 32 ? q1 - q : 32) * HD * 2;
+            l2_prefetch(a.k_next + ((size_t)item * a.kv_cap + q) * HD, n);
+            l2_prefetch(a.v_next + ((size_t)item * a.kv_cap + q) * HD, n);
+        }
+    }
+    if (EPI == kResidual && a.ahead != nullptr && warp == 1 && lane < 8)
+        l2_prefetch(a.ahead + ((size_t)blockIdx.x * 8 + lane) * a.ahead_bytes, a.ahead_bytes);
+    const unsigned char* wr = w_s + (tile * 16 + g) * LD + col * 2;
+    if constexpr (kNorm) reinterpret_cast<uint32_t*>(gain_s)[tid] = reinterpret_cast<const uint32_t*>(a.gain)[tid];
+    __syncthreads();                                   // the barrier exists for every warp, and the gain has arrived: a load
+                                                       // left open here may be scheduled behind the wait
+    pdl_wait();
+    if (a.late_trigger) pdl_trigger();
+    uint4 x[NJ];
+    if constexpr (kNorm) norm_rows<NB>(a.x, gain_s, xs, ss_s, tid, a.eps);
+#pragma unroll
+    for (int j = 0; j < NJ; ++j) {
+        if constexpr (kNorm) x[j] = g < NB ? *reinterpret_cast<const uint4*>(xs + g * kXsLd + col + 32 * j) : make_uint4(0u, 0u, 0u, 0u);
+        else x[j] = g < NB ? ldcg128(a.x + (size_t)g * K + col + 32 * j) : make_uint4(0u, 0u, 0u, 0u);
+    }
+    float res = 0.f;
+    if constexpr (EPI == kResidual) {
+        if (tid < 8 * NB) res = ldcg_bf16(a.res + (size_t)(tid >> 3) * D + row0 + (tid & 7));
+    }
+    const bool ok = mbar_wait_bounded(&landed, 0, kSpinParked);
+#pragma unroll
+    for (int n = 0; n < NT; ++n) {
+        float d0[4] = {0.f, 0.f, 0.f, 0.f}, d1[4] = {0.f, 0.f, 0.f, 0.f};
+#pragma unroll
+        for (int j = 0; j < NJ; ++j) {
+            const uint4 lo = *reinterpret_cast<const uint4*>(wr + 16 * n * LD + 64 * j);
+            const uint4 hi = NR == 2 ? *reinterpret_cast<const uint4*>(wr + (16 * n + 8) * LD + 64 * j) : make_uint4(0u, 0u, 0u, 0u);
+            mma16816(d0, lo.x, hi.x, lo.y, hi.y, x[j].x, x[j].y);
+            mma16816(d1, lo.z, hi.z, lo.w, hi.w, x[j].z, x[j].w);
+        }
+        float* p = &part[kc][0][(tile + n) * 16 + g];
+        if (2 * t < NB) { p[2 * t * ROWS] = d0[0] + d1[0]; if (NR == 2) p[2 * t * ROWS + 8] = d0[2] + d1[2]; }
+        if (2 * t + 1 < NB) { p[(2 * t + 1) * ROWS] = d0[1] + d1[1]; if (NR == 2) p[(2 * t + 1) * ROWS + 8] = d0[3] + d1[3]; }
+    }
+    __syncthreads();
+    if constexpr (ROWS >= 32) {
+        // two threads of a warp side by side hold two rows of one sequence
+#pragma unroll
+        for (int i0 = 0; i0 < ROWS * NB; i0 += kGemvThreads) {
+            const int i = i0 + tid;
+            if (i0 + 32 * warp < ROWS * NB) {
+                const int b = i / ROWS, r = i % ROWS;      // a warp may span two sequences, an aligned group of 16 never does
+                float s = 0.f;
+                if (i < ROWS * NB) {
+#pragma unroll
+                    for (int k = 0; k < KC; ++k) s += part[k][b][r];
+                }
+                if constexpr (EPI == kPlain) {
+                    const float o = __shfl_down_sync(0xffffffffu, s, 1);
+                    if ((lane & 1) == 0 && i < ROWS * NB) *reinterpret_cast<uint32_t*>(a.out + (size_t)b * a.ld_out + row0 + r) = pack_bf16x2(s, o);
+                } else {
+                    // rows 2i, 2i + 1 are (gate, up): act = bf16(bf16(silu(bf16 gate)) * bf16 up)
+                    const float up = bf16r(__shfl_down_sync(0xffffffffu, s, 1)), gate = bf16r(s);
+                    const float v = bf16r(gate / (1.0f + expf(-gate))) * up;
+                    const float v2 = __shfl_down_sync(0xffffffffu, v, 2);
+                    if ((lane & 3) == 0 && i < ROWS * NB) *reinterpret_cast<uint32_t*>(a.out + (size_t)b * a.ld_out + (row0 + r) / 2) = pack_bf16x2(v, v2);
+                }
+            }
+        }
+    } else {
+        if (tid < 8 * NB) {                             // eight rows of a sequence side by side
+            const int b = tid >> 3, r = tid & 7;
+            float s = 0.f;
+#pragma unroll
+            for (int k = 0; k < KC; ++k) s += part[k][b][r];
+            a.out[(size_t)b * a.ld_out + row0 + r] = __float2bfloat16_rn(res + bf16r(s));
+        }
+    }
+    if (!ok && lane == 0 && atomicCAS(&a.status[0], 0u, (uint32_t)ITTAI_ST_STREAM_TIMEOUT) == 0u) { a.status[1] = row0; a.status[2] = blockIdx.x; }
+}
+
+// ---- lm_head: logits = E bf16(norm(h)), with the arg-max candidates of this CTA's rows ----------------------------------
+// One CTA per SM walks its contiguous share of the table, 16 rows (32 KB) per ring stage, five stages: they fit beside a CTA
+// of the last down-projection, so the ring is full when the hidden state arrives.  A warp multiplies the 16 rows with one of
+// 16 K chunks; 311 MB of weights at the memory rate are the whole of it (loads through registers, two 64 KB steps ahead,
+// gave 93 us instead of 49).
+struct HeadArgs {
+    const bf16* w;          // [V][D]
+    const bf16* x;          // [B][D]
+    const bf16* gain;
+    bf16* logits;           // [B][V] or nullptr
+    float* cand_val;        // [CTAs][B]
+    int32_t* cand_idx;
+    uint32_t* status;
+    int vocab;
+    float eps;
+};
+constexpr int kHeadRing = 5, kHeadRows = 16, kHeadLd = D * 2 + 64;
+constexpr uint32_t kHeadSmem = kHeadRing * kHeadRows * kHeadLd;
+template <int NB>
+__global__ void __launch_bounds__(kGemvThreads + 32, 1) head_kernel(const HeadArgs a) {
+    constexpr int KW = D / 16, NJ = KW / 32;
+    extern __shared__ __align__(128) unsigned char w_s[];
+    __shared__ float part[2][16][NB][kHeadRows];
+    __shared__ float ss_s[16];
+    __shared__ __align__(16) bf16 gain_s[D];
+    __shared__ __align__(16) bf16 xs[NB * kXsLd];
+    __shared__ unsigned long long full[kHeadRing], empty[kHeadRing];
+    __shared__ volatile uint32_t failed;
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, g = lane >> 2, t = lane & 3;
+    const int r_lo = (int)((long long)a.vocab * blockIdx.x / gridDim.x), r_hi = (int)((long long)a.vocab * (blockIdx.x + 1) / gridDim.x);
+    const int n_it = (r_hi - r_lo + kHeadRows - 1) / kHeadRows;
+    if (tid == 0) {
+        for (int s = 0; s < kHeadRing; ++s) { mbar_init(&full[s], 1); mbar_init(&empty[s], 16); }
+        failed = 0;
+        fence_mbar_init();
+    }
+    __syncthreads();
+    pdl_trigger();
+    if (warp == 16) {                    // the feeding warp: one row per lane
+        for (int it = 0; it < n_it && !failed; ++it) {
+            const int s = it % kHeadRing, r0 = r_lo + it * kHeadRows, n = r_hi - r0 < kHeadRows ? r_hi - r0 : kHeadRows;
+            if (it >= kHeadRing && !mbar_wait_bounded(&empty[s], ((it / kHeadRing) - 1) & 1, kSpinParked)) { failed = 1; break; }
+            if (lane == 0) mbar_expect_tx(&full[s], (uint32_t)n * D * 2);
+            __syncwarp();
+            if (lane < n) bulk_g2s(w_s + (s * kHeadRows + lane) * kHeadLd, a.w + (size_t)(r0 + lane) * D, D * 2, &full[s]);
+        }
+        pdl_wait();
+        return;
+    }
+    reinterpret_cast<uint32_t*>(gain_s)[tid] = reinterpret_cast<const uint32_t*>(a.gain)[tid];
+    gemv_sync();                         // the gain has arrived (see gemv_kernel)
+    pdl_wait();
+    norm_rows<NB>(a.x, gain_s, xs, ss_s, tid, a.eps);
+    const int col = warp * KW + 8 * t;
+    uint4 x[NJ];
+#pragma unroll
+    for (int j = 0; j < NJ; ++j) x[j] = g < NB ? *reinterpret_cast<const uint4*>(xs + g * kXsLd + col + 32 * j) : make_uint4(0u, 0u, 0u, 0u);
+    float best = -INFINITY;
+    int best_i = 0x7fffffff;
+    const int rb = tid / kHeadRows, rr = tid % kHeadRows;          // reducing threads: sequence, row of the stage
+    for (int it = 0; it < n_it; ++it) {
+        const int s = it % kHeadRing, buf = it & 1;
+        bool ok = true;
+        uint32_t spins = 0;
+        while (!mbar_try_wait_parked(&full[s], (it / kHeadRing) & 1)) { if (++spins >= kSpinParked || failed) { ok = false; break; } }
+        if (!ok) failed = 1;
+        const unsigned char* wr = w_s + (s * kHeadRows + g) * kHeadLd + col * 2;
+        float d0[4] = {0.f, 0.f, 0.f, 0.f}, d1[4] = {0.f, 0.f, 0.f, 0.f};
+#pragma unroll
+        for (int j = 0; j < NJ; ++j) {
+            const uint4 lo = *reinterpret_cast<const uint4*>(wr + 64 * j), hi = *reinterpret_cast<const uint4*>(wr + 8 * kHeadLd + 64 * j);
+            mma16816(d0, lo.x, hi.x, lo.y, hi.y, x[j].x, x[j].y);
+            mma16816(d1, lo.z, hi.z, lo.w, hi.w, x[j].z, x[j].w);
+        }
+        __syncwarp();
+        if (lane == 0) asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(&empty[s])) : "memory");
+        float* p = &part[buf][warp][0][g];
+        if (2 * t < NB) { p[2 * t * kHeadRows] = d0[0] + d1[0]; p[2 * t * kHeadRows + 8] = d0[2] + d1[2]; }
+        if (2 * t + 1 < NB) { p[(2 * t + 1) * kHeadRows] = d0[1] + d1[1]; p[(2 * t + 1) * kHeadRows + 8] = d0[3] + d1[3]; }
+        gemv_sync();                     // readers of the other buffer have passed the barrier before this one
+        if (tid < kHeadRows * NB) {
+            float sum = 0.f;
+#pragma unroll
+            for (int k = 0; k < 16; ++k) sum += part[buf][k][rb][rr];
+            const int row = r_lo + it * kHeadRows + rr;
+            if (row < r_hi) {
+                const float v = bf16r(sum);
+                if (a.logits != nullptr) a.logits[(size_t)rb * a.vocab + row] = __float2bfloat16_rn(v);
+                if (v > best) { best = v; best_i = row; }        // rows ascend: the first maximum is kept
+            }
+        }
+    }
+    if (tid < (kHeadRows * NB < 32 ? 32 : kHeadRows * NB)) {
+#pragma unroll
+        for (int o = kHeadRows / 2; o > 0; o >>= 1) {       // highest value, lowest row on ties
+            const float ov = __shfl_xor_sync(0xffffffffu, best, o);
+            const int oi = __shfl_xor_sync(0xffffffffu, best_i, o);
+            if (ov > best || (ov == best && oi < best_i)) { best = ov; best_i = oi; }
+        }
+        if (rr == 0 && rb < NB) { a.cand_val[blockIdx.x * NB + rb] = best; a.cand_idx[blockIdx.x * NB + rb] = best_i; }
+    }
+    if (failed && tid == 0) {
+        if (atomicCAS(&a.status[0], 0u, (uint32_t)ITTAI_ST_STREAM_TIMEOUT) == 0u) { a.status[1] = (uint32_t)r_lo; a.status[2] = blockIdx.x; }
+        const long long t0 = clock64();                    // copies still in flight land before the shared memory is handed back
+        while (clock64() - t0 < 2000000) {}
+    }
+}
+
+// ---- token feedback -------------------------------------------------------------------------------------------------------
+struct TokenArgs {
+    State* st;
+    const bf16* embed;
+    bf16* h;
+    const float* cand_val;
+    const int32_t* cand_idx;
+    int n_cand;
+    int32_t* pos;
+    int32_t* next_id;
+    uint32_t* status;
+    int vocab, kv_cap;
+};
+__device__ __forceinline__ void bad_token(const TokenArgs& a, int id, int step, int pos, int b) {
+    if (atomicCAS(&a.status[0], 0u, (uint32_t)ITTAI_ST_BAD_TOKEN) == 0u) {
+        a.status[1] = (uint32_t)id; a.status[2] = (uint32_t)step; a.status[3] = (uint32_t)pos; a.status[4] = (uint32_t)b;
+    }
+}
+// Embedding row of sequence b's next token.  One warp.
+__device__ __forceinline__ void embed_row(const TokenArgs& a, int b, int id, int lane) {
+    const int row = id < 0 ? 0 : (id >= a.vocab ? a.vocab - 1 : id);
+#pragma unroll
+    for (int i = 0; i < 4; ++i)
+        *reinterpret_cast<uint4*>(a.h + (size_t)b * D + (lane + 32 * i) * 8) = *reinterpret_cast<const uint4*>(a.embed + (size_t)row * D + (lane + 32 * i) * 8);
+}
+
+// First kernel of a call: one warp per sequence.  Takes the call's parameters into the device state, checks the first ids
+// and positions, gathers the first embedding rows.
+template <int NB>
+__global__ void __launch_bounds__(32 * NB) begin_kernel(const TokenArgs a, int32_t* out_ids, const int32_t* forced, uint64_t* step_ns, int n_steps, int n_forced) {
+    const int b = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    __shared__ int bad;
+    if (threadIdx.x < ITTAI_STATUS_WORDS) a.status[threadIdx.x] = 0u;
+    if (threadIdx.x == 0) {
+        bad = 0;
+        State s;
+        s.step = 0; s.n_steps = n_steps; s.n_forced = n_forced; s.abort = 0;
+        s.out_ids = out_ids; s.forced = forced; s.step_ns = step_ns;
+        a.st->step = s.step; a.st->n_steps = s.n_steps; a.st->n_forced = s.n_forced;
+        a.st->out_ids = s.out_ids; a.st->forced = s.forced; a.st->step_ns = s.step_ns;
+    }
+    __syncthreads();
+    const int id = n_forced > 0 ? forced[b] : a.next_id[b], pos = a.pos[b];
+    if (id < 0 || id >= a.vocab || pos < 0 || pos >= a.kv_cap) {
+        if (lane == 0) { bad_token(a, id, 0, pos, b); bad = 1; }
+    }
+    __syncthreads();
+    if (lane == 0) a.st->cur_pos[b] = bad ? -1 : pos;
+    if (threadIdx.x == 0) a.st->abort = bad;
+    embed_row(a, b, id, lane);
+}
+
+// Last kernel of a token, one warp per sequence.  With HEAD: arg-max over the head's candidates, stored as the step's id and
+// fed back.  Without: a forced step whose logits nobody asked for.  Then the next token's row and position; after the last
+// step of the call the cache lengths `pos` advance, unless a step found an id or a position out of range.
+template <int NB, bool HEAD>
+__global__ void __launch_bounds__(32 * NB) finish_kernel(const TokenArgs a) {
+    pdl_trigger();
+    pdl_wait();
+    const int b = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    __shared__ int bad;
+    State* st = a.st;
+    const int step = st->step, n_steps = st->n_steps, abort = st->abort, pos = st->cur_pos[b];
+    int32_t* out_ids = st->out_ids;
+    if (threadIdx.x == 0) bad = abort;
+    __syncthreads();
+    int id = -1;
+    if constexpr (HEAD) {
+        float v = -INFINITY;
+        int ix = 0x7fffffff;
+        for (int k = lane; k < a.n_cand; k += 32) {
+            const float vk = a.cand_val[k * NB + b];
+            const int ik = a.cand_idx[k * NB + b];
+            if (vk > v || (vk == v && ik < ix)) { v = vk; ix = ik; }
+        }
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) {
+            const float ov = __shfl_xor_sync(0xffffffffu, v, o);
+            const int oi = __shfl_xor_sync(0xffffffffu, ix, o);
+            if (ov > v || (ov == v && oi < ix)) { v = ov; ix = oi; }
+        }
+        id = ix;
+        // no logit compared greater than -inf (a row of NaNs): reported instead of fed back
+        if (ix == 0x7fffffff && lane == 0 && !abort) { bad_token(a, ix, step, pos, b); bad = 1; }
+    }
+    if (lane == 0 && !abort) {
+        out_ids[(size_t)step * NB + b] = id;
+        if (HEAD) a.next_id[b] = id;
+    }
+    const bool last = step + 1 >= n_steps;
+    int next = id;
+    if (!last) {
+        if (step + 1 < st->n_forced) next = st->forced[(size_t)(step + 1) * NB + b];
+        if (!HEAD && step + 1 >= st->n_forced) next = a.next_id[b];
+        if (lane == 0 && !abort && (next < 0 || next >= a.vocab || pos + 1 >= a.kv_cap)) { bad_token(a, next, step + 1, pos + 1, b); bad = 1; }
+    }
+    __syncthreads();
+    if (lane == 0) {
+        st->cur_pos[b] = bad ? -1 : pos + 1;
+        if (last && !bad) a.pos[b] = pos + 1;
+    }
+    if (threadIdx.x == 0) {
+        st->step = step + 1;
+        st->abort = bad;
+        if (st->step_ns != nullptr) st->step_ns[step] = globaltimer_ns();
+    }
+    if (!last) embed_row(a, b, next, lane);
+}
+
+// ---- attention ------------------------------------------------------------------------------------------------------------
+// One cluster of CS CTAs per (sequence, kv head); rank r takes the r-th piece of the cached positions, rank 0 also the new
+// one (norm, rotation, append, and its own score).  Three groups of two compute warps take turns on 32-position tiles, a
+// warp 16 positions of each with its own softmax; a seventh warp feeds a ring of six 16 KB tiles (two CTAs per SM).  A
+// warp's 16 positions are 16 MMAs: scores with the keys as A (M = positions) and the two query heads as N columns, P V with
+// V^T as A (ldmatrix.trans on the swizzled tile) and P as B, its high parts in columns 0-1, its low parts in columns 2-3.
+// A tile is about 1000 dependent cycles for a warp, which is why the tiles are small and the warps many.
+constexpr int kGroups = 3, kAttnWarps = 2 * kGroups, kAttnThreads = 32 * kAttnWarps + 32, kTilePos = 32, kRing = 2 * kGroups;
+// Tile `it` belongs to group it % 3, which has two ring slots of its own: a slot's phases are waited for by the same two
+// warps in order (a slot shared by groups that skip each other's phases cannot be told apart by parity).
+__device__ __forceinline__ int ring_slot(int it) { return (it % kGroups) * 2 + ((it / kGroups) & 1); }
+__device__ __forceinline__ uint32_t ring_parity(int it) { return (uint32_t)(it / (2 * kGroups)) & 1u; }
+constexpr uint32_t kHalfTile = kTilePos * 128;                 // 32 positions x 64 dims
+constexpr uint32_t kTileBytes = 4 * kHalfTile;                 // K low / high dims, V low / high dims
+constexpr uint32_t kAttnSmem = kRing * kTileBytes + 1024;
+constexpr float kScoreScale = 0.08838834764831845f * 1.4426950408889634f;   // head_dim^-0.5 * log2(e)
+
+struct AttnChainArgs {
+    const State* st;
+    const bf16* qkv;        // [B][DQKV]
+    const bf16* qn;
+    const bf16* kn;
+    const bf16* rope;
+    bf16* kcache;           // this layer [B][8][cap][128]
+    bf16* vcache;
+    bf16* attn;             // [B][DQ]
+    uint32_t* status;
+    int layer, batch, kv_cap;
+    float eps;
+};
+
+__device__ __forceinline__ float ex2f(float x) {
+    float y;
+    asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+    return y;
+}
+__device__ __forceinline__ void ldsm4(uint32_t (&r)[4], uint32_t addr) {
+    asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0,%1,%2,%3}, [%4];" : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(addr) : "memory");
+}
+__device__ __forceinline__ void ldsm4_t(uint32_t (&r)[4], uint32_t addr) {
+    asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0,%1,%2,%3}, [%4];" : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(addr) : "memory");
+}
+__device__ __forceinline__ uint32_t movm_t(uint32_t a) {
+    uint32_t d;
+    asm volatile("movmatrix.sync.aligned.m8n8.trans.b16 %0, %1;" : "=r"(d) : "r"(a));
+    return d;
+}
+__device__ __forceinline__ void compute_sync() { asm volatile("bar.sync 1, %0;" ::"n"(32 * kAttnWarps) : "memory"); }
+__device__ __forceinline__ void tma_load_2d_hint(void* dst, const void* tmap, int x, int y, void* bar, uint64_t policy) {
+    asm volatile("cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes.L2::cache_hint [%0], [%1, {%2, %3}], [%4], %5;"
+                 ::"r"(smem_u32(dst)), "l"(tmap), "r"(x), "r"(y), "r"(smem_u32(bar)), "l"(policy) : "memory");
+}
+// Byte address of the 16-byte chunk `chunk` (0..7) of row `row` of a half tile under the 128-byte swizzle.
+__device__ __forceinline__ uint32_t swz(uint32_t base, int row, int chunk) { return base + (uint32_t)row * 128u + (uint32_t)((chunk ^ (row & 7)) << 4); }
+__device__ __forceinline__ void st_cluster_f32(float* p, int rank, float v) {
+    uint32_t a;
+    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(a) : "r"(smem_u32(p)), "r"(rank));
+    asm volatile("st.shared::cluster.f32 [%0], %1;" ::"r"(a), "f"(v) : "memory");
+}
+
+template <int CS>
+__global__ void __launch_bounds__(kAttnThreads, 2) attn_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constant__ CUtensorMap tm_v, const AttnChainArgs a) {
+    extern __shared__ __align__(1024) unsigned char ring_raw[];
+    unsigned char* ring = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(ring_raw) + 1023) & ~(uintptr_t)1023);
+    __shared__ unsigned long long full[kRing], empty[kRing];
+    __shared__ __align__(16) bf16 q_s[2][HD];
+    __shared__ __align__(16) bf16 k_s[HD];
+    __shared__ float pm[kAttnWarps + 1][2], pl[kAttnWarps + 1][2], po[kAttnWarps + 1][2][HD];   // partials of the warps and of the new position
+    __shared__ __align__(8) bf16 rot_s[4][HD];                  // q gain, k gain, cos | sin of the new position
+    __shared__ float rv[CS][CS == 1 ? 1 : 2 * HD / CS], rm[CS][2], rl[CS][2];     // partials of all ranks for this rank's outputs
+    __shared__ volatile uint32_t failed;
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const int rank = CS == 1 ? 0 : (int)(blockIdx.x % CS), item = blockIdx.x / CS, b = item / NKV, kvh = item % NKV;
+    const size_t head_row = (size_t)(a.layer * a.batch + b) * NKV + kvh;          // in units of kv_cap rows of the whole cache
+    if (tid == 0) {
+        for (int s = 0; s < kRing; ++s) { mbar_init(&full[s], 1); mbar_init(&empty[s], 2); }
+        failed = 0;
+        fence_mbar_init();
+    }
+    __syncthreads();
+    // another CTA's shared memory may be written only once that CTA runs: every thread arrives here, waits before the merge
+    if constexpr (CS > 1) asm volatile("barrier.cluster.arrive.release;" ::: "memory");
+    pdl_trigger();
+    // Positions and older cache rows are complete before the first kernel of this token lets its successors start
+    // (late_trigger), so they may be read ahead of the wait.
+    const int pos = (int)ld_relaxed(reinterpret_cast<const uint32_t*>(&a.st->cur_pos[b]));
+    const int n_old = pos < 0 ? 0 : pos;
+    const int chunk = ((n_old + CS - 1) / CS + 15) & ~15;
+    const int p0 = rank * chunk < n_old ? rank * chunk : n_old, p1 = p0 + chunk < n_old ? p0 + chunk : n_old;
+    const int n_tiles = (p1 - p0 + kTilePos - 1) / kTilePos;
+    const int row_base = (int)(head_row * (size_t)a.kv_cap) + p0;
+    uint64_t policy = 0;
+    auto issue = [&](int it) {
+        const int s = ring_slot(it);
+        unsigned char* t = ring + s * kTileBytes;
+        mbar_expect_tx(&full[s], kTileBytes);
+        const int y = row_base + it * kTilePos;
+        tma_load_2d_hint(t, &tm_k, 0, y, &full[s], policy);
+        tma_load_2d_hint(t + kHalfTile, &tm_k, 64, y, &full[s], policy);
+        tma_load_2d_hint(t + 2 * kHalfTile, &tm_v, 0, y, &full[s], policy);
+        tma_load_2d_hint(t + 3 * kHalfTile, &tm_v, 64, y, &full[s], policy);
+    };
+    if (warp == kAttnWarps) {
+        if (lane == 0) {
+            asm volatile("createpolicy.fractional.L2::evict_first.b64 %0, 1.0;" : "=l"(policy));
+            for (int it = 0; it < n_tiles && it < kRing; ++it) issue(it);
+        }
+        pdl_wait();
+        if (lane == 0) {
+            for (int it = kRing; it < n_tiles; ++it) {
+                if (!mbar_wait_bounded(&empty[ring_slot(it)], ring_parity(it) ^ 1, kSpinParked)) { failed = 1; break; }
+                issue(it);
+            }
+        }
+        __syncwarp();
+    } else {
+        // rotary row and gains do not depend on the token's vectors: in shared memory before the wait
+        const bool is_q = warp < 2;
+        const int hi_half = lane >> 4, ei = 4 * (lane & 15), g = lane >> 2, t = lane & 3;
+        if (warp < 3) {
+            const bf16* src = warp == 0 ? a.qn : warp == 1 ? a.kn : a.rope + (size_t)n_old * HD;
+            *reinterpret_cast<uint2*>(&rot_s[warp][4 * lane]) = *reinterpret_cast<const uint2*>(src + 4 * lane);
+        }
+        compute_sync();
+        const int e0 = is_q ? (2 * kvh + warp) * HD : (warp == 2 ? DQ : DQ + NKV * HD) + kvh * HD;
+        const bf16* src_row = a.qkv + (size_t)b * DQKV + e0 + 4 * lane;
+        const size_t cache_row = ((size_t)(b * NKV + kvh) * a.kv_cap + n_old) * HD + 4 * lane;
+        const int mat = lane >> 3, r8 = lane & 7;
+        const int group = warp >> 1, w4 = warp & 1;              // the warp's 16 rows of its group's tiles
+        const int krow = 16 * w4 + (mat & 1) * 8 + r8, kchunk = mat >> 1;       // keys: rows +8 in matrix bit 0, columns +8 in bit 1
+        const int vrow = 16 * w4 + (mat >> 1) * 8 + r8, vchunk = mat & 1;       // values: the other way round
+        pdl_wait();
+        const bool owner = rank == 0 && pos >= 0;             // of the new position
+        float r[4] = {0.f, 0.f, 0.f, 0.f};
+        {
+            uint2 u = make_uint2(0u, 0u);
+            if (warp < 4) asm volatile("ld.global.cg.v2.u32 {%0,%1}, [%2];" : "=r"(u.x), "=r"(u.y) : "l"(src_row));
+            float x[4] = {bf_lo(u.x), bf_hi(u.x), bf_lo(u.y), bf_hi(u.y)};
+            if (warp == 3) {
+                if (owner) {
+                    *reinterpret_cast<uint2*>(a.vcache + cache_row) = u;
+#pragma unroll
+                    for (int j = 0; j < 4; ++j) { po[kAttnWarps][0][4 * lane + j] = x[j]; po[kAttnWarps][1][4 * lane + j] = x[j]; }
+                }
+            } else if (is_q || (warp == 2 && owner)) {
+                const float ss = warp_sum(x[0] * x[0] + x[1] * x[1] + x[2] * x[2] + x[3] * x[3]);
+                const float rstd = rsqrt_full(ss * (1.0f / HD) + a.eps);
+                const uint2 gq = *reinterpret_cast<const uint2*>(&rot_s[is_q ? 0 : 1][4 * lane]);
+                const uint2 cq = *reinterpret_cast<const uint2*>(&rot_s[2][ei]), sq = *reinterpret_cast<const uint2*>(&rot_s[2][HD / 2 + ei]);
+                const float gn[4] = {bf_lo(gq.x), bf_hi(gq.x), bf_lo(gq.y), bf_hi(gq.y)};
+                const float cs[4] = {bf_lo(cq.x), bf_hi(cq.x), bf_lo(cq.y), bf_hi(cq.y)};
+                const float sn[4] = {bf_lo(sq.x), bf_hi(sq.x), bf_lo(sq.y), bf_hi(sq.y)};
+#pragma unroll
+                for (int j = 0; j < 4; ++j) {
+                    x[j] = bf16r(bf16r(x[j] * rstd) * gn[j]);
+                    const float y = __shfl_xor_sync(0xffffffffu, x[j], 16);      // element j +- 64
+                    r[j] = hi_half ? bf16r(bf16r(x[j] * cs[j]) + bf16r(y * sn[j])) : bf16r(bf16r(x[j] * cs[j]) + bf16r(-y * sn[j]));
+                }
+                const uint2 pk = make_uint2(pack_bf16x2(r[0], r[1]), pack_bf16x2(r[2], r[3]));
+                *reinterpret_cast<uint2*>((is_q ? q_s[warp] : k_s) + 4 * lane) = pk;
+                if (!is_q) *reinterpret_cast<uint2*>(a.kcache + cache_row) = pk;
+            }
+        }
+        compute_sync();
+        if (warp < 2) {
+            if (owner) {                           // the new position's score for this head
+                const uint2 k2 = *reinterpret_cast<const uint2*>(k_s + 4 * lane);
+                const float s = warp_sum(r[0] * bf_lo(k2.x) + r[1] * bf_hi(k2.x) + r[2] * bf_lo(k2.y) + r[3] * bf_hi(k2.y));
+                if (lane == 0) { pm[kAttnWarps][warp] = s * kScoreScale; pl[kAttnWarps][warp] = 1.f; }
+            } else {
+                if (lane == 0) { pm[kAttnWarps][warp] = -INFINITY; pl[kAttnWarps][warp] = 0.f; }
+#pragma unroll
+                for (int j = 0; j < 4; ++j) po[kAttnWarps][warp][4 * lane + j] = 0.f;
+            }
+        }
+        uint32_t qb[8][2];
+#pragma unroll
+        for (int k = 0; k < 8; ++k) {
+            qb[k][0] = *reinterpret_cast<const uint32_t*>(&q_s[g & 1][16 * k + 2 * t]);         // N columns: heads 0, 1, 0, 1, ...
+            qb[k][1] = *reinterpret_cast<const uint32_t*>(&q_s[g & 1][16 * k + 8 + 2 * t]);
+        }
+        float m0 = -INFINITY, m1 = -INFINITY, l0 = 0.f, l1 = 0.f;
+        float o[8][4];
+#pragma unroll
+        for (int i = 0; i < 8; ++i) { o[i][0] = 0.f; o[i][1] = 0.f; o[i][2] = 0.f; o[i][3] = 0.f; }
+#pragma unroll 1
+        for (int it = group; it < n_tiles; it += kGroups) {
+            const int s = ring_slot(it);
+            bool ok = true;
+            uint32_t spins = 0;
+            while (!mbar_try_wait(&full[s], ring_parity(it))) { if (++spins >= kSpin || failed) { ok = false; break; } }
+            if (!ok) { failed = 1; break; }
+            const int nv = p1 - p0 - it * kTilePos - 16 * w4;  // valid positions of this warp's sixteen
+            if (nv > 0) {
+                const uint32_t tk = smem_u32(ring + s * kTileBytes), tv = tk + 2 * kHalfTile;
+                if (nv < 16) {
+                    // rows past the sequence: whatever the cache holds there (it may be NaN) must not reach P V
+                    for (int i = lane; i < (16 - nv) * 16; i += 32) {
+                        const int row = 16 * w4 + nv + (i >> 4), c = i & 15;
+                        asm volatile("st.shared.v4.u32 [%0], {%1, %1, %1, %1};" ::"r"(swz(tv + (c >> 3) * kHalfTile, row, c & 7)), "r"(0u) : "memory");
+                    }
+                    __syncwarp();
+                }
+                float sa[4] = {0.f, 0.f, 0.f, 0.f}, sb[4] = {0.f, 0.f, 0.f, 0.f};
+#pragma unroll
+                for (int k = 0; k < 8; k += 2) {
+                    uint32_t f[4];
+                    ldsm4(f, swz(tk + (k >> 2) * kHalfTile, krow, 2 * (k & 3) + kchunk));
+                    mma16816(sa, f[0], f[1], f[2], f[3], qb[k][0], qb[k][1]);
+                    ldsm4(f, swz(tk + (k >> 2) * kHalfTile, krow, 2 * ((k + 1) & 3) + kchunk));
+                    mma16816(sb, f[0], f[1], f[2], f[3], qb[k + 1][0], qb[k + 1][1]);
+                }
+                // every lane holds (position g, heads 0 and 1) and (position g + 8, ...)
+                float s0 = (sa[0] + sb[0]) * kScoreScale, s1 = (sa[1] + sb[1]) * kScoreScale;
+                float s2 = (sa[2] + sb[2]) * kScoreScale, s3 = (sa[3] + sb[3]) * kScoreScale;
+                if (g >= nv) { s0 = -INFINITY; s1 = -INFINITY; }
+                if (g + 8 >= nv) { s2 = -INFINITY; s3 = -INFINITY; }
+                // The reference may lag behind the maximum: sums and probabilities are floating point, so nothing is lost
+                // until a score passes it by 2^60.  It starts as the maximum of the warp's first positions.
+                const bool over = fmaxf(s0, s2) > m0 + 60.f || fmaxf(s1, s3) > m1 + 60.f;
+                if (__any_sync(0xffffffffu, over)) {
+                    float x0 = fmaxf(s0, s2), x1 = fmaxf(s1, s3);
+#pragma unroll
+                    for (int of = 4; of < 32; of <<= 1) {
+                        x0 = fmaxf(x0, __shfl_xor_sync(0xffffffffu, x0, of));
+                        x1 = fmaxf(x1, __shfl_xor_sync(0xffffffffu, x1, of));
+                    }
+                    const float n0 = fmaxf(m0, x0), n1 = fmaxf(m1, x1);
+                    const float c0 = ex2f(m0 - n0), c1 = ex2f(m1 - n1);
+                    m0 = n0; m1 = n1; l0 *= c0; l1 *= c1;
+#pragma unroll
+                    for (int i = 0; i < 8; ++i) { o[i][0] *= c0; o[i][1] *= c1; o[i][2] *= c0; o[i][3] *= c1; }
+                }
+                const float e0 = ex2f(s0 - m0), e1 = ex2f(s1 - m1), e2 = ex2f(s2 - m0), e3 = ex2f(s3 - m1);
+                l0 += e0 + e2; l1 += e1 + e3;
+                const uint32_t h01 = pack_bf16x2(e0, e1), h23 = pack_bf16x2(e2, e3);
+                uint32_t u = 0u, v = 0u;
+                if (t == 0) { u = h01; v = h23; }
+                if (t == 1) { u = pack_bf16x2(e0 - bf_lo(h01), e1 - bf_hi(h01)); v = pack_bf16x2(e2 - bf_lo(h23), e3 - bf_hi(h23)); }
+                const uint32_t b0 = movm_t(u), b1 = movm_t(v);
+#pragma unroll
+                for (int i = 0; i < 8; ++i) {
+                    uint32_t f[4];
+                    ldsm4_t(f, swz(tv + (i >> 2) * kHalfTile, vrow, 2 * (i & 3) + vchunk));
+                    mma16816(o[i], f[0], f[1], f[2], f[3], b0, b1);
+                }
+            }
+            __syncwarp();
+            if (lane == 0) asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(&empty[s])) : "memory");
+        }
+#pragma unroll
+        for (int of = 4; of < 32; of <<= 1) { l0 += __shfl_xor_sync(0xffffffffu, l0, of); l1 += __shfl_xor_sync(0xffffffffu, l1, of); }
+        if (lane == 0) { pm[warp][0] = m0; pm[warp][1] = m1; pl[warp][0] = l0; pl[warp][1] = l1; }
+#pragma unroll
+        for (int i = 0; i < 8; ++i) {
+            float v[4];
+#pragma unroll
+            for (int j = 0; j < 4; ++j) v[j] = o[i][j] + __shfl_xor_sync(0xffffffffu, o[i][j], 1);    // high part + low part
+            if (t == 0) { po[warp][0][16 * i + g] = v[0]; po[warp][1][16 * i + g] = v[1]; po[warp][0][16 * i + 8 + g] = v[2]; po[warp][1][16 * i + 8 + g] = v[3]; }
+        }
+        compute_sync();
+        bf16* out = a.attn + (size_t)b * DQ + 2 * kvh * HD;
+        if constexpr (CS > 1) asm volatile("barrier.cluster.wait.acquire;" ::: "memory");
+#pragma unroll
+        for (int e0 = 0; e0 < 2 * HD; e0 += 32 * kAttnWarps) {
+            const int e = e0 + tid, h = e / HD, d = e % HD;
+            if (e >= 2 * HD) break;
+            float m = -1e30f, l = 0.f, acc = 0.f;
+#pragma unroll
+            for (int w = 0; w <= kAttnWarps; ++w) m = fmaxf(m, pm[w][h]);
+#pragma unroll
+            for (int w = 0; w <= kAttnWarps; ++w) { const float c = ex2f(pm[w][h] - m); l = fmaf(pl[w][h], c, l); acc = fmaf(po[w][h][d], c, acc); }
+            if constexpr (CS == 1) {
+                out[e] = __float2bfloat16_rn(l > 0.f ? acc / l : 0.f);
+            } else {
+                // each rank merges NE of the 256 outputs: the partial goes to the rank that owns it
+                constexpr int NE = 2 * HD / CS;
+                st_cluster_f32(&rv[rank][e % NE], e / NE, acc);
+                if (d < CS) { st_cluster_f32(&rm[rank][h], d, m); st_cluster_f32(&rl[rank][h], d, l); }
+            }
+        }
+        if constexpr (CS > 1) {
+            cluster_sync_all();
+            constexpr int NE = 2 * HD / CS;
+            if (tid < NE) {
+                const int e = rank * NE + tid, h = e / HD;
+                float m = -1e30f, acc = 0.f, l = 0.f;
+#pragma unroll
+                for (int q = 0; q < CS; ++q) m = fmaxf(m, rm[q][h]);
+#pragma unroll
+                for (int q = 0; q < CS; ++q) { const float c = ex2f(rm[q][h] - m); acc = fmaf(rv[q][tid], c, acc); l = fmaf(rl[q][h], c, l); }
+                out[e] = __float2bfloat16_rn(l > 0.f ? acc / l : 0.f);
+            }
+        }
+    }
+    if constexpr (CS > 1) {
+        if (warp == kAttnWarps) {                                // the feeding warp's share of the two barriers
+            asm volatile("barrier.cluster.wait.acquire;" ::: "memory");
+            cluster_sync_all();
+        }
+    }
+    __syncthreads();
+    if (failed) {
+        if (tid == 0) {
+            if (atomicCAS(&a.status[0], 0u, (uint32_t)ITTAI_ST_STREAM_TIMEOUT) == 0u) { a.status[1] = (uint32_t)n_tiles; a.status[2] = blockIdx.x; }
+            const long long t0 = clock64();                    // copies still in flight land before the shared memory is handed back
+            while (clock64() - t0 < 2000000) {}
+        }
+        __syncthreads();
+    }
+}
+
+// ---- host side --------------------------------------------------------------------------------------------------------------
+struct Plan {
+    IttaiQwen3Decode p;
+    Buffers w;
+    CUtensorMap tm_k, tm_v;
+    int n_sms = 0;
+    bool bound = false;
+    cudaStream_t side = nullptr;
+    cudaEvent_t last = nullptr;
+    cudaGraphExec_t exec[5][2] = {};      // by log2(CS) and whether the head runs
+    std::mutex mu;
+};
+
+template <typename F>
+static cudaError_t prefer_shared(F* fn, int dynamic = 0) {
+    // every kernel of the chain asks for the same carve-out: CTAs of two kernels share an SM only under one L1 / shared split
+    cudaError_t e = cudaFuncSetAttribute(fn, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared);
+    if (e == cudaSuccess && dynamic > 0) e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, dynamic);
+    return e;
+}
+template <int NB>
+static cudaError_t set_attributes_nb() {
+    cudaError_t e = prefer_shared(gemv_kernel<NB, D, 32, kPlain>, gemv_smem<D, 32>());
+    if (e == cudaSuccess) e = prefer_shared(gemv_kernel<NB, D, 48, kSwiglu>, gemv_smem<D, 48>());
+    if (e == cudaSuccess) e = prefer_shared(gemv_kernel<NB, DQ, 8, kResidual>, gemv_smem<DQ, 8>());
+    if (e == cudaSuccess) e = prefer_shared(gemv_kernel<NB, FF, 8, kResidual>, gemv_smem<FF, 8>());
+    if (e == cudaSuccess) e = prefer_shared(head_kernel<NB>, kHeadSmem);
+    if (e == cudaSuccess) e = prefer_shared(finish_kernel<NB, true>);
+    if (e == cudaSuccess) e = prefer_shared(finish_kernel<NB, false>);
+    return e;
+}
+static cudaError_t set_attributes() {
+    static thread_local int attr_dev = -1;
+    int dev = 0;
+    cudaGetDevice(&dev);
+    if (attr_dev == dev) return cudaSuccess;
+    cudaError_t e = set_attributes_nb<1>();
+    if (e == cudaSuccess) e = set_attributes_nb<2>();
+    if (e == cudaSuccess) e = set_attributes_nb<4>();
+    if (e == cudaSuccess) e = set_attributes_nb<8>();
+    if (e == cudaSuccess) e = prefer_shared(attn_kernel<1>, kAttnSmem);
+    if (e == cudaSuccess) e = prefer_shared(attn_kernel<2>, kAttnSmem);
+    if (e == cudaSuccess) e = prefer_shared(attn_kernel<4>, kAttnSmem);
+    if (e == cudaSuccess) e = prefer_shared(attn_kernel<8>, kAttnSmem);
+    if (e == cudaSuccess) e = prefer_shared(attn_kernel<16>, kAttnSmem);
+    if (e == cudaSuccess) e = cudaFuncSetAttribute(attn_kernel<16>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
+    if (e == cudaSuccess) attr_dev = dev;
+    return e;
+}
+
+template <int CS>
+static cudaError_t launch_attn(const Plan& pl, const AttnChainArgs& a, cudaStream_t st) {
+    return launch_pdl(attn_kernel<CS>, dim3(a.batch * NKV * CS), dim3(kAttnThreads), kAttnSmem, st, CS, pl.tm_k, pl.tm_v, a);
+}
+
+// The kernels of one token, in order, on `st` (captured into a graph, or launched as they are).
+template <int NB>
+static cudaError_t enqueue_token(const Plan& pl, int cs, bool head, cudaStream_t st) {
+    const IttaiQwen3Decode& p = pl.p;
+    const Buffers& w = pl.w;
+    auto bp = [](const void* q, size_t off = 0) { return reinterpret_cast<const bf16*>(q) + off; };
+    cudaError_t e = cudaSuccess;
+    for (int l = 0; l < p.n_layers && e == cudaSuccess; ++l) {
+        const size_t kv = (size_t)l * NB * NKV * p.kv_cap * HD;
+        GemvArgs q{bp(p.wqkv, (size_t)l * DQKV * D), w.h, bp(p.ln1, (size_t)l * D), nullptr, w.qkv, DQKV, p.eps, p.status, nullptr, nullptr, nullptr, 0, nullptr, 0, l == 0};
+        e = launch_pdl(gemv_kernel<NB, D, 32, kPlain>, dim3(DQKV / 32), dim3(kGemvThreads), gemv_smem<D, 32>(), st, 1, q);
+        if (e != cudaSuccess) break;
+        AttnChainArgs a{w.st, w.qkv, bp(p.qn, (size_t)l * HD), bp(p.kn, (size_t)l * HD), bp(p.rope), reinterpret_cast<bf16*>(p.kcache) + kv,
+                        reinterpret_cast<bf16*>(p.vcache) + kv, w.attn, p.status, l, NB, p.kv_cap, p.eps};
+        switch (cs) {
+            case 1: e = launch_attn<1>(pl, a, st); break;
+            case 2: e = launch_attn<2>(pl, a, st); break;
+            case 4: e = launch_attn<4>(pl, a, st); break;
+            case 8: e = launch_attn<8>(pl, a, st); break;
+            default: e = launch_attn<16>(pl, a, st); break;
+        }
+        if (e != cudaSuccess) break;
+        // gate/up finds no room on an SM while attention is there: its weights come as far as L2
+        GemvArgs o{bp(p.wo, (size_t)l * D * DQ), w.attn, nullptr, w.h, w.hmid, D, p.eps, p.status, nullptr, nullptr, nullptr, 0,
+                   reinterpret_cast<const unsigned char*>(bp(p.wgu, (size_t)l * DGU * D)), DGU * D * 2 / (D / 8) / 8, 0};
+        e = launch_pdl(gemv_kernel<NB, DQ, 8, kResidual>, dim3(D / 8), dim3(kGemvThreads), gemv_smem<DQ, 8>(), st, 1, o);
+        if (e != cudaSuccess) break;
+        const bool kv_ahead = l + 1 < p.n_layers;
+        const size_t kv1 = kv + (size_t)NB * NKV * p.kv_cap * HD;
+        GemvArgs gu{bp(p.wgu, (size_t)l * DGU * D), w.hmid, bp(p.ln2, (size_t)l * D), nullptr, w.act, FF, p.eps, p.status, w.st,
+                    kv_ahead ? reinterpret_cast<const bf16*>(p.kcache) + kv1 : nullptr, reinterpret_cast<const bf16*>(p.vcache) + kv1, p.kv_cap, nullptr, 0, 0};
+        e = launch_pdl(gemv_kernel<NB, D, 48, kSwiglu>, dim3(DGU / 48), dim3(kGemvThreads), gemv_smem<D, 48>(), st, 1, gu);
+        if (e != cudaSuccess) break;
+        GemvArgs dn{bp(p.wd, (size_t)l * D * FF), w.act, nullptr, w.hmid, w.h, D, p.eps, p.status, nullptr, nullptr, nullptr, 0, nullptr, 0, 0};
+        e = launch_pdl(gemv_kernel<NB, FF, 8, kResidual>, dim3(D / 8), dim3(kGemvThreads), gemv_smem<FF, 8>(), st, 1, dn);
+    }
+    if (e != cudaSuccess) return e;
+    TokenArgs t{w.st, bp(p.embed), w.h, w.cand_val, w.cand_idx, pl.n_sms, p.pos, p.next_id, p.status, p.vocab, p.kv_cap};
+    if (!head) return launch_pdl(finish_kernel<NB, false>, dim3(1), dim3(32 * NB), 0, st, 1, t);
+    HeadArgs h{bp(p.embed), w.h, bp(p.fin_w), p.write_logits ? reinterpret_cast<bf16*>(p.logits) : nullptr, w.cand_val, w.cand_idx, p.status, p.vocab, p.eps};
+    e = launch_pdl(head_kernel<NB>, dim3(pl.n_sms), dim3(kGemvThreads + 32), kHeadSmem, st, 1, h);
+    if (e != cudaSuccess) return e;
+    return launch_pdl(finish_kernel<NB, true>, dim3(1), dim3(32 * NB), 0, st, 1, t);
+}
+static cudaError_t enqueue_token(const Plan& pl, int cs, bool head, cudaStream_t st) {
+    switch (pl.p.batch) {
+        case 1: return enqueue_token<1>(pl, cs, head, st);
+        case 2: return enqueue_token<2>(pl, cs, head, st);
+        case 4: return enqueue_token<4>(pl, cs, head, st);
+        default: return enqueue_token<8>(pl, cs, head, st);
+    }
+}
+static void enqueue_begin(const Plan& pl, const IttaiQwen3Decode& c, cudaStream_t st) {
+    const IttaiQwen3Decode& p = pl.p;
+    TokenArgs t{pl.w.st, reinterpret_cast<const bf16*>(p.embed), pl.w.h, pl.w.cand_val, pl.w.cand_idx, pl.n_sms, p.pos, p.next_id, p.status, p.vocab, p.kv_cap};
+    switch (p.batch) {
+        case 1: begin_kernel<1><<<1, 32, 0, st>>>(t, c.out_ids, c.forced, c.step_ns, c.n_steps, c.n_forced); break;
+        case 2: begin_kernel<2><<<1, 64, 0, st>>>(t, c.out_ids, c.forced, c.step_ns, c.n_steps, c.n_forced); break;
+        case 4: begin_kernel<4><<<1, 128, 0, st>>>(t, c.out_ids, c.forced, c.step_ns, c.n_steps, c.n_forced); break;
+        default: begin_kernel<8><<<1, 256, 0, st>>>(t, c.out_ids, c.forced, c.step_ns, c.n_steps, c.n_forced); break;
+    }
+}
+
+// log2 of the CTAs per (sequence, kv head) at `len` cached positions.  Measured over all splits and lengths 30 to 8100 (us per
+// step, best split first): 128 CTAs in all are best nearly everywhere (batch 4, 8100: 4 CTAs 1019, 8 1095, 2 1346; batch 2,
+// 8100: 8 CTAs 733, 16 852), because the next projection then still finds room.  Exceptions: a few positions need no split (batch 1, 30:
+// 425, else 428-443), clusters of 16 pay their barrier only from 1200 positions on (batch 1, 800: 8 CTAs 445, 16 451; 3000:
+// 501 and 478), and the longest caches at batch 8 want two CTAs per SM (8100: 4 CTAs 1577, 2 1623; 500: 604 and 592).
+static int cluster_log2(int batch, int len) {
+    if (batch == 4) return 2;
+    if (len <= 48) return 0;
+    if (batch == 1) return len <= 1200 ? 3 : 4;
+    if (batch == 2) return len <= 400 ? 2 : 3;
+    return len <= 700 ? 1 : 2;
+}
+
+static void drop_graphs(Plan* pl) {
+    for (auto& row : pl->exec)
+        for (cudaGraphExec_t& x : row)
+            if (x != nullptr) { cudaGraphExecDestroy(x); x = nullptr; }
+}
+
+}  // namespace chain
+
+void set_error(const char* fmt, ...);
+int cuda_fail(cudaError_t e, const char* what);
+int decode_check_args(const IttaiQwen3Decode* p);      // qwen3_decode.cu
+
+namespace chain {
+
+static int bind(Plan* pl, const IttaiQwen3Decode* p) {
+    pl->p = *p;
+    layout(p->batch, reinterpret_cast<char*>(p->workspace), &pl->w);
+    const long long rows = (long long)p->n_layers * p->batch * NKV * p->kv_cap;
+    if (rows >= (1ll << 31)) { set_error("the cache has %lld rows; at most 2^31 - 1 are supported", rows); return ITTAI_E_ARG; }
+    int rc = make_tmap_bf16(&pl->tm_k, p->kcache, rows, HD, HD, kTilePos);
+    if (rc == ITTAI_OK) rc = make_tmap_bf16(&pl->tm_v, p->vcache, rows, HD, HD, kTilePos);
+    return rc;
+}
+// Whether a graph captured for `a` also serves `b`: everything but the per-call parameters, which travel in State.
+static bool same_binding(const IttaiQwen3Decode& a, const IttaiQwen3Decode& b) {
+    return a.n_layers == b.n_layers && a.vocab == b.vocab && a.kv_cap == b.kv_cap && a.batch == b.batch && a.eps == b.eps && a.write_logits == b.write_logits &&
+           a.wqkv == b.wqkv && a.wo == b.wo && a.wgu == b.wgu && a.wd == b.wd && a.ln1 == b.ln1 && a.ln2 == b.ln2 && a.qn == b.qn && a.kn == b.kn &&
+           a.fin_w == b.fin_w && a.embed == b.embed && a.rope == b.rope && a.kcache == b.kcache && a.vcache == b.vcache && a.pos == b.pos &&
+           a.next_id == b.next_id && a.logits == b.logits && a.workspace == b.workspace && a.status == b.status;
+}
+
+static int capture(Plan* pl, int lg, bool head, cudaGraphExec_t* out) {
+    if (pl->side == nullptr) {
+        const cudaError_t e = cudaStreamCreateWithFlags(&pl->side, cudaStreamNonBlocking);
+        if (e != cudaSuccess) return cuda_fail(e, "cudaStreamCreateWithFlags");
+    }
+    cudaGraph_t g = nullptr;
+    cudaError_t e = cudaStreamBeginCapture(pl->side, cudaStreamCaptureModeThreadLocal);
+    if (e != cudaSuccess) return cuda_fail(e, "cudaStreamBeginCapture");
+    const cudaError_t el = enqueue_token(*pl, 1 << lg, head, pl->side);
+    e = cudaStreamEndCapture(pl->side, &g);
+    if (el != cudaSuccess || e != cudaSuccess) {
+        if (g != nullptr) cudaGraphDestroy(g);
+        cudaGetLastError();
+        return cuda_fail(el != cudaSuccess ? el : e, "capture of a decode step");
+    }
+    e = cudaGraphInstantiate(out, g, 0);
+    cudaGraphDestroy(g);
+    if (e != cudaSuccess) return cuda_fail(e, "cudaGraphInstantiate");
+    return ITTAI_OK;
+}
+
+}  // namespace chain
+}  // namespace ittai
+
+using namespace ittai;
+
+extern "C" int ittai_qwen3_chain_create(void** plan) {
+    if (!plan) { set_error("null plan"); return ITTAI_E_ARG; }
+    *plan = new chain::Plan();
+    return ITTAI_OK;
+}
+
+extern "C" int ittai_qwen3_chain_destroy(void* plan) {
+    chain::Plan* pl = reinterpret_cast<chain::Plan*>(plan);
+    if (pl == nullptr) return ITTAI_OK;
+    if (pl->last != nullptr) { cudaEventSynchronize(pl->last); cudaEventDestroy(pl->last); }
+    chain::drop_graphs(pl);
+    if (pl->side != nullptr) cudaStreamDestroy(pl->side);
+    delete pl;
+    return ITTAI_OK;
+}
+
+extern "C" int ittai_qwen3_chain_run(void* plan, const IttaiQwen3Decode* p, int32_t max_len, void* stream) {
+    chain::Plan* pl = reinterpret_cast<chain::Plan*>(plan);
+    if (!pl || max_len < 0) { set_error("chain_run: null plan or negative length"); return ITTAI_E_ARG; }
+    int rc = decode_check_args(p);
+    if (rc != ITTAI_OK) return rc;
+    cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
+    std::lock_guard<std::mutex> lock(pl->mu);
+    cudaError_t e = chain::set_attributes();
+    if (e != cudaSuccess) return cuda_fail(e, "cudaFuncSetAttribute(decode chain)");
+    if (pl->n_sms == 0) {
+        int dev = 0;
+        cudaGetDevice(&dev);
+        e = cudaDeviceGetAttribute(&pl->n_sms, cudaDevAttrMultiProcessorCount, dev);
+        if (e != cudaSuccess) return cuda_fail(e, "cudaDeviceGetAttribute(sm count)");
+        if (pl->n_sms > chain::kMaxHeadCtas) pl->n_sms = chain::kMaxHeadCtas;
+        e = cudaEventCreateWithFlags(&pl->last, cudaEventDisableTiming);
+        if (e != cudaSuccess) return cuda_fail(e, "cudaEventCreateWithFlags");
+    }
+    if (!pl->bound || !chain::same_binding(pl->p, *p)) {
+        if (pl->bound) { cudaEventSynchronize(pl->last); chain::drop_graphs(pl); }
+        pl->bound = false;
+        rc = chain::bind(pl, p);
+        if (rc != ITTAI_OK) return rc;
+        pl->bound = true;
+    }
+    cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+    e = cudaStreamIsCapturing(st, &cap);
+    if (e != cudaSuccess) return cuda_fail(e, "cudaStreamIsCapturing");
+    chain::enqueue_begin(*pl, *p, st);
+    for (int i = 0; i < p->n_steps; ++i) {
+        const bool head = i >= p->n_forced - 1;
+        const int lg = chain::cluster_log2(p->batch, max_len + i);
+        if (cap != cudaStreamCaptureStatusNone) {      // a graph launch cannot be captured: the kernels themselves can
+            e = chain::enqueue_token(*pl, 1 << lg, head, st);
+        } else {
+            cudaGraphExec_t& x = pl->exec[lg][head ? 1 : 0];
+            if (x == nullptr) {
+                rc = chain::capture(pl, lg, head, &x);
+                if (rc != ITTAI_OK) return rc;
+            }
+            e = cudaGraphLaunch(x, st);
+        }
+        if (e != cudaSuccess) return cuda_fail(e, "launch of a decode step");
+    }
+    if (cap == cudaStreamCaptureStatusNone) {
+        e = cudaEventRecord(pl->last, st);
+        if (e != cudaSuccess) return cuda_fail(e, "cudaEventRecord");
+    }
+    e = cudaGetLastError();
+    return e == cudaSuccess ? ITTAI_OK : cuda_fail(e, "decode chain");
+}

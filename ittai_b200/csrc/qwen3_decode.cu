@@ -1252,7 +1252,7 @@ __global__ void __launch_bounds__(kBlock, 1) q3_phase_kernel(const __grid_consta
 void set_error(const char* fmt, ...);
 int cuda_fail(cudaError_t e, const char* what);
 
-static int check_args(const IttaiQwen3Decode* p) {
+int decode_check_args(const IttaiQwen3Decode* p) {
     if (!p) { set_error("null IttaiQwen3Decode"); return ITTAI_E_ARG; }
     if (p->batch != 1 && p->batch != 2 && p->batch != 4 && p->batch != 8) { set_error("batch %d: supported sizes are 1, 2, 4, 8", p->batch); return ITTAI_E_ARG; }
     if (p->n_layers < 1 || p->vocab < 1 || p->kv_cap < 1 || p->n_steps < 1) { set_error("n_layers, vocab, kv_cap and n_steps must be positive"); return ITTAI_E_ARG; }
@@ -1358,7 +1358,7 @@ static int launch_nb(const IttaiQwen3Decode* p, int phase, int layer, cudaStream
 }
 
 static int launch(const IttaiQwen3Decode* p, int phase, int layer, void* stream) {
-    int rc = check_args(p);
+    int rc = decode_check_args(p);
     if (rc != ITTAI_OK) return rc;
     cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
     switch (p->batch) {

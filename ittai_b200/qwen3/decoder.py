@@ -9,6 +9,7 @@ the argmax fed back on the device.
 from __future__ import annotations
 
 import ctypes as C
+import weakref
 
 import torch
 
@@ -102,6 +103,10 @@ class Qwen3Decoder:
         self._keep = None
         self._phase_clk = None
         self._core = None                    # dense prefill buffers, created at the first long prompt
+        plan = C.c_void_p()                  # graphs of the decode chain, captured at the first token that needs them
+        _C.check(self.lib.ittai_qwen3_chain_create(C.byref(plan)))
+        self._plan = plan
+        weakref.finalize(self, self.lib.ittai_qwen3_chain_destroy, plan)
 
     # ---- plumbing -------------------------------------------------------------------------------
     def _params(self, n_steps, n_forced, forced, out_ids, step_ns, write_logits=True) -> _C.Qwen3Decode:
@@ -166,7 +171,10 @@ class Qwen3Decoder:
         step_ns = torch.zeros(n_steps, dtype=torch.int64, device=self.dev) if timed else None
         p = self._params(n_steps, n_forced, forced, out_ids, step_ns)
         self._keep = (p, forced, out_ids, step_ns)
-        _C.check(self.lib.ittai_qwen3_decode_launch(C.byref(p), self._stream()))
+        if self.flags or self._phase_clk is not None:      # test hooks and the in-kernel profile: the persistent kernel
+            _C.check(self.lib.ittai_qwen3_decode_launch(C.byref(p), self._stream()))
+        else:
+            _C.check(self.lib.ittai_qwen3_chain_run(self._plan, C.byref(p), max(self.lengths) + self._unchecked, self._stream()))
         self._unchecked += n_steps
         if check:
             self.check_status()
