@@ -196,6 +196,12 @@ enum {
                              (reference: the qkv epilogue, src/ittai/qwen3/base.py:84-109) */
 };
 
+/* OR'ed into IttaiGemm.epi: the caller keeps `w` as constant weights (nothing still in flight writes it) and takes any order
+ * of the sum over K.  Where the problem has few output tiles the launch then shares K out over several CTAs, fetches W before
+ * the kernels ahead of it have finished, and covers folded norms, stats_out and ITTAI_EPI_QKROPE at M <= 128 too.  Without it
+ * a row's sums are taken in the same order whatever M is, in a chain (ittai_gemm_chain_launch) too.  Not for chained GEMMs. */
+#define ITTAI_GEMM_STATIC_W 0x100
+
 /* Arguments of ITTAI_EPI_QKROPE: the same arrays ittai_qwen3_qk_rope_scatter takes (all device pointers). */
 typedef struct IttaiQkRope {
     const void* qn;        /* [128] bf16 q_norm gain of this layer */
@@ -285,6 +291,38 @@ typedef struct IttaiAttention {
     uint32_t* status;      /* [ITTAI_STATUS_WORDS] device words, or NULL */
 } IttaiAttention;
 int ittai_attention_launch(const IttaiAttention* a, void* stream);
+
+/* ---- Qwen3 prefill ------------------------------------------------------------------------------------- */
+
+/* One forward of the layer stack over a packed [tokens, 1024] activation matrix: embedding rows, then per layer norm, QKV
+ * projection, QK-norm + RoPE + cache scatter, causal attention, O-projection, gate/up + SwiGLU and down projection, all
+ * launched on `stream` by this one call (about 200 kernels; nothing is allocated, copied or waited for).  The caller owns every
+ * buffer; the residual stream is left in `h`.  The reference's forward: src/ittai/qwen3/engine.py:153-187. */
+typedef struct IttaiQwen3Prefill {
+    int32_t n_layers, vocab;
+    int32_t tokens;        /* T */
+    int32_t n_seqs, max_q_len;
+    int32_t kv_cap;        /* cache rows per (sequence, head) */
+    int32_t fused_rope;    /* 1: QK-norm + RoPE + scatter in the QKV projection's epilogue where one covers it, 0: a pass of its own */
+    int32_t split_k;       /* 1: small forwards may split sums over K (ITTAI_GEMM_STATIC_W), so that a token's values depend on
+                              T in their last bits; 0: they do not depend on what else is packed into the forward */
+    int32_t reserved0;
+    float eps;
+    const void *wqkv, *wo, *wgu, *wd, *ln1, *ln2, *qn, *kn, *embed, *rope;   /* as in IttaiQwen3Decode */
+    const void *wqkv_f, *wgu_f; /* both or neither: the weights with the norm gains folded in along K; the norms then run inside the
+                              GEMMs from T > 128 on (layer 0's first norm reads the embedding rows and stays a pass) */
+    const int32_t *ids, *pos, *seq, *slot;  /* [T] device */
+    const int32_t* seqs;   /* [n_seqs][4] device, as in IttaiAttention */
+    void *kcache, *vcache; /* layer 0's store */
+    int64_t kv_layer;      /* elements from one layer's store to the next (0: one store reused by every layer) */
+    int64_t k_row, k_head, k_seq;  /* strides of the store, elements */
+    int64_t kv_rows_total; /* rows of one layer's store */
+    void *h, *xn, *qkv, *attn, *act;  /* bf16 [T, 1024], [T, 1024], [T, 4096], [T, 2048], [T, 3072] */
+    float* stats;          /* [T][8][2], used with folded norms */
+    const float* zeros;    /* [6144] zeros (the column sums of a folded RMSNorm), used with folded norms */
+    uint32_t* status;      /* as in IttaiGemm */
+} IttaiQwen3Prefill;
+int ittai_qwen3_prefill_launch(const IttaiQwen3Prefill* p, void* stream);
 
 /* ---- row-wise passes around the GEMMs ------------------------------------------------------------------- */
 

@@ -23,9 +23,10 @@ EXPORTS = (
     "ittai_qwen3_decode_workspace_bytes", "ittai_qwen3_decode_launch", "ittai_qwen3_phase_launch",
     "ittai_qwen3_decode_launch_static", "ittai_qwen3_chain_create", "ittai_qwen3_chain_run", "ittai_qwen3_chain_destroy",
     "ittai_gemm_bf16_launch", "ittai_gemm_chain_launch", "ittai_attention_launch", "ittai_rmsnorm_rows", "ittai_layernorm_rows", "ittai_row_stats",
-    "ittai_qwen3_qk_rope_scatter", "ittai_siglip_im2col", "ittai_embed_rows", "ittai_qwen3_final_pool",
+    "ittai_qwen3_prefill_launch", "ittai_qwen3_qk_rope_scatter", "ittai_siglip_im2col", "ittai_embed_rows", "ittai_qwen3_final_pool",
 )
 EPI_NONE, EPI_GELU, EPI_SWIGLU, EPI_QKROPE = range(4)
+GEMM_STATIC_W = 0x100
 
 
 class IttaiError(RuntimeError):
@@ -79,6 +80,21 @@ class Attention(C.Structure):
     ]
 
 
+class Qwen3Prefill(C.Structure):
+    """Mirror of ``struct IttaiQwen3Prefill``."""
+    _fields_ = [
+        ("n_layers", C.c_int32), ("vocab", C.c_int32), ("tokens", C.c_int32), ("n_seqs", C.c_int32), ("max_q_len", C.c_int32),
+        ("kv_cap", C.c_int32), ("fused_rope", C.c_int32), ("split_k", C.c_int32), ("reserved0", C.c_int32), ("eps", C.c_float),
+        ("wqkv", C.c_void_p), ("wo", C.c_void_p), ("wgu", C.c_void_p), ("wd", C.c_void_p), ("ln1", C.c_void_p), ("ln2", C.c_void_p),
+        ("qn", C.c_void_p), ("kn", C.c_void_p), ("embed", C.c_void_p), ("rope", C.c_void_p), ("wqkv_f", C.c_void_p), ("wgu_f", C.c_void_p),
+        ("ids", C.c_void_p), ("pos", C.c_void_p), ("seq", C.c_void_p), ("slot", C.c_void_p), ("seqs", C.c_void_p),
+        ("kcache", C.c_void_p), ("vcache", C.c_void_p), ("kv_layer", C.c_int64), ("k_row", C.c_int64), ("k_head", C.c_int64),
+        ("k_seq", C.c_int64), ("kv_rows_total", C.c_int64),
+        ("h", C.c_void_p), ("xn", C.c_void_p), ("qkv", C.c_void_p), ("attn", C.c_void_p), ("act", C.c_void_p),
+        ("stats", C.c_void_p), ("zeros", C.c_void_p), ("status", C.c_void_p),
+    ]
+
+
 _lib = None
 
 
@@ -104,6 +120,7 @@ def lib() -> C.CDLL:
     L.ittai_gemm_bf16_launch.argtypes = [C.POINTER(Gemm), C.c_void_p]
     L.ittai_gemm_chain_launch.argtypes = [C.POINTER(Gemm), C.c_int32, C.c_void_p, C.c_void_p]
     L.ittai_attention_launch.argtypes = [C.POINTER(Attention), C.c_void_p]
+    L.ittai_qwen3_prefill_launch.argtypes = [C.POINTER(Qwen3Prefill), C.c_void_p]
     vp, i32, f32 = C.c_void_p, C.c_int, C.c_float
     L.ittai_rmsnorm_rows.argtypes = [vp, i32, vp, vp, i32, i32, f32, vp]
     L.ittai_layernorm_rows.argtypes = [vp, i32, vp, vp, vp, i32, i32, i32, f32, vp]

@@ -4,8 +4,9 @@
 // GEMM epilogues fuse (src/ittai/qwen3/base.py:110-129, src/ittai/siglip/kernel.py:266-333): bias, residual add,
 // GELU-tanh, SwiGLU on interleaved gate/up columns.
 //
-// This file: argument checking and dispatch (M > 128 goes to the two-SM kernel of gemm2_sm100.cu), and the one-SM
-// kernel for M <= 128.  Persistent, one CTA per SM, looping over 128 x TN output tiles (tile t = blockIdx.x +
+// This file: argument checking and dispatch (split-K kernel of gemm_split_sm100.cu: constant weights and few output tiles;
+// M > 128: the two-SM kernel of gemm2_sm100.cu), and the one-SM kernel for M <= 128 where K may not be split: it and the
+// two-SM kernel sum in the same order, so that a row's result does not depend on how many rows share the launch.  Persistent, one CTA per SM, looping over 128 x TN output tiles (tile t = blockIdx.x +
 // i * gridDim.x, N fastest, the reference's "N-tile outer, M-block inner" grouping: src/ittai/qwen3/engine.py:53-63).
 // Warp 0 (one lane) streams 128 x 64 A tiles and TN x 64 W tiles through a ring of shared-memory stages with TMA
 // (128-byte swizzle); warp 1 owns the TMEM columns as two TN-column accumulators and (one lane) issues four
@@ -16,6 +17,7 @@
 #include <cuda.h>
 
 #include "gemm_epilogue.cuh"
+#include "gemm_split.h"
 #include "tmap.h"
 #include "launch.h"
 
@@ -165,34 +167,35 @@ int cuda_fail(cudaError_t e, const char* what);
 
 int gemm2_bf16_launch(const CUtensorMap& tm_a, const CUtensorMap& tm_b, const GemmArgs& g, cudaStream_t st);   // gemm2_sm100.cu
 
-// Checks one IttaiGemm and turns it into kernel arguments and the operand tensor maps (`pair`: the two-SM kernel's W box).
-int gemm_args_from_abi(const IttaiGemm* a, GemmArgs* gp, CUtensorMap* tm_a, CUtensorMap* tm_b, bool pair) {
+// Checks one IttaiGemm and turns it into kernel arguments and the operand tensor maps (`box_w`: rows of a W box).
+// `any_m`: folded norms, output statistics and the rotary epilogue are allowed at M <= 128 too (ITTAI_GEMM_STATIC_W).
+int gemm_args_from_abi(const IttaiGemm* a, GemmArgs* gp, CUtensorMap* tm_a, CUtensorMap* tm_b, int epi, bool any_m, int box_w) {
     if (!a || !a->a || !a->w || !a->out || !a->status) { set_error("null pointer in IttaiGemm"); return ITTAI_E_ARG; }
     if (a->m < 1 || a->n < GN || a->n % GN != 0 || a->k < GK || a->k % GK != 0) {
         set_error("gemm shape M=%d N=%d K=%d: N must be a multiple of %d and K of %d", a->m, a->n, a->k, GN, GK);
         return ITTAI_E_ARG;
     }
-    if (a->epi < ITTAI_EPI_NONE || a->epi > ITTAI_EPI_QKROPE) { set_error("unknown epilogue %d", a->epi); return ITTAI_E_ARG; }
-    if (a->epi == ITTAI_EPI_QKROPE) {
+    if (epi < ITTAI_EPI_NONE || epi > ITTAI_EPI_QKROPE) { set_error("unknown epilogue %d", a->epi); return ITTAI_E_ARG; }
+    if (epi == ITTAI_EPI_QKROPE) {
         const IttaiQkRope* r = a->qk_rope;
-        if (a->n != ITTAI_Q3_DQKV || a->m <= GM || a->bias || a->residual || (a->row_stats && !(a->stats_rms && a->stats_parts > 0)) || a->stats_out ||
+        if (a->n != ITTAI_Q3_DQKV || (a->m <= GM && !any_m) || a->bias || a->residual || (a->row_stats && !(a->stats_rms && a->stats_parts > 0)) || a->stats_out ||
             !r || !r->qn || !r->kn || !r->rope ||
             !r->pos || !r->seq || !r->slot || !r->kcache_layer || !r->vcache_layer || r->kv_cap < 1) {
             set_error("the QK-norm + RoPE epilogue needs N = %d, M > %d, no bias / residual / output statistics, row statistics only as RMS partial sums, and a complete IttaiQkRope", ITTAI_Q3_DQKV, GM);
             return ITTAI_E_ARG;
         }
     }
-    if (a->epi == ITTAI_EPI_SWIGLU && a->residual) { set_error("SwiGLU epilogue takes no residual"); return ITTAI_E_ARG; }
-    if ((a->row_stats == nullptr) != (a->col_sums == nullptr) || (a->row_stats != nullptr && a->m <= GM)) {
+    if (epi == ITTAI_EPI_SWIGLU && a->residual) { set_error("SwiGLU epilogue takes no residual"); return ITTAI_E_ARG; }
+    if ((a->row_stats == nullptr) != (a->col_sums == nullptr) || (a->row_stats != nullptr && a->m <= GM && !any_m)) {
         set_error("a folded LayerNorm needs both row_stats and col_sums, and M > %d", GM);
         return ITTAI_E_ARG;
     }
-    if (a->stats_out != nullptr && (a->m <= GM || a->epi == ITTAI_EPI_SWIGLU)) { set_error("stats_out needs M > %d and no SwiGLU", GM); return ITTAI_E_ARG; }
+    if (a->stats_out != nullptr && ((a->m <= GM && !any_m) || epi == ITTAI_EPI_SWIGLU)) { set_error("stats_out needs M > %d and no SwiGLU", GM); return ITTAI_E_ARG; }
     if (a->stats_parts < 0 || a->stats_parts > 64) { set_error("stats_parts %d out of range", a->stats_parts); return ITTAI_E_ARG; }
     if (a->stats_k < 0 || a->stats_k > a->k) { set_error("stats_k %d: between 0 and K", a->stats_k); return ITTAI_E_ARG; }
     if (a->stats_rms != 0 && (a->stats_rms != 1 || a->stats_parts <= 0)) { set_error("stats_rms is 0 or 1 and needs partial sums (stats_parts > 0)"); return ITTAI_E_ARG; }
     const int ld_a = a->ld_a ? a->ld_a : a->k, ld_w = a->ld_w ? a->ld_w : a->k;
-    const int n_out = a->epi == ITTAI_EPI_SWIGLU ? a->n / 2 : a->n;
+    const int n_out = epi == ITTAI_EPI_SWIGLU ? a->n / 2 : a->n;
     const int ld_out = a->ld_out ? a->ld_out : n_out, ld_res = a->ld_res ? a->ld_res : a->n;
     if (((uintptr_t)a->a & 15) || ((uintptr_t)a->w & 15) || ((uintptr_t)a->out & 15) || ((uintptr_t)a->residual & 15) ||
         ((uintptr_t)a->bias & 15) || ld_a % 8 || ld_w % 8 || ld_out % 8 || ld_res % 8) {
@@ -201,10 +204,10 @@ int gemm_args_from_abi(const IttaiGemm* a, GemmArgs* gp, CUtensorMap* tm_a, CUte
     }
     int rc = make_tmap_bf16(tm_a, a->a, a->m, a->k, ld_a, GM);
     if (rc != ITTAI_OK) return rc;
-    rc = make_tmap_bf16(tm_b, a->w, a->n, a->k, ld_w, pair ? GN / 2 : 64);
+    rc = make_tmap_bf16(tm_b, a->w, a->n, a->k, ld_w, box_w);
     if (rc != ITTAI_OK) return rc;
     GemmArgs& g = *gp;
-    g.M = a->m; g.N = a->n; g.K = a->k; g.epi = a->epi;
+    g.M = a->m; g.N = a->n; g.K = a->k; g.epi = epi;
     g.bias = reinterpret_cast<const float*>(a->bias);
     g.residual = reinterpret_cast<const bf16*>(a->residual);
     g.ld_res = ld_res;
@@ -218,32 +221,31 @@ int gemm_args_from_abi(const IttaiGemm* a, GemmArgs* gp, CUtensorMap* tm_a, CUte
     g.stats_eps = a->stats_eps;
     g.stats_k = a->stats_k;
     g.stats_rms = a->stats_rms;
-    if (a->epi == ITTAI_EPI_QKROPE) g.rope = *a->qk_rope; else g.rope = IttaiQkRope{};
+    if (epi == ITTAI_EPI_QKROPE) g.rope = *a->qk_rope; else g.rope = IttaiQkRope{};
     return ITTAI_OK;
 }
 
 int gemm_bf16_launch(const IttaiGemm* a, cudaStream_t st) {
-    // more than one 128-row tile: the two-SM kernel (each CTA of a pair loads 128 rows of A and 128 rows of W per stage)
-    const bool pair = a != nullptr && a->m > GM;
-    CUtensorMap tm_a, tm_b;
-    GemmArgs g;
-    const int rc = gemm_args_from_abi(a, &g, &tm_a, &tm_b, pair);
-    if (rc != ITTAI_OK) return rc;
-    static thread_local int attr_dev = -1, n_sms = 0;
+    static thread_local int sm_dev = -1, attr_dev = -1, n_sms = 0;
     int dev = 0;
     cudaGetDevice(&dev);
+    if (sm_dev != dev && cudaDeviceGetAttribute(&n_sms, cudaDevAttrMultiProcessorCount, dev) == cudaSuccess) sm_dev = dev;
+    const bool static_w = a != nullptr && (a->epi & ITTAI_GEMM_STATIC_W) != 0;
+    const bool split = static_w && gemm_split_wins(a->m, a->n, n_sms), pair = !split && a != nullptr && a->m > GM;
+    CUtensorMap tm_a, tm_b;
+    GemmArgs g;
+    const int rc = gemm_args_from_abi(a, &g, &tm_a, &tm_b, a ? a->epi & ~ITTAI_GEMM_STATIC_W : 0, split, split || pair ? 128 : 64);
+    if (rc != ITTAI_OK) return rc;
+    if (split) return gemm_split_launch(tm_a, tm_b, g, n_sms, st);
+    if (pair) return gemm2_bf16_launch(tm_a, tm_b, g, st);
     if (attr_dev != dev) {
-        cudaError_t e = cudaFuncSetAttribute(gemm_bf16_kernel<64, 8>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)GemmCfg<64, 8>::kSmem);
+        const cudaError_t e = cudaFuncSetAttribute(gemm_bf16_kernel<64, 8>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)GemmCfg<64, 8>::kSmem);
         if (e != cudaSuccess) return cuda_fail(e, "cudaFuncSetAttribute(gemm)");
-        e = cudaDeviceGetAttribute(&n_sms, cudaDevAttrMultiProcessorCount, dev);
-        if (e != cudaSuccess) return cuda_fail(e, "cudaDeviceGetAttribute(sm count)");
         attr_dev = dev;
     }
-    if (pair) return gemm2_bf16_launch(tm_a, tm_b, g, st);
     const int tiles = ((a->m + GM - 1) / GM) * (a->n / 64);
-    cudaError_t e = launch_pdl(gemm_bf16_kernel<64, 8>, dim3(tiles < n_sms ? tiles : n_sms), dim3(kGemmThreads), GemmCfg<64, 8>::kSmem, st, 1, tm_a, tm_b, g);
-    if (e != cudaSuccess) return cuda_fail(e, "launch gemm_bf16_kernel");
-    return ITTAI_OK;
+    const cudaError_t e = launch_pdl(gemm_bf16_kernel<64, 8>, dim3(tiles < n_sms ? tiles : n_sms), dim3(kGemmThreads), GemmCfg<64, 8>::kSmem, st, 1, tm_a, tm_b, g);
+    return e == cudaSuccess ? ITTAI_OK : cuda_fail(e, "launch gemm_bf16_kernel");
 }
 
 }  // namespace ittai

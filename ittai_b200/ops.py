@@ -24,7 +24,7 @@ def _stream(t: torch.Tensor):
 def gemm_desc(a: torch.Tensor, w: torch.Tensor, status: torch.Tensor, bias: torch.Tensor | None = None,
               residual: torch.Tensor | None = None, epi: int = _C.EPI_NONE, out: torch.Tensor | None = None,
               row_stats: torch.Tensor | None = None, col_sums: torch.Tensor | None = None, stats_out: torch.Tensor | None = None,
-              stats_eps: float = 0.0, qk_rope: dict | None = None, stats_k: int = 0, stats_rms: bool = False):
+              stats_eps: float = 0.0, qk_rope: dict | None = None, stats_k: int = 0, stats_rms: bool = False, static_w: bool = False):
     """The ``IttaiGemm`` record of ``gemm(...)`` with the same arguments, and its output tensor: ``(record, out)``.
 
     ``out = epilogue(a @ w.T)`` on the tcgen05 GEMM: a [M, K] and w [N, K] bf16 (last dim contiguous), bias fp32 [N],
@@ -34,7 +34,9 @@ def gemm_desc(a: torch.Tensor, w: torch.Tensor, status: torch.Tensor, bias: torc
     (fp32 [M, N/128, 2]) receives the (sum, sum of squares) of every 128-column slice of the output rows; passed as the
     ``row_stats`` of the next GEMM (3-D, with ``stats_eps``) it replaces the separate statistics pass.  ``epi=EPI_QKROPE``
     (Qwen3 QKV projection, N = 4096, M > 128) takes ``qk_rope`` = dict(qn, kn, rope, pos, seq, slot, kcache, vcache,
-    kv_cap, eps) and does the work of the QK-norm + RoPE + cache-scatter pass in its epilogue."""
+    kv_cap, eps) and does the work of the QK-norm + RoPE + cache-scatter pass in its epilogue.  ``static_w``: ``w`` is constant
+    weights, long written, and any order of the sum over K is fine: few output tiles are then split over K, and the
+    M > 128 limits fall away."""
     assert a.dtype == torch.bfloat16 and w.dtype == torch.bfloat16 and a.stride(1) == 1 and w.stride(1) == 1
     m, k = a.shape
     n = w.shape[0]
@@ -43,7 +45,7 @@ def gemm_desc(a: torch.Tensor, w: torch.Tensor, status: torch.Tensor, bias: torc
     if out is None:
         out = torch.empty(m, n_out, dtype=torch.bfloat16, device=a.device)
     g = _C.Gemm()
-    g.m, g.n, g.k, g.epi = m, n, k, epi
+    g.m, g.n, g.k, g.epi = m, n, k, epi | (_C.GEMM_STATIC_W if static_w else 0)
     g.ld_a, g.ld_w, g.ld_out = a.stride(0), w.stride(0), out.stride(0)
     g.a, g.w, g.out, g.status = a.data_ptr(), w.data_ptr(), out.data_ptr(), status.data_ptr()
     if bias is not None:

@@ -11,6 +11,7 @@ from __future__ import annotations
 import ctypes as C
 import weakref
 
+import numpy as np
 import torch
 
 from .. import _C
@@ -91,7 +92,9 @@ class Qwen3Decoder:
         self.pos = z(self.B, dt=torch.int32)
         self.next_id = z(self.B, dt=torch.int32)
         self.logits = z(self.B, self.V)
-        self.status = z(_C.STATUS_WORDS, dt=torch.int32)
+        self._status = z(2, _C.STATUS_WORDS, dt=torch.int32)     # the decode kernels' words, then the prefill kernels'
+        self.status = self._status[0]
+        self._prefilled = False              # a prefill was queued whose status has not been read yet
         nbytes = C.c_size_t()
         _C.check(self.lib.ittai_qwen3_decode_workspace_bytes(self.B, C.byref(nbytes)))
         self.workspace = z(nbytes.value + 256, dt=torch.uint8)
@@ -134,8 +137,12 @@ class Qwen3Decoder:
         A launch that aborts leaves the device positions where they were (the kernel advances ``pos`` only when every
         step completed), so the host mirror ``lengths`` is advanced here, after the verdict, and re-read from the device
         when a launch failed: a later prefill or decode then works on consistent positions."""
+        decode, prefill = self._status.cpu().tolist()
         try:
-            _C.decode_status(self.status.cpu().tolist())
+            if self._prefilled:
+                self._prefilled = False
+                _C.decode_status(prefill)
+            _C.decode_status(decode)
         except _C.IttaiError:
             self._unchecked = 0
             self.lengths = self.pos.cpu().tolist()
@@ -198,7 +205,7 @@ class Qwen3Decoder:
         if tensor_cores is None:
             tensor_cores = T >= 32
         if tensor_cores and T > 1:
-            self._prefill_dense(ids[:, :T - 1])
+            self._prefill_dense(ids[:, :T - 1], check=False)     # the launch below reads both verdicts
             ids = ids[:, T - 1:]
         forced = ids.t().contiguous().to(self.dev, non_blocking=True)       # [T, B]
         out, _ = self._launch(forced.shape[0], forced=forced)
@@ -208,42 +215,14 @@ class Qwen3Decoder:
         """Append token ids to the caches of SOME sequences of the batch, each with its own length: ``prompts`` maps a
         sequence index to a 1-D id list.  The other sequences' caches and positions stay as they are.  Tensor-core
         prefill, tokens of all named sequences packed into one activation matrix (the varlen packing of the reference's
-        engine, ``src/ittai/qwen3/engine.py:20,149-150``); no logits are produced."""
-        from .engine import PrefillCore
-        if self._unchecked:
-            self.check_status()
-        todo = {int(b): torch.as_tensor(t, dtype=torch.int32).reshape(-1) for b, t in prompts.items() if len(t) > 0}
-        if not todo:
-            return
-        for b, t in todo.items():
+        engine, ``src/ittai/qwen3/engine.py:20,149-150``); no logits are produced.  Nothing is waited for: the verdict of
+        the kernels' bounded waits is read by the next ``check_status``, which every ``decode`` calls."""
+        todo = {int(b): torch.as_tensor(t, dtype=torch.int32).reshape(-1).cpu().numpy() for b, t in prompts.items() if len(t) > 0}
+        for b in todo:
             if not 0 <= b < self.B:
                 raise ValueError(f"sequence {b} outside 0..{self.B - 1}")
-            if int(t.min()) < 0 or int(t.max()) >= self.V:
-                raise ValueError(f"token id outside [0, {self.V})")
-            if self.lengths[b] + len(t) > self.cap:
-                raise ValueError(f"KV capacity {self.cap} exceeded: {self.lengths[b]} cached + {len(t)} prompt tokens")
-        total = sum(len(t) for t in todo.values())
-        if self._core is None or self._core.M < total:
-            self._core = PrefillCore(self.w, self.L, max(total, 256), self.dev)
-        i32 = lambda x: torch.as_tensor(x, dtype=torch.int32).to(self.dev, non_blocking=True)
-        tokens, pos, seq, seqs, row = [], [], [], [], 0
-        for b in range(self.B):                       # one record per sequence of the batch: the record index names the cache
-            n = len(todo[b]) if b in todo else 0
-            seqs.append([row, n, 0, self.lengths[b] + n])
-            if n:
-                tokens.append(todo[b])
-                pos.append(torch.arange(self.lengths[b], self.lengths[b] + n, dtype=torch.int32))
-                seq.append(torch.full((n,), b, dtype=torch.int32))
-                row += n
-        pos_d = i32(torch.cat(pos))
-        self._core.status.zero_()
-        self._core.run(total, i32(torch.cat(tokens)), pos_d, i32(torch.cat(seq)), pos_d, i32(seqs), max(len(t) for t in todo.values()),
-                       self.rope, lambda l: (self.kcache[l], self.vcache[l]), self.cap, (HD, self.cap * HD, NKV * self.cap * HD))
-        for b, t in todo.items():
-            self.lengths[b] += len(t)
-        self.pos.copy_(i32(self.lengths))
-        from .. import ops
-        ops.check_status(self._core.status)
+        if todo:
+            self._prefill_rows(todo, check=False, split_k=False)     # a request's tokens must not depend on its neighbours
 
     def set_length(self, b: int, length: int) -> None:
         """Set ONE sequence's cache length (0 frees the slot for a new request)."""
@@ -254,32 +233,41 @@ class Qwen3Decoder:
         self.lengths[b] = length
         self.pos[b] = length
 
-    def _prefill_dense(self, ids: torch.Tensor) -> None:
+    def _prefill_dense(self, ids: torch.Tensor, check: bool = True) -> None:
         """Append ``ids`` ([B, n]) to every sequence's cache with the dense prefill kernels."""
-        from .engine import PrefillCore
-        B, n = ids.shape
-        if self._unchecked:
+        self._prefill_rows(dict(enumerate(ids.cpu().numpy())), check)
+
+    def _prefill_rows(self, todo: dict, check: bool, split_k: bool = True) -> None:
+        """``todo``: ids (int32 numpy, at least one) per sequence index, in any order."""
+        from .engine import PrefillCore, upload
+        if self._unchecked or self._prefilled:
             self.check_status()
-        if int(ids.min()) < 0 or int(ids.max()) >= self.V:
-            raise ValueError(f"token id outside [0, {self.V})")
-        if max(self.lengths) + n > self.cap:
-            raise ValueError(f"KV capacity {self.cap} exceeded: {max(self.lengths)} cached + {n} prompt tokens")
-        if self._core is None or self._core.M < B * n:
-            self._core = PrefillCore(self.w, self.L, max(B * n, 256), self.dev)
-        i32 = lambda x: torch.as_tensor(x, dtype=torch.int32).to(self.dev, non_blocking=True)
-        base = torch.tensor(self.lengths, dtype=torch.int32)
-        pos = (base[:, None] + torch.arange(n, dtype=torch.int32)[None, :]).reshape(-1)
-        seq = torch.arange(B, dtype=torch.int32)[:, None].expand(B, n).reshape(-1)
-        seqs = torch.tensor([[b * n, n, 0, self.lengths[b] + n] for b in range(B)], dtype=torch.int32)
-        pos_d = i32(pos)
+        for b, t in todo.items():
+            if int(t.min()) < 0 or int(t.max()) >= self.V:
+                raise ValueError(f"token id outside [0, {self.V})")
+            if self.lengths[b] + len(t) > self.cap:
+                raise ValueError(f"KV capacity {self.cap} exceeded: {self.lengths[b]} cached + {len(t)} prompt tokens")
+        total = sum(len(t) for t in todo.values())
+        if self._core is None or self._core.M < total:
+            self._core = PrefillCore(self.w, self.L, max(total, 256), self.dev, status=self._status[1])
+        none = np.zeros(0, np.int32)
+        rows = [todo.get(b, none) for b in range(self.B)]         # one record per sequence: the record index names the cache
+        counts, base = np.array([len(t) for t in rows]), np.array(self.lengths)
+        first = np.cumsum(counts) - counts
+        seqs = np.stack([first, counts, np.zeros_like(counts), base + counts], 1)
+        pos = np.arange(total) - np.repeat(first - base, counts)
+        meta = upload((seqs, base + counts, np.concatenate(rows), pos, np.repeat(np.arange(self.B), counts))).to(self.dev, non_blocking=True)
+        seqs_d, lengths_d = meta[:4 * self.B].view(self.B, 4), meta[4 * self.B:5 * self.B]
+        tokens_d, pos_d, seq_d = meta[5 * self.B:].view(3, total)
         cap = self.cap
         self._core.status.zero_()
-        self._core.run(B * n, i32(ids.reshape(-1)), pos_d, i32(seq), pos_d, i32(seqs), n, self.rope,
-                       lambda l: (self.kcache[l], self.vcache[l]), cap, (HD, cap * HD, NKV * cap * HD))
-        self.pos += n
-        self.lengths = [x + n for x in self.lengths]
-        from .. import ops
-        ops.check_status(self._core.status)
+        self._core.run(total, tokens_d, pos_d, seq_d, pos_d, seqs_d, int(counts.max()), self.rope, self.kcache, self.vcache,
+                       self.B * NKV * cap * HD, cap, (HD, cap * HD, NKV * cap * HD), split_k)
+        self.pos.copy_(lengths_d)
+        self.lengths = (base + counts).tolist()
+        self._prefilled = True
+        if check:
+            self.check_status()
 
     @torch.no_grad()
     def decode(self, n_steps: int, timed: bool = False, check: bool = True):

@@ -10,6 +10,7 @@ decoder reuses it to fill its KV cache from a prompt.
 from __future__ import annotations
 
 import ctypes as C
+import itertools
 
 import numpy as np
 import torch
@@ -43,14 +44,24 @@ def packing(seqlens):
     return pos, seq, slot, seqs, T
 
 
+def upload(arrays) -> torch.Tensor:
+    """int32 arrays behind one another in one host tensor, to be copied to the device at once.  A large one is pinned (a
+    pageable copy beyond the driver's staging size would wait for the stream); torch's host allocator keeps the block until
+    the copy has run."""
+    n = sum(a.size for a in arrays)
+    t = torch.empty(n, dtype=torch.int32, pin_memory=n > 8192)
+    np.concatenate([a.reshape(-1) for a in arrays], out=t.numpy())
+    return t
+
+
 class PrefillCore:
     """The 28-layer loop over a packed ``[T, 1024]`` activation matrix.  Owns the activation buffers (torch tensors, as
     the reference's Engine owns its buffers: ``src/ittai/qwen3/engine.py:123-134``); weights and the key/value store are
     borrowed."""
 
-    def __init__(self, w: dict, n_layers: int, max_tokens: int, device, fused_rope: bool = True, fold_norm: bool = False):
+    def __init__(self, w: dict, n_layers: int, max_tokens: int, device, fused_rope: bool = True, fold_norm: bool = False, status=None):
         self.w, self.L, self.M, self.dev = w, n_layers, max_tokens, device
-        self.fused_rope = fused_rope       # QK-norm + RoPE + cache scatter inside the QKV GEMM's epilogue (needs > 128 rows)
+        self.fused_rope = fused_rope       # QK-norm + RoPE + cache scatter inside the QKV GEMM's epilogue
         # ``fold_norm``: the RMSNorms in front of the QKV and gate/up projections are folded into those GEMMs, as in the
         # reference's kernels (``src/ittai/qwen3/engine.py:107-114``: gain folded into the weights in fp32 and rounded once;
         # ``base.py:59-78``: the residual epilogue before leaves per-row partial sums of squares, the consuming epilogue
@@ -61,48 +72,30 @@ class PrefillCore:
             fold = lambda W, g: (W.float() * g.float()[:, None, :]).to(torch.bfloat16).contiguous()
             self.wqkv_f, self.wgu_f = fold(w["wqkv"], w["ln1"]), fold(w["wgu"], w["ln2"])
             self.stats = torch.zeros(max_tokens, D // 128, 2, dtype=torch.float32, device=device)
-            self.zeros_qkv, self.zeros_gu = (torch.zeros(n, dtype=torch.float32, device=device) for n in (DQKV, DGU))
+            self.zeros = torch.zeros(DGU, dtype=torch.float32, device=device)
         z = lambda *s: torch.empty(*s, dtype=torch.bfloat16, device=device)
         self.h, self.xn, self.qkv, self.attn, self.act = z(max_tokens, D), z(max_tokens, D), z(max_tokens, DQKV), z(max_tokens, DQ), z(max_tokens, FF)
-        self.status = ops.new_status(device)
+        self.status = ops.new_status(device) if status is None else status
 
-    def run(self, T, tokens, pos, seq, slot, seqs, max_q_len, rope, kv_layer, kv_cap, k_strides):
-        """``tokens/pos/seq/slot``: int32 device ``[T]``; ``seqs``: int32 device ``[n, 4]``; ``kv_layer(l)`` returns the
-        (K, V) tensors of layer ``l`` laid out ``[B, 8, kv_cap, 128]``; ``k_strides`` = (row, head, seq) in elements."""
-        L, st, w = _C.lib(), self.status, self.w
-        h, xn, qkv, attn, act = self.h[:T], self.xn[:T], self.qkv[:T], self.attn[:T], self.act[:T]
-        s = ops._stream(h)
-        _C.check(L.ittai_embed_rows(tokens.data_ptr(), w["embed"].data_ptr(), h.data_ptr(), T, w["embed"].shape[0], s))
-        fold = self.fold_norm and T > 128
-        for l in range(self.L):
-            kc, vc = kv_layer(l)
-            # layer 0 reads the embedding rows, which no GEMM epilogue produced: its first norm is a pass of its own
-            folded = fold and l > 0
-            if folded:
-                x_in, wq, ln = h, self.wqkv_f[l], dict(row_stats=self.stats[:T], col_sums=self.zeros_qkv, stats_eps=EPS, stats_rms=True)
-            else:
-                ops.rmsnorm_rows(h, w["ln1"][l], EPS, out=xn)
-                x_in, wq, ln = xn, w["wqkv"][l], {}
-            if T > 128 and self.fused_rope:
-                # QK-norm + RoPE + cache scatter inside the QKV GEMM's epilogue (the reference's qkv epilogue, base.py:84-109)
-                ops.gemm(x_in, wq, st, out=qkv, epi=_C.EPI_QKROPE, **ln,
-                         qk_rope=dict(qn=w["qn"][l], kn=w["kn"][l], rope=rope, pos=pos, seq=seq, slot=slot, kcache=kc, vcache=vc, kv_cap=kv_cap, eps=EPS))
-            else:
-                ops.gemm(x_in, wq, st, out=qkv, **ln)
-                _C.check(L.ittai_qwen3_qk_rope_scatter(qkv.data_ptr(), w["qn"][l].data_ptr(), w["kn"][l].data_ptr(), rope.data_ptr(),
-                                                       pos.data_ptr(), seq.data_ptr(), slot.data_ptr(), kc.data_ptr(), vc.data_ptr(),
-                                                       T, kv_cap, EPS, s))
-            ops.attention(qkv, kc, vc, attn, seqs, n_heads=NH, group=NH // NKV, head_dim=HD, causal=True, max_q_len=max_q_len,
-                          q_strides=(DQKV, HD), k_strides=k_strides, v_strides=k_strides, o_strides=(DQ, HD),
-                          q_rows_total=T, kv_rows_total=kc.numel() // HD, status=st)
-            ops.gemm(attn, w["wo"][l], st, residual=h, out=h, stats_out=self.stats[:T] if fold else None)
-            if fold:
-                ops.gemm(h, self.wgu_f[l], st, epi=_C.EPI_SWIGLU, out=act, row_stats=self.stats[:T], col_sums=self.zeros_gu, stats_eps=EPS, stats_rms=True)
-            else:
-                ops.rmsnorm_rows(h, w["ln2"][l], EPS, out=xn)
-                ops.gemm(xn, w["wgu"][l], st, epi=_C.EPI_SWIGLU, out=act)
-            ops.gemm(act, w["wd"][l], st, residual=h, out=h, stats_out=self.stats[:T] if fold and l + 1 < self.L else None)
-        return h
+    def run(self, T, tokens, pos, seq, slot, seqs, max_q_len, rope, kcache, vcache, kv_layer, kv_cap, k_strides,
+            split_k=True):
+        """``tokens/pos/seq/slot``: int32 device ``[T]``; ``seqs``: int32 device ``[n, 4]``; ``kcache`` / ``vcache``: the store
+        of layer 0, laid out ``[B, 8, kv_cap, 128]``, each further layer ``kv_layer`` elements behind (0: one store for all);
+        ``k_strides`` = (row, head, seq) in elements.  ``split_k=False``: a token's values do not depend on what
+        else is packed into the forward.  Queues the whole stack on the current stream with one library call."""
+        p, w = _C.Qwen3Prefill(), self.w
+        p.n_layers, p.vocab, p.tokens, p.n_seqs, p.max_q_len, p.kv_cap = self.L, w["embed"].shape[0], T, seqs.shape[0], max_q_len, kv_cap
+        p.fused_rope, p.split_k, p.eps = int(self.fused_rope), int(split_k), EPS
+        for name in ("wqkv", "wo", "wgu", "wd", "ln1", "ln2", "qn", "kn", "embed"):
+            setattr(p, name, w[name].data_ptr())
+        if self.fold_norm:
+            p.wqkv_f, p.wgu_f, p.stats, p.zeros = self.wqkv_f.data_ptr(), self.wgu_f.data_ptr(), self.stats.data_ptr(), self.zeros.data_ptr()
+        p.rope, p.ids, p.pos, p.seq, p.slot, p.seqs = (t.data_ptr() for t in (rope, tokens, pos, seq, slot, seqs))
+        p.kcache, p.vcache, p.kv_layer = kcache.data_ptr(), vcache.data_ptr(), kv_layer
+        (p.k_row, p.k_head, p.k_seq), p.kv_rows_total = k_strides, (kv_layer or kcache.numel()) // HD
+        p.h, p.xn, p.qkv, p.attn, p.act, p.status = (t.data_ptr() for t in (self.h, self.xn, self.qkv, self.attn, self.act, self.status))
+        _C.check(_C.lib().ittai_qwen3_prefill_launch(C.byref(p), ops._stream(self.h)))
+        return self.h[:T]
 
 
 class Engine:
@@ -124,61 +117,60 @@ class Engine:
         z = lambda *s, dt: torch.zeros(*s, dtype=dt, device=self.dev)
         # one packed key/value store reused by every layer: the embedding pass keeps no cache
         self.kbuf, self.vbuf = z(1, NKV, self.M, HD, dt=torch.bfloat16), z(1, NKV, self.M, HD, dt=torch.bfloat16)
-        self.tokens, self.pos, self.seq, self.slot = (z(self.M, dt=torch.int32) for _ in range(4))
-        self.seqs, self.last = z(max_seqs, 4, dt=torch.int32), z(max_seqs, dt=torch.int32)
+        # the packing of a forward, written by one copy: seqs [B, 4], last [B], then tokens, pos, seq, slot [T] (see ``_views``)
+        self.meta = z(5 * max_seqs + 4 * self.M, dt=torch.int32)
         self.out = z(max_seqs, D, dt=torch.float32)
-        self.use_graph, self._graphs, self._meta = graph, {}, {}
+        self.use_graph, self._graphs, self._seen, self._checked = graph, {}, {}, False
 
-    def _tasks(self, seqlens):
-        """Packing metadata, cached per tuple of lengths like the reference's task lists (``engine.py:144-151``)."""
-        key = tuple(seqlens)
-        if key not in self._meta:
-            pos, seq, slot, seqs, T = packing(seqlens)
-            dev = lambda a: torch.from_numpy(np.ascontiguousarray(a, dtype=np.int32))
-            self._meta[key] = (dev(pos), dev(seq), dev(slot), dev(seqs), dev(seqs[:, 0] + seqs[:, 1] - 1), T)
-        return self._meta[key]
+    def _views(self, T, B):
+        """The parts of ``meta`` for a forward of ``T`` tokens in ``B`` sequences; ``seqs`` first: it is read 16 bytes at a time."""
+        m, o = self.meta, 5 * B
+        return m[:4 * B].view(B, 4), m[4 * B:o], *(m[o + i * T:o + (i + 1) * T] for i in range(4))
 
     def _body(self, T, B, max_len):
-        kv = lambda l: (self.kbuf, self.vbuf)
-        h = self.core.run(T, self.tokens, self.pos, self.seq, self.slot, self.seqs[:B], max_len, self.rope, kv, self.M,
-                          (HD, self.M * HD, 0))
-        _C.check(_C.lib().ittai_qwen3_final_pool(h.data_ptr(), self.last.data_ptr(), self.fin_w.data_ptr(), self.out.data_ptr(), B, EPS,
+        seqs, last, tokens, pos, seq, slot = self._views(T, B)
+        h = self.core.run(T, tokens, pos, seq, slot, seqs, max_len, self.rope, self.kbuf, self.vbuf, 0, self.M, (HD, self.M * HD, 0))
+        _C.check(_C.lib().ittai_qwen3_final_pool(h.data_ptr(), last.data_ptr(), self.fin_w.data_ptr(), self.out.data_ptr(), B, EPS,
                                                  ops._stream(h)))
+
+    # Up to this many tokens a repeated shape is replayed from a CUDA graph; above, the GPU is busy for longer than the host
+    # needs to queue the launches.
+    GRAPH_TOKENS, GRAPHS, SHAPES = 1024, 16, 256
 
     @torch.no_grad()
     def forward(self, input_ids):
         seqlens = [len(x) for x in input_ids]
         T, B = sum(seqlens), len(seqlens)
         assert T <= self.M and B <= self.Bmax and min(seqlens) > 0
-        pos, seq, slot, seqs, last, _ = self._tasks(seqlens)
-        flat = torch.tensor([t for s in input_ids for t in s], dtype=torch.int32)
+        pos, seq, slot, seqs, _ = packing(seqlens)
+        flat = np.fromiter(itertools.chain.from_iterable(input_ids), np.int32, T)
         if int(flat.min()) < 0 or int(flat.max()) >= self.embed.shape[0]:
             raise ValueError(f"token id outside [0, {self.embed.shape[0]})")      # the gather kernel would clamp it silently
-        self.tokens[:T].copy_(flat, non_blocking=True)
-        self.pos[:T].copy_(pos, non_blocking=True)
-        self.seq[:T].copy_(seq, non_blocking=True)
-        self.slot[:T].copy_(slot, non_blocking=True)
-        self.seqs[:B].copy_(seqs, non_blocking=True)
-        self.last[:B].copy_(last, non_blocking=True)
-        key = tuple(seqlens)
-        if not self.use_graph:
-            self._body(T, B, max(seqlens))
-        else:
-            if key not in self._graphs:
-                if len(self._graphs) >= 8:
-                    self._graphs.pop(next(iter(self._graphs)))
-                self.core.status.zero_()
-                s = torch.cuda.Stream()
-                s.wait_stream(torch.cuda.current_stream())
-                with torch.cuda.stream(s):
-                    self._body(T, B, max(seqlens))
-                torch.cuda.current_stream().wait_stream(s)
-                ops.check_status(self.core.status)
-                g = torch.cuda.CUDAGraph()
-                with torch.cuda.graph(g):
-                    self._body(T, B, max(seqlens))
-                self._graphs[key] = g
+        meta = upload((seqs, seqs[:, 0] + seqs[:, 1] - 1, flat, pos, seq, slot))
+        self.meta[:meta.numel()].copy_(meta, non_blocking=True)
+        # the launches depend on these three numbers alone, the packing itself is read on the device
+        key = (T, B, max(seqlens))
+        if key in self._graphs:
             self._graphs[key].replay()
+        elif not self.use_graph or T > self.GRAPH_TOKENS or key not in self._seen:
+            # a shape's first forward runs as plain launches: a capture costs more than it could give back
+            self._seen[key] = True
+            if len(self._seen) > self.SHAPES:
+                self._seen.pop(next(iter(self._seen)))
+            self._body(*key)
+            if not self._checked:
+                self.check()
+                self._checked = True
+        else:
+            if len(self._graphs) >= self.GRAPHS:
+                old = next(iter(self._graphs))
+                self._graphs.pop(old)
+                self._seen.pop(old, None)
+            g = torch.cuda.CUDAGraph()
+            with torch.cuda.graph(g):
+                self._body(*key)
+            self._graphs[key] = g
+            g.replay()
         return self.out[:B]
 
     def check(self) -> None:

@@ -167,7 +167,7 @@ class Engine:
         kv_max = S
         embed = dict(bias=self.bpe, residual=self.pos, out=self.x, stats_out=self.stats_m if fold else None)
         if not self.chain:
-            ops.gemm(self.patches, self.wpe, st, **embed)
+            ops.gemm(self.patches, self.wpe, st, static_w=True, **embed)
         def attention():
             ops.attention(self.qkv, self.qkv[:, D:], self.qkv[:, 2 * D:], self.attn, self.seqs, n_heads=H, group=1, head_dim=hd,
                           causal=False, max_q_len=S, q_strides=(3 * D, hd), k_strides=(3 * D, hd, 0), v_strides=(3 * D, hd, 0),
@@ -194,34 +194,34 @@ class Engine:
                 ops.gemm_chain(descs, self.chain_flags[i])
         for w in (() if self.chain else self.layers):
             if fold:
-                ops.gemm(self.x, w["qkv_f"][0], st, bias=w["qkv_f"][1], out=self.qkv, row_stats=self.stats_m, col_sums=w["qkv_f"][2], stats_eps=eps)
+                ops.gemm(self.x, w["qkv_f"][0], st, static_w=True, bias=w["qkv_f"][1], out=self.qkv, row_stats=self.stats_m, col_sums=w["qkv_f"][2], stats_eps=eps)
             else:
                 ops.layernorm_rows(self.x, *w["ln1"], eps, out=self.y)
-                ops.gemm(self.y, w["wqkv"], st, bias=w["bqkv"], out=self.qkv)
+                ops.gemm(self.y, w["wqkv"], st, static_w=True, bias=w["bqkv"], out=self.qkv)
             attention()
-            ops.gemm(self.attn, w["wo"], st, bias=w["bo"], residual=self.x, out=self.x, stats_out=self.stats_a if fold else None)
+            ops.gemm(self.attn, w["wo"], st, static_w=True, bias=w["bo"], residual=self.x, out=self.x, stats_out=self.stats_a if fold else None)
             if fold:
-                ops.gemm(self.x, w["fc1_f"][0], st, bias=w["fc1_f"][1], epi=_C.EPI_GELU, out=self.h, row_stats=self.stats_a, col_sums=w["fc1_f"][2],
+                ops.gemm(self.x, w["fc1_f"][0], st, static_w=True, bias=w["fc1_f"][1], epi=_C.EPI_GELU, out=self.h, row_stats=self.stats_a, col_sums=w["fc1_f"][2],
                          stats_eps=eps)
             else:
                 ops.layernorm_rows(self.x, *w["ln2"], eps, out=self.y)
-                ops.gemm(self.y, w["w1"], st, bias=w["b1"], epi=_C.EPI_GELU, out=self.h)
-            ops.gemm(self.h, w["w2"], st, bias=w["b2"], residual=self.x, out=self.x, stats_out=self.stats_m if fold else None)
+                ops.gemm(self.y, w["w1"], st, static_w=True, bias=w["b1"], epi=_C.EPI_GELU, out=self.h)
+            ops.gemm(self.h, w["w2"], st, static_w=True, bias=w["b2"], residual=self.x, out=self.x, stats_out=self.stats_m if fold else None)
         # post-LayerNorm + MAP head: probe attends over the tokens, then LayerNorm + MLP with a residual
         if self.chain:
             pass                                         # the last chain wrote self.kv
         elif fold:
-            ops.gemm(self.x, self.kv_f[0], st, bias=self.kv_f[1], out=self.kv, row_stats=self.stats_m, col_sums=self.kv_f[2], stats_eps=eps)
+            ops.gemm(self.x, self.kv_f[0], st, static_w=True, bias=self.kv_f[1], out=self.kv, row_stats=self.stats_m, col_sums=self.kv_f[2], stats_eps=eps)
         else:
             ops.layernorm_rows(self.x, *self.post, eps, out=self.y)
-            ops.gemm(self.y, self.wkv, st, bias=self.bkv, out=self.kv)
+            ops.gemm(self.y, self.wkv, st, static_w=True, bias=self.bkv, out=self.kv)
         ops.attention(self.probe_q, self.kv, self.kv[:, D:], self.pool_a, self.pool_seqs, n_heads=H, group=1, head_dim=hd,
                       causal=False, max_q_len=1, q_strides=(0, hd), k_strides=(2 * D, hd, 0), v_strides=(2 * D, hd, 0),
                       o_strides=(D, hd))
-        ops.gemm(self.pool_a, self.who, st, bias=self.bho, out=self.pool_r)
+        ops.gemm(self.pool_a, self.who, st, static_w=True, bias=self.bho, out=self.pool_r)
         ops.layernorm_rows(self.pool_r, *self.hln, eps, out=self.pool_y)
-        ops.gemm(self.pool_y, self.hw1, st, bias=self.hb1, epi=_C.EPI_GELU, out=self.pool_h)
-        ops.gemm(self.pool_h, self.hw2, st, bias=self.hb2, residual=self.pool_r, out=self.embeds)
+        ops.gemm(self.pool_y, self.hw1, st, static_w=True, bias=self.hb1, epi=_C.EPI_GELU, out=self.pool_h)
+        ops.gemm(self.pool_h, self.hw2, st, static_w=True, bias=self.hb2, residual=self.pool_r, out=self.embeds)
 
     @torch.no_grad()
     def forward(self, inp):

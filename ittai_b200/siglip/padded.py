@@ -143,8 +143,9 @@ class PaddedEngine:
                           q_rows_total=self.M, kv_rows_total=self.M, status=st, **att)
 
         if self.fold_ln:
-            ln = dict(stats_eps=eps, stats_k=D)
-            embed = ops.gemm_desc(self.patches, self.wpe, st, bias=self.bpe, residual=self.pos, out=self.x, stats_out=self.stats_m)[0]
+            sw = dict(static_w=not self.chain)                  # a chained GEMM takes no such flag
+            ln = dict(stats_eps=eps, stats_k=D, **sw)
+            embed = ops.gemm_desc(self.patches, self.wpe, st, **sw, bias=self.bpe, residual=self.pos, out=self.x, stats_out=self.stats_m)[0]
             qkv = lambda w: ops.gemm_desc(self.x, w["qkv_f"][0], st, bias=w["qkv_f"][1], out=self.qkv, row_stats=self.stats_m,
                                           col_sums=w["qkv_f"][2], **ln)[0]
             run = (lambda descs, flags: ops.gemm_chain(descs, flags)) if self.chain else \
@@ -154,32 +155,32 @@ class PaddedEngine:
             run([embed, qkv(self.layers[0])], self.chain_flags[len(self.layers)])
             for i, w in enumerate(self.layers):
                 attention()
-                descs = [ops.gemm_desc(self.attn, w["wo"], st, bias=w["bo"], residual=self.x, out=self.x, stats_out=self.stats_a)[0],
+                descs = [ops.gemm_desc(self.attn, w["wo"], st, **sw, bias=w["bo"], residual=self.x, out=self.x, stats_out=self.stats_a)[0],
                          ops.gemm_desc(self.x, w["fc1_f"][0], st, bias=w["fc1_f"][1], epi=_C.EPI_GELU, out=self.h, row_stats=self.stats_a,
                                        col_sums=w["fc1_f"][2], **ln)[0],
-                         ops.gemm_desc(self.h, w["w2"], st, bias=w["b2"], residual=self.x, out=self.x, stats_out=self.stats_m)[0]]
+                         ops.gemm_desc(self.h, w["w2"], st, **sw, bias=w["b2"], residual=self.x, out=self.x, stats_out=self.stats_m)[0]]
                 descs.append(qkv(self.layers[i + 1]) if i + 1 < len(self.layers) else
                              ops.gemm_desc(self.x, self.kv_f[0], st, bias=self.kv_f[1], out=self.kv, row_stats=self.stats_m, col_sums=self.kv_f[2], **ln)[0])
                 run(descs, self.chain_flags[i])
         else:
-            ops.gemm(self.patches, self.wpe, st, bias=self.bpe, residual=self.pos, out=self.x)
+            ops.gemm(self.patches, self.wpe, st, static_w=True, bias=self.bpe, residual=self.pos, out=self.x)
             for w in self.layers:
                 ops.layernorm_rows(self.x[:, :D], *w["ln1"], eps, out=self.y[:, :D])
-                ops.gemm(self.y, w["wqkv"], st, bias=w["bqkv"], out=self.qkv)
+                ops.gemm(self.y, w["wqkv"], st, static_w=True, bias=w["bqkv"], out=self.qkv)
                 attention()
-                ops.gemm(self.attn, w["wo"], st, bias=w["bo"], residual=self.x, out=self.x)
+                ops.gemm(self.attn, w["wo"], st, static_w=True, bias=w["bo"], residual=self.x, out=self.x)
                 ops.layernorm_rows(self.x[:, :D], *w["ln2"], eps, out=self.y[:, :D])
-                ops.gemm(self.y, w["w1"], st, bias=w["b1"], epi=_C.EPI_GELU, out=self.h)
-                ops.gemm(self.h, w["w2"], st, bias=w["b2"], residual=self.x, out=self.x)
+                ops.gemm(self.y, w["w1"], st, static_w=True, bias=w["b1"], epi=_C.EPI_GELU, out=self.h)
+                ops.gemm(self.h, w["w2"], st, static_w=True, bias=w["b2"], residual=self.x, out=self.x)
             # post-LayerNorm + MAP head: the probe attends over the image's tokens, then LayerNorm + MLP with a residual
             ops.layernorm_rows(self.x[:, :D], *self.post, eps, out=self.y[:, :D])
-            ops.gemm(self.y, self.wkv, st, bias=self.bkv, out=self.kv)
+            ops.gemm(self.y, self.wkv, st, static_w=True, bias=self.bkv, out=self.kv)
         ops.attention(self.probe_q, self.kv, self.kv[:, Hp:], self.pool_a, self.pool_seqs, max_q_len=1, q_strides=(0, hdp),
                       k_strides=(2 * Hp, hdp, 0), v_strides=(2 * Hp, hdp, 0), o_strides=(Hp, hdp), **att)
-        ops.gemm(self.pool_a, self.who, st, bias=self.bho, out=self.pool_r)
+        ops.gemm(self.pool_a, self.who, st, static_w=True, bias=self.bho, out=self.pool_r)
         ops.layernorm_rows(self.pool_r[:, :D], *self.hln, eps, out=self.pool_y[:, :D])
-        ops.gemm(self.pool_y, self.hw1, st, bias=self.hb1, epi=_C.EPI_GELU, out=self.pool_h)
-        ops.gemm(self.pool_h, self.hw2, st, bias=self.hb2, residual=self.pool_r, out=self.embeds_p)
+        ops.gemm(self.pool_y, self.hw1, st, static_w=True, bias=self.hb1, epi=_C.EPI_GELU, out=self.pool_h)
+        ops.gemm(self.pool_h, self.hw2, st, static_w=True, bias=self.hb2, residual=self.pool_r, out=self.embeds_p)
 
     @torch.no_grad()
     def forward(self, inp):
