@@ -347,6 +347,12 @@ int ittai_qwen3_qk_rope_scatter(void* qkv, const void* qn, const void* kn, const
  * leaves the columns beyond untouched (zero-padded K).  Even patch sizes and widths; H/p and W/p round down, the pixels
  * beyond the last whole patch are dropped (a stride-p convolution without padding). */
 int ittai_siglip_im2col(const float* pixels, void* patches, int batch, int height, int width, int patch, int ld_out, void* stream);
+/* Position rows of variable-resolution images, bf16 [n_images * rows][ld_out]: the learned fp32 grid [side, side, width] resized
+ * to shapes[i] = (height, width) in patches (bilinear, antialiased, fp32), row-major; rows past height * width get the image's
+ * first row.  Also stores height * width in the fourth word of seqs[i] and pool_seqs[i] (IttaiAttention records).  The caller
+ * has checked 1 <= height * width <= rows (reference: src/ittai/siglip/kernel.py:638-649). */
+int ittai_siglip_positions(const float* grid, int side, int width, const int32_t* shapes, int n_images, int rows, void* out, int ld_out,
+                           int32_t* seqs, int32_t* pool_seqs, void* stream);
 /* out[t, :] = table[ids[t], :], rows of 1024 bf16 (src/ittai/qwen3/base.py:147-162). */
 int ittai_embed_rows(const int32_t* ids, const void* table, void* out, int rows, int vocab, void* stream);
 /* Embedding head: out[s] = l2_normalise(rmsnorm(h[rows[s]]) * gain) in fp32 (src/ittai/qwen3/base.py:131-145). */

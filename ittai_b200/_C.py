@@ -23,7 +23,7 @@ EXPORTS = (
     "ittai_qwen3_decode_workspace_bytes", "ittai_qwen3_decode_launch", "ittai_qwen3_phase_launch",
     "ittai_qwen3_decode_launch_static", "ittai_qwen3_chain_create", "ittai_qwen3_chain_run", "ittai_qwen3_chain_destroy",
     "ittai_gemm_bf16_launch", "ittai_gemm_chain_launch", "ittai_attention_launch", "ittai_rmsnorm_rows", "ittai_layernorm_rows", "ittai_row_stats",
-    "ittai_qwen3_prefill_launch", "ittai_qwen3_qk_rope_scatter", "ittai_siglip_im2col", "ittai_embed_rows", "ittai_qwen3_final_pool",
+    "ittai_qwen3_prefill_launch", "ittai_qwen3_qk_rope_scatter", "ittai_siglip_im2col", "ittai_siglip_positions", "ittai_embed_rows", "ittai_qwen3_final_pool",
 )
 EPI_NONE, EPI_GELU, EPI_SWIGLU, EPI_QKROPE = range(4)
 GEMM_STATIC_W = 0x100
@@ -127,6 +127,7 @@ def lib() -> C.CDLL:
     L.ittai_row_stats.argtypes = [vp, i32, vp, i32, i32, f32, vp]
     L.ittai_qwen3_qk_rope_scatter.argtypes = [vp, vp, vp, vp, vp, vp, vp, vp, vp, i32, i32, f32, vp]
     L.ittai_siglip_im2col.argtypes = [vp, vp, i32, i32, i32, i32, i32, vp]
+    L.ittai_siglip_positions.argtypes = [vp, i32, i32, vp, i32, i32, vp, i32, vp, vp, vp]
     L.ittai_embed_rows.argtypes = [vp, vp, vp, i32, i32, vp]
     L.ittai_qwen3_final_pool.argtypes = [vp, vp, vp, vp, i32, f32, vp]
     if L.ittai_version() != ABI_VERSION:

@@ -235,6 +235,56 @@ __global__ void __launch_bounds__(256) im2col_kernel(const float* __restrict__ p
     }
 }
 
+// Position rows of variable-resolution images: the learned [side][side][width] grid resized to every image's patch grid
+// (bilinear with antialiasing: a triangle filter widened by the scale where the grid shrinks, weights normalised over the
+// taps inside the grid), row-major, rows past the image's last patch filled with its first row.  One warp per output row,
+// fp32 throughout, one rounding at the end.  A handful of library launches and host-to-device index copies per distinct patch
+// shape otherwise: 61 of them, about 1.2 ms, for 24 photos of mixed aspect ratio against 6 us here.
+struct ResizeTaps { int first, count; float scale, inv; float center; };
+__device__ __forceinline__ ResizeTaps resize_taps(int i, int in, int out) {
+    ResizeTaps t;
+    t.scale = (float)in / (float)out;
+    const float support = fmaxf(t.scale, 1.0f);
+    t.inv = 1.0f / support;
+    t.center = t.scale * ((float)i + 0.5f);
+    t.first = max((int)(t.center - support + 0.5f), 0);
+    t.count = min((int)(t.center + support + 0.5f), in) - t.first;
+    return t;
+}
+__device__ __forceinline__ float resize_weight(const ResizeTaps& t, int j) {
+    return fmaxf(1.0f - fabsf(((float)(t.first + j) - t.center + 0.5f) * t.inv), 0.0f);
+}
+__global__ void __launch_bounds__(kRowThreads) positions_kernel(const float* __restrict__ grid, int side, int width, const int2* __restrict__ shapes,
+                                                                  int n_images, int rows, bf16* __restrict__ out, int ld_out,
+                                                                  int4* __restrict__ seqs, int4* __restrict__ pool_seqs) {
+    pdl_trigger();
+    pdl_wait();
+    const int r = blockIdx.x * (kRowThreads / 32) + (threadIdx.x >> 5), lane = threadIdx.x & 31;
+    if (r >= n_images * rows) return;
+    const int img = r / rows, p = r - img * rows;
+    const int2 hw = shapes[img];
+    const int n = hw.x * hw.y, q = p < n ? p : 0;
+    if (p == 0 && lane == 0) { seqs[img].w = n; pool_seqs[img].w = n; }       // the attention kernels see the image's own keys only
+    const ResizeTaps ty = resize_taps(q / hw.y, side, hw.x), tx = resize_taps(q % hw.y, side, hw.y);
+    float sy = 0.f, sx = 0.f;
+    for (int j = 0; j < ty.count; ++j) sy += resize_weight(ty, j);
+    for (int j = 0; j < tx.count; ++j) sx += resize_weight(tx, j);
+    for (int c = lane * 4; c < width; c += 128) {
+        float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
+        for (int jy = 0; jy < ty.count; ++jy) {
+            const float wy = resize_weight(ty, jy) / sy;
+            float4 line = make_float4(0.f, 0.f, 0.f, 0.f);
+            for (int jx = 0; jx < tx.count; ++jx) {
+                const float wx = resize_weight(tx, jx) / sx;
+                const float4 v = __ldg(reinterpret_cast<const float4*>(grid + ((size_t)(ty.first + jy) * side + tx.first + jx) * width + c));
+                line.x = fmaf(wx, v.x, line.x); line.y = fmaf(wx, v.y, line.y); line.z = fmaf(wx, v.z, line.z); line.w = fmaf(wx, v.w, line.w);
+            }
+            acc.x = fmaf(wy, line.x, acc.x); acc.y = fmaf(wy, line.y, acc.y); acc.z = fmaf(wy, line.z, acc.z); acc.w = fmaf(wy, line.w, acc.w);
+        }
+        *reinterpret_cast<uint2*>(out + (size_t)r * ld_out + c) = make_uint2(pack_bf16x2(acc.x, acc.y), pack_bf16x2(acc.z, acc.w));
+    }
+}
+
 // Embedding rows: out[t] = table[ids[t]], width 1024 (reference src/ittai/qwen3/base.py:147-162).
 __global__ void __launch_bounds__(kRowThreads) embed_rows_kernel(const int* __restrict__ ids, const bf16* __restrict__ table,
                                                                    bf16* __restrict__ out, int rows, int vocab) {
@@ -337,6 +387,19 @@ extern "C" int ittai_siglip_im2col(const float* pixels, void* patches, int batch
     if (v == 4) launch_pdl(im2col_kernel<4>, dim3(grid), dim3(256), 0, (cudaStream_t)stream, 1, pixels, (bf16*)patches, batch, height, width, patch, ld_out);
     else launch_pdl(im2col_kernel<2>, dim3(grid), dim3(256), 0, (cudaStream_t)stream, 1, pixels, (bf16*)patches, batch, height, width, patch, ld_out);
     return launched("im2col_kernel");
+}
+
+extern "C" int ittai_siglip_positions(const float* grid, int side, int width, const int32_t* shapes, int n_images, int rows, void* out, int ld_out,
+                                      int32_t* seqs, int32_t* pool_seqs, void* stream) {
+    if (!grid || !shapes || !out || !seqs || !pool_seqs || side < 1 || width < 4 || width % 4 || n_images < 1 || rows < 1 || ld_out < width || ld_out % 4 ||
+        ((uintptr_t)grid & 15) || ((uintptr_t)out & 7) || ((uintptr_t)shapes & 7) || ((uintptr_t)seqs & 15) || ((uintptr_t)pool_seqs & 15) ||
+        (long long)n_images * rows > 0x7fffffffll) {
+        set_error("positions: bad argument (width and ld_out multiples of 4)");
+        return ITTAI_E_ARG;
+    }
+    const cudaError_t e = launch_pdl(positions_kernel, dim3(row_grid((long long)n_images * rows)), dim3(kRowThreads), 0, (cudaStream_t)stream, 1,
+                                     grid, side, width, (const int2*)shapes, n_images, rows, (bf16*)out, ld_out, (int4*)seqs, (int4*)pool_seqs);
+    return e == cudaSuccess ? ITTAI_OK : cuda_fail(e, "launch positions_kernel");
 }
 
 extern "C" int ittai_embed_rows(const int32_t* ids, const void* table, void* out, int rows, int vocab, void* stream) {

@@ -52,6 +52,24 @@ def resize_positions(grid: torch.Tensor, shapes, max_len: int) -> torch.Tensor:
     return out
 
 
+def checked_shapes(inp, n: int, S: int) -> torch.Tensor:
+    """The ``(height, width)`` patch grids of ``n`` variable-resolution images as int32 ``[n, 2]`` on the host, checked against
+    the mask and the ``S`` position rows an image has."""
+    shapes = torch.as_tensor(inp["spatial_shapes"]).to(torch.int64).cpu()
+    key_len = inp["pixel_attention_mask"].to(torch.int64).sum(1).cpu()
+    if not torch.equal(key_len, shapes.prod(1)) or int(key_len.min()) < 1:
+        raise ValueError("pixel_attention_mask must mark exactly height * width leading rows of every image")
+    if len(shapes) != n or int(shapes.min()) < 1 or int(key_len.max()) > S:
+        raise ValueError(f"patch grids {shapes.tolist()} do not fit {S} positions")
+    return shapes.to(torch.int32).contiguous()
+
+
+def part_size(n: int, B: int, S: int, chain: bool) -> int:
+    """Images to run for a short batch of ``n``: at least the 1024 rows from which on the chained GEMMs are used where the full
+    batch of ``B`` uses them, so that an image's result does not depend on the batch it came in."""
+    return max(n, min(B, -(-1024 // S))) if chain else n
+
+
 def _vision_model(m):
     return m.vision_model if hasattr(m, "vision_model") else m
 
@@ -67,6 +85,8 @@ class Engine:
     """``Engine(vm, B)``: fixed batch ``B``; ``forward({"pixel_values": fp32 [B,3,H,W]})`` returns bf16 ``[B, D]`` pooled
     embeddings (a persistent buffer, like the reference's ``self.embeds``).  The reference's tuning arguments
     (``tile_n, stages, warps, fold_k, group_m, kv_block``) are accepted and ignored: there is one sm_100a kernel."""
+
+    PARTS = 8                # graphs of short batches kept beside the full batch's
 
     def __new__(cls, vm, B, *args, **kw):
         """ViT-B-like geometries (head_dim 64, widths in multiples of 128) get this class; anything else (so400m: width
@@ -153,11 +173,16 @@ class Engine:
         self.chain = bool(chain) and self.fold_ln and M >= 1024      # a few row blocks only: nothing to overlap, one launch per GEMM is faster
         self.chain_flags = torch.zeros(len(self.layers) + 1, 4 * 2 * ((M + 255) // 256), dtype=torch.int32, device=dev)
         self.status = ops.new_status(dev)
-        self.graph = None if graph else False
+        self.use_graph, self._graphs, self._seen, self._checked = graph, {}, set(), False      # per number of images
 
-    def _body(self):
-        D, S, B, H, hd, eps = self.D, self.S0, self.B, self.H, self.hd, self.eps
+    def _body(self, B):
+        """Queue the forward of the first ``B`` images of the buffers."""
+        D, S, H, hd, eps = self.D, self.S0, self.H, self.hd, self.eps
+        M = B * S
         L, st = _C.lib(), self.status
+        patches, pos, x, y, h, qkv_b, attn, kv = (t[:M] for t in (self.patches, self.pos, self.x, self.y, self.h, self.qkv, self.attn, self.kv))
+        stats_a, stats_m, seqs, pool_seqs = self.stats_a[:M], self.stats_m[:M], self.seqs[:B], self.pool_seqs[:B]
+        pool_a, pool_r, pool_y, pool_h, embeds = (t[:B] for t in (self.pool_a, self.pool_r, self.pool_y, self.pool_h, self.embeds))
         if self.conv:
             _C.check(L.ittai_siglip_im2col(self.pixels.data_ptr(), self.patches.data_ptr(), B, self.img, self.img, self.p, 0,
                                            ops._stream(self.pixels)))
@@ -165,104 +190,127 @@ class Engine:
         # with variable-resolution inputs an image's keys are its first key_len rows (the records in `seqs` say how many);
         # the tensor-memory kernel takes up to 256 keys and queries per image, longer sequences fall to the register tiles
         kv_max = S
-        embed = dict(bias=self.bpe, residual=self.pos, out=self.x, stats_out=self.stats_m if fold else None)
+        embed = dict(bias=self.bpe, residual=pos, out=x, stats_out=stats_m if fold else None)
         if not self.chain:
-            ops.gemm(self.patches, self.wpe, st, static_w=True, **embed)
+            ops.gemm(patches, self.wpe, st, static_w=True, **embed)
         def attention():
-            ops.attention(self.qkv, self.qkv[:, D:], self.qkv[:, 2 * D:], self.attn, self.seqs, n_heads=H, group=1, head_dim=hd,
+            ops.attention(qkv_b, qkv_b[:, D:], qkv_b[:, 2 * D:], attn, seqs, n_heads=H, group=1, head_dim=hd,
                           causal=False, max_q_len=S, q_strides=(3 * D, hd), k_strides=(3 * D, hd, 0), v_strides=(3 * D, hd, 0),
                           o_strides=(D, hd), max_kv_len=kv_max, q_rows_total=self.M, kv_rows_total=self.M, status=st)
 
         if self.chain:
             self.chain_flags.zero_()
-            qkv = lambda w: ops.gemm_desc(self.x, w["qkv_f"][0], st, bias=w["qkv_f"][1], out=self.qkv, row_stats=self.stats_m,
+            qkv = lambda w: ops.gemm_desc(x, w["qkv_f"][0], st, bias=w["qkv_f"][1], out=qkv_b, row_stats=stats_m,
                                           col_sums=w["qkv_f"][2], stats_eps=eps)[0]
             # patch embedding + the first QKV projection; then per layer out-proj, fc1, fc2 and the next layer's QKV (after
             # the last layer: the K/V projection of the pooling head)
-            ops.gemm_chain([ops.gemm_desc(self.patches, self.wpe, st, **embed)[0], qkv(self.layers[0])], self.chain_flags[len(self.layers)])
+            ops.gemm_chain([ops.gemm_desc(patches, self.wpe, st, **embed)[0], qkv(self.layers[0])], self.chain_flags[len(self.layers)])
             for i, w in enumerate(self.layers):
                 attention()
-                descs = [ops.gemm_desc(self.attn, w["wo"], st, bias=w["bo"], residual=self.x, out=self.x, stats_out=self.stats_a)[0],
-                         ops.gemm_desc(self.x, w["fc1_f"][0], st, bias=w["fc1_f"][1], epi=_C.EPI_GELU, out=self.h, row_stats=self.stats_a,
+                descs = [ops.gemm_desc(attn, w["wo"], st, bias=w["bo"], residual=x, out=x, stats_out=stats_a)[0],
+                         ops.gemm_desc(x, w["fc1_f"][0], st, bias=w["fc1_f"][1], epi=_C.EPI_GELU, out=h, row_stats=stats_a,
                                        col_sums=w["fc1_f"][2], stats_eps=eps)[0],
-                         ops.gemm_desc(self.h, w["w2"], st, bias=w["b2"], residual=self.x, out=self.x, stats_out=self.stats_m)[0]]
+                         ops.gemm_desc(h, w["w2"], st, bias=w["b2"], residual=x, out=x, stats_out=stats_m)[0]]
                 if i + 1 < len(self.layers):
                     descs.append(qkv(self.layers[i + 1]))
                 else:
-                    descs.append(ops.gemm_desc(self.x, self.kv_f[0], st, bias=self.kv_f[1], out=self.kv, row_stats=self.stats_m,
+                    descs.append(ops.gemm_desc(x, self.kv_f[0], st, bias=self.kv_f[1], out=kv, row_stats=stats_m,
                                                col_sums=self.kv_f[2], stats_eps=eps)[0])
                 ops.gemm_chain(descs, self.chain_flags[i])
         for w in (() if self.chain else self.layers):
             if fold:
-                ops.gemm(self.x, w["qkv_f"][0], st, static_w=True, bias=w["qkv_f"][1], out=self.qkv, row_stats=self.stats_m, col_sums=w["qkv_f"][2], stats_eps=eps)
+                ops.gemm(x, w["qkv_f"][0], st, static_w=True, bias=w["qkv_f"][1], out=qkv_b, row_stats=stats_m, col_sums=w["qkv_f"][2], stats_eps=eps)
             else:
-                ops.layernorm_rows(self.x, *w["ln1"], eps, out=self.y)
-                ops.gemm(self.y, w["wqkv"], st, static_w=True, bias=w["bqkv"], out=self.qkv)
+                ops.layernorm_rows(x, *w["ln1"], eps, out=y)
+                ops.gemm(y, w["wqkv"], st, static_w=True, bias=w["bqkv"], out=qkv_b)
             attention()
-            ops.gemm(self.attn, w["wo"], st, static_w=True, bias=w["bo"], residual=self.x, out=self.x, stats_out=self.stats_a if fold else None)
+            ops.gemm(attn, w["wo"], st, static_w=True, bias=w["bo"], residual=x, out=x, stats_out=stats_a if fold else None)
             if fold:
-                ops.gemm(self.x, w["fc1_f"][0], st, static_w=True, bias=w["fc1_f"][1], epi=_C.EPI_GELU, out=self.h, row_stats=self.stats_a, col_sums=w["fc1_f"][2],
+                ops.gemm(x, w["fc1_f"][0], st, static_w=True, bias=w["fc1_f"][1], epi=_C.EPI_GELU, out=h, row_stats=stats_a, col_sums=w["fc1_f"][2],
                          stats_eps=eps)
             else:
-                ops.layernorm_rows(self.x, *w["ln2"], eps, out=self.y)
-                ops.gemm(self.y, w["w1"], st, static_w=True, bias=w["b1"], epi=_C.EPI_GELU, out=self.h)
-            ops.gemm(self.h, w["w2"], st, static_w=True, bias=w["b2"], residual=self.x, out=self.x, stats_out=self.stats_m if fold else None)
+                ops.layernorm_rows(x, *w["ln2"], eps, out=y)
+                ops.gemm(y, w["w1"], st, static_w=True, bias=w["b1"], epi=_C.EPI_GELU, out=h)
+            ops.gemm(h, w["w2"], st, static_w=True, bias=w["b2"], residual=x, out=x, stats_out=stats_m if fold else None)
         # post-LayerNorm + MAP head: probe attends over the tokens, then LayerNorm + MLP with a residual
         if self.chain:
             pass                                         # the last chain wrote self.kv
         elif fold:
-            ops.gemm(self.x, self.kv_f[0], st, static_w=True, bias=self.kv_f[1], out=self.kv, row_stats=self.stats_m, col_sums=self.kv_f[2], stats_eps=eps)
+            ops.gemm(x, self.kv_f[0], st, static_w=True, bias=self.kv_f[1], out=kv, row_stats=stats_m, col_sums=self.kv_f[2], stats_eps=eps)
         else:
-            ops.layernorm_rows(self.x, *self.post, eps, out=self.y)
-            ops.gemm(self.y, self.wkv, st, static_w=True, bias=self.bkv, out=self.kv)
-        ops.attention(self.probe_q, self.kv, self.kv[:, D:], self.pool_a, self.pool_seqs, n_heads=H, group=1, head_dim=hd,
+            ops.layernorm_rows(x, *self.post, eps, out=y)
+            ops.gemm(y, self.wkv, st, static_w=True, bias=self.bkv, out=kv)
+        ops.attention(self.probe_q, kv, kv[:, D:], pool_a, pool_seqs, n_heads=H, group=1, head_dim=hd,
                       causal=False, max_q_len=1, q_strides=(0, hd), k_strides=(2 * D, hd, 0), v_strides=(2 * D, hd, 0),
                       o_strides=(D, hd))
-        ops.gemm(self.pool_a, self.who, st, static_w=True, bias=self.bho, out=self.pool_r)
-        ops.layernorm_rows(self.pool_r, *self.hln, eps, out=self.pool_y)
-        ops.gemm(self.pool_y, self.hw1, st, static_w=True, bias=self.hb1, epi=_C.EPI_GELU, out=self.pool_h)
-        ops.gemm(self.pool_h, self.hw2, st, static_w=True, bias=self.hb2, residual=self.pool_r, out=self.embeds)
+        ops.gemm(pool_a, self.who, st, static_w=True, bias=self.bho, out=pool_r)
+        ops.layernorm_rows(pool_r, *self.hln, eps, out=pool_y)
+        ops.gemm(pool_y, self.hw1, st, static_w=True, bias=self.hb1, epi=_C.EPI_GELU, out=pool_h)
+        ops.gemm(pool_h, self.hw2, st, static_w=True, bias=self.hb2, residual=pool_r, out=embeds)
 
     @torch.no_grad()
     def forward(self, inp):
         """``inp["pixel_values"]``: ``[B, 3, H, W]`` on any device; copied into the engine's buffer, then one graph replay.
         A NaFlex tower takes ``pixel_values`` ``[B, S, 3 p p]`` (patch rows), ``pixel_attention_mask`` ``[B, S]`` (valid rows
         first) and ``spatial_shapes`` ``[B, 2]``, like the reference's engine (``:638-649``)."""
-        px = inp["pixel_values"]
+        self._load(inp, self.B)
+        self._run(self.B)
+        return self.embeds
+
+    @torch.no_grad()
+    def forward_part(self, inp):
+        """``forward`` of a short batch: 1 to ``B`` images; returns bf16 ``[n, D]``, a view of the same buffer."""
+        n = len(inp["pixel_values"])
+        assert 1 <= n <= self.B, f"1 to {self.B} images, got {n}"
+        self._load(inp, n)
+        self._run(part_size(n, self.B, self.S0, self.chain))
+        return self.embeds[:n]
+
+    def _load(self, inp, n):
+        """Copy ``n`` images and what goes with them into the buffers."""
+        px, S = inp["pixel_values"], self.S0
         if self.conv:
             if "spatial_shapes" in inp:
                 raise ValueError("this tower has a fixed-resolution patch embedding; it takes [B, 3, H, W] pixels only")
-            assert tuple(px.shape) == tuple(self.pixels.shape), f"expected {tuple(self.pixels.shape)}, got {tuple(px.shape)}"
-            self.pixels.copy_(px, non_blocking=True)
-        else:
-            S = self.S0
-            assert tuple(px.shape) == (self.B, S, self.patches.shape[1]), f"expected {(self.B, S, self.patches.shape[1])}, got {tuple(px.shape)}"
-            mask, shapes = inp["pixel_attention_mask"], inp["spatial_shapes"]
-            key_len = mask.to(torch.int64).sum(1).cpu()
-            area = torch.as_tensor(shapes).to(torch.int64).cpu().prod(1)
-            if not torch.equal(key_len, area) or int(key_len.min()) < 1:
-                raise ValueError("pixel_attention_mask must mark exactly height * width leading rows of every image")
-            self.patches.copy_(px.reshape(self.M, -1), non_blocking=True)
-            self.pos.copy_(resize_positions(self.pos_grid, torch.as_tensor(shapes).tolist(), S).reshape(self.M, -1))
-            kl = key_len.to(torch.int32).to(self.dev, non_blocking=True)
-            self.seqs[:, 3].copy_(kl)
-            self.pool_seqs[:, 3].copy_(kl)
-        if self.graph is None:
+            assert px.shape[0] == n and px.shape[1:] == self.pixels.shape[1:], f"expected {(n, *self.pixels.shape[1:])}, got {tuple(px.shape)}"
+            self.pixels[:n].copy_(px, non_blocking=True)
+            return
+        K = 3 * self.p * self.p
+        assert tuple(px.shape) == (n, S, K), f"expected {(n, S, K)}, got {tuple(px.shape)}"
+        shapes = checked_shapes(inp, n, S)
+        self.patches[:n * S, :K].copy_(px.reshape(n * S, K), non_blocking=True)
+        shapes_d = shapes.to(self.dev, non_blocking=True)
+        _C.check(_C.lib().ittai_siglip_positions(self.pos_grid.data_ptr(), self.pos_grid.shape[0], self.D, shapes_d.data_ptr(), n, S, self.pos.data_ptr(),
+                                                 self.pos.stride(0), self.seqs.data_ptr(), self.pool_seqs.data_ptr(), ops._stream(self.pos)))
+
+    def _run(self, n):
+        """The forward over the first ``n`` images of the buffers.  The full batch is captured at its first use; a part runs as
+        plain launches the first time its size is seen and is captured the second time."""
+        graph = self._graphs.get(n)
+        if graph is None and not self._checked:
             self.status.zero_()
             s = torch.cuda.Stream()
             s.wait_stream(torch.cuda.current_stream())
             with torch.cuda.stream(s):
-                self._body()
+                self._body(n)
             torch.cuda.current_stream().wait_stream(s)
             ops.check_status(self.status)
-            self.graph = torch.cuda.CUDAGraph()
-            with torch.cuda.graph(self.graph):
-                self._body()
-        if self.graph:
-            self.graph.replay()
+            self._checked = True
+            if n != self.B:
+                self._seen.add(n)
+                return
+        if graph is None and self.use_graph and (n == self.B or n in self._seen):
+            if len(self._graphs) > self.PARTS:
+                self._graphs.pop(next(k for k in self._graphs if k != self.B))
+            graph = torch.cuda.CUDAGraph()
+            with torch.cuda.graph(graph):
+                self._body(n)
+            self._graphs[n] = graph
+        self._seen.add(n)
+        if graph is not None:
+            graph.replay()
         else:
-            self._body()
-        return self.embeds
+            self._body(n)
 
     def launches_per_forward(self) -> int:
         """Kernels in one forward (all inside one CUDA graph)."""
@@ -349,6 +397,9 @@ class Siglip2Embedder:
         stream of their own: batch k + 1 crosses PCIe while batch k is in the encoder (pinned host tensors make the copy
         asynchronous for the host as well).  Inputs already on the device go straight to the engine.  ``to_host=True``
         returns pinned host tensors instead, each copied back right behind its batch (synchronise before reading them)."""
+        return self._stream_batches(batches, to_host, self.engine.forward)
+
+    def _stream_batches(self, batches, to_host, forward):
         dev = torch.device(self.device)
         main = torch.cuda.current_stream(dev)
         if getattr(self, "_copy_stream", None) is None:
@@ -364,8 +415,9 @@ class Siglip2Embedder:
             if px.device.type == "cuda":
                 return inp, None
             buf = self._staged[slot]
-            if buf is None or buf.shape != px.shape or buf.dtype != px.dtype:
+            if buf is None or buf.shape[1:] != px.shape[1:] or len(buf) < len(px) or buf.dtype != px.dtype:
                 buf = self._staged[slot] = torch.empty(px.shape, dtype=px.dtype, device=dev)
+            buf = buf[:len(px)]
             ready = torch.cuda.Event()
             with torch.cuda.stream(self._copy_stream):
                 self._copy_stream.wait_event(self._free[slot])
@@ -383,7 +435,7 @@ class Siglip2Embedder:
             staged = stage(nxt, (k + 1) & 1) if nxt is not None else None      # issued before this batch's forward
             if ready is not None:
                 main.wait_event(ready)
-            emb = self.engine.forward(cur)
+            emb = forward(cur)
             if to_host:
                 host = torch.empty(emb.shape, dtype=emb.dtype).pin_memory()
                 host.copy_(emb, non_blocking=True)
@@ -407,12 +459,7 @@ class Siglip2Embedder:
         else:
             inp = dict(self.processor(images=images, return_tensors="pt"))
         total = len(inp["pixel_values"])
-        counts = [min(self.B, total - k) for k in range(0, total, self.B)]
-
-        def batches():
-            for k, n in zip(range(0, total, self.B), counts):
-                # a short last batch is filled up with copies of its final image (reference ``:720-723``)
-                fill = lambda t: t[k:k + n] if n == self.B else torch.cat([t[k:k + n], t[k + n - 1:k + n].expand(self.B - n, *t.shape[1:])])
-                yield {name: fill(t) for name, t in inp.items()}
-
-        return torch.cat([e[:n] for e, n in zip(self.embed_batches(batches()), counts)])
+        # slices of the caller's tensors, so that pinned ones stay pinned; a short last batch runs as what it is (the reference
+        # fills it up with copies of its final image, ``:720-723``)
+        parts = ({name: t[k:k + self.B] for name, t in inp.items()} for k in range(0, total, self.B))
+        return torch.cat(self._stream_batches(parts, False, self.engine.forward_part))

@@ -28,6 +28,8 @@ def _up(n: int, m: int) -> int:
 class PaddedEngine:
     """Same surface as ``Engine``: ``forward(inputs) -> bf16 [B, D]`` view of a persistent buffer, ``check()``, ``flops()``."""
 
+    PARTS = 8                # as in ``Engine``
+
     @torch.no_grad()
     def __init__(self, vm, B, graph=True, fold_ln=True, chain=True, **ignored):
         from .kernel import _vision_model
@@ -126,11 +128,17 @@ class PaddedEngine:
         self.seqs = torch.tensor([[b * S, S, b * S, S] for b in range(B)], dtype=torch.int32, device=dev)
         self.pool_seqs = torch.tensor([[b, 1, b * S, S] for b in range(B)], dtype=torch.int32, device=dev)
         self.status = ops.new_status(dev)
-        self.graph = None if graph else False
+        self.use_graph, self._graphs, self._seen, self._checked = graph, {}, set(), False      # per number of images
 
-    def _body(self):
-        D, S, B, H, hdp, eps, st = self.D, self.S0, self.B, self.H, self.hdp, self.eps, self.status
-        Hp = H * hdp
+    def _body(self, B):
+        """Queue the forward of the first ``B`` images of the buffers."""
+        D, S, H, hdp, eps, st = self.D, self.S0, self.H, self.hdp, self.eps, self.status
+        Hp, M = H * hdp, B * S
+        patches, pos, x, y, h, qkv_b, attn, kv = (t[:M] for t in (self.patches, self.pos, self.x, self.y, self.h, self.qkv, self.attn, self.kv))
+        if self.fold_ln:
+            stats_a, stats_m = self.stats_a[:M], self.stats_m[:M]
+        seqs, pool_seqs = self.seqs[:B], self.pool_seqs[:B]
+        pool_a, pool_r, pool_y, pool_h, embeds = (t[:B] for t in (self.pool_a, self.pool_r, self.pool_y, self.pool_h, self.embeds_p))
         if self.conv:       # patch rows in (channel, row, column) order: what a Conv2d weight flattens to; the padding columns stay zero
             _C.check(_C.lib().ittai_siglip_im2col(self.pixels.data_ptr(), self.patches.data_ptr(), B, self.img, self.img, self.p, self.Kp,
                                                   ops._stream(self.pixels)))
@@ -138,85 +146,82 @@ class PaddedEngine:
 
         def attention():
             # row totals + status words: the tcgen05 key-loop kernel (head_dim 128, keys and values packed like the queries)
-            ops.attention(self.qkv, self.qkv[:, Hp:], self.qkv[:, 2 * Hp:], self.attn, self.seqs, max_q_len=S, q_strides=(3 * Hp, hdp),
+            ops.attention(qkv_b, qkv_b[:, Hp:], qkv_b[:, 2 * Hp:], attn, seqs, max_q_len=S, q_strides=(3 * Hp, hdp),
                           k_strides=(3 * Hp, hdp, 0), v_strides=(3 * Hp, hdp, 0), o_strides=(Hp, hdp), max_kv_len=S,
                           q_rows_total=self.M, kv_rows_total=self.M, status=st, **att)
 
         if self.fold_ln:
             sw = dict(static_w=not self.chain)                  # a chained GEMM takes no such flag
             ln = dict(stats_eps=eps, stats_k=D, **sw)
-            embed = ops.gemm_desc(self.patches, self.wpe, st, **sw, bias=self.bpe, residual=self.pos, out=self.x, stats_out=self.stats_m)[0]
-            qkv = lambda w: ops.gemm_desc(self.x, w["qkv_f"][0], st, bias=w["qkv_f"][1], out=self.qkv, row_stats=self.stats_m,
+            embed = ops.gemm_desc(patches, self.wpe, st, **sw, bias=self.bpe, residual=pos, out=x, stats_out=stats_m)[0]
+            qkv = lambda w: ops.gemm_desc(x, w["qkv_f"][0], st, bias=w["qkv_f"][1], out=qkv_b, row_stats=stats_m,
                                           col_sums=w["qkv_f"][2], **ln)[0]
             run = (lambda descs, flags: ops.gemm_chain(descs, flags)) if self.chain else \
-                  (lambda descs, flags: [_C.check(_C.lib().ittai_gemm_bf16_launch(C.byref(d), ops._stream(self.x))) for d in descs])
+                  (lambda descs, flags: [_C.check(_C.lib().ittai_gemm_bf16_launch(C.byref(d), ops._stream(x))) for d in descs])
             if self.chain:
                 self.chain_flags.zero_()
             run([embed, qkv(self.layers[0])], self.chain_flags[len(self.layers)])
             for i, w in enumerate(self.layers):
                 attention()
-                descs = [ops.gemm_desc(self.attn, w["wo"], st, **sw, bias=w["bo"], residual=self.x, out=self.x, stats_out=self.stats_a)[0],
-                         ops.gemm_desc(self.x, w["fc1_f"][0], st, bias=w["fc1_f"][1], epi=_C.EPI_GELU, out=self.h, row_stats=self.stats_a,
+                descs = [ops.gemm_desc(attn, w["wo"], st, **sw, bias=w["bo"], residual=x, out=x, stats_out=stats_a)[0],
+                         ops.gemm_desc(x, w["fc1_f"][0], st, bias=w["fc1_f"][1], epi=_C.EPI_GELU, out=h, row_stats=stats_a,
                                        col_sums=w["fc1_f"][2], **ln)[0],
-                         ops.gemm_desc(self.h, w["w2"], st, **sw, bias=w["b2"], residual=self.x, out=self.x, stats_out=self.stats_m)[0]]
+                         ops.gemm_desc(h, w["w2"], st, **sw, bias=w["b2"], residual=x, out=x, stats_out=stats_m)[0]]
                 descs.append(qkv(self.layers[i + 1]) if i + 1 < len(self.layers) else
-                             ops.gemm_desc(self.x, self.kv_f[0], st, bias=self.kv_f[1], out=self.kv, row_stats=self.stats_m, col_sums=self.kv_f[2], **ln)[0])
+                             ops.gemm_desc(x, self.kv_f[0], st, bias=self.kv_f[1], out=kv, row_stats=stats_m, col_sums=self.kv_f[2], **ln)[0])
                 run(descs, self.chain_flags[i])
         else:
-            ops.gemm(self.patches, self.wpe, st, static_w=True, bias=self.bpe, residual=self.pos, out=self.x)
+            ops.gemm(patches, self.wpe, st, static_w=True, bias=self.bpe, residual=pos, out=x)
             for w in self.layers:
-                ops.layernorm_rows(self.x[:, :D], *w["ln1"], eps, out=self.y[:, :D])
-                ops.gemm(self.y, w["wqkv"], st, static_w=True, bias=w["bqkv"], out=self.qkv)
+                ops.layernorm_rows(x[:, :D], *w["ln1"], eps, out=y[:, :D])
+                ops.gemm(y, w["wqkv"], st, static_w=True, bias=w["bqkv"], out=qkv_b)
                 attention()
-                ops.gemm(self.attn, w["wo"], st, static_w=True, bias=w["bo"], residual=self.x, out=self.x)
-                ops.layernorm_rows(self.x[:, :D], *w["ln2"], eps, out=self.y[:, :D])
-                ops.gemm(self.y, w["w1"], st, static_w=True, bias=w["b1"], epi=_C.EPI_GELU, out=self.h)
-                ops.gemm(self.h, w["w2"], st, static_w=True, bias=w["b2"], residual=self.x, out=self.x)
+                ops.gemm(attn, w["wo"], st, static_w=True, bias=w["bo"], residual=x, out=x)
+                ops.layernorm_rows(x[:, :D], *w["ln2"], eps, out=y[:, :D])
+                ops.gemm(y, w["w1"], st, static_w=True, bias=w["b1"], epi=_C.EPI_GELU, out=h)
+                ops.gemm(h, w["w2"], st, static_w=True, bias=w["b2"], residual=x, out=x)
             # post-LayerNorm + MAP head: the probe attends over the image's tokens, then LayerNorm + MLP with a residual
-            ops.layernorm_rows(self.x[:, :D], *self.post, eps, out=self.y[:, :D])
-            ops.gemm(self.y, self.wkv, st, static_w=True, bias=self.bkv, out=self.kv)
-        ops.attention(self.probe_q, self.kv, self.kv[:, Hp:], self.pool_a, self.pool_seqs, max_q_len=1, q_strides=(0, hdp),
+            ops.layernorm_rows(x[:, :D], *self.post, eps, out=y[:, :D])
+            ops.gemm(y, self.wkv, st, static_w=True, bias=self.bkv, out=kv)
+        ops.attention(self.probe_q, kv, kv[:, Hp:], pool_a, pool_seqs, max_q_len=1, q_strides=(0, hdp),
                       k_strides=(2 * Hp, hdp, 0), v_strides=(2 * Hp, hdp, 0), o_strides=(Hp, hdp), **att)
-        ops.gemm(self.pool_a, self.who, st, static_w=True, bias=self.bho, out=self.pool_r)
-        ops.layernorm_rows(self.pool_r[:, :D], *self.hln, eps, out=self.pool_y[:, :D])
-        ops.gemm(self.pool_y, self.hw1, st, static_w=True, bias=self.hb1, epi=_C.EPI_GELU, out=self.pool_h)
-        ops.gemm(self.pool_h, self.hw2, st, static_w=True, bias=self.hb2, residual=self.pool_r, out=self.embeds_p)
+        ops.gemm(pool_a, self.who, st, static_w=True, bias=self.bho, out=pool_r)
+        ops.layernorm_rows(pool_r[:, :D], *self.hln, eps, out=pool_y[:, :D])
+        ops.gemm(pool_y, self.hw1, st, static_w=True, bias=self.hb1, epi=_C.EPI_GELU, out=pool_h)
+        ops.gemm(pool_h, self.hw2, st, static_w=True, bias=self.hb2, residual=pool_r, out=embeds)
 
     @torch.no_grad()
     def forward(self, inp):
-        from .kernel import resize_positions
-        px = inp["pixel_values"]
-        if self.conv:
-            assert tuple(px.shape) == tuple(self.pixels.shape), f"expected {tuple(self.pixels.shape)}, got {tuple(px.shape)}"
-            self.pixels.copy_(px, non_blocking=True)
-        else:
-            S = self.S0
-            assert tuple(px.shape) == (self.B, S, self.Kp0), f"expected {(self.B, S, self.Kp0)}, got {tuple(px.shape)}"
-            mask, shapes = inp["pixel_attention_mask"], torch.as_tensor(inp["spatial_shapes"])
-            key_len = mask.to(torch.int64).sum(1).cpu()
-            if not torch.equal(key_len, shapes.to(torch.int64).cpu().prod(1)) or int(key_len.min()) < 1:
-                raise ValueError("pixel_attention_mask must mark exactly height * width leading rows of every image")
-            self.patches[:, :self.Kp0].copy_(px.reshape(self.M, -1), non_blocking=True)
-            self.pos[:, :self.D].copy_(resize_positions(self.pos_grid, shapes.tolist(), S).reshape(self.M, -1))
-            kl = key_len.to(torch.int32).to(self.dev, non_blocking=True)
-            self.seqs[:, 3].copy_(kl)
-            self.pool_seqs[:, 3].copy_(kl)
-        if self.graph is None:
-            self.status.zero_()
-            s = torch.cuda.Stream()
-            s.wait_stream(torch.cuda.current_stream())
-            with torch.cuda.stream(s):
-                self._body()
-            torch.cuda.current_stream().wait_stream(s)
-            ops.check_status(self.status)
-            self.graph = torch.cuda.CUDAGraph()
-            with torch.cuda.graph(self.graph):
-                self._body()
-        if self.graph:
-            self.graph.replay()
-        else:
-            self._body()
+        self._load(inp, self.B)
+        self._run(self.B)
         return self.embeds_p[:, :self.D]
+
+    @torch.no_grad()
+    def forward_part(self, inp):
+        from .kernel import part_size
+        n = len(inp["pixel_values"])
+        assert 1 <= n <= self.B, f"1 to {self.B} images, got {n}"
+        self._load(inp, n)
+        self._run(part_size(n, self.B, self.S0, self.chain))
+        return self.embeds_p[:n, :self.D]
+
+    def _load(self, inp, n):
+        from .kernel import checked_shapes
+        px, S, K = inp["pixel_values"], self.S0, self.Kp0
+        if self.conv:
+            assert px.shape[0] == n and px.shape[1:] == self.pixels.shape[1:], f"expected {(n, *self.pixels.shape[1:])}, got {tuple(px.shape)}"
+            self.pixels[:n].copy_(px, non_blocking=True)
+            return
+        assert tuple(px.shape) == (n, S, K), f"expected {(n, S, K)}, got {tuple(px.shape)}"
+        shapes = checked_shapes(inp, n, S)
+        self.patches[:n * S, :K].copy_(px.reshape(n * S, K), non_blocking=True)
+        shapes_d = shapes.to(self.dev, non_blocking=True)
+        _C.check(_C.lib().ittai_siglip_positions(self.pos_grid.data_ptr(), self.pos_grid.shape[0], self.D, shapes_d.data_ptr(), n, S, self.pos.data_ptr(),
+                                                 self.pos.stride(0), self.seqs.data_ptr(), self.pool_seqs.data_ptr(), ops._stream(self.pos)))
+
+    def _run(self, n):
+        from .kernel import Engine
+        Engine._run(self, n)
 
     def check(self) -> None:
         ops.check_status(self.status)

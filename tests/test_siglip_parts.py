@@ -1,0 +1,66 @@
+"""Short batches and the position-row kernel of the vision engines (GPU)."""
+import pytest
+import torch
+
+from oracle import siglip_hf as hf
+
+gpu = pytest.mark.gpu
+SHAPES = [(16, 16), (12, 20), (1, 1), (10, 25), (1, 256), (200, 1), (3, 5), (27, 9)]
+
+
+@gpu
+@pytest.mark.parametrize("side,width,ld", [(16, 768, 768), (27, 1152, 1280)])
+def test_position_rows_match_the_torch_resize(side, width, ld):
+    """Grids smaller and larger than the learned one, one row, one column, one patch.  Both sides sum at most some 60 products
+    of a weight and an fp32 value: one bf16 rounding (2^-8 relative) and 1e-5 of the largest value for the sums."""
+    from ittai_b200 import _C, ops
+    from ittai_b200.siglip.kernel import resize_positions
+    g = torch.Generator(device="cuda").manual_seed(side)
+    grid = torch.randn(side, side, width, generator=g, device="cuda")
+    n, rows = len(SHAPES), 256
+    out = torch.full((n * rows + 1, ld), 9.0, dtype=torch.bfloat16, device="cuda")
+    seqs, pool = (torch.full((n, 4), -1, dtype=torch.int32, device="cuda") for _ in range(2))
+    shapes = torch.tensor(SHAPES, dtype=torch.int32, device="cuda")
+    _C.check(_C.lib().ittai_siglip_positions(grid.data_ptr(), side, width, shapes.data_ptr(), n, rows, out.data_ptr(), ld, seqs.data_ptr(), pool.data_ptr(),
+                                             ops._stream(out)))
+    want = resize_positions(grid, SHAPES, rows).reshape(n * rows, width)
+    got = out[:-1, :width].float()
+    assert ((got - want).abs() <= 2.0 ** -8 * want.abs() + 1e-5 * want.abs().max()).all(), (got - want).abs().max()
+    assert (out[-1] == 9.0).all() and (ld == width or (out[:, width:] == 9.0).all())
+    area = torch.tensor([h * w for h, w in SHAPES], dtype=torch.int32, device="cuda")
+    for t in (seqs, pool):
+        assert torch.equal(t[:, 3], area) and (t[:, :3] == -1).all()
+
+
+@gpu
+@pytest.mark.parametrize("batch,images", [(8, 11), (8, 7), (2, 3), (16, 16)])
+def test_a_short_batch_gives_what_the_full_batch_gives(batch, images):
+    """The images behind the last whole batch run as a smaller forward: the same rows, bit for bit, as in a full batch, on the
+    first pass (plain launches) and on repeated ones (a graph)."""
+    from ittai_b200.siglip.kernel import Siglip2Embedder
+    emb = Siglip2Embedder(hf.build_hf(seed=0, device="cuda"), batch_size=batch)
+    g = torch.Generator().manual_seed(5)
+    px = torch.randn(images, 3, 224, 224, generator=g)
+    padded = torch.cat([px, px[-1:].expand(-images % batch, -1, -1, -1)])
+    want = torch.cat(emb.embed_batches([padded[k:k + batch] for k in range(0, len(padded), batch)]))[:images]
+    for _ in range(3):
+        got = emb.embed(px)
+        assert got.shape == want.shape
+        cos = torch.nn.functional.cosine_similarity(got.float(), want.float(), dim=-1).min()
+        assert torch.equal(got, want) if batch >= 6 else cos >= 0.9999, cos
+    emb.engine.check()
+
+
+@gpu
+def test_a_short_naflex_batch():
+    from ittai_b200.siglip.kernel import Siglip2Embedder
+    shapes = [(16, 16), (9, 21), (3, 5), (12, 20), (1, 1), (10, 25), (16, 15)]
+    emb = Siglip2Embedder(hf.build_hf_naflex(seed=2, device="cuda"), batch_size=5)
+    inp = hf.naflex_inputs(shapes, seed=8)
+    full = {k: torch.cat([v, v[:3]]) for k, v in inp.items()}
+    want = emb.embed(full)[:7]
+    for _ in range(2):
+        assert torch.equal(emb.embed(inp), want)
+    bad = dict(inp, spatial_shapes=torch.tensor([(17, 16)] + shapes[1:]))
+    with pytest.raises(ValueError):
+        emb.embed(bad)
