@@ -284,7 +284,8 @@ typedef struct IttaiAttention {
      * (q_head = k_head = v_head = 64, k_seq = v_seq = 0); and head_dim 128 with a key loop, causal or dense, q_head = 128,
      * more than 64 queries in some sequence, keys and values either as dense rows (k_row = v_row = 128, head and sequence
      * strides multiples of 128, equal for k and v: the cache layout) or packed like the queries (k_head = v_head = 128,
-     * k_seq = v_seq = 0, k_row = v_row > 128: the heads of a token side by side in one row). */
+     * k_seq = v_seq = 0, k_row = v_row > 128: the heads of a token side by side in one row).  head_dim 80 is taken in that packed
+     * form only (q_head = k_head = v_head = 80). */
     int32_t q_rows_total;  /* rows of the matrix behind q (every sequence's q_row0 + q rows lies inside) */
     int32_t kv_rows_total; /* rows of the matrices behind k and v */
     int32_t reserved0;

@@ -406,7 +406,10 @@ using namespace ittai;
 
 extern "C" int ittai_attention_launch(const IttaiAttention* p, void* stream) {
     if (!p || !p->q || !p->k || !p->v || !p->o || !p->seqs) { set_error("attention: null pointer"); return ITTAI_E_ARG; }
-    if (p->head_dim != 64 && p->head_dim != 128) { set_error("attention: head_dim %d (64 or 128)", p->head_dim); return ITTAI_E_ARG; }
+    if (p->head_dim != 64 && p->head_dim != 128 && !(p->head_dim == 80 && attn_fa_supported(p))) {
+        set_error("attention: head_dim %d (64, 128, or 80 in the packed layout of the key-loop kernel)", p->head_dim);
+        return ITTAI_E_ARG;
+    }
     if (p->n_seqs < 1 || p->n_heads < 1 || p->group < 1 || p->max_q_len < 1) { set_error("attention: bad sizes"); return ITTAI_E_ARG; }
     const long long strides[] = {p->q_row, p->q_head, p->k_row, p->k_head, p->k_seq, p->v_row, p->v_head, p->v_seq, p->o_row};
     for (long long s : strides) if (s % 8) { set_error("attention: strides must be multiples of 8 elements"); return ITTAI_E_ARG; }

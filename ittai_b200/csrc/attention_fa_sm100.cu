@@ -36,7 +36,7 @@ struct AttnFaArgs {
     long long o_row, o_head;
     int group, causal;
     int k_seq_rows, k_head_rows;             // cache layout: strides in rows of 128 elements
-    int k_head_cols;                         // packed layout (heads side by side in a row, sequences by their row offsets): 128, else 0
+    int k_head_cols;                         // packed layout (heads side by side in a row, sequences by their row offsets): HDIM, else 0
     float scale_log2;
     uint32_t* status;
 };
@@ -57,6 +57,11 @@ __device__ __forceinline__ float fa_ex2(float x) {
     return y;
 }
 
+// HDIM: 128, or 80 for heads packed 80 columns apart (a head_dim of 72, zero-padded to whole k-steps of 16): S then takes five
+// k-steps instead of eight and the projections around the kernel are 80/128 as wide.  The loads still fetch 128 columns (the
+// next head's, or zeros past the last one) and P V still computes 128: an MN-major operand comes in whole 64-column atoms.
+// The surplus columns of O are never read.
+template <int HDIM>
 __global__ void __launch_bounds__(kFaThreads, 2)
 attn_fa_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUtensorMap tm_k,
                const __grid_constant__ CUtensorMap tm_v, const AttnFaArgs a) {
@@ -75,7 +80,7 @@ attn_fa_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
         pdl_wait();
         for (int i = threadIdx.x; i < kFaBlk * 16; i += kFaThreads) {
             const int row = r0 + (i >> 4);
-            if (row < q_len) *reinterpret_cast<uint4*>(a.o + (long long)(sinfo.x + row) * a.o_row + (long long)head * a.o_head + (i & 15) * 8) = make_uint4(0, 0, 0, 0);
+            if (row < q_len && (i & 15) < HDIM / 8) *reinterpret_cast<uint4*>(a.o + (long long)(sinfo.x + row) * a.o_row + (long long)head * a.o_head + (i & 15) * 8) = make_uint4(0, 0, 0, 0);
         }
         return;
     }
@@ -100,8 +105,8 @@ attn_fa_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
         fence_mbar_init();
         pdl_wait();                                        // q, k, v come from the kernels before this one
         mbar_expect_tx(bar_q, 32768);
-        tma_load_2d(sm + kFaQ, &tm_q, head * 128, sinfo.x + r0, bar_q);
-        tma_load_2d(sm + kFaQ + 16384, &tm_q, head * 128 + 64, sinfo.x + r0, bar_q);
+        tma_load_2d(sm + kFaQ, &tm_q, head * HDIM, sinfo.x + r0, bar_q);
+        tma_load_2d(sm + kFaQ + 16384, &tm_q, head * HDIM + 64, sinfo.x + r0, bar_q);
         mbar_expect_tx(bar_k, 32768);
         tma_load_2d(sm + kFaK, &tm_k, kc, kv_row, bar_k);
         tma_load_2d(sm + kFaK + 16384, &tm_k, kc + 64, kv_row, bar_k);
@@ -127,7 +132,7 @@ attn_fa_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
                 tc_fence_after();
                 // ---- S = Q K^T over the 128 dims: atoms of 64 dims, 4 k-steps each
 #pragma unroll
-                for (int k = 0; k < 8; ++k)
+                for (int k = 0; k < HDIM / 16; ++k)
                     umma_bf16(tmem_base, umma_desc_sw128(sm + kFaQ + (k >> 2) * 16384) + 2 * (k & 3),
                               umma_desc_sw128(sm + kFaK + (k >> 2) * 16384) + 2 * (k & 3), idesc_s, k > 0 ? 1u : 0u);
                 umma_commit(bar_s);
@@ -217,7 +222,7 @@ attn_fa_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
                     if (need) m_used = bm;
                     l0 *= alpha; l1 *= alpha;
 #pragma unroll 1
-                    for (int c0 = 0; c0 < 128; c0 += 32) {
+                    for (int c0 = 0; c0 < HDIM; c0 += 32) {
                         uint32_t v[32];
                         tmem_ld_32x32(t_row + kFaOCol + c0, v);
                         tmem_ld_wait();
@@ -290,7 +295,7 @@ attn_fa_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
         const float inv = l > 0.f ? 1.0f / l : 0.f;
         unsigned char* stage = sm + kFaQ;
 #pragma unroll 1
-        for (int c0 = 0; c0 < 128; c0 += 32) {
+        for (int c0 = 0; c0 < HDIM; c0 += 32) {
             uint32_t v[32];
             tmem_ld_32x32(t_row + kFaOCol + c0, v);
             tmem_ld_wait();
@@ -308,7 +313,7 @@ attn_fa_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
         for (int it = 0; it < 16; ++it) {
             const int rr = q4 * 32 + it * 2 + (lane >> 4), row = r0 + rr;
             const uint4 val = *reinterpret_cast<const uint4*>(stage + rr * 256 + ((sub ^ (rr & 15)) << 4));
-            if (row < q_len) *reinterpret_cast<uint4*>(a.o + (long long)(sinfo.x + row) * a.o_row + (long long)head * a.o_head + 8 * sub) = val;
+            if (row < q_len && sub < HDIM / 8) *reinterpret_cast<uint4*>(a.o + (long long)(sinfo.x + row) * a.o_row + (long long)head * a.o_head + 8 * sub) = val;
         }
     } while (false);
     tc_fence_before();
@@ -330,20 +335,21 @@ int cuda_fail(cudaError_t e, const char* what);
 // of 128 elements (the cache layout), identical strides for k and v, more than 64 query rows in some sequence.
 // Keys and values either in the cache layout (rows of 128 elements; heads and sequences whole numbers of rows apart) or
 // packed like the queries (the heads of a token side by side in one row, sequences told apart by their row offsets).
-static bool fa_packed_kv(const IttaiAttention* p) { return p->k_seq == 0 && p->v_seq == 0 && p->k_head == 128 && p->v_head == 128 && p->k_row == p->v_row && p->k_row > 128; }
+static bool fa_packed_kv(const IttaiAttention* p) { return p->k_seq == 0 && p->v_seq == 0 && p->k_head == p->head_dim && p->v_head == p->head_dim && p->k_row == p->v_row && p->k_row > 128; }
 bool attn_fa_supported(const IttaiAttention* p) {
-    const bool cache = p->k_row == 128 && p->v_row == 128 && p->k_head % 128 == 0 && p->k_seq % 128 == 0;
-    return p->head_dim == 128 && p->status != nullptr && p->max_q_len > 64 && p->q_head == 128 && (cache || fa_packed_kv(p)) &&
+    const bool cache = p->head_dim == 128 && p->k_row == 128 && p->v_row == 128 && p->k_head % 128 == 0 && p->k_seq % 128 == 0;
+    return (p->head_dim == 128 || p->head_dim == 80) && p->status != nullptr && p->max_q_len > 64 && p->q_head == p->head_dim && (cache || fa_packed_kv(p)) &&
            p->v_head == p->k_head && p->v_seq == p->k_seq && p->q_rows_total > 0 &&
            p->kv_rows_total > 0 && ((uintptr_t)p->q & 15) == 0 && ((uintptr_t)p->k & 15) == 0 && ((uintptr_t)p->v & 15) == 0 &&
            ((uintptr_t)p->o & 15) == 0 && p->o_row % 8 == 0 && p->o_head % 8 == 0;
 }
 
-int attn_fa_launch(const IttaiAttention* p, cudaStream_t st) {
+template <int HDIM>
+static int attn_fa_launch_t(const IttaiAttention* p, cudaStream_t st) {
     CUtensorMap tq, tk, tv;
-    int rc = make_tmap_bf16(&tq, p->q, p->q_rows_total, (long long)p->n_heads * 128, p->q_row, 128);
+    int rc = make_tmap_bf16(&tq, p->q, p->q_rows_total, (long long)p->n_heads * HDIM, p->q_row, 128);
     const bool packed = fa_packed_kv(p);
-    const long long kv_cols = packed ? (long long)(p->n_heads / p->group) * 128 : 128, kv_ld = packed ? p->k_row : 128;
+    const long long kv_cols = packed ? (long long)(p->n_heads / p->group) * HDIM : 128, kv_ld = packed ? p->k_row : 128;
     if (rc == ITTAI_OK) rc = make_tmap_bf16(&tk, p->k, p->kv_rows_total, kv_cols, kv_ld, 128);
     if (rc == ITTAI_OK) rc = make_tmap_bf16(&tv, p->v, p->kv_rows_total, kv_cols, kv_ld, 128);
     if (rc != ITTAI_OK) return rc;
@@ -351,7 +357,7 @@ int attn_fa_launch(const IttaiAttention* p, cudaStream_t st) {
     int dev = 0;
     cudaGetDevice(&dev);
     if (attr_dev != dev) {
-        const cudaError_t e = cudaFuncSetAttribute(attn_fa_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kFaSmem);
+        const cudaError_t e = cudaFuncSetAttribute(attn_fa_kernel<HDIM>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kFaSmem);
         if (e != cudaSuccess) return cuda_fail(e, "cudaFuncSetAttribute(attn_fa_kernel)");
         attr_dev = dev;
     }
@@ -361,11 +367,13 @@ int attn_fa_launch(const IttaiAttention* p, cudaStream_t st) {
     a.o_row = p->o_row; a.o_head = p->o_head;
     a.group = p->group; a.causal = p->causal;
     a.k_seq_rows = packed ? 0 : (int)(p->k_seq / 128); a.k_head_rows = packed ? 0 : (int)(p->k_head / 128);
-    a.k_head_cols = packed ? 128 : 0;
-    a.scale_log2 = 1.4426950408889634f * 0.08838834764831845f;
+    a.k_head_cols = packed ? HDIM : 0;
+    a.scale_log2 = 1.4426950408889634f / sqrtf((float)HDIM);
     a.status = p->status;
-    const cudaError_t e = launch_pdl(attn_fa_kernel, dim3(p->n_heads, p->n_seqs, (p->max_q_len + 127) / 128), dim3(kFaThreads), kFaSmem, st, 1, tq, tk, tv, a);
+    const cudaError_t e = launch_pdl(attn_fa_kernel<HDIM>, dim3(p->n_heads, p->n_seqs, (p->max_q_len + 127) / 128), dim3(kFaThreads), kFaSmem, st, 1, tq, tk, tv, a);
     return e == cudaSuccess ? ITTAI_OK : cuda_fail(e, "launch attn_fa_kernel");
 }
+
+int attn_fa_launch(const IttaiAttention* p, cudaStream_t st) { return p->head_dim == 80 ? attn_fa_launch_t<80>(p, st) : attn_fa_launch_t<128>(p, st); }
 
 }  // namespace ittai

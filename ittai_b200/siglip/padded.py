@@ -3,8 +3,8 @@ patch 14): the same kernels on zero-padded weights.
 
 The reference pads too (head_dim to a multiple of 16, the MLP width to a multiple of 128, the patch row to a multiple of
 32, tokens per image to a multiple of 128: ``src/ittai/siglip/kernel.py:537-539,551-563``).  Here the widths go up to what
-the kernels of this build take: model width and MLP width to multiples of 256 (the two-SM GEMM's tile), head_dim to 128
-(the attention kernels know 64 and 128), the patch row to a multiple of 64.  Everything that is padding is zero and stays
+the kernels of this build take: model width and MLP width to multiples of 256 (the two-SM GEMM's tile), head_dim to 80
+in the encoder and 128 in the pooling head (the attention kernels know 64, 80 and 128), the patch row to a multiple of 64.  Everything that is padding is zero and stays
 zero: padded weight rows and bias entries are zero, so the padded columns of every activation are zero, so the padded
 weight columns never contribute.  The softmax scale of the attention kernels is ``padded head_dim ** -0.5``; the q
 projection is pre-scaled by ``sqrt(padded / true)`` so that the scores carry the true ``head_dim ** -0.5``.  LayerNorm runs
@@ -57,26 +57,30 @@ class PaddedEngine:
         def pad2(w, rows, cols):                     # fp32 [r, c] -> fp32 [rows, cols], zero-filled
             return F.pad(f(w), (0, cols - w.shape[1], 0, rows - w.shape[0]))
 
-        def heads_out(w, b, scale=1.0):              # a projection INTO head space: [H*hd, D], [H*hd] -> [H*hdp, Dp], [H*hdp]
-            w = F.pad(f(w).view(H, hd, D) * scale, (0, Dp - D, 0, hdp - hd)).reshape(Hp, Dp)
-            b = F.pad(f(b).view(H, hd) * scale, (0, hdp - hd)).reshape(Hp)
+        def heads_out(w, b, to, scale=1.0):          # a projection INTO head space: [H*hd, D], [H*hd] -> [H*to, Dp], [H*to]
+            w = F.pad(f(w).view(H, hd, D) * scale, (0, Dp - D, 0, to - hd)).reshape(H * to, Dp)
+            b = F.pad(f(b).view(H, hd) * scale, (0, to - hd)).reshape(H * to)
             return w, b
 
-        def heads_in(w):                             # a projection OUT OF head space: [D, H*hd] -> [Dp, H*hdp]
-            return F.pad(f(w).view(D, H, hd), (0, hdp - hd, 0, 0, 0, Dp - D)).reshape(Dp, Hp)
+        def heads_in(w, to):                         # a projection OUT OF head space: [D, H*hd] -> [Dp, H*to]
+            return F.pad(f(w).view(D, H, hd), (0, to - hd, 0, 0, 0, Dp - D)).reshape(Dp, H * to)
 
-        qs = math.sqrt(hdp / hd)
+        # the encoder's heads go to 80 columns where the key-loop kernel's packed form covers them (so400m: 72), the one-query
+        # pooling head keeps ``hdp``
+        self.hde = 80 if 64 < hd <= 80 and self.S0 > 64 and 3 * H * 80 % 256 == 0 and H * 80 % 64 == 0 else hdp
+        hde, He = self.hde, H * self.hde
+        qs = math.sqrt(hde / hd)
         pe = emb.patch_embedding
         self.wpe, self.bpe = bf(pad2(pe.weight.reshape(D, -1), Dp, self.Kp)), F.pad(f(pe.bias), (0, Dp - D)).contiguous()
         self.layers = []
         for lyr in vm.encoder.layers:
             a, m = lyr.self_attn, lyr.mlp
-            parts = [heads_out(a.q_proj.weight, a.q_proj.bias, qs), heads_out(a.k_proj.weight, a.k_proj.bias), heads_out(a.v_proj.weight, a.v_proj.bias)]
+            parts = [heads_out(a.q_proj.weight, a.q_proj.bias, hde, qs), heads_out(a.k_proj.weight, a.k_proj.bias, hde), heads_out(a.v_proj.weight, a.v_proj.bias, hde)]
             self.layers.append(dict(
                 ln1=(f(lyr.layer_norm1.weight).contiguous(), f(lyr.layer_norm1.bias).contiguous()),
                 ln2=(f(lyr.layer_norm2.weight).contiguous(), f(lyr.layer_norm2.bias).contiguous()),
                 wqkv=bf(torch.cat([w for w, _ in parts])), bqkv=torch.cat([b for _, b in parts]).contiguous(),
-                wo=bf(heads_in(a.out_proj.weight)), bo=F.pad(f(a.out_proj.bias), (0, Dp - D)).contiguous(),
+                wo=bf(heads_in(a.out_proj.weight, hde)), bo=F.pad(f(a.out_proj.bias), (0, Dp - D)).contiguous(),
                 w1=bf(pad2(m.fc1.weight, Fp, Dp)), b1=F.pad(f(m.fc1.bias), (0, Fp - Fm)).contiguous(),
                 w2=bf(pad2(m.fc2.weight, Dp, Fp)), b2=F.pad(f(m.fc2.bias), (0, Dp - D)).contiguous()))
         self.post = (f(vm.post_layernorm.weight).contiguous(), f(vm.post_layernorm.bias).contiguous())
@@ -85,10 +89,10 @@ class PaddedEngine:
         # the probe's query does not depend on the image: projected once, as the eager module would (bf16 Linear), then laid
         # out in padded head space with the score scale folded in
         q = F.linear(h.probe[0].to(dev, torch.bfloat16), inw[:D].to(dev, torch.bfloat16), inb[:D].to(dev, torch.bfloat16)).float()
-        self.probe_q = bf(F.pad(q.view(H, hd) * qs, (0, hdp - hd)).reshape(1, Hp))
-        kv = [heads_out(inw[D:2 * D], inb[D:2 * D]), heads_out(inw[2 * D:], inb[2 * D:])]
+        self.probe_q = bf(F.pad(q.view(H, hd) * math.sqrt(hdp / hd), (0, hdp - hd)).reshape(1, Hp))
+        kv = [heads_out(inw[D:2 * D], inb[D:2 * D], hdp), heads_out(inw[2 * D:], inb[2 * D:], hdp)]
         self.wkv, self.bkv = bf(torch.cat([w for w, _ in kv])), torch.cat([b for _, b in kv]).contiguous()
-        self.who, self.bho = bf(heads_in(h.attention.out_proj.weight)), F.pad(f(h.attention.out_proj.bias), (0, Dp - D)).contiguous()
+        self.who, self.bho = bf(heads_in(h.attention.out_proj.weight, hdp)), F.pad(f(h.attention.out_proj.bias), (0, Dp - D)).contiguous()
         self.hln = (f(h.layernorm.weight).contiguous(), f(h.layernorm.bias).contiguous())
         self.hw1, self.hb1 = bf(pad2(h.mlp.fc1.weight, Fp, Dp)), F.pad(f(h.mlp.fc1.bias), (0, Fp - Fm)).contiguous()
         self.hw2, self.hb2 = bf(pad2(h.mlp.fc2.weight, Dp, Fp)), F.pad(f(h.mlp.fc2.bias), (0, Dp - D)).contiguous()
@@ -121,7 +125,7 @@ class PaddedEngine:
             side = int(round(self.S0 ** 0.5))
             self.pos_grid = f(emb.position_embedding.weight).reshape(side, side, D)
         self.patches, self.x, self.y = z(M, self.Kp), z(M, Dp), z(M, Dp)
-        self.qkv, self.attn, self.h = z(M, 3 * Hp), z(M, Hp), z(M, Fp)
+        self.qkv, self.attn, self.h = z(M, 3 * He), z(M, He), z(M, Fp)
         self.kv, self.pool_a, self.pool_r, self.pool_y, self.pool_h = z(M, 2 * Hp), z(B, Hp), z(B, Dp), z(B, Dp), z(B, Fp)
         self.embeds_p = z(B, Dp)
         S = self.S0
@@ -142,13 +146,12 @@ class PaddedEngine:
         if self.conv:       # patch rows in (channel, row, column) order: what a Conv2d weight flattens to; the padding columns stay zero
             _C.check(_C.lib().ittai_siglip_im2col(self.pixels.data_ptr(), self.patches.data_ptr(), B, self.img, self.img, self.p, self.Kp,
                                                   ops._stream(self.pixels)))
-        att = dict(n_heads=H, group=1, head_dim=hdp, causal=False)
-
         def attention():
-            # row totals + status words: the tcgen05 key-loop kernel (head_dim 128, keys and values packed like the queries)
-            ops.attention(qkv_b, qkv_b[:, Hp:], qkv_b[:, 2 * Hp:], attn, seqs, max_q_len=S, q_strides=(3 * Hp, hdp),
-                          k_strides=(3 * Hp, hdp, 0), v_strides=(3 * Hp, hdp, 0), o_strides=(Hp, hdp), max_kv_len=S,
-                          q_rows_total=self.M, kv_rows_total=self.M, status=st, **att)
+            # row totals + status words: the tcgen05 key-loop kernel (keys and values packed like the queries)
+            he, He = self.hde, H * self.hde
+            ops.attention(qkv_b, qkv_b[:, He:], qkv_b[:, 2 * He:], attn, seqs, n_heads=H, group=1, head_dim=he, causal=False, max_q_len=S,
+                          q_strides=(3 * He, he), k_strides=(3 * He, he, 0), v_strides=(3 * He, he, 0), o_strides=(He, he), max_kv_len=S,
+                          q_rows_total=self.M, kv_rows_total=self.M, status=st)
 
         if self.fold_ln:
             sw = dict(static_w=not self.chain)                  # a chained GEMM takes no such flag
@@ -183,8 +186,8 @@ class PaddedEngine:
             # post-LayerNorm + MAP head: the probe attends over the image's tokens, then LayerNorm + MLP with a residual
             ops.layernorm_rows(x[:, :D], *self.post, eps, out=y[:, :D])
             ops.gemm(y, self.wkv, st, static_w=True, bias=self.bkv, out=kv)
-        ops.attention(self.probe_q, kv, kv[:, Hp:], pool_a, pool_seqs, max_q_len=1, q_strides=(0, hdp),
-                      k_strides=(2 * Hp, hdp, 0), v_strides=(2 * Hp, hdp, 0), o_strides=(Hp, hdp), **att)
+        ops.attention(self.probe_q, kv, kv[:, Hp:], pool_a, pool_seqs, n_heads=H, group=1, head_dim=hdp, causal=False, max_q_len=1, q_strides=(0, hdp),
+                      k_strides=(2 * Hp, hdp, 0), v_strides=(2 * Hp, hdp, 0), o_strides=(Hp, hdp))
         ops.gemm(pool_a, self.who, st, static_w=True, bias=self.bho, out=pool_r)
         ops.layernorm_rows(pool_r[:, :D], *self.hln, eps, out=pool_y[:, :D])
         ops.gemm(pool_y, self.hw1, st, static_w=True, bias=self.hb1, epi=_C.EPI_GELU, out=pool_h)

@@ -64,3 +64,32 @@ def test_a_short_naflex_batch():
     bad = dict(inp, spatial_shapes=torch.tensor([(17, 16)] + shapes[1:]))
     with pytest.raises(ValueError):
         emb.embed(bad)
+
+
+@gpu
+@pytest.mark.parametrize("lens", [[729, 729], [128, 65, 1, 200], [257]])
+def test_packed_attention_with_80_columns_per_head(lens):
+    """The key-loop kernel on heads 80 columns apart against fp32 softmax attention: P and the output are rounded to bf16 once
+    each (2^-8 relative on P's unit row sums, 2^-9 on the result), with the scores exact to fp32: 2^-7 of the largest value."""
+    from ittai_b200 import ops
+    H, hd = 5, 80
+    total = sum(lens)
+    g = torch.Generator(device="cuda").manual_seed(total)
+    qkv = torch.randn(total, 3 * H * hd, generator=g, device="cuda").to(torch.bfloat16)
+    out = torch.full((total + 1, H * hd), 9.0, dtype=torch.bfloat16, device="cuda")
+    first = [sum(lens[:i]) for i in range(len(lens))]
+    seqs = torch.tensor([[f, n, f, n] for f, n in zip(first, lens)], dtype=torch.int32, device="cuda")
+    st = ops.new_status("cuda")
+    kw = dict(n_heads=H, group=1, head_dim=hd, causal=False, q_strides=(3 * H * hd, hd), k_strides=(3 * H * hd, hd, 0),
+              v_strides=(3 * H * hd, hd, 0), o_strides=(H * hd, hd), q_rows_total=total, kv_rows_total=total, status=st)
+    ops.attention(qkv, qkv[:, H * hd:], qkv[:, 2 * H * hd:], out, seqs, max_q_len=max(lens), **kw)
+    ops.check_status(st)
+    for f, n in zip(first, lens):
+        q, k, v = (qkv[f:f + n, i * H * hd:(i + 1) * H * hd].float().view(n, H, hd).transpose(0, 1) for i in range(3))
+        want = torch.softmax(q @ k.transpose(1, 2) / hd ** 0.5, -1) @ v
+        got = out[f:f + n].float().view(n, H, hd).transpose(0, 1)
+        assert (got - want).abs().max() <= 2.0 ** -7 * want.abs().max()
+    assert (out[-1] == 9.0).all()
+    from ittai_b200 import _C
+    with pytest.raises(_C.IttaiError, match="head_dim 80"):
+        ops.attention(qkv, qkv[:, H * hd:], qkv[:, 2 * H * hd:], out, seqs, max_q_len=64, **kw)
