@@ -22,6 +22,8 @@ struct GemmArgs {
     float stats_eps;
     int stats_k;             // columns the folded LayerNorm's statistics are over (A may be zero-padded beyond them); 0 = K
     int stats_rms;           // 1: the folded norm is an RMSNorm (mean 0, rstd from the sum of squares alone)
+    const bf16* a_gain;      // [K] or nullptr.  Split-K kernel only: A is RMS-normalised on its way into the MMAs, with the rounding
+                             // steps of rmsnorm_rows_kernel; row_stats then holds the partial sums of A's rows (stats_parts > 0)
     IttaiQkRope rope;        // ITTAI_EPI_QKROPE only
 };
 

@@ -221,11 +221,12 @@ int gemm_args_from_abi(const IttaiGemm* a, GemmArgs* gp, CUtensorMap* tm_a, CUte
     g.stats_eps = a->stats_eps;
     g.stats_k = a->stats_k;
     g.stats_rms = a->stats_rms;
+    g.a_gain = nullptr;
     if (epi == ITTAI_EPI_QKROPE) g.rope = *a->qk_rope; else g.rope = IttaiQkRope{};
     return ITTAI_OK;
 }
 
-int gemm_bf16_launch(const IttaiGemm* a, cudaStream_t st) {
+int gemm_bf16_launch(const IttaiGemm* a, cudaStream_t st, const void* a_gain) {
     static thread_local int sm_dev = -1, attr_dev = -1, n_sms = 0;
     int dev = 0;
     cudaGetDevice(&dev);
@@ -236,6 +237,10 @@ int gemm_bf16_launch(const IttaiGemm* a, cudaStream_t st) {
     GemmArgs g;
     const int rc = gemm_args_from_abi(a, &g, &tm_a, &tm_b, a ? a->epi & ~ITTAI_GEMM_STATIC_W : 0, split, split || pair ? 128 : 64);
     if (rc != ITTAI_OK) return rc;
+    if (a_gain != nullptr) {
+        if (!split || g.stats_parts <= 0 || !g.stats_rms || ((uintptr_t)a_gain & 15)) { set_error("a norm inside the GEMM needs the split-K kernel and RMS partial sums"); return ITTAI_E_ARG; }
+        g.a_gain = reinterpret_cast<const bf16*>(a_gain);
+    }
     if (split) return gemm_split_launch(tm_a, tm_b, g, n_sms, st);
     if (pair) return gemm2_bf16_launch(tm_a, tm_b, g, st);
     if (attr_dev != dev) {
@@ -248,8 +253,10 @@ int gemm_bf16_launch(const IttaiGemm* a, cudaStream_t st) {
     return e == cudaSuccess ? ITTAI_OK : cuda_fail(e, "launch gemm_bf16_kernel");
 }
 
+int gemm_normed_launch(const IttaiGemm* a, const void* gain, cudaStream_t st) { return gemm_bf16_launch(a, st, gain); }
+
 }  // namespace ittai
 
 extern "C" int ittai_gemm_bf16_launch(const IttaiGemm* a, void* stream) {
-    return ittai::gemm_bf16_launch(a, reinterpret_cast<cudaStream_t>(stream));
+    return ittai::gemm_bf16_launch(a, reinterpret_cast<cudaStream_t>(stream), nullptr);
 }

@@ -9,6 +9,9 @@
 //   first stages are requested BEFORE griddepcontrol.wait: the caller has declared W constant (ITTAI_GEMM_STATIC_W), and two
 //   CTAs fit an SM (97 KB each), so the next GEMM's weights arrive while this one's epilogue runs;
 // * warp 1 (one lane) issues tcgen05.mma M128 N128 K16 into 128 columns of tensor memory;
+// * with GemmArgs::a_gain the other six warps RMS-normalise each landed A tile in place (valid rows only, the rounding steps of
+//   rmsnorm_rows_kernel) before the MMAs read it: the norm's own launch, a kernel boundary and a round trip of the activations
+//   through L2 twice per layer, goes;
 // * all eight warps then copy the valid rows of the partial tile to shared memory as fp32 (the ring is free by then), the
 //   cluster meets, and the rows are dealt out over its CTAs: a warp takes a row, lane l its columns 4l .. 4l+3, adds the
 //   splits in rank order through distributed shared memory and runs the epilogue.  A row in one warp makes the head norm
@@ -31,8 +34,9 @@ constexpr int kSplitStages = 3, kSplitThreads = 256, kMaxSplit = 8;
 constexpr uint32_t kSplitA = SM_ * SK * 2, kSplitB = SN * SK * 2;
 constexpr int kPartLd = SN + 4;                                  // fp32 per row of the partial tile: 16 bytes of padding keep
                                                                  // the row-per-thread 128-bit stores free of bank conflicts
-constexpr uint32_t kSplitSmem = kSplitStages * (kSplitA + kSplitB) + 1024 /*alignment*/ + 128 /*barriers*/;
+constexpr uint32_t kSplitSmem = kSplitStages * (kSplitA + kSplitB) + 1024 /*alignment*/ + 128 /*barriers*/ + SM_ * 4 /*row scales*/;
 static_assert(SM_ * kPartLd * 4 <= kSplitStages * (kSplitA + kSplitB), "the partial tile reuses the ring");
+constexpr int kNormWarps = kSplitThreads / 32 - 2;
 constexpr uint32_t kSplitSpin = 1u << 22;
 constexpr uint32_t kSplitCols = 128;
 
@@ -49,7 +53,7 @@ __device__ __forceinline__ float4 ld_cluster_f4(uint32_t addr) {
 // Epilogue of one row piece: lane l holds columns col0 + 4l .. + 3 of row `row` (whole warp, converged).
 __device__ __forceinline__ void split_epilogue_row(const GemmArgs& g, float (&v)[4], int row, int col0, int lane) {
     const int c = col0 + 4 * lane;
-    if (g.row_stats != nullptr) {
+    if (g.row_stats != nullptr && g.a_gain == nullptr) {
         float mean, rstd;
         if (g.stats_parts == 0) {
             const float2 ms = *reinterpret_cast<const float2*>(g.row_stats + 2 * (size_t)row);
@@ -139,7 +143,9 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constan
     unsigned long long* full = bars;
     unsigned long long* empty = bars + kSplitStages;
     unsigned long long* acc_full = bars + 2 * kSplitStages;
-    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 2 * kSplitStages + 1);
+    unsigned long long* ready = bars + 2 * kSplitStages + 1;          // [stages] A normalised
+    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 3 * kSplitStages + 1);
+    float* scale = reinterpret_cast<float*>(bars + 16);              // [128] 1 / rms of A's rows
     volatile uint32_t* abort_flag = tmem_slot + 1;
 
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -148,7 +154,7 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constan
     const int rows = min(SM_, g.M - tile_m * SM_);
 
     if (threadIdx.x == 0) {
-        for (int s = 0; s < kSplitStages; ++s) { mbar_init(&full[s], 1); mbar_init(&empty[s], 1); }
+        for (int s = 0; s < kSplitStages; ++s) { mbar_init(&full[s], 1); mbar_init(&empty[s], 1); mbar_init(&ready[s], kNormWarps); }
         mbar_init(acc_full, 1);
         *abort_flag = 0;
         fence_mbar_init();
@@ -185,7 +191,7 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constan
         bool ok = true;
         for (int kb = 0; kb < n_kb; ++kb) {
             const int s = kb % kSplitStages, use = kb / kSplitStages;
-            ok = mbar_wait_bounded(&full[s], use & 1, kSplitSpin) && !*abort_flag;
+            ok = mbar_wait_bounded(g.a_gain != nullptr ? &ready[s] : &full[s], use & 1, kSplitSpin) && !*abort_flag;
             if (!ok) break;
             tc_fence_after();
             const uint64_t da = umma_desc_sw128(sa + s * kSplitA), db = umma_desc_sw128(sb + s * kSplitB);
@@ -194,6 +200,45 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constan
             umma_commit(&empty[s]);
         }
         if (ok) umma_commit(acc_full); else *abort_flag = 1;
+    } else if (warp >= 2 && g.a_gain != nullptr) {
+        // a thread keeps to one 16-byte column piece of the tiles (192 threads, eight pieces a row), so its gains are one
+        // vector per k-block; the first is fetched ahead of the wait like the weights
+        const int t = threadIdx.x - 64, piece = t & 7;
+        const uint4* gains = reinterpret_cast<const uint4*>(g.a_gain + (size_t)kb0 * SK) + piece;
+        uint4 next = gains[0];
+        pdl_wait();
+        if (t < rows) {
+            const float2* ps = reinterpret_cast<const float2*>(g.row_stats) + (size_t)(tile_m * SM_ + t) * g.stats_parts;
+            float ss = 0.f;
+            for (int i = 0; i < g.stats_parts; ++i) ss += ps[i].y;
+            scale[t] = 1.0f / sqrtf(ss * (1.0f / (float)g.K) + g.stats_eps);
+        }
+        asm volatile("bar.sync 1, %0;" ::"n"(32 * kNormWarps) : "memory");
+        for (int kb = 0; kb < n_kb; ++kb) {
+            const int s = kb % kSplitStages, use = kb / kSplitStages;
+            const uint4 gq = next;
+            if (kb + 1 < n_kb) next = gains[8 * (kb + 1)];
+            bool ok = true;
+            uint32_t spins = 0;
+            while (!mbar_try_wait_parked(&full[s], use & 1)) {
+                if (((++spins) & 255u) == 0u && (*abort_flag || spins >= kSplitSpin)) { ok = false; break; }
+            }
+            if (!ok) { *abort_flag = 1; break; }
+            const uint32_t gw[4] = {gq.x, gq.y, gq.z, gq.w};
+            for (int r = t >> 3; r < rows; r += 4 * kNormWarps) {
+                uint4* p = reinterpret_cast<uint4*>(sa + s * kSplitA + r * 128 + ((piece ^ (r & 7)) << 4));
+                const uint4 x = *p;
+                const uint32_t xw[4] = {x.x, x.y, x.z, x.w};
+                const float rs = scale[r];
+                uint32_t o[4];
+#pragma unroll
+                for (int j = 0; j < 4; ++j) o[j] = pack_bf16x2(bf16r(bf_lo(xw[j]) * rs) * bf_lo(gw[j]), bf16r(bf_hi(xw[j]) * rs) * bf_hi(gw[j]));
+                *p = make_uint4(o[0], o[1], o[2], o[3]);
+            }
+            fence_proxy_async_smem();                                // the MMAs read through the async proxy
+            __syncwarp();
+            if (lane == 0) mbar_arrive(&ready[s]);
+        }
     }
     __syncwarp();
     pdl_wait();                                                      // the epilogue reads what the kernels before wrote

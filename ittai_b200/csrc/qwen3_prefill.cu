@@ -5,10 +5,12 @@
 #include <cuda_runtime.h>
 
 #include "../../include/ittai_b200.h"
+#include "gemm_split.h"
 
 namespace ittai {
 
 void set_error(const char* fmt, ...);
+int embed_rows_launch(const int32_t* ids, const void* table, void* out, int rows, int vocab, float* stats, void* stream);   // rowwise.cu
 
 constexpr int D = ITTAI_Q3_D, DQ = ITTAI_Q3_DQ, DQKV = ITTAI_Q3_DQKV, DGU = ITTAI_Q3_DGU, FF = ITTAI_Q3_FF, HD = ITTAI_Q3_HD, NKV = ITTAI_Q3_NKV;
 constexpr int NH = DQ / HD;
@@ -19,22 +21,28 @@ static int prefill_launch(const IttaiQwen3Prefill* p, void* st) {
     if (!p || p->n_layers < 1 || p->tokens < 1 || p->n_seqs < 1 || p->max_q_len < 1 || p->kv_cap < 1 || p->vocab < 1) { set_error("prefill: bad sizes"); return ITTAI_E_ARG; }
     if (!p->wqkv || !p->wo || !p->wgu || !p->wd || !p->ln1 || !p->ln2 || !p->qn || !p->kn || !p->embed || !p->rope || !p->ids || !p->pos || !p->seq ||
         !p->slot || !p->seqs || !p->kcache || !p->vcache || !p->h || !p->xn || !p->qkv || !p->attn || !p->act || !p->status ||
-        !p->wqkv_f != !p->wgu_f || (p->wqkv_f && (!p->stats || !p->zeros))) {
+        !p->wqkv_f != !p->wgu_f || ((p->wqkv_f || p->split_k) && (!p->stats || !p->zeros))) {
         set_error("prefill: null pointer");
         return ITTAI_E_ARG;
     }
     const int T = p->tokens;
     const bool fused = p->fused_rope && (T > 128 || p->split_k);     // at most 128 rows: only the split-K kernel rotates
     const bool fold = p->wqkv_f != nullptr && T > 128;
-    int rc = ittai_embed_rows(p->ids, p->embed, p->h, T, p->vocab, st);
-    auto gemm = [&](const void* a, const void* w, void* out, int n, int k, int epi, const void* residual, bool norm, bool stats, const IttaiQkRope* rope) {
+    int dev = 0, n_sms = 0;
+    cudaGetDevice(&dev);
+    cudaDeviceGetAttribute(&n_sms, cudaDevAttrMultiProcessorCount, dev);
+    // a small forward: both normalised projections run as split-K GEMMs, which normalise their input themselves
+    const bool normed = p->split_k && !fold && gemm_split_wins(T, DGU, n_sms) && gemm_split_wins(T, DQKV, n_sms);
+    int rc = embed_rows_launch(p->ids, p->embed, p->h, T, p->vocab, normed ? p->stats : nullptr, st);
+    auto gemm = [&](const void* a, const void* w, void* out, int n, int k, int epi, const void* residual, bool norm, bool stats, const IttaiQkRope* rope,
+                    const void* gain = nullptr) {
         if (rc != ITTAI_OK) return;
         IttaiGemm g = {};
         g.m = T; g.n = n; g.k = k; g.epi = epi | (p->split_k ? ITTAI_GEMM_STATIC_W : 0);
         g.a = a; g.w = w; g.out = out; g.residual = residual; g.status = p->status; g.qk_rope = rope;
         if (norm) { g.row_stats = p->stats; g.col_sums = p->zeros; g.stats_parts = D / 128; g.stats_eps = p->eps; g.stats_rms = 1; }
         if (stats) g.stats_out = p->stats;
-        rc = ittai_gemm_bf16_launch(&g, st);
+        rc = gain ? gemm_normed_launch(&g, gain, (cudaStream_t)st) : ittai_gemm_bf16_launch(&g, st);
     };
     auto norm = [&](const void* gain) { if (rc == ITTAI_OK) rc = ittai_rmsnorm_rows(p->h, D, gain, p->xn, D, T, p->eps, st); };
     for (int l = 0; l < p->n_layers && rc == ITTAI_OK; ++l) {
@@ -43,16 +51,17 @@ static int prefill_launch(const IttaiQwen3Prefill* p, void* st) {
         const void *qn = at(p->qn, (size_t)l * HD), *kn = at(p->kn, (size_t)l * HD);
         // layer 0 reads the embedding rows, which no GEMM epilogue produced: its first norm is a pass of its own
         const bool folded = fold && l > 0;
-        if (!folded) norm(at(p->ln1, (size_t)l * D));
-        const void* x = folded ? p->h : p->xn;
+        const void *g1 = at(p->ln1, (size_t)l * D), *g2 = at(p->ln2, (size_t)l * D);
+        if (!folded && !normed) norm(g1);
+        const void* x = folded || normed ? p->h : p->xn;
         const void* wq = at(folded ? p->wqkv_f : p->wqkv, (size_t)l * DQKV * D);
         if (fused) {
             IttaiQkRope r = {};
             r.qn = qn; r.kn = kn; r.rope = p->rope; r.pos = p->pos; r.seq = p->seq; r.slot = p->slot;
             r.kcache_layer = kc; r.vcache_layer = vc; r.kv_cap = p->kv_cap; r.eps = p->eps;
-            gemm(x, wq, p->qkv, DQKV, D, ITTAI_EPI_QKROPE, nullptr, folded, false, &r);
+            gemm(x, wq, p->qkv, DQKV, D, ITTAI_EPI_QKROPE, nullptr, folded || normed, false, &r, normed ? g1 : nullptr);
         } else {
-            gemm(x, wq, p->qkv, DQKV, D, ITTAI_EPI_NONE, nullptr, folded, false, nullptr);
+            gemm(x, wq, p->qkv, DQKV, D, ITTAI_EPI_NONE, nullptr, folded || normed, false, nullptr, normed ? g1 : nullptr);
             if (rc == ITTAI_OK) rc = ittai_qwen3_qk_rope_scatter(p->qkv, qn, kn, p->rope, p->pos, p->seq, p->slot, kc, vc, T, p->kv_cap, p->eps, st);
         }
         IttaiAttention a = {};
@@ -62,10 +71,10 @@ static int prefill_launch(const IttaiQwen3Prefill* p, void* st) {
         a.seqs = p->seqs; a.n_seqs = p->n_seqs; a.n_heads = NH; a.group = NH / NKV; a.head_dim = HD; a.causal = 1; a.max_q_len = p->max_q_len;
         a.q_rows_total = T; a.kv_rows_total = (int32_t)p->kv_rows_total; a.status = p->status;
         if (rc == ITTAI_OK) rc = ittai_attention_launch(&a, st);
-        gemm(p->attn, at(p->wo, (size_t)l * D * DQ), p->h, D, DQ, ITTAI_EPI_NONE, p->h, false, fold, nullptr);
-        if (!fold) norm(at(p->ln2, (size_t)l * D));
-        gemm(fold ? p->h : p->xn, at(fold ? p->wgu_f : p->wgu, (size_t)l * DGU * D), p->act, DGU, D, ITTAI_EPI_SWIGLU, nullptr, fold, false, nullptr);
-        gemm(p->act, at(p->wd, (size_t)l * D * FF), p->h, D, FF, ITTAI_EPI_NONE, p->h, false, fold && l + 1 < p->n_layers, nullptr);
+        gemm(p->attn, at(p->wo, (size_t)l * D * DQ), p->h, D, DQ, ITTAI_EPI_NONE, p->h, false, fold || normed, nullptr);
+        if (!fold && !normed) norm(g2);
+        gemm(fold || normed ? p->h : p->xn, at(fold ? p->wgu_f : p->wgu, (size_t)l * DGU * D), p->act, DGU, D, ITTAI_EPI_SWIGLU, nullptr, fold || normed, false, nullptr, normed ? g2 : nullptr);
+        gemm(p->act, at(p->wd, (size_t)l * D * FF), p->h, D, FF, ITTAI_EPI_NONE, p->h, false, (fold || normed) && l + 1 < p->n_layers, nullptr);
     }
     return rc;
 }

@@ -285,9 +285,10 @@ __global__ void __launch_bounds__(kRowThreads) positions_kernel(const float* __r
     }
 }
 
-// Embedding rows: out[t] = table[ids[t]], width 1024 (reference src/ittai/qwen3/base.py:147-162).
+// Embedding rows: out[t] = table[ids[t]], width 1024 (reference src/ittai/qwen3/base.py:147-162).  `stats` or null: [rows][8][2]
+// (sum, sum of squares) of every 128-column slice, as a GEMM's stats_out leaves them (16 lanes hold a slice).
 __global__ void __launch_bounds__(kRowThreads) embed_rows_kernel(const int* __restrict__ ids, const bf16* __restrict__ table,
-                                                                   bf16* __restrict__ out, int rows, int vocab) {
+                                                                   bf16* __restrict__ out, int rows, int vocab, float* __restrict__ stats) {
     pdl_trigger();
     pdl_wait();
     const int row = blockIdx.x * (kRowThreads / 32) + (threadIdx.x >> 5), lane = threadIdx.x & 31;
@@ -295,9 +296,19 @@ __global__ void __launch_bounds__(kRowThreads) embed_rows_kernel(const int* __re
     int id = ids[row];
     id = id < 0 ? 0 : (id >= vocab ? vocab - 1 : id);
 #pragma unroll
-    for (int i = 0; i < 4; ++i)
-        *reinterpret_cast<uint4*>(out + (size_t)row * 1024 + (lane + 32 * i) * 8) =
-            *reinterpret_cast<const uint4*>(table + (size_t)id * 1024 + (lane + 32 * i) * 8);
+    for (int i = 0; i < 4; ++i) {
+        const uint4 v = *reinterpret_cast<const uint4*>(table + (size_t)id * 1024 + (lane + 32 * i) * 8);
+        *reinterpret_cast<uint4*>(out + (size_t)row * 1024 + (lane + 32 * i) * 8) = v;
+        if (stats != nullptr) {
+            const uint32_t w[4] = {v.x, v.y, v.z, v.w};
+            float s1 = 0.f, s2 = 0.f;
+#pragma unroll
+            for (int j = 0; j < 4; ++j) { const float lo = bf_lo(w[j]), hi = bf_hi(w[j]); s1 += lo + hi; s2 = fmaf(lo, lo, fmaf(hi, hi, s2)); }
+#pragma unroll
+            for (int o = 8; o > 0; o >>= 1) { s1 += __shfl_xor_sync(0xffffffffu, s1, o); s2 += __shfl_xor_sync(0xffffffffu, s2, o); }
+            if ((lane & 15) == 0) *reinterpret_cast<float2*>(stats + 2 * ((size_t)row * 8 + 2 * i + (lane >> 4))) = make_float2(s1, s2);
+        }
+    }
 }
 
 // Embedding head of the reference: final RMSNorm of one row per sequence in fp32, then L2 normalisation
@@ -402,10 +413,16 @@ extern "C" int ittai_siglip_positions(const float* grid, int side, int width, co
     return e == cudaSuccess ? ITTAI_OK : cuda_fail(e, "launch positions_kernel");
 }
 
-extern "C" int ittai_embed_rows(const int32_t* ids, const void* table, void* out, int rows, int vocab, void* stream) {
+namespace ittai {
+int embed_rows_launch(const int32_t* ids, const void* table, void* out, int rows, int vocab, float* stats, void* stream) {
     if (!ids || !table || !out || rows < 1 || vocab < 1) { set_error("embed_rows: bad argument"); return ITTAI_E_ARG; }
-    launch_pdl(embed_rows_kernel, dim3(row_grid(rows)), dim3(kRowThreads), 0, (cudaStream_t)stream, 1, ids, (const bf16*)table, (bf16*)out, rows, vocab);
+    launch_pdl(embed_rows_kernel, dim3(row_grid(rows)), dim3(kRowThreads), 0, (cudaStream_t)stream, 1, ids, (const bf16*)table, (bf16*)out, rows, vocab, stats);
     return launched("embed_rows_kernel");
+}
+}  // namespace ittai
+
+extern "C" int ittai_embed_rows(const int32_t* ids, const void* table, void* out, int rows, int vocab, void* stream) {
+    return embed_rows_launch(ids, table, out, rows, vocab, nullptr, stream);
 }
 
 extern "C" int ittai_qwen3_final_pool(const void* h, const int32_t* rows, const void* gain, float* out, int n_seq, float eps, void* stream) {

@@ -71,8 +71,8 @@ class PrefillCore:
         if fold_norm:
             fold = lambda W, g: (W.float() * g.float()[:, None, :]).to(torch.bfloat16).contiguous()
             self.wqkv_f, self.wgu_f = fold(w["wqkv"], w["ln1"]), fold(w["wgu"], w["ln2"])
-            self.stats = torch.zeros(max_tokens, D // 128, 2, dtype=torch.float32, device=device)
-            self.zeros = torch.zeros(DGU, dtype=torch.float32, device=device)
+        self.stats = torch.empty(max_tokens, D // 128, 2, dtype=torch.float32, device=device)
+        self.zeros = torch.zeros(DGU, dtype=torch.float32, device=device)
         z = lambda *s: torch.empty(*s, dtype=torch.bfloat16, device=device)
         self.h, self.xn, self.qkv, self.attn, self.act = z(max_tokens, D), z(max_tokens, D), z(max_tokens, DQKV), z(max_tokens, DQ), z(max_tokens, FF)
         self.status = ops.new_status(device) if status is None else status
@@ -89,11 +89,12 @@ class PrefillCore:
         for name in ("wqkv", "wo", "wgu", "wd", "ln1", "ln2", "qn", "kn", "embed"):
             setattr(p, name, w[name].data_ptr())
         if self.fold_norm:
-            p.wqkv_f, p.wgu_f, p.stats, p.zeros = self.wqkv_f.data_ptr(), self.wgu_f.data_ptr(), self.stats.data_ptr(), self.zeros.data_ptr()
+            p.wqkv_f, p.wgu_f = self.wqkv_f.data_ptr(), self.wgu_f.data_ptr()
         p.rope, p.ids, p.pos, p.seq, p.slot, p.seqs = (t.data_ptr() for t in (rope, tokens, pos, seq, slot, seqs))
         p.kcache, p.vcache, p.kv_layer = kcache.data_ptr(), vcache.data_ptr(), kv_layer
         (p.k_row, p.k_head, p.k_seq), p.kv_rows_total = k_strides, (kv_layer or kcache.numel()) // HD
-        p.h, p.xn, p.qkv, p.attn, p.act, p.status = (t.data_ptr() for t in (self.h, self.xn, self.qkv, self.attn, self.act, self.status))
+        p.h, p.xn, p.qkv, p.attn, p.act, p.stats, p.zeros, p.status = (
+            t.data_ptr() for t in (self.h, self.xn, self.qkv, self.attn, self.act, self.stats, self.zeros, self.status))
         _C.check(_C.lib().ittai_qwen3_prefill_launch(C.byref(p), ops._stream(self.h)))
         return self.h[:T]
 
