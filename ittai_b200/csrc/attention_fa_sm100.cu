@@ -14,8 +14,14 @@
 //     then has to be rescaled (load, multiply, store), which is rare after the first blocks; P may exceed 1 by up to
 //     2^8 in between, harmless in bf16/fp32, and the final O / rowsum is exact either way.
 // TMEM (256 columns, two CTAs per SM): S / P in columns 0..127, O in 128..255.  Shared memory: Q, K, V tiles of 32 KB each
-// (two 128-byte-swizzled atoms of 64 dims); the Q tile doubles as the output staging area.  Every wait is a bounded
-// mbarrier wait; on expiry the abort flag routes all roles to the common exit, where TMEM is freed.
+// (two 128-byte-swizzled atoms of 64 dims); the V tile doubles as the output staging area.
+//
+// A CTA does not end with its tile: it takes over the next tile that no CTA has begun (clusterlaunchcontrol.try_cancel: the
+// hardware hands the CTAs out in index order as before, so the balance stays dynamic and the longest tiles first) and works
+// across the seam: the next Q and first K block travel from the moment the last S of this tile is complete, and the next
+// tile's first S is computed while this one's output is stored.  Launch, barrier set-up, tensor-memory allocation, the first
+// loads and the first S were 7 us of a tile's 13 at 512 tokens (2.3 us per key block).  Every wait is a bounded mbarrier
+// wait; on expiry the abort flag routes all roles to the common exit, where TMEM is freed.
 #include "launch.h"
 #include "tcgen05.cuh"
 #include "tmap.h"
@@ -57,6 +63,65 @@ __device__ __forceinline__ float fa_ex2(float x) {
     return y;
 }
 
+__device__ __forceinline__ bool fa_test(void* bar, uint32_t parity) {
+    uint32_t ok;
+    asm volatile("{\n.reg .pred p;\nmbarrier.test_wait.parity.shared::cta.b64 p, [%1], %2;\nselp.u32 %0, 1, 0, p;\n}\n" : "=r"(ok) : "r"(smem_u32(bar)), "r"(parity) : "memory");
+    return ok != 0;
+}
+// Asks for a CTA of this grid that has not begun; the 16-byte answer is counted on `bar`.
+__device__ __forceinline__ void fa_try_cancel(void* answer, void* bar) {
+    asm volatile("clusterlaunchcontrol.try_cancel.async.shared::cta.mbarrier::complete_tx::bytes.b128 [%0], [%1];" ::"r"(smem_u32(answer)), "r"(smem_u32(bar)) : "memory");
+}
+// (x, y, z) of the CTA taken over and 1, or w = 0: none was left.
+__device__ __forceinline__ int4 fa_answer(const void* answer) {
+    int4 id = make_int4(0, 0, 0, 0);
+    asm volatile(
+        "{\n"
+        ".reg .pred p;\n"
+        ".reg .b128 r;\n"
+        "ld.shared.b128 r, [%4];\n"
+        "clusterlaunchcontrol.query_cancel.is_canceled.pred.b128 p, r;\n"
+        "selp.s32 %3, 1, 0, p;\n"
+        "@p clusterlaunchcontrol.query_cancel.get_first_ctaid.v4.b32.b128 {%0, %1, %2, _}, r;\n"
+        "}\n"
+        : "+r"(id.x), "+r"(id.y), "+r"(id.z), "=r"(id.w) : "r"(smem_u32(answer)) : "memory");
+    return id;
+}
+// One query tile: where it lies and how many key blocks it sees.
+struct FaTile { int head, r0, q_len, kv_len, n_blk, q_row, q_col, kv_row, kv_col; };
+template <int HDIM>
+__device__ __forceinline__ FaTile fa_tile(const AttnFaArgs& a, int x, int y, int z) {
+    const int4 sinfo = a.seqs[y];                          // written by the host long before: safe ahead of pdl_wait
+    FaTile t;
+    t.head = x; t.r0 = ((int)gridDim.z - 1 - z) * kFaBlk; t.q_len = sinfo.y; t.kv_len = sinfo.w;
+    // causal: query r sees keys <= r + (kv_len - q_len)
+    const int last_key = a.causal ? min(t.kv_len - 1, t.r0 + kFaBlk - 1 + t.kv_len - t.q_len) : t.kv_len - 1;
+    t.n_blk = last_key < 0 ? 0 : last_key / kFaBlk + 1;
+    const int kvh = x / a.group;
+    t.q_row = sinfo.x + t.r0; t.q_col = x * HDIM;
+    t.kv_row = y * a.k_seq_rows + kvh * a.k_head_rows + sinfo.z; t.kv_col = kvh * a.k_head_cols;
+    return t;
+}
+template <int HDIM>
+__device__ __forceinline__ FaTile fa_tile(const AttnFaArgs& a, int index) {
+    const int yz = index / (int)gridDim.x;
+    return fa_tile<HDIM>(a, index - yz * (int)gridDim.x, yz % (int)gridDim.y, yz / (int)gridDim.y);
+}
+template <int HDIM>
+__device__ __forceinline__ void fa_zero_rows(const AttnFaArgs& a, const FaTile& t, int tid, int threads) {
+    for (int i = tid; i < kFaBlk * 16; i += threads) {
+        const int row = i >> 4;
+        if (t.r0 + row < t.q_len && (i & 15) < HDIM / 8)
+            *reinterpret_cast<uint4*>(a.o + (long long)(t.q_row + row) * a.o_row + (long long)t.head * a.o_head + (i & 15) * 8) = make_uint4(0, 0, 0, 0);
+    }
+}
+// Both 64-column atoms of a tile of 128 rows.
+__device__ __forceinline__ void fa_load(unsigned char* dst, const CUtensorMap* tm, int col, int row, void* bar) {
+    mbar_expect_tx(bar, 32768);
+    tma_load_2d(dst, tm, col, row, bar);
+    tma_load_2d(dst + 16384, tm, col + 64, row, bar);
+}
+
 // HDIM: 128, or 80 for heads packed 80 columns apart (a head_dim of 72, zero-padded to whole k-steps of 16): S then takes five
 // k-steps instead of eight and the projections around the kernel are 80/128 as wide.  The loads still fetch 128 columns (the
 // next head's, or zeros past the last one) and P V still computes 128: an MN-major operand comes in whole 64-column atoms.
@@ -67,21 +132,13 @@ attn_fa_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
                const __grid_constant__ CUtensorMap tm_v, const AttnFaArgs a) {
     pdl_trigger();
     // Grid (heads, sequences, query tiles) with the tiles in descending order: CTAs are handed out in index order, so the
-    // causal tiles that walk the most key blocks start first and the last wave is made of the short ones.
-    const int head = blockIdx.x, seq = blockIdx.y, mt = (int)gridDim.z - 1 - (int)blockIdx.z, kvh = head / a.group;
-    const int4 sinfo = a.seqs[seq];                        // written by the host long before: safe ahead of pdl_wait
-    const int q_len = sinfo.y, kv_len = sinfo.w, r0 = mt * kFaBlk;
-    if (r0 >= q_len) return;                               // the whole CTA: nothing allocated yet
-    const int offset = kv_len - q_len;                     // causal: query r sees keys <= r + offset
-    const int last_key = a.causal ? min(kv_len - 1, r0 + kFaBlk - 1 + offset) : kv_len - 1;
-    const int n_blk = last_key < 0 ? 0 : last_key / kFaBlk + 1;
+    // causal tiles that walk the most key blocks start first and the last ones are short.
+    const FaTile first = fa_tile<HDIM>(a, blockIdx.x, blockIdx.y, blockIdx.z);
+    if (first.r0 >= first.q_len) return;                   // the whole CTA: nothing allocated yet
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    if (n_blk == 0) {                                      // no visible key: zero rows
+    if (first.n_blk == 0) {                                // no visible key: zero rows
         pdl_wait();
-        for (int i = threadIdx.x; i < kFaBlk * 16; i += kFaThreads) {
-            const int row = r0 + (i >> 4);
-            if (row < q_len && (i & 15) < HDIM / 8) *reinterpret_cast<uint4*>(a.o + (long long)(sinfo.x + row) * a.o_row + (long long)head * a.o_head + (i & 15) * 8) = make_uint4(0, 0, 0, 0);
-        }
+        fa_zero_rows<HDIM>(a, first, threadIdx.x, kFaThreads);
         return;
     }
 
@@ -94,25 +151,23 @@ attn_fa_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
     unsigned long long* bar_s = bars + 3;         // S of the block ready (also: K buffer free)
     unsigned long long* bar_p = bars + 4;         // P written, O rescaled (one arrival per softmax warp)
     unsigned long long* bar_o = bars + 5;         // PV of the block done (also: V buffer free)
-    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 8);
+    unsigned long long* bar_e = bars + 6;         // output stored: V buffer and O free (one arrival per softmax warp, one phase per tile)
+    unsigned long long* bar_t = bars + 7;         // [2] next tile published, tile n in slot n % 2
+    unsigned long long* bar_c = bars + 9;         // answer to try_cancel landed
+    unsigned char* answer = reinterpret_cast<unsigned char*>(bars + 10);     // 16 bytes
+    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 12);
     volatile uint32_t* abort_flag = tmem_slot + 1;
-    const int kv_row = seq * a.k_seq_rows + kvh * a.k_head_rows + sinfo.z;   // first key row of this (sequence, kv head)
-    const int kc = kvh * a.k_head_cols;                                             // and its first column
+    volatile int* next_tile = reinterpret_cast<volatile int*>(tmem_slot + 2);    // [2] CTA index, -1: none
 
     if (threadIdx.x == 0) {
         mbar_init(bar_q, 1); mbar_init(bar_k, 1); mbar_init(bar_v, 1); mbar_init(bar_s, 1); mbar_init(bar_p, 4); mbar_init(bar_o, 1);
+        mbar_init(bar_e, 4); mbar_init(bar_t, 1); mbar_init(bar_t + 1, 1); mbar_init(bar_c, 1);
         *abort_flag = 0;
         fence_mbar_init();
         pdl_wait();                                        // q, k, v come from the kernels before this one
-        mbar_expect_tx(bar_q, 32768);
-        tma_load_2d(sm + kFaQ, &tm_q, head * HDIM, sinfo.x + r0, bar_q);
-        tma_load_2d(sm + kFaQ + 16384, &tm_q, head * HDIM + 64, sinfo.x + r0, bar_q);
-        mbar_expect_tx(bar_k, 32768);
-        tma_load_2d(sm + kFaK, &tm_k, kc, kv_row, bar_k);
-        tma_load_2d(sm + kFaK + 16384, &tm_k, kc + 64, kv_row, bar_k);
-        mbar_expect_tx(bar_v, 32768);
-        tma_load_2d(sm + kFaV, &tm_v, kc, kv_row, bar_v);
-        tma_load_2d(sm + kFaV + 16384, &tm_v, kc + 64, kv_row, bar_v);
+        fa_load(sm + kFaQ, &tm_q, first.q_col, first.q_row, bar_q);
+        fa_load(sm + kFaK, &tm_k, first.kv_col, first.kv_row, bar_k);
+        fa_load(sm + kFaV, &tm_v, first.kv_col, first.kv_row, bar_v);
     }
     if (warp == 0) { __syncwarp(); tmem_alloc(tmem_slot, kFaCols); }
     tc_fence_before();
@@ -124,56 +179,112 @@ attn_fa_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
     if (warp == 0) {
         if (lane == 0) {
             constexpr uint32_t idesc_s = umma_idesc_bf16(128, 128), idesc_o = umma_idesc_bf16(128, 128) | umma_idesc_b_mn;
-            bool ok = fa_wait(bar_q, 0, abort_flag);
-            for (int j = 0; j < n_blk && ok; ++j) {
-                const uint32_t ph = j & 1;
-                ok = fa_wait(bar_k, ph, abort_flag);
-                if (!ok) break;
-                tc_fence_after();
-                // ---- S = Q K^T over the 128 dims: atoms of 64 dims, 4 k-steps each
-#pragma unroll
-                for (int k = 0; k < HDIM / 16; ++k)
-                    umma_bf16(tmem_base, umma_desc_sw128(sm + kFaQ + (k >> 2) * 16384) + 2 * (k & 3),
-                              umma_desc_sw128(sm + kFaK + (k >> 2) * 16384) + 2 * (k & 3), idesc_s, k > 0 ? 1u : 0u);
-                umma_commit(bar_s);
-                if (j > 0) {
-                    // the previous PV has finished reading the V buffer: refill it
-                    ok = fa_wait(bar_o, (j - 1) & 1, abort_flag);
+            FaTile cur = first, nt = first;
+            uint32_t c = 0, asked = 0, nq = 0;               // key blocks before this tile, questions answered, Q tiles before this one
+            int next;                                        // CTA index taken over, -1: none left, -2: not known yet
+            bool ok = true;
+            auto ask = [&]() {
+                fence_proxy_async_smem();                    // the last answer has been read
+                mbar_expect_tx(bar_c, 16);
+                fa_try_cancel(answer, bar_c);
+            };
+            // Takes the answer if it is there (or waits for it); an empty tile is passed over.
+            auto resolve = [&](bool wait) {
+                while (next == -2) {
+                    if (!fa_test(bar_c, asked & 1)) {
+                        if (!wait) return;
+                        if (!fa_wait(bar_c, asked & 1, abort_flag)) { ok = false; return; }
+                    }
+                    ++asked;
+                    const int4 id = fa_answer(answer);
+                    if (id.w == 0) { next = -1; return; }
+                    nt = fa_tile<HDIM>(a, id.x, id.y, id.z);
+                    if (nt.r0 >= nt.q_len) ask();
+                    else next = (id.z * (int)gridDim.y + id.y) * (int)gridDim.x + id.x;
+                }
+            };
+            auto load_next = [&]() {                         // Q and K are free once the last S of this tile is complete
+                if (nt.n_blk == 0) return;
+                fa_load(sm + kFaQ, &tm_q, nt.q_col, nt.q_row, bar_q);
+                fa_load(sm + kFaK, &tm_k, nt.kv_col, nt.kv_row, bar_k);
+            };
+            for (int t = 0; ok; ++t) {
+                const int n_blk = cur.n_blk;
+                bool loaded = false;
+                next = -2;
+                if (n_blk == 0) ask();
+                else ok = fa_wait(bar_q, nq & 1, abort_flag);
+                for (int j = 0; j < n_blk && ok; ++j) {
+                    const uint32_t ph = (c + j) & 1;
+                    ok = fa_wait(bar_k, ph, abort_flag);
                     if (!ok) break;
-                    mbar_expect_tx(bar_v, 32768);
-                    tma_load_2d(sm + kFaV, &tm_v, kc, kv_row + j * kFaBlk, bar_v);
-                    tma_load_2d(sm + kFaV + 16384, &tm_v, kc + 64, kv_row + j * kFaBlk, bar_v);
-                }
-                ok = fa_wait(bar_s, ph, abort_flag);
-                if (!ok) break;
-                if (j + 1 < n_blk) {
-                    // S is complete, so the K buffer is free: the next block's keys travel during this block's softmax
-                    mbar_expect_tx(bar_k, 32768);
-                    tma_load_2d(sm + kFaK, &tm_k, kc, kv_row + (j + 1) * kFaBlk, bar_k);
-                    tma_load_2d(sm + kFaK + 16384, &tm_k, kc + 64, kv_row + (j + 1) * kFaBlk, bar_k);
-                }
-                ok = fa_wait(bar_p, ph, abort_flag) && fa_wait(bar_v, ph, abort_flag);
-                if (!ok) break;
-                tc_fence_after();
-                // ---- O += P V: P from tensor memory (8 columns per 16 keys), V rows 16 at a time, one series per dim half
-                {
-                    const uint64_t dv = umma_desc_sw128_mn(sm + kFaV, 16384);      // both 64-dim atoms of the V tile: N = 128
+                    tc_fence_after();
+                    if (j == n_blk - 1) ask();
+                    // ---- S = Q K^T over the head's dims: atoms of 64 dims, 4 k-steps each
 #pragma unroll
-                    for (int ks = 0; ks < 8; ++ks)
-                        umma_bf16_tmem_a(tmem_base + kFaOCol, tmem_base + 8 * ks, dv + (uint64_t)ks * (2048 >> 4), idesc_o,
-                                         (j > 0 || ks > 0) ? 1u : 0u);
+                    for (int k = 0; k < HDIM / 16; ++k)
+                        umma_bf16(tmem_base, umma_desc_sw128(sm + kFaQ + (k >> 2) * 16384) + 2 * (k & 3),
+                                  umma_desc_sw128(sm + kFaK + (k >> 2) * 16384) + 2 * (k & 3), idesc_s, k > 0 ? 1u : 0u);
+                    umma_commit(bar_s);
+                    if (j > 0 || t > 0) {
+                        // the previous PV has finished reading the V buffer, or the tile before has left it: refill it (waiting
+                        // for bar_e twice, after a tile without keys, passes at once)
+                        ok = j > 0 ? fa_wait(bar_o, (c + j - 1) & 1, abort_flag) : fa_wait(bar_e, (t - 1) & 1, abort_flag);
+                        if (!ok) break;
+                        tc_fence_after();
+                        fa_load(sm + kFaV, &tm_v, cur.kv_col, cur.kv_row + j * kFaBlk, bar_v);
+                    }
+                    ok = fa_wait(bar_s, ph, abort_flag);
+                    if (!ok) break;
+                    if (j + 1 < n_blk) {
+                        // S is complete, so the K buffer is free: the next block's keys travel during this block's softmax
+                        fa_load(sm + kFaK, &tm_k, cur.kv_col, cur.kv_row + (j + 1) * kFaBlk, bar_k);
+                    } else {
+                        // the same for the next tile, if it is known before the softmax is through
+                        for (uint32_t spins = 0; next == -2 && spins < kFaSpin && !fa_test(bar_p, ph); ++spins) resolve(false);
+                        if (next >= 0) { load_next(); loaded = true; }
+                    }
+                    ok = fa_wait(bar_p, ph, abort_flag) && fa_wait(bar_v, ph, abort_flag);
+                    if (!ok) break;
+                    tc_fence_after();
+                    // ---- O += P V: P from tensor memory (8 columns per 16 keys), V rows 16 at a time, one series per dim half
+                    {
+                        const uint64_t dv = umma_desc_sw128_mn(sm + kFaV, 16384);      // both 64-dim atoms of the V tile: N = 128
+#pragma unroll
+                        for (int ks = 0; ks < 8; ++ks)
+                            umma_bf16_tmem_a(tmem_base + kFaOCol, tmem_base + 8 * ks, dv + (uint64_t)ks * (2048 >> 4), idesc_o,
+                                             (j > 0 || ks > 0) ? 1u : 0u);
+                    }
+                    umma_commit(bar_o);
                 }
-                umma_commit(bar_o);
+                if (!ok) break;
+                resolve(true);
+                if (!ok) break;
+                if (next >= 0 && !loaded) load_next();
+                // a tile without keys passes through no MMA: bar_e would get a phase ahead of this thread
+                if (next >= 0 && nt.n_blk == 0 && !fa_wait(bar_e, t & 1, abort_flag)) break;
+                // slot (t + 1) % 2 was read before tile t - 1 ended, which bar_e has shown
+                next_tile[(t + 1) & 1] = next;
+                fa_arrive(bar_t + ((t + 1) & 1));
+                if (next < 0) break;
+                c += n_blk;
+                nq += n_blk > 0 ? 1 : 0;
+                cur = nt;
             }
         }
-    } else do {
+    } else {
+      int index = ((int)blockIdx.z * (int)gridDim.y + (int)blockIdx.y) * (int)gridDim.x + (int)blockIdx.x;
+      uint32_t c = 0;                                        // key blocks before this tile
+      for (int t = 0;; ++t) {
         const int q4 = warp & 3, r = q4 * 32 + lane;         // TMEM lane quarter; query row inside the tile
+        const FaTile tile = fa_tile<HDIM>(a, index);
+        const int n_blk = tile.n_blk, kv_len = tile.kv_len;
         const uint32_t t_row = tmem_base + ((uint32_t)(q4 * 32) << 16);
-        const int row_limit = a.causal ? min(kv_len - 1, r0 + r + offset) : kv_len - 1;   // last key this row sees
+        const int row_limit = a.causal ? min(kv_len - 1, tile.r0 + r + kv_len - tile.q_len) : kv_len - 1;   // last key this row sees
         float m_used = -INFINITY, l0 = 0.f, l1 = 0.f;       // running maximum in scaled (log2) units, running sum
         bool ok = true;
         for (int j = 0; j < n_blk; ++j) {
-            const uint32_t ph = j & 1;
+            const uint32_t ph = (c + j) & 1;
             ok = fa_wait(bar_s, ph, abort_flag);
             if (!ok) break;
             tc_fence_after();
@@ -215,7 +326,7 @@ attn_fa_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
             } else {
                 const bool need = bm - m_used > kFaRescale;      // false for NaN / -inf
                 if (__any_sync(0xffffffffu, need)) {
-                    ok = fa_wait(bar_o, (j - 1) & 1, abort_flag);   // O must be complete before it is rewritten
+                    ok = fa_wait(bar_o, (c + j - 1) & 1, abort_flag);   // O must be complete before it is rewritten
                     if (!ok) break;
                     tc_fence_after();
                     const float alpha = need ? fa_ex2(m_used - bm) : 1.0f;
@@ -287,13 +398,14 @@ attn_fa_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
             if (lane == 0) fa_arrive(bar_p);
         }
         if (!ok) break;
-        // ---- epilogue: O / rowsum -> bf16 -> staging tile (the Q tile is dead) -> whole 256-byte rows
-        ok = fa_wait(bar_o, (n_blk - 1) & 1, abort_flag);
+        if (n_blk > 0) {
+        // ---- epilogue: O / rowsum -> bf16 -> staging tile (the V tile is dead) -> whole rows
+        ok = fa_wait(bar_o, (c + n_blk - 1) & 1, abort_flag);
         if (!ok) break;
         tc_fence_after();
         const float l = l0 + l1;
         const float inv = l > 0.f ? 1.0f / l : 0.f;
-        unsigned char* stage = sm + kFaQ;
+        unsigned char* stage = sm + kFaV;
 #pragma unroll 1
         for (int c0 = 0; c0 < HDIM; c0 += 32) {
             uint32_t v[32];
@@ -309,13 +421,24 @@ attn_fa_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
         }
         __syncwarp();
         const int sub = lane & 15;
+        const FaTile out = fa_tile<HDIM>(a, index);          // once more: kept across the key loop it would cost registers there
 #pragma unroll 4
         for (int it = 0; it < 16; ++it) {
-            const int rr = q4 * 32 + it * 2 + (lane >> 4), row = r0 + rr;
+            const int rr = q4 * 32 + it * 2 + (lane >> 4), row = out.r0 + rr;
             const uint4 val = *reinterpret_cast<const uint4*>(stage + rr * 256 + ((sub ^ (rr & 15)) << 4));
-            if (row < q_len && sub < HDIM / 8) *reinterpret_cast<uint4*>(a.o + (long long)(sinfo.x + row) * a.o_row + (long long)head * a.o_head + 8 * sub) = val;
+            if (row < out.q_len && sub < HDIM / 8) *reinterpret_cast<uint4*>(a.o + (long long)(out.q_row + rr) * a.o_row + (long long)out.head * a.o_head + 8 * sub) = val;
         }
-    } while (false);
+        } else fa_zero_rows<HDIM>(a, tile, threadIdx.x - 32, 128);
+        fence_proxy_async_smem();                            // the next V block is written through the async proxy
+        tc_fence_before();
+        __syncwarp();
+        if (lane == 0) fa_arrive(bar_e);
+        c += n_blk;
+        if (!fa_wait(bar_t + ((t + 1) & 1), (t >> 1) & 1, abort_flag)) break;
+        index = next_tile[(t + 1) & 1];
+        if (index < 0) break;
+      }
+    }
     tc_fence_before();
     __syncthreads();
     if (*abort_flag) {

@@ -1,0 +1,47 @@
+"""The key-loop attention kernel on grids of many more tiles than can be resident, so that CTAs take over one another's (GPU)."""
+import pytest
+import torch
+
+gpu = pytest.mark.gpu
+
+
+@gpu
+@pytest.mark.parametrize("causal", [True, False])
+@pytest.mark.parametrize("lens,prefix", [([0, 600, 1, 64, 129, 0, 128, 257, 511, 512, 65, 0] * 4, 0), ([130] * 40, 37), ([2000, 0, 700], 0), ([65], 0)])
+def test_ragged_tiles(lens, prefix, causal):
+    """Empty sequences, one-row tiles, sequences without a single key (rows of zeros) and a cached prefix.  P is rounded to bf16
+    (2^-9 relative on weights that sum to 1) and so is the result: 2^-7 of the largest value."""
+    from ittai_b200 import ops
+    H, KV, hd = 4, 2, 128
+    n, total = len(lens), sum(lens)
+    cap = max(lens) + prefix
+    kv = [0 if i % 7 == 6 and not causal else m + prefix if m else 0 for i, m in enumerate(lens)]
+    g = torch.Generator(device="cuda").manual_seed(total + prefix)
+    q = torch.randn(total, H * hd, generator=g, device="cuda").to(torch.bfloat16)
+    kc, vc = (torch.randn(n, KV, cap, hd, generator=g, device="cuda").to(torch.bfloat16) for _ in range(2))
+    for i, m in enumerate(kv):
+        vc[i, :, m:] = float("nan")                        # never written cache rows
+    first = [sum(lens[:i]) for i in range(n)]
+    seqs = torch.tensor([[f, m, 0, k] for f, m, k in zip(first, lens, kv)], dtype=torch.int32, device="cuda")
+    out = torch.full((total + 1, H * hd), 9.0, dtype=torch.bfloat16, device="cuda")
+    st = ops.new_status("cuda")
+    for _ in range(2):
+        ops.attention(q, kc, vc, out, seqs, n_heads=H, group=H // KV, head_dim=hd, causal=causal, max_q_len=max(lens), q_strides=(H * hd, hd),
+                      k_strides=(hd, cap * hd, KV * cap * hd), v_strides=(hd, cap * hd, KV * cap * hd), o_strides=(H * hd, hd),
+                      q_rows_total=total, kv_rows_total=n * KV * cap, status=st)
+    ops.check_status(st)
+    assert (out[-1] == 9.0).all()
+    for i, (f, m, k) in enumerate(zip(first, lens, kv)):
+        if m == 0:
+            continue
+        got = out[f:f + m].float().view(m, H, hd).transpose(0, 1)
+        if k == 0:
+            assert (got == 0).all()
+            continue
+        qi = q[f:f + m].float().view(m, H, hd).transpose(0, 1)
+        ki, vi = (c[i, :, :k].float().repeat_interleave(H // KV, 0) for c in (kc, vc))
+        s = qi @ ki.transpose(1, 2) / hd ** 0.5
+        if causal:
+            s = s.masked_fill(torch.arange(k, device="cuda")[None, :] > torch.arange(m, device="cuda")[:, None] + k - m, float("-inf"))
+        want = torch.softmax(s, -1) @ vi
+        assert (got - want).abs().max() <= 2.0 ** -7 * want.abs().max(), (i, m, k)
