@@ -16,6 +16,9 @@
 
 namespace ittai {
 
+__device__ __forceinline__ __nv_bfloat162 as_bf162(uint32_t u) { __nv_bfloat162 v; memcpy(&v, &u, 4); return v; }
+__device__ __forceinline__ uint32_t as_u32(__nv_bfloat162 v) { uint32_t u; memcpy(&u, &v, 4); return u; }
+
 // ITTAI_EPI_QKROPE: one warp = 32 tokens x one head (its 128 accumulator columns).  The thread that owns a token's row
 // rounds the 128 values to bf16 (the Linear output), and for q / k heads applies the head RMSNorm and the half-split
 // rotary embedding with the rounding steps of the eager modules (the arithmetic of qk_rope_scatter_kernel); q goes
@@ -36,11 +39,14 @@ __device__ __forceinline__ void epilogue_qkrope(const GemmArgs& g, const CUtenso
         for (int i = 0; i < 16; ++i) pk[16 * ch + i] = pack_bf16x2(__uint_as_float(r[2 * i]) * row_scale, __uint_as_float(r[2 * i + 1]) * row_scale);   // a folded RMSNorm's rstd of the row, else 1
     }
     if (head < 24) {
-        float ss = 0.f;
+        float s0 = 0.f, s1 = 0.f;
 #pragma unroll
-        for (int i = 0; i < 64; ++i) { const float lo = bf_lo(pk[i]), hi = bf_hi(pk[i]); ss = fmaf(lo, lo, fmaf(hi, hi, ss)); }
-        const float rstd = 1.0f / sqrtf(ss * (1.0f / HD) + g.rope.eps);
+        for (int i = 0; i < 64; ++i) { const float lo = bf_lo(pk[i]), hi = bf_hi(pk[i]); s0 = fmaf(lo, lo, s0); s1 = fmaf(hi, hi, s1); }
+        const float rstd = 1.0f / sqrtf((s0 + s1) * (1.0f / HD) + g.rope.eps);
         const bf16* rp = reinterpret_cast<const bf16*>(g.rope.rope) + (size_t)(valid ? g.rope.pos[t] : 0) * HD;
+        // Only x * rstd is an fp32 product; every later step is a product or a sum of two bf16 values rounded to bf16, which is
+        // one packed instruction for two elements (the _rn forms: never contracted into an FMA).  Through fp32 and back each step was a conversion per element, ten per
+        // pair on a pipe of 16 lanes per SM: 10 k cycles of a tile's 14 k (main loop: 8 k).
 #pragma unroll
         for (int jj = 0; jj < 8; ++jj) {                  // elements 8jj .. 8jj+7 and their partners 64 + the same
             const uint4 cw = *reinterpret_cast<const uint4*>(rp + 8 * jj), sw = *reinterpret_cast<const uint4*>(rp + HD / 2 + 8 * jj);
@@ -49,18 +55,12 @@ __device__ __forceinline__ void epilogue_qkrope(const GemmArgs& g, const CUtenso
             const uint32_t wga[4] = {ga.x, ga.y, ga.z, ga.w}, wgb[4] = {gb.x, gb.y, gb.z, gb.w};
 #pragma unroll
             for (int j = 0; j < 4; ++j) {
-                float lo[2], hi[2];
-#pragma unroll
-                for (int h = 0; h < 2; ++h) {
-                    const float xa = h ? bf_hi(pk[4 * jj + j]) : bf_lo(pk[4 * jj + j]), xb = h ? bf_hi(pk[32 + 4 * jj + j]) : bf_lo(pk[32 + 4 * jj + j]);
-                    const float g0 = h ? bf_hi(wga[j]) : bf_lo(wga[j]), g1 = h ? bf_hi(wgb[j]) : bf_lo(wgb[j]);
-                    const float cs = h ? bf_hi(wc[j]) : bf_lo(wc[j]), sn = h ? bf_hi(ws[j]) : bf_lo(ws[j]);
-                    const float x0 = bf16r(bf16r(xa * rstd) * g0), x1 = bf16r(bf16r(xb * rstd) * g1);
-                    lo[h] = bf16r(bf16r(x0 * cs) + bf16r(-x1 * sn));
-                    hi[h] = bf16r(bf16r(x1 * cs) + bf16r(x0 * sn));
-                }
-                pk[4 * jj + j] = pack_bf16x2(lo[0], lo[1]);
-                pk[32 + 4 * jj + j] = pack_bf16x2(hi[0], hi[1]);
+                const uint32_t ua = pk[4 * jj + j], ub = pk[32 + 4 * jj + j];
+                const __nv_bfloat162 x0 = __hmul2_rn(as_bf162(pack_bf16x2(bf_lo(ua) * rstd, bf_hi(ua) * rstd)), as_bf162(wga[j]));
+                const __nv_bfloat162 x1 = __hmul2_rn(as_bf162(pack_bf16x2(bf_lo(ub) * rstd, bf_hi(ub) * rstd)), as_bf162(wgb[j]));
+                const __nv_bfloat162 cs = as_bf162(wc[j]), sn = as_bf162(ws[j]);
+                pk[4 * jj + j] = as_u32(__hsub2_rn(__hmul2_rn(x0, cs), __hmul2_rn(x1, sn)));
+                pk[32 + 4 * jj + j] = as_u32(__hadd2_rn(__hmul2_rn(x1, cs), __hmul2_rn(x0, sn)));
             }
         }
     }
