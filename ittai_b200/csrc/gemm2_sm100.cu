@@ -19,16 +19,37 @@ namespace ittai {
 __device__ __forceinline__ __nv_bfloat162 as_bf162(uint32_t u) { __nv_bfloat162 v; memcpy(&v, &u, 4); return v; }
 __device__ __forceinline__ uint32_t as_u32(__nv_bfloat162 v) { uint32_t u; memcpy(&u, &v, 4); return u; }
 
+// Both warps of a lane quarter (64 threads) meet; true in both if either passes true.
+__device__ __forceinline__ bool pair_vote(int q, bool v) {
+    uint32_t r;
+    asm volatile("{\n.reg .pred p, o;\nsetp.ne.u32 p, %1, 0;\nbarrier.cta.red.or.pred o, %2, 64, p;\nselp.u32 %0, 1, 0, o;\n}\n" : "=r"(r) : "r"((uint32_t)v), "r"(1 + q) : "memory");
+    return r != 0;
+}
+// The cos | sin rows (256 bytes) of the 32 tokens of a lane quarter, fetched while the accumulator is still being filled: the
+// quarter's two warps (two heads of the same tokens) bring 16 rows each into their staging tiles, two whole rows per load
+// instruction, 16-byte pieces XOR-swizzled by the row.  Row-per-thread loads of both heads were 64 pieces of 32 different lines
+// each per warp, out of the L2 that feeds the main loop: 131 -> 117 us at 16384 tokens, 273 -> 236 at 32768.
+__device__ __forceinline__ void stage_rope_rows(const GemmArgs& g, unsigned char* so, int row0, int cq, int lane) {
+    const int t = row0 + 16 * cq + (lane & 15);
+    const int p = t < g.M ? g.rope.pos[t] : 0;
+    const uint4* table = reinterpret_cast<const uint4*>(g.rope.rope);
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+        const int rr = 2 * i + (lane >> 4);
+        const uint4 v = table[(size_t)__shfl_sync(0xffffffffu, p, rr) * (ITTAI_Q3_HD / 8) + (lane & 15)];
+        *reinterpret_cast<uint4*>(so + rr * 256 + (((lane & 15) ^ rr) << 4)) = v;
+    }
+}
+
 // ITTAI_EPI_QKROPE: one warp = 32 tokens x one head (its 128 accumulator columns).  The thread that owns a token's row
 // rounds the 128 values to bf16 (the Linear output), and for q / k heads applies the head RMSNorm and the half-split
 // rotary embedding with the rounding steps of the eager modules (the arithmetic of qk_rope_scatter_kernel); q goes
 // to the output matrix through the staging tile and a TMA store, k and v go to their cache rows through the staging
 // tile with four lanes per 64-byte row piece (whole sectors), each lane having looked up the rows it stores.
 __device__ __forceinline__ void epilogue_qkrope(const GemmArgs& g, const CUtensorMap* tm_out, uint32_t t_addr, unsigned char* so,
-                                                const uint32_t* sgain, uint32_t& cc, int row0, int col0, int lane, float row_scale) {
+                                                const unsigned char* rope_rows, const uint32_t* sgain, uint32_t& cc, int row0, int col0, int lane, float row_scale) {
     constexpr int HD = ITTAI_Q3_HD, NKV = ITTAI_Q3_NKV;
-    const int head = col0 / HD, t = row0 + lane;
-    const bool valid = t < g.M;
+    const int head = col0 / HD;
     uint32_t pk[64];
 #pragma unroll
     for (int ch = 0; ch < 4; ++ch) {
@@ -43,13 +64,13 @@ __device__ __forceinline__ void epilogue_qkrope(const GemmArgs& g, const CUtenso
 #pragma unroll
         for (int i = 0; i < 64; ++i) { const float lo = bf_lo(pk[i]), hi = bf_hi(pk[i]); s0 = fmaf(lo, lo, s0); s1 = fmaf(hi, hi, s1); }
         const float rstd = 1.0f / sqrtf((s0 + s1) * (1.0f / HD) + g.rope.eps);
-        const bf16* rp = reinterpret_cast<const bf16*>(g.rope.rope) + (size_t)(valid ? g.rope.pos[t] : 0) * HD;
+        const unsigned char* rp = rope_rows + (lane & 15) * 256;
         // Only x * rstd is an fp32 product; every later step is a product or a sum of two bf16 values rounded to bf16, which is
         // one packed instruction for two elements (the _rn forms: never contracted into an FMA).  Through fp32 and back each step was a conversion per element, ten per
         // pair on a pipe of 16 lanes per SM: 10 k cycles of a tile's 14 k (main loop: 8 k).
 #pragma unroll
         for (int jj = 0; jj < 8; ++jj) {                  // elements 8jj .. 8jj+7 and their partners 64 + the same
-            const uint4 cw = *reinterpret_cast<const uint4*>(rp + 8 * jj), sw = *reinterpret_cast<const uint4*>(rp + HD / 2 + 8 * jj);
+            const uint4 cw = *reinterpret_cast<const uint4*>(rp + ((jj ^ (lane & 15)) << 4)), sw = *reinterpret_cast<const uint4*>(rp + (((jj + 8) ^ (lane & 15)) << 4));
             const uint4 ga = *reinterpret_cast<const uint4*>(sgain + 4 * jj), gb = *reinterpret_cast<const uint4*>(sgain + 32 + 4 * jj);
             const uint32_t wc[4] = {cw.x, cw.y, cw.z, cw.w}, ws[4] = {sw.x, sw.y, sw.z, sw.w};
             const uint32_t wga[4] = {ga.x, ga.y, ga.z, ga.w}, wgb[4] = {gb.x, gb.y, gb.z, gb.w};
@@ -63,6 +84,7 @@ __device__ __forceinline__ void epilogue_qkrope(const GemmArgs& g, const CUtenso
                 pk[32 + 4 * jj + j] = as_u32(__hadd2_rn(__hmul2_rn(x1, cs), __hmul2_rn(x0, sn)));
             }
         }
+        pair_vote((threadIdx.x >> 5) & 3, false);         // both warps are done with the rows: their staging tiles take outputs again
     }
     const int swz = (lane >> 1) & 3;
     // cache rows of the four tokens this lane stores pieces of (k / v heads)
@@ -242,6 +264,14 @@ gemm2_bf16_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constan
             if (g.epi == ITTAI_EPI_QKROPE && col0 < ITTAI_Q3_DQ + ITTAI_Q3_DKV && lane < 16)   // this head's norm gain, 128 bf16
                 *reinterpret_cast<uint4*>(sbias + 4 * lane) = *reinterpret_cast<const uint4*>(reinterpret_cast<const bf16*>(col0 < ITTAI_Q3_DQ ? g.rope.qn : g.rope.kn) + 8 * lane);
             __syncwarp();
+            // (the two warps of a pair leave the loop together: each meeting carries a vote)
+            const bool rotate = g.epi == ITTAI_EPI_QKROPE && col0 < ITTAI_Q3_DQ + ITTAI_Q3_DKV;
+            if (rotate) {
+                if (lane == 0) tma_store_wait_read<0>();
+                __syncwarp();
+                if (pair_vote(q, *abort_flag != 0)) break;
+                stage_rope_rows(g, so, row0, cq, lane);
+            }
             bool ok = true;
             {
                 uint32_t spins = 0;
@@ -249,11 +279,13 @@ gemm2_bf16_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constan
                     if (((++spins) & 255u) == 0u && (*abort_flag || spins >= kSpin2)) { ok = false; break; }
                 }
             }
+            __syncwarp();
+            if (rotate && pair_vote(q, !ok)) ok = false;
             if (!ok) { *abort_flag = 1; break; }
             tc_fence_after();
             if (g.epi == ITTAI_EPI_QKROPE) {
                 epilogue_qkrope(g, &tm_out, tmem_base + ((uint32_t)(q * 32) << 16) + (uint32_t)(buf * PN + kEpiCols * cq), so,
-                                reinterpret_cast<const uint32_t*>(sbias), cc, row0, col0, lane, rstd);
+                                sout + ((ew & 3) + 4 * (lane >> 4)) * kStageOut, reinterpret_cast<const uint32_t*>(sbias), cc, row0, col0, lane, rstd);
             } else
 #pragma unroll 1
             for (uint32_t ch = 0; ch < kChunks && ok; ++ch, ++cc) {
