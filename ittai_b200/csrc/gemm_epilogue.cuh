@@ -119,21 +119,21 @@ __device__ __forceinline__ void epilogue_pack(const GemmArgs& g, const uint32_t 
     }
     if (g.epi == ITTAI_EPI_SWIGLU) {
         // adjacent columns are (gate, up): act = bf16(bf16(silu(bf16 gate)) * bf16 up), silu(x) = x / (1 + 2^(-x log2 e)) with
-        // the hardware exponential and reciprocal (their error is far below the bf16 rounding of the result); the
-        // roundings of the Linear outputs run on the integer pipe
+        // the hardware exponential and reciprocal (their error is far below the bf16 rounding of the result).  A pair is
+        // rounded by one conversion, and the last product, of two bf16 values, by one packed multiply for two outputs
 #pragma unroll
         for (int i = 0; i < 16; i += 2) {
-            float gt[2], up[2], sl[2];
+            const uint32_t p0 = pack_bf16x2(v[i].x, v[i].y), p1 = pack_bf16x2(v[i + 1].x, v[i + 1].y);
+            const float gt[2] = {bf_lo(p0), bf_lo(p1)};
+            float sl[2];
 #pragma unroll
             for (int h = 0; h < 2; ++h) {
-                gt[h] = __uint_as_float(bf16r_bits(__float_as_uint(v[i + h].x)));
-                up[h] = __uint_as_float(bf16r_bits(__float_as_uint(v[i + h].y)));
                 float e, rc;
                 asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(e) : "f"(gt[h] * -1.4426950408889634f));
                 asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(rc) : "f"(1.0f + e));
-                sl[h] = __uint_as_float(bf16r_bits(__float_as_uint(gt[h] * rc)));
+                sl[h] = gt[h] * rc;
             }
-            o[i / 2] = pack_bf16x2(sl[0] * up[0], sl[1] * up[1]);
+            asm("mul.rn.bf16x2 %0, %1, %2;" : "=r"(o[i / 2]) : "r"(pack_bf16x2(sl[0], sl[1])), "r"(__byte_perm(p0, p1, 0x7632)));
         }
         return;
     }

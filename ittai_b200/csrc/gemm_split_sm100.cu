@@ -19,7 +19,7 @@
 //   plain shuffles.
 //
 // The tensor memory is allocated BEFORE launch_dependents: a later kernel that shares the SM can then never hold columns
-// this one still waits for (three such CTAs, or two and an attention CTA of the same size, fit an SM's 512 columns).
+// this one still waits for (an SM holds two such CTAs, or one and an attention CTA of 256 columns, of its 512).
 // Waits are bounded as in the other GEMM kernels.
 #include <cuda.h>
 
