@@ -313,7 +313,7 @@ def main():
             ev[k][0].record()
             ids_seen.append(dec.decode(DECODE, check=False))
             ev[k][1].record()
-            launches += 1
+            launches += DECODE * dec.kernels_per_token
         t1.record()
         barrier()
     dec.check_status()
@@ -337,7 +337,7 @@ def main():
         dec.next_id.copy_(host_in, non_blocking=True)
         out = dec.decode(DECODE, check=False)
         host_out.copy_(out, non_blocking=True)
-        launches += 1
+        launches += DECODE * dec.kernels_per_token
     e1.record()
     barrier()
     dec.check_status()
@@ -374,7 +374,7 @@ def main():
                          "mean_kernel": kern_ms_avg * 1e3 / DECODE},
         "roofline": {"bound": "hbm", "achieved": achieved, "peak": peaks["hbm_gbs"], "unit": "GB/s",
                      "frac": achieved / peaks["hbm_gbs"], "traffic": ncu_tok * DECODE / 1e9 if ncu_tok else None,
-                     "traffic_unit": f"GB per launch (ncu dram read+write of an 8-token launch at commit {ncu_commit}, scaled by tokens)",
+                     "traffic_unit": f"GB per step (ncu dram read+write of 8 tokens in the persistent decode kernel at commit {ncu_commit}, which streams the same weights and cache rows, scaled by tokens)",
                      "peak_kind": peak_kind,
                      "frac_of_nominal_8TBs": achieved / 8000.0, "bytes_per_token": mean_bytes},
         "e2e": {"value": toks / (e2e_ms / 1e3), "unit": UNIT, "h2d_bytes_per_step": 4, "d2h_bytes_per_step": 4 * DECODE},

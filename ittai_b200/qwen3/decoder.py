@@ -110,6 +110,7 @@ class Qwen3Decoder:
         _C.check(self.lib.ittai_qwen3_chain_create(C.byref(plan)))
         self._plan = plan
         weakref.finalize(self, self.lib.ittai_qwen3_chain_destroy, plan)
+        self.kernels_per_token = 5 * self.L + 2      # QKV, attention, O-proj, gate/up, down per layer; head; finish
 
     # ---- plumbing -------------------------------------------------------------------------------
     def _params(self, n_steps, n_forced, forced, out_ids, step_ns, write_logits=True) -> _C.Qwen3Decode:
