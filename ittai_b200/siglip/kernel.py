@@ -284,8 +284,8 @@ class Engine:
                                                  self.pos.stride(0), self.seqs.data_ptr(), self.pool_seqs.data_ptr(), ops._stream(self.pos)))
 
     def _run(self, n):
-        """The forward over the first ``n`` images of the buffers.  The full batch is captured at its first use; a part runs as
-        plain launches the first time its size is seen and is captured the second time."""
+        """The forward over the first ``n`` images of the buffers.  Plain launches the first time a size is seen (the very
+        first also reads the status words), a CUDA graph from the second time on."""
         graph = self._graphs.get(n)
         if graph is None and not self._checked:
             self.status.zero_()
@@ -296,10 +296,9 @@ class Engine:
             torch.cuda.current_stream().wait_stream(s)
             ops.check_status(self.status)
             self._checked = True
-            if n != self.B:
-                self._seen.add(n)
-                return
-        if graph is None and self.use_graph and (n == self.B or n in self._seen):
+            self._seen.add(n)
+            return
+        if graph is None and self.use_graph and n in self._seen:
             if len(self._graphs) > self.PARTS:
                 self._graphs.pop(next(k for k in self._graphs if k != self.B))
             graph = torch.cuda.CUDAGraph()
