@@ -288,7 +288,9 @@ typedef struct IttaiAttention {
      * form only (q_head = k_head = v_head = 80). */
     int32_t q_rows_total;  /* rows of the matrix behind q (every sequence's q_row0 + q rows lies inside) */
     int32_t kv_rows_total; /* rows of the matrices behind k and v */
-    int32_t reserved0;
+    int32_t seqs_ready;    /* 1: `seqs` was complete before the first kernel of the run of dependent launches in front of this call
+                              started (a copy or the host wrote it), so that it may be read before those kernels have ended;
+                              0: always right */
     uint32_t* status;      /* [ITTAI_STATUS_WORDS] device words, or NULL */
 } IttaiAttention;
 int ittai_attention_launch(const IttaiAttention* a, void* stream);
@@ -313,7 +315,8 @@ typedef struct IttaiQwen3Prefill {
     const void *wqkv_f, *wgu_f; /* both or neither: the weights with the norm gains folded in along K; the norms then run inside the
                               GEMMs from T > 128 on (layer 0's first norm reads the embedding rows and stays a pass) */
     const int32_t *ids, *pos, *seq, *slot;  /* [T] device */
-    const int32_t* seqs;   /* [n_seqs][4] device, as in IttaiAttention */
+    const int32_t* seqs;   /* [n_seqs][4] device, as in IttaiAttention with seqs_ready = 1: written by a copy, not by a kernel that
+                              this library queued just before */
     void *kcache, *vcache; /* layer 0's store */
     int64_t kv_layer;      /* elements from one layer's store to the next (0: one store reused by every layer) */
     int64_t k_row, k_head, k_seq;  /* strides of the store, elements */

@@ -76,7 +76,7 @@ class Attention(C.Structure):
         ("seqs", C.c_void_p),
         ("n_seqs", C.c_int32), ("n_heads", C.c_int32), ("group", C.c_int32), ("head_dim", C.c_int32),
         ("causal", C.c_int32), ("max_q_len", C.c_int32), ("max_kv_len", C.c_int32), ("q_rows_total", C.c_int32),
-        ("kv_rows_total", C.c_int32), ("reserved0", C.c_int32), ("status", C.c_void_p),
+        ("kv_rows_total", C.c_int32), ("seqs_ready", C.c_int32), ("status", C.c_void_p),
     ]
 
 

@@ -40,7 +40,7 @@ struct AttnFaArgs {
     const int4* seqs;
     bf16* o;
     long long o_row, o_head;
-    int group, causal;
+    int group, causal, seqs_ready;
     int k_seq_rows, k_head_rows;             // cache layout: strides in rows of 128 elements
     int k_head_cols;                         // packed layout (heads side by side in a row, sequences by their row offsets): HDIM, else 0
     float scale_log2;
@@ -91,7 +91,7 @@ __device__ __forceinline__ int4 fa_answer(const void* answer) {
 struct FaTile { int head, r0, q_len, kv_len, n_blk, q_row, q_col, kv_row, kv_col; };
 template <int HDIM>
 __device__ __forceinline__ FaTile fa_tile(const AttnFaArgs& a, int x, int y, int z) {
-    const int4 sinfo = a.seqs[y];                          // written by the host long before: safe ahead of pdl_wait
+    const int4 sinfo = a.seqs[y];
     FaTile t;
     t.head = x; t.r0 = ((int)gridDim.z - 1 - z) * kFaBlk; t.q_len = sinfo.y; t.kv_len = sinfo.w;
     // causal: query r sees keys <= r + (kv_len - q_len)
@@ -131,6 +131,10 @@ __global__ void __launch_bounds__(kFaThreads, 2)
 attn_fa_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUtensorMap tm_k,
                const __grid_constant__ CUtensorMap tm_v, const AttnFaArgs a) {
     pdl_trigger();
+    // The first tile's record is read here, ahead of the kernels that may still be running, only where the caller says that
+    // none of them writes it.  A kernel of the same run of dependent launches may (position rows of variable-resolution
+    // images): every launch in between lets its successors start on entry, so nothing but the wait orders the two.
+    if (!a.seqs_ready) pdl_wait();
     // Grid (heads, sequences, query tiles) with the tiles in descending order: CTAs are handed out in index order, so the
     // causal tiles that walk the most key blocks start first and the last ones are short.
     const FaTile first = fa_tile<HDIM>(a, blockIdx.x, blockIdx.y, blockIdx.z);
@@ -488,7 +492,7 @@ static int attn_fa_launch_t(const IttaiAttention* p, cudaStream_t st) {
     a.seqs = reinterpret_cast<const int4*>(p->seqs);
     a.o = reinterpret_cast<bf16*>(p->o);
     a.o_row = p->o_row; a.o_head = p->o_head;
-    a.group = p->group; a.causal = p->causal;
+    a.group = p->group; a.causal = p->causal; a.seqs_ready = p->seqs_ready;
     a.k_seq_rows = packed ? 0 : (int)(p->k_seq / 128); a.k_head_rows = packed ? 0 : (int)(p->k_head / 128);
     a.k_head_cols = packed ? HDIM : 0;
     a.scale_log2 = 1.4426950408889634f / sqrtf((float)HDIM);

@@ -69,7 +69,7 @@ static int prefill_launch(const IttaiQwen3Prefill* p, void* st) {
         a.q_row = DQKV; a.q_head = HD; a.o_row = DQ; a.o_head = HD;
         a.k_row = a.v_row = p->k_row; a.k_head = a.v_head = p->k_head; a.k_seq = a.v_seq = p->k_seq;
         a.seqs = p->seqs; a.n_seqs = p->n_seqs; a.n_heads = NH; a.group = NH / NKV; a.head_dim = HD; a.causal = 1; a.max_q_len = p->max_q_len;
-        a.q_rows_total = T; a.kv_rows_total = (int32_t)p->kv_rows_total; a.status = p->status;
+        a.q_rows_total = T; a.kv_rows_total = (int32_t)p->kv_rows_total; a.status = p->status; a.seqs_ready = 1;
         if (rc == ITTAI_OK) rc = ittai_attention_launch(&a, st);
         gemm(p->attn, at(p->wo, (size_t)l * D * DQ), p->h, D, DQ, ITTAI_EPI_NONE, p->h, false, fold || normed, nullptr);
         if (!fold && !normed) norm(g2);

@@ -114,13 +114,14 @@ def fold_layernorm(w: torch.Tensor, bias: torch.Tensor | None, gain: torch.Tenso
 
 def attention(q, k, v, o, seqs: torch.Tensor, *, n_heads: int, group: int, head_dim: int, causal: bool, max_q_len: int,
               q_strides, k_strides, v_strides, o_strides, max_kv_len: int = 0, q_rows_total: int = 0, kv_rows_total: int = 0,
-              status: torch.Tensor | None = None) -> None:
+              status: torch.Tensor | None = None, seqs_ready: bool = False) -> None:
     """Flash attention over sequences described by ``seqs`` (int32 [n, 4] device: q row0, q rows, kv row0, kv rows).
 
     ``q_strides`` = (row, head), ``k_strides`` / ``v_strides`` = (row, head, seq), ``o_strides`` = (row, head), in elements;
     q, k, v, o are any bf16 tensors whose ``data_ptr`` is the origin those strides refer to.  ``q_rows_total``,
     ``kv_rows_total`` (rows of the matrices behind q and k/v) and ``status`` enable the tensor-memory kernel for short
-    dense sequences; it reports a timed-out wait through ``status`` (see ``check_status``)."""
+    dense sequences; it reports a timed-out wait through ``status`` (see ``check_status``).  ``seqs_ready``: no kernel queued
+    just before writes ``seqs`` (a copy or an earlier stream of work did), so that it may be read ahead of them."""
     a = _C.Attention()
     a.q, a.k, a.v, a.o = q.data_ptr(), k.data_ptr(), v.data_ptr(), o.data_ptr()
     a.q_row, a.q_head = q_strides
@@ -131,6 +132,7 @@ def attention(q, k, v, o, seqs: torch.Tensor, *, n_heads: int, group: int, head_
     a.n_seqs, a.n_heads, a.group, a.head_dim, a.causal, a.max_q_len = seqs.shape[0], n_heads, group, head_dim, int(causal), max_q_len
     a.max_kv_len, a.q_rows_total, a.kv_rows_total = max_kv_len, q_rows_total, kv_rows_total
     a.status = status.data_ptr() if status is not None else None
+    a.seqs_ready = int(seqs_ready)
     _C.check(_C.lib().ittai_attention_launch(C.byref(a), _stream(q)))
 
 

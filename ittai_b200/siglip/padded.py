@@ -151,7 +151,7 @@ class PaddedEngine:
             he, He = self.hde, H * self.hde
             ops.attention(qkv_b, qkv_b[:, He:], qkv_b[:, 2 * He:], attn, seqs, n_heads=H, group=1, head_dim=he, causal=False, max_q_len=S,
                           q_strides=(3 * He, he), k_strides=(3 * He, he, 0), v_strides=(3 * He, he, 0), o_strides=(He, he), max_kv_len=S,
-                          q_rows_total=self.M, kv_rows_total=self.M, status=st)
+                          q_rows_total=self.M, kv_rows_total=self.M, status=st, seqs_ready=self.conv)   # else the position kernel writes them
 
         if self.fold_ln:
             sw = dict(static_w=not self.chain)                  # a chained GEMM takes no such flag

@@ -93,3 +93,26 @@ def test_packed_attention_with_80_columns_per_head(lens):
     from ittai_b200 import _C
     with pytest.raises(_C.IttaiError, match="head_dim 80"):
         ops.attention(qkv, qkv[:, H * hd:], qkv[:, 2 * H * hd:], out, seqs, max_q_len=64, **kw)
+
+
+@gpu
+@pytest.mark.parametrize("batch", [1, 3])
+def test_key_counts_of_the_batch_before_are_not_seen(batch):
+    """A padded variable-resolution tower on plain launches, the host far ahead: the key counts that the position kernel writes
+    alternate from batch to batch, and the attention kernel, which may start before that kernel has ended, must see its own
+    batch's.  Every batch gives, bit for bit, what it gives alone on an idle device."""
+    from ittai_b200.siglip.kernel import Engine
+    eng = Engine(hf.build_hf_so400m(True, n_layers=2, device="cuda"), batch, graph=False)
+    assert eng.hde == 80 and not eng.chain
+    inputs = []
+    for i, shapes in enumerate([[(16, 16), (12, 20), (9, 21)], [(1, 1), (3, 5), (2, 2)], [(10, 25), (1, 200), (16, 9)]]):
+        inp = hf.naflex_inputs(shapes[:batch], seed=20 + i)
+        inputs.append(dict(inp, pixel_values=inp["pixel_values"].cuda()))
+    want = []
+    for inp in inputs:
+        want.append(eng.forward(inp).clone())
+        torch.cuda.synchronize()
+    got = [eng.forward(inputs[i % 3]).clone() for i in range(48)]
+    eng.check()
+    for i, t in enumerate(got):
+        assert torch.equal(t, want[i % 3]), i
