@@ -174,8 +174,8 @@ int ittai_qwen3_phase_launch(const IttaiQwen3Decode* p, int phase, int layer, vo
  * results (the arithmetic and its rounding points are those of ittai_qwen3_decode_launch; sums run in another order).
  * `plan` owns the graphs, which are captured at the first token that needs each of them (a graph per power-of-two split
  * of the attention, 2 ms each) and again when a pointer or size of *p other than n_steps, n_forced, forced, out_ids,
- * step_ns changes.  `max_len`: an upper bound of pos[b] over the sequences (it picks the split; results do not depend on
- * it).  p->flags, spin_limit and phase_clk are not used.  An id or position out of range ends in ITTAI_ST_BAD_TOKEN with
+ * step_ns changes.  `max_len`: an upper bound of pos[b] over the sequences.  It picks the cluster size of a launch; a
+ * sequence's results follow from its own length and `batch` alone, bit for bit.  p->flags, spin_limit and phase_clk are not used.  An id or position out of range ends in ITTAI_ST_BAD_TOKEN with
  * `pos` unchanged.  A stream that is being captured gets the kernels themselves.  Calls on one plan are serialised. */
 int ittai_qwen3_chain_create(void** plan);
 int ittai_qwen3_chain_run(void* plan, const IttaiQwen3Decode* p, int32_t max_len, void* stream);

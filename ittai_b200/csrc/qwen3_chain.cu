@@ -485,8 +485,8 @@ __global__ void __launch_bounds__(32 * NB) finish_kernel(const TokenArgs a) {
 }
 
 // ---- attention ------------------------------------------------------------------------------------------------------------
-// One cluster of CS CTAs per (sequence, kv head); rank r takes the r-th piece of the cached positions, rank 0 also the new
-// one (norm, rotation, append, and its own score).  Three groups of two compute warps take turns on 32-position tiles, a
+// One cluster of CS CTAs per (sequence, kv head); rank r takes the r-th piece of the cached positions (if the sequence is long
+// enough for so many, see split_log2), rank 0 also the new one (norm, rotation, append, and its own score).  Three groups of two compute warps take turns on 32-position tiles, a
 // warp 16 positions of each with its own softmax; a seventh warp feeds a ring of six 16 KB tiles (two CTAs per SM).  A
 // warp's 16 positions are 16 MMAs: scores with the keys as A (M = positions) and the two query heads as N columns, P V with
 // V^T as A (ldmatrix.trans on the swizzled tile) and P as B, its high parts in columns 0-1, its low parts in columns 2-3.
@@ -544,6 +544,23 @@ __device__ __forceinline__ void st_cluster_f32(float* p, int rank, float v) {
     asm volatile("st.shared::cluster.f32 [%0], %1;" ::"r"(a), "f"(v) : "memory");
 }
 
+// log2 of the pieces that the cache of a sequence with `len` positions is cut into, one CTA each.  Measured over all splits and
+// lengths 30 to 8100 (us per step, best split first): 128 CTAs in all are best nearly everywhere (batch 4, 8100: 4 CTAs 1019,
+// 8 1095, 2 1346; batch 2, 8100: 8 CTAs 733, 16 852), because the next projection then still finds room.  Exceptions: a few
+// positions need no split (batch 1, 30: 425, else 428-443), clusters of 16 pay their barrier only from 1200 positions on
+// (batch 1, 800: 8 CTAs 445, 16 451; 3000: 501 and 478), and the longest caches at batch 8 want two CTAs per SM (8100: 4 CTAs
+// 1577, 2 1623; 500: 604 and 592).
+// A sequence's pieces follow from its OWN length, so that its sums are taken in the same order whatever the others of the
+// batch hold; the clusters of a launch have the size that the longest needs (the rule does not fall with `len`), and in those of
+// a shorter sequence the ranks past its pieces add exact zeros.
+__host__ __device__ constexpr int split_log2(int batch, int len) {
+    if (batch == 4) return 2;
+    if (len <= 48) return 0;
+    if (batch == 1) return len <= 1200 ? 3 : 4;
+    if (batch == 2) return len <= 400 ? 2 : 3;
+    return len <= 700 ? 1 : 2;
+}
+
 template <int CS>
 __global__ void __launch_bounds__(kAttnThreads, 2) attn_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constant__ CUtensorMap tm_v, const AttnChainArgs a) {
     extern __shared__ __align__(1024) unsigned char ring_raw[];
@@ -571,7 +588,9 @@ __global__ void __launch_bounds__(kAttnThreads, 2) attn_kernel(const __grid_cons
     // (late_trigger), so they may be read ahead of the wait.
     const int pos = (int)ld_relaxed(reinterpret_cast<const uint32_t*>(&a.st->cur_pos[b]));
     const int n_old = pos < 0 ? 0 : pos;
-    const int chunk = ((n_old + CS - 1) / CS + 15) & ~15;
+    constexpr int kCsLog2 = CS == 16 ? 4 : CS == 8 ? 3 : CS == 4 ? 2 : CS == 2 ? 1 : 0;
+    const int own = split_log2(a.batch, n_old), lg = own < kCsLog2 ? own : kCsLog2;
+    const int chunk = (((n_old + (1 << lg) - 1) >> lg) + 15) & ~15;
     const int p0 = rank * chunk < n_old ? rank * chunk : n_old, p1 = p0 + chunk < n_old ? p0 + chunk : n_old;
     const int n_tiles = (p1 - p0 + kTilePos - 1) / kTilePos;
     const int row_base = (int)(head_row * (size_t)a.kv_cap) + p0;
@@ -914,19 +933,6 @@ static void enqueue_begin(const Plan& pl, const IttaiQwen3Decode& c, cudaStream_
     }
 }
 
-// log2 of the CTAs per (sequence, kv head) at `len` cached positions.  Measured over all splits and lengths 30 to 8100 (us per
-// step, best split first): 128 CTAs in all are best nearly everywhere (batch 4, 8100: 4 CTAs 1019, 8 1095, 2 1346; batch 2,
-// 8100: 8 CTAs 733, 16 852), because the next projection then still finds room.  Exceptions: a few positions need no split (batch 1, 30:
-// 425, else 428-443), clusters of 16 pay their barrier only from 1200 positions on (batch 1, 800: 8 CTAs 445, 16 451; 3000:
-// 501 and 478), and the longest caches at batch 8 want two CTAs per SM (8100: 4 CTAs 1577, 2 1623; 500: 604 and 592).
-static int cluster_log2(int batch, int len) {
-    if (batch == 4) return 2;
-    if (len <= 48) return 0;
-    if (batch == 1) return len <= 1200 ? 3 : 4;
-    if (batch == 2) return len <= 400 ? 2 : 3;
-    return len <= 700 ? 1 : 2;
-}
-
 static void drop_graphs(Plan* pl) {
     for (auto& row : pl->exec)
         for (cudaGraphExec_t& x : row)
@@ -1031,7 +1037,7 @@ extern "C" int ittai_qwen3_chain_run(void* plan, const IttaiQwen3Decode* p, int3
     chain::enqueue_begin(*pl, *p, st);
     for (int i = 0; i < p->n_steps; ++i) {
         const bool head = i >= p->n_forced - 1;
-        const int lg = chain::cluster_log2(p->batch, max_len + i);
+        const int lg = chain::split_log2(p->batch, max_len + i);
         if (cap != cudaStreamCaptureStatusNone) {      // a graph launch cannot be captured: the kernels themselves can
             e = chain::enqueue_token(*pl, 1 << lg, head, st);
         } else {

@@ -1,0 +1,55 @@
+"""Properties of a call of the decode chain (``csrc/qwen3_chain.cu``): what a sequence sees of its neighbours, what is left behind by
+a call that fails, calls on several streams (GPU)."""
+import pytest
+import torch
+
+from oracle import qwen3_hf as hf
+
+gpu = pytest.mark.gpu
+
+
+@gpu
+@pytest.mark.parametrize("batch", [2, 4, 8])
+@pytest.mark.parametrize("length", [0, 20, 47, 399, 450, 699])
+def test_a_sequence_does_not_depend_on_its_neighbours(tiny_hf, batch, length):
+    """Ids, logits and cache rows of a sequence are the same, bit for bit, whatever lengths the others have, on both sides of
+    every line of the split rule; the four steps cross the lines."""
+    from ittai_b200.qwen3 import Qwen3Decoder
+    model, dims = tiny_hf
+    g = torch.Generator().manual_seed(batch + length)
+    d = Qwen3Decoder(model, max_batch=batch, kv_capacity=1200)
+    kv = [(torch.randn(d.kcache.shape, generator=g) * s).to(torch.bfloat16) for s in (1.0, 0.5)]
+    ids = torch.randint(0, dims.vocab, (batch,), generator=g, dtype=torch.int32)
+
+    def run(other):
+        for c, t in zip((d.kcache, d.vcache), kv):
+            c.copy_(t)
+        d.reset()
+        for b in range(batch):
+            d.set_length(b, length if b == 0 else other)
+        d.next_id.copy_(ids)
+        out = d.decode(4)[0].clone()
+        return out, d.logits[0].clone(), *(c[:, 0, :, length:length + 4].clone() for c in (d.kcache, d.vcache))
+
+    want = run(1)
+    for other in (46, 399, 699, 1100):
+        for got, ref in zip(run(other), want):
+            assert torch.equal(got, ref), (other, (got.float() - ref.float()).abs().max())
+
+
+@gpu
+@pytest.mark.parametrize("slots", [2, 8])
+def test_served_tokens_do_not_depend_on_the_other_requests(tiny_hf, slots):
+    """Short requests beside ones past 400 and 700 positions give the tokens of their solo runs."""
+    from ittai_b200.qwen3 import DecodeServer, Qwen3Decoder
+    model, dims = tiny_hf
+    d = Qwen3Decoder(model, max_batch=slots, kv_capacity=1024)
+    prompts = [hf.prompt_ids(n, seed=170 + i, vocab=dims.vocab).tolist() for i, n in enumerate((20, 720, 45, 410, 33, 90, 12, 500))]
+    budgets = [24, 9, 20, 12, 17, 8, 30, 6]
+    srv = DecodeServer(d, chunk=4)
+    rids = [srv.submit(p, m) for p, m in zip(prompts, budgets)]
+    out = dict(srv.run())
+    for rid, p, m in zip(rids, prompts, budgets):
+        solo = DecodeServer(d, chunk=4)
+        r = solo.submit(p, m)
+        assert solo.run()[r] == out[rid], f"request {rid} (prompt {len(p)}, {m} tokens) depends on its neighbours"
