@@ -43,7 +43,9 @@ extern "C" {
 
 /* IttaiQwen3Decode.flags */
 #define ITTAI_F_TEST_DROP_CTA 2 /* test hook: CTA 0 leaves at once, so the words it would publish never arrive and
-                                  the other CTAs' bounded waits run out and report ITTAI_ST_FLAG_TIMEOUT */
+                                  the other CTAs' bounded waits run out and report ITTAI_ST_FLAG_TIMEOUT; in the decode
+                                  chain CTA 0 of every projection leaves its weight rows out, so that its own wait runs
+                                  out and reports ITTAI_ST_STREAM_TIMEOUT */
 
 enum {
     ITTAI_OK = 0,
@@ -175,8 +177,9 @@ int ittai_qwen3_phase_launch(const IttaiQwen3Decode* p, int phase, int layer, vo
  * `plan` owns the graphs, which are captured at the first token that needs each of them (a graph per power-of-two split
  * of the attention, 2 ms each) and again when a pointer or size of *p other than n_steps, n_forced, forced, out_ids,
  * step_ns changes.  `max_len`: an upper bound of pos[b] over the sequences.  It picks the cluster size of a launch; a
- * sequence's results follow from its own length and `batch` alone, bit for bit.  p->flags, spin_limit and phase_clk are not used.  An id or position out of range ends in ITTAI_ST_BAD_TOKEN with
- * `pos` unchanged.  A stream that is being captured gets the kernels themselves.  Calls on one plan are serialised. */
+ * sequence's results follow from its own length and `batch` alone, bit for bit.  p->phase_clk is not used.  An id or position out of range ends in ITTAI_ST_BAD_TOKEN, a wait that runs out in
+ * ITTAI_ST_STREAM_TIMEOUT: the steps from there on store no id, `next_id` keeps the last good
+ * step's id and `pos` is what it was before the call.  A stream that is being captured gets the kernels themselves.  Calls on one plan are serialised. */
 int ittai_qwen3_chain_create(void** plan);
 int ittai_qwen3_chain_run(void* plan, const IttaiQwen3Decode* p, int32_t max_len, void* stream);
 int ittai_qwen3_chain_destroy(void* plan);

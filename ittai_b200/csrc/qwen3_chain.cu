@@ -150,6 +150,8 @@ struct GemvArgs {
     const unsigned char* ahead;      // O-proj: weights to bring into L2, eight pieces of ahead_bytes per CTA (nullptr: none)
     uint32_t ahead_bytes;
     int late_trigger;       // first kernel of a token: dependents start only once everything before this kernel is complete
+    int drop;               // test hook: CTA 0 leaves its weight rows out, so that its wait runs out
+    uint32_t limit;         // polls before the wait for the weights gives up
 };
 
 // out = epilogue(W x).  ROWS = 32 or 48: 16-row tiles; ROWS = 8: half a tile.  KC K chunks x (16 / KC) tile groups over the 16
@@ -179,7 +181,7 @@ __global__ void __launch_bounds__(kGemvThreads, 2) gemv_kernel(const GemvArgs a)
     const int col = kc * KW + 8 * t;
     if (tid == 0) { mbar_init(&landed, 1); fence_mbar_init(); mbar_expect_tx(&landed, ROWS * K * 2); }
     __syncwarp();
-    if (warp == 0) {
+    if (warp == 0 && !(a.drop && blockIdx.x == 0)) {
         for (int r = lane; r < ROWS; r += 32) bulk_g2s(w_s + r * LD, a.w + (size_t)(row0 + r) * K, K * 2, &landed);
     }
     if (!a.late_trigger) pdl_trigger();
@@ -215,7 +217,7 @@ __global__ void __launch_bounds__(kGemvThreads, 2) gemv_kernel(const GemvArgs a)
     if constexpr (EPI == kResidual) {
         if (tid < 8 * NB) res = ldcg_bf16(a.res + (size_t)(tid >> 3) * D + row0 + (tid & 7));
     }
-    const bool ok = mbar_wait_bounded(&landed, 0, kSpinParked);
+    const bool ok = mbar_wait_bounded(&landed, 0, a.limit);
 #pragma unroll
     for (int n = 0; n < NT; ++n) {
         float d0[4] = {0.f, 0.f, 0.f, 0.f}, d1[4] = {0.f, 0.f, 0.f, 0.f};
@@ -264,7 +266,11 @@ __global__ void __launch_bounds__(kGemvThreads, 2) gemv_kernel(const GemvArgs a)
             a.out[(size_t)b * a.ld_out + row0 + r] = __float2bfloat16_rn(res + bf16r(s));
         }
     }
-    if (!ok && lane == 0 && atomicCAS(&a.status[0], 0u, (uint32_t)ITTAI_ST_STREAM_TIMEOUT) == 0u) { a.status[1] = row0; a.status[2] = blockIdx.x; }
+    if (!ok) {
+        if (lane == 0 && atomicCAS(&a.status[0], 0u, (uint32_t)ITTAI_ST_STREAM_TIMEOUT) == 0u) { a.status[1] = row0; a.status[2] = blockIdx.x; }
+        const long long t0 = clock64();                    // copies still in flight land before the shared memory is handed back
+        while (clock64() - t0 < 2000000) {}
+    }
 }
 
 // ---- lm_head: logits = E bf16(norm(h)), with the arg-max candidates of this CTA's rows ----------------------------------
@@ -282,6 +288,7 @@ struct HeadArgs {
     uint32_t* status;
     int vocab;
     float eps;
+    uint32_t limit;
 };
 constexpr int kHeadRing = 5, kHeadRows = 16, kHeadLd = D * 2 + 64;
 constexpr uint32_t kHeadSmem = kHeadRing * kHeadRows * kHeadLd;
@@ -308,7 +315,7 @@ __global__ void __launch_bounds__(kGemvThreads + 32, 1) head_kernel(const HeadAr
     if (warp == 16) {                    // the feeding warp: one row per lane
         for (int it = 0; it < n_it && !failed; ++it) {
             const int s = it % kHeadRing, r0 = r_lo + it * kHeadRows, n = r_hi - r0 < kHeadRows ? r_hi - r0 : kHeadRows;
-            if (it >= kHeadRing && !mbar_wait_bounded(&empty[s], ((it / kHeadRing) - 1) & 1, kSpinParked)) { failed = 1; break; }
+            if (it >= kHeadRing && !mbar_wait_bounded(&empty[s], ((it / kHeadRing) - 1) & 1, a.limit)) { failed = 1; break; }
             if (lane == 0) mbar_expect_tx(&full[s], (uint32_t)n * D * 2);
             __syncwarp();
             if (lane < n) bulk_g2s(w_s + (s * kHeadRows + lane) * kHeadLd, a.w + (size_t)(r0 + lane) * D, D * 2, &full[s]);
@@ -331,7 +338,7 @@ __global__ void __launch_bounds__(kGemvThreads + 32, 1) head_kernel(const HeadAr
         const int s = it % kHeadRing, buf = it & 1;
         bool ok = true;
         uint32_t spins = 0;
-        while (!mbar_try_wait_parked(&full[s], (it / kHeadRing) & 1)) { if (++spins >= kSpinParked || failed) { ok = false; break; } }
+        while (!mbar_try_wait_parked(&full[s], (it / kHeadRing) & 1)) { if (++spins >= a.limit || failed) { ok = false; break; } }
         if (!ok) failed = 1;
         const unsigned char* wr = w_s + (s * kHeadRows + g) * kHeadLd + col * 2;
         float d0[4] = {0.f, 0.f, 0.f, 0.f}, d1[4] = {0.f, 0.f, 0.f, 0.f};
@@ -429,18 +436,20 @@ __global__ void __launch_bounds__(32 * NB) begin_kernel(const TokenArgs a, int32
 
 // Last kernel of a token, one warp per sequence.  With HEAD: arg-max over the head's candidates, stored as the step's id and
 // fed back.  Without: a forced step whose logits nobody asked for.  Then the next token's row and position; after the last
-// step of the call the cache lengths `pos` advance, unless a step found an id or a position out of range.
+// step of the call the cache lengths `pos` advance, unless a step found an id or a position out of range or a wait of one of its
+// kernels ran out: from there on nothing that was computed is stored as an id, fed back or counted.
 template <int NB, bool HEAD>
 __global__ void __launch_bounds__(32 * NB) finish_kernel(const TokenArgs a) {
     pdl_trigger();
     pdl_wait();
     const int b = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    __shared__ int bad;
+    __shared__ int bad, stopped;
     State* st = a.st;
-    const int step = st->step, n_steps = st->n_steps, abort = st->abort, pos = st->cur_pos[b];
+    const int step = st->step, n_steps = st->n_steps, pos = st->cur_pos[b];
     int32_t* out_ids = st->out_ids;
-    if (threadIdx.x == 0) bad = abort;
+    if (threadIdx.x == 0) bad = stopped = st->abort != 0 || ld_relaxed(a.status) != 0u;
     __syncthreads();
+    const bool abort = stopped != 0;                   // as it was before this kernel reported anything itself
     int id = -1;
     if constexpr (HEAD) {
         float v = -INFINITY;
@@ -513,6 +522,7 @@ struct AttnChainArgs {
     uint32_t* status;
     int layer, batch, kv_cap;
     float eps;
+    uint32_t limit, limit_parked;
 };
 
 __device__ __forceinline__ float ex2f(float x) {
@@ -613,7 +623,7 @@ __global__ void __launch_bounds__(kAttnThreads, 2) attn_kernel(const __grid_cons
         pdl_wait();
         if (lane == 0) {
             for (int it = kRing; it < n_tiles; ++it) {
-                if (!mbar_wait_bounded(&empty[ring_slot(it)], ring_parity(it) ^ 1, kSpinParked)) { failed = 1; break; }
+                if (!mbar_wait_bounded(&empty[ring_slot(it)], ring_parity(it) ^ 1, a.limit_parked)) { failed = 1; break; }
                 issue(it);
             }
         }
@@ -693,7 +703,7 @@ __global__ void __launch_bounds__(kAttnThreads, 2) attn_kernel(const __grid_cons
             const int s = ring_slot(it);
             bool ok = true;
             uint32_t spins = 0;
-            while (!mbar_try_wait(&full[s], ring_parity(it))) { if (++spins >= kSpin || failed) { ok = false; break; } }
+            while (!mbar_try_wait(&full[s], ring_parity(it))) { if (++spins >= a.limit || failed) { ok = false; break; } }
             if (!ok) { failed = 1; break; }
             const int nv = p1 - p0 - it * kTilePos - 16 * w4;  // valid positions of this warp's sixteen
             if (nv > 0) {
@@ -876,14 +886,16 @@ static cudaError_t enqueue_token(const Plan& pl, int cs, bool head, cudaStream_t
     const IttaiQwen3Decode& p = pl.p;
     const Buffers& w = pl.w;
     auto bp = [](const void* q, size_t off = 0) { return reinterpret_cast<const bf16*>(q) + off; };
+    const uint32_t limit = p.spin_limit > 0 ? (uint32_t)p.spin_limit : kSpin, limit_parked = p.spin_limit > 0 ? (uint32_t)p.spin_limit : kSpinParked;
+    const int drop = (p.flags & ITTAI_F_TEST_DROP_CTA) != 0;
     cudaError_t e = cudaSuccess;
     for (int l = 0; l < p.n_layers && e == cudaSuccess; ++l) {
         const size_t kv = (size_t)l * NB * NKV * p.kv_cap * HD;
-        GemvArgs q{bp(p.wqkv, (size_t)l * DQKV * D), w.h, bp(p.ln1, (size_t)l * D), nullptr, w.qkv, DQKV, p.eps, p.status, nullptr, nullptr, nullptr, 0, nullptr, 0, l == 0};
+        GemvArgs q{bp(p.wqkv, (size_t)l * DQKV * D), w.h, bp(p.ln1, (size_t)l * D), nullptr, w.qkv, DQKV, p.eps, p.status, nullptr, nullptr, nullptr, 0, nullptr, 0, l == 0, drop, limit_parked};
         e = launch_pdl(gemv_kernel<NB, D, 32, kPlain>, dim3(DQKV / 32), dim3(kGemvThreads), gemv_smem<D, 32>(), st, 1, q);
         if (e != cudaSuccess) break;
         AttnChainArgs a{w.st, w.qkv, bp(p.qn, (size_t)l * HD), bp(p.kn, (size_t)l * HD), bp(p.rope), reinterpret_cast<bf16*>(p.kcache) + kv,
-                        reinterpret_cast<bf16*>(p.vcache) + kv, w.attn, p.status, l, NB, p.kv_cap, p.eps};
+                        reinterpret_cast<bf16*>(p.vcache) + kv, w.attn, p.status, l, NB, p.kv_cap, p.eps, limit, limit_parked};
         switch (cs) {
             case 1: e = launch_attn<1>(pl, a, st); break;
             case 2: e = launch_attn<2>(pl, a, st); break;
@@ -894,22 +906,22 @@ static cudaError_t enqueue_token(const Plan& pl, int cs, bool head, cudaStream_t
         if (e != cudaSuccess) break;
         // gate/up finds no room on an SM while attention is there: its weights come as far as L2
         GemvArgs o{bp(p.wo, (size_t)l * D * DQ), w.attn, nullptr, w.h, w.hmid, D, p.eps, p.status, nullptr, nullptr, nullptr, 0,
-                   reinterpret_cast<const unsigned char*>(bp(p.wgu, (size_t)l * DGU * D)), DGU * D * 2 / (D / 8) / 8, 0};
+                   reinterpret_cast<const unsigned char*>(bp(p.wgu, (size_t)l * DGU * D)), DGU * D * 2 / (D / 8) / 8, 0, drop, limit_parked};
         e = launch_pdl(gemv_kernel<NB, DQ, 8, kResidual>, dim3(D / 8), dim3(kGemvThreads), gemv_smem<DQ, 8>(), st, 1, o);
         if (e != cudaSuccess) break;
         const bool kv_ahead = l + 1 < p.n_layers;
         const size_t kv1 = kv + (size_t)NB * NKV * p.kv_cap * HD;
         GemvArgs gu{bp(p.wgu, (size_t)l * DGU * D), w.hmid, bp(p.ln2, (size_t)l * D), nullptr, w.act, FF, p.eps, p.status, w.st,
-                    kv_ahead ? reinterpret_cast<const bf16*>(p.kcache) + kv1 : nullptr, reinterpret_cast<const bf16*>(p.vcache) + kv1, p.kv_cap, nullptr, 0, 0};
+                    kv_ahead ? reinterpret_cast<const bf16*>(p.kcache) + kv1 : nullptr, reinterpret_cast<const bf16*>(p.vcache) + kv1, p.kv_cap, nullptr, 0, 0, drop, limit_parked};
         e = launch_pdl(gemv_kernel<NB, D, 48, kSwiglu>, dim3(DGU / 48), dim3(kGemvThreads), gemv_smem<D, 48>(), st, 1, gu);
         if (e != cudaSuccess) break;
-        GemvArgs dn{bp(p.wd, (size_t)l * D * FF), w.act, nullptr, w.hmid, w.h, D, p.eps, p.status, nullptr, nullptr, nullptr, 0, nullptr, 0, 0};
+        GemvArgs dn{bp(p.wd, (size_t)l * D * FF), w.act, nullptr, w.hmid, w.h, D, p.eps, p.status, nullptr, nullptr, nullptr, 0, nullptr, 0, 0, drop, limit_parked};
         e = launch_pdl(gemv_kernel<NB, FF, 8, kResidual>, dim3(D / 8), dim3(kGemvThreads), gemv_smem<FF, 8>(), st, 1, dn);
     }
     if (e != cudaSuccess) return e;
     TokenArgs t{w.st, bp(p.embed), w.h, w.cand_val, w.cand_idx, pl.n_sms, p.pos, p.next_id, p.status, p.vocab, p.kv_cap};
     if (!head) return launch_pdl(finish_kernel<NB, false>, dim3(1), dim3(32 * NB), 0, st, 1, t);
-    HeadArgs h{bp(p.embed), w.h, bp(p.fin_w), p.write_logits ? reinterpret_cast<bf16*>(p.logits) : nullptr, w.cand_val, w.cand_idx, p.status, p.vocab, p.eps};
+    HeadArgs h{bp(p.embed), w.h, bp(p.fin_w), p.write_logits ? reinterpret_cast<bf16*>(p.logits) : nullptr, w.cand_val, w.cand_idx, p.status, p.vocab, p.eps, limit_parked};
     e = launch_pdl(head_kernel<NB>, dim3(pl.n_sms), dim3(kGemvThreads + 32), kHeadSmem, st, 1, h);
     if (e != cudaSuccess) return e;
     return launch_pdl(finish_kernel<NB, true>, dim3(1), dim3(32 * NB), 0, st, 1, t);
@@ -959,6 +971,7 @@ static int bind(Plan* pl, const IttaiQwen3Decode* p) {
 // Whether a graph captured for `a` also serves `b`: everything but the per-call parameters, which travel in State.
 static bool same_binding(const IttaiQwen3Decode& a, const IttaiQwen3Decode& b) {
     return a.n_layers == b.n_layers && a.vocab == b.vocab && a.kv_cap == b.kv_cap && a.batch == b.batch && a.eps == b.eps && a.write_logits == b.write_logits &&
+           a.flags == b.flags && a.spin_limit == b.spin_limit &&
            a.wqkv == b.wqkv && a.wo == b.wo && a.wgu == b.wgu && a.wd == b.wd && a.ln1 == b.ln1 && a.ln2 == b.ln2 && a.qn == b.qn && a.kn == b.kn &&
            a.fin_w == b.fin_w && a.embed == b.embed && a.rope == b.rope && a.kcache == b.kcache && a.vcache == b.vcache && a.pos == b.pos &&
            a.next_id == b.next_id && a.logits == b.logits && a.workspace == b.workspace && a.status == b.status;

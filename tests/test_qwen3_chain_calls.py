@@ -53,3 +53,28 @@ def test_served_tokens_do_not_depend_on_the_other_requests(tiny_hf, slots):
         solo = DecodeServer(d, chunk=4)
         r = solo.submit(p, m)
         assert solo.run()[r] == out[rid], f"request {rid} (prompt {len(p)}, {m} tokens) depends on its neighbours"
+
+
+@gpu
+@pytest.mark.parametrize("batch", [1, 8])
+def test_a_wait_that_runs_out_ends_the_call(tiny_hf, batch):
+    """CTA 0 of every projection leaves its weights out and gives up after a shortened wait: the call reports it, stores no id,
+    and leaves positions and the next input where they were; the next call goes on from there."""
+    import ctypes as C
+    from ittai_b200 import _C
+    from ittai_b200.qwen3 import Qwen3Decoder
+    model, dims = tiny_hf
+    d = Qwen3Decoder(model, max_batch=batch, kv_capacity=64)
+    d.next_id.fill_(7)
+    want = d.decode(6).cpu()
+    d.reset()
+    d.next_id.fill_(7)
+    assert torch.equal(d.decode(2).cpu(), want[:, :2])
+    out = torch.full((3, batch), -7, dtype=torch.int32, device="cuda")
+    p = d._params(3, 0, None, out, None)
+    p.flags, p.spin_limit = _C.F_TEST_DROP_CTA, 64
+    _C.check(d.lib.ittai_qwen3_chain_run(d._plan, C.byref(p), 2, d._stream()))
+    with pytest.raises(_C.IttaiError, match="stream"):
+        d.check_status()
+    assert (out == -7).all() and d.pos.tolist() == d.lengths == [2] * batch
+    assert torch.equal(d.decode(4).cpu(), want[:, 2:])
