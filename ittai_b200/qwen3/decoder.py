@@ -145,6 +145,7 @@ class Qwen3Decoder:
                 _C.decode_status(prefill)
             _C.decode_status(decode)
         except _C.IttaiError:
+            self._status.zero_()             # reported once: a prefill after this one is judged by its own words
             self._unchecked = 0
             self.lengths = self.pos.cpu().tolist()
             raise

@@ -78,3 +78,22 @@ def test_a_wait_that_runs_out_ends_the_call(tiny_hf, batch):
         d.check_status()
     assert (out == -7).all() and d.pos.tolist() == d.lengths == [2] * batch
     assert torch.equal(d.decode(4).cpu(), want[:, 2:])
+
+
+@gpu
+def test_a_reported_failure_is_not_reported_again(tiny_hf):
+    """After a failed decode, prefills that go well are accepted; so is what follows a second failure."""
+    from ittai_b200._C import IttaiError
+    from ittai_b200.qwen3 import Qwen3Decoder
+    model, dims = tiny_hf
+    d = Qwen3Decoder(model, max_batch=1, kv_capacity=256)
+    for _ in range(2):
+        d.next_id.fill_(10 ** 6)
+        with pytest.raises(IttaiError, match="out of range"):
+            d.decode(1)
+        d.reset()
+        d.prefill_cache(hf.prompt_ids(40, seed=1, vocab=dims.vocab))
+        d.prefill_slots({0: [1, 2, 3]})
+        d.prefill_slots({0: [4, 5]})
+        d.check_status()
+        assert d.lengths == d.pos.tolist() == [45]
