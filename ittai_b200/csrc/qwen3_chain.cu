@@ -12,8 +12,10 @@
 //   meet in shared memory, in fixed order.
 // * Attention (attn_kernel): a cluster of CS CTAs per (sequence, kv head) splits the cache; K/V tiles of 32 positions
 //   arrive by TMA (128-byte swizzle), the first six before the wait; scores and P V on mma.sync, the splits meet
-//   through distributed shared memory.  Probabilities enter P V as a high and a low bf16 part in separate N columns (the
-//   columns are idle anyway), so nothing is lost against fp32 probabilities.
+//   through distributed shared memory.  Probabilities enter P V as three bf16 parts in separate N columns (the columns
+//   are idle anyway): 3 x 8 bits are all of an fp32 probability.  With two parts 1.5-3.3e-3 of the outputs were not the 64-bit
+//   result rounded once, with three 0.6-3.6e-4, which is what fp32 sums leave, at the same time per step (batch 1, 4096: 523 us,
+//   519; batch 2, 8000: 727, 730).
 // * finish_kernel: argmax over the head's candidates, token feedback, positions, next token's embedding row.
 //
 // Rounding points are the eager modules' (the same as in qwen3_decode.cu).
@@ -495,10 +497,10 @@ __global__ void __launch_bounds__(32 * NB) finish_kernel(const TokenArgs a) {
 
 // ---- attention ------------------------------------------------------------------------------------------------------------
 // One cluster of CS CTAs per (sequence, kv head); rank r takes the r-th piece of the cached positions (if the sequence is long
-// enough for so many, see split_log2), rank 0 also the new one (norm, rotation, append, and its own score).  Three groups of two compute warps take turns on 32-position tiles, a
-// warp 16 positions of each with its own softmax; a seventh warp feeds a ring of six 16 KB tiles (two CTAs per SM).  A
-// warp's 16 positions are 16 MMAs: scores with the keys as A (M = positions) and the two query heads as N columns, P V with
-// V^T as A (ldmatrix.trans on the swizzled tile) and P as B, its high parts in columns 0-1, its low parts in columns 2-3.
+// enough for so many, see split_log2), rank 0 also the new one (norm, rotation, append, and its own score).  Three groups of two
+// compute warps take turns on 32-position tiles, a warp 16 positions of each with its own softmax; a seventh warp feeds a ring
+// of six 16 KB tiles (two CTAs per SM).  A warp's 16 positions are 16 MMAs: scores with the keys as A (M = positions) and the two query heads as N columns, P V with
+// V^T as A (ldmatrix.trans on the swizzled tile) and P as B, its middle, low and high parts in columns 0-1, 2-3 and 4-5.
 // A tile is about 1000 dependent cycles for a warp, which is why the tiles are small and the warps many.
 constexpr int kGroups = 3, kAttnWarps = 2 * kGroups, kAttnThreads = 32 * kAttnWarps + 32, kTilePos = 32, kRing = 2 * kGroups;
 // Tile `it` belongs to group it % 3, which has two ring slots of its own: a slot's phases are waited for by the same two
@@ -749,9 +751,12 @@ __global__ void __launch_bounds__(kAttnThreads, 2) attn_kernel(const __grid_cons
                 const float e0 = ex2f(s0 - m0), e1 = ex2f(s1 - m1), e2 = ex2f(s2 - m0), e3 = ex2f(s3 - m1);
                 l0 += e0 + e2; l1 += e1 + e3;
                 const uint32_t h01 = pack_bf16x2(e0, e1), h23 = pack_bf16x2(e2, e3);
-                uint32_t u = 0u, v = 0u;
-                if (t == 0) { u = h01; v = h23; }
-                if (t == 1) { u = pack_bf16x2(e0 - bf_lo(h01), e1 - bf_hi(h01)); v = pack_bf16x2(e2 - bf_lo(h23), e3 - bf_hi(h23)); }
+                // Lane t = 2 supplies the high part, 0 the middle one, 1 the low one (both differences are exact), 3 nothing.
+                const float r0 = e0 - bf_lo(h01), r1 = e1 - bf_hi(h01), r2 = e2 - bf_lo(h23), r3 = e3 - bf_hi(h23);
+                const uint32_t m01 = pack_bf16x2(r0, r1), m23 = pack_bf16x2(r2, r3);
+                uint32_t u = t == 2 ? h01 : m01, v = t == 2 ? h23 : m23;
+                if (t == 1) { u = pack_bf16x2(r0 - bf_lo(m01), r1 - bf_hi(m01)); v = pack_bf16x2(r2 - bf_lo(m23), r3 - bf_hi(m23)); }
+                if (t == 3) { u = 0u; v = 0u; }
                 const uint32_t b0 = movm_t(u), b1 = movm_t(v);
 #pragma unroll
                 for (int i = 0; i < 8; ++i) {
@@ -766,13 +771,20 @@ __global__ void __launch_bounds__(kAttnThreads, 2) attn_kernel(const __grid_cons
 #pragma unroll
         for (int of = 4; of < 32; of <<= 1) { l0 += __shfl_xor_sync(0xffffffffu, l0, of); l1 += __shfl_xor_sync(0xffffffffu, l1, of); }
         if (lane == 0) { pm[warp][0] = m0; pm[warp][1] = m1; pl[warp][0] = l0; pl[warp][1] = l1; }
+        // The three parts of an output lie in lanes t = 0, 1, 2: added up (middle + low, then high) in two exchanges that leave each
+        // lane a quarter of the sums, lane t the rows with bit 3 = t & 1 and bit 4 = t >> 1, so that the 32 lanes of a store hit
+        // 32 banks.
+        const bool t0 = (t & 1) != 0, t1 = (t & 2) != 0;
+        float w[8][2];
 #pragma unroll
-        for (int i = 0; i < 8; ++i) {
-            float v[4];
+        for (int i = 0; i < 8; ++i)
 #pragma unroll
-            for (int j = 0; j < 4; ++j) v[j] = o[i][j] + __shfl_xor_sync(0xffffffffu, o[i][j], 1);    // high part + low part
-            if (t == 0) { po[warp][0][16 * i + g] = v[0]; po[warp][1][16 * i + g] = v[1]; po[warp][0][16 * i + 8 + g] = v[2]; po[warp][1][16 * i + 8 + g] = v[3]; }
-        }
+            for (int j = 0; j < 2; ++j) w[i][j] = (t0 ? o[i][j + 2] : o[i][j]) + __shfl_xor_sync(0xffffffffu, t0 ? o[i][j] : o[i][j + 2], 1);
+#pragma unroll
+        for (int i = 0; i < 8; i += 2)
+#pragma unroll
+            for (int j = 0; j < 2; ++j)
+                po[warp][j][16 * (i + (t >> 1)) + 8 * (t & 1) + g] = (t1 ? w[i + 1][j] : w[i][j]) + __shfl_xor_sync(0xffffffffu, t1 ? w[i][j] : w[i + 1][j], 2);
         compute_sync();
         bf16* out = a.attn + (size_t)b * DQ + 2 * kvh * HD;
         if constexpr (CS > 1) asm volatile("barrier.cluster.wait.acquire;" ::: "memory");
