@@ -92,11 +92,12 @@ __device__ __forceinline__ uint4 ldg_weight(const void* p, uint64_t pol) {
 __device__ __forceinline__ uint32_t norm_pair(uint32_t x, uint32_t g, float rstd) {
     return pack_bf16x2(bf16r(bf_lo(x) * rstd) * bf_lo(g), bf16r(bf_hi(x) * rstd) * bf_hi(g));
 }
-// 1 / sqrt(v) to fp32 accuracy: the hardware approximation and one Newton step (1.0f / sqrtf(v) is two long dependent
-// sequences, and every kernel that normalises has one on its critical path).
+// 1 / sqrt(v): the hardware approximation and one Newton step (1.0f / sqrtf(v) is two long dependent sequences, and every kernel
+// that normalises has one on its critical path).  Over every float of [1, 4) at most 1.00 ulp from the 64-bit value and 0.28 on
+// average; 1.0f / sqrtf(v): 1.49 and 0.35.
 __device__ __forceinline__ float rsqrt_full(float v) {
-    const float r = rsqrtf(v);
-    return fmaf(r * 0.5f, fmaf(-v * r, r, 1.0f), r);
+    const float r = rsqrtf(v), y = fmaf(r * 0.5f, fmaf(-v * r, r, 1.0f), r);
+    return v < INFINITY && v > 0.f ? y : r;           // 0 for a sum of squares that overflowed, not inf * 0
 }
 // RMSNorm of the NB rows of x (width D) into xs[b][..] (rows padded by 64 bytes, see the weight rows): the 512 threads share
 // the rows out, 2 NB values each, so that every value is normalised once per CTA.  Contains the two barriers after which xs

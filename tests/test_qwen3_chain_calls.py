@@ -97,3 +97,21 @@ def test_a_reported_failure_is_not_reported_again(tiny_hf):
         d.prefill_slots({0: [4, 5]})
         d.check_status()
         assert d.lengths == d.pos.tolist() == [45]
+
+
+@gpu
+@pytest.mark.parametrize("batch", [1, 4])
+def test_a_sum_of_squares_that_overflows(tiny_hf, batch):
+    """Hidden values whose squares overflow fp32 normalise to zero, as 1 / sqrt(inf) has it: the ids and logits are the persistent
+    kernel's (which an unused flag bit selects), not a row of NaNs."""
+    from ittai_b200.qwen3 import Qwen3Decoder
+    model, dims = tiny_hf
+    sd = {k: v.clone() for k, v in model.state_dict().items()}
+    sd["model.embed_tokens.weight"][5] = 3e19
+    d = Qwen3Decoder(sd, max_batch=batch, kv_capacity=64)
+    got = []
+    for d.flags in (1 << 20, 0):
+        d.reset()
+        d.next_id.fill_(5)
+        got.append((d.decode(1).clone(), d.logits.clone()))
+    assert all(torch.equal(a, b) for a, b in zip(*got)) and not got[1][1].isnan().any()
