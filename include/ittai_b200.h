@@ -179,7 +179,8 @@ int ittai_qwen3_phase_launch(const IttaiQwen3Decode* p, int phase, int layer, vo
  * step_ns changes.  `max_len`: an upper bound of pos[b] over the sequences.  It picks the cluster size of a launch; a
  * sequence's results follow from its own length and `batch` alone, bit for bit.  p->phase_clk is not used.  An id or position out of range ends in ITTAI_ST_BAD_TOKEN, a wait that runs out in
  * ITTAI_ST_STREAM_TIMEOUT: the steps from there on store no id, `next_id` keeps the last good
- * step's id and `pos` is what it was before the call.  A stream that is being captured gets the kernels themselves.  Calls on one plan are serialised. */
+ * step's id and `pos` is what it was before the call.  A stream that is being captured gets the kernels themselves.  Calls on one plan are serialised,
+ * on the host and on the device, whatever streams they are on; only a captured call's replays are the caller's to order. */
 int ittai_qwen3_chain_create(void** plan);
 int ittai_qwen3_chain_run(void* plan, const IttaiQwen3Decode* p, int32_t max_len, void* stream);
 int ittai_qwen3_chain_destroy(void* plan);

@@ -1011,6 +1011,29 @@ static int capture(Plan* pl, int lg, bool head, cudaGraphExec_t* out) {
     return ITTAI_OK;
 }
 
+// Everything one call queues on `st`.
+static int enqueue_call(Plan* pl, const IttaiQwen3Decode& p, int max_len, bool captured, cudaStream_t st) {
+    enqueue_begin(*pl, p, st);
+    for (int i = 0; i < p.n_steps; ++i) {
+        const bool head = i >= p.n_forced - 1;
+        const int lg = split_log2(p.batch, max_len + i);
+        cudaError_t e;
+        if (captured) {                                // a graph launch cannot be captured: the kernels themselves can
+            e = enqueue_token(*pl, 1 << lg, head, st);
+        } else {
+            cudaGraphExec_t& x = pl->exec[lg][head ? 1 : 0];
+            if (x == nullptr) {
+                const int rc = capture(pl, lg, head, &x);
+                if (rc != ITTAI_OK) return rc;
+            }
+            e = cudaGraphLaunch(x, st);
+        }
+        if (e != cudaSuccess) return cuda_fail(e, "launch of a decode step");
+    }
+    const cudaError_t e = cudaGetLastError();
+    return e == cudaSuccess ? ITTAI_OK : cuda_fail(e, "decode chain");
+}
+
 }  // namespace chain
 }  // namespace ittai
 
@@ -1060,26 +1083,15 @@ extern "C" int ittai_qwen3_chain_run(void* plan, const IttaiQwen3Decode* p, int3
     cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
     e = cudaStreamIsCapturing(st, &cap);
     if (e != cudaSuccess) return cuda_fail(e, "cudaStreamIsCapturing");
-    chain::enqueue_begin(*pl, *p, st);
-    for (int i = 0; i < p->n_steps; ++i) {
-        const bool head = i >= p->n_forced - 1;
-        const int lg = chain::split_log2(p->batch, max_len + i);
-        if (cap != cudaStreamCaptureStatusNone) {      // a graph launch cannot be captured: the kernels themselves can
-            e = chain::enqueue_token(*pl, 1 << lg, head, st);
-        } else {
-            cudaGraphExec_t& x = pl->exec[lg][head ? 1 : 0];
-            if (x == nullptr) {
-                rc = chain::capture(pl, lg, head, &x);
-                if (rc != ITTAI_OK) return rc;
-            }
-            e = cudaGraphLaunch(x, st);
-        }
-        if (e != cudaSuccess) return cuda_fail(e, "launch of a decode step");
+    const bool captured = cap != cudaStreamCaptureStatusNone;
+    if (!captured) {                                   // the call before may be on another stream; both use one state record
+        e = cudaStreamWaitEvent(st, pl->last, 0);      // (no wait before the first call has recorded it)
+        if (e != cudaSuccess) return cuda_fail(e, "cudaStreamWaitEvent");
     }
-    if (cap == cudaStreamCaptureStatusNone) {
+    rc = chain::enqueue_call(pl, *p, max_len, captured, st);
+    if (!captured) {                                   // also where the call failed half way: what it has queued still runs
         e = cudaEventRecord(pl->last, st);
-        if (e != cudaSuccess) return cuda_fail(e, "cudaEventRecord");
+        if (rc == ITTAI_OK && e != cudaSuccess) return cuda_fail(e, "cudaEventRecord");
     }
-    e = cudaGetLastError();
-    return e == cudaSuccess ? ITTAI_OK : cuda_fail(e, "decode chain");
+    return rc;
 }

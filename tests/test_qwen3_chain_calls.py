@@ -115,3 +115,23 @@ def test_a_sum_of_squares_that_overflows(tiny_hf, batch):
         d.next_id.fill_(5)
         got.append((d.decode(1).clone(), d.logits.clone()))
     assert all(torch.equal(a, b) for a, b in zip(*got)) and not got[1][1].isnan().any()
+
+
+@gpu
+def test_calls_on_two_streams_follow_one_another(tiny_hf):
+    """Calls of one decoder queued on two streams, nothing waited for in between: the second starts where the first ends."""
+    from ittai_b200.qwen3 import Qwen3Decoder
+    model, dims = tiny_hf
+    d = Qwen3Decoder(model, max_batch=2, kv_capacity=256)
+    d.next_id.fill_(9)
+    want = d.decode(90).cpu()
+    d.reset()
+    d.next_id.fill_(9)
+    torch.cuda.synchronize()
+    streams, parts = [torch.cuda.Stream(), torch.cuda.Stream()], []
+    for i, n in enumerate((40, 7, 1, 30, 12)):
+        with torch.cuda.stream(streams[i % 2]):
+            parts.append(d.decode(n, check=False))
+    torch.cuda.synchronize()
+    d.check_status()
+    assert torch.equal(torch.cat([t.cpu() for t in parts], 1), want) and d.pos.tolist() == d.lengths == [90, 90]
