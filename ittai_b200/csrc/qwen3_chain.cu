@@ -28,6 +28,7 @@
 // next kernel's weight loads in the load pipe), normalisation in every warp's fragments (509: issue-bound), constants
 // loaded ahead of the wait but scheduled behind it, the head through registers (93 us instead of 47).
 #include <mutex>
+#include <new>
 
 #include "gemm2_common.cuh"
 #include "launch.h"
@@ -1041,7 +1042,8 @@ using namespace ittai;
 
 extern "C" int ittai_qwen3_chain_create(void** plan) {
     if (!plan) { set_error("null plan"); return ITTAI_E_ARG; }
-    *plan = new chain::Plan();
+    *plan = new (std::nothrow) chain::Plan();
+    if (*plan == nullptr) { set_error("chain_create: out of host memory"); return ITTAI_E_ARG; }
     return ITTAI_OK;
 }
 
