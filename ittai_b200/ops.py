@@ -14,7 +14,13 @@ def new_status(device) -> torch.Tensor:
 
 
 def check_status(status: torch.Tensor) -> None:
-    _C.decode_status(status.cpu().tolist())
+    """Wait for the work queued so far and raise if it reported a failed wait; the words are cleared then, so that a failure is
+    reported once."""
+    try:
+        _C.decode_status(status.cpu().tolist())
+    except _C.IttaiError:
+        status.zero_()
+        raise
 
 
 def _stream(t: torch.Tensor):

@@ -121,7 +121,8 @@ class Engine:
         # the packing of a forward, written by one copy: seqs [B, 4], last [B], then tokens, pos, seq, slot [T] (see ``_views``)
         self.meta = z(5 * max_seqs + 4 * self.M, dt=torch.int32)
         self.out = z(max_seqs, D, dt=torch.float32)
-        self.use_graph, self._graphs, self._seen, self._checked = graph, {}, {}, False
+        self.use_graph, self._graphs, self._seen = graph, {}, {}
+        self._unread = False                 # a shape ran for the first time and its status words have not been read yet
 
     def _views(self, T, B):
         """The parts of ``meta`` for a forward of ``T`` tokens in ``B`` sequences; ``seqs`` first: it is read 16 bytes at a time."""
@@ -139,7 +140,9 @@ class Engine:
     GRAPH_TOKENS, GRAPHS, SHAPES = 1024, 16, 256
 
     @torch.no_grad()
-    def forward(self, input_ids):
+    def forward(self, input_ids, check=True):
+        """Embeddings of the packed sequences.  The first forward of a shape is waited for and its status words are read; with
+        ``check=False`` that is left to ``check_new``, for callers that queue several forwards."""
         seqlens = [len(x) for x in input_ids]
         T, B = sum(seqlens), len(seqlens)
         assert T <= self.M and B <= self.Bmax and min(seqlens) > 0
@@ -155,13 +158,11 @@ class Engine:
             self._graphs[key].replay()
         elif not self.use_graph or T > self.GRAPH_TOKENS or key not in self._seen:
             # a shape's first forward runs as plain launches: a capture costs more than it could give back
+            self._unread |= key not in self._seen
             self._seen[key] = True
             if len(self._seen) > self.SHAPES:
                 self._seen.pop(next(iter(self._seen)))
             self._body(*key)
-            if not self._checked:
-                self.check()
-                self._checked = True
         else:
             if len(self._graphs) >= self.GRAPHS:
                 old = next(iter(self._graphs))
@@ -172,10 +173,19 @@ class Engine:
                 self._body(*key)
             self._graphs[key] = g
             g.replay()
+        if check:
+            self.check_new()
         return self.out[:B]
 
     def check(self) -> None:
+        """Wait for the queued forwards and raise if a bounded wait of theirs ran out."""
+        self._unread = False
         ops.check_status(self.core.status)
+
+    def check_new(self) -> None:
+        """``check`` if a shape has run for the first time since the last one."""
+        if self._unread:
+            self.check()
 
     def task_list(self, seqlens, group_m=8):
         """The forward over ``seqlens`` as the reference's device queue would see it: ``(tasks, expect, T)`` of

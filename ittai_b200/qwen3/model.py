@@ -87,7 +87,8 @@ class Qwen3Embedder:
     def embed(self, texts, max_length=2048):
         """fp32 ``[N, 1024]`` embeddings; every batch's result is cloned out of the engine's persistent buffer."""
         ids = self._ids(texts, max_length)
-        parts = [self.engine.forward(ids[a:a + n]).clone() for a, n in self._batches([len(s) for s in ids])]
+        parts = [self.engine.forward(ids[a:a + n], check=False).clone() for a, n in self._batches([len(s) for s in ids])]
+        self.engine.check_new()
         return torch.cat(parts) if parts else torch.zeros(0, 1024)
 
     @torch.no_grad()

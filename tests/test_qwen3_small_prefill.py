@@ -25,3 +25,21 @@ def test_small_forwards_match_the_oracle(tiny_hf, lens):
         R = ref.Qwen3Ref(model.state_dict(), dims, 256)
         R.forward(torch.tensor(s))
         assert F.cosine_similarity(out[i].cpu(), R.embed_pool(), dim=0) >= 0.9995, (i, lens)
+
+
+@gpu
+def test_a_failed_wait_of_any_new_shape_is_reported(tiny_hf):
+    """A status word planted ahead of a forward: the first forward of every shape reads it, alone and inside ``embed``, and it is
+    reported once."""
+    from ittai_b200._C import IttaiError
+    from ittai_b200.qwen3 import Qwen3Embedder
+    model, dims = tiny_hf
+    emb = Qwen3Embedder(model, max_tokens=256, max_seqs=4)
+    ids = lambda n: list(range(1, n + 1))
+    want = emb.embed([ids(7)]).clone()
+    for call in (lambda: emb.engine.forward([ids(9)]), lambda: emb.embed([ids(11), ids(3)]), lambda: emb.embed([ids(40)] * 5)):
+        emb.engine.core.status[0] = 5
+        with pytest.raises(IttaiError, match="GEMM"):
+            call()
+        assert torch.equal(emb.embed([ids(7)]), want)
+        emb.engine.check()
