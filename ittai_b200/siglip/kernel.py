@@ -173,7 +173,7 @@ class Engine:
         self.chain = bool(chain) and self.fold_ln and M >= 1024      # a few row blocks only: nothing to overlap, one launch per GEMM is faster
         self.chain_flags = torch.zeros(len(self.layers) + 1, 4 * 2 * ((M + 255) // 256), dtype=torch.int32, device=dev)
         self.status = ops.new_status(dev)
-        self.use_graph, self._graphs, self._seen, self._checked = graph, {}, set(), False      # per number of images
+        self.use_graph, self._graphs, self._seen, self._unread = graph, {}, set(), False       # per number of images
 
     def _body(self, B):
         """Queue the forward of the first ``B`` images of the buffers."""
@@ -255,15 +255,19 @@ class Engine:
         first) and ``spatial_shapes`` ``[B, 2]``, like the reference's engine (``:638-649``)."""
         self._load(inp, self.B)
         self._run(self.B)
+        self.check_new()
         return self.embeds
 
     @torch.no_grad()
-    def forward_part(self, inp):
-        """``forward`` of a short batch: 1 to ``B`` images; returns bf16 ``[n, D]``, a view of the same buffer."""
+    def forward_part(self, inp, check=True):
+        """``forward`` of a short batch: 1 to ``B`` images; returns bf16 ``[n, D]``, a view of the same buffer.  With
+        ``check=False`` reading the status words of a size's first forward is left to ``check_new``."""
         n = len(inp["pixel_values"])
         assert 1 <= n <= self.B, f"1 to {self.B} images, got {n}"
         self._load(inp, n)
         self._run(part_size(n, self.B, self.S0, self.chain))
+        if check:
+            self.check_new()
         return self.embeds[:n]
 
     def _load(self, inp, n):
@@ -284,20 +288,9 @@ class Engine:
                                                  self.pos.stride(0), self.seqs.data_ptr(), self.pool_seqs.data_ptr(), ops._stream(self.pos)))
 
     def _run(self, n):
-        """The forward over the first ``n`` images of the buffers.  Plain launches the first time a size is seen (the very
-        first also reads the status words), a CUDA graph from the second time on."""
+        """The forward over the first ``n`` images of the buffers.  Plain launches the first time a size is seen (``check_new``
+        then reads the status words), a CUDA graph from the second time on."""
         graph = self._graphs.get(n)
-        if graph is None and not self._checked:
-            self.status.zero_()
-            s = torch.cuda.Stream()
-            s.wait_stream(torch.cuda.current_stream())
-            with torch.cuda.stream(s):
-                self._body(n)
-            torch.cuda.current_stream().wait_stream(s)
-            ops.check_status(self.status)
-            self._checked = True
-            self._seen.add(n)
-            return
         if graph is None and self.use_graph and n in self._seen:
             if len(self._graphs) > self.PARTS:
                 self._graphs.pop(next(k for k in self._graphs if k != self.B))
@@ -305,6 +298,7 @@ class Engine:
             with torch.cuda.graph(graph):
                 self._body(n)
             self._graphs[n] = graph
+        self._unread |= n not in self._seen
         self._seen.add(n)
         if graph is not None:
             graph.replay()
@@ -318,8 +312,14 @@ class Engine:
         return (1 if self.conv else 0) + encoder + 5       # + pooling head: attention, projection, LayerNorm, two MLP GEMMs
 
     def check(self) -> None:
-        """Synchronise and raise if any GEMM pipeline wait ran out since construction."""
+        """Synchronise and raise if any bounded wait ran out since the last report."""
+        self._unread = False
         ops.check_status(self.status)
+
+    def check_new(self) -> None:
+        """``check`` if a size has run for the first time since the last one."""
+        if self._unread:
+            self.check()
 
     def flops(self, formula: str = "reference") -> float:
         """FLOPs of one forward.  ``reference``: the reference benchmark's formula (``benchmarks/siglip.py:35``), which
@@ -461,4 +461,6 @@ class Siglip2Embedder:
         # slices of the caller's tensors, so that pinned ones stay pinned; a short last batch runs as what it is (the reference
         # fills it up with copies of its final image, ``:720-723``)
         parts = ({name: t[k:k + self.B] for name, t in inp.items()} for k in range(0, total, self.B))
-        return torch.cat(self._stream_batches(parts, False, self.engine.forward_part))
+        out = torch.cat(self._stream_batches(parts, False, lambda part: self.engine.forward_part(part, check=False)))
+        self.engine.check_new()
+        return out

@@ -132,7 +132,7 @@ class PaddedEngine:
         self.seqs = torch.tensor([[b * S, S, b * S, S] for b in range(B)], dtype=torch.int32, device=dev)
         self.pool_seqs = torch.tensor([[b, 1, b * S, S] for b in range(B)], dtype=torch.int32, device=dev)
         self.status = ops.new_status(dev)
-        self.use_graph, self._graphs, self._seen, self._checked = graph, {}, set(), False      # per number of images
+        self.use_graph, self._graphs, self._seen, self._unread = graph, {}, set(), False       # per number of images
 
     def _body(self, B):
         """Queue the forward of the first ``B`` images of the buffers."""
@@ -197,15 +197,18 @@ class PaddedEngine:
     def forward(self, inp):
         self._load(inp, self.B)
         self._run(self.B)
+        self.check_new()
         return self.embeds_p[:, :self.D]
 
     @torch.no_grad()
-    def forward_part(self, inp):
+    def forward_part(self, inp, check=True):
         from .kernel import part_size
         n = len(inp["pixel_values"])
         assert 1 <= n <= self.B, f"1 to {self.B} images, got {n}"
         self._load(inp, n)
         self._run(part_size(n, self.B, self.S0, self.chain))
+        if check:
+            self.check_new()
         return self.embeds_p[:n, :self.D]
 
     def _load(self, inp, n):
@@ -227,7 +230,12 @@ class PaddedEngine:
         Engine._run(self, n)
 
     def check(self) -> None:
+        self._unread = False
         ops.check_status(self.status)
+
+    def check_new(self) -> None:
+        if self._unread:
+            self.check()
 
     def launches_per_forward(self) -> int:
         """Kernels in one forward (all inside one CUDA graph)."""

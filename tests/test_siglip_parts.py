@@ -116,3 +116,19 @@ def test_key_counts_of_the_batch_before_are_not_seen(batch):
     eng.check()
     for i, t in enumerate(got):
         assert torch.equal(t, want[i % 3]), i
+
+
+@gpu
+def test_a_failed_wait_of_any_new_size_is_reported():
+    """A status word planted ahead of a forward: the first forward of every batch size reads it, and it is reported once."""
+    from ittai_b200._C import IttaiError
+    from ittai_b200.siglip.kernel import Siglip2Embedder
+    emb = Siglip2Embedder(hf.build_hf(seed=0, device="cuda", n_layers=1), batch_size=4)
+    px = hf.pixels(4, seed=3)
+    want = emb.embed(px)
+    for call in (lambda: emb.embed(px[:3]), lambda: emb.engine.forward_part({"pixel_values": px[:1]}), lambda: emb.embed(torch.cat([px, px[:2]]))):
+        emb.engine.status[0] = 5
+        with pytest.raises(IttaiError, match="GEMM"):
+            call()
+        assert torch.equal(emb.embed(px), want)
+        emb.engine.check()
