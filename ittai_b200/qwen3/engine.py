@@ -16,6 +16,7 @@ import numpy as np
 import torch
 
 from .. import _C, ops
+from ..graphs import Graphs
 from .config import BM, D, DGU, DQ, DQKV, EPS, FF, HD, NH, NKV, QB
 from .decoder import _strip, pack_weights, rope_table
 from .tasks import build_tasks
@@ -121,7 +122,7 @@ class Engine:
         # the packing of a forward, written by one copy: seqs [B, 4], last [B], then tokens, pos, seq, slot [T] (see ``_views``)
         self.meta = z(5 * max_seqs + 4 * self.M, dt=torch.int32)
         self.out = z(max_seqs, D, dt=torch.float32)
-        self.use_graph, self._graphs, self._seen = graph, {}, {}
+        self._graphs, self._plain = Graphs(self.GRAPHS if graph else 0), Graphs(0)
         self._unread = False                 # a shape ran for the first time and its status words have not been read yet
 
     def _views(self, T, B):
@@ -137,7 +138,7 @@ class Engine:
 
     # Up to this many tokens a repeated shape is replayed from a CUDA graph; above, the GPU is busy for longer than the host
     # needs to queue the launches.
-    GRAPH_TOKENS, GRAPHS, SHAPES = 1024, 16, 256
+    GRAPH_TOKENS, GRAPHS = 1024, 16
 
     @torch.no_grad()
     def forward(self, input_ids, check=True):
@@ -154,25 +155,17 @@ class Engine:
         self.meta[:meta.numel()].copy_(meta, non_blocking=True)
         # the launches depend on these three numbers alone, the packing itself is read on the device
         key = (T, B, max(seqlens))
-        if key in self._graphs:
-            self._graphs[key].replay()
-        elif not self.use_graph or T > self.GRAPH_TOKENS or key not in self._seen:
-            # a shape's first forward runs as plain launches: a capture costs more than it could give back
-            self._unread |= key not in self._seen
-            self._seen[key] = True
-            if len(self._seen) > self.SHAPES:
-                self._seen.pop(next(iter(self._seen)))
-            self._body(*key)
-        else:
-            if len(self._graphs) >= self.GRAPHS:
-                old = next(iter(self._graphs))
-                self._graphs.pop(old)
-                self._seen.pop(old, None)
-            g = torch.cuda.CUDAGraph()
-            with torch.cuda.graph(g):
+        new, graph, capture = (self._graphs if T <= self.GRAPH_TOKENS else self._plain).use(key)
+        self._unread |= new
+        if capture:
+            graph = torch.cuda.CUDAGraph()
+            with torch.cuda.graph(graph):
                 self._body(*key)
-            self._graphs[key] = g
-            g.replay()
+            self._graphs.put(key, graph)
+        if graph is not None:
+            graph.replay()
+        else:
+            self._body(*key)
         if check:
             self.check_new()
         return self.out[:B]

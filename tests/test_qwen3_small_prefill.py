@@ -43,3 +43,20 @@ def test_a_failed_wait_of_any_new_shape_is_reported(tiny_hf):
             call()
         assert torch.equal(emb.embed([ids(7)]), want)
         emb.engine.check()
+
+
+@gpu
+def test_more_shapes_than_graphs(tiny_hf):
+    """Queries of more lengths than the engine keeps graphs for, in turn: every length is captured at most once, and gives on plain
+    launches and from a graph what it gave the first time."""
+    from ittai_b200.qwen3 import Engine
+    model, dims = tiny_hf
+    eng = Engine(model, 128, 4)
+    eng._graphs.limit = 3
+    ids = lambda n: list(range(1, n + 1))
+    want = {n: eng.forward([ids(n)]).clone() for n in range(2, 9)}
+    for _ in range(4):
+        for n, w in want.items():
+            assert torch.equal(eng.forward([ids(n)]), w), n
+        assert sorted(eng._graphs.graphs) == [(n, 1, n) for n in (2, 3, 4)]
+    eng.check()
