@@ -10,9 +10,13 @@ class Graphs:
     A key's first forward runs as plain launches and its second one is captured while there is room.  When there is none, a
     graph gives way only after ``idle`` forwards without a use, the one unused for longest first; until then the other keys stay
     on plain launches.  A capture costs several forwards, and with more keys in turn than graphs every capture would throw out a
-    graph that is about to be used: at most ``limit`` captures per ``idle`` forwards are left.  The last ``keys`` keys are known."""
+    graph that is about to be used: at most ``limit`` captures per ``idle`` forwards are left.  The last ``keys`` keys are known.
 
-    def __init__(self, limit: int, keys: int = 256, idle: int = 1024):
+    Measured on a B200, us a call with every call waited for, first in first out before -> this rule: queries of 5 to 60 tokens
+    over 16 graphs 1418 -> 1126 (of 5 to 15 tokens, where all fit, 912 both), 1 to 64 images of ViT-B/16 over 8 graphs
+    2510 -> 1749 (1 to 8 images, three sizes: 1010 both)."""
+
+    def __init__(self, limit: int, keys: int = 256, idle: int = 256):
         self.limit, self.keys, self.idle = limit, keys, idle
         self.seen: OrderedDict = OrderedDict()       # keys of earlier forwards, the one unused for longest first
         self.graphs: OrderedDict = OrderedDict()     # key -> (graph, forward of its last use), likewise

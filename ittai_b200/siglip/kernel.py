@@ -14,6 +14,7 @@ import ctypes as C
 import torch
 
 from .. import _C, ops
+from ..graphs import Graphs
 
 
 def fold_ln(W, b, g, beta, dtype=torch.bfloat16):
@@ -173,7 +174,7 @@ class Engine:
         self.chain = bool(chain) and self.fold_ln and M >= 1024      # a few row blocks only: nothing to overlap, one launch per GEMM is faster
         self.chain_flags = torch.zeros(len(self.layers) + 1, 4 * 2 * ((M + 255) // 256), dtype=torch.int32, device=dev)
         self.status = ops.new_status(dev)
-        self.use_graph, self._graphs, self._seen, self._unread = graph, {}, set(), False       # per number of images
+        self._full, self._graphs, self._unread = Graphs(1 if graph else 0), Graphs(self.PARTS if graph else 0), False
 
     def _body(self, B):
         """Queue the forward of the first ``B`` images of the buffers."""
@@ -289,17 +290,15 @@ class Engine:
 
     def _run(self, n):
         """The forward over the first ``n`` images of the buffers.  Plain launches the first time a size is seen (``check_new``
-        then reads the status words), a CUDA graph from the second time on."""
-        graph = self._graphs.get(n)
-        if graph is None and self.use_graph and n in self._seen:
-            if len(self._graphs) > self.PARTS:
-                self._graphs.pop(next(k for k in self._graphs if k != self.B))
+        then reads the status words), a CUDA graph from the second time on while there is room (see ``Graphs``)."""
+        graphs = self._full if n == self.B else self._graphs
+        new, graph, capture = graphs.use(n)
+        self._unread |= new
+        if capture:
             graph = torch.cuda.CUDAGraph()
             with torch.cuda.graph(graph):
                 self._body(n)
-            self._graphs[n] = graph
-        self._unread |= n not in self._seen
-        self._seen.add(n)
+            graphs.put(n, graph)
         if graph is not None:
             graph.replay()
         else:

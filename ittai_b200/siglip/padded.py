@@ -19,6 +19,7 @@ import torch
 import torch.nn.functional as F
 
 from .. import _C, ops
+from ..graphs import Graphs
 
 
 def _up(n: int, m: int) -> int:
@@ -132,7 +133,7 @@ class PaddedEngine:
         self.seqs = torch.tensor([[b * S, S, b * S, S] for b in range(B)], dtype=torch.int32, device=dev)
         self.pool_seqs = torch.tensor([[b, 1, b * S, S] for b in range(B)], dtype=torch.int32, device=dev)
         self.status = ops.new_status(dev)
-        self.use_graph, self._graphs, self._seen, self._unread = graph, {}, set(), False       # per number of images
+        self._full, self._graphs, self._unread = Graphs(1 if graph else 0), Graphs(self.PARTS if graph else 0), False
 
     def _body(self, B):
         """Queue the forward of the first ``B`` images of the buffers."""

@@ -132,3 +132,20 @@ def test_a_failed_wait_of_any_new_size_is_reported():
             call()
         assert torch.equal(emb.embed(px), want)
         emb.engine.check()
+
+
+@gpu
+def test_more_batch_sizes_than_graphs():
+    """Short batches of more sizes than the engine keeps graphs for, in turn, with the full batch among them: each size is captured
+    at most once, and every size gives what it gave the first time."""
+    from ittai_b200.siglip.kernel import Siglip2Embedder
+    emb = Siglip2Embedder(hf.build_hf(seed=0, device="cuda", n_layers=1), batch_size=5)
+    eng = emb.engine
+    eng._graphs.limit = 2
+    px = hf.pixels(5, seed=3).cuda()
+    want = {n: emb.embed(px[:n]) for n in (1, 2, 3, 4, 5)}
+    for _ in range(4):
+        for n, w in want.items():
+            assert torch.equal(emb.embed(px[:n]), w), n
+        assert sorted(eng._graphs.graphs) == [1, 2] and list(eng._full.graphs) == [5]
+    eng.check()
