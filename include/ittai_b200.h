@@ -312,7 +312,8 @@ typedef struct IttaiQwen3Prefill {
     int32_t kv_cap;        /* cache rows per (sequence, head) */
     int32_t fused_rope;    /* 1: QK-norm + RoPE + scatter in the QKV projection's epilogue where one covers it, 0: a pass of its own */
     int32_t split_k;       /* 1: small forwards may split sums over K (ITTAI_GEMM_STATIC_W), so that a token's values depend on
-                              T in their last bits; 0: they do not depend on what else is packed into the forward */
+                              T in their last bits; 0: every sum over K is taken in one order.  What is left then are two choices
+                              of kernel: rotation in the epilogue or as a pass (T > 128) and the attention kernel (max_q_len > 64) */
     int32_t reserved0;
     float eps;
     const void *wqkv, *wo, *wgu, *wd, *ln1, *ln2, *qn, *kn, *embed, *rope;   /* as in IttaiQwen3Decode */

@@ -1,8 +1,12 @@
 // Host helper: kernel launches that let the NEXT kernel of the stream begin its prologue before this one has drained
-// (programmatic dependent launch).  Every kernel launched through launch_pdl calls pdl_trigger() on entry and
-// pdl_wait() before its first access to global memory another kernel may have written or may still read, so the only
-// work that overlaps is barrier initialisation, tensor-memory allocation and descriptor prefetch, plus the launch
-// latency itself.  ITTAI_PDL=0 in the environment turns the attribute off (plain stream order).
+// (programmatic dependent launch).  Every kernel launched through launch_pdl calls pdl_wait() before its first access to global
+// memory that another kernel of the run may have written or may still read, and pdl_trigger() on entry, or once the resources
+// that it shares with its successors are its own.  So a kernel may be resident while several kernels in front of it still run
+// (each of them triggers before it waits): what it reads ahead of its wait has to be complete before the FIRST of them starts.
+// Ahead of the wait run barrier initialisation, tensor-memory allocation and descriptor prefetch, and in some kernels loads of
+// such data: weights in the split-K GEMM and the decode chain; in the chain also positions and older cache rows, which the
+// late trigger of a token's first kernel makes safe; sequence records in the key-loop attention, where the caller vouches for
+// them.  ITTAI_PDL=0 in the environment turns the attribute off (plain stream order).
 #pragma once
 #include <cuda_runtime.h>
 

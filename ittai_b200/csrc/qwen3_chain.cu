@@ -2,14 +2,15 @@
 //
 // A decoded token is 28 x (QKV, attention, O-proj, gate/up, down) + head + finish: 142 launches whose only dependency is
 // one short vector.  With programmatic dependent launch every kernel is resident, and has fetched its weights, while its
-// predecessor still runs; what remains per hand-off is a kernel boundary, 1.1 us in a graph on a B200 (1.5 us with a
-// cluster barrier), against 1.4-2.9 us for a polled flag word that 148 CTAs read (qwen3_decode.cu).
+// predecessor still runs; what remains per hand-off is a kernel boundary, 0.7-0.9 us in a graph on a B200 (last store of a
+// kernel to the release of the next), against 1.4-2.9 us for a polled flag word that 148 CTAs read (qwen3_decode.cu).
 //
 // * GEMV kernels (gemv_kernel): 512 threads; a CTA's whole slice of a projection (32 to 96 KB) is on its way to
 //   shared memory BEFORE griddepcontrol.wait (weights do not depend on the token); after the wait it is multiplied with
 //   the activations of all sequences as mma.sync m16n8k16 tiles (the sequences are the N dimension), a warp taking 16 (or
-//   8) rows x one K chunk.  Two such CTAs fit an SM, so the next kernel's weights stream while this one waits.  The K chunks
-//   meet in shared memory, in fixed order.
+//   8) rows x one K chunk.  CTAs of two neighbouring kernels fit an SM (the largest pair, gate/up and down at batch 8: 142 + 54
+//   of 228 KB; attention and gate/up do not), so the next kernel's weights stream while this one waits.  The K chunks meet in
+//   shared memory, in fixed order.
 // * Attention (attn_kernel): a cluster of CS CTAs per (sequence, kv head) splits the cache; K/V tiles of 32 positions
 //   arrive by TMA (128-byte swizzle), the first six before the wait; scores and P V on mma.sync, the splits meet
 //   through distributed shared memory.  Probabilities enter P V as three bf16 parts in separate N columns (the columns
@@ -22,8 +23,7 @@
 //
 // Measured on a B200, us per step, the persistent kernel of qwen3_decode.cu -> this chain: batch 1 at 47 / 4096 / 8100 cached
 // positions 558 -> 426, 579 -> 525, 658 -> 590; batch 4 at 47 / 1000 / 8100 792 -> 454, 813 -> 540, 1418 -> 1020; batch 8 at 1000 /
-// 8100 1009 -> 668, 2206 -> 1577.  A layer takes 13 us at a short cache: five boundaries of 0.7-0.9 us (last store of a kernel
-// to the release of the next), attention 2.6, gate/up 2.2, QKV 2.0, down 1.5, O-proj 1.1; the head 47 us at 6.6 TB/s.  What had
+// 8100 1009 -> 668, 2206 -> 1577.  A layer takes 13 us at a short cache: five boundaries, attention 2.6, gate/up 2.2, QKV 2.0, down 1.5, O-proj 1.1; the head 47 us at 6.6 TB/s.  What had
 // to go on the way (batch 1, 47 positions): weights through registers (800 us: a kernel's activation loads stand behind the
 // next kernel's weight loads in the load pipe), normalisation in every warp's fragments (509: issue-bound), constants
 // loaded ahead of the wait but scheduled behind it, the head through registers (93 us instead of 47).
@@ -75,19 +75,6 @@ inline size_t layout(int batch, char* base, Buffers* w) {
 __device__ __forceinline__ void mma16816(float (&d)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0, uint32_t b1) {
     asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, {%0, %1, %2, %3};"
                  : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3]) : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
-}
-// Weights: read once per token.  Their L2 lines are the first to go, so that 1.2 GB of them per token do not push out what
-// every kernel needs again: its instructions, its parameters, the activation vectors.
-__device__ __forceinline__ uint64_t evict_first_policy() {
-    uint64_t pol;
-    asm volatile("createpolicy.fractional.L2::evict_first.b64 %0, 1.0;" : "=l"(pol));
-    return pol;
-}
-__device__ __forceinline__ uint4 ldg_weight(const void* p, uint64_t pol) {
-    uint4 v;
-    asm volatile("ld.global.nc.L1::no_allocate.L2::cache_hint.v4.u32 {%0,%1,%2,%3}, [%4], %5;"
-                 : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "l"(p), "l"(pol));
-    return v;
 }
 // bf16 pair of x -> bf16(bf16(x * rstd) * gain)
 __device__ __forceinline__ uint32_t norm_pair(uint32_t x, uint32_t g, float rstd) {
@@ -278,10 +265,11 @@ __global__ void __launch_bounds__(kGemvThreads, 2) gemv_kernel(const GemvArgs a)
 }
 
 // ---- lm_head: logits = E bf16(norm(h)), with the arg-max candidates of this CTA's rows ----------------------------------
-// One CTA per SM walks its contiguous share of the table, 16 rows (32 KB) per ring stage, five stages: they fit beside a CTA
-// of the last down-projection, so the ring is full when the hidden state arrives.  A warp multiplies the 16 rows with one of
+// One CTA per SM walks its contiguous share of the table, 16 rows (32 KB) per ring stage, five stages: at batch 1 and 2 they fit
+// beside a CTA of the last down-projection (222 and 227 of 228 KB), so that the ring is full when the hidden state arrives; at
+// batch 4 and 8 (236 and 254 KB) it starts to fill when that kernel ends.  A warp multiplies the 16 rows with one of
 // 16 K chunks; 311 MB of weights at the memory rate are the whole of it (loads through registers, two 64 KB steps ahead,
-// gave 93 us instead of 49).
+// gave 93 us instead of 47).
 struct HeadArgs {
     const bf16* w;          // [V][D]
     const bf16* x;          // [B][D]
@@ -563,7 +551,8 @@ __device__ __forceinline__ void st_cluster_f32(float* p, int rank, float v) {
 // 8 1095, 2 1346; batch 2, 8100: 8 CTAs 733, 16 852), because the next projection then still finds room.  Exceptions: a few
 // positions need no split (batch 1, 30: 425, else 428-443), clusters of 16 pay their barrier only from 1200 positions on
 // (batch 1, 800: 8 CTAs 445, 16 451; 3000: 501 and 478), and the longest caches at batch 8 want two CTAs per SM (8100: 4 CTAs
-// 1577, 2 1623; 500: 604 and 592).
+// 1577, 2 1623; 500: 604 and 592).  Batch 4 is cut in four at every length, which below 48 positions is not the best (30: 471,
+// uncut 442, in two 465).
 // A sequence's pieces follow from its OWN length, so that its sums are taken in the same order whatever the others of the
 // batch hold; the clusters of a launch have the size that the longest needs (the rule does not fall with `len`), and in those of
 // a shorter sequence the ranks past its pieces add exact zeros.

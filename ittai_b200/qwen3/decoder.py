@@ -3,8 +3,8 @@
 The reference's ``Engine`` (reference ``src/ittai/qwen3/engine.py:87-187``) packs weights, owns every
 device buffer as a torch tensor and launches one persistent kernel per forward; this class keeps that
 shape for the decode loop the reference does not have: torch owns the buffers, the C-ABI library
-borrows raw pointers and the current stream, and one cooperative launch runs ``n_steps`` tokens with
-the argmax fed back on the device.
+borrows raw pointers and the current stream, and one call queues ``n_steps`` tokens with the argmax fed
+back on the device.
 """
 from __future__ import annotations
 
@@ -224,7 +224,7 @@ class Qwen3Decoder:
             if not 0 <= b < self.B:
                 raise ValueError(f"sequence {b} outside 0..{self.B - 1}")
         if todo:
-            self._prefill_rows(todo, check=False, split_k=False)     # a request's tokens must not depend on its neighbours
+            self._prefill_rows(todo, check=False, split_k=False)     # one order of sums, whatever prompts are admitted together
 
     def set_length(self, b: int, length: int) -> None:
         """Set ONE sequence's cache length (0 frees the slot for a new request)."""

@@ -82,8 +82,8 @@ class PrefillCore:
             split_k=True):
         """``tokens/pos/seq/slot``: int32 device ``[T]``; ``seqs``: int32 device ``[n, 4]``; ``kcache`` / ``vcache``: the store
         of layer 0, laid out ``[B, 8, kv_cap, 128]``, each further layer ``kv_layer`` elements behind (0: one store for all);
-        ``k_strides`` = (row, head, seq) in elements.  ``split_k=False``: a token's values do not depend on what
-        else is packed into the forward.  Queues the whole stack on the current stream with one library call."""
+        ``k_strides`` = (row, head, seq) in elements.  ``split_k=False``: sums over K in one order,
+        whatever else is packed into the forward (see ``IttaiQwen3Prefill``).  Queues the whole stack on the current stream with one library call."""
         p, w = _C.Qwen3Prefill(), self.w
         p.n_layers, p.vocab, p.tokens, p.n_seqs, p.max_q_len, p.kv_cap = self.L, w["embed"].shape[0], T, seqs.shape[0], max_q_len, kv_cap
         p.fused_rope, p.split_k, p.eps = int(self.fused_rope), int(split_k), EPS

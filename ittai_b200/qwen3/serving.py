@@ -4,7 +4,7 @@ independent prompts), so this is the serving-side counterpart of its ``embed`` b
 
 Every iteration admits waiting requests into free slots (their prompts, minus the last token, go through the tensor-core
 prefill into the slot's own cache region; the last token becomes the slot's next input), runs ``chunk`` greedy steps of
-the whole batch as ONE persistent launch, and retires requests that reached their token budget or produced their stop
+the whole batch with one call of the decode chain, and retires requests that reached their token budget or produced their stop
 id.  A slot's cache is one contiguous region of ``kv_capacity`` rows: there is no paging, a request longer than the
 capacity is refused at submission.  Idle slots decode a dummy token at position 0 (the kernel's batch is fixed); their
 output is dropped and their position is reset every iteration.

@@ -67,7 +67,8 @@ def checked_shapes(inp, n: int, S: int) -> torch.Tensor:
 
 def part_size(n: int, B: int, S: int, chain: bool) -> int:
     """Images to run for a short batch of ``n``: at least the 1024 rows from which on the chained GEMMs are used where the full
-    batch of ``B`` uses them, so that an image's result does not depend on the batch it came in."""
+    batch of ``B`` uses them: an image's result then does not depend on the batch it came in.  Without chains (fewer than 1024
+    rows in the full batch) the GEMMs may split their sums over K by the number of rows, and it does in its last bits."""
     return max(n, min(B, -(-1024 // S))) if chain else n
 
 
