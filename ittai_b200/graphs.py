@@ -18,23 +18,21 @@ class Graphs:
 
     def __init__(self, limit: int, keys: int = 256, idle: int = 256):
         self.limit, self.keys, self.idle = limit, keys, idle
-        self.seen: OrderedDict = OrderedDict()       # keys of earlier forwards, the one unused for longest first
-        self.graphs: OrderedDict = OrderedDict()     # key -> (graph, forward of its last use), likewise
+        self.seen: OrderedDict = OrderedDict()       # keys of earlier forwards without a graph, the one unused for longest first
+        self.graphs: OrderedDict = OrderedDict()     # key -> [graph, forward of its last use], likewise
         self.clock = 0
 
     def use(self, key):
         """A forward of ``key`` begins.  ``(new, graph, capture)``: whether ``key`` is unknown, its graph if it has one, and
         whether the caller is to capture one now and hand it to ``put``."""
         self.clock += 1
+        entry = self.graphs.get(key)
+        if entry is not None:
+            entry[1] = self.clock
+            self.graphs.move_to_end(key)
+            return False, entry[0], False
         new = key not in self.seen
-        self.seen[key] = True
-        self.seen.move_to_end(key)
-        if len(self.seen) > self.keys:
-            self.seen.popitem(last=False)
-        if key in self.graphs:
-            graph, _ = self.graphs.pop(key)
-            self.graphs[key] = (graph, self.clock)
-            return new, graph, False
+        self._remember(key)
         if new or self.limit < 1:
             return new, None, False
         if len(self.graphs) >= self.limit:
@@ -42,7 +40,15 @@ class Graphs:
             if self.clock - last < self.idle:
                 return new, None, False
             self.graphs.pop(oldest)
+            self._remember(oldest)
         return new, None, True
 
     def put(self, key, graph) -> None:
-        self.graphs[key] = (graph, self.clock)
+        self.graphs[key] = [graph, self.clock]
+        self.seen.pop(key, None)
+
+    def _remember(self, key) -> None:
+        self.seen[key] = True
+        self.seen.move_to_end(key)
+        if len(self.seen) > self.keys:
+            self.seen.popitem(last=False)
