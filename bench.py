@@ -110,10 +110,10 @@ SIGLIP_BATCH = 64
 
 
 def ncu_traffic_per_token():
-    """DRAM bytes (read + write) of the decode kernel per decoded token from the last ncu capture, or None.  The figures
+    """DRAM bytes (read + write) of the decode chain per decoded token from the last ncu capture, or None.  The figures
     sit in a small JSON beside the capture's summary, with the commit they were measured at: traffic grows with the
     tokens of a launch, so the bench scales the per-token figure by its own 256."""
-    path = os.path.join(ROOT, "profiles", "qwen3_decode_kernel_b1_ctx4096.traffic.json")
+    path = os.path.join(ROOT, "profiles", "qwen3_decode_chain_b1_ctx4096.traffic.json")
     try:
         t = json.load(open(path))
         return (t["dram_bytes_read"] + t["dram_bytes_write"]) / t["tokens_per_launch"], t.get("measured_at_commit")
@@ -374,7 +374,7 @@ def main():
                          "mean_kernel": kern_ms_avg * 1e3 / DECODE},
         "roofline": {"bound": "hbm", "achieved": achieved, "peak": peaks["hbm_gbs"], "unit": "GB/s",
                      "frac": achieved / peaks["hbm_gbs"], "traffic": ncu_tok * DECODE / 1e9 if ncu_tok else None,
-                     "traffic_unit": f"GB per step (ncu dram read+write of 8 tokens in the persistent decode kernel at commit {ncu_commit}, which streams the same weights and cache rows, scaled by tokens)",
+                     "traffic_unit": f"GB per step (ncu dram read+write of the decode chain's kernels over 8 tokens at commit {ncu_commit}, scaled by tokens)",
                      "peak_kind": peak_kind,
                      "frac_of_nominal_8TBs": achieved / 8000.0, "bytes_per_token": mean_bytes},
         "e2e": {"value": toks / (e2e_ms / 1e3), "unit": UNIT, "h2d_bytes_per_step": 4, "d2h_bytes_per_step": 4 * DECODE},

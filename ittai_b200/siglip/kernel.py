@@ -39,7 +39,8 @@ def resize_positions(grid: torch.Tensor, shapes, max_len: int) -> torch.Tensor:
     """Position rows of variable-resolution (NaFlex) images: the learned ``[side, side, D]`` grid resized to every image's
     ``(height, width)`` patch grid (bilinear, antialiased, in fp32), flattened row-major and padded to ``max_len`` rows with
     the image's first row, as the eager embedding module does and the reference's ``_prepare`` restates
-    (``src/ittai/siglip/kernel.py:638-649``).  ``grid``: fp32 ``[side, side, D]``; returns fp32 ``[B, max_len, D]``."""
+    (``src/ittai/siglip/kernel.py:638-649``).  ``grid``: fp32 ``[side, side, D]``; returns fp32 ``[B, max_len, D]``.  The engines
+    get these rows from ``ittai_siglip_positions``; this is the statement of it that runs anywhere."""
     g = grid.permute(2, 0, 1)[None].float()
     shapes = [tuple(int(v) for v in hw) for hw in shapes]
     out = torch.empty(len(shapes), max_len, grid.shape[-1], dtype=torch.float32, device=grid.device)
