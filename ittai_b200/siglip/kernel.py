@@ -417,6 +417,7 @@ class Siglip2Embedder:
             buf = self._staged[slot]
             if buf is None or buf.shape[1:] != px.shape[1:] or len(buf) < len(px) or buf.dtype != px.dtype:
                 buf = self._staged[slot] = torch.empty(px.shape, dtype=px.dtype, device=dev)
+                self._free[slot].record(main)              # the block may be one that work queued on this stream still uses
             buf = buf[:len(px)]
             ready = torch.cuda.Event()
             with torch.cuda.stream(self._copy_stream):

@@ -149,3 +149,27 @@ def test_more_batch_sizes_than_graphs():
             assert torch.equal(emb.embed(px[:n]), w), n
         assert sorted(eng._graphs.graphs) == [1, 2] and list(eng._full.graphs) == [5]
     eng.check()
+
+
+@gpu
+@pytest.mark.parametrize("slot", [0, 1])
+def test_a_new_staging_buffer_waits_for_the_block_s_last_user(slot):
+    """A batch larger than the ones before gets a new staging buffer.  The allocator may hand out a block that the caller has just
+    freed and that queued work still reads: the copy on the side stream must not overtake that work."""
+    from ittai_b200.siglip.kernel import Siglip2Embedder
+    emb = Siglip2Embedder(hf.build_hf(seed=0, device="cuda", n_layers=1), batch_size=16)
+    px = hf.pixels(32, seed=3).pin_memory()
+    want = emb.embed(px.cuda())
+    emb.embed(px[:1])                                      # a buffer of one image in the first slot
+    if slot == 1:
+        emb.embed(px[:16])                                 # the first slot has its full size, the second none
+    torch.cuda.synchronize()
+    torch.cuda.empty_cache()
+    mine = torch.arange(16 * 3 * 224 * 224, dtype=torch.float32, device="cuda")
+    torch.cuda._sleep(40_000_000)                          # some 20 ms
+    seen = mine * 1.0
+    ptr = mine.data_ptr()
+    del mine
+    got = emb.embed(px)
+    assert any(b.data_ptr() == ptr for b in emb._staged), "the block was not reused: the test does not test"
+    assert torch.equal(seen, torch.arange(seen.numel(), dtype=torch.float32, device="cuda")) and torch.equal(got, want)
