@@ -302,7 +302,7 @@ gemm2_chain_kernel(const __grid_constant__ ChainParams P) {
 
 void set_error(const char* fmt, ...);
 int cuda_fail(cudaError_t e, const char* what);
-int gemm_args_from_abi(const IttaiGemm* a, GemmArgs* g, CUtensorMap* tm_a, CUtensorMap* tm_b, int epi, bool any_m, int box_w);   // gemm_sm100.cu
+int gemm_args_from_abi(const IttaiGemm* a, GemmArgs* g, CUtensorMap* tm_a, CUtensorMap* tm_b, int epi, bool any_m, int box_w, int box_a);   // gemm_sm100.cu
 
 int gemm2_chain_launch(const IttaiGemm* gemms, int n, uint32_t* flags, cudaStream_t st) {
     if (!gemms || !flags || n < 1 || n > kChainMax) { set_error("a GEMM chain holds 1 to %d GEMMs and needs a flag buffer", kChainMax); return ITTAI_E_ARG; }
@@ -314,7 +314,7 @@ int gemm2_chain_launch(const IttaiGemm* gemms, int n, uint32_t* flags, cudaStrea
         if (a->m <= 128 || a->m != gemms[0].m) { set_error("every GEMM of a chain needs the same M > 128"); return ITTAI_E_ARG; }
         if (a->epi != ITTAI_EPI_NONE && a->epi != ITTAI_EPI_GELU) { set_error("a GEMM chain takes the plain and GELU epilogues only"); return ITTAI_E_ARG; }
         if (i > 0 && (a->a != gemms[i - 1].out || a->k != gemms[i - 1].n)) { set_error("GEMM %d of the chain must read GEMM %d's output as A", i, i - 1); return ITTAI_E_ARG; }
-        int rc = gemm_args_from_abi(a, &C.g[i], &C.tm_a[i], &C.tm_b[i], a->epi, false, 128);
+        int rc = gemm_args_from_abi(a, &C.g[i], &C.tm_a[i], &C.tm_b[i], a->epi, false, 128, 128);
         if (rc != ITTAI_OK) return rc;
         rc = make_tmap_bf16(&C.tm_out[i], C.g[i].out, C.g[i].M, C.g[i].N, C.g[i].ld_out, 32, 32);
         if (rc != ITTAI_OK) return rc;

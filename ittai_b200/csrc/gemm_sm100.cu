@@ -167,9 +167,9 @@ int cuda_fail(cudaError_t e, const char* what);
 
 int gemm2_bf16_launch(const CUtensorMap& tm_a, const CUtensorMap& tm_b, const GemmArgs& g, cudaStream_t st);   // gemm2_sm100.cu
 
-// Checks one IttaiGemm and turns it into kernel arguments and the operand tensor maps (`box_w`: rows of a W box).
+// Checks one IttaiGemm and turns it into kernel arguments and the operand tensor maps (`box_w`, `box_a`: rows of a box of W and of A).
 // `any_m`: folded norms, output statistics and the rotary epilogue are allowed at M <= 128 too (ITTAI_GEMM_STATIC_W).
-int gemm_args_from_abi(const IttaiGemm* a, GemmArgs* gp, CUtensorMap* tm_a, CUtensorMap* tm_b, int epi, bool any_m, int box_w) {
+int gemm_args_from_abi(const IttaiGemm* a, GemmArgs* gp, CUtensorMap* tm_a, CUtensorMap* tm_b, int epi, bool any_m, int box_w, int box_a) {
     if (!a || !a->a || !a->w || !a->out || !a->status) { set_error("null pointer in IttaiGemm"); return ITTAI_E_ARG; }
     if (a->m < 1 || a->n < GN || a->n % GN != 0 || a->k < GK || a->k % GK != 0) {
         set_error("gemm shape M=%d N=%d K=%d: N must be a multiple of %d and K of %d", a->m, a->n, a->k, GN, GK);
@@ -202,7 +202,7 @@ int gemm_args_from_abi(const IttaiGemm* a, GemmArgs* gp, CUtensorMap* tm_a, CUte
         set_error("gemm operands must be 16-byte aligned with leading dimensions that are multiples of 8");
         return ITTAI_E_ARG;
     }
-    int rc = make_tmap_bf16(tm_a, a->a, a->m, a->k, ld_a, GM);
+    int rc = make_tmap_bf16(tm_a, a->a, a->m, a->k, ld_a, box_a);
     if (rc != ITTAI_OK) return rc;
     rc = make_tmap_bf16(tm_b, a->w, a->n, a->k, ld_w, box_w);
     if (rc != ITTAI_OK) return rc;
@@ -233,15 +233,16 @@ int gemm_bf16_launch(const IttaiGemm* a, cudaStream_t st, const void* a_gain) {
     if (sm_dev != dev && cudaDeviceGetAttribute(&n_sms, cudaDevAttrMultiProcessorCount, dev) == cudaSuccess) sm_dev = dev;
     const bool static_w = a != nullptr && (a->epi & ITTAI_GEMM_STATIC_W) != 0;
     const bool split = static_w && gemm_split_wins(a->m, a->n, n_sms), pair = !split && a != nullptr && a->m > GM;
+    const int box_a = split ? gemm_split_rows(a->m, a->n, a->k, n_sms) : GM;
     CUtensorMap tm_a, tm_b;
     GemmArgs g;
-    const int rc = gemm_args_from_abi(a, &g, &tm_a, &tm_b, a ? a->epi & ~ITTAI_GEMM_STATIC_W : 0, split, split || pair ? 128 : 64);
+    const int rc = gemm_args_from_abi(a, &g, &tm_a, &tm_b, a ? a->epi & ~ITTAI_GEMM_STATIC_W : 0, split, split || pair ? 128 : 64, box_a);
     if (rc != ITTAI_OK) return rc;
     if (a_gain != nullptr) {
         if (!split || g.stats_parts <= 0 || !g.stats_rms || ((uintptr_t)a_gain & 15)) { set_error("a norm inside the GEMM needs the split-K kernel and RMS partial sums"); return ITTAI_E_ARG; }
         g.a_gain = reinterpret_cast<const bf16*>(a_gain);
     }
-    if (split) return gemm_split_launch(tm_a, tm_b, g, n_sms, st);
+    if (split) return gemm_split_launch(tm_a, tm_b, g, box_a, n_sms, st);
     if (pair) return gemm2_bf16_launch(tm_a, tm_b, g, st);
     if (attr_dev != dev) {
         const cudaError_t e = cudaFuncSetAttribute(gemm_bf16_kernel<64, 8>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)GemmCfg<64, 8>::kSmem);

@@ -12,6 +12,8 @@ struct GemmArgs;
 int gemm_normed_launch(const IttaiGemm* a, const void* gain, cudaStream_t st);
 // Whether the split-K kernel is the faster one for this shape.
 bool gemm_split_wins(int m, int n, int n_sms);
-// `tm_b`: boxes of 128 rows; W is constant (fetched ahead of the kernels that may still be running).
-int gemm_split_launch(const CUtensorMap& tm_a, const CUtensorMap& tm_b, const GemmArgs& g, int n_sms, cudaStream_t st);
+// Rows of a tile of A (32, 64 or 128), and of a box of its tensor map.
+int gemm_split_rows(int m, int n, int k, int n_sms);
+// `tm_w`: boxes of 128 rows; W is constant (fetched ahead of the kernels that may still be running).
+int gemm_split_launch(const CUtensorMap& tm_a, const CUtensorMap& tm_w, const GemmArgs& g, int tile_rows, int n_sms, cudaStream_t st);
 }  // namespace ittai

@@ -2,21 +2,32 @@
 //
 // A prompt of 23 tokens or a single image gives the persistent kernels a handful of tiles: 128 x 64 tiles of one row block
 // are 16 CTAs for N = 1024, 256 x 256 pair tiles of 196 rows are 3 pairs for N = 768, and each walks the whole K alone.
-// Such a GEMM is bound by how many SMs fetch weights and by the length of the serial chain, not by the tensor cores.  Here
-// an output tile is 128 x 128 and belongs to a cluster of up to 8 CTAs that share its K out between them:
+// Such a GEMM is bound by how many SMs fetch weights and by the length of the serial chain, not by the tensor cores.  Here an
+// output tile is 128 columns x 32, 64 or 128 token rows and belongs to a cluster of up to 8 CTAs that share its K out:
 //
-// * warp 0 (one lane) streams 128 x 64 tiles of A and W through a ring of three stages.  The W tiles of the
-//   first stages are requested BEFORE griddepcontrol.wait: the caller has declared W constant (ITTAI_GEMM_STATIC_W), and two
-//   CTAs fit an SM (97 KB each), so the next GEMM's weights arrive while this one's epilogue runs;
-// * warp 1 (one lane) issues tcgen05.mma M128 N128 K16 into 128 columns of tensor memory;
+// * the weights are the M operand of the MMA and the token rows its N, so that a few rows cost a narrow MMA and little shared
+//   memory instead of a padded 128-row operand;
+// * warp 0 (one lane) streams k-blocks of 64 columns of W and A through a ring of three or four stages.  The W tiles of the first
+//   stages are requested BEFORE griddepcontrol.wait: the caller has declared W constant (ITTAI_GEMM_STATIC_W), and two CTAs fit
+//   an SM, so the next GEMM's weights arrive while this one's epilogue runs;
+// * warp 1 (one lane) issues tcgen05.mma M128 N<rows> K16 into <rows> columns of tensor memory;
 // * with GemmArgs::a_gain the other six warps RMS-normalise each landed A tile in place (valid rows only, the rounding steps of
 //   rmsnorm_rows_kernel) before the MMAs read it: the norm's own launch, a kernel boundary and a round trip of the activations
 //   through L2 twice per layer, goes;
-// * all eight warps then copy the valid rows of the partial tile to shared memory as fp32 (the ring is free by then), the
-//   cluster meets, and the rows are dealt out over its CTAs: a warp takes a row, lane l its columns 4l .. 4l+3, adds the
-//   splits in rank order through distributed shared memory and runs the epilogue.  A row in one warp makes the head norm
-//   and the rotary partner of the QKV projection, the output statistics of a folded norm and coalesced 256-byte stores
-//   plain shuffles.
+// * a thread holds one column of the accumulator, a warp 32 neighbouring ones of every row: they are stored straight from the
+//   registers into the shared memory of the CTA that finishes the row (row r: rank r mod splits), one cluster barrier follows,
+//   and the epilogue reads only its own shared memory.  (With the partials kept where they arise, the meeting was a store, a
+//   barrier, loads through distributed shared memory at each one's latency, and a second barrier before anyone might leave);
+// * a warp takes a row, lane l its columns 4l .. 4l+3, one to four rows side by side.  A row in one warp makes the head norm and
+//   the rotary partner of the QKV projection, the output statistics of a folded norm and coalesced 256-byte stores plain
+//   shuffles.  What the epilogue reads from memory (residual, row statistics, rotary rows, bias) is requested while the
+//   accumulator fills.
+//
+// Measured on a B200 inside a CUDA graph, weights from HBM, us, the layout described in brackets (A as a 128-row M operand, one
+// row of a warp at a time, its loads behind the accumulator) -> this one, M 23 / 128 / 196 / 512: N 4096 K 1024 6.1 -> 4.7,
+// 8.5 -> 6.6, 9.0 -> 8.1; N 6144 K 1024 7.2 -> 5.4, 9.1 -> 7.9; N 1024 K 3072 6.0 -> 5.4, 8.6 -> 7.2, 9.1 -> 8.1, 12.0 -> 9.9;
+// N 768 K 768 4.4 -> 4.1, 6.4 -> 4.4, 6.7 -> 4.7, 7.6 -> 5.6; N 768 K 3072 6.0 -> 5.3, 8.9 -> 6.2, 9.9 -> 6.9, 10.9 -> 9.2.  It is
+// bound by its own chain: a kernel boundary (0.8 us), the activations through TMA, 12 to 48 dependent MMAs, one exchange.
 //
 // The tensor memory is allocated BEFORE launch_dependents: a later kernel that shares the SM can then never hold columns
 // this one still waits for (an SM holds two such CTAs, or one and an attention CTA of 256 columns, of its 512).
@@ -29,63 +40,148 @@
 
 namespace ittai {
 
-constexpr int SM_ = 128, SN = 128, SK = 64;
-constexpr int kSplitStages = 3, kSplitThreads = 256, kMaxSplit = 8;
-constexpr uint32_t kSplitA = SM_ * SK * 2, kSplitB = SN * SK * 2;
-constexpr int kPartLd = SN + 4;                                  // fp32 per row of the partial tile: 16 bytes of padding keep
-                                                                 // the row-per-thread 128-bit stores free of bank conflicts
-constexpr uint32_t kSplitSmem = kSplitStages * (kSplitA + kSplitB) + 1024 /*alignment*/ + 128 /*barriers*/ + SM_ * 4 /*row scales*/;
-static_assert(SM_ * kPartLd * 4 <= kSplitStages * (kSplitA + kSplitB), "the partial tile reuses the ring");
+constexpr int SN = 128, SK = 64;                                 // weight rows of a tile (the M of the MMA), k-block
+constexpr int kSplitThreads = 256, kMaxSplit = 8;
+constexpr uint32_t kSplitW = SN * SK * 2;
 constexpr int kNormWarps = kSplitThreads / 32 - 2;
 constexpr uint32_t kSplitSpin = 1u << 22;
-constexpr uint32_t kSplitCols = 128;
+// TN token rows (the N of the MMA).  The partials of a cluster go to the CTA that finishes the row: up to 64 rows into a buffer of
+// their own, 128 rows into the ring, once every CTA of the cluster has stopped using it (kAlias).
+template <int TN>
+struct SplitCfg {
+    static constexpr bool kAlias = TN > 64;
+    static constexpr int kStages = TN == 32 ? 4 : 3;
+    static constexpr int kRows = TN / 32;                        // output rows a warp works on side by side
+    static constexpr uint32_t kA = TN * SK * 2;
+    static constexpr uint32_t kRing = kStages * (kA + kSplitW);
+    static constexpr uint32_t kRecv = kAlias ? 0 : TN * SN * 4;
+    static constexpr uint32_t kSmem = kRing + kRecv + 1024 /*alignment*/ + 192 /*barriers*/ + TN * 4 /*row scales*/;
+    static_assert(!kAlias || TN * SN * 4 <= kRing, "the partial tiles reuse the ring");
+    static_assert(2 * (kSmem + 1024) <= 228 * 1024, "two CTAs per SM");
+};
 
-__device__ __forceinline__ void split_cluster_sync() {
-    asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
-    asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
-}
-__device__ __forceinline__ float4 ld_cluster_f4(uint32_t addr) {
+__device__ __forceinline__ void split_cluster_arrive() { asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory"); }
+__device__ __forceinline__ void split_cluster_wait() { asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory"); }
+__device__ __forceinline__ float4 lds_f4(uint32_t addr) {
     float4 v;
-    asm volatile("ld.shared::cluster.v4.f32 {%0,%1,%2,%3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "r"(addr) : "memory");
+    asm volatile("ld.shared.v4.f32 {%0,%1,%2,%3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "r"(addr) : "memory");
     return v;
 }
+__device__ __forceinline__ uint32_t split_mapa(uint32_t addr, int rank) {
+    uint32_t a;
+    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(a) : "r"(addr), "r"(rank));
+    return a;
+}
 
-// Epilogue of one row piece: lane l holds columns col0 + 4l .. + 3 of row `row` (whole warp, converged).
-__device__ __forceinline__ void split_epilogue_row(const GemmArgs& g, float (&v)[4], int row, int col0, int lane) {
+// What the epilogue of one output row needs besides the sums.  Requested while the accumulator still fills: after it, each of
+// these loads would be a round trip to L2 on the critical path of the launch.
+struct SplitRow {
+    float mean, rstd;        // folded norm
+    uint2 res;               // four residual values
+    uint2 cos, sin;          // rotary row (q and k heads)
+    bf16* cache;             // cache row of a k or v head
+};
+struct SplitCols {           // the same for every row: a lane keeps to its four columns
+    float4 bias, csum;
+    uint2 gain;
+};
+
+template <int EPI>
+__device__ __forceinline__ SplitCols split_cols(const GemmArgs& g, int col0, int lane) {
+    SplitCols k;
+    const int c = col0 + 4 * lane;
+    k.bias = g.bias != nullptr ? *reinterpret_cast<const float4*>(g.bias + c) : make_float4(0.f, 0.f, 0.f, 0.f);
+    k.csum = g.row_stats != nullptr && g.a_gain == nullptr ? *reinterpret_cast<const float4*>(g.col_sums + c) : make_float4(0.f, 0.f, 0.f, 0.f);
+    k.gain = make_uint2(0u, 0u);
+    if (EPI == ITTAI_EPI_QKROPE && col0 / ITTAI_Q3_HD < 24)
+        k.gain = *reinterpret_cast<const uint2*>(reinterpret_cast<const bf16*>(col0 / ITTAI_Q3_HD < 16 ? g.rope.qn : g.rope.kn) + 4 * lane);
+    return k;
+}
+
+// Rows row0 + u * step (u < U) below `end`; whole warp, converged.
+template <int EPI, int U>
+__device__ __forceinline__ void split_load_rows(const GemmArgs& g, SplitRow (&in)[U], int row0, int step, int end, int col0, int lane) {
+    if (g.row_stats != nullptr && g.a_gain == nullptr) {
+        if (g.stats_parts == 0) {
+#pragma unroll
+            for (int u = 0; u < U; ++u) {
+                const int row = row0 + u * step;
+                const float2 ms = row < end ? *reinterpret_cast<const float2*>(g.row_stats + 2 * (size_t)row) : make_float2(0.f, 0.f);
+                in[u].mean = ms.x; in[u].rstd = ms.y;
+            }
+        } else {
+            float2 t[U];
+#pragma unroll
+            for (int u = 0; u < U; ++u) {
+                const int row = row0 + u * step;
+                const float2* ps = reinterpret_cast<const float2*>(g.row_stats) + (size_t)row * g.stats_parts;
+                t[u] = make_float2(0.f, 0.f);
+                if (row < end) {
+                    if (lane < g.stats_parts) t[u] = ps[lane];
+                    if (lane + 32 < g.stats_parts) { const float2 w = ps[lane + 32]; t[u].x += w.x; t[u].y += w.y; }
+                }
+            }
+            const float inv_k = 1.0f / (float)(g.stats_k > 0 ? g.stats_k : g.K);
+#pragma unroll
+            for (int u = 0; u < U; ++u) {
+                const float s1 = warp_sum(t[u].x), s2 = warp_sum(t[u].y), mean = g.stats_rms ? 0.f : s1 * inv_k;
+                in[u].mean = mean;
+                in[u].rstd = rsqrtf(fmaxf(s2 * inv_k - mean * mean, 0.f) + g.stats_eps);
+            }
+        }
+    }
+    if constexpr (EPI == ITTAI_EPI_QKROPE) {
+        constexpr int HD = ITTAI_Q3_HD, NKV = ITTAI_Q3_NKV;
+        const int head = col0 / HD;
+        if (head < 24) {
+            int pos[U];
+#pragma unroll
+            for (int u = 0; u < U; ++u) pos[u] = row0 + u * step < end ? g.rope.pos[row0 + u * step] : 0;
+#pragma unroll
+            for (int u = 0; u < U; ++u) {
+                const bf16* rp = reinterpret_cast<const bf16*>(g.rope.rope) + (size_t)pos[u] * HD + 4 * (lane & 15);
+                in[u].cos = make_uint2(0u, 0u); in[u].sin = in[u].cos;
+                if (row0 + u * step < end) { in[u].cos = *reinterpret_cast<const uint2*>(rp); in[u].sin = *reinterpret_cast<const uint2*>(rp + HD / 2); }
+            }
+        }
+        if (head >= 16) {
+            bf16* cache = reinterpret_cast<bf16*>(head < 24 ? g.rope.kcache_layer : g.rope.vcache_layer);
+#pragma unroll
+            for (int u = 0; u < U; ++u) {
+                const int row = row0 + u * step;
+                in[u].cache = row < end ? cache + (((size_t)g.rope.seq[row] * NKV + (head < 24 ? head - 16 : head - 24)) * g.rope.kv_cap + g.rope.slot[row]) * HD + 4 * lane : nullptr;
+            }
+        }
+    }
+    if (g.residual != nullptr) {
+#pragma unroll
+        for (int u = 0; u < U; ++u) {
+            const int row = row0 + u * step;
+            in[u].res = row < end ? *reinterpret_cast<const uint2*>(g.residual + (size_t)row * g.ld_res + col0 + 4 * lane) : make_uint2(0u, 0u);
+        }
+    }
+}
+
+// Epilogue of one row piece: lane l holds columns col0 + 4l .. + 3 of row `row` (whole warp, converged).  `store`: the row exists
+// (uniform; rows past the end take part in the arithmetic so that the rows of a batch are one straight run of instructions).
+template <int EPI>
+__device__ __forceinline__ void split_epilogue_row(const GemmArgs& g, const SplitCols& k, const SplitRow& in, float (&v)[4], int row, bool store, int col0, int lane) {
     const int c = col0 + 4 * lane;
     if (g.row_stats != nullptr && g.a_gain == nullptr) {
-        float mean, rstd;
-        if (g.stats_parts == 0) {
-            const float2 ms = *reinterpret_cast<const float2*>(g.row_stats + 2 * (size_t)row);
-            mean = ms.x; rstd = ms.y;
-        } else {
-            const float2* ps = reinterpret_cast<const float2*>(g.row_stats) + (size_t)row * g.stats_parts;
-            float s1 = 0.f, s2 = 0.f;
-            for (int i = lane; i < g.stats_parts; i += 32) { const float2 t = ps[i]; s1 += t.x; s2 += t.y; }
-            s1 = warp_sum(s1);
-            s2 = warp_sum(s2);
-            const float inv_k = 1.0f / (float)(g.stats_k > 0 ? g.stats_k : g.K);
-            mean = g.stats_rms ? 0.f : s1 * inv_k;
-            rstd = rsqrtf(fmaxf(s2 * inv_k - mean * mean, 0.f) + g.stats_eps);
-        }
-        const float4 cs = *reinterpret_cast<const float4*>(g.col_sums + c);
-        v[0] = rstd * fmaf(-mean, cs.x, v[0]); v[1] = rstd * fmaf(-mean, cs.y, v[1]);
-        v[2] = rstd * fmaf(-mean, cs.z, v[2]); v[3] = rstd * fmaf(-mean, cs.w, v[3]);
+        v[0] = in.rstd * fmaf(-in.mean, k.csum.x, v[0]); v[1] = in.rstd * fmaf(-in.mean, k.csum.y, v[1]);
+        v[2] = in.rstd * fmaf(-in.mean, k.csum.z, v[2]); v[3] = in.rstd * fmaf(-in.mean, k.csum.w, v[3]);
     }
-    if (g.bias != nullptr) {
-        const float4 b4 = *reinterpret_cast<const float4*>(g.bias + c);
-        v[0] += b4.x; v[1] += b4.y; v[2] += b4.z; v[3] += b4.w;
-    }
-    if (g.epi == ITTAI_EPI_SWIGLU) {
+    if (g.bias != nullptr) { v[0] += k.bias.x; v[1] += k.bias.y; v[2] += k.bias.z; v[3] += k.bias.w; }
+    if constexpr (EPI == ITTAI_EPI_SWIGLU) {
         const float g0 = bf16r(v[0]), u0 = bf16r(v[1]), g1 = bf16r(v[2]), u1 = bf16r(v[3]);
-        *reinterpret_cast<uint32_t*>(g.out + (size_t)row * g.ld_out + c / 2) =
-            pack_bf16x2(bf16r(g0 / (1.0f + expf(-g0))) * u0, bf16r(g1 / (1.0f + expf(-g1))) * u1);
+        const uint32_t o = pack_bf16x2(bf16r(g0 / (1.0f + expf(-g0))) * u0, bf16r(g1 / (1.0f + expf(-g1))) * u1);
+        if (store) *reinterpret_cast<uint32_t*>(g.out + (size_t)row * g.ld_out + c / 2) = o;
         return;
     }
-    if (g.epi == ITTAI_EPI_QKROPE) {
+    if constexpr (EPI == ITTAI_EPI_QKROPE) {
         // the Linear output rounded, then (q and k heads) the head norm and the half-split rotary embedding with the rounding
         // steps of qk_rope_scatter_kernel; the partner element 64 columns away is 16 lanes away
-        constexpr int HD = ITTAI_Q3_HD, NKV = ITTAI_Q3_NKV;
+        constexpr int HD = ITTAI_Q3_HD;
         const int head = col0 / HD;
         float x[4];
 #pragma unroll
@@ -93,110 +189,107 @@ __device__ __forceinline__ void split_epilogue_row(const GemmArgs& g, float (&v)
         if (head < 24) {
             const float ss = warp_sum(fmaf(x[0], x[0], fmaf(x[1], x[1], fmaf(x[2], x[2], x[3] * x[3]))));
             const float rstd = 1.0f / sqrtf(ss * (1.0f / HD) + g.rope.eps);
-            const bf16* gain = reinterpret_cast<const bf16*>(head < 16 ? g.rope.qn : g.rope.kn) + 4 * lane;
-            const bf16* rp = reinterpret_cast<const bf16*>(g.rope.rope) + (size_t)g.rope.pos[row] * HD + 4 * (lane & 15);
-            const uint2 gw = *reinterpret_cast<const uint2*>(gain), cw = *reinterpret_cast<const uint2*>(rp), sw = *reinterpret_cast<const uint2*>(rp + HD / 2);
-            const float ga[4] = {bf_lo(gw.x), bf_hi(gw.x), bf_lo(gw.y), bf_hi(gw.y)}, cs[4] = {bf_lo(cw.x), bf_hi(cw.x), bf_lo(cw.y), bf_hi(cw.y)};
-            const float sn[4] = {bf_lo(sw.x), bf_hi(sw.x), bf_lo(sw.y), bf_hi(sw.y)};
+            const float ga[4] = {bf_lo(k.gain.x), bf_hi(k.gain.x), bf_lo(k.gain.y), bf_hi(k.gain.y)}, cs[4] = {bf_lo(in.cos.x), bf_hi(in.cos.x), bf_lo(in.cos.y), bf_hi(in.cos.y)};
+            const float sn[4] = {bf_lo(in.sin.x), bf_hi(in.sin.x), bf_lo(in.sin.y), bf_hi(in.sin.y)};
 #pragma unroll
             for (int i = 0; i < 4; ++i) {
                 const float mine = bf16r(bf16r(x[i] * rstd) * ga[i]), other = __shfl_xor_sync(0xffffffffu, mine, 16);
                 x[i] = bf16r(bf16r(mine * cs[i]) + bf16r((lane < 16 ? -other : other) * sn[i]));
             }
         }
-        bf16* dst;
-        if (head < 16) dst = g.out + (size_t)row * g.ld_out + c;
-        else {
-            bf16* cache = reinterpret_cast<bf16*>(head < 24 ? g.rope.kcache_layer : g.rope.vcache_layer);
-            dst = cache + (((size_t)g.rope.seq[row] * NKV + (head < 24 ? head - 16 : head - 24)) * g.rope.kv_cap + g.rope.slot[row]) * HD + 4 * lane;
-        }
-        *reinterpret_cast<uint2*>(dst) = make_uint2(pack_bf16x2(x[0], x[1]), pack_bf16x2(x[2], x[3]));
+        bf16* dst = head < 16 ? g.out + (size_t)row * g.ld_out + c : in.cache;
+        if (store) *reinterpret_cast<uint2*>(dst) = make_uint2(pack_bf16x2(x[0], x[1]), pack_bf16x2(x[2], x[3]));
         return;
     }
-    if (g.epi == ITTAI_EPI_GELU) {
+    if constexpr (EPI == ITTAI_EPI_GELU) {
 #pragma unroll
         for (int i = 0; i < 4; ++i) v[i] = gelu_tanh(bf16r(v[i]));
     }
     if (g.residual != nullptr) {
-        const uint2 rs = *reinterpret_cast<const uint2*>(g.residual + (size_t)row * g.ld_res + c);
-        v[0] = bf_lo(rs.x) + bf16r(v[0]); v[1] = bf_hi(rs.x) + bf16r(v[1]);
-        v[2] = bf_lo(rs.y) + bf16r(v[2]); v[3] = bf_hi(rs.y) + bf16r(v[3]);
+        v[0] = bf_lo(in.res.x) + bf16r(v[0]); v[1] = bf_hi(in.res.x) + bf16r(v[1]);
+        v[2] = bf_lo(in.res.y) + bf16r(v[2]); v[3] = bf_hi(in.res.y) + bf16r(v[3]);
     }
     const uint2 o = make_uint2(pack_bf16x2(v[0], v[1]), pack_bf16x2(v[2], v[3]));
-    *reinterpret_cast<uint2*>(g.out + (size_t)row * g.ld_out + c) = o;
+    if (store) *reinterpret_cast<uint2*>(g.out + (size_t)row * g.ld_out + c) = o;
     if (g.stats_out != nullptr) {
         const float a0 = bf_lo(o.x), a1 = bf_hi(o.x), a2 = bf_lo(o.y), a3 = bf_hi(o.y);
         const float s1 = warp_sum((a0 + a1) + (a2 + a3)), s2 = warp_sum(fmaf(a0, a0, fmaf(a1, a1, fmaf(a2, a2, a3 * a3))));
-        if (lane == 0) *reinterpret_cast<float2*>(g.stats_out + 2 * ((size_t)row * (g.N / SN) + col0 / SN)) = make_float2(s1, s2);
+        if (store && lane == 0) *reinterpret_cast<float2*>(g.stats_out + 2 * ((size_t)row * (g.N / SN) + col0 / SN)) = make_float2(s1, s2);
     }
 }
 
-// Grid (splits, N / 128, row blocks), clusters of `splits` CTAs along x.
+// Grid (splits, N / 128, row tiles of tile_rows <= TN), clusters of `splits` CTAs along x.
+template <int TN, int EPI>
 __global__ void __launch_bounds__(kSplitThreads, 2)
-gemm_split_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant__ CUtensorMap tm_b, const GemmArgs g) {
+gemm_split_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant__ CUtensorMap tm_w, const GemmArgs g, const int tile_rows, const int lg) {
+    using Cfg = SplitCfg<TN>;
+    constexpr int kStages = Cfg::kStages;
     extern __shared__ __align__(1024) unsigned char gsm_raw[];
     unsigned char* gsm = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(gsm_raw) + 1023) & ~(uintptr_t)1023);
-    unsigned char* sa = gsm;                                         // [stages][128 rows][128 B]
-    unsigned char* sb = gsm + kSplitStages * kSplitA;
-    float* part = reinterpret_cast<float*>(gsm);                     // [128][kPartLd], once the ring is idle
-    unsigned long long* bars = reinterpret_cast<unsigned long long*>(gsm + kSplitStages * (kSplitA + kSplitB));
+    unsigned char* sw = gsm;                                         // [stages][128 weight rows][128 B]
+    unsigned char* sa = gsm + kStages * kSplitW;                     // [stages][TN token rows][128 B]
+    float* part = reinterpret_cast<float*>(Cfg::kAlias ? gsm : gsm + Cfg::kRing);   // [splits][TN / splits][128]: the partials of this CTA's rows
+    unsigned long long* bars = reinterpret_cast<unsigned long long*>(gsm + Cfg::kRing + Cfg::kRecv);
     unsigned long long* full = bars;
-    unsigned long long* empty = bars + kSplitStages;
-    unsigned long long* acc_full = bars + 2 * kSplitStages;
-    unsigned long long* ready = bars + 2 * kSplitStages + 1;          // [stages] A normalised
-    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 3 * kSplitStages + 1);
-    float* scale = reinterpret_cast<float*>(bars + 16);              // [128] 1 / rms of A's rows
+    unsigned long long* empty = bars + kStages;
+    unsigned long long* acc_full = bars + 2 * kStages;
+    unsigned long long* ready = bars + 2 * kStages + 1;              // [stages] A normalised
+    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 3 * kStages + 1);
+    float* scale = reinterpret_cast<float*>(bars + 16);              // [TN] 1 / rms of A's rows
     volatile uint32_t* abort_flag = tmem_slot + 1;
+    static_assert(3 * kStages + 2 <= 16, "barriers and flags end before the row scales");
 
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int rank = blockIdx.x, splits = gridDim.x, tile_n = blockIdx.y, tile_m = blockIdx.z;
-    const int n_kb_all = g.K / SK, kb0 = n_kb_all * rank / splits, n_kb = n_kb_all * (rank + 1) / splits - kb0;   // >= 1: splits <= K / 64
-    const int rows = min(SM_, g.M - tile_m * SM_);
+    const int rank = blockIdx.x, splits = 1 << lg, tile_n = blockIdx.y, row_base = blockIdx.z * tile_rows;
+    const int n_kb_all = g.K / SK, kb0 = n_kb_all * rank >> lg, n_kb = (n_kb_all * (rank + 1) >> lg) - kb0;   // >= 1: splits <= K / 64
+    const int rows = min(tile_rows, g.M - row_base);
 
     if (threadIdx.x == 0) {
-        for (int s = 0; s < kSplitStages; ++s) { mbar_init(&full[s], 1); mbar_init(&empty[s], 1); mbar_init(&ready[s], kNormWarps); }
+        for (int s = 0; s < kStages; ++s) { mbar_init(&full[s], 1); mbar_init(&empty[s], 1); mbar_init(&ready[s], kNormWarps); }
         mbar_init(acc_full, 1);
         *abort_flag = 0;
         fence_mbar_init();
         tma_prefetch_desc(&tm_a);
-        tma_prefetch_desc(&tm_b);
+        tma_prefetch_desc(&tm_w);
     }
-    if (warp == 1) tmem_alloc(tmem_slot, kSplitCols);
+    if (warp == 1) tmem_alloc(tmem_slot, TN);
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
+    // another CTA's shared memory may be written only once that CTA runs; waited for ahead of the first write
+    if (!Cfg::kAlias && splits > 1) split_cluster_arrive();
     pdl_trigger();
     const uint32_t tmem_base = *tmem_slot;
 
     if (warp == 0) {
         if (lane == 0) {
-            const int ahead = min(kSplitStages, n_kb);
+            const int ahead = min(kStages, n_kb);
             for (int kb = 0; kb < ahead; ++kb) {
-                mbar_expect_tx(&full[kb], kSplitA + kSplitB);
-                tma_load_2d(sb + kb * kSplitB, &tm_b, (kb0 + kb) * SK, tile_n * SN, &full[kb]);
+                mbar_expect_tx(&full[kb], Cfg::kA + kSplitW);
+                tma_load_2d(sw + kb * kSplitW, &tm_w, (kb0 + kb) * SK, tile_n * SN, &full[kb]);
             }
             pdl_wait();
             for (int kb = 0; kb < n_kb && !*abort_flag; ++kb) {
-                const int s = kb % kSplitStages, use = kb / kSplitStages;
+                const int s = kb % kStages, use = kb / kStages;
                 if (use > 0 && !mbar_wait_bounded(&empty[s], (use - 1) & 1, kSplitSpin)) { *abort_flag = 1; break; }
                 if (kb >= ahead) {
-                    mbar_expect_tx(&full[s], kSplitA + kSplitB);
-                    tma_load_2d(sb + s * kSplitB, &tm_b, (kb0 + kb) * SK, tile_n * SN, &full[s]);
+                    mbar_expect_tx(&full[s], Cfg::kA + kSplitW);
+                    tma_load_2d(sw + s * kSplitW, &tm_w, (kb0 + kb) * SK, tile_n * SN, &full[s]);
                 }
-                tma_load_2d(sa + s * kSplitA, &tm_a, (kb0 + kb) * SK, tile_m * SM_, &full[s]);
+                tma_load_2d(sa + s * Cfg::kA, &tm_a, (kb0 + kb) * SK, row_base, &full[s]);
             }
         }
     } else if (warp == 1 && lane == 0) {
-        constexpr uint32_t idesc = umma_idesc_bf16(SM_, SN);
+        constexpr uint32_t idesc = umma_idesc_bf16(SN, TN);
         bool ok = true;
         for (int kb = 0; kb < n_kb; ++kb) {
-            const int s = kb % kSplitStages, use = kb / kSplitStages;
+            const int s = kb % kStages, use = kb / kStages;
             ok = mbar_wait_bounded(g.a_gain != nullptr ? &ready[s] : &full[s], use & 1, kSplitSpin) && !*abort_flag;
             if (!ok) break;
             tc_fence_after();
-            const uint64_t da = umma_desc_sw128(sa + s * kSplitA), db = umma_desc_sw128(sb + s * kSplitB);
+            const uint64_t dw = umma_desc_sw128(sw + s * kSplitW), da = umma_desc_sw128(sa + s * Cfg::kA);
 #pragma unroll
-            for (int k = 0; k < SK / 16; ++k) umma_bf16(tmem_base, da + 2 * k, db + 2 * k, idesc, (kb > 0 || k > 0) ? 1u : 0u);
+            for (int k = 0; k < SK / 16; ++k) umma_bf16(tmem_base, dw + 2 * k, da + 2 * k, idesc, (kb > 0 || k > 0) ? 1u : 0u);
             umma_commit(&empty[s]);
         }
         if (ok) umma_commit(acc_full); else *abort_flag = 1;
@@ -208,14 +301,15 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constan
         uint4 next = gains[0];
         pdl_wait();
         if (t < rows) {
-            const float2* ps = reinterpret_cast<const float2*>(g.row_stats) + (size_t)(tile_m * SM_ + t) * g.stats_parts;
+            const float2* ps = reinterpret_cast<const float2*>(g.row_stats) + (size_t)(row_base + t) * g.stats_parts;
             float ss = 0.f;
+#pragma unroll 8
             for (int i = 0; i < g.stats_parts; ++i) ss += ps[i].y;
             scale[t] = 1.0f / sqrtf(ss * (1.0f / (float)g.K) + g.stats_eps);
         }
         asm volatile("bar.sync 1, %0;" ::"n"(32 * kNormWarps) : "memory");
         for (int kb = 0; kb < n_kb; ++kb) {
-            const int s = kb % kSplitStages, use = kb / kSplitStages;
+            const int s = kb % kStages, use = kb / kStages;
             const uint4 gq = next;
             if (kb + 1 < n_kb) next = gains[8 * (kb + 1)];
             bool ok = true;
@@ -226,7 +320,7 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constan
             if (!ok) { *abort_flag = 1; break; }
             const uint32_t gw[4] = {gq.x, gq.y, gq.z, gq.w};
             for (int r = t >> 3; r < rows; r += 4 * kNormWarps) {
-                uint4* p = reinterpret_cast<uint4*>(sa + s * kSplitA + r * 128 + ((piece ^ (r & 7)) << 4));
+                uint4* p = reinterpret_cast<uint4*>(sa + s * Cfg::kA + r * 128 + ((piece ^ (r & 7)) << 4));
                 const uint4 x = *p;
                 const uint32_t xw[4] = {x.x, x.y, x.z, x.w};
                 const float rs = scale[r];
@@ -242,6 +336,12 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constan
     }
     __syncwarp();
     pdl_wait();                                                      // the epilogue reads what the kernels before wrote
+    // Row r of the tile belongs to rank r % splits and there to warp (r / splits) % 8, U of them at a time.
+    constexpr int U = Cfg::kRows;
+    const int col0 = tile_n * SN, first = rank + splits * warp, step = splits * (kSplitThreads / 32);
+    SplitRow in[U];
+    const SplitCols cols = split_cols<EPI>(g, col0, lane);
+    split_load_rows<EPI, U>(g, in, row_base + first, step, row_base + rows, col0, lane);
     bool ok = true;
     {
         uint32_t spins = 0;
@@ -252,39 +352,57 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constan
     if (!ok) *abort_flag = 1;
     __syncwarp();
     tc_fence_after();
-    // every MMA has finished, so every stage has been read: the ring becomes the partial tile.  Warp w reads TMEM lanes
-    // 32 (w % 4) .. + 31 (32 rows of the tile), the two warps of a lane quarter half of the columns each.
-    const int q = warp & 3;
-    if (ok && q * 32 < rows) {
-        float* dst = part + (size_t)(q * 32 + lane) * kPartLd + (warp >> 2) * (SN / 2);
+    if (splits > 1) {                // every CTA of the cluster runs; kAlias: and its MMAs have read its ring
+        if (Cfg::kAlias) split_cluster_arrive();
+        split_cluster_wait();
+    } else if (Cfg::kAlias) {
+        __syncthreads();
+    }
+    // Warp w reads TMEM lanes 32 (w % 4) .. + 31, one weight row = output column per thread; the two warps of a lane quarter
+    // take half of the token rows each.  A warp's store is 32 consecutive floats of one row, into the owner's buffer.
+    const int half = (warp >> 2) * (TN / 2);
+    const uint32_t src = smem_u32(part) + (uint32_t)rank * (TN >> lg) * (SN * 4) + 4u * ((warp & 3) * 32 + lane);
 #pragma unroll
-        for (int c0 = 0; c0 < SN / 2; c0 += 32) {
-            uint32_t r[32];
-            tmem_ld_32x32(tmem_base + ((uint32_t)(q * 32) << 16) + (uint32_t)((warp >> 2) * (SN / 2) + c0), r);
-            tmem_ld_wait();
+    for (int c = 0; c < TN / 2; c += 16) {
+        if (!ok || half + c >= rows) break;
+        uint32_t acc[16];
+        tmem_ld_32x16(tmem_base + ((uint32_t)((warp & 3) * 32) << 16) + half + c, acc);
+        tmem_ld_wait16(acc);
 #pragma unroll
-            for (int i = 0; i < 8; ++i) *reinterpret_cast<uint4*>(dst + c0 + 4 * i) = make_uint4(r[4 * i], r[4 * i + 1], r[4 * i + 2], r[4 * i + 3]);
+        for (int i = 0; i < 16; ++i) {
+            const int n = half + c + i;
+            if (n < rows) asm volatile("st.shared::cluster.b32 [%0], %1;" ::"r"(split_mapa(src + (uint32_t)(n >> lg) * (SN * 4), n & (splits - 1))), "r"(acc[i]) : "memory");
         }
     }
     tc_fence_before();
     __syncthreads();
-    if (warp == 1) tmem_dealloc(tmem_base, kSplitCols);
-    if (splits > 1) split_cluster_sync();
-    uint32_t base[kMaxSplit];
+    if (splits > 1) { split_cluster_arrive(); split_cluster_wait(); }
+    if (warp == 1) tmem_dealloc(tmem_base, TN);
+    const uint32_t mine = smem_u32(part) + 16u * lane;
+    for (int r0 = first; r0 < rows; r0 += U * step) {
+        if (r0 != first) split_load_rows<EPI, U>(g, in, row_base + r0, step, row_base + rows, col0, lane);
+        uint32_t off[U];
 #pragma unroll
-    for (int s = 0; s < kMaxSplit; ++s)
-        asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(base[s]) : "r"(smem_u32(part) + 16u * lane), "r"(s < splits ? s : 0));
-    const int col0 = tile_n * SN;
-    for (int r = rank + splits * warp; r < rows; r += splits * (kSplitThreads / 32)) {
-        float4 p[kMaxSplit];
+        for (int u = 0; u < U; ++u) {
+            off[u] = (uint32_t)(min(r0 + u * step, TN - 1) >> lg) * (SN * 4);      // rows past the end: whatever lies there
+        }
+        float v[U][4];
 #pragma unroll
-        for (int s = 0; s < kMaxSplit; ++s)
-            if (s < splits) p[s] = ld_cluster_f4(base[s] + (uint32_t)r * (kPartLd * 4));
-        float v[4] = {p[0].x, p[0].y, p[0].z, p[0].w};
+        for (int s = 0; s < kMaxSplit; ++s) {
+            if (s < splits) {
+                const uint32_t base = mine + (uint32_t)s * (TN >> lg) * (SN * 4);
+                float4 p[U];
 #pragma unroll
-        for (int s = 1; s < kMaxSplit; ++s)
-            if (s < splits) { v[0] += p[s].x; v[1] += p[s].y; v[2] += p[s].z; v[3] += p[s].w; }
-        split_epilogue_row(g, v, tile_m * SM_ + r, col0, lane);
+                for (int u = 0; u < U; ++u) p[u] = lds_f4(base + off[u]);
+#pragma unroll
+                for (int u = 0; u < U; ++u) {
+                    if (s == 0) { v[u][0] = p[u].x; v[u][1] = p[u].y; v[u][2] = p[u].z; v[u][3] = p[u].w; }
+                    else { v[u][0] += p[u].x; v[u][1] += p[u].y; v[u][2] += p[u].z; v[u][3] += p[u].w; }
+                }
+            }
+        }
+#pragma unroll
+        for (int u = 0; u < U; ++u) split_epilogue_row<EPI>(g, cols, in[u], v[u], row_base + r0 + u * step, r0 + u * step < rows, col0, lane);
     }
     __syncthreads();
     if (*abort_flag) {
@@ -296,7 +414,6 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constan
         }
         __syncthreads();
     }
-    if (splits > 1) split_cluster_sync();                            // no CTA leaves while another may still read its part
 }
 
 int cuda_fail(cudaError_t e, const char* what);
@@ -304,10 +421,10 @@ int cuda_fail(cudaError_t e, const char* what);
 // CTAs that share a tile's K: a power of two (clusters of 3, 5 or 7 cost 5-15 % more than the next smaller power), at least three
 // k-blocks each (12 k-blocks, 36 tiles: 7.2 us in four parts, 12.6 in eight), and two CTAs per SM at most save for a few
 // (48 tiles: 6.8 us as 192 CTAs, 7.1 as 96; 72 tiles: 10.0 us as 288 CTAs, 8.7 as 144).
-static int split_count(int tiles, int n_kb, int n_sms) {
-    int s = 1;
-    while (s < kMaxSplit && 2 * s * tiles * 4 <= 7 * n_sms && 2 * s * 3 <= n_kb) s *= 2;
-    return s;
+static int split_log2(int tiles, int n_kb, int n_sms) {
+    int lg = 0;
+    while (2 << lg <= kMaxSplit && (2 << lg) * tiles * 4 <= 7 * n_sms && (2 << lg) * 3 <= n_kb) ++lg;
+    return lg;
 }
 
 // The persistent pair kernel is the faster one as soon as a tile's K cannot be shared.  Measured on a B200 with weights from
@@ -315,19 +432,50 @@ static int split_count(int tiles, int n_kb, int n_sms) {
 // 22.2 -> 25.0; N 768 K 768 at M 196 / 1536 / 2048: 9.3 -> 5.9, 9.6 -> 8.7, 9.7 -> 11.0; N 2304 K 768 at M 512 / 784:
 // 10.1 -> 8.8, 10.2 -> 11.6.  Against 128 x 64 tiles walked by one CTA each (M <= 128): N 1024 K 3072 at M 32 / 128 18.6 -> 6.1,
 // 19.0 -> 8.3; N 768 K 768 6.2 -> 4.2, 6.9 -> 5.9.
-bool gemm_split_wins(int m, int n, int n_sms) { return m > 0 && n > 0 && 2ll * ((m + SM_ - 1) / SM_) * (n / SN) <= n_sms; }
+bool gemm_split_wins(int m, int n, int n_sms) { return m > 0 && n > 0 && 2ll * ((m + 127) / 128) * (n / SN) <= n_sms; }
 
-int gemm_split_launch(const CUtensorMap& tm_a, const CUtensorMap& tm_b, const GemmArgs& g, int n_sms, cudaStream_t st) {
+// Rows of a tile.  32 rows are the shortest chain while they cost nothing in splits and leave most SMs one CTA (N 768 K 768 at
+// M 128 / 196: 4.4 and 4.7 us against 4.7 and 4.9; N 768 K 3072 at M 128: 6.2 against 7.2; but N 2304 K 768 at M 128, two splits
+// instead of four, 5.6 against 5.2, and N 4096 K 1024 at M 64, 256 CTAs instead of 128, 5.9 against 5.6).  128 rows are
+// for a long K that smaller tiles leave too few splits for: N 1024 K 3072 at M 640 / 1024 12.4 and 12.8 against 13.5 and 14.4 (24
+// k-blocks to a CTA become 12); with 16 k-blocks left it is no matter (N 1024 K 2048: 11.0 and 11.1 against 10.5 and 11.5).
+int gemm_split_rows(int m, int n, int k, int n_sms) {
+    const int tiles_n = n / SN, n_kb = k / SK;
+    const auto tiles = [&](int tn) { return (m + tn - 1) / tn * tiles_n; };
+    const auto lg = [&](int tn) { return split_log2(tiles(tn), n_kb, n_sms); };
+    if (m <= 32 || (lg(32) == lg(64) && 3 * (tiles(32) << lg(32)) <= 4 * n_sms)) return 32;
+    const int share = n_kb >> lg(64);
+    return share > 16 && n_kb >> lg(128) < share ? 128 : 64;
+}
+
+template <int TN, int EPI>
+static cudaError_t split_launch(const CUtensorMap& tm_a, const CUtensorMap& tm_w, const GemmArgs& g, int n_sms, cudaStream_t st) {
     static thread_local int attr_dev = -1;
     int dev = 0;
     cudaGetDevice(&dev);
     if (attr_dev != dev) {
-        const cudaError_t e = cudaFuncSetAttribute(gemm_split_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSplitSmem);
-        if (e != cudaSuccess) return cuda_fail(e, "cudaFuncSetAttribute(gemm_split)");
+        const cudaError_t e = cudaFuncSetAttribute(gemm_split_kernel<TN, EPI>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SplitCfg<TN>::kSmem);
+        if (e != cudaSuccess) return e;
         attr_dev = dev;
     }
-    const int tiles_m = (g.M + SM_ - 1) / SM_, tiles_n = g.N / SN, splits = split_count(tiles_m * tiles_n, g.K / SK, n_sms);
-    const cudaError_t e = launch_pdl(gemm_split_kernel, dim3(splits, tiles_n, tiles_m), dim3(kSplitThreads), kSplitSmem, st, splits, tm_a, tm_b, g);
+    const int tiles_m = (g.M + TN - 1) / TN, tiles_n = g.N / SN, lg = split_log2(tiles_m * tiles_n, g.K / SK, n_sms);
+    // even row tiles: 196 rows are 98 and 98, not 128 and 68
+    return launch_pdl(gemm_split_kernel<TN, EPI>, dim3(1 << lg, tiles_n, tiles_m), dim3(kSplitThreads), SplitCfg<TN>::kSmem, st, 1 << lg, tm_a, tm_w, g,
+                      (g.M + tiles_m - 1) / tiles_m, lg);
+}
+template <int TN>
+static cudaError_t split_launch_epi(const CUtensorMap& tm_a, const CUtensorMap& tm_w, const GemmArgs& g, int n_sms, cudaStream_t st) {
+    switch (g.epi) {
+        case ITTAI_EPI_GELU: return split_launch<TN, ITTAI_EPI_GELU>(tm_a, tm_w, g, n_sms, st);
+        case ITTAI_EPI_SWIGLU: return split_launch<TN, ITTAI_EPI_SWIGLU>(tm_a, tm_w, g, n_sms, st);
+        case ITTAI_EPI_QKROPE: return split_launch<TN, ITTAI_EPI_QKROPE>(tm_a, tm_w, g, n_sms, st);
+        default: return split_launch<TN, ITTAI_EPI_NONE>(tm_a, tm_w, g, n_sms, st);
+    }
+}
+
+int gemm_split_launch(const CUtensorMap& tm_a, const CUtensorMap& tm_w, const GemmArgs& g, int tile_rows, int n_sms, cudaStream_t st) {
+    const cudaError_t e = tile_rows == 32 ? split_launch_epi<32>(tm_a, tm_w, g, n_sms, st) : tile_rows == 64 ? split_launch_epi<64>(tm_a, tm_w, g, n_sms, st)
+                                                                                   : split_launch_epi<128>(tm_a, tm_w, g, n_sms, st);
     return e == cudaSuccess ? ITTAI_OK : cuda_fail(e, "launch gemm_split_kernel");
 }
 

@@ -32,6 +32,25 @@ def test_split_k_plain_and_residual(m, n, k):
 
 
 @gpu
+@pytest.mark.parametrize("n,k", [(768, 768), (1024, 3072)])
+@pytest.mark.parametrize("m", [31, 32, 33, 64, 65, 97, 640, 769])
+def test_split_k_row_tiles(m, n, k):
+    """Both sides of the lines between tiles of 32, 64 and 128 rows, uneven last tiles; K = 3072 at 640 rows takes 128."""
+    from ittai_b200 import ops
+    a, w, res = _rand(m, k, seed=41), _rand(n, k, scale=0.05, seed=42), _rand(m, n, seed=43)
+    st = ops.new_status("cuda")
+    acc = a.float() @ w.float().t()
+    guard = torch.full((m + 1, n), 7.0, dtype=torch.bfloat16, device="cuda")
+    parts = torch.full((m, n // 128, 2), float("nan"), device="cuda")
+    got = ops.gemm(a, w, st, out=guard[:m], residual=res, stats_out=parts, static_w=True)
+    ops.check_status(st)
+    _check(got, res.float() + rb(acc), f"{m}x{n}x{k}", mid=acc)
+    assert (guard[m] == 7.0).all(), "a row past M was written"
+    xf = got.float().view(m, n // 128, 128)
+    assert torch.allclose(parts[..., 0], xf.sum(-1), rtol=1e-5, atol=1e-3) and torch.allclose(parts[..., 1], xf.pow(2).sum(-1), rtol=1e-5, atol=1e-3)
+
+
+@gpu
 @pytest.mark.parametrize("m", [3, 196])
 def test_split_k_activations(m):
     from ittai_b200 import _C, ops
