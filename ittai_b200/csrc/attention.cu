@@ -54,12 +54,12 @@ template <int HD, bool CAUSAL, int WARPS>
 __global__ void __launch_bounds__(WARPS * 32) attn_fwd_kernel(const AttnArgs a) {
     pdl_trigger();
     pdl_wait();
+    const int4 sinfo = a.seqs[blockIdx.z];
     constexpr int kAttnBM = 16 * WARPS, kAttnThreads = 32 * WARPS;
     // shared memory: Q tile, then two (K, V) tile pairs so that block kb+1 streams in while block kb is multiplied
     extern __shared__ __align__(128) unsigned char attn_smem[];
     bf16* sq = reinterpret_cast<bf16*>(attn_smem);
     bf16* skv = sq + kAttnBM * HD;                                    // [2][K | V][64 * HD]
-    const int4 sinfo = a.seqs[blockIdx.z];
     const int q_len = sinfo.y, kv_len = sinfo.w;
     const int qb = blockIdx.x * kAttnBM;
     if (qb >= q_len) return;

@@ -59,6 +59,7 @@ struct AttnTcArgs {
     bf16* o;
     long long o_row, o_head;
     int group, n_heads, n_items;
+    int lone;                // 1: an item is ONE query tile of a (sequence, head), two items each; 0: all its tiles
     float scale_log2;
     uint32_t* status;
 };
@@ -125,18 +126,18 @@ attn_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
             // the sequence record of an item: {first query row, queries, first key row, keys}
             auto issue_q = [&](int it, const int4& si, int mt, uint32_t tile) {      // `tile`: running tile number, picks the buffer
                 mbar_expect_tx(bar_q, 128 * 128);
-                tma_load_2d(sm + kOffQ + (tile % n_qbuf) * 16384, &tm_q, (it % a.n_heads) * kTcHD, si.x + mt * 128, bar_q);
+                tma_load_2d(sm + kOffQ + (tile % n_qbuf) * 16384, &tm_q, ((it >> a.lone) % a.n_heads) * kTcHD, si.x + mt * 128, bar_q);
             };
             auto issue_k = [&](int it, const int4& si) {
                 mbar_expect_tx(bar_k, KVBOX * 128);
-                tma_load_2d(sm + kOffK, &tm_k, ((it % a.n_heads) / a.group) * kTcHD, si.z, bar_k);
+                tma_load_2d(sm + kOffK, &tm_k, (((it >> a.lone) % a.n_heads) / a.group) * kTcHD, si.z, bar_k);
             };
             auto issue_v = [&](int it, const int4& si) {
                 mbar_expect_tx(bar_v, KVBOX * 128);
-                tma_load_2d(sm + kOffV, &tm_v, ((it % a.n_heads) / a.group) * kTcHD, si.z, bar_v);
+                tma_load_2d(sm + kOffV, &tm_v, (((it >> a.lone) % a.n_heads) / a.group) * kTcHD, si.z, bar_v);
             };
             int4 snext = make_int4(0, 0, 0, 0);
-            if (first < a.n_items) { snext = a.seqs[first / a.n_heads]; issue_q(first, snext, 0, 0u); issue_k(first, snext); issue_v(first, snext); }
+            if (first < a.n_items) { snext = a.seqs[(first >> a.lone) / a.n_heads]; issue_q(first, snext, a.lone ? first & 1 : 0, 0u); issue_k(first, snext); issue_v(first, snext); }
             const uint64_t dk = umma_desc_sw128(sm + kOffK), dv = umma_desc_sw128(sm + kOffV);
             constexpr uint32_t idesc_o = umma_idesc_bf16(128, kTcHD) | umma_idesc_b_mn;
             uint32_t tcount = 0, icount = 0;
@@ -145,17 +146,17 @@ attn_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
             for (int it = first; ok && it < a.n_items; it += stride, ++icount) {
                 const int4 sinfo = snext;
                 const bool more = it + stride < a.n_items;
-                if (more) snext = a.seqs[(it + stride) / a.n_heads];     // long before it is used
-                const int n_tiles = min(2, max(1, (sinfo.y + 127) >> 7));
+                if (more) snext = a.seqs[((it + stride) >> a.lone) / a.n_heads];     // long before it is used
+                const int mt0 = a.lone ? it & 1 : 0, mt1 = a.lone ? mt0 + 1 : min(2, max(1, (sinfo.y + 127) >> 7));
                 const int n_keys = max(16, (sinfo.w + 15) & ~15);
                 const int half = tc_half(n_keys), n_a = min(n_keys, half), n_b = n_keys - n_a;
                 const uint64_t dkb = dk + (uint64_t)((half * 128) >> 4);
                 const uint32_t idesc_a = umma_idesc_bf16(128, n_a), idesc_b = umma_idesc_bf16(128, max(n_b, 16));
                 ok = mbar_wait_abortable(bar_k, icount & 1u, abort_flag);
 #pragma unroll 1
-                for (int mt = 0; ok && mt < n_tiles; ++mt, ++tcount) {
+                for (int mt = mt0; ok && mt < mt1; ++mt, ++tcount) {
                     const uint32_t ph = tcount & 1u;
-                    const bool last = mt == n_tiles - 1;
+                    const bool last = mt == mt1 - 1;
                     ok = mbar_wait_abortable(bar_q, ph, abort_flag);
                     if (ok && tcount > 0) ok = mbar_wait_abortable(bar_free, ph ^ 1u, abort_flag);   // the tile before has read its O back
                     if (!ok) break;
@@ -173,7 +174,7 @@ attn_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
                     if (!last || more) {
                         // the next tile's Q: at once into the other buffer, or into the only one when the score MMAs have
                         // read it; the next item's K when this item's last score MMA has read K
-                        const int q_it = last ? it + stride : it, q_mt = last ? 0 : mt + 1;
+                        const int q_it = last ? it + stride : it, q_mt = last ? (a.lone ? q_it & 1 : 0) : mt + 1;
                         const int4& q_si = last ? snext : sinfo;
                         if (n_qbuf == 2u) issue_q(q_it, q_si, q_mt, tcount + 1);
                         if (n_qbuf == 1u || last) {
@@ -217,20 +218,20 @@ attn_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
         const float2 sc2 = make_float2(a.scale_log2, a.scale_log2);
         uint32_t tcount = 0, icount = 0;
         bool ok = true;
-        int4 snext = first < a.n_items ? a.seqs[first / a.n_heads] : make_int4(0, 0, 0, 0);
+        int4 snext = first < a.n_items ? a.seqs[(first >> a.lone) / a.n_heads] : make_int4(0, 0, 0, 0);
 #pragma unroll 1
         for (int it = first; ok && it < a.n_items; it += stride, ++icount) {
             const int4 sinfo = snext;
-            if (it + stride < a.n_items) snext = a.seqs[(it + stride) / a.n_heads];   // long before it is used
-            const int head = it % a.n_heads;
+            if (it + stride < a.n_items) snext = a.seqs[((it + stride) >> a.lone) / a.n_heads];   // long before it is used
+            const int head = (it >> a.lone) % a.n_heads;
             const int q_len = sinfo.y, kv_len = sinfo.w;
-            const int n_tiles = min(2, max(1, (q_len + 127) >> 7));
+            const int mt0 = a.lone ? it & 1 : 0, mt1 = a.lone ? mt0 + 1 : min(2, max(1, (q_len + 127) >> 7));
             const int n_keys = max(16, (kv_len + 15) & ~15);
             const int half = tc_half(n_keys), n_a = min(n_keys, half), n_b = n_keys - n_a;
             const int c_lo = hf * half, c_hi = c_lo + (hf ? n_b : n_a);
             const bool has = c_lo < c_hi;                    // false for half B when the sequence has at most 112 keys
 #pragma unroll 1
-            for (int mt = 0; mt < n_tiles; ++mt, ++tcount) {
+            for (int mt = mt0; mt < mt1; ++mt, ++tcount) {
                 const uint32_t ph = tcount & 1u;
                 const bool live = mt * 128 + q4 * 32 < q_len;    // a warp whose 32 rows are all padding skips the arithmetic
                 if (has) {
@@ -325,7 +326,7 @@ attn_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
                     }
                     tmem_st_wait();
                 }
-                if (mt == 0) {
+                if (mt == mt0) {
                     // keys between the sequence's end and the MMA's K extent belong to a neighbour: zero those V rows so
                     // that 0 * V stays 0 whatever they hold (V landed long ago; the wait only orders the stores behind it)
                     ok = mbar_wait_abortable(bar_v, icount & 1u, abort_flag);
@@ -441,12 +442,16 @@ int attn_tc_launch(const IttaiAttention* p, cudaStream_t st) {
     a.scale_log2 = 1.4426950408889634f / 8.0f;
     a.status = p->status;
     a.n_heads = p->n_heads;
-    a.n_items = p->n_heads * p->n_seqs;
+    // Items of one query tile where that shortens the longest group's list: a single image's 12 heads are 24 items for 296 groups,
+    // each half as long; 768 heads x images are 3 rounds of two tiles or 6 of one alike, and then K and V are loaded once for both.
+    const int whole = p->n_heads * p->n_seqs, groups = 2 * n_sms;
+    a.lone = p->max_q_len > 128 && (2 * whole + groups - 1) / groups < 2 * ((whole + groups - 1) / groups);
+    a.n_items = whole << a.lone;
     // the fewest CTAs that finish in the same number of rounds: 768 items take three rounds on 296 groups and on 256 alike,
     // and the SMs left out do not draw power (the sustained rate is power-capped)
     int grid = std::max(1, std::min(n_sms, a.n_items));
     if (a.n_items > n_sms) {
-        const int rounds = (a.n_items + 2 * n_sms - 1) / (2 * n_sms);
+        const int rounds = (a.n_items + groups - 1) / groups;
         grid = std::min(n_sms, ((a.n_items + rounds - 1) / rounds + 1) / 2);
     }
     const cudaError_t e = kv_box == 224 ? launch_pdl(attn_tc_kernel<224>, dim3(grid), dim3(kTcThreads), kTcSmem, st, 1, tq, tk, tv, a)

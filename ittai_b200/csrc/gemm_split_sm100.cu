@@ -55,7 +55,7 @@ struct SplitCfg {
     static constexpr uint32_t kA = TN * SK * 2;
     static constexpr uint32_t kRing = kStages * (kA + kSplitW);
     static constexpr uint32_t kRecv = kAlias ? 0 : TN * SN * 4;
-    static constexpr uint32_t kSmem = kRing + kRecv + 1024 /*alignment*/ + 192 /*barriers*/ + TN * 4 /*row scales*/;
+    static constexpr uint32_t kSmem = kRing + kRecv + 1024 /*alignment*/ + 192 /*barriers*/ + TN * 8 /*row statistics*/;
     static_assert(!kAlias || TN * SN * 4 <= kRing, "the partial tiles reuse the ring");
     static_assert(2 * (kSmem + 1024) <= 228 * 1024, "two CTAs per SM");
 };
@@ -73,10 +73,9 @@ __device__ __forceinline__ uint32_t split_mapa(uint32_t addr, int rank) {
     return a;
 }
 
-// What the epilogue of one output row needs besides the sums.  Requested while the accumulator still fills: after it, each of
-// these loads would be a round trip to L2 on the critical path of the launch.
+// What the epilogue of one output row needs besides the sums.  Requested by every warp as soon as the kernels before have ended,
+// ahead of its share of the main loop: behind the accumulator each of these loads is a round trip to L2 on the critical path.
 struct SplitRow {
-    float mean, rstd;        // folded norm
     uint2 res;               // four residual values
     uint2 cos, sin;          // rotary row (q and k heads)
     bf16* cache;             // cache row of a k or v head
@@ -101,42 +100,20 @@ __device__ __forceinline__ SplitCols split_cols(const GemmArgs& g, int col0, int
 // Rows row0 + u * step (u < U) below `end`; whole warp, converged.
 template <int EPI, int U>
 __device__ __forceinline__ void split_load_rows(const GemmArgs& g, SplitRow (&in)[U], int row0, int step, int end, int col0, int lane) {
-    if (g.row_stats != nullptr && g.a_gain == nullptr) {
-        if (g.stats_parts == 0) {
-#pragma unroll
-            for (int u = 0; u < U; ++u) {
-                const int row = row0 + u * step;
-                const float2 ms = row < end ? *reinterpret_cast<const float2*>(g.row_stats + 2 * (size_t)row) : make_float2(0.f, 0.f);
-                in[u].mean = ms.x; in[u].rstd = ms.y;
-            }
-        } else {
-            float2 t[U];
-#pragma unroll
-            for (int u = 0; u < U; ++u) {
-                const int row = row0 + u * step;
-                const float2* ps = reinterpret_cast<const float2*>(g.row_stats) + (size_t)row * g.stats_parts;
-                t[u] = make_float2(0.f, 0.f);
-                if (row < end) {
-                    if (lane < g.stats_parts) t[u] = ps[lane];
-                    if (lane + 32 < g.stats_parts) { const float2 w = ps[lane + 32]; t[u].x += w.x; t[u].y += w.y; }
-                }
-            }
-            const float inv_k = 1.0f / (float)(g.stats_k > 0 ? g.stats_k : g.K);
-#pragma unroll
-            for (int u = 0; u < U; ++u) {
-                const float s1 = warp_sum(t[u].x), s2 = warp_sum(t[u].y), mean = g.stats_rms ? 0.f : s1 * inv_k;
-                in[u].mean = mean;
-                in[u].rstd = rsqrtf(fmaxf(s2 * inv_k - mean * mean, 0.f) + g.stats_eps);
-            }
-        }
-    }
     if constexpr (EPI == ITTAI_EPI_QKROPE) {
         constexpr int HD = ITTAI_Q3_HD, NKV = ITTAI_Q3_NKV;
         const int head = col0 / HD;
-        if (head < 24) {
-            int pos[U];
+        int pos[U], seq[U], slot[U];
 #pragma unroll
-            for (int u = 0; u < U; ++u) pos[u] = row0 + u * step < end ? g.rope.pos[row0 + u * step] : 0;
+        for (int u = 0; u < U; ++u) {
+            const int row = row0 + u * step;
+            pos[u] = seq[u] = slot[u] = 0;
+            if (row < end) {
+                if (head < 24) pos[u] = g.rope.pos[row];
+                if (head >= 16) { seq[u] = g.rope.seq[row]; slot[u] = g.rope.slot[row]; }
+            }
+        }
+        if (head < 24) {
 #pragma unroll
             for (int u = 0; u < U; ++u) {
                 const bf16* rp = reinterpret_cast<const bf16*>(g.rope.rope) + (size_t)pos[u] * HD + 4 * (lane & 15);
@@ -147,10 +124,7 @@ __device__ __forceinline__ void split_load_rows(const GemmArgs& g, SplitRow (&in
         if (head >= 16) {
             bf16* cache = reinterpret_cast<bf16*>(head < 24 ? g.rope.kcache_layer : g.rope.vcache_layer);
 #pragma unroll
-            for (int u = 0; u < U; ++u) {
-                const int row = row0 + u * step;
-                in[u].cache = row < end ? cache + (((size_t)g.rope.seq[row] * NKV + (head < 24 ? head - 16 : head - 24)) * g.rope.kv_cap + g.rope.slot[row]) * HD + 4 * lane : nullptr;
-            }
+            for (int u = 0; u < U; ++u) in[u].cache = cache + (((size_t)seq[u] * NKV + (head < 24 ? head - 16 : head - 24)) * g.rope.kv_cap + slot[u]) * HD + 4 * lane;
         }
     }
     if (g.residual != nullptr) {
@@ -162,14 +136,29 @@ __device__ __forceinline__ void split_load_rows(const GemmArgs& g, SplitRow (&in
     }
 }
 
-// Epilogue of one row piece: lane l holds columns col0 + 4l .. + 3 of row `row` (whole warp, converged).  `store`: the row exists
+// (sum, sum of squares) of a row of A from its partial sums, eight requests at a time.
+__device__ __forceinline__ float2 split_row_sums(const GemmArgs& g, int row) {
+    const float2* ps = reinterpret_cast<const float2*>(g.row_stats) + (size_t)row * g.stats_parts;
+    float2 t = make_float2(0.f, 0.f);
+    for (int i0 = 0; i0 < g.stats_parts; i0 += 8) {
+        float2 w[8];
+#pragma unroll
+        for (int i = 0; i < 8; ++i) w[i] = i0 + i < g.stats_parts ? ps[i0 + i] : make_float2(0.f, 0.f);
+#pragma unroll
+        for (int i = 0; i < 8; ++i) { t.x += w[i].x; t.y += w[i].y; }
+    }
+    return t;
+}
+
+// Epilogue of one row piece: lane l holds columns col0 + 4l .. + 3 of row `row` (whole warp, converged).  `norm`: mean and 1 / standard
+// deviation of a folded norm.  `store`: the row exists
 // (uniform; rows past the end take part in the arithmetic so that the rows of a batch are one straight run of instructions).
 template <int EPI>
-__device__ __forceinline__ void split_epilogue_row(const GemmArgs& g, const SplitCols& k, const SplitRow& in, float (&v)[4], int row, bool store, int col0, int lane) {
+__device__ __forceinline__ void split_epilogue_row(const GemmArgs& g, const SplitCols& k, const SplitRow& in, float2 norm, float (&v)[4], int row, bool store, int col0, int lane) {
     const int c = col0 + 4 * lane;
     if (g.row_stats != nullptr && g.a_gain == nullptr) {
-        v[0] = in.rstd * fmaf(-in.mean, k.csum.x, v[0]); v[1] = in.rstd * fmaf(-in.mean, k.csum.y, v[1]);
-        v[2] = in.rstd * fmaf(-in.mean, k.csum.z, v[2]); v[3] = in.rstd * fmaf(-in.mean, k.csum.w, v[3]);
+        v[0] = norm.y * fmaf(-norm.x, k.csum.x, v[0]); v[1] = norm.y * fmaf(-norm.x, k.csum.y, v[1]);
+        v[2] = norm.y * fmaf(-norm.x, k.csum.z, v[2]); v[3] = norm.y * fmaf(-norm.x, k.csum.w, v[3]);
     }
     if (g.bias != nullptr) { v[0] += k.bias.x; v[1] += k.bias.y; v[2] += k.bias.z; v[3] += k.bias.w; }
     if constexpr (EPI == ITTAI_EPI_SWIGLU) {
@@ -235,7 +224,8 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constan
     unsigned long long* acc_full = bars + 2 * kStages;
     unsigned long long* ready = bars + 2 * kStages + 1;              // [stages] A normalised
     uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 3 * kStages + 1);
-    float* scale = reinterpret_cast<float*>(bars + 16);              // [TN] 1 / rms of A's rows
+    float* scale = reinterpret_cast<float*>(bars + 16);              // a_gain: [TN] 1 / rms of A's rows
+    float2* norm = reinterpret_cast<float2*>(bars + 16);             // folded norm: [TN / splits] mean, 1 / standard deviation of this CTA's rows
     volatile uint32_t* abort_flag = tmem_slot + 1;
     static_assert(3 * kStages + 2 <= 16, "barriers and flags end before the row scales");
 
@@ -261,52 +251,59 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constan
     pdl_trigger();
     const uint32_t tmem_base = *tmem_slot;
 
+    // Row r of the tile belongs to rank r % splits and there to warp (r / splits) % 8, U of them at a time.
+    constexpr int U = Cfg::kRows;
+    const int col0 = tile_n * SN, first = rank + splits * warp, step = splits * (kSplitThreads / 32);
+    const int ahead = min(kStages, n_kb);
+    if (warp == 0 && lane == 0) {
+        for (int kb = 0; kb < ahead; ++kb) {
+            mbar_expect_tx(&full[kb], Cfg::kA + kSplitW);
+            tma_load_2d(sw + kb * kSplitW, &tm_w, (kb0 + kb) * SK, tile_n * SN, &full[kb]);
+        }
+    }
+    __syncwarp();
+    pdl_wait();                                                      // from here on what the kernels before wrote
+    if (warp == 0 && lane == 0) {
+        for (int kb = 0; kb < ahead; ++kb) tma_load_2d(sa + kb * Cfg::kA, &tm_a, (kb0 + kb) * SK, row_base, &full[kb]);
+    }
+    __syncwarp();
+    SplitRow in[U];
+    const SplitCols cols = split_cols<EPI>(g, col0, lane);
+    split_load_rows<EPI, U>(g, in, row_base + first, step, row_base + rows, col0, lane);
+
     if (warp == 0) {
         if (lane == 0) {
-            const int ahead = min(kStages, n_kb);
-            for (int kb = 0; kb < ahead; ++kb) {
-                mbar_expect_tx(&full[kb], Cfg::kA + kSplitW);
-                tma_load_2d(sw + kb * kSplitW, &tm_w, (kb0 + kb) * SK, tile_n * SN, &full[kb]);
-            }
-            pdl_wait();
-            for (int kb = 0; kb < n_kb && !*abort_flag; ++kb) {
+            for (int kb = ahead; kb < n_kb && !*abort_flag; ++kb) {
                 const int s = kb % kStages, use = kb / kStages;
-                if (use > 0 && !mbar_wait_bounded(&empty[s], (use - 1) & 1, kSplitSpin)) { *abort_flag = 1; break; }
-                if (kb >= ahead) {
-                    mbar_expect_tx(&full[s], Cfg::kA + kSplitW);
-                    tma_load_2d(sw + s * kSplitW, &tm_w, (kb0 + kb) * SK, tile_n * SN, &full[s]);
-                }
+                if (!mbar_wait_bounded(&empty[s], (use - 1) & 1, kSplitSpin)) { *abort_flag = 1; break; }
+                mbar_expect_tx(&full[s], Cfg::kA + kSplitW);
+                tma_load_2d(sw + s * kSplitW, &tm_w, (kb0 + kb) * SK, tile_n * SN, &full[s]);
                 tma_load_2d(sa + s * Cfg::kA, &tm_a, (kb0 + kb) * SK, row_base, &full[s]);
             }
         }
-    } else if (warp == 1 && lane == 0) {
-        constexpr uint32_t idesc = umma_idesc_bf16(SN, TN);
-        bool ok = true;
-        for (int kb = 0; kb < n_kb; ++kb) {
-            const int s = kb % kStages, use = kb / kStages;
-            ok = mbar_wait_bounded(g.a_gain != nullptr ? &ready[s] : &full[s], use & 1, kSplitSpin) && !*abort_flag;
-            if (!ok) break;
-            tc_fence_after();
-            const uint64_t dw = umma_desc_sw128(sw + s * kSplitW), da = umma_desc_sw128(sa + s * Cfg::kA);
+    } else if (warp == 1) {
+        if (lane == 0) {
+            constexpr uint32_t idesc = umma_idesc_bf16(SN, TN);
+            bool ok = true;
+            for (int kb = 0; kb < n_kb; ++kb) {
+                const int s = kb % kStages, use = kb / kStages;
+                ok = mbar_wait_bounded(g.a_gain != nullptr ? &ready[s] : &full[s], use & 1, kSplitSpin) && !*abort_flag;
+                if (!ok) break;
+                tc_fence_after();
+                const uint64_t dw = umma_desc_sw128(sw + s * kSplitW), da = umma_desc_sw128(sa + s * Cfg::kA);
 #pragma unroll
-            for (int k = 0; k < SK / 16; ++k) umma_bf16(tmem_base, dw + 2 * k, da + 2 * k, idesc, (kb > 0 || k > 0) ? 1u : 0u);
-            umma_commit(&empty[s]);
+                for (int k = 0; k < SK / 16; ++k) umma_bf16(tmem_base, dw + 2 * k, da + 2 * k, idesc, (kb > 0 || k > 0) ? 1u : 0u);
+                umma_commit(&empty[s]);
+            }
+            if (ok) umma_commit(acc_full); else *abort_flag = 1;
         }
-        if (ok) umma_commit(acc_full); else *abort_flag = 1;
-    } else if (warp >= 2 && g.a_gain != nullptr) {
+    } else if (g.a_gain != nullptr) {
         // a thread keeps to one 16-byte column piece of the tiles (192 threads, eight pieces a row), so its gains are one
-        // vector per k-block; the first is fetched ahead of the wait like the weights
+        // vector per k-block
         const int t = threadIdx.x - 64, piece = t & 7;
         const uint4* gains = reinterpret_cast<const uint4*>(g.a_gain + (size_t)kb0 * SK) + piece;
         uint4 next = gains[0];
-        pdl_wait();
-        if (t < rows) {
-            const float2* ps = reinterpret_cast<const float2*>(g.row_stats) + (size_t)(row_base + t) * g.stats_parts;
-            float ss = 0.f;
-#pragma unroll 8
-            for (int i = 0; i < g.stats_parts; ++i) ss += ps[i].y;
-            scale[t] = 1.0f / sqrtf(ss * (1.0f / (float)g.K) + g.stats_eps);
-        }
+        if (t < rows) scale[t] = 1.0f / sqrtf(split_row_sums(g, row_base + t).y * (1.0f / (float)g.K) + g.stats_eps);
         asm volatile("bar.sync 1, %0;" ::"n"(32 * kNormWarps) : "memory");
         for (int kb = 0; kb < n_kb; ++kb) {
             const int s = kb % kStages, use = kb / kStages;
@@ -333,15 +330,22 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constan
             __syncwarp();
             if (lane == 0) mbar_arrive(&ready[s]);
         }
+    } else if (g.row_stats != nullptr) {
+        // a thread per row; the barrier behind the main loop hands the results to the epilogue
+        const int t = threadIdx.x - 64, row = rank + splits * t;
+        if (row < rows) {
+            float2 ms;
+            if (g.stats_parts == 0) ms = *reinterpret_cast<const float2*>(g.row_stats + 2 * (size_t)(row_base + row));
+            else {
+                const float2 ss = split_row_sums(g, row_base + row);
+                const float inv_k = 1.0f / (float)(g.stats_k > 0 ? g.stats_k : g.K);
+                ms.x = g.stats_rms ? 0.f : ss.x * inv_k;
+                ms.y = rsqrtf(fmaxf(ss.y * inv_k - ms.x * ms.x, 0.f) + g.stats_eps);
+            }
+            norm[t] = ms;
+        }
     }
     __syncwarp();
-    pdl_wait();                                                      // the epilogue reads what the kernels before wrote
-    // Row r of the tile belongs to rank r % splits and there to warp (r / splits) % 8, U of them at a time.
-    constexpr int U = Cfg::kRows;
-    const int col0 = tile_n * SN, first = rank + splits * warp, step = splits * (kSplitThreads / 32);
-    SplitRow in[U];
-    const SplitCols cols = split_cols<EPI>(g, col0, lane);
-    split_load_rows<EPI, U>(g, in, row_base + first, step, row_base + rows, col0, lane);
     bool ok = true;
     {
         uint32_t spins = 0;
@@ -379,6 +383,7 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constan
     if (splits > 1) { split_cluster_arrive(); split_cluster_wait(); }
     if (warp == 1) tmem_dealloc(tmem_base, TN);
     const uint32_t mine = smem_u32(part) + 16u * lane;
+    const bool folded = g.row_stats != nullptr && g.a_gain == nullptr;
     for (int r0 = first; r0 < rows; r0 += U * step) {
         if (r0 != first) split_load_rows<EPI, U>(g, in, row_base + r0, step, row_base + rows, col0, lane);
         uint32_t off[U];
@@ -402,7 +407,7 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constan
             }
         }
 #pragma unroll
-        for (int u = 0; u < U; ++u) split_epilogue_row<EPI>(g, cols, in[u], v[u], row_base + r0 + u * step, r0 + u * step < rows, col0, lane);
+        for (int u = 0; u < U; ++u) split_epilogue_row<EPI>(g, cols, in[u], folded ? norm[min(r0 + u * step, TN - 1) >> lg] : make_float2(0.f, 1.f), v[u], row_base + r0 + u * step, r0 + u * step < rows, col0, lane);
     }
     __syncthreads();
     if (*abort_flag) {

@@ -65,6 +65,31 @@ def test_attention_tensor_memory_kernel(lens):
 
 
 @gpu
+@pytest.mark.parametrize("longest", [224, 256])
+@pytest.mark.parametrize("n", [1, 12, 13, 20, 25, 37, 38])
+def test_attention_tensor_memory_kernel_item_lists(n, longest):
+    """Items of one query tile (1 to 12, 25 to 37 sequences of twelve heads on 148 SMs: one and several rounds) and of two, with
+    sequences whose second tile is empty."""
+    from ittai_b200 import ops
+    H, hd = 12, 64
+    lens = [(longest, 3, 130, 128, 129, 196, 64)[i % 7] for i in range(n)]
+    starts = [sum(lens[:i]) for i in range(n)]
+    rows = sum(lens)
+    qkv = _rand(rows, 3 * H * hd, seed=n)
+    out = torch.full((rows + 1, H * hd), 5.0, dtype=torch.bfloat16, device="cuda")
+    seqs = torch.tensor([[s, l, s, l] for s, l in zip(starts, lens)], dtype=torch.int32, device="cuda")
+    st = ops.new_status("cuda")
+    ops.attention(qkv, qkv[:, H * hd:], qkv[:, 2 * H * hd:], out, seqs, n_heads=H, group=1, head_dim=hd, causal=False, max_q_len=longest,
+                  q_strides=(3 * H * hd, hd), k_strides=(3 * H * hd, hd, 0), v_strides=(3 * H * hd, hd, 0), o_strides=(H * hd, hd),
+                  max_kv_len=longest, q_rows_total=rows, kv_rows_total=rows, status=st)
+    ops.check_status(st)
+    assert (out[rows] == 5.0).all()
+    for s, l in zip(starts, lens):
+        q, k, v = (qkv[s:s + l, i * H * hd:(i + 1) * H * hd].float().view(l, H, hd).transpose(0, 1) for i in range(3))
+        _check(out[s:s + l], F.scaled_dot_product_attention(q, k, v).transpose(0, 1).reshape(l, H * hd), f"{n} sequences, length {l}")
+
+
+@gpu
 @pytest.mark.parametrize("kind", ["ramp", "step"])
 @pytest.mark.parametrize("n", [196, 224, 120, 256])
 def test_attention_tensor_memory_kernel_rising_scores(n, kind):
