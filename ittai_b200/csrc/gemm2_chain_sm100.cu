@@ -15,8 +15,8 @@
 // unfinished task can always run; every wait is bounded all the same.  In-place residuals are safe under the same
 // flags: the tile of GEMM g+1 that overwrites rows of a matrix starts after every tile of GEMM g that read those rows.
 // Kernel roles, tile shape, pipeline and epilogue arithmetic are those of gemm2_bf16_kernel; residual chunks are
-// prefetched inside a tile only (the next tile may belong to a GEMM whose inputs are not complete yet), and the row
-// statistics of a folded LayerNorm are read after the accumulator is ready (their producer is then known complete).
+// prefetched inside a tile only (the next tile may belong to a GEMM whose inputs are not complete yet); they and the row
+// statistics of a folded LayerNorm are requested as soon as the producer has seen the row block complete.
 #include "gemm2_common.cuh"
 
 namespace ittai {
@@ -49,7 +49,8 @@ gemm2_chain_kernel(const __grid_constant__ ChainParams P) {
     unsigned long long* acc_full = bars + 2 * kStages2;              // [2]       MMA -> this CTA's epilogue
     unsigned long long* acc_empty = bars + 2 * kStages2 + 2;         // [2]       both epilogues -> leader's MMA
     unsigned long long* res_bars = bars + 2 * kStages2 + 4;          // [epilogue warps][2] residual chunk landed
-    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 2 * kStages2 + 4 + 2 * kEpiWarps);
+    unsigned long long* inputs = bars + 2 * kStages2 + 4 + 2 * kEpiWarps;   // [4]  the rows that tile `local` (mod 4) reads are complete
+    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(inputs + 4);
     volatile uint32_t* abort_flag = tmem_slot + 1;
 
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -72,6 +73,7 @@ gemm2_chain_kernel(const __grid_constant__ ChainParams P) {
         for (int s = 0; s < kStages2; ++s) { mbar_init(&full[s], 1); mbar_init(&empty[s], 1); }
         for (int b = 0; b < 2; ++b) { mbar_init(&acc_full[b], 1); mbar_init(&acc_empty[b], 2 * kEpiWarps); }
         for (int b = 0; b < 2 * kEpiWarps; ++b) mbar_init(&res_bars[b], 1);
+        for (int b = 0; b < 4; ++b) mbar_init(&inputs[b], 1);
         *abort_flag = 0;
         fence_mbar_init();
         tma_prefetch_desc(&P.tm_a[0]);
@@ -89,8 +91,8 @@ gemm2_chain_kernel(const __grid_constant__ ChainParams P) {
     if (warp == 0) {
         if (lane == 0) {
             // ---- TMA producer for this CTA's halves; one running k-block counter across all of the pair's tiles
-            int it = 0;
-            for (int t = pair; t < total && !*abort_flag; t += n_pairs) {
+            int it = 0, local = 0;
+            for (int t = pair; t < total && !*abort_flag; t += n_pairs, ++local) {
                 int gi, tile;
                 locate(t, gi, tile);
                 const int tiles_n = P.g[gi].N / PN, n_kb = P.g[gi].K / PK;
@@ -107,6 +109,7 @@ gemm2_chain_kernel(const __grid_constant__ ChainParams P) {
                     if (*abort_flag) break;
                     fence_proxy_async();                             // the loads below go through the async proxy
                 }
+                mbar_arrive(&inputs[local & 3]);
                 for (int kb = 0; kb < n_kb; ++kb, ++it) {
                     const int s = it % kStages2, use = it / kStages2;
                     if (use > 0 && !mbar_wait_bounded(&empty[s], (use - 1) & 1, kSpin2)) { *abort_flag = 1; break; }
@@ -177,16 +180,16 @@ gemm2_chain_kernel(const __grid_constant__ ChainParams P) {
             if (bias != nullptr && lane < kEpiCols / 4) *reinterpret_cast<float4*>(sbias + 4 * lane) = *reinterpret_cast<const float4*>(bias + col0 + 4 * lane);
             if (fold && lane < kEpiCols / 4) *reinterpret_cast<float4*>(scsum + 4 * lane) = *reinterpret_cast<const float4*>(g.col_sums + col0 + 4 * lane);
             __syncwarp();
+            // This CTA's producer has seen the row block of GEMM gi - 1 complete; take the same acquire here for the statistics and
+            // the residual this warp reads itself, so that they arrive while the accumulator fills.  (The producer is three tiles
+            // ahead at most: its next tile but two needs an accumulator that this warp has not handed back.)
             {
                 uint32_t spins = 0;
-                while (!mbar_try_wait_parked(&acc_full[buf], round & 1)) {
+                while (!mbar_try_wait_parked(&inputs[local & 3], (local >> 2) & 1)) {
                     if (((++spins) & 255u) == 0u && (*abort_flag || spins >= kSpin2)) { ok = false; break; }
                 }
             }
             if (!ok) { *abort_flag = 1; break; }
-            tc_fence_after();
-            // The accumulator exists, so this CTA's producer saw the row block of GEMM gi - 1 complete; take the same
-            // acquire here for the statistics and the residual this warp reads itself.
             if (gi > 0 && (fold || has_res)) {
                 if (lane == 0) {
                     (void)ld_acquire_gpu_u32(P.flags + (size_t)(gi - 1) * 2 * tiles_m + 2 * tile_m + rank);
@@ -209,14 +212,21 @@ gemm2_chain_kernel(const __grid_constant__ ChainParams P) {
                     mean = ms.x; rstd = ms.y;
                 } else {
                     // partial (sum, sum of squares) of the K columns in slices, added in slice order
-                    const float2* ps = reinterpret_cast<const float2*>(g.row_stats) + (size_t)(row0 + lane) * g.stats_parts;
-                    float s1 = 0.f, s2 = 0.f;
-                    for (int i = 0; i < g.stats_parts; ++i) { const float2 tt = ps[i]; s1 += tt.x; s2 += tt.y; }
+                    const float2 ss = row_sums(g, row0 + lane);
+                    const float s1 = ss.x, s2 = ss.y;
                     const float inv_k = 1.0f / (float)(g.stats_k > 0 ? g.stats_k : g.K);
                     mean = g.stats_rms ? 0.f : s1 * inv_k;
                     rstd = rsqrtf(fmaxf(s2 * inv_k - mean * mean, 0.f) + g.stats_eps);
                 }
             }
+            {
+                uint32_t spins = 0;
+                while (!mbar_try_wait_parked(&acc_full[buf], round & 1)) {
+                    if (((++spins) & 255u) == 0u && (*abort_flag || spins >= kSpin2)) { ok = false; break; }
+                }
+            }
+            if (!ok) { *abort_flag = 1; break; }
+            tc_fence_after();
             float st1 = 0.f, st2 = 0.f;                               // statistics of this row's output slice
 #pragma unroll 1
             for (uint32_t ch = 0; ch < kChunks && ok; ++ch, ++cc) {

@@ -251,9 +251,8 @@ gemm2_bf16_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constan
                         mean = ms.x; rstd = ms.y;
                     } else {
                         // partial (sum, sum of squares) of the K columns in slices, added in slice order
-                        const float2* ps = reinterpret_cast<const float2*>(g.row_stats) + (size_t)(row0 + lane) * g.stats_parts;
-                        float s1 = 0.f, s2 = 0.f;
-                        for (int i = 0; i < g.stats_parts; ++i) { const float2 t = ps[i]; s1 += t.x; s2 += t.y; }
+                        const float2 ss = row_sums(g, row0 + lane);
+                        const float s1 = ss.x, s2 = ss.y;
                         const float inv_k = 1.0f / (float)(g.stats_k > 0 ? g.stats_k : g.K);
                         mean = g.stats_rms ? 0.f : s1 * inv_k;
                         rstd = rsqrtf(fmaxf(s2 * inv_k - mean * mean, 0.f) + g.stats_eps);

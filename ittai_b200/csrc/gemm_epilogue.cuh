@@ -38,6 +38,21 @@ __device__ __forceinline__ void mbar_arrive(void* bar) {
     asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(bar)) : "memory");
 }
 
+// (sum, sum of squares) of a row of A from its partial sums, added in their order, eight requests at a time (one after the other
+// they are a round trip to L2 each).
+__device__ __forceinline__ float2 row_sums(const GemmArgs& g, int row) {
+    const float2* ps = reinterpret_cast<const float2*>(g.row_stats) + (size_t)row * g.stats_parts;
+    float2 t = make_float2(0.f, 0.f);
+    for (int i0 = 0; i0 < g.stats_parts; i0 += 8) {
+        float2 w[8];
+#pragma unroll
+        for (int i = 0; i < 8; ++i) w[i] = i0 + i < g.stats_parts ? ps[i0 + i] : make_float2(0.f, 0.f);
+#pragma unroll
+        for (int i = 0; i < 8; ++i) { t.x += w[i].x; t.y += w[i].y; }
+    }
+    return t;
+}
+
 // One 32-column slice of an accumulator row: bias, activation, residual, rounding, 128-bit stores.
 __device__ __forceinline__ void epilogue_chunk(const GemmArgs& g, const uint32_t (&r)[32], int row, int col) {
     float v[32];

@@ -136,20 +136,6 @@ __device__ __forceinline__ void split_load_rows(const GemmArgs& g, SplitRow (&in
     }
 }
 
-// (sum, sum of squares) of a row of A from its partial sums, eight requests at a time.
-__device__ __forceinline__ float2 split_row_sums(const GemmArgs& g, int row) {
-    const float2* ps = reinterpret_cast<const float2*>(g.row_stats) + (size_t)row * g.stats_parts;
-    float2 t = make_float2(0.f, 0.f);
-    for (int i0 = 0; i0 < g.stats_parts; i0 += 8) {
-        float2 w[8];
-#pragma unroll
-        for (int i = 0; i < 8; ++i) w[i] = i0 + i < g.stats_parts ? ps[i0 + i] : make_float2(0.f, 0.f);
-#pragma unroll
-        for (int i = 0; i < 8; ++i) { t.x += w[i].x; t.y += w[i].y; }
-    }
-    return t;
-}
-
 // Epilogue of one row piece: lane l holds columns col0 + 4l .. + 3 of row `row` (whole warp, converged).  `norm`: mean and 1 / standard
 // deviation of a folded norm.  `store`: the row exists
 // (uniform; rows past the end take part in the arithmetic so that the rows of a batch are one straight run of instructions).
@@ -303,7 +289,7 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constan
         const int t = threadIdx.x - 64, piece = t & 7;
         const uint4* gains = reinterpret_cast<const uint4*>(g.a_gain + (size_t)kb0 * SK) + piece;
         uint4 next = gains[0];
-        if (t < rows) scale[t] = 1.0f / sqrtf(split_row_sums(g, row_base + t).y * (1.0f / (float)g.K) + g.stats_eps);
+        if (t < rows) scale[t] = 1.0f / sqrtf(row_sums(g, row_base + t).y * (1.0f / (float)g.K) + g.stats_eps);
         asm volatile("bar.sync 1, %0;" ::"n"(32 * kNormWarps) : "memory");
         for (int kb = 0; kb < n_kb; ++kb) {
             const int s = kb % kStages, use = kb / kStages;
@@ -337,7 +323,7 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constan
             float2 ms;
             if (g.stats_parts == 0) ms = *reinterpret_cast<const float2*>(g.row_stats + 2 * (size_t)(row_base + row));
             else {
-                const float2 ss = split_row_sums(g, row_base + row);
+                const float2 ss = row_sums(g, row_base + row);
                 const float inv_k = 1.0f / (float)(g.stats_k > 0 ? g.stats_k : g.K);
                 ms.x = g.stats_rms ? 0.f : ss.x * inv_k;
                 ms.y = rsqrtf(fmaxf(ss.y * inv_k - ms.x * ms.x, 0.f) + g.stats_eps);
