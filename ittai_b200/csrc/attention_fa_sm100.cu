@@ -181,7 +181,7 @@ attn_fa_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
     const uint32_t tmem_base = *tmem_slot;
 
     if (warp == 0) {
-        if (lane == 0) {
+        if (elect_one()) {
             constexpr uint32_t idesc_s = umma_idesc_bf16(128, 128), idesc_o = umma_idesc_bf16(128, 128) | umma_idesc_b_mn;
             FaTile cur = first, nt = first;
             uint32_t c = 0, asked = 0, nq = 0;               // key blocks before this tile, questions answered, Q tiles before this one

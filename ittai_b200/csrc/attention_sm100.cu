@@ -122,7 +122,7 @@ attn_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
     const int first = blockIdx.x + grp * gridDim.x, stride = gridDim.x * 2;   // the second group only works when the items outnumber the CTAs
 
     if (warp == 0) {
-        if (lane == 0) {
+        if (elect_one()) {
             // the sequence record of an item: {first query row, queries, first key row, keys}
             auto issue_q = [&](int it, const int4& si, int mt, uint32_t tile) {      // `tile`: running tile number, picks the buffer
                 mbar_expect_tx(bar_q, 128 * 128);

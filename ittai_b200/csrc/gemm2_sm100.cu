@@ -165,7 +165,7 @@ gemm2_bf16_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constan
     const uint32_t tmem_base = *tmem_slot;
 
     if (warp == 0) {
-        if (lane == 0) {
+        if (elect_one()) {
             // ---- TMA producer for this CTA's halves; one running k-block counter across all of the pair's tiles
             int it = 0;
             for (int tile = pair; tile < n_tiles && !*abort_flag; tile += n_pairs) {
@@ -182,11 +182,11 @@ gemm2_bf16_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constan
             }
         }
     } else if (warp == 1) {
-        if (lane == 0 && rank == 0) {
+        if (rank == 0 && elect_one()) {
             // ---- MMA issuer (leader only)
             constexpr uint32_t idesc = umma_idesc_bf16(PM, PN);
             int it = 0, local = 0;
-            bool ok = true;
+            bool ok = true, next = false;
             for (int tile = pair; tile < n_tiles && ok; tile += n_pairs, ++local) {
                 const int buf = local & 1, round = local >> 1;
                 ok = (round == 0 || mbar_wait_bounded(&acc_empty[buf], (round - 1) & 1, kSpin2)) && !*abort_flag;
@@ -195,9 +195,10 @@ gemm2_bf16_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constan
                 const uint32_t d_tmem = tmem_base + (uint32_t)(buf * PN);
                 for (int kb = 0; kb < n_kb; ++kb, ++it) {
                     const int s = it % kStages2, use = it / kStages2;
-                    ok = mbar_wait_bounded(&full[s], use & 1, kSpin2) && !*abort_flag;
+                    if (!next) ok = mbar_wait_bounded(&full[s], use & 1, kSpin2) && !*abort_flag;
                     if (!ok) break;
                     tc_fence_after();
+                    next = mbar_test(&full[(it + 1) % kStages2], ((it + 1) / kStages2) & 1);
                     const uint64_t da = umma_desc_sw128(sa + s * kHalfA), db = umma_desc_sw128(sb + s * kHalfB);
 #pragma unroll
                     for (int k = 0; k < PK / 16; ++k)

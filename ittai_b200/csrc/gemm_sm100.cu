@@ -73,7 +73,7 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant
     const uint32_t tmem_base = *tmem_slot;
 
     if (warp == 0) {
-        if (lane == 0) {
+        if (elect_one()) {
             // ---- TMA producer: one running k-block counter across all of this CTA's tiles
             int it = 0;
             for (int tile = blockIdx.x; tile < n_tiles && !*abort_flag; tile += gridDim.x) {
@@ -89,11 +89,11 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant
             }
         }
     } else if (warp == 1) {
-        if (lane == 0) {
+        if (elect_one()) {
             // ---- MMA issuer
             constexpr uint32_t idesc = umma_idesc_bf16(GM, TN);
             int it = 0, local = 0;
-            bool ok = true;
+            bool ok = true, next = false;
             for (int tile = blockIdx.x; tile < n_tiles && ok; tile += gridDim.x, ++local) {
                 const int buf = local & 1, round = local >> 1;
                 // the epilogue must have drained this accumulator (passes at once on its first use)
@@ -103,9 +103,10 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant
                 const uint32_t d_tmem = tmem_base + (uint32_t)(buf * TN);
                 for (int kb = 0; kb < n_kb; ++kb, ++it) {
                     const int s = it % STAGES, use = it / STAGES;
-                    ok = mbar_wait_bounded(&full[s], use & 1, kGemmSpin) && !*abort_flag;
+                    if (!next) ok = mbar_wait_bounded(&full[s], use & 1, kGemmSpin) && !*abort_flag;
                     if (!ok) break;
                     tc_fence_after();
+                    next = mbar_test(&full[(it + 1) % STAGES], ((it + 1) / STAGES) & 1);
                     const uint64_t da = umma_desc_sw128(sa + s * kStageBytesA), db = umma_desc_sw128(sb + s * GemmCfg<TN, STAGES>::kStageBytesB);
 #pragma unroll
                     for (int k = 0; k < GK / 16; ++k)      // 16 bf16 = 32 bytes = 2 descriptor address units per step

@@ -241,7 +241,7 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constan
     constexpr int U = Cfg::kRows;
     const int col0 = tile_n * SN, first = rank + splits * warp, step = splits * (kSplitThreads / 32);
     const int ahead = min(kStages, n_kb);
-    if (warp == 0 && lane == 0) {
+    if (warp == 0 && elect_one()) {
         for (int kb = 0; kb < ahead; ++kb) {
             mbar_expect_tx(&full[kb], Cfg::kA + kSplitW);
             tma_load_2d(sw + kb * kSplitW, &tm_w, (kb0 + kb) * SK, tile_n * SN, &full[kb]);
@@ -249,7 +249,7 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constan
     }
     __syncwarp();
     pdl_wait();                                                      // from here on what the kernels before wrote
-    if (warp == 0 && lane == 0) {
+    if (warp == 0 && elect_one()) {
         for (int kb = 0; kb < ahead; ++kb) tma_load_2d(sa + kb * Cfg::kA, &tm_a, (kb0 + kb) * SK, row_base, &full[kb]);
     }
     __syncwarp();
@@ -258,7 +258,7 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constan
     split_load_rows<EPI, U>(g, in, row_base + first, step, row_base + rows, col0, lane);
 
     if (warp == 0) {
-        if (lane == 0) {
+        if (elect_one()) {
             for (int kb = ahead; kb < n_kb && !*abort_flag; ++kb) {
                 const int s = kb % kStages, use = kb / kStages;
                 if (!mbar_wait_bounded(&empty[s], (use - 1) & 1, kSplitSpin)) { *abort_flag = 1; break; }
@@ -268,14 +268,16 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constan
             }
         }
     } else if (warp == 1) {
-        if (lane == 0) {
+        if (elect_one()) {
             constexpr uint32_t idesc = umma_idesc_bf16(SN, TN);
-            bool ok = true;
+            unsigned long long* landed = g.a_gain != nullptr ? ready : full;
+            bool ok = true, next = false;
             for (int kb = 0; kb < n_kb; ++kb) {
                 const int s = kb % kStages, use = kb / kStages;
-                ok = mbar_wait_bounded(g.a_gain != nullptr ? &ready[s] : &full[s], use & 1, kSplitSpin) && !*abort_flag;
+                if (!next) ok = mbar_wait_bounded(&landed[s], use & 1, kSplitSpin) && !*abort_flag;
                 if (!ok) break;
                 tc_fence_after();
+                next = mbar_test(&landed[(kb + 1) % kStages], ((kb + 1) / kStages) & 1);
                 const uint64_t dw = umma_desc_sw128(sw + s * kSplitW), da = umma_desc_sw128(sa + s * Cfg::kA);
 #pragma unroll
                 for (int k = 0; k < SK / 16; ++k) umma_bf16(tmem_base, dw + 2 * k, da + 2 * k, idesc, (kb > 0 || k > 0) ? 1u : 0u);
