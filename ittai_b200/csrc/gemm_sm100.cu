@@ -5,9 +5,10 @@
 // GELU-tanh, SwiGLU on interleaved gate/up columns.
 //
 // This file: argument checking and dispatch (split-K kernel of gemm_split_sm100.cu: constant weights and few output tiles;
-// M > 128: the two-SM kernel of gemm2_sm100.cu), and the one-SM kernel for M <= 128 where K may not be split: it and the
-// two-SM kernel sum in the same order, so that a row's result does not depend on how many rows share the launch.  Persistent, one CTA per SM, looping over 128 x TN output tiles (tile t = blockIdx.x +
-// i * gridDim.x, N fastest, the reference's "N-tile outer, M-block inner" grouping: src/ittai/qwen3/engine.py:53-63).
+// M > 128: the two-SM kernel of gemm2_sm100.cu), and the one-SM kernel for M <= 128, and for few tiles, where K may not be split:
+// it and the two-SM kernel sum in the same order, so that a row's result does not depend on how many rows share the launch.
+// Persistent, one CTA per SM, looping over 128 x TN output tiles (tile t = blockIdx.x + i * gridDim.x, N fastest, the
+// reference's "N-tile outer, M-block inner" grouping: src/ittai/qwen3/engine.py:53-63).
 // Warp 0 (one lane) streams 128 x 64 A tiles and TN x 64 W tiles through a ring of shared-memory stages with TMA
 // (128-byte swizzle); warp 1 owns the TMEM columns as two TN-column accumulators and (one lane) issues four
 // tcgen05.mma (M128 N=TN K16) per stage, releasing the stage with tcgen05.commit; warps 2-9 read a finished
@@ -26,9 +27,8 @@ namespace ittai {
 constexpr int GM = 128, GN = 256, GK = 64;     // GN: tile width of the wide kernel and the granularity N must have
 constexpr int kGemmThreads = 320;        // TMA warp, MMA warp, 8 epilogue warps
 constexpr uint32_t kStageBytesA = GM * GK * 2;
-// Instantiated with tiles 128 x 64 and 8 stages: this kernel serves M <= 128 (larger problems go to the two-SM kernel),
-// where a GEMM has one row tile and only the number of column tiles puts CTAs to work (the MAP head: N = 768 would be 3
-// tiles of 256 columns but is 12 of 64).
+// Instantiated with tiles 128 x 64 and 8 stages: this kernel serves problems where only many tiles put SMs to work (the MAP
+// head: N = 768 would be 3 tiles of 256 columns but is 12 of 64).
 template <int TN, int STAGES>
 struct GemmCfg {
     static constexpr uint32_t kStageBytesB = TN * GK * 2;
@@ -76,12 +76,16 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant
         if (elect_one()) {
             // ---- TMA producer: one running k-block counter across all of this CTA's tiles
             int it = 0;
+            bool free = true;                                        // the next stage is known to be empty
             for (int tile = blockIdx.x; tile < n_tiles && !*abort_flag; tile += gridDim.x) {
                 const int tile_m = tile / tiles_n, tile_n = tile % tiles_n;
                 for (int kb = 0; kb < n_kb; ++kb, ++it) {
-                    const int s = it % STAGES, use = it / STAGES;
-                    if (use > 0 && !mbar_wait_bounded(&empty[s], (use - 1) & 1, kGemmSpin)) { *abort_flag = 1; break; }
-                    if (*abort_flag) break;
+                    const int s = it % STAGES;
+                    if (!free) {
+                        if (!mbar_wait_bounded(&empty[s], (it / STAGES - 1) & 1, kGemmSpin)) *abort_flag = 1;
+                        if (*abort_flag) break;
+                    }
+                    free = it + 1 < STAGES || mbar_test(&empty[(it + 1) % STAGES], ((it + 1) / STAGES - 1) & 1);
                     mbar_expect_tx(&full[s], kStageBytesA + GemmCfg<TN, STAGES>::kStageBytesB);
                     tma_load_2d(sa + s * kStageBytesA, &tm_a, kb * GK, tile_m * GM, &full[s]);
                     tma_load_2d(sb + s * GemmCfg<TN, STAGES>::kStageBytesB, &tm_b, kb * GK, tile_n * TN, &full[s]);
@@ -233,7 +237,11 @@ int gemm_bf16_launch(const IttaiGemm* a, cudaStream_t st, const void* a_gain) {
     cudaGetDevice(&dev);
     if (sm_dev != dev && cudaDeviceGetAttribute(&n_sms, cudaDevAttrMultiProcessorCount, dev) == cudaSuccess) sm_dev = dev;
     const bool static_w = a != nullptr && (a->epi & ITTAI_GEMM_STATIC_W) != 0;
-    const bool split = static_w && gemm_split_wins(a->m, a->n, n_sms), pair = !split && a != nullptr && a->m > GM;
+    const bool split = static_w && gemm_split_wins(a->m, a->n, n_sms);
+    // One-SM tiles also where they fill no more than one round of the SMs and the epilogue is one that both kernels have, value for
+    // value: 256 x 256 pair tiles leave most of the GPU idle then.  M 200 to 1152, N 1024: K 2048 14.7 -> 8.5 us, K 3072 19.3 -> 10.9.
+    const bool narrow = a != nullptr && a->epi == ITTAI_EPI_NONE && !a->row_stats && !a->stats_out && (long long)((a->m + GM - 1) / GM) * (a->n / 64) <= n_sms;
+    const bool pair = !split && a != nullptr && a->m > GM && !narrow;
     const int box_a = split ? gemm_split_rows(a->m, a->n, a->k, n_sms) : GM;
     CUtensorMap tm_a, tm_b;
     GemmArgs g;

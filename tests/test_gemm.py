@@ -37,6 +37,25 @@ def test_gemm_plain(m, n, k):
 
 
 @gpu
+@pytest.mark.parametrize("n,k", [(1024, 2048), (768, 64), (256, 3072)])
+def test_one_sm_and_two_sm_kernels_agree_bit_for_bit(n, k):
+    """A row's value does not depend on how many rows share the launch: up to one round of 128 x 64 tiles on the SMs the one-SM
+    kernel runs, above it the two-SM kernel (both sides of the line, and one row past a tile)."""
+    from ittai_b200 import ops
+    n_sms = torch.cuda.get_device_properties(0).multi_processor_count
+    last = n_sms // (n // 64) * 128
+    a, w, bias, res = _rand(last + 200, k, seed=51), _rand(n, k, scale=0.05, seed=52), _rand(n, seed=53).float(), _rand(last + 200, n, seed=54)
+    st = ops.new_status("cuda")
+    want = ops.gemm(a, w, st, bias=bias, residual=res)
+    _check(want, res.float() + (a.float() @ w.float().t() + bias).to(torch.bfloat16).float(), "two-SM", mid=a.float() @ w.float().t() + bias)
+    for m in (1, 128, 129, 300, last, last + 1):
+        guard = torch.full((m + 1, n), 3.0, dtype=torch.bfloat16, device="cuda")
+        got = ops.gemm(a[:m], w, st, bias=bias, residual=res[:m], out=guard[:m])
+        assert torch.equal(got, want[:m]) and (guard[m] == 3.0).all(), m
+    ops.check_status(st)
+
+
+@gpu
 def test_gemm_row_identity():
     """A = rows of the identity picks out columns of W: catches a wrong swizzle or K-step in the operand descriptors."""
     from ittai_b200 import ops
