@@ -52,6 +52,7 @@ struct SplitCfg {
     static constexpr bool kAlias = TN > 64;
     static constexpr int kStages = TN == 32 ? 4 : 3;
     static constexpr int kRows = TN / 32;                        // output rows a warp works on side by side
+    static constexpr int kNormGroup = TN == 32 ? 1 : TN == 64 ? 2 : 3;   // warps that normalise a k-block, other groups the next ones
     static constexpr uint32_t kA = TN * SK * 2;
     static constexpr uint32_t kRing = kStages * (kA + kSplitW);
     static constexpr uint32_t kRecv = kAlias ? 0 : TN * SN * 4;
@@ -80,6 +81,7 @@ struct SplitRow {
     uint2 cos, sin;          // rotary row (q and k heads)
     bf16* cache;             // cache row of a k or v head
 };
+struct SplitIndex { int pos, seq, slot; };
 struct SplitCols {           // the same for every row: a lane keeps to its four columns
     float4 bias, csum;
     uint2 gain;
@@ -97,26 +99,32 @@ __device__ __forceinline__ SplitCols split_cols(const GemmArgs& g, int col0, int
     return k;
 }
 
-// Rows row0 + u * step (u < U) below `end`; whole warp, converged.
+// Rows row0 + u * step (u < U) below `end`; whole warp, converged.  In two parts because the rotary rows and the cache rows hang
+// on loads of their own: what a warp does between the two is not held up by the first.
 template <int EPI, int U>
-__device__ __forceinline__ void split_load_rows(const GemmArgs& g, SplitRow (&in)[U], int row0, int step, int end, int col0, int lane) {
+__device__ __forceinline__ void split_load_index(const GemmArgs& g, SplitIndex (&ix)[U], int row0, int step, int end, int col0) {
     if constexpr (EPI == ITTAI_EPI_QKROPE) {
-        constexpr int HD = ITTAI_Q3_HD, NKV = ITTAI_Q3_NKV;
-        const int head = col0 / HD;
-        int pos[U], seq[U], slot[U];
+        const int head = col0 / ITTAI_Q3_HD;
 #pragma unroll
         for (int u = 0; u < U; ++u) {
             const int row = row0 + u * step;
-            pos[u] = seq[u] = slot[u] = 0;
+            ix[u].pos = ix[u].seq = ix[u].slot = 0;
             if (row < end) {
-                if (head < 24) pos[u] = g.rope.pos[row];
-                if (head >= 16) { seq[u] = g.rope.seq[row]; slot[u] = g.rope.slot[row]; }
+                if (head < 24) ix[u].pos = g.rope.pos[row];
+                if (head >= 16) { ix[u].seq = g.rope.seq[row]; ix[u].slot = g.rope.slot[row]; }
             }
         }
+    }
+}
+template <int EPI, int U>
+__device__ __forceinline__ void split_load_rows(const GemmArgs& g, const SplitIndex (&ix)[U], SplitRow (&in)[U], int row0, int step, int end, int col0, int lane) {
+    if constexpr (EPI == ITTAI_EPI_QKROPE) {
+        constexpr int HD = ITTAI_Q3_HD, NKV = ITTAI_Q3_NKV;
+        const int head = col0 / HD;
         if (head < 24) {
 #pragma unroll
             for (int u = 0; u < U; ++u) {
-                const bf16* rp = reinterpret_cast<const bf16*>(g.rope.rope) + (size_t)pos[u] * HD + 4 * (lane & 15);
+                const bf16* rp = reinterpret_cast<const bf16*>(g.rope.rope) + (size_t)ix[u].pos * HD + 4 * (lane & 15);
                 in[u].cos = make_uint2(0u, 0u); in[u].sin = in[u].cos;
                 if (row0 + u * step < end) { in[u].cos = *reinterpret_cast<const uint2*>(rp); in[u].sin = *reinterpret_cast<const uint2*>(rp + HD / 2); }
             }
@@ -124,7 +132,7 @@ __device__ __forceinline__ void split_load_rows(const GemmArgs& g, SplitRow (&in
         if (head >= 16) {
             bf16* cache = reinterpret_cast<bf16*>(head < 24 ? g.rope.kcache_layer : g.rope.vcache_layer);
 #pragma unroll
-            for (int u = 0; u < U; ++u) in[u].cache = cache + (((size_t)seq[u] * NKV + (head < 24 ? head - 16 : head - 24)) * g.rope.kv_cap + slot[u]) * HD + 4 * lane;
+            for (int u = 0; u < U; ++u) in[u].cache = cache + (((size_t)ix[u].seq * NKV + (head < 24 ? head - 16 : head - 24)) * g.rope.kv_cap + ix[u].slot) * HD + 4 * lane;
         }
     }
     if (g.residual != nullptr) {
@@ -221,7 +229,7 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constan
     const int rows = min(tile_rows, g.M - row_base);
 
     if (threadIdx.x == 0) {
-        for (int s = 0; s < kStages; ++s) { mbar_init(&full[s], 1); mbar_init(&empty[s], 1); mbar_init(&ready[s], kNormWarps); }
+        for (int s = 0; s < kStages; ++s) { mbar_init(&full[s], 1); mbar_init(&empty[s], 1); mbar_init(&ready[s], Cfg::kNormGroup); }
         mbar_init(acc_full, 1);
         *abort_flag = 0;
         fence_mbar_init();
@@ -248,14 +256,24 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constan
         }
     }
     __syncwarp();
+    const bool normalises = warp >= 2 && g.a_gain != nullptr;
+    // its k-blocks: group, group + kGroups, ...; a thread keeps to one 16-byte column piece (eight pieces a row), so its gains are
+    // one vector per k-block, the first of them fetched ahead of the wait like the weights
+    constexpr int kNormThreads = 32 * Cfg::kNormGroup, kGroups = kNormWarps / Cfg::kNormGroup;
+    const int group = (warp - 2) / Cfg::kNormGroup, nt = (threadIdx.x - 64) % kNormThreads, piece = nt & 7;
+    const uint4* gains = reinterpret_cast<const uint4*>(g.a_gain + (size_t)kb0 * SK) + piece;
+    uint4 gain = make_uint4(0u, 0u, 0u, 0u);
+    if (normalises && group < n_kb) gain = gains[8 * group];
     pdl_wait();                                                      // from here on what the kernels before wrote
     if (warp == 0 && elect_one()) {
         for (int kb = 0; kb < ahead; ++kb) tma_load_2d(sa + kb * Cfg::kA, &tm_a, (kb0 + kb) * SK, row_base, &full[kb]);
     }
     __syncwarp();
     SplitRow in[U];
+    SplitIndex ix[U];
+    split_load_index<EPI, U>(g, ix, row_base + first, step, row_base + rows, col0);
     const SplitCols cols = split_cols<EPI>(g, col0, lane);
-    split_load_rows<EPI, U>(g, in, row_base + first, step, row_base + rows, col0, lane);
+    if (!normalises) split_load_rows<EPI, U>(g, ix, in, row_base + first, step, row_base + rows, col0, lane);
 
     if (warp == 0) {
         if (elect_one()) {
@@ -286,17 +304,13 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constan
             if (ok) umma_commit(acc_full); else *abort_flag = 1;
         }
     } else if (g.a_gain != nullptr) {
-        // a thread keeps to one 16-byte column piece of the tiles (192 threads, eight pieces a row), so its gains are one
-        // vector per k-block
-        const int t = threadIdx.x - 64, piece = t & 7;
-        const uint4* gains = reinterpret_cast<const uint4*>(g.a_gain + (size_t)kb0 * SK) + piece;
-        uint4 next = gains[0];
+        const int t = threadIdx.x - 64;
         if (t < rows) scale[t] = 1.0f / sqrtf(row_sums(g, row_base + t).y * (1.0f / (float)g.K) + g.stats_eps);
         asm volatile("bar.sync 1, %0;" ::"n"(32 * kNormWarps) : "memory");
-        for (int kb = 0; kb < n_kb; ++kb) {
+        for (int kb = group; kb < n_kb; kb += kGroups) {
             const int s = kb % kStages, use = kb / kStages;
-            const uint4 gq = next;
-            if (kb + 1 < n_kb) next = gains[8 * (kb + 1)];
+            const uint4 gq = gain;
+            if (kb + kGroups < n_kb) gain = gains[8 * (kb + kGroups)];
             bool ok = true;
             uint32_t spins = 0;
             while (!mbar_try_wait_parked(&full[s], use & 1)) {
@@ -304,7 +318,9 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constan
             }
             if (!ok) { *abort_flag = 1; break; }
             const uint32_t gw[4] = {gq.x, gq.y, gq.z, gq.w};
-            for (int r = t >> 3; r < rows; r += 4 * kNormWarps) {
+            constexpr int kStep = kNormThreads / 8;
+#pragma unroll 4
+            for (int r = nt >> 3; r < rows; r += kStep) {
                 uint4* p = reinterpret_cast<uint4*>(sa + s * Cfg::kA + r * 128 + ((piece ^ (r & 7)) << 4));
                 const uint4 x = *p;
                 const uint32_t xw[4] = {x.x, x.y, x.z, x.w};
@@ -318,6 +334,7 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constan
             __syncwarp();
             if (lane == 0) mbar_arrive(&ready[s]);
         }
+        split_load_rows<EPI, U>(g, ix, in, row_base + first, step, row_base + rows, col0, lane);
     } else if (g.row_stats != nullptr) {
         // a thread per row; the barrier behind the main loop hands the results to the epilogue
         const int t = threadIdx.x - 64, row = rank + splits * t;
@@ -373,7 +390,10 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constan
     const uint32_t mine = smem_u32(part) + 16u * lane;
     const bool folded = g.row_stats != nullptr && g.a_gain == nullptr;
     for (int r0 = first; r0 < rows; r0 += U * step) {
-        if (r0 != first) split_load_rows<EPI, U>(g, in, row_base + r0, step, row_base + rows, col0, lane);
+        if (r0 != first) {
+            split_load_index<EPI, U>(g, ix, row_base + r0, step, row_base + rows, col0);
+            split_load_rows<EPI, U>(g, ix, in, row_base + r0, step, row_base + rows, col0, lane);
+        }
         uint32_t off[U];
 #pragma unroll
         for (int u = 0; u < U; ++u) {
