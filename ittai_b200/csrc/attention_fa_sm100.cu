@@ -7,12 +7,15 @@
 //     has completed) and every MMA: S = Q K^T (M128 N128, 8 k-steps over the 128 dims), then O += P V as one
 //     M128 N128 series whose A operand P is read from tensor memory and whose B operand V is used as loaded (MN-major:
 //     the two 64-dim swizzle atoms of the tile are one operand, 16 KB apart in the descriptor's leading-dimension field).
-//   warps 1-4: one thread per query row, no cross-thread exchange at all: row maximum over the block's 128 scores
-//     (all requested from tensor memory at once, the first 64 kept in registers for the second pass),
-//     P = 2^(s*scale - m) packed to bf16 and written back over the consumed S columns, running row sum.  The running
-//     maximum m is only raised when the block's maximum exceeds it by more than 8 (in log2 units): O in tensor memory
-//     then has to be rescaled (load, multiply, store), which is rare after the first blocks; P may exceed 1 by up to
-//     2^8 in between, harmless in bf16/fp32, and the final O / rowsum is exact either way.
+//   warps 1-8: two threads per query row, one for the first 64 keys of a block and one for the others, ONE pass over the scores:
+//     P = 2^(s*scale - ref) packed to bf16 over the consumed scores of the same half, and the half's running sum.  ref is the maximum
+//     of the row's first 16 keys, raised only when a sum passes 2^60: P, sums and O are floating point, so a reference that lags
+//     behind the maximum costs nothing, and there is no maximum to find ahead of the exponentials.  Raising is rare: the thread
+//     rescales what it has written, and a vote of the quarter's two warps, which ends every block, brings the other half and O
+//     to the same reference.  The halves' sums meet in the epilogue.
+//     (One thread a row, two passes, a maximum kept within 2^8: 175 us a layer at 8 x 2048 tokens, 135 at 64 x 512, 53 for 55 texts of
+//     16 to 512; this way 150, 119 and 46, of which the elected issuing lane gave about a quarter.  Without any softmax, the two
+//     CTAs' MMAs and hand-offs alone: 115 at 8 x 2048.)
 // TMEM (256 columns, two CTAs per SM): S / P in columns 0..127, O in 128..255.  Shared memory: Q, K, V tiles of 32 KB each
 // (two 128-byte-swizzled atoms of 64 dims); the V tile doubles as the output staging area.
 //
@@ -28,13 +31,14 @@
 
 namespace ittai {
 
-constexpr int kFaThreads = 160;
+constexpr int kFaThreads = 288;               // the issuing warp and eight softmax warps
 constexpr int kFaBlk = 128;                  // keys per block = query rows per tile = head_dim
 constexpr uint32_t kFaCols = 256, kFaOCol = 128;
 constexpr uint32_t kFaSpin = 1u << 22;
 constexpr uint32_t kFaQ = 0, kFaK = 32768, kFaV = 65536, kFaBar = 98304;
-constexpr uint32_t kFaSmem = kFaBar + 256 + 1024;
-constexpr float kFaRescale = 8.0f;           // raise the running maximum only past this gap (log2 units)
+constexpr uint32_t kFaX = kFaBar + 256;      // float [2 halves][128 rows]: what the two threads of a row tell each other
+constexpr uint32_t kFaSmem = kFaX + 1024 + 1024;
+constexpr float kFaRaise = 1.152921504606847e18f;   // 2^60: the reference is raised once a row's sum passes this
 
 struct AttnFaArgs {
     const int4* seqs;
@@ -86,6 +90,26 @@ __device__ __forceinline__ int4 fa_answer(const void* answer) {
         "}\n"
         : "+r"(id.x), "+r"(id.y), "+r"(id.z), "=r"(id.w) : "r"(smem_u32(answer)) : "memory");
     return id;
+}
+// The two warps of a lane quarter (64 threads) meet; true in both if either passes true.
+__device__ __forceinline__ bool fa_vote(int q4, bool v) {
+    uint32_t r;
+    asm volatile("{\n.reg .pred p, o;\nsetp.ne.u32 p, %1, 0;\nbarrier.cta.red.or.pred o, %2, 64, p;\nselp.u32 %0, 1, 0, o;\n}\n" : "=r"(r) : "r"((uint32_t)v), "r"(1 + q4) : "memory");
+    return r != 0;
+}
+// The first `cols` keys of this thread's P (bf16 pairs in tensor memory) times f.  Warp-wide; rare.
+__device__ __noinline__ void fa_rescale_p(uint32_t t_half, int cols, float f) {
+    tmem_st_wait();
+#pragma unroll 1
+    for (int cp = 0; cp < cols; cp += 16) {
+        uint32_t u[8];
+        tmem_ld_32x8(t_half + (uint32_t)(cp >> 1), u);
+        tmem_ld_wait();
+#pragma unroll
+        for (int i = 0; i < 8; ++i) { asm volatile("" : "+r"(u[i])); u[i] = pack_bf16x2(__uint_as_float(u[i] << 16) * f, __uint_as_float(u[i] & 0xFFFF0000u) * f); }
+        tmem_st_32x8(t_half + (uint32_t)(cp >> 1), u);
+    }
+    tmem_st_wait();
 }
 // One query tile: where it lies and how many key blocks it sees.
 struct FaTile { int head, r0, q_len, kv_len, n_blk, q_row, q_col, kv_row, kv_col; };
@@ -164,8 +188,8 @@ attn_fa_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
     volatile int* next_tile = reinterpret_cast<volatile int*>(tmem_slot + 2);    // [2] CTA index, -1: none
 
     if (threadIdx.x == 0) {
-        mbar_init(bar_q, 1); mbar_init(bar_k, 1); mbar_init(bar_v, 1); mbar_init(bar_s, 1); mbar_init(bar_p, 4); mbar_init(bar_o, 1);
-        mbar_init(bar_e, 4); mbar_init(bar_t, 1); mbar_init(bar_t + 1, 1); mbar_init(bar_c, 1);
+        mbar_init(bar_q, 1); mbar_init(bar_k, 1); mbar_init(bar_v, 1); mbar_init(bar_s, 1); mbar_init(bar_p, 8); mbar_init(bar_o, 1);
+        mbar_init(bar_e, 8); mbar_init(bar_t, 1); mbar_init(bar_t + 1, 1); mbar_init(bar_c, 1);
         *abort_flag = 0;
         fence_mbar_init();
         pdl_wait();                                        // q, k, v come from the kernels before this one
@@ -251,12 +275,12 @@ attn_fa_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
                     ok = fa_wait(bar_p, ph, abort_flag) && fa_wait(bar_v, ph, abort_flag);
                     if (!ok) break;
                     tc_fence_after();
-                    // ---- O += P V: P from tensor memory (8 columns per 16 keys), V rows 16 at a time, one series per dim half
+                    // ---- O += P V: P from tensor memory (8 columns per 16 keys, a half of the keys over its own scores), V rows 16 at a time
                     {
                         const uint64_t dv = umma_desc_sw128_mn(sm + kFaV, 16384);      // both 64-dim atoms of the V tile: N = 128
 #pragma unroll
                         for (int ks = 0; ks < 8; ++ks)
-                            umma_bf16_tmem_a(tmem_base + kFaOCol, tmem_base + 8 * ks, dv + (uint64_t)ks * (2048 >> 4), idesc_o,
+                            umma_bf16_tmem_a(tmem_base + kFaOCol, tmem_base + (ks < 4 ? 8 * ks : 64 + 8 * (ks - 4)), dv + (uint64_t)ks * (2048 >> 4), idesc_o,
                                              (j > 0 || ks > 0) ? 1u : 0u);
                     }
                     umma_commit(bar_o);
@@ -280,121 +304,138 @@ attn_fa_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
       int index = ((int)blockIdx.z * (int)gridDim.y + (int)blockIdx.y) * (int)gridDim.x + (int)blockIdx.x;
       uint32_t c = 0;                                        // key blocks before this tile
       for (int t = 0;; ++t) {
-        const int q4 = warp & 3, r = q4 * 32 + lane;         // TMEM lane quarter; query row inside the tile
+        const int q4 = warp & 3, half = (warp - 1) >> 2, r = q4 * 32 + lane;   // TMEM lane quarter; keys 64 half .. + 63 of a block; query row inside the tile
         const FaTile tile = fa_tile<HDIM>(a, index);
         const int n_blk = tile.n_blk, kv_len = tile.kv_len;
-        const uint32_t t_row = tmem_base + ((uint32_t)(q4 * 32) << 16);
+        const uint32_t t_row = tmem_base + ((uint32_t)(q4 * 32) << 16), t_half = t_row + 64 * half;
         const int row_limit = a.causal ? min(kv_len - 1, tile.r0 + r + kv_len - tile.q_len) : kv_len - 1;   // last key this row sees
-        float m_used = -INFINITY, l0 = 0.f, l1 = 0.f;       // running maximum in scaled (log2) units, running sum
+        float* xrow = reinterpret_cast<float*>(sm + kFaX) + r;       // [2 halves], 128 floats apart
+        float ref = 0.f;                                     // P = 2^(s * scale - ref); between blocks the same for both threads of a row
+        float2 l2 = make_float2(0.f, 0.f);                   // this half's sum of P, even / odd keys
         bool ok = true;
         for (int j = 0; j < n_blk; ++j) {
             const uint32_t ph = (c + j) & 1;
             ok = fa_wait(bar_s, ph, abort_flag);
-            if (!ok) break;
             tc_fence_after();
-            const int lim = row_limit - j * kFaBlk;          // columns 0..lim of this block are visible to this row
-            const bool full = __all_sync(0xffffffffu, lim >= kFaBlk - 1);
-            // ---- pass 1: the block's row maximum.  All 128 scores are requested at once (one wait instead of four round
-            //      trips to tensor memory); the first 64 stay in registers for pass 2, the others are read again there
-            //      (holding all 128 would spill: two CTAs per SM leave a thread 168 registers).
-            uint32_t sv[64], su[64];
-#pragma unroll
-            for (int c0 = 0; c0 < 64; c0 += 16) {
-                tmem_ld_32x16(t_row + c0, *reinterpret_cast<uint32_t(*)[16]>(&sv[c0]));
-                tmem_ld_32x16(t_row + 64 + c0, *reinterpret_cast<uint32_t(*)[16]>(&su[c0]));
-            }
-            tmem_ld_wait();
-#pragma unroll
-            for (int c0 = 0; c0 < 64; c0 += 16) {
-                tmem_ld_tie16(*reinterpret_cast<uint32_t(*)[16]>(&sv[c0]));
-                tmem_ld_tie16(*reinterpret_cast<uint32_t(*)[16]>(&su[c0]));
-            }
-            float mx0 = -INFINITY, mx1 = -INFINITY, mx2 = -INFINITY, mx3 = -INFINITY;
-            if (full) {
-#pragma unroll
-                for (int i = 0; i < 64; i += 4) {
-                    mx0 = fmaxf(mx0, fmaxf(__uint_as_float(sv[i]), __uint_as_float(su[i]))); mx1 = fmaxf(mx1, fmaxf(__uint_as_float(sv[i + 1]), __uint_as_float(su[i + 1])));
-                    mx2 = fmaxf(mx2, fmaxf(__uint_as_float(sv[i + 2]), __uint_as_float(su[i + 2]))); mx3 = fmaxf(mx3, fmaxf(__uint_as_float(sv[i + 3]), __uint_as_float(su[i + 3])));
-                }
-            } else {
-#pragma unroll
-                for (int i = 0; i < 64; ++i) {
-                    if (i <= lim) mx0 = fmaxf(mx0, __uint_as_float(sv[i]));
-                    if (64 + i <= lim) mx1 = fmaxf(mx1, __uint_as_float(su[i]));
-                }
-            }
-            const float bm = fmaxf(fmaxf(mx0, mx1), fmaxf(mx2, mx3)) * a.scale_log2;
-            // ---- raise the running maximum (and rescale O) only when the block exceeds it by more than the gap
             if (j == 0) {
-                m_used = bm;
-            } else {
-                const bool need = bm - m_used > kFaRescale;      // false for NaN / -inf
-                if (__any_sync(0xffffffffu, need)) {
-                    ok = fa_wait(bar_o, (c + j - 1) & 1, abort_flag);   // O must be complete before it is rewritten
-                    if (!ok) break;
-                    tc_fence_after();
-                    const float alpha = need ? fa_ex2(m_used - bm) : 1.0f;
-                    if (need) m_used = bm;
-                    l0 *= alpha; l1 *= alpha;
-#pragma unroll 1
-                    for (int c0 = 0; c0 < HDIM; c0 += 32) {
-                        uint32_t v[32];
-                        tmem_ld_32x32(t_row + kFaOCol + c0, v);
-                        tmem_ld_wait();
+                // both threads of a row start from the maximum of its first 16 keys; the vote keeps half 0 from writing P over them
+                if (ok) {
+                    uint32_t v[16];
+                    tmem_ld_32x16(t_row, v);
+                    tmem_ld_wait16(v);
+                    float m = -INFINITY;
 #pragma unroll
-                        for (int i = 0; i < 32; ++i) v[i] = __float_as_uint(__uint_as_float(v[i]) * alpha);
-#pragma unroll
-                        for (int i = 0; i < 32; i += 8) {
-                            const uint32_t w[8] = {v[i], v[i + 1], v[i + 2], v[i + 3], v[i + 4], v[i + 5], v[i + 6], v[i + 7]};
-                            tmem_st_32x8(t_row + kFaOCol + c0 + i, w);
-                        }
-                    }
+                    for (int i = 0; i < 16; ++i) if (i <= row_limit) m = fmaxf(m, __uint_as_float(v[i]));
+                    ref = m == -INFINITY ? 0.f : m * a.scale_log2;
                 }
+                if (fa_vote(q4, !ok)) { ok = false; break; }
             }
-            const float mb = m_used == -INFINITY ? 0.f : m_used;
-            // ---- pass 2: p = 2^(s * scale - m), row sum, packed bf16 P over the consumed S columns
-            auto emit_p = [&](uint32_t (&v)[16], int c0) {
-                uint32_t w[8];
+            const float ref0 = ref;
+            if (ok) {
+                const int lim = row_limit - j * kFaBlk - 64 * half;  // columns 0..lim of this half are visible to this row
+                const bool full = __all_sync(0xffffffffu, lim >= 63);
+                auto emit_p = [&](uint32_t (&v)[16], int c0) {
+                    uint32_t w[8];
+                    if (!full && !__any_sync(0xffffffffu, c0 <= lim)) {      // no row of the warp sees these keys
 #pragma unroll
-                for (int i = 0; i < 16; i += 2) {
-                    float p0 = fa_ex2(fmaf(__uint_as_float(v[i]), a.scale_log2, -mb));
-                    float p1 = fa_ex2(fmaf(__uint_as_float(v[i + 1]), a.scale_log2, -mb));
-                    if (!full) { p0 = c0 + i <= lim ? p0 : 0.f; p1 = c0 + i + 1 <= lim ? p1 : 0.f; }
-                    l0 += p0; l1 += p1;
-                    w[i >> 1] = pack_bf16x2_alu(p0, p1);
-                }
-                tmem_st_32x8(t_row + (c0 >> 1), w);
-            };
-            {
-                // the second half of the scores is on its way again while the first half, still in registers, is worked on
+                        for (int i = 0; i < 8; ++i) w[i] = 0u;
+                        tmem_st_32x8(t_half + (uint32_t)(c0 >> 1), w);
+                        return;
+                    }
+                    float2 p[8], cs;
+                    auto exps = [&]() {
+                        const float2 nr = make_float2(-ref, -ref), sc2 = make_float2(a.scale_log2, a.scale_log2);
+#pragma unroll
+                        for (int i = 0; i < 8; ++i) {
+                            const float2 t = __ffma2_rn(make_float2(__uint_as_float(v[2 * i]), __uint_as_float(v[2 * i + 1])), sc2, nr);
+                            p[i] = make_float2(fa_ex2(t.x), fa_ex2(t.y));
+                        }
+                        if (!full) {
+#pragma unroll
+                            for (int i = 0; i < 8; ++i) { if (c0 + 2 * i > lim) p[i].x = 0.f; if (c0 + 2 * i + 1 > lim) p[i].y = 0.f; }
+                        }
+                        cs = __fadd2_rn(__fadd2_rn(__fadd2_rn(p[0], p[1]), __fadd2_rn(p[2], p[3])), __fadd2_rn(__fadd2_rn(p[4], p[5]), __fadd2_rn(p[6], p[7])));
+                    };
+                    auto store_p = [&]() {
+#pragma unroll
+                        for (int i = 0; i < 8; ++i) w[i] = pack_bf16x2(p[i].x, p[i].y);
+                        tmem_st_32x8(t_half + (uint32_t)(c0 >> 1), w);
+                    };
+                    exps();
+                    store_p();
+                    // The reference lags behind the maximum: sums and P are floating point, so nothing is lost until a sum passes
+                    // 2^60 (or is infinite).  Then this thread's reference is raised to the chunk's maximum (by a whole number, so
+                    // that rescaling is exact), what it has written of this block is rescaled, and the chunk written again; the
+                    // other half and O follow after the block.
+                    const bool raise = (l2.x + l2.y) + (cs.x + cs.y) > kFaRaise;
+                    if (__any_sync(0xffffffffu, raise)) {
+                        float m = -INFINITY;
+#pragma unroll
+                        for (int i = 0; i < 16; ++i) if (c0 + i <= lim) m = fmaxf(m, __uint_as_float(v[i]));
+                        const float nref = raise ? ref + ceilf(fmaxf(fmaf(m, a.scale_log2, -ref), 0.f)) : ref, f = fa_ex2(ref - nref);
+                        l2.x *= f; l2.y *= f;
+                        fa_rescale_p(t_half, c0, f);
+                        ref = nref;
+                        exps();
+                        store_p();
+                    }
+                    l2 = __fadd2_rn(l2, cs);
+                };
+                // sixteen scores at a time, the next sixteen on their way
                 uint32_t va[16], vb[16];
-                tmem_ld_32x16(t_row + 64, va);
-                tmem_ld_32x16(t_row + 80, vb);
+                tmem_ld_32x16(t_half, va);
 #pragma unroll
-                for (int c0 = 0; c0 < 64; c0 += 16) emit_p(*reinterpret_cast<uint32_t(*)[16]>(&sv[c0]), c0);
-                tmem_ld_wait16(va);
-                tmem_ld_tie16(vb);
-                emit_p(va, 64);
-                tmem_ld_32x16(t_row + 96, va);
-                emit_p(vb, 80);
-                tmem_ld_32x16(t_row + 112, vb);
-                tmem_ld_wait16(va);
-                tmem_ld_tie16(vb);
-                emit_p(va, 96);
-                emit_p(vb, 112);
+                for (int c0 = 0; c0 < 64; c0 += 32) {
+                    tmem_ld_wait16(va);
+                    tmem_ld_32x16(t_half + (uint32_t)(c0 + 16), vb);
+                    emit_p(va, c0);
+                    tmem_ld_wait16(vb);
+                    if (c0 == 0) tmem_ld_32x16(t_half + 32, va);
+                    emit_p(vb, c0 + 16);
+                }
                 tmem_st_wait();
             }
             if (j == n_blk - 1 && (kv_len & (kFaBlk - 1)) != 0 && kv_len < (j + 1) * kFaBlk) {
                 // rows of the V tile past the sequence belong to a neighbour (or are unwritten cache): zero them, so that
                 // 0 * V stays 0 whatever they hold
-                ok = fa_wait(bar_v, ph, abort_flag);
-                if (!ok) break;
+                if (ok) ok = fa_wait(bar_v, ph, abort_flag);
                 const int first = kv_len - j * kFaBlk;       // first row to clear
-                for (int i = threadIdx.x - 32; i < (kFaBlk - first) * 16; i += 128) {
-                    const int row = first + (i >> 4), piece = i & 15;
-                    *reinterpret_cast<uint4*>(sm + kFaV + (piece >> 3) * 16384 + row * 128 + (piece & 7) * 16) = make_uint4(0, 0, 0, 0);
+                if (ok) {
+                    for (int i = threadIdx.x - 32; i < (kFaBlk - first) * 16; i += 256) {
+                        const int row = first + (i >> 4), piece = i & 15;
+                        *reinterpret_cast<uint4*>(sm + kFaV + (piece >> 3) * 16384 + row * 128 + (piece & 7) * 16) = make_uint4(0, 0, 0, 0);
+                    }
+                    fence_proxy_async_smem();
                 }
-                fence_proxy_async_smem();
+            }
+            // Both warps of a quarter leave together, so that no meeting waits for a warp that has gone: a wait that ran out is part of
+            // the vote.  A raised reference is too: it has to be the same for both halves and O before P is used.
+            if (fa_vote(q4, !ok || __any_sync(0xffffffffu, ref != ref0))) {
+                xrow[128 * half] = ref;
+                if (fa_vote(q4, !ok)) { ok = false; break; }
+                const float m = fmaxf(ref, xrow[128 * (half ^ 1)]), f = fa_ex2(ref - m);
+                l2.x *= f; l2.y *= f;
+                fa_rescale_p(t_half, 64, f);
+                ref = m;
+                if (j > 0) {
+                    ok = fa_wait(bar_o, (c + j - 1) & 1, abort_flag);        // O must be complete before it is rewritten
+                    tc_fence_after();
+                    const float fo = fa_ex2(ref0 - m);
+                    for (int c0 = 16 * half; ok && c0 < HDIM; c0 += 32) {
+                        uint32_t v[16];
+                        tmem_ld_32x16(t_row + kFaOCol + c0, v);
+                        tmem_ld_wait16(v);
+#pragma unroll
+                        for (int i = 0; i < 16; i += 8) {
+                            uint32_t w[8];
+#pragma unroll
+                            for (int k = 0; k < 8; ++k) w[k] = __float_as_uint(__uint_as_float(v[i + k]) * fo);
+                            tmem_st_32x8(t_row + kFaOCol + c0 + i, w);
+                        }
+                    }
+                    tmem_st_wait();
+                }
+                if (fa_vote(q4, !ok)) { ok = false; break; }
             }
             // one arrival per warp: 32 lanes arriving on one barrier word are 32 shared-memory atomics one after the other
             tc_fence_before();
@@ -403,42 +444,44 @@ attn_fa_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
         }
         if (!ok) break;
         if (n_blk > 0) {
-        // ---- epilogue: O / rowsum -> bf16 -> staging tile (the V tile is dead) -> whole rows
+        // ---- epilogue: O / rowsum -> bf16 -> staging tile (the V tile is dead) -> whole rows; the warps of a quarter take every
+        //      other 16 columns, then 16 rows each
         ok = fa_wait(bar_o, (c + n_blk - 1) & 1, abort_flag);
-        if (!ok) break;
         tc_fence_after();
-        const float l = l0 + l1;
+        xrow[128 * half] = l2.x + l2.y;
+        if (fa_vote(q4, !ok)) break;
+        const float l = xrow[0] + xrow[128];
         const float inv = l > 0.f ? 1.0f / l : 0.f;
         unsigned char* stage = sm + kFaV;
 #pragma unroll 1
-        for (int c0 = 0; c0 < HDIM; c0 += 32) {
-            uint32_t v[32];
-            tmem_ld_32x32(t_row + kFaOCol + c0, v);
-            tmem_ld_wait();
+        for (int c0 = 16 * half; c0 < HDIM; c0 += 32) {
+            uint32_t v[16];
+            tmem_ld_32x16(t_row + kFaOCol + c0, v);
+            tmem_ld_wait16(v);
 #pragma unroll
-            for (int jj = 0; jj < 4; ++jj)
+            for (int jj = 0; jj < 2; ++jj)
                 *reinterpret_cast<uint4*>(stage + r * 256 + ((((c0 >> 3) + jj) ^ (r & 15)) << 4)) =
                     make_uint4(pack_bf16x2(__uint_as_float(v[8 * jj]) * inv, __uint_as_float(v[8 * jj + 1]) * inv),
                                pack_bf16x2(__uint_as_float(v[8 * jj + 2]) * inv, __uint_as_float(v[8 * jj + 3]) * inv),
                                pack_bf16x2(__uint_as_float(v[8 * jj + 4]) * inv, __uint_as_float(v[8 * jj + 5]) * inv),
                                pack_bf16x2(__uint_as_float(v[8 * jj + 6]) * inv, __uint_as_float(v[8 * jj + 7]) * inv));
         }
-        __syncwarp();
+        fa_vote(q4, false);
         const int sub = lane & 15;
         const FaTile out = fa_tile<HDIM>(a, index);          // once more: kept across the key loop it would cost registers there
 #pragma unroll 4
-        for (int it = 0; it < 16; ++it) {
-            const int rr = q4 * 32 + it * 2 + (lane >> 4), row = out.r0 + rr;
+        for (int it = 0; it < 8; ++it) {
+            const int rr = q4 * 32 + half * 16 + it * 2 + (lane >> 4), row = out.r0 + rr;
             const uint4 val = *reinterpret_cast<const uint4*>(stage + rr * 256 + ((sub ^ (rr & 15)) << 4));
             if (row < out.q_len && sub < HDIM / 8) *reinterpret_cast<uint4*>(a.o + (long long)(out.q_row + rr) * a.o_row + (long long)out.head * a.o_head + 8 * sub) = val;
         }
-        } else fa_zero_rows<HDIM>(a, tile, threadIdx.x - 32, 128);
+        } else fa_zero_rows<HDIM>(a, tile, threadIdx.x - 32, 256);
         fence_proxy_async_smem();                            // the next V block is written through the async proxy
         tc_fence_before();
         __syncwarp();
         if (lane == 0) fa_arrive(bar_e);
         c += n_blk;
-        if (!fa_wait(bar_t + ((t + 1) & 1), (t >> 1) & 1, abort_flag)) break;
+        if (fa_vote(q4, !fa_wait(bar_t + ((t + 1) & 1), (t >> 1) & 1, abort_flag))) break;
         index = next_tile[(t + 1) & 1];
         if (index < 0) break;
       }

@@ -45,3 +45,38 @@ def test_ragged_tiles(lens, prefix, causal):
             s = s.masked_fill(torch.arange(k, device="cuda")[None, :] > torch.arange(m, device="cuda")[:, None] + k - m, float("-inf"))
         want = torch.softmax(s, -1) @ vi
         assert (got - want).abs().max() <= 2.0 ** -7 * want.abs().max(), (i, m, k)
+
+
+@gpu
+@pytest.mark.parametrize("causal", [True, False])
+@pytest.mark.parametrize("kind", ["ramp", "step 40", "step 100", "step 300"])
+def test_rising_scores(kind, causal):
+    """Scores that grow along the keys by far more than a row's softmax reference (taken from its first 16 keys) may lag behind,
+    inside a chunk, in the other half of a block and in later blocks: P, the sums of both halves and O have to be rescaled.  "ramp":
+    key j is (j / 8) x the query direction (0.55 log2 units a key); "step k": keys from k on are 60 x it (+265).  Key head 1 holds the
+    same keys in reverse order.  Bound as above."""
+    from ittai_b200 import ops
+    H, KV, hd, n = 4, 2, 128, 450
+    g = torch.Generator(device="cuda").manual_seed(11)
+    u = torch.nn.functional.normalize(torch.randn(hd, generator=g, device="cuda"), dim=0)
+    j = torch.arange(n, device="cuda", dtype=torch.float32)
+    mag = j / 8 if kind == "ramp" else (j >= int(kind[5:])).float() * 60
+    q = (u * 34.6).repeat(n, H).to(torch.bfloat16)
+    kc = torch.stack([mag[:, None] * u, mag.flip(0)[:, None] * u])[None].to(torch.bfloat16).contiguous()
+    vc = torch.randn(1, KV, n, hd, generator=g, device="cuda").to(torch.bfloat16)
+    out = torch.zeros(n, H * hd, dtype=torch.bfloat16, device="cuda")
+    seqs = torch.tensor([[0, n, 0, n]], dtype=torch.int32, device="cuda")
+    st = ops.new_status("cuda")
+    ops.attention(q, kc, vc, out, seqs, n_heads=H, group=H // KV, head_dim=hd, causal=causal, max_q_len=n, q_strides=(H * hd, hd),
+                  k_strides=(hd, n * hd, KV * n * hd), v_strides=(hd, n * hd, KV * n * hd), o_strides=(H * hd, hd),
+                  q_rows_total=n, kv_rows_total=KV * n, status=st)
+    ops.check_status(st)
+    qi = q.float().view(n, H, hd).transpose(0, 1)
+    ki, vi = (c[0].float().repeat_interleave(H // KV, 0) for c in (kc, vc))
+    s = qi @ ki.transpose(1, 2) / hd ** 0.5
+    assert float((s[0, -1].max() - s[0, -1, :16].max()) * 1.4427) > 64, "the case no longer forces a raise of the reference"
+    if causal:
+        s = s.masked_fill(j[None, :] > j[:, None], float("-inf"))
+    want = torch.softmax(s, -1) @ vi
+    got = out.float().view(n, H, hd).transpose(0, 1)
+    assert torch.isfinite(got).all() and (got - want).abs().max() <= 2.0 ** -7 * want.abs().max()
