@@ -461,8 +461,14 @@ class Siglip2Embedder:
             inp = dict(self.processor(images=images, return_tensors="pt"))
         total = len(inp["pixel_values"])
         # slices of the caller's tensors, so that pinned ones stay pinned; a short last batch runs as what it is (the reference
-        # fills it up with copies of its final image, ``:720-723``)
-        parts = ({name: t[k:k + self.B] for name, t in inp.items()} for k in range(0, total, self.B))
-        out = torch.cat(self._stream_batches(parts, False, lambda part: self.engine.forward_part(part, check=False)))
+        # fills it up with copies of its final image, ``:720-723``).  From host memory it runs FIRST: nothing hides the first
+        # batch's copy, and the copy of the next one hides behind it (200 images in batches of 64: 9.36 -> 9.21 ms)
+        starts = list(range(0, total, self.B))
+        first = len(starts) > 1 and total % self.B != 0 and inp["pixel_values"].device.type == "cpu"
+        if first:
+            starts = starts[-1:] + starts[:-1]
+        parts = ({name: t[k:k + self.B] for name, t in inp.items()} for k in starts)
+        out = self._stream_batches(parts, False, lambda part: self.engine.forward_part(part, check=False))
+        out = torch.cat(out[1:] + out[:1] if first else out)
         self.engine.check_new()
         return out
