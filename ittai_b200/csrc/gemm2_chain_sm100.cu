@@ -7,7 +7,7 @@
 // round-robin to the co-resident clusters, and a tile waits only for the row block it reads:
 //
 //   flags[g][2 * tile_m + rank]   counts the epilogue warps that have finished a tile of GEMM g in that 128-row block
-//                                 (their TMA stores complete, then a gpu-scope release); 8 per column tile.
+//                                 (their TMA stores complete, then a gpu-scope release by a publishing warp); 8 per column tile.
 //   producer of a tile of GEMM g+1, CTA `rank`   acquires flags[g][2 * tile_m + rank] == 8 * column tiles of GEMM g,
 //                                 fences the async proxy, then issues its loads.
 //
@@ -22,6 +22,7 @@
 namespace ittai {
 
 constexpr int kChainMax = 4;
+constexpr int kThreadsChain = kThreads2 + 32;     // one more warp, which publishes finished tiles
 
 struct ChainParams {
     CUtensorMap tm_a[kChainMax], tm_b[kChainMax], tm_out[kChainMax], tm_res[kChainMax];
@@ -36,7 +37,14 @@ __device__ __forceinline__ uint32_t ld_acquire_gpu_u32(const uint32_t* p) {
     return v;
 }
 
-__global__ void __launch_bounds__(kThreads2, 1)
+__device__ __forceinline__ void st_release_cta_u32(uint32_t* p, uint32_t v) { asm volatile("st.release.cta.shared.u32 [%0], %1;" ::"r"(smem_u32(p)), "r"(v) : "memory"); }
+__device__ __forceinline__ uint32_t ld_acquire_cta_u32(const uint32_t* p) {
+    uint32_t v;
+    asm volatile("ld.acquire.cta.shared.u32 %0, [%1];" : "=r"(v) : "r"(smem_u32(p)) : "memory");
+    return v;
+}
+
+__global__ void __launch_bounds__(kThreadsChain, 1)
 gemm2_chain_kernel(const __grid_constant__ ChainParams P) {
     extern __shared__ __align__(1024) unsigned char gsm_raw[];
     unsigned char* gsm = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(gsm_raw) + 1023) & ~(uintptr_t)1023);
@@ -50,7 +58,8 @@ gemm2_chain_kernel(const __grid_constant__ ChainParams P) {
     unsigned long long* acc_empty = bars + 2 * kStages2 + 2;         // [2]       both epilogues -> leader's MMA
     unsigned long long* res_bars = bars + 2 * kStages2 + 4;          // [epilogue warps][2] residual chunk landed
     unsigned long long* inputs = bars + 2 * kStages2 + 4 + 2 * kEpiWarps;   // [4]  the rows that tile `local` (mod 4) reads are complete
-    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(inputs + 4);
+    uint32_t* stored = reinterpret_cast<uint32_t*>(inputs + 4);      // [epilogue warps] tiles that other GEMMs read and this warp has stored
+    uint32_t* tmem_slot = stored + kEpiWarps;
     volatile uint32_t* abort_flag = tmem_slot + 1;
 
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -74,6 +83,7 @@ gemm2_chain_kernel(const __grid_constant__ ChainParams P) {
         for (int b = 0; b < 2; ++b) { mbar_init(&acc_full[b], 1); mbar_init(&acc_empty[b], 2 * kEpiWarps); }
         for (int b = 0; b < 2 * kEpiWarps; ++b) mbar_init(&res_bars[b], 1);
         for (int b = 0; b < 4; ++b) mbar_init(&inputs[b], 1);
+        for (int b = 0; b < kEpiWarps; ++b) stored[b] = 0;
         *abort_flag = 0;
         fence_mbar_init();
         tma_prefetch_desc(&P.tm_a[0]);
@@ -153,6 +163,27 @@ gemm2_chain_kernel(const __grid_constant__ ChainParams P) {
             }
             if (!ok) *abort_flag = 1;
         }
+    } else if (warp == 2 + kEpiWarps) {
+        // ---- publisher: a tile whose eight warps have all stored it is counted for the consumers of its row block.  The fences in
+        //      front of the count take about as long as a third of an epilogue; here they hold nobody up.
+        uint32_t n = 0;
+        for (int t = pair; t < total; t += n_pairs) {
+            int gi, tile;
+            locate(t, gi, tile);
+            if (gi + 1 >= n_g) continue;
+            ++n;
+            uint32_t spins = 0;
+            while (!__all_sync(0xffffffffu, lane >= kEpiWarps || ld_acquire_cta_u32(&stored[lane & (kEpiWarps - 1)]) >= n)) {
+                if (((++spins) & 255u) == 0u && (*abort_flag || spins >= kSpin2)) { *abort_flag = 1; break; }
+            }
+            if (__any_sync(0xffffffffu, *abort_flag != 0)) break;
+            if (lane == 0) {
+                fence_proxy_async();
+                __threadfence();
+                atomicAdd(P.flags + (size_t)gi * 2 * tiles_m + 2 * (tile / (P.g[gi].N / PN)) + rank, (uint32_t)kEpiWarps);
+            }
+            __syncwarp();
+        }
     } else {
         // ---- epilogue: warp w may touch TMEM lanes 32*(w%4)..+31 = 32 rows of this CTA's half tile; the two warps that
         //      share a lane quarter split the 256 columns
@@ -165,7 +196,8 @@ gemm2_chain_kernel(const __grid_constant__ ChainParams P) {
         constexpr uint32_t kChunks = kEpiCols / 32;                  // 32-column chunks per tile for this warp
         uint32_t cc = 0, rcnt = 0;                                   // chunks stored / residual chunks consumed so far
         int local = 0;
-        bool ok = true;
+        bool ok = true, pending = false;                              // pending (lane 0): the tile before is stored, but not yet said so
+        uint32_t n_stored = 0;
         for (int t = pair; t < total && ok; t += n_pairs, ++local) {
             int gi, tile;
             locate(t, gi, tile);
@@ -273,7 +305,11 @@ gemm2_chain_kernel(const __grid_constant__ ChainParams P) {
                     *reinterpret_cast<uint4*>(sto + lane * 64 + ((j ^ swz) << 4)) = make_uint4(o[4 * j], o[4 * j + 1], o[4 * j + 2], o[4 * j + 3]);
                 fence_proxy_async_smem();
                 __syncwarp();
-                if (lane == 0) { tma_store_2d(&P.tm_out[gi], sto, col0 + 32 * (int)ch, row0); tma_store_commit(); }
+                if (lane == 0) {
+                    tma_store_2d(&P.tm_out[gi], sto, col0 + 32 * (int)ch, row0);
+                    tma_store_commit();
+                    if (ch == 0 && pending) { tma_store_wait_done<1>(); st_release_cta_u32(&stored[ew], ++n_stored); pending = false; }   // all but this one
+                }
             }
             if (!ok) break;
             if (has_res) rcnt += kChunks;
@@ -282,16 +318,13 @@ gemm2_chain_kernel(const __grid_constant__ ChainParams P) {
             tc_fence_before();
             __syncwarp();
             if (lane == 0) mbar_arrive_cluster(map_to_cta(&acc_empty[buf], 0));
-            if (gi + 1 < n_g) {
-                // publish: this warp's stores of the tile are complete (bulk stores and the statistics of all its lanes)
-                if (lane == 0) {
-                    tma_store_wait_all();
-                    fence_proxy_async();
-                    __threadfence();
-                    atomicAdd(P.flags + (size_t)gi * 2 * tiles_m + 2 * tile_m + rank, 1u);
-                }
-                __syncwarp();
+            // Tell the publisher that this warp's stores of the tile are complete (bulk stores and the statistics of all its lanes).  While
+            // the next accumulator is already there they are not waited for: a chunk into that tile they have arrived.
+            if (gi + 1 < n_g && lane == 0) {
+                pending = t + n_pairs < total && mbar_test(&acc_full[(local + 1) & 1], ((local + 1) >> 1) & 1);
+                if (!pending) { tma_store_wait_all(); st_release_cta_u32(&stored[ew], ++n_stored); }
             }
+            __syncwarp();
         }
         if (lane == 0) tma_store_wait_all();                          // shared memory stays valid until the stores are done
     }
@@ -347,7 +380,7 @@ int gemm2_chain_launch(const IttaiGemm* gemms, int n, uint32_t* flags, cudaStrea
         cudaLaunchAttribute attr[1];
         attr[0].id = cudaLaunchAttributeClusterDimension;
         attr[0].val.clusterDim.x = 2; attr[0].val.clusterDim.y = 1; attr[0].val.clusterDim.z = 1;
-        cfg.blockDim = dim3(kThreads2);
+        cfg.blockDim = dim3(kThreadsChain);
         cfg.dynamicSmemBytes = kSmem2;
         cfg.attrs = attr;
         cfg.numAttrs = 1;
@@ -362,7 +395,7 @@ int gemm2_chain_launch(const IttaiGemm* gemms, int n, uint32_t* flags, cudaStrea
     const int tiles_m = (C.g[0].M + PM - 1) / PM;
     int total = 0;
     for (int i = 0; i < n; ++i) total += tiles_m * (C.g[i].N / PN);
-    const cudaError_t e = launch_pdl(gemm2_chain_kernel, dim3(2 * (total < max_pairs ? total : max_pairs)), dim3(kThreads2), kSmem2, st, 2, C);
+    const cudaError_t e = launch_pdl(gemm2_chain_kernel, dim3(2 * (total < max_pairs ? total : max_pairs)), dim3(kThreadsChain), kSmem2, st, 2, C);
     if (e != cudaSuccess) return cuda_fail(e, "launch gemm2_chain_kernel");
     return ITTAI_OK;
 }
