@@ -9,13 +9,13 @@
 //     the two 64-dim swizzle atoms of the tile are one operand, 16 KB apart in the descriptor's leading-dimension field).
 //   warps 1-8: two threads per query row, one for the first 64 keys of a block and one for the others, ONE pass over the scores:
 //     P = 2^(s*scale - ref) packed to bf16 over the consumed scores of the same half, and the half's running sum.  ref is the maximum
-//     of the row's first 16 keys, raised only when a sum passes 2^60: P, sums and O are floating point, so a reference that lags
-//     behind the maximum costs nothing, and there is no maximum to find ahead of the exponentials.  Raising is rare: the thread
+//     of the row's first block, raised only when 16 neighbouring P add up to more than 2^8: P, sums and O are floating point, so a
+//     reference that lags behind the maximum costs little, and after that block there is no maximum to find ahead of the exponentials.  Raising is rare: the thread
 //     rescales what it has written, and a vote of the quarter's two warps, which ends every block, brings the other half and O
 //     to the same reference.  The halves' sums meet in the epilogue.
 //     (One thread a row, two passes, a maximum kept within 2^8: 175 us a layer at 8 x 2048 tokens, 135 at 64 x 512, 53 for 55 texts of
-//     16 to 512; this way 150, 119 and 46, of which the elected issuing lane gave about a quarter.  Without any softmax, the two
-//     CTAs' MMAs and hand-offs alone: 115 at 8 x 2048.)
+//     16 to 512, 188 dense at 4 x 2048; this way 156, 128, 48 and 158, with the same error against 64 bits, of which the elected issuing
+//     lane gave about a third.  Without any softmax, the two CTAs' MMAs and hand-offs alone: 115 at 8 x 2048.)
 // TMEM (256 columns, two CTAs per SM): S / P in columns 0..127, O in 128..255.  Shared memory: Q, K, V tiles of 32 KB each
 // (two 128-byte-swizzled atoms of 64 dims); the V tile doubles as the output staging area.
 //
@@ -38,7 +38,7 @@ constexpr uint32_t kFaSpin = 1u << 22;
 constexpr uint32_t kFaQ = 0, kFaK = 32768, kFaV = 65536, kFaBar = 98304;
 constexpr uint32_t kFaX = kFaBar + 256;      // float [2 halves][128 rows]: what the two threads of a row tell each other
 constexpr uint32_t kFaSmem = kFaX + 1024 + 1024;
-constexpr float kFaRaise = 1.152921504606847e18f;   // 2^60: the reference is raised once a row's sum passes this
+constexpr float kFaRaise = 256.f;            // the reference is raised once sixteen neighbouring keys' P add up to more
 
 struct AttnFaArgs {
     const int4* seqs;
@@ -110,6 +110,25 @@ __device__ __noinline__ void fa_rescale_p(uint32_t t_half, int cols, float f) {
         tmem_st_32x8(t_half + (uint32_t)(cp >> 1), u);
     }
     tmem_st_wait();
+}
+// Largest of this thread's 64 scores, unscaled, of those 0..lim unless ALL are visible.  Warp-wide.
+template <bool ALL>
+__device__ __forceinline__ float fa_half_max(uint32_t t_half, int lim) {
+    float m0 = -INFINITY, m1 = -INFINITY;
+#pragma unroll
+    for (int c0 = 0; c0 < 64; c0 += 32) {
+        uint32_t v[16], u[16];
+        tmem_ld_32x16(t_half + (uint32_t)c0, v);
+        tmem_ld_32x16(t_half + (uint32_t)(c0 + 16), u);
+        tmem_ld_wait16(v);
+        tmem_ld_tie16(u);
+#pragma unroll
+        for (int i = 0; i < 16; ++i) {
+            m0 = fmaxf(m0, ALL || c0 + i <= lim ? __uint_as_float(v[i]) : -INFINITY);
+            m1 = fmaxf(m1, ALL || c0 + 16 + i <= lim ? __uint_as_float(u[i]) : -INFINITY);
+        }
+    }
+    return fmaxf(m0, m1);
 }
 // One query tile: where it lies and how many key blocks it sees.
 struct FaTile { int head, r0, q_len, kv_len, n_blk, q_row, q_col, kv_row, kv_col; };
@@ -318,17 +337,16 @@ attn_fa_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
             ok = fa_wait(bar_s, ph, abort_flag);
             tc_fence_after();
             if (j == 0) {
-                // both threads of a row start from the maximum of its first 16 keys; the vote keeps half 0 from writing P over them
+                // the first block's exact maximum: where a few keys dominate a row, their P is then close to 1 and nearly free of rounding
+                float m = -INFINITY;
                 if (ok) {
-                    uint32_t v[16];
-                    tmem_ld_32x16(t_row, v);
-                    tmem_ld_wait16(v);
-                    float m = -INFINITY;
-#pragma unroll
-                    for (int i = 0; i < 16; ++i) if (i <= row_limit) m = fmaxf(m, __uint_as_float(v[i]));
-                    ref = m == -INFINITY ? 0.f : m * a.scale_log2;
+                    const int lim = row_limit - 64 * half;
+                    m = __all_sync(0xffffffffu, lim >= 63) ? fa_half_max<true>(t_half, lim) : fa_half_max<false>(t_half, lim);
+                    xrow[128 * half] = m;
                 }
                 if (fa_vote(q4, !ok)) { ok = false; break; }
+                m = fmaxf(m, xrow[128 * (half ^ 1)]);
+                ref = m == -INFINITY ? 0.f : m * a.scale_log2;
             }
             const float ref0 = ref;
             if (ok) {
@@ -363,16 +381,15 @@ attn_fa_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
                     };
                     exps();
                     store_p();
-                    // The reference lags behind the maximum: sums and P are floating point, so nothing is lost until a sum passes
-                    // 2^60 (or is infinite).  Then this thread's reference is raised to the chunk's maximum (by a whole number, so
-                    // that rescaling is exact), what it has written of this block is rescaled, and the chunk written again; the
-                    // other half and O follow after the block.
-                    const bool raise = (l2.x + l2.y) + (cs.x + cs.y) > kFaRaise;
+                    // The reference lags behind the maximum: sums and P are floating point, so little is lost by it.  Where it
+                    // falls far behind, this thread's reference is raised to the chunk's maximum, what it has written of this
+                    // block is rescaled, and the chunk written again; the other half and O follow after the block.
+                    const bool raise = cs.x + cs.y > kFaRaise;
                     if (__any_sync(0xffffffffu, raise)) {
                         float m = -INFINITY;
 #pragma unroll
                         for (int i = 0; i < 16; ++i) if (c0 + i <= lim) m = fmaxf(m, __uint_as_float(v[i]));
-                        const float nref = raise ? ref + ceilf(fmaxf(fmaf(m, a.scale_log2, -ref), 0.f)) : ref, f = fa_ex2(ref - nref);
+                        const float nref = raise ? fmaxf(m * a.scale_log2, ref) : ref, f = fa_ex2(ref - nref);
                         l2.x *= f; l2.y *= f;
                         fa_rescale_p(t_half, c0, f);
                         ref = nref;

@@ -49,9 +49,9 @@ def test_ragged_tiles(lens, prefix, causal):
 
 @gpu
 @pytest.mark.parametrize("causal", [True, False])
-@pytest.mark.parametrize("kind", ["ramp", "step 40", "step 100", "step 300"])
+@pytest.mark.parametrize("kind", ["ramp", "step 100", "step 140", "step 200", "step 300"])
 def test_rising_scores(kind, causal):
-    """Scores that grow along the keys by far more than a row's softmax reference (taken from its first 16 keys) may lag behind,
+    """Scores that grow along the keys by far more than a row's softmax reference (taken from its first block of 128) may lag behind,
     inside a chunk, in the other half of a block and in later blocks: P, the sums of both halves and O have to be rescaled.  "ramp":
     key j is (j / 8) x the query direction (0.55 log2 units a key); "step k": keys from k on are 60 x it (+265).  Key head 1 holds the
     same keys in reverse order.  Bound as above."""
@@ -74,7 +74,8 @@ def test_rising_scores(kind, causal):
     qi = q.float().view(n, H, hd).transpose(0, 1)
     ki, vi = (c[0].float().repeat_interleave(H // KV, 0) for c in (kc, vc))
     s = qi @ ki.transpose(1, 2) / hd ** 0.5
-    assert float((s[0, -1].max() - s[0, -1, :16].max()) * 1.4427) > 64, "the case no longer forces a raise of the reference"
+    if kind != "step 100":
+        assert float((s[0, -1].max() - s[0, -1, :128].max()) * 1.4427) > 64, "the case no longer forces a raise of the reference"
     if causal:
         s = s.masked_fill(j[None, :] > j[:, None], float("-inf"))
     want = torch.softmax(s, -1) @ vi
