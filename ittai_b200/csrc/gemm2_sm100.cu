@@ -1,7 +1,6 @@
 // Two-SM bf16 GEMM: C[M,N] = A[M,K] * W[N,K]^T (+ fused epilogue) with tcgen05.mma.cta_group::2.  A cluster of two CTAs
 // owns a 256 x 256 output tile: each CTA loads 128 rows of A and 128 rows of W per 64-wide k-block (32 KB instead of the
-// 48 KB a lone CTA needs for its 128 x 256 tile, which is what bounds the one-SM kernel: the L2 cannot feed 96 bytes
-// per clock to every SM), the leader CTA issues M256 N256 K16 MMAs that read both CTAs' shared memory, and each CTA
+// 48 KB a lone CTA needs for its 128 x 256 tile: 64 bytes per clock and SM instead of 96), the leader CTA issues M256 N256 K16 MMAs that read both CTAs' shared memory, and each CTA
 // keeps the accumulator rows of its own 128 rows of A in its own tensor memory (two 256-column buffers, so the epilogue of
 // one tile overlaps the main loop of the next).
 //
