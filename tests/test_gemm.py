@@ -194,3 +194,46 @@ def test_gemm_chain_equals_separate_launches(m):
 
     for got, want, name in zip(run(True), run(False), ("x", "h", "qkv", "stats_a", "stats_m")):
         assert torch.equal(got, want), f"{name}: chained GEMMs differ from separate launches ({(got.float() - want.float()).abs().max().item():.4g})"
+
+
+@gpu
+@pytest.mark.parametrize("m", [129, 1300, 2500, 5001])
+def test_consecutive_tiles_keep_to_their_rows(m):
+    """GEMMs that fetch something per token give a pair of CTAs consecutive tiles: runs that begin and end inside a row block, and
+    cross one (m 1300 to 5001).  Rotary epilogue with a folded RMSNorm against the same GEMM and the row-wise pass (the same rounding
+    steps; the head norm's sum is taken in another order, which flips a rounding now and then), and a folded LayerNorm with residual and
+    output statistics against torch."""
+    from ittai_b200 import _C, ops
+    from ittai_b200.qwen3.decoder import rope_table
+    g = torch.Generator(device="cuda").manual_seed(m)
+    x, w, st = _rand(m, 1024, seed=61), _rand(4096, 1024, scale=0.05, seed=62), ops.new_status("cuda")
+    cap = m + 7
+    qn, kn = (torch.rand(128, generator=g, device="cuda") + 0.5).to(torch.bfloat16), (torch.rand(128, generator=g, device="cuda") + 0.5).to(torch.bfloat16)
+    pos = torch.randint(0, 4000, (m,), generator=g, device="cuda", dtype=torch.int32)
+    seq, slot = torch.zeros(m, dtype=torch.int32, device="cuda"), torch.randperm(cap, generator=g, device="cuda")[:m].int()
+    rope = rope_table(4000, "cuda")
+    xf = x.float().view(m, 8, 128)
+    fold = dict(row_stats=torch.stack([xf.sum(-1), xf.pow(2).sum(-1)], -1).contiguous(), col_sums=torch.zeros(4096, device="cuda"), stats_eps=1e-6, stats_rms=True)
+    kc, vc, kc2, vc2 = (torch.full((1, 8, cap, 128), 5.0, dtype=torch.bfloat16, device="cuda") for _ in range(4))
+    want = ops.gemm(x, w, st, **fold)
+    _C.check(_C.lib().ittai_qwen3_qk_rope_scatter(want.data_ptr(), qn.data_ptr(), kn.data_ptr(), rope.data_ptr(), pos.data_ptr(), seq.data_ptr(),
+                                                  slot.data_ptr(), kc.data_ptr(), vc.data_ptr(), m, cap, 1e-6, ops._stream(x)))
+    got = torch.zeros(m, 4096, dtype=torch.bfloat16, device="cuda")
+    ops.gemm(x, w, st, out=got, epi=_C.EPI_QKROPE, qk_rope=dict(qn=qn, kn=kn, rope=rope, pos=pos, seq=seq, slot=slot, kcache=kc2, vcache=vc2, kv_cap=cap, eps=1e-6), **fold)
+    ops.check_status(st)
+    assert torch.equal(vc, vc2)
+    for a, b in ((want[:, :2048], got[:, :2048]), (kc, kc2)):
+        d = (a.float() - b.float()).abs()
+        assert (d > 0).float().mean() < 1e-3 and d.max() <= 2.0 ** -6 * a.float().abs().max()
+    # LayerNorm, residual, statistics
+    n, d = 768, 768
+    y, wl, res, gain, beta, bias = _rand(m, d, seed=63), _rand(n, d, scale=0.05, seed=64), _rand(m, n, seed=65), torch.rand(d, device="cuda") + 0.5, torch.randn(d, device="cuda") * 0.1, torch.randn(n, device="cuda")
+    yf = y.float().view(m, 6, 128)
+    wp, bp, cs = ops.fold_layernorm(wl, bias, gain, beta)
+    parts = torch.full((m, n // 128, 2), float("nan"), device="cuda")
+    out = ops.gemm(y, wp, st, bias=bp, residual=res, row_stats=torch.stack([yf.sum(-1), yf.pow(2).sum(-1)], -1).contiguous(), col_sums=cs, stats_eps=1e-6, stats_out=parts)
+    ops.check_status(st)
+    lin = torch.nn.functional.linear(torch.nn.functional.layer_norm(y.float(), (d,), gain, beta, 1e-6), wl.float(), bias)
+    _check(out, res.float() + lin.to(torch.bfloat16).float(), "LayerNorm + residual", mid=lin)
+    of = out.float().view(m, n // 128, 128)
+    assert torch.allclose(parts[..., 0], of.sum(-1), rtol=1e-5, atol=1e-3) and torch.allclose(parts[..., 1], of.pow(2).sum(-1), rtol=1e-5, atol=1e-3)
