@@ -197,10 +197,10 @@ def test_gemm_chain_equals_separate_launches(m):
 
 
 @gpu
-@pytest.mark.parametrize("m", [129, 1300, 2500, 5001])
+@pytest.mark.parametrize("m", [129, 1300, 2500])
 def test_consecutive_tiles_keep_to_their_rows(m):
     """GEMMs that fetch something per token give a pair of CTAs consecutive tiles: runs that begin and end inside a row block, and
-    cross one (m 1300 to 5001).  Rotary epilogue with a folded RMSNorm against the same GEMM and the row-wise pass (the same rounding
+    cross one (m 1300, 2500).  Rotary epilogue with a folded RMSNorm against the same GEMM and the row-wise pass (the same rounding
     steps; the head norm's sum is taken in another order, which flips a rounding now and then), and a folded LayerNorm with residual and
     output statistics against torch."""
     from ittai_b200 import _C, ops
@@ -209,9 +209,9 @@ def test_consecutive_tiles_keep_to_their_rows(m):
     x, w, st = _rand(m, 1024, seed=61), _rand(4096, 1024, scale=0.05, seed=62), ops.new_status("cuda")
     cap = m + 7
     qn, kn = (torch.rand(128, generator=g, device="cuda") + 0.5).to(torch.bfloat16), (torch.rand(128, generator=g, device="cuda") + 0.5).to(torch.bfloat16)
-    pos = torch.randint(0, 4000, (m,), generator=g, device="cuda", dtype=torch.int32)
+    pos = torch.randint(0, 400, (m,), generator=g, device="cuda", dtype=torch.int32)
     seq, slot = torch.zeros(m, dtype=torch.int32, device="cuda"), torch.randperm(cap, generator=g, device="cuda")[:m].int()
-    rope = rope_table(4000, "cuda")
+    rope = rope_table(400, "cuda")
     xf = x.float().view(m, 8, 128)
     fold = dict(row_stats=torch.stack([xf.sum(-1), xf.pow(2).sum(-1)], -1).contiguous(), col_sums=torch.zeros(4096, device="cuda"), stats_eps=1e-6, stats_rms=True)
     kc, vc, kc2, vc2 = (torch.full((1, 8, cap, 128), 5.0, dtype=torch.bfloat16, device="cuda") for _ in range(4))
