@@ -84,7 +84,9 @@ __device__ __forceinline__ void epilogue_qkrope(const GemmArgs& g, const CUtenso
     }
     // four staging tiles of 32 columns, so that the tile is fenced and stored at once
     const int swz = (lane >> 1) & 3;
-    if (head < 16 && lane == 0) tma_store_wait_read<0>();     // the tile before has left them
+    // The tile before has left them.  For k and v heads too, although they store nothing through TMA: in a run of consecutive tiles
+    // the first k tile of a row block follows the last q tile, whose stores may still be reading.  At once where none is pending.
+    if (lane == 0) tma_store_wait_read<0>();
     __syncwarp();
 #pragma unroll
     for (int ch = 0; ch < 4; ++ch)

@@ -237,3 +237,51 @@ def test_consecutive_tiles_keep_to_their_rows(m):
     _check(out, res.float() + lin.to(torch.bfloat16).float(), "LayerNorm + residual", mid=lin)
     of = out.float().view(m, n // 128, 128)
     assert torch.allclose(parts[..., 0], of.sum(-1), rtol=1e-5, atol=1e-3) and torch.allclose(parts[..., 1], of.pow(2).sum(-1), rtol=1e-5, atol=1e-3)
+
+
+def _qk_runs(m, n_sms):
+    """Runs of consecutive QKV tiles (16 column tiles a row block) that the pairs of SMs walk."""
+    tiles, pairs = (m + 255) // 256 * 16, min((m + 255) // 256 * 16, n_sms // 2)
+    return [range(tiles * p // pairs, tiles * (p + 1) // pairs) for p in range(pairs)]
+
+
+@gpu
+@pytest.mark.parametrize("m", [2304, 16384])
+def test_rotary_runs_equal_single_tiles_bit_for_bit(m):
+    """A pair's run goes from the last q tile of a row block (column tile 7) to the first k tile (8) and on to the next row block; the
+    warps' staging tiles change hands between bulk stores and ordinary ones there.  The same rows in launches that give every pair one
+    tile: no order of sums depends on the rows, so q, k and v are the same bits."""
+    from ittai_b200 import _C, ops
+    from ittai_b200.qwen3.decoder import rope_table
+    n_sms = torch.cuda.get_device_properties(0).multi_processor_count
+    piece = n_sms // 2 // 16 * 256
+    assert all(len(r) == 1 for r in _qk_runs(piece, n_sms))
+    assert sum(7 in [t % 16 for t in r[:-1]] for r in _qk_runs(m, n_sms)) >= m // 512, "too few runs cross from q to k"
+    g = torch.Generator(device="cuda").manual_seed(m)
+    x, w, st = _rand(m, 1024, seed=71), _rand(4096, 1024, scale=0.05, seed=72), ops.new_status("cuda")
+    qn, kn = (torch.rand(128, generator=g, device="cuda") + 0.5).to(torch.bfloat16), (torch.rand(128, generator=g, device="cuda") + 0.5).to(torch.bfloat16)
+    pos, seq, slot = torch.randint(0, 400, (m,), generator=g, device="cuda", dtype=torch.int32), torch.zeros(m, dtype=torch.int32, device="cuda"), torch.randperm(m, generator=g, device="cuda").int()
+    rope = rope_table(400, "cuda")
+
+    def run(step):
+        kc, vc = (torch.full((1, 8, m, 128), 5.0, dtype=torch.bfloat16, device="cuda") for _ in range(2))
+        out = torch.zeros(m, 4096, dtype=torch.bfloat16, device="cuda")
+        for a in range(0, m, step):
+            z = slice(a, a + step)
+            ops.gemm(x[z], w, st, out=out[z], epi=_C.EPI_QKROPE, qk_rope=dict(qn=qn, kn=kn, rope=rope, pos=pos[z], seq=seq[z], slot=slot[z], kcache=kc, vcache=vc, kv_cap=m, eps=1e-6))
+        return out[:, :2048], kc, vc
+
+    want = run(piece)
+    for _ in range(4):
+        got = run(m)
+        for a, b, name in zip(got, want, "qkv"):
+            assert torch.equal(a, b), f"{name}: {int((a != b).sum())} values differ"
+    ops.check_status(st)
+
+
+@pytest.mark.parametrize("m", [2304, 16384])
+def test_rotary_runs_cross_from_q_to_k(m):
+    """The sizes above do what they are there for, and the runs share out every tile once (148 SMs)."""
+    runs = _qk_runs(m, 148)
+    assert [t for r in runs for t in r] == list(range((m + 255) // 256 * 16))
+    assert sum(7 in [t % 16 for t in r[:-1]] for r in runs) >= m // 512
