@@ -197,6 +197,7 @@ gemm2_chain_kernel(const __grid_constant__ ChainParams P) {
         uint32_t cc = 0, rcnt = 0;                                   // chunks stored / residual chunks consumed so far
         int local = 0;
         bool ok = true, pending = false;                              // pending (lane 0): the tile before is stored, but not yet said so
+        bool one_buffer = false;                                      // the tile before stored every chunk from staging tile 0
         uint32_t n_stored = 0;
         for (int t = pair; t < total && ok; t += n_pairs, ++local) {
             int gi, tile;
@@ -296,9 +297,11 @@ gemm2_chain_kernel(const __grid_constant__ ChainParams P) {
                         st2 = fmaf(lo, lo, fmaf(hi, hi, st2));
                     }
                 }
-                // the store that last used this staging tile must have finished reading it
+                // The store that last used this staging tile must have finished reading it: the third newest where the three tiles
+                // rotate, the newest where a residual leaves only tile 0, and at the step from such a tile to the rotation, whose
+                // first chunk may fall on tile 0 as well.
                 unsigned char* sto = has_res ? so : so + (cc % 3u) * 2048;
-                if (lane == 0) { if (has_res) tma_store_wait_read<0>(); else tma_store_wait_read<2>(); }
+                if (lane == 0) { if (has_res || (one_buffer && ch == 0)) tma_store_wait_read<0>(); else tma_store_wait_read<2>(); }
                 __syncwarp();
 #pragma unroll
                 for (int j = 0; j < 4; ++j)
@@ -312,6 +315,7 @@ gemm2_chain_kernel(const __grid_constant__ ChainParams P) {
                 }
             }
             if (!ok) break;
+            one_buffer = has_res;
             if (has_res) rcnt += kChunks;
             if (g.stats_out != nullptr && row0 + lane < g.M)
                 *reinterpret_cast<float2*>(g.stats_out + 2 * ((size_t)(row0 + lane) * (g.N / 128) + col0 / 128)) = make_float2(st1, st2);

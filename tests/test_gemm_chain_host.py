@@ -33,3 +33,31 @@ def test_a_task_that_waits_for_a_later_task_is_reported():
             gc.simulate(512, [256, 256], 2, random.Random(0))
     finally:
         gc.chain_tasks = real
+
+
+def _staging_conflicts(residual, drain_at_step):
+    """Chunks of consecutive tiles (``residual[i]``: tile i adds one) as an epilogue warp of the chain kernel stages them, no tile's
+    stores awaited at its end: (tile, chunk) pairs written while a bulk store issued before may still read the same staging tile."""
+    unread, bad, cc, one_buffer = [], [], 0, False         # staging tiles of the stores that may still be reading, oldest first
+    for tile, has_res in enumerate(residual):
+        if has_res:
+            unread.clear()                                 # staging tiles 1 and 2 become load targets
+        for ch in range(4):
+            keep = 0 if has_res or (drain_at_step and one_buffer and ch == 0) else 2
+            del unread[:max(0, len(unread) - keep)]
+            buf = 0 if has_res else cc % 3
+            if buf in unread:
+                bad.append((tile, ch))
+            unread.append(buf)
+            cc += 1
+        one_buffer = has_res
+    return bad
+
+
+@pytest.mark.parametrize("before", range(6))
+def test_staging_tiles_are_read_before_they_are_written_again(before):
+    """A layer's order (residual, none, residual, none) with 0 to 5 tiles ahead of it; without the wait at the step from a tile with a
+    residual to one without, every third position writes a tile that is still read."""
+    order = [False] * before + [True] * 2 + [False] * 3 + [True, False, True, False, False]
+    assert not _staging_conflicts(order, True)
+    assert any(_staging_conflicts([False] * n + order, False) for n in range(3))
