@@ -23,6 +23,13 @@ namespace ittai {
 
 constexpr int kChainMax = 4;
 constexpr int kThreadsChain = kThreads2 + 32;     // one more warp, which publishes finished tiles
+// Barriers that say the rows a tile reads are complete, tile `local` of a pair on barrier local % kInputs.  While an epilogue warp has
+// not looked at the one of tile e, the MMAs end with tile e + 1, the stages hold k-blocks of later tiles, at least one each, and the
+// producer signals a tile before it waits for a stage: it is at tile e + 2 + kStages2 at most.  One barrier fewer and it could
+// complete tile e's a second time, which a waiter on parity cannot tell from never.
+constexpr int kInputs = 8;
+static_assert(kInputs >= kStages2 + 3 && (kInputs & (kInputs - 1)) == 0, "a barrier of `inputs` is signalled again only after it was looked at");
+static_assert((2 * kStages2 + 4 + 2 * kEpiWarps + kInputs) * 8 + (kEpiWarps + 2) * 4 <= 512, "barriers and flags of the shared-memory plan");
 
 struct ChainParams {
     CUtensorMap tm_a[kChainMax], tm_b[kChainMax], tm_out[kChainMax], tm_res[kChainMax];
@@ -57,8 +64,8 @@ gemm2_chain_kernel(const __grid_constant__ ChainParams P) {
     unsigned long long* acc_full = bars + 2 * kStages2;              // [2]       MMA -> this CTA's epilogue
     unsigned long long* acc_empty = bars + 2 * kStages2 + 2;         // [2]       both epilogues -> leader's MMA
     unsigned long long* res_bars = bars + 2 * kStages2 + 4;          // [epilogue warps][2] residual chunk landed
-    unsigned long long* inputs = bars + 2 * kStages2 + 4 + 2 * kEpiWarps;   // [4]  the rows that tile `local` (mod 4) reads are complete
-    uint32_t* stored = reinterpret_cast<uint32_t*>(inputs + 4);      // [epilogue warps] tiles that other GEMMs read and this warp has stored
+    unsigned long long* inputs = bars + 2 * kStages2 + 4 + 2 * kEpiWarps;   // [kInputs] the rows that a tile reads are complete
+    uint32_t* stored = reinterpret_cast<uint32_t*>(inputs + kInputs);      // [epilogue warps] tiles that other GEMMs read and this warp has stored
     uint32_t* tmem_slot = stored + kEpiWarps;
     volatile uint32_t* abort_flag = tmem_slot + 1;
 
@@ -82,7 +89,7 @@ gemm2_chain_kernel(const __grid_constant__ ChainParams P) {
         for (int s = 0; s < kStages2; ++s) { mbar_init(&full[s], 1); mbar_init(&empty[s], 1); }
         for (int b = 0; b < 2; ++b) { mbar_init(&acc_full[b], 1); mbar_init(&acc_empty[b], 2 * kEpiWarps); }
         for (int b = 0; b < 2 * kEpiWarps; ++b) mbar_init(&res_bars[b], 1);
-        for (int b = 0; b < 4; ++b) mbar_init(&inputs[b], 1);
+        for (int b = 0; b < kInputs; ++b) mbar_init(&inputs[b], 1);
         for (int b = 0; b < kEpiWarps; ++b) stored[b] = 0;
         *abort_flag = 0;
         fence_mbar_init();
@@ -119,7 +126,7 @@ gemm2_chain_kernel(const __grid_constant__ ChainParams P) {
                     if (*abort_flag) break;
                     fence_proxy_async();                             // the loads below go through the async proxy
                 }
-                mbar_arrive(&inputs[local & 3]);
+                mbar_arrive(&inputs[local % kInputs]);
                 for (int kb = 0; kb < n_kb; ++kb, ++it) {
                     const int s = it % kStages2, use = it / kStages2;
                     if (use > 0 && !mbar_wait_bounded(&empty[s], (use - 1) & 1, kSpin2)) { *abort_flag = 1; break; }
@@ -215,11 +222,10 @@ gemm2_chain_kernel(const __grid_constant__ ChainParams P) {
             if (fold && lane < kEpiCols / 4) *reinterpret_cast<float4*>(scsum + 4 * lane) = *reinterpret_cast<const float4*>(g.col_sums + col0 + 4 * lane);
             __syncwarp();
             // This CTA's producer has seen the row block of GEMM gi - 1 complete; take the same acquire here for the statistics and
-            // the residual this warp reads itself, so that they arrive while the accumulator fills.  (The producer is three tiles
-            // ahead at most: its next tile but two needs an accumulator that this warp has not handed back.)
+            // the residual this warp reads itself, so that they arrive while the accumulator fills.
             {
                 uint32_t spins = 0;
-                while (!mbar_try_wait_parked(&inputs[local & 3], (local >> 2) & 1)) {
+                while (!mbar_try_wait_parked(&inputs[local % kInputs], (local / kInputs) & 1)) {
                     if (((++spins) & 255u) == 0u && (*abort_flag || spins >= kSpin2)) { ok = false; break; }
                 }
             }

@@ -197,6 +197,24 @@ def test_gemm_chain_equals_separate_launches(m):
 
 
 @gpu
+@pytest.mark.parametrize("k", [64, 128, 192])
+def test_gemm_chain_with_a_short_first_gemm(k):
+    """K of one to three k-blocks: the loads run up to seven tiles ahead of the epilogue, over eight tiles of the first GEMM for
+    every pair of SMs.  The same bits as separate launches."""
+    from ittai_b200 import _C, ops
+    n = 512
+    m = torch.cuda.get_device_properties(0).multi_processor_count // 2 * 1024
+    a, w0, w1, b0, st = _rand(m, k, seed=91), _rand(n, k, scale=0.05, seed=92), _rand(n, n, scale=0.05, seed=93), _rand(n, seed=94).float(), ops.new_status("cuda")
+    x, y = (torch.zeros(m, n, dtype=torch.bfloat16, device="cuda") for _ in range(2))
+    want_x = ops.gemm(a, w0, st, bias=b0, epi=_C.EPI_GELU)
+    want_y = ops.gemm(want_x, w1, st)
+    flags = torch.zeros(2 * 2 * ((m + 255) // 256), dtype=torch.int32, device="cuda")
+    ops.gemm_chain([ops.gemm_desc(a, w0, st, bias=b0, epi=_C.EPI_GELU, out=x)[0], ops.gemm_desc(x, w1, st, out=y)[0]], flags)
+    ops.check_status(st)
+    assert torch.equal(x, want_x) and torch.equal(y, want_y)
+
+
+@gpu
 def test_gemm_chain_from_residual_to_plain_tiles():
     """As many tiles of a GEMM with a residual as make three for every pair of SMs, then one without: the warps go from one staging
     tile to three in rotation, on the first again.  Short main loops, so that the next accumulator is there before a tile is stored.  The

@@ -3,7 +3,7 @@ import random
 
 import pytest
 
-from ittai_b200.gemm_chain import chain_tasks, simulate
+from ittai_b200.gemm_chain import INPUTS, STAGES, chain_tasks, simulate, simulate_pair
 
 SIGLIP_LAYER = [768, 3072, 768, 2304]          # out-proj, fc1, fc2, next QKV
 
@@ -61,3 +61,26 @@ def test_staging_tiles_are_read_before_they_are_written_again(before):
     order = [False] * before + [True] * 2 + [False] * 3 + [True, False, True, False, False]
     assert not _staging_conflicts(order, True)
     assert any(_staging_conflicts([False] * n + order, False) for n in range(3))
+
+
+@pytest.mark.parametrize("m,ns,clusters", [(12544, SIGLIP_LAYER, 74), (2048, [256, 1024], 5), (300, [256, 256, 256, 256], 3)])
+def test_tiles_counted_late_never_deadlock(m, ns, clusters):
+    """Finished tiles told to the publishing warp only with the next one, loads up to the longest lead ahead."""
+    for seed in range(3):
+        for ahead in (2, 2 + STAGES):
+            r = simulate(m, ns, clusters, random.Random(seed), ahead=ahead, late=True)
+            assert r["steps"] == 2 * r["tasks"]
+
+
+@pytest.mark.parametrize("n_kb", [1, 2, 3, 4, 12, 48])
+def test_an_inputs_barrier_is_not_completed_again_before_it_was_looked_at(n_kb):
+    """K = 64 is the longest lead: two accumulators and five stages.  The ring of four barriers that K >= 192 would do with fails
+    there and at K = 128."""
+    lead = max(simulate_pair([n_kb] * 40, random.Random(seed)) for seed in range(200))
+    assert lead <= STAGES + 2 < INPUTS
+    if n_kb == 1:
+        assert lead == STAGES + 2
+    if n_kb <= 2:
+        with pytest.raises(RuntimeError, match="completed again"):
+            for seed in range(200):
+                simulate_pair([n_kb] * 40, random.Random(seed), inputs=4)
