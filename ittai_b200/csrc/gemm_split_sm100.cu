@@ -52,7 +52,11 @@ struct SplitCfg {
     static constexpr bool kAlias = TN > 64;
     static constexpr int kStages = TN == 32 ? 4 : 3;
     static constexpr int kRows = TN / 32;                        // output rows a warp works on side by side
-    static constexpr int kNormGroup = TN == 32 ? 1 : TN == 64 ? 2 : 3;   // warps that normalise a k-block, other groups the next ones
+    // Warps that normalise a k-block, in as many groups as stages: a group keeps to one stage and so waits for every use of its
+    // barrier, one after the other.  (A group that skips uses, or that first looks at a later one, is let through by the parity of
+    // the phase before and normalises what has not landed.)
+    static constexpr int kNormGroup = kNormWarps / kStages;
+    static_assert(kNormGroup >= 1, "a group for every stage");
     static constexpr uint32_t kA = TN * SK * 2;
     static constexpr uint32_t kRing = kStages * (kA + kSplitW);
     static constexpr uint32_t kRecv = kAlias ? 0 : TN * SN * 4;
@@ -257,10 +261,10 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constan
     }
     __syncwarp();
     const bool normalises = warp >= 2 && g.a_gain != nullptr;
-    // its k-blocks: group, group + kGroups, ...; a thread keeps to one 16-byte column piece (eight pieces a row), so its gains are
-    // one vector per k-block, the first of them fetched ahead of the wait like the weights
-    constexpr int kNormThreads = 32 * Cfg::kNormGroup, kGroups = kNormWarps / Cfg::kNormGroup;
-    const int group = (warp - 2) / Cfg::kNormGroup, nt = (threadIdx.x - 64) % kNormThreads, piece = nt & 7;
+    // its k-blocks: group, group + kStages, ... (none for the warps left over); a thread keeps to one 16-byte column piece (eight
+    // pieces a row), so its gains are one vector per k-block, the first of them fetched ahead of the wait like the weights
+    constexpr int kNormThreads = 32 * Cfg::kNormGroup;
+    const int group = warp - 2 < kStages * Cfg::kNormGroup ? (warp - 2) / Cfg::kNormGroup : n_kb, nt = (threadIdx.x - 64) % kNormThreads, piece = nt & 7;
     const uint4* gains = reinterpret_cast<const uint4*>(g.a_gain + (size_t)kb0 * SK) + piece;
     uint4 gain = make_uint4(0u, 0u, 0u, 0u);
     if (normalises && group < n_kb) gain = gains[8 * group];
@@ -307,10 +311,10 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constan
         const int t = threadIdx.x - 64;
         if (t < rows) scale[t] = 1.0f / sqrtf(row_sums(g, row_base + t).y * (1.0f / (float)g.K) + g.stats_eps);
         asm volatile("bar.sync 1, %0;" ::"n"(32 * kNormWarps) : "memory");
-        for (int kb = group; kb < n_kb; kb += kGroups) {
+        for (int kb = group; kb < n_kb; kb += kStages) {
             const int s = kb % kStages, use = kb / kStages;
             const uint4 gq = gain;
-            if (kb + kGroups < n_kb) gain = gains[8 * (kb + kGroups)];
+            if (kb + kStages < n_kb) gain = gains[8 * (kb + kStages)];
             bool ok = true;
             uint32_t spins = 0;
             while (!mbar_try_wait_parked(&full[s], use & 1)) {

@@ -125,6 +125,53 @@ def test_split_k_rope_epilogue_matches_the_separate_pass(T):
         assert torch.equal(got == 3.0, want == 3.0) or name == "q", f"{name}: other cache rows written"
 
 
+def _early(stages, groups, n_kb=48):
+    """k-blocks whose wait a group may leave a phase early: use u of a stage is waited for by the parity of u, which the end of use
+    u - 2 satisfies as well, unless the group has seen use u - 1 end."""
+    bad = []
+    for g in range(groups):
+        seen = {}
+        for kb in range(g, n_kb, groups):
+            s, u = kb % stages, kb // stages
+            if u > seen.get(s, -1) + 1:
+                bad.append(kb)
+            seen[s] = u
+    return bad
+
+
+def test_normalising_groups_wait_for_every_use_of_a_stage():
+    """As many groups as stages; six on four stages or two on three would be let through early."""
+    assert not _early(4, 4) and not _early(3, 3)
+    assert _early(4, 6)[0] == 4 and _early(3, 2)
+
+
+@gpu
+@pytest.mark.parametrize("m,n,k", [(7, 256, 64), (32, 256, 2560), (23, 256, 4096), (32, 256, 8192), (31, 4096, 2048), (64, 4096, 1024), (40, 4096, 2048), (100, 4096, 3072),
+                                   (640, 1024, 3072), (768, 1024, 6144)])
+def test_normalisation_inside_the_gemm(m, n, k):
+    """One to 24 k-blocks a CTA, up to eight uses of a stage, tiles of 32, 64 and 128 rows, against the same GEMM on rows normalised
+    beforehand with the same roundings (the reciprocal root may differ by an ulp and tip one).  The gains tell the k-blocks apart."""
+    import ctypes as C
+    from ittai_b200 import _C, ops
+    launch = getattr(_C.lib(), "_ZN5ittai18gemm_normed_launchEPK9IttaiGemmPKvP11CUstream_st")       # used by the prefill, not exported
+    launch.argtypes = [C.c_void_p, C.c_void_p, C.c_void_p]
+    x, w, st = (_rand(m, k, seed=61).float() * 3).to(torch.bfloat16), _rand(n, k, scale=0.05, seed=62), ops.new_status("cuda")
+    gain = ((torch.arange(k, device="cuda") // 64 % 7 + 1) * 0.25).to(torch.bfloat16)
+    xf = x.float().view(m, -1, 64 if k < 128 else 128)
+    parts = torch.stack([xf.sum(-1), xf.pow(2).sum(-1)], -1).contiguous()
+    normed = rb(rb(x.float() * torch.rsqrt(xf.pow(2).sum((1, 2)) / k + 1e-6)[:, None]) * gain.float()).to(torch.bfloat16)
+    want = ops.gemm(normed, w, st, static_w=True)
+    g, out = ops.gemm_desc(x, w, st, static_w=True)
+    zeros = torch.zeros(n, device="cuda")
+    g.row_stats, g.col_sums, g.stats_parts, g.stats_eps, g.stats_rms = parts.data_ptr(), zeros.data_ptr(), parts.shape[1], 1e-6, 1
+    for _ in range(3):
+        out.zero_()
+        _C.check(launch(C.addressof(g), gain.data_ptr(), ops._stream(x)))
+        ops.check_status(st)
+        _check(out, want, f"{m}x{n}x{k}")
+    _check(out, normed.float() @ w.float().t(), f"{m}x{n}x{k} against fp32")
+
+
 def test_limits_without_the_flag():
     """What needs more than 128 rows (or constant weights) is refused without the flag, and the flag is no epilogue of a chain."""
     import ctypes as C
