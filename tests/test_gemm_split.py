@@ -142,7 +142,7 @@ def _early(stages, groups, n_kb=48):
 def test_normalising_groups_wait_for_every_use_of_a_stage():
     """As many groups as stages; six on four stages or two on three would be let through early."""
     assert not _early(4, 4) and not _early(3, 3)
-    assert _early(4, 6)[0] == 4 and _early(3, 2)
+    assert {4, 5, 6} <= set(_early(4, 6)) and 3 in _early(3, 2)
 
 
 @gpu
