@@ -184,6 +184,7 @@ gemm2_chain_kernel(const __grid_constant__ ChainParams P) {
                 if (((++spins) & 255u) == 0u && (*abort_flag || spins >= kSpin2)) { *abort_flag = 1; break; }
             }
             if (__any_sync(0xffffffffu, *abort_flag != 0)) break;
+            __syncwarp();                                            // eight lanes have acquired a word each, lane 0 counts for all: votes order no memory
             if (lane == 0) {
                 fence_proxy_async();
                 __threadfence();

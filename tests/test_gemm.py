@@ -218,20 +218,23 @@ def test_gemm_chain_with_a_short_first_gemm(k):
 def test_gemm_chain_from_residual_to_plain_tiles():
     """As many tiles of a GEMM with a residual as make three for every pair of SMs, then one without: the warps go from one staging
     tile to three in rotation, on the first again.  Short main loops, so that the next accumulator is there before a tile is stored.  The
-    same bits as separate launches, several times."""
+    second GEMM also reads the row statistics that all lanes of the first one's epilogue warps wrote with ordinary stores.  The same bits
+    as separate launches, several times."""
     from ittai_b200 import ops
     n, k = 768, 256
     m = torch.cuda.get_device_properties(0).multi_processor_count // 2 * 256
     a, w0, w1, x0, st = _rand(m, k, seed=81), _rand(n, k, scale=0.05, seed=82), _rand(n, n, scale=0.05, seed=83), _rand(m, n, seed=84), ops.new_status("cuda")
-    x, y = torch.empty_like(x0), torch.empty_like(x0)
-    want_x = ops.gemm(a, w0, st, residual=x0)
-    want_y = ops.gemm(want_x, w1, st)
+    x, y, want_s, s = torch.empty_like(x0), torch.empty_like(x0), *(torch.empty(m, n // 128, 2, device="cuda") for _ in range(2))
+    cs = w1.float().sum(1)
+    want_x = ops.gemm(a, w0, st, residual=x0, stats_out=want_s)
+    want_y = ops.gemm(want_x, w1, st, row_stats=want_s, col_sums=cs, stats_eps=1e-6)
     flags = torch.zeros(2 * 2 * ((m + 255) // 256), dtype=torch.int32, device="cuda")
     for _ in range(4):
         flags.zero_()
-        ops.gemm_chain([ops.gemm_desc(a, w0, st, residual=x0, out=x)[0], ops.gemm_desc(x, w1, st, out=y)[0]], flags)
+        s.fill_(float("nan"))
+        ops.gemm_chain([ops.gemm_desc(a, w0, st, residual=x0, out=x, stats_out=s)[0], ops.gemm_desc(x, w1, st, out=y, row_stats=s, col_sums=cs, stats_eps=1e-6)[0]], flags)
         ops.check_status(st)
-        assert torch.equal(x, want_x) and torch.equal(y, want_y)
+        assert torch.equal(x, want_x) and torch.equal(s, want_s) and torch.equal(y, want_y)
 
 
 @gpu
