@@ -352,7 +352,7 @@ attn_fa_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
             if (ok) {
                 const int lim = row_limit - j * kFaBlk - 64 * half;  // columns 0..lim of this half are visible to this row
                 const bool full = __all_sync(0xffffffffu, lim >= 63);
-                auto emit_p = [&](uint32_t (&v)[16], int c0) {
+                auto emit_p = [&](uint32_t (&v)[16], uint32_t (&flight)[16], int c0) {      // flight: the next sixteen scores, requested (c0 < 48)
                     uint32_t w[8];
                     if (!full && !__any_sync(0xffffffffu, c0 <= lim)) {      // no row of the warp sees these keys
 #pragma unroll
@@ -386,6 +386,8 @@ attn_fa_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
                     // block is rescaled, and the chunk written again; the other half and O follow after the block.
                     const bool raise = cs.x + cs.y > kFaRaise;
                     if (__any_sync(0xffffffffu, raise)) {
+                        // a call follows, around which registers may be moved: none of them may still be waiting for tensor memory
+                        if (c0 < 48) tmem_ld_wait16(flight);
                         float m = -INFINITY;
 #pragma unroll
                         for (int i = 0; i < 16; ++i) if (c0 + i <= lim) m = fmaxf(m, __uint_as_float(v[i]));
@@ -405,10 +407,10 @@ attn_fa_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
                 for (int c0 = 0; c0 < 64; c0 += 32) {
                     tmem_ld_wait16(va);
                     tmem_ld_32x16(t_half + (uint32_t)(c0 + 16), vb);
-                    emit_p(va, c0);
+                    emit_p(va, vb, c0);
                     tmem_ld_wait16(vb);
                     if (c0 == 0) tmem_ld_32x16(t_half + 32, va);
-                    emit_p(vb, c0 + 16);
+                    emit_p(vb, va, c0 + 16);
                 }
                 tmem_st_wait();
             }

@@ -81,3 +81,25 @@ def test_rising_scores(kind, causal):
     want = torch.softmax(s, -1) @ vi
     got = out.float().view(n, H, hd).transpose(0, 1)
     assert torch.isfinite(got).all() and (got - want).abs().max() <= 2.0 ** -7 * want.abs().max()
+
+
+@gpu
+@pytest.mark.parametrize("step", list(range(128, 256, 16)) + [133, 255])
+def test_a_raise_in_every_chunk(step):
+    """The reference is raised in each of the eight chunks of sixteen keys of a block, while the next chunk's scores are on their way:
+    keys from ``step`` on score 265 log2 units more and differ among themselves by up to four, so that scores of another chunk would
+    show.  Dense, 128 rows; bound as above."""
+    from ittai_b200 import ops
+    hd, n = 128, 300
+    g = torch.Generator(device="cuda").manual_seed(step)
+    u = torch.nn.functional.normalize(torch.randn(hd, generator=g, device="cuda"), dim=0)
+    j = torch.arange(n, device="cuda")
+    mag = torch.where(j >= step, 60.0, 0.0) + (j * 37 % 64).float() / 64
+    q = (u * 34.6).repeat(128, 1).to(torch.bfloat16)
+    kc, vc = (mag[:, None] * u).to(torch.bfloat16).view(1, 1, n, hd), torch.randn(1, 1, n, hd, generator=g, device="cuda").to(torch.bfloat16)
+    out, st = torch.zeros(128, hd, dtype=torch.bfloat16, device="cuda"), ops.new_status("cuda")
+    ops.attention(q, kc, vc, out, torch.tensor([[0, 128, 0, n]], dtype=torch.int32, device="cuda"), n_heads=1, group=1, head_dim=hd, causal=False, max_q_len=128,
+                  q_strides=(hd, hd), k_strides=(hd, n * hd, n * hd), v_strides=(hd, n * hd, n * hd), o_strides=(hd, hd), q_rows_total=128, kv_rows_total=n, status=st)
+    ops.check_status(st)
+    want = torch.softmax(q.double() @ kc[0, 0].double().t() / hd ** 0.5, -1) @ vc[0, 0].double()
+    assert (out.double() - want).abs().max() <= 2.0 ** -7 * want.abs().max()
