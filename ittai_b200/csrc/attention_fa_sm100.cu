@@ -61,6 +61,10 @@ __device__ __forceinline__ bool fa_wait(void* bar, uint32_t parity, volatile uin
     }
     return true;
 }
+// The same for a whole warp: one answer for all lanes, which go on with warp-wide steps.
+__device__ __forceinline__ bool fa_wait_warp(void* bar, uint32_t parity, volatile uint32_t* abort_flag) {
+    return __all_sync(0xffffffffu, fa_wait(bar, parity, abort_flag)) != 0;
+}
 __device__ __forceinline__ float fa_ex2(float x) {
     float y;
     asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
@@ -334,7 +338,7 @@ attn_fa_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
         bool ok = true;
         for (int j = 0; j < n_blk; ++j) {
             const uint32_t ph = (c + j) & 1;
-            ok = fa_wait(bar_s, ph, abort_flag);
+            ok = fa_wait_warp(bar_s, ph, abort_flag);
             tc_fence_after();
             if (j == 0) {
                 // the first block's exact maximum: where a few keys dominate a row, their P is then close to 1 and nearly free of rounding
@@ -417,7 +421,7 @@ attn_fa_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
             if (j == n_blk - 1 && (kv_len & (kFaBlk - 1)) != 0 && kv_len < (j + 1) * kFaBlk) {
                 // rows of the V tile past the sequence belong to a neighbour (or are unwritten cache): zero them, so that
                 // 0 * V stays 0 whatever they hold
-                if (ok) ok = fa_wait(bar_v, ph, abort_flag);
+                if (ok) ok = fa_wait_warp(bar_v, ph, abort_flag);
                 const int first = kv_len - j * kFaBlk;       // first row to clear
                 if (ok) {
                     for (int i = threadIdx.x - 32; i < (kFaBlk - first) * 16; i += 256) {
@@ -437,7 +441,7 @@ attn_fa_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
                 fa_rescale_p(t_half, 64, f);
                 ref = m;
                 if (j > 0) {
-                    ok = fa_wait(bar_o, (c + j - 1) & 1, abort_flag);        // O must be complete before it is rewritten
+                    ok = fa_wait_warp(bar_o, (c + j - 1) & 1, abort_flag);        // O must be complete before it is rewritten
                     tc_fence_after();
                     const float fo = fa_ex2(ref0 - m);
                     for (int c0 = 16 * half; ok && c0 < HDIM; c0 += 32) {
@@ -465,7 +469,7 @@ attn_fa_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
         if (n_blk > 0) {
         // ---- epilogue: O / rowsum -> bf16 -> staging tile (the V tile is dead) -> whole rows; the warps of a quarter take every
         //      other 16 columns, then 16 rows each
-        ok = fa_wait(bar_o, (c + n_blk - 1) & 1, abort_flag);
+        ok = fa_wait_warp(bar_o, (c + n_blk - 1) & 1, abort_flag);
         tc_fence_after();
         xrow[128 * half] = l2.x + l2.y;
         if (fa_vote(q4, !ok)) break;
@@ -500,7 +504,7 @@ attn_fa_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
         __syncwarp();
         if (lane == 0) fa_arrive(bar_e);
         c += n_blk;
-        if (fa_vote(q4, !fa_wait(bar_t + ((t + 1) & 1), (t >> 1) & 1, abort_flag))) break;
+        if (fa_vote(q4, !fa_wait_warp(bar_t + ((t + 1) & 1), (t >> 1) & 1, abort_flag))) break;
         index = next_tile[(t + 1) & 1];
         if (index < 0) break;
       }

@@ -179,11 +179,12 @@ gemm2_chain_kernel(const __grid_constant__ ChainParams P) {
             locate(t, gi, tile);
             if (gi + 1 >= n_g) continue;
             ++n;
+            bool gone = false;                                       // the same in every lane
             uint32_t spins = 0;
             while (!__all_sync(0xffffffffu, lane >= kEpiWarps || ld_acquire_cta_u32(&stored[lane & (kEpiWarps - 1)]) >= n)) {
-                if (((++spins) & 255u) == 0u && (*abort_flag || spins >= kSpin2)) { *abort_flag = 1; break; }
+                if (((++spins) & 255u) == 0u && __any_sync(0xffffffffu, *abort_flag || spins >= kSpin2)) { gone = true; break; }
             }
-            if (__any_sync(0xffffffffu, *abort_flag != 0)) break;
+            if (gone) { *abort_flag = 1; break; }
             __syncwarp();                                            // eight lanes have acquired a word each, lane 0 counts for all: votes order no memory
             if (lane == 0) {
                 fence_proxy_async();
@@ -230,6 +231,7 @@ gemm2_chain_kernel(const __grid_constant__ ChainParams P) {
                     if (((++spins) & 255u) == 0u && (*abort_flag || spins >= kSpin2)) { ok = false; break; }
                 }
             }
+            ok = __all_sync(0xffffffffu, ok);                         // one answer for all lanes: what follows is warp-wide
             if (!ok) { *abort_flag = 1; break; }
             if (gi > 0 && (fold || has_res)) {
                 if (lane == 0) {
@@ -266,6 +268,7 @@ gemm2_chain_kernel(const __grid_constant__ ChainParams P) {
                     if (((++spins) & 255u) == 0u && (*abort_flag || spins >= kSpin2)) { ok = false; break; }
                 }
             }
+            ok = __all_sync(0xffffffffu, ok);
             if (!ok) { *abort_flag = 1; break; }
             tc_fence_after();
             float st1 = 0.f, st2 = 0.f;                               // statistics of this row's output slice

@@ -267,12 +267,13 @@ gemm2_bf16_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constan
         float mean = 0.f, rstd = 1.f;
         uint32_t cache_row = 0;
         bool ok = true;
-        auto wait = [&](void* bar, uint32_t parity) {                // bounded, and given up when another role aborted
+        auto wait = [&](void* bar, uint32_t parity) {                // whole warp; bounded, given up when another role aborted; one answer for all lanes
+            bool done = true;
             uint32_t spins = 0;
             while (!mbar_try_wait_parked(bar, parity)) {
-                if (((++spins) & 255u) == 0u && (*abort_flag || spins >= kSpin2)) return false;
+                if (((++spins) & 255u) == 0u && (*abort_flag || spins >= kSpin2)) { done = false; break; }
             }
-            return true;
+            return __all_sync(0xffffffffu, done) != 0;
         };
         for (int tile = t_first; tile < t_end; tile += t_step, ++local) {
             const int buf = local & 1, round = local >> 1;

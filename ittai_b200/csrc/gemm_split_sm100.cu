@@ -320,7 +320,7 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constan
             while (!mbar_try_wait_parked(&full[s], use & 1)) {
                 if (((++spins) & 255u) == 0u && (*abort_flag || spins >= kSplitSpin)) { ok = false; break; }
             }
-            if (!ok) { *abort_flag = 1; break; }
+            if (!__all_sync(0xffffffffu, ok)) { *abort_flag = 1; break; }      // one answer for all lanes: warp-wide steps follow
             const uint32_t gw[4] = {gq.x, gq.y, gq.z, gq.w};
             constexpr int kStep = kNormThreads / 8;
 #pragma unroll 4
@@ -362,6 +362,7 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constan
             if (((++spins) & 255u) == 0u && (*abort_flag || spins >= kSplitSpin)) { ok = false; break; }
         }
     }
+    ok = __all_sync(0xffffffffu, ok);
     if (!ok) *abort_flag = 1;
     __syncwarp();
     tc_fence_after();
