@@ -14,8 +14,11 @@
 //     rescales what it has written, and a vote of the quarter's two warps, which ends every block, brings the other half and O
 //     to the same reference.  The halves' sums meet in the epilogue.
 //     (One thread a row, two passes, a maximum kept within 2^8: 175 us a layer at 8 x 2048 tokens, 135 at 64 x 512, 53 for 55 texts of
-//     16 to 512, 188 dense at 4 x 2048; this way 156, 128, 48 and 158, with the same error against 64 bits, of which the elected issuing
-//     lane gave about a third.  Without any softmax, the two CTAs' MMAs and hand-offs alone: 115 at 8 x 2048.)
+//     16 to 512, 188 dense at 4 x 2048; this way 156, 128, 48 and 158.  Of the difference, a third came with the elected issuing lane.
+//     Without any softmax, the two CTAs' MMAs and hand-offs alone: 115 at 8 x 2048.)
+//     The error against 64 bits is that of two passes for scores without an order (0.994 to 1.011 of it at 256 to 3000 keys and scores up
+//     to 30 log2 units wide).  What a raise finds already written is rounded to bf16 a second time, which two passes did not do: where the
+//     scores keep rising along the keys the result stays within 2^-7 of the largest value, as tested, but is not as exact.
 // TMEM (256 columns, two CTAs per SM): S / P in columns 0..127, O in 128..255.  Shared memory: Q, K, V tiles of 32 KB each
 // (two 128-byte-swizzled atoms of 64 dims); the V tile doubles as the output staging area.
 //
@@ -71,11 +74,6 @@ __device__ __forceinline__ float fa_ex2(float x) {
     return y;
 }
 
-__device__ __forceinline__ bool fa_test(void* bar, uint32_t parity) {
-    uint32_t ok;
-    asm volatile("{\n.reg .pred p;\nmbarrier.test_wait.parity.shared::cta.b64 p, [%1], %2;\nselp.u32 %0, 1, 0, p;\n}\n" : "=r"(ok) : "r"(smem_u32(bar)), "r"(parity) : "memory");
-    return ok != 0;
-}
 // Asks for a CTA of this grid that has not begun; the 16-byte answer is counted on `bar`.
 __device__ __forceinline__ void fa_try_cancel(void* answer, void* bar) {
     asm volatile("clusterlaunchcontrol.try_cancel.async.shared::cta.mbarrier::complete_tx::bytes.b128 [%0], [%1];" ::"r"(smem_u32(answer)), "r"(smem_u32(bar)) : "memory");
@@ -242,7 +240,7 @@ attn_fa_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
             // Takes the answer if it is there (or waits for it); an empty tile is passed over.
             auto resolve = [&](bool wait) {
                 while (next == -2) {
-                    if (!fa_test(bar_c, asked & 1)) {
+                    if (!mbar_test(bar_c, asked & 1)) {
                         if (!wait) return;
                         if (!fa_wait(bar_c, asked & 1, abort_flag)) { ok = false; return; }
                     }
@@ -292,7 +290,7 @@ attn_fa_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
                         fa_load(sm + kFaK, &tm_k, cur.kv_col, cur.kv_row + (j + 1) * kFaBlk, bar_k);
                     } else {
                         // the same for the next tile, if it is known before the softmax is through
-                        for (uint32_t spins = 0; next == -2 && spins < kFaSpin && !fa_test(bar_p, ph); ++spins) resolve(false);
+                        for (uint32_t spins = 0; next == -2 && spins < kFaSpin && !mbar_test(bar_p, ph); ++spins) resolve(false);
                         if (next >= 0) { load_next(); loaded = true; }
                     }
                     ok = fa_wait(bar_p, ph, abort_flag) && fa_wait(bar_v, ph, abort_flag);

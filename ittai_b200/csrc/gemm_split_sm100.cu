@@ -436,20 +436,25 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constan
 
 int cuda_fail(cudaError_t e, const char* what);
 
-// CTAs that share a tile's K: a power of two (clusters of 3, 5 or 7 cost 5-15 % more than the next smaller power), at least three
-// k-blocks each (12 k-blocks, 36 tiles: 7.2 us in four parts, 12.6 in eight), and two CTAs per SM at most save for a few
-// (48 tiles: 6.8 us as 192 CTAs, 7.1 as 96; 72 tiles: 10.0 us as 288 CTAs, 8.7 as 144).
+// CTAs that share a tile's K: a power of two (clusters of 3, 5 or 7 cost 5-15 % more than the next smaller power, measured with
+// tiles of 128 x 128), at least three k-blocks each (N 768 K 768, us in two / four / eight parts: M 128, 24 tiles, 4.3 / 3.5 / 3.8;
+// M 196, 48 tiles, 5.1 / 4.2 / 4.6), and no more CTAs than 7/4 per SM: beyond two per SM some run after the others (N 1024 K 3072 in
+// tiles of 64 rows: M 512, 128 tiles as 128 / 256 / 512 CTAs 11.1 / 8.9 / 15.0; M 1280, 160 / 320 CTAs 19.0 / 21.1).  Between 7/4 and
+// two per SM there is one such shape in reach, which the line leaves out (M 1152, 144 / 288 CTAs 18.8 / 12.6; it gets 14.2).
 static int split_log2(int tiles, int n_kb, int n_sms) {
     int lg = 0;
     while (2 << lg <= kMaxSplit && (2 << lg) * tiles * 4 <= 7 * n_sms && (2 << lg) * 3 <= n_kb) ++lg;
     return lg;
 }
 
-// The persistent pair kernel is the faster one as soon as a tile's K cannot be shared.  Measured on a B200 with weights from
-// HBM, us, pair kernel -> this one: N 1024 K 3072 at M 196 / 512 / 1024 / 1536: 22.0 -> 9.1, 22.0 -> 11.6, 22.3 -> 15.9,
-// 22.2 -> 25.0; N 768 K 768 at M 196 / 1536 / 2048: 9.3 -> 5.9, 9.6 -> 8.7, 9.7 -> 11.0; N 2304 K 768 at M 512 / 784:
-// 10.1 -> 8.8, 10.2 -> 11.6.  Against 128 x 64 tiles walked by one CTA each (M <= 128): N 1024 K 3072 at M 32 / 128 18.6 -> 6.1,
-// 19.0 -> 8.3; N 768 K 768 6.2 -> 4.2, 6.9 -> 5.9.
+// Up to half as many tiles of 128 x 128 as SMs.  Measured on a B200 with weights from HBM inside a CUDA graph, us, the kernel that
+// would run otherwise -> this one.  Pair kernel: N 1024 K 3072 at M 196 / 512 / 1024 / 1152 19.1 -> 7.3, 19.0 -> 8.9, 19.3 -> 11.9,
+// 19.5 -> 14.2, beyond the line at 1536 19.1 -> 15.9; N 768 K 768 at M 196 / 1024 / 1536 8.7 -> 3.7, 8.7 -> 5.7, 8.8 -> 7.6, beyond it at
+// 2048 8.8 -> 7.9; N 2304 K 768 at M 512 8.9 -> 7.7, beyond it at 784 9.0 -> 8.1.  128 x 64 tiles of one CTA each (M <= 128): N 1024
+// K 3072 at M 32 / 128 10.0 -> 4.6, 10.4 -> 6.5; N 768 K 768 4.5 -> 3.1, 5.2 -> 3.5; N 4096 K 1024 at M 128 5.8 -> 6.4, N 6144 6.7 -> 7.0.
+// The line dates from an earlier form of both kernels and lies on the safe side of today's crossing with the pair kernel.  The
+// one-CTA tiles, which only unsplit GEMMs reach above 128 rows, are the fastest of the three where they fill most of one round of the
+// SMs: 5.1 us for N 768 K 768 at M 1536, 10.3 for N 1024 K 3072 at M 1152, 5.4 for N 2304 K 768 at M 512.
 bool gemm_split_wins(int m, int n, int n_sms) { return m > 0 && n > 0 && 2ll * ((m + 127) / 128) * (n / SN) <= n_sms; }
 
 // Rows of a tile.  32 rows are the shortest chain while they cost nothing in splits and leave most SMs one CTA (N 768 K 768 at

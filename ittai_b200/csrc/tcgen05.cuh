@@ -147,11 +147,11 @@ __device__ __forceinline__ void tmem_ld_tie16(uint32_t (&r)[16]) {
                  :: "memory");
 }
 
-// True in one lane of a converged warp.  Roles that one thread carries (issuing TMA loads and MMAs) run inside `if (elect_one())`:
-// the compiler then knows that a single lane is active and keeps descriptors and addresses in uniform registers.  Inside
-// `if (lane == 0)` it moves every operand over for every instruction: on a B200 the issuing loop of a GEMM (wait, four
-// tcgen05.mma, commit) takes 594 cycles per k-block that way, whatever the width of the MMA, and 204 this way with mbar_test
-// asking for the next k-block ahead of this one's MMAs; four 128 x 128 x 16 MMAs themselves take 260.
+// True in one lane of a converged warp.  Roles that one thread carries (issuing TMA loads and MMAs) run inside `if (elect_one())`.
+// Measured on a B200: the issuing loop of a GEMM (wait, four tcgen05.mma, commit) takes 594 cycles per k-block inside
+// `if (lane == 0)`, whatever the width of the MMA, and 204 this way with mbar_test asking for the next k-block ahead of this one's
+// MMAs; four 128 x 128 x 16 MMAs themselves take 260.  (The likely cause: with elect.sync the compiler can tell that a single lane is
+// active, and these instructions take their operands from registers that a warp shares.)
 __device__ __forceinline__ bool elect_one() {
     uint32_t one;
     asm volatile(
