@@ -11,7 +11,7 @@
 //   stages are requested BEFORE griddepcontrol.wait: the caller has declared W constant (ITTAI_GEMM_STATIC_W), and two CTAs fit
 //   an SM, so the next GEMM's weights arrive while this one's epilogue runs;
 // * warp 1 (one lane) issues tcgen05.mma M128 N<rows> K16 into <rows> columns of tensor memory;
-// * with GemmArgs::a_gain the other six warps RMS-normalise each landed A tile in place (valid rows only, the rounding steps of
+// * with GemmArgs::a_gain the other warps, one or two to a stage, RMS-normalise each landed A tile in place (valid rows only, the rounding steps of
 //   rmsnorm_rows_kernel) before the MMAs read it: the norm's own launch, a kernel boundary and a round trip of the activations
 //   through L2 twice per layer, goes;
 // * a thread holds one column of the accumulator, a warp 32 neighbouring ones of every row: they are stored straight from the
@@ -439,8 +439,9 @@ int cuda_fail(cudaError_t e, const char* what);
 // CTAs that share a tile's K: a power of two (clusters of 3, 5 or 7 cost 5-15 % more than the next smaller power, measured with
 // tiles of 128 x 128), at least three k-blocks each (N 768 K 768, us in two / four / eight parts: M 128, 24 tiles, 4.3 / 3.5 / 3.8;
 // M 196, 48 tiles, 5.1 / 4.2 / 4.6), and no more CTAs than 7/4 per SM: beyond two per SM some run after the others (N 1024 K 3072 in
-// tiles of 64 rows: M 512, 128 tiles as 128 / 256 / 512 CTAs 11.1 / 8.9 / 15.0; M 1280, 160 / 320 CTAs 19.0 / 21.1).  Between 7/4 and
-// two per SM there is one such shape in reach, which the line leaves out (M 1152, 144 / 288 CTAs 18.8 / 12.6; it gets 14.2).
+// tiles of 64 rows: M 512, 128 tiles as 128 / 256 / 512 CTAs 11.1 / 8.9 / 15.0; M 1280, 160 / 320 CTAs 19.0 / 21.1).  The shapes between
+// 7/4 and two per SM, which 128 x 128 tiles lost on, would gain with today's (288 CTAs against what the line gives: N 1024 K 3072 at
+// M 1152 12.6 / 14.2, N 768 K 768 at M 1536 6.7 / 7.6, N 2304 K 768 at M 512 6.8 / 7.7).
 static int split_log2(int tiles, int n_kb, int n_sms) {
     int lg = 0;
     while (2 << lg <= kMaxSplit && (2 << lg) * tiles * 4 <= 7 * n_sms && (2 << lg) * 3 <= n_kb) ++lg;
