@@ -83,6 +83,11 @@ __device__ __forceinline__ float dot8(const uint4& w, const float* x, float acc)
 }
 
 // ---- reductions ----------------------------------------------------------------------------------
+// The warp's index in the CTA, as a value the compiler knows to be the same in all lanes.  Branches on threadIdx.x >> 5 count as
+// divergent for it: every shuffle, vote and .aligned instruction behind one then carries its own reconvergence (24 shuffles: 3.7 KB of
+// code instead of 1.7).  Every lane has to be there: called at the top of a kernel.
+__device__ __forceinline__ int warp_index() { return __shfl_sync(0xffffffffu, (int)(threadIdx.x >> 5), 0); }
+
 __device__ __forceinline__ float warp_sum(float v) {
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);

@@ -166,7 +166,7 @@ __global__ void __launch_bounds__(kGemvThreads, 2) gemv_kernel(const GemvArgs a)
     __shared__ __align__(16) bf16 gain_s[kNorm ? D : 8];
     __shared__ __align__(16) bf16 xs[kNorm ? NB * kXsLd : 8];
     __shared__ unsigned long long landed;
-    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, g = lane >> 2, t = lane & 3;
+    const int tid = threadIdx.x, warp = warp_index(), lane = tid & 31, g = lane >> 2, t = lane & 3;
     const int kc = ROWS == 32 ? warp & 7 : warp, tile = ROWS == 32 ? warp >> 3 : 0;
     const int row0 = blockIdx.x * ROWS;
     const int col = kc * KW + 8 * t;
@@ -294,7 +294,7 @@ __global__ void __launch_bounds__(kGemvThreads + 32, 1) head_kernel(const HeadAr
     __shared__ __align__(16) bf16 xs[NB * kXsLd];
     __shared__ unsigned long long full[kHeadRing], empty[kHeadRing];
     __shared__ volatile uint32_t failed;
-    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, g = lane >> 2, t = lane & 3;
+    const int tid = threadIdx.x, warp = warp_index(), lane = tid & 31, g = lane >> 2, t = lane & 3;
     const int r_lo = (int)((long long)a.vocab * blockIdx.x / gridDim.x), r_hi = (int)((long long)a.vocab * (blockIdx.x + 1) / gridDim.x);
     const int n_it = (r_hi - r_lo + kHeadRows - 1) / kHeadRows;
     if (tid == 0) {
@@ -404,7 +404,7 @@ __device__ __forceinline__ void embed_row(const TokenArgs& a, int b, int id, int
 // and positions, gathers the first embedding rows.
 template <int NB>
 __global__ void __launch_bounds__(32 * NB) begin_kernel(const TokenArgs a, int32_t* out_ids, const int32_t* forced, uint64_t* step_ns, int n_steps, int n_forced) {
-    const int b = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int b = warp_index(), lane = threadIdx.x & 31;
     __shared__ int bad;
     if (threadIdx.x < ITTAI_STATUS_WORDS) a.status[threadIdx.x] = 0u;
     if (threadIdx.x == 0) {
@@ -434,7 +434,7 @@ template <int NB, bool HEAD>
 __global__ void __launch_bounds__(32 * NB) finish_kernel(const TokenArgs a) {
     pdl_trigger();
     pdl_wait();
-    const int b = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int b = warp_index(), lane = threadIdx.x & 31;
     __shared__ int bad, stopped;
     State* st = a.st;
     const int step = st->step, n_steps = st->n_steps, pos = st->cur_pos[b];
@@ -491,7 +491,14 @@ __global__ void __launch_bounds__(32 * NB) finish_kernel(const TokenArgs a) {
 // compute warps take turns on 32-position tiles, a warp 16 positions of each with its own softmax; a seventh warp feeds a ring
 // of six 16 KB tiles (two CTAs per SM).  A warp's 16 positions are 16 MMAs: scores with the keys as A (M = positions) and the two query heads as N columns, P V with
 // V^T as A (ldmatrix.trans on the swizzled tile) and P as B, its middle, low and high parts in columns 0-1, 2-3 and 4-5.
-// A tile is about 1000 dependent cycles for a warp, which is why the tiles are small and the warps many.
+// A tile is about 1000 dependent cycles for a warp the first time and 600 from then on, which is why the tiles are small and the warps
+// many; the difference is instruction supply.  Every kernel of a layer runs once, so its code comes from the second-level instruction
+// cache at about three cycles an instruction: code off the straight path costs the same as data that has to be fetched.  Hence the warp
+// index as a uniform value, rolled loops where nothing is gained by unrolling, packed bf16 arithmetic in the rotation, the operand words
+// of q in the order in which a lane reads them, and one pass over the merge: 34.9 -> 19.7 KB.  With the partials sent by st.async instead
+// of stored ahead of a second cluster barrier (1500 cycles of 6300), us per step before -> after: batch 1 at 47 / 800 / 4096 / 8000
+// positions 420 -> 390, 440 -> 409, 520 -> 498, 584 -> 573; batch 2 and 4 at 1000 475 -> 450 and 530 -> 497; batch 8 at 1000 / 8100
+// 681 -> 629 and 1587 -> 1563.
 constexpr int kGroups = 3, kAttnWarps = 2 * kGroups, kAttnThreads = 32 * kAttnWarps + 32, kTilePos = 32, kRing = 2 * kGroups;
 // Tile `it` belongs to group it % 3, which has two ring slots of its own: a slot's phases are waited for by the same two
 // warps in order (a slot shared by groups that skip each other's phases cannot be told apart by parity).
@@ -540,10 +547,27 @@ __device__ __forceinline__ void tma_load_2d_hint(void* dst, const void* tmap, in
 }
 // Byte address of the 16-byte chunk `chunk` (0..7) of row `row` of a half tile under the 128-byte swizzle.
 __device__ __forceinline__ uint32_t swz(uint32_t base, int row, int chunk) { return base + (uint32_t)row * 128u + (uint32_t)((chunk ^ (row & 7)) << 4); }
-__device__ __forceinline__ void st_cluster_f32(float* p, int rank, float v) {
-    uint32_t a;
-    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(a) : "r"(smem_u32(p)), "r"(rank));
-    asm volatile("st.shared::cluster.f32 [%0], %1;" ::"r"(a), "f"(v) : "memory");
+// Two floats into rank `rank`'s copy of `p`, counted on its copy of `bar`.
+__device__ __forceinline__ void st_async_f32x2(void* p, int rank, float x, float y, void* bar) {
+    asm volatile("st.async.weak.shared::cluster.mbarrier::complete_tx::bytes.v2.f32 [%0], {%1, %2}, [%3];"
+                 ::"r"(map_to_cta(p, (uint32_t)rank)), "f"(x), "f"(y), "r"(map_to_cta(bar, (uint32_t)rank)) : "memory");
+}
+// The data of st_async_f32x2 from other CTAs is visible once this has returned true.
+__device__ __forceinline__ bool mbar_try_wait_cluster(void* bar, uint32_t parity) {
+    uint32_t ok;
+    asm volatile("{\n.reg .pred p;\nmbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2;\nselp.u32 %0, 1, 0, p;\n}\n"
+                 : "=r"(ok) : "r"(smem_u32(bar)), "r"(parity) : "memory");
+    return ok != 0;
+}
+__device__ __forceinline__ uint32_t mul_bf16x2(uint32_t a, uint32_t b) {
+    uint32_t d;
+    asm("mul.rn.bf16x2 %0, %1, %2;" : "=r"(d) : "r"(a), "r"(b));
+    return d;
+}
+__device__ __forceinline__ uint32_t add_bf16x2(uint32_t a, uint32_t b) {
+    uint32_t d;
+    asm("add.rn.bf16x2 %0, %1, %2;" : "=r"(d) : "r"(a), "r"(b));
+    return d;
 }
 
 // log2 of the pieces that the cache of a sequence with `len` positions is cut into, one CTA each.  Measured over all splits and
@@ -568,20 +592,25 @@ template <int CS>
 __global__ void __launch_bounds__(kAttnThreads, 2) attn_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constant__ CUtensorMap tm_v, const AttnChainArgs a) {
     extern __shared__ __align__(1024) unsigned char ring_raw[];
     unsigned char* ring = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(ring_raw) + 1023) & ~(uintptr_t)1023);
-    __shared__ unsigned long long full[kRing], empty[kRing];
-    __shared__ __align__(16) bf16 q_s[2][HD];
+    constexpr int NE = 2 * HD / CS;                             // outputs that a rank merges
+    __shared__ unsigned long long full[kRing], empty[kRing], arrived;
+    __shared__ __align__(16) uint32_t q_s[2][4][20];            // [head][t]: the 16 words that lane t of a quad holds as MMA operand
     __shared__ __align__(16) bf16 k_s[HD];
-    __shared__ float pm[kAttnWarps + 1][2], pl[kAttnWarps + 1][2], po[kAttnWarps + 1][2][HD];   // partials of the warps and of the new position
+    __shared__ __align__(8) float2 pml[2][kAttnWarps + 1];      // reference and sum of the warps' partials and of the new position
+    __shared__ __align__(8) float po[kAttnWarps + 1][2][HD];
     __shared__ __align__(8) bf16 rot_s[4][HD];                  // q gain, k gain, cos | sin of the new position
-    __shared__ float rv[CS][CS == 1 ? 1 : 2 * HD / CS], rm[CS][2], rl[CS][2];     // partials of all ranks for this rank's outputs
+    __shared__ __align__(8) float rv[CS][CS == 1 ? 2 : NE];     // partials of all ranks for this rank's outputs, which are of one head
+    __shared__ __align__(8) float2 rml[CS];
     __shared__ volatile uint32_t failed;
-    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const int tid = threadIdx.x, warp = warp_index(), lane = tid & 31;
     const int rank = CS == 1 ? 0 : (int)(blockIdx.x % CS), item = blockIdx.x / CS, b = item / NKV, kvh = item % NKV;
     const size_t head_row = (size_t)(a.layer * a.batch + b) * NKV + kvh;          // in units of kv_cap rows of the whole cache
     if (tid == 0) {
         for (int s = 0; s < kRing; ++s) { mbar_init(&full[s], 1); mbar_init(&empty[s], 2); }
         failed = 0;
+        mbar_init(&arrived, 1);
         fence_mbar_init();
+        if constexpr (CS > 1) mbar_expect_tx(&arrived, CS * (NE * 4 + 8));
     }
     __syncthreads();
     // another CTA's shared memory may be written only once that CTA runs: every thread arrives here, waits before the merge
@@ -611,12 +640,9 @@ __global__ void __launch_bounds__(kAttnThreads, 2) attn_kernel(const __grid_cons
     if (warp == kAttnWarps) {
         if (lane == 0) {
             asm volatile("createpolicy.fractional.L2::evict_first.b64 %0, 1.0;" : "=l"(policy));
-            for (int it = 0; it < n_tiles && it < kRing; ++it) issue(it);
-        }
-        pdl_wait();
-        if (lane == 0) {
-            for (int it = kRing; it < n_tiles; ++it) {
-                if (!mbar_wait_bounded(&empty[ring_slot(it)], ring_parity(it) ^ 1, a.limit_parked)) { failed = 1; break; }
+#pragma unroll 1
+            for (int it = 0; it < n_tiles; ++it) {
+                if (it >= kRing && !mbar_wait_bounded(&empty[ring_slot(it)], ring_parity(it) ^ 1, a.limit_parked)) { failed = 1; break; }
                 issue(it);
             }
         }
@@ -637,55 +663,56 @@ __global__ void __launch_bounds__(kAttnThreads, 2) attn_kernel(const __grid_cons
         const int group = warp >> 1, w4 = warp & 1;              // the warp's 16 rows of its group's tiles
         const int krow = 16 * w4 + (mat & 1) * 8 + r8, kchunk = mat >> 1;       // keys: rows +8 in matrix bit 0, columns +8 in bit 1
         const int vrow = 16 * w4 + (mat >> 1) * 8 + r8, vchunk = mat & 1;       // values: the other way round
+        const uint32_t k_off = swz(0u, krow, kchunk), v_off = swz(0u, vrow, vchunk);
         pdl_wait();
         const bool owner = rank == 0 && pos >= 0;             // of the new position
-        float r[4] = {0.f, 0.f, 0.f, 0.f};
+        uint2 r = make_uint2(0u, 0u);
         {
             uint2 u = make_uint2(0u, 0u);
             if (warp < 4) asm volatile("ld.global.cg.v2.u32 {%0,%1}, [%2];" : "=r"(u.x), "=r"(u.y) : "l"(src_row));
-            float x[4] = {bf_lo(u.x), bf_hi(u.x), bf_lo(u.y), bf_hi(u.y)};
+            const float x[4] = {bf_lo(u.x), bf_hi(u.x), bf_lo(u.y), bf_hi(u.y)};
             if (warp == 3) {
                 if (owner) {
                     *reinterpret_cast<uint2*>(a.vcache + cache_row) = u;
-#pragma unroll
-                    for (int j = 0; j < 4; ++j) { po[kAttnWarps][0][4 * lane + j] = x[j]; po[kAttnWarps][1][4 * lane + j] = x[j]; }
+                    *reinterpret_cast<float4*>(&po[kAttnWarps][0][4 * lane]) = make_float4(x[0], x[1], x[2], x[3]);
+                    *reinterpret_cast<float4*>(&po[kAttnWarps][1][4 * lane]) = make_float4(x[0], x[1], x[2], x[3]);
                 }
             } else if (is_q || (warp == 2 && owner)) {
+                // the rounding steps of qk_rope_scatter_kernel on packed pairs: a product or a sum of two bf16 values, rounded once
                 const float ss = warp_sum(x[0] * x[0] + x[1] * x[1] + x[2] * x[2] + x[3] * x[3]);
                 const float rstd = rsqrt_full(ss * (1.0f / HD) + a.eps);
                 const uint2 gq = *reinterpret_cast<const uint2*>(&rot_s[is_q ? 0 : 1][4 * lane]);
                 const uint2 cq = *reinterpret_cast<const uint2*>(&rot_s[2][ei]), sq = *reinterpret_cast<const uint2*>(&rot_s[2][HD / 2 + ei]);
-                const float gn[4] = {bf_lo(gq.x), bf_hi(gq.x), bf_lo(gq.y), bf_hi(gq.y)};
-                const float cs[4] = {bf_lo(cq.x), bf_hi(cq.x), bf_lo(cq.y), bf_hi(cq.y)};
-                const float sn[4] = {bf_lo(sq.x), bf_hi(sq.x), bf_lo(sq.y), bf_hi(sq.y)};
-#pragma unroll
-                for (int j = 0; j < 4; ++j) {
-                    x[j] = bf16r(bf16r(x[j] * rstd) * gn[j]);
-                    const float y = __shfl_xor_sync(0xffffffffu, x[j], 16);      // element j +- 64
-                    r[j] = hi_half ? bf16r(bf16r(x[j] * cs[j]) + bf16r(y * sn[j])) : bf16r(bf16r(x[j] * cs[j]) + bf16r(-y * sn[j]));
+                const uint32_t n0 = mul_bf16x2(pack_bf16x2(x[0] * rstd, x[1] * rstd), gq.x), n1 = mul_bf16x2(pack_bf16x2(x[2] * rstd, x[3] * rstd), gq.y);
+                const uint32_t neg = hi_half ? 0u : 0x80008000u;
+                const uint32_t y0 = __shfl_xor_sync(0xffffffffu, n0, 16) ^ neg, y1 = __shfl_xor_sync(0xffffffffu, n1, 16) ^ neg;      // elements j +- 64
+                r.x = add_bf16x2(mul_bf16x2(n0, cq.x), mul_bf16x2(y0, sq.x));
+                r.y = add_bf16x2(mul_bf16x2(n1, cq.y), mul_bf16x2(y1, sq.y));
+                if (is_q) {                        // words 2 lane and 2 lane + 1: k-step lane / 4, half (lane / 2) % 2, t = 2 (lane % 2) and the next
+                    uint32_t* w = &q_s[warp][2 * (lane & 1)][2 * (lane >> 2) + ((lane >> 1) & 1)];
+                    w[0] = r.x; w[20] = r.y;
+                } else {
+                    *reinterpret_cast<uint2*>(k_s + 4 * lane) = r;
+                    *reinterpret_cast<uint2*>(a.kcache + cache_row) = r;
                 }
-                const uint2 pk = make_uint2(pack_bf16x2(r[0], r[1]), pack_bf16x2(r[2], r[3]));
-                *reinterpret_cast<uint2*>((is_q ? q_s[warp] : k_s) + 4 * lane) = pk;
-                if (!is_q) *reinterpret_cast<uint2*>(a.kcache + cache_row) = pk;
             }
         }
         compute_sync();
         if (warp < 2) {
             if (owner) {                           // the new position's score for this head
                 const uint2 k2 = *reinterpret_cast<const uint2*>(k_s + 4 * lane);
-                const float s = warp_sum(r[0] * bf_lo(k2.x) + r[1] * bf_hi(k2.x) + r[2] * bf_lo(k2.y) + r[3] * bf_hi(k2.y));
-                if (lane == 0) { pm[kAttnWarps][warp] = s * kScoreScale; pl[kAttnWarps][warp] = 1.f; }
+                const float s = warp_sum(bf_lo(r.x) * bf_lo(k2.x) + bf_hi(r.x) * bf_hi(k2.x) + bf_lo(r.y) * bf_lo(k2.y) + bf_hi(r.y) * bf_hi(k2.y));
+                if (lane == 0) pml[warp][kAttnWarps] = make_float2(s * kScoreScale, 1.f);
             } else {
-                if (lane == 0) { pm[kAttnWarps][warp] = -INFINITY; pl[kAttnWarps][warp] = 0.f; }
-#pragma unroll
-                for (int j = 0; j < 4; ++j) po[kAttnWarps][warp][4 * lane + j] = 0.f;
+                if (lane == 0) pml[warp][kAttnWarps] = make_float2(-INFINITY, 0.f);
+                *reinterpret_cast<float4*>(&po[kAttnWarps][warp][4 * lane]) = make_float4(0.f, 0.f, 0.f, 0.f);
             }
         }
-        uint32_t qb[8][2];
+        uint32_t qb[8][2];                                     // N columns: heads 0, 1, 0, 1, ...
 #pragma unroll
-        for (int k = 0; k < 8; ++k) {
-            qb[k][0] = *reinterpret_cast<const uint32_t*>(&q_s[g & 1][16 * k + 2 * t]);         // N columns: heads 0, 1, 0, 1, ...
-            qb[k][1] = *reinterpret_cast<const uint32_t*>(&q_s[g & 1][16 * k + 8 + 2 * t]);
+        for (int k = 0; k < 8; k += 2) {
+            const uint4 q = *reinterpret_cast<const uint4*>(&q_s[g & 1][t][2 * k]);
+            qb[k][0] = q.x; qb[k][1] = q.y; qb[k + 1][0] = q.z; qb[k + 1][1] = q.w;
         }
         float m0 = -INFINITY, m1 = -INFINITY, l0 = 0.f, l1 = 0.f;
         float o[8][4];
@@ -697,12 +724,14 @@ __global__ void __launch_bounds__(kAttnThreads, 2) attn_kernel(const __grid_cons
             bool ok = true;
             uint32_t spins = 0;
             while (!mbar_try_wait(&full[s], ring_parity(it))) { if (++spins >= a.limit || failed) { ok = false; break; } }
-            if (!ok) { failed = 1; break; }
+            if (!__all_sync(0xffffffffu, ok)) { failed = 1; break; }          // one answer for the warp
             const int nv = p1 - p0 - it * kTilePos - 16 * w4;  // valid positions of this warp's sixteen
             if (nv > 0) {
                 const uint32_t tk = smem_u32(ring + s * kTileBytes), tv = tk + 2 * kHalfTile;
+                const uint32_t ak = tk + k_off, av = tv + v_off;               // chunk 0 of this lane's row; chunk 2 c: that ^ (c << 5)
                 if (nv < 16) {
                     // rows past the sequence: whatever the cache holds there (it may be NaN) must not reach P V
+#pragma unroll 1
                     for (int i = lane; i < (16 - nv) * 16; i += 32) {
                         const int row = 16 * w4 + nv + (i >> 4), c = i & 15;
                         asm volatile("st.shared.v4.u32 [%0], {%1, %1, %1, %1};" ::"r"(swz(tv + (c >> 3) * kHalfTile, row, c & 7)), "r"(0u) : "memory");
@@ -713,9 +742,9 @@ __global__ void __launch_bounds__(kAttnThreads, 2) attn_kernel(const __grid_cons
 #pragma unroll
                 for (int k = 0; k < 8; k += 2) {
                     uint32_t f[4];
-                    ldsm4(f, swz(tk + (k >> 2) * kHalfTile, krow, 2 * (k & 3) + kchunk));
+                    ldsm4(f, (ak ^ ((k & 3) << 5)) + (k >> 2) * kHalfTile);
                     mma16816(sa, f[0], f[1], f[2], f[3], qb[k][0], qb[k][1]);
-                    ldsm4(f, swz(tk + (k >> 2) * kHalfTile, krow, 2 * ((k + 1) & 3) + kchunk));
+                    ldsm4(f, (ak ^ (((k + 1) & 3) << 5)) + (k >> 2) * kHalfTile);
                     mma16816(sb, f[0], f[1], f[2], f[3], qb[k + 1][0], qb[k + 1][1]);
                 }
                 // every lane holds (position g, heads 0 and 1) and (position g + 8, ...)
@@ -752,7 +781,7 @@ __global__ void __launch_bounds__(kAttnThreads, 2) attn_kernel(const __grid_cons
 #pragma unroll
                 for (int i = 0; i < 8; ++i) {
                     uint32_t f[4];
-                    ldsm4_t(f, swz(tv + (i >> 2) * kHalfTile, vrow, 2 * (i & 3) + vchunk));
+                    ldsm4_t(f, (av ^ ((i & 3) << 5)) + (i >> 2) * kHalfTile);
                     mma16816(o[i], f[0], f[1], f[2], f[3], b0, b1);
                 }
             }
@@ -761,7 +790,7 @@ __global__ void __launch_bounds__(kAttnThreads, 2) attn_kernel(const __grid_cons
         }
 #pragma unroll
         for (int of = 4; of < 32; of <<= 1) { l0 += __shfl_xor_sync(0xffffffffu, l0, of); l1 += __shfl_xor_sync(0xffffffffu, l1, of); }
-        if (lane == 0) { pm[warp][0] = m0; pm[warp][1] = m1; pl[warp][0] = l0; pl[warp][1] = l1; }
+        if (lane == 0) { pml[0][warp] = make_float2(m0, l0); pml[1][warp] = make_float2(m1, l1); }
         // The three parts of an output lie in lanes t = 0, 1, 2: added up (middle + low, then high) in two exchanges that leave each
         // lane a quarter of the sums, lane t the rows with bit 3 = t & 1 and bit 4 = t >> 1, so that the 32 lanes of a store hit
         // 32 banks.
@@ -779,42 +808,48 @@ __global__ void __launch_bounds__(kAttnThreads, 2) attn_kernel(const __grid_cons
         compute_sync();
         bf16* out = a.attn + (size_t)b * DQ + 2 * kvh * HD;
         if constexpr (CS > 1) asm volatile("barrier.cluster.wait.acquire;" ::: "memory");
+        // two outputs a thread; with more than one rank the partials go to the rank that owns them (st.async: the receiver waits for
+        // the bytes on a barrier of its own, one way, where stores and a cluster barrier took a round trip more)
+        if (tid < HD) {
+            const int e = 2 * tid, h = tid >> 6, d = e % HD;
+            float m = -1e30f, l = 0.f;
+            float2 acc = make_float2(0.f, 0.f);
 #pragma unroll
-        for (int e0 = 0; e0 < 2 * HD; e0 += 32 * kAttnWarps) {
-            const int e = e0 + tid, h = e / HD, d = e % HD;
-            if (e >= 2 * HD) break;
-            float m = -1e30f, l = 0.f, acc = 0.f;
+            for (int w = 0; w <= kAttnWarps; ++w) m = fmaxf(m, pml[h][w].x);
 #pragma unroll
-            for (int w = 0; w <= kAttnWarps; ++w) m = fmaxf(m, pm[w][h]);
-#pragma unroll
-            for (int w = 0; w <= kAttnWarps; ++w) { const float c = ex2f(pm[w][h] - m); l = fmaf(pl[w][h], c, l); acc = fmaf(po[w][h][d], c, acc); }
+            for (int w = 0; w <= kAttnWarps; ++w) {
+                const float2 ml = pml[h][w], p = *reinterpret_cast<const float2*>(&po[w][h][d]);
+                const float c = ex2f(ml.x - m);
+                l = fmaf(ml.y, c, l); acc.x = fmaf(p.x, c, acc.x); acc.y = fmaf(p.y, c, acc.y);
+            }
             if constexpr (CS == 1) {
-                out[e] = __float2bfloat16_rn(l > 0.f ? acc / l : 0.f);
+                *reinterpret_cast<uint32_t*>(out + e) = l > 0.f ? pack_bf16x2(acc.x / l, acc.y / l) : 0u;
             } else {
-                // each rank merges NE of the 256 outputs: the partial goes to the rank that owns it
-                constexpr int NE = 2 * HD / CS;
-                st_cluster_f32(&rv[rank][e % NE], e / NE, acc);
-                if (d < CS) { st_cluster_f32(&rm[rank][h], d, m); st_cluster_f32(&rl[rank][h], d, l); }
+                st_async_f32x2(&rv[rank][e % NE], e / NE, acc.x, acc.y, &arrived);
+                if (e % NE == 0) st_async_f32x2(&rml[rank], e / NE, m, l, &arrived);
             }
         }
         if constexpr (CS > 1) {
-            cluster_sync_all();
-            constexpr int NE = 2 * HD / CS;
-            if (tid < NE) {
-                const int e = rank * NE + tid, h = e / HD;
-                float m = -1e30f, acc = 0.f, l = 0.f;
+            if (tid < NE / 2) {
+                uint32_t spins = 0;
+                while (!mbar_try_wait_cluster(&arrived, 0)) { if (++spins >= a.limit) { failed = 1; break; } }
+                float m = -1e30f, l = 0.f;
+                float2 acc = make_float2(0.f, 0.f);
 #pragma unroll
-                for (int q = 0; q < CS; ++q) m = fmaxf(m, rm[q][h]);
+                for (int q = 0; q < CS; ++q) m = fmaxf(m, rml[q].x);
 #pragma unroll
-                for (int q = 0; q < CS; ++q) { const float c = ex2f(rm[q][h] - m); acc = fmaf(rv[q][tid], c, acc); l = fmaf(rl[q][h], c, l); }
-                out[e] = __float2bfloat16_rn(l > 0.f ? acc / l : 0.f);
+                for (int q = 0; q < CS; ++q) {
+                    const float2 ml = rml[q], p = *reinterpret_cast<const float2*>(&rv[q][2 * tid]);
+                    const float c = ex2f(ml.x - m);
+                    l = fmaf(ml.y, c, l); acc.x = fmaf(p.x, c, acc.x); acc.y = fmaf(p.y, c, acc.y);
+                }
+                *reinterpret_cast<uint32_t*>(out + rank * NE + 2 * tid) = l > 0.f ? pack_bf16x2(acc.x / l, acc.y / l) : 0u;
             }
         }
     }
     if constexpr (CS > 1) {
-        if (warp == kAttnWarps) {                                // the feeding warp's share of the two barriers
+        if (warp == kAttnWarps) {                                // the feeding warp's share of the barrier
             asm volatile("barrier.cluster.wait.acquire;" ::: "memory");
-            cluster_sync_all();
         }
     }
     __syncthreads();
