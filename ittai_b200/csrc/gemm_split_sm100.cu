@@ -227,7 +227,7 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constan
     volatile uint32_t* abort_flag = tmem_slot + 1;
     static_assert(3 * kStages + 2 <= 16, "barriers and flags end before the row scales");
 
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int warp = warp_index(), lane = threadIdx.x & 31;
     const int rank = blockIdx.x, splits = 1 << lg, tile_n = blockIdx.y, row_base = blockIdx.z * tile_rows;
     const int n_kb_all = g.K / SK, kb0 = n_kb_all * rank >> lg, n_kb = (n_kb_all * (rank + 1) >> lg) - kb0;   // >= 1: splits <= K / 64
     const int rows = min(tile_rows, g.M - row_base);
