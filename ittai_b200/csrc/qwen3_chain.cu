@@ -124,6 +124,12 @@ __device__ __forceinline__ void norm_rows(const bf16* x, const bf16* gain_s, bf1
     gemv_sync();
 }
 
+__device__ __forceinline__ uint4 lds128(const void* p) {          // volatile: stays where it is written
+    uint4 v;
+    asm volatile("ld.shared.v4.u32 {%0,%1,%2,%3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "r"(smem_u32(p)) : "memory");
+    return v;
+}
+
 enum { kPlain = 0, kSwiglu = 1, kResidual = 2 };
 
 struct GemvArgs {
@@ -181,7 +187,9 @@ __global__ void __launch_bounds__(kGemvThreads, 2) gemv_kernel(const GemvArgs a)
         constexpr int kItems = NB * NKV, kParts = DGU / 48 / kItems;
         const int item = blockIdx.x % kItems, piece = blockIdx.x / kItems;
         int pos = (int)ld_relaxed(reinterpret_cast<const uint32_t*>(&a.st->cur_pos[item / NKV]));
-        if ((long long)NB * NKV * pos * HD * 4 > (24 << 20)) pos = 0;            // more than L2 keeps until it is read
+        // More than L2 keeps until it is read.  us per step without / with it: batch 1 at 6500 / 8000 positions (27 / 33 MB a layer) 554 / 531
+        // and 588 / 570, batch 2 at 3500 / 5000 (29 / 41 MB) 548 / 532 and 595 / 606, batch 4 at 1800 (29 MB) 549 / 550, batch 8 at 1000 (33 MB) 614 / 645.
+        if ((long long)NB * NKV * pos * HD * 4 > ((NB <= 2 ? 36 : 24) << 20)) pos = 0;
         const int q0 = (int)((long long)pos * piece / kParts), q1 = (int)((long long)pos * (piece + 1) / kParts);
         for (int q = q0 + 32 * lane; q < q1; q += 32 * 32) {
             const uint32_t n = (uint32_t)(q1 - q < 32 ? q1 - q : 32) * HD * 2;
@@ -195,6 +203,24 @@ __global__ void __launch_bounds__(kGemvThreads, 2) gemv_kernel(const GemvArgs a)
     if constexpr (kNorm) reinterpret_cast<uint32_t*>(gain_s)[tid] = reinterpret_cast<const uint32_t*>(a.gain)[tid];
     __syncthreads();                                   // the barrier exists for every warp, and the gain has arrived: a load
                                                        // left open here may be scheduled behind the wait
+    // A warp's weights in registers ahead of the wait: 64 KB of a QKV slice take the shared memory 512 cycles, which stood between the
+    // activations and the sums.  Gate/up would need 48 registers for it on top of its own and starts late (its last CTAs find room when
+    // attention ends): held there too, us per step 512 instead of 485 (batch 1, 4096), 499 instead of 482 (batch 4, 1000).  Waiting for the
+    // weights in front of the dependency costs nothing where they are late: asking once and loading the activations first
+    // 413 instead of 400 (batch 1, 800).  None held -> this: batch 1 at 47 / 4096 391 -> 380, 498 -> 485, batch 4 and 8 at 1000 497 -> 482, 629 -> 614.
+    constexpr bool kHeld = ROWS != 48;
+    uint4 wl[kHeld ? NT : 1][kHeld ? NJ : 1], wh[kHeld && NR == 2 ? NT : 1][kHeld && NR == 2 ? NJ : 1];
+    bool ok = true;
+    if constexpr (kHeld) {
+        ok = mbar_wait_bounded(&landed, 0, a.limit);
+#pragma unroll
+        for (int n = 0; n < NT; ++n)
+#pragma unroll
+            for (int j = 0; j < NJ; ++j) {
+                wl[n][j] = lds128(wr + 16 * n * LD + 64 * j);
+                if constexpr (NR == 2) wh[n][j] = lds128(wr + (16 * n + 8) * LD + 64 * j);
+            }
+    }
     pdl_wait();
     if (a.late_trigger) pdl_trigger();
     uint4 x[NJ];
@@ -208,14 +234,15 @@ __global__ void __launch_bounds__(kGemvThreads, 2) gemv_kernel(const GemvArgs a)
     if constexpr (EPI == kResidual) {
         if (tid < 8 * NB) res = ldcg_bf16(a.res + (size_t)(tid >> 3) * D + row0 + (tid & 7));
     }
-    const bool ok = mbar_wait_bounded(&landed, 0, a.limit);
+    if constexpr (!kHeld) ok = mbar_wait_bounded(&landed, 0, a.limit);
 #pragma unroll
     for (int n = 0; n < NT; ++n) {
         float d0[4] = {0.f, 0.f, 0.f, 0.f}, d1[4] = {0.f, 0.f, 0.f, 0.f};
 #pragma unroll
         for (int j = 0; j < NJ; ++j) {
-            const uint4 lo = *reinterpret_cast<const uint4*>(wr + 16 * n * LD + 64 * j);
-            const uint4 hi = NR == 2 ? *reinterpret_cast<const uint4*>(wr + (16 * n + 8) * LD + 64 * j) : make_uint4(0u, 0u, 0u, 0u);
+            uint4 lo, hi = make_uint4(0u, 0u, 0u, 0u);
+            if constexpr (kHeld) { lo = wl[n][j]; if constexpr (NR == 2) hi = wh[n][j]; }
+            else { lo = lds128(wr + 16 * n * LD + 64 * j); if constexpr (NR == 2) hi = lds128(wr + (16 * n + 8) * LD + 64 * j); }
             mma16816(d0, lo.x, hi.x, lo.y, hi.y, x[j].x, x[j].y);
             mma16816(d1, lo.z, hi.z, lo.w, hi.w, x[j].z, x[j].w);
         }
