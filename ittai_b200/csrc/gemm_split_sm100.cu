@@ -11,12 +11,13 @@
 //   stages are requested BEFORE griddepcontrol.wait: the caller has declared W constant (ITTAI_GEMM_STATIC_W), and two CTAs fit
 //   an SM, so the next GEMM's weights arrive while this one's epilogue runs;
 // * warp 1 (one lane) issues tcgen05.mma M128 N<rows> K16 into <rows> columns of tensor memory;
-// * with GemmArgs::a_gain the other warps, one or two to a stage, RMS-normalise each landed A tile in place (valid rows only, the rounding steps of
+// * with GemmArgs::a_gain the other warps RMS-normalise each landed A tile in place (valid rows only, the rounding steps of
 //   rmsnorm_rows_kernel) before the MMAs read it: the norm's own launch, a kernel boundary and a round trip of the activations
-//   through L2 twice per layer, goes;
+//   through L2 twice per layer, goes.  All six take every k-block where there are no more of them than stages, otherwise one or two keep
+//   to a stage;
 // * a thread holds one column of the accumulator, a warp 32 neighbouring ones of every row: they are stored straight from the
-//   registers into the shared memory of the CTA that finishes the row (row r: rank r mod splits), one cluster barrier follows,
-//   and the epilogue reads only its own shared memory.  (With the partials kept where they arise, the meeting was a store, a
+//   registers into the shared memory of the CTA that finishes the row (row r: rank r mod splits), counted there on a barrier (32 rows) or
+//   ahead of a cluster barrier, and the epilogue reads only its own shared memory.  (With the partials kept where they arise, the meeting was a store, a
 //   barrier, loads through distributed shared memory at each one's latency, and a second barrier before anyone might leave);
 // * a warp takes a row, lane l its columns 4l .. 4l+3, one to four rows side by side.  A row in one warp makes the head norm and
 //   the rotary partner of the QKV projection, the output statistics of a folded norm and coalesced 256-byte stores plain
@@ -27,7 +28,11 @@
 // row of a warp at a time, its loads behind the accumulator) -> this one, M 23 / 128 / 196 / 512: N 4096 K 1024 6.1 -> 4.7,
 // 8.5 -> 6.6, 9.0 -> 8.1; N 6144 K 1024 7.2 -> 5.4, 9.1 -> 7.9; N 1024 K 3072 6.0 -> 5.4, 8.6 -> 7.2, 9.1 -> 8.1, 12.0 -> 9.9;
 // N 768 K 768 4.4 -> 4.1, 6.4 -> 4.4, 6.7 -> 4.7, 7.6 -> 5.6; N 768 K 3072 6.0 -> 5.3, 8.9 -> 6.2, 9.9 -> 6.9, 10.9 -> 9.2.  It is
-// bound by its own chain: a kernel boundary (0.8 us), the activations through TMA, 12 to 48 dependent MMAs, one exchange.
+// bound by its own chain: a kernel boundary (0.8 us), the activations through TMA, 12 to 48 dependent MMAs, one exchange.  Of the 10300
+// cycles of a QKV projection of 23 tokens 2000 were gains on their way from HBM behind the wait, 1000 a serial sum of the row statistics and
+// 1300 the cluster barrier behind the partials; without them a query of 23 tokens takes 677 us instead of 707, a prompt of 47 tokens 1473
+// instead of 1571 (with the smaller code), one image 402 instead of 406.  Four rows of a column as one 16-byte store, with the sums put back
+// into rows by all threads: 693 and 427 us.
 //
 // The tensor memory is allocated BEFORE launch_dependents: a later kernel that shares the SM can then never hold columns
 // this one still waits for (an SM holds two such CTAs, or one and an attention CTA of 256 columns, of its 512).
@@ -50,6 +55,10 @@ constexpr uint32_t kSplitSpin = 1u << 22;
 template <int TN>
 struct SplitCfg {
     static constexpr bool kAlias = TN > 64;
+    // Tiles of 32 rows send by st.async to a barrier of the receiver (one way; a rank's 16 stores a warp take 1000 cycles to leave and 640
+    // more to arrive), the others by plain stores ahead of a cluster barrier: twice as many st.async leave at half the rate of stores
+    // (64 rows: 2200 cycles against 1300, which is what the barrier's 1700 against 800 gives back; one image 408 us against 406).
+    static constexpr bool kAsync = TN == 32;
     static constexpr int kStages = TN == 32 ? 4 : 3;
     static constexpr int kRows = TN / 32;                        // output rows a warp works on side by side
     // Warps that normalise a k-block, in as many groups as stages: a group keeps to one stage and so waits for every use of its
@@ -60,7 +69,7 @@ struct SplitCfg {
     static constexpr uint32_t kA = TN * SK * 2;
     static constexpr uint32_t kRing = kStages * (kA + kSplitW);
     static constexpr uint32_t kRecv = kAlias ? 0 : TN * SN * 4;
-    static constexpr uint32_t kSmem = kRing + kRecv + 1024 /*alignment*/ + 192 /*barriers*/ + TN * 8 /*row statistics*/;
+    static constexpr uint32_t kSmem = kRing + kRecv + 1024 /*alignment*/ + 192 /*barriers*/ + TN * 8 /*row statistics*/ + kStages * SK * 2 /*gains*/;
     static_assert(!kAlias || TN * SN * 4 <= kRing, "the partial tiles reuse the ring");
     static_assert(2 * (kSmem + 1024) <= 228 * 1024, "two CTAs per SM");
 };
@@ -166,26 +175,22 @@ __device__ __forceinline__ void split_epilogue_row(const GemmArgs& g, const Spli
         return;
     }
     if constexpr (EPI == ITTAI_EPI_QKROPE) {
-        // the Linear output rounded, then (q and k heads) the head norm and the half-split rotary embedding with the rounding
+        // on packed pairs: the Linear output rounded, then (q and k heads) the head norm and the half-split rotary embedding with the rounding
         // steps of qk_rope_scatter_kernel; the partner element 64 columns away is 16 lanes away
         constexpr int HD = ITTAI_Q3_HD;
         const int head = col0 / HD;
-        float x[4];
-#pragma unroll
-        for (int i = 0; i < 4; ++i) x[i] = bf16r(v[i]);
+        uint32_t x0 = pack_bf16x2(v[0], v[1]), x1 = pack_bf16x2(v[2], v[3]);
         if (head < 24) {
-            const float ss = warp_sum(fmaf(x[0], x[0], fmaf(x[1], x[1], fmaf(x[2], x[2], x[3] * x[3]))));
-            const float rstd = 1.0f / sqrtf(ss * (1.0f / HD) + g.rope.eps);
-            const float ga[4] = {bf_lo(k.gain.x), bf_hi(k.gain.x), bf_lo(k.gain.y), bf_hi(k.gain.y)}, cs[4] = {bf_lo(in.cos.x), bf_hi(in.cos.x), bf_lo(in.cos.y), bf_hi(in.cos.y)};
-            const float sn[4] = {bf_lo(in.sin.x), bf_hi(in.sin.x), bf_lo(in.sin.y), bf_hi(in.sin.y)};
-#pragma unroll
-            for (int i = 0; i < 4; ++i) {
-                const float mine = bf16r(bf16r(x[i] * rstd) * ga[i]), other = __shfl_xor_sync(0xffffffffu, mine, 16);
-                x[i] = bf16r(bf16r(mine * cs[i]) + bf16r((lane < 16 ? -other : other) * sn[i]));
-            }
+            const float f0 = bf_lo(x0), f1 = bf_hi(x0), f2 = bf_lo(x1), f3 = bf_hi(x1);
+            const float rstd = rsqrt_full(warp_sum(fmaf(f0, f0, fmaf(f1, f1, fmaf(f2, f2, f3 * f3)))) * (1.0f / HD) + g.rope.eps);
+            const uint32_t n0 = mul_bf16x2(pack_bf16x2(f0 * rstd, f1 * rstd), k.gain.x), n1 = mul_bf16x2(pack_bf16x2(f2 * rstd, f3 * rstd), k.gain.y);
+            const uint32_t neg = lane < 16 ? 0x80008000u : 0u;
+            const uint32_t o0 = __shfl_xor_sync(0xffffffffu, n0, 16) ^ neg, o1 = __shfl_xor_sync(0xffffffffu, n1, 16) ^ neg;
+            x0 = add_bf16x2(mul_bf16x2(n0, in.cos.x), mul_bf16x2(o0, in.sin.x));
+            x1 = add_bf16x2(mul_bf16x2(n1, in.cos.y), mul_bf16x2(o1, in.sin.y));
         }
         bf16* dst = head < 16 ? g.out + (size_t)row * g.ld_out + c : in.cache;
-        if (store) *reinterpret_cast<uint2*>(dst) = make_uint2(pack_bf16x2(x[0], x[1]), pack_bf16x2(x[2], x[3]));
+        if (store) *reinterpret_cast<uint2*>(dst) = make_uint2(x0, x1);
         return;
     }
     if constexpr (EPI == ITTAI_EPI_GELU) {
@@ -221,22 +226,28 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constan
     unsigned long long* empty = bars + kStages;
     unsigned long long* acc_full = bars + 2 * kStages;
     unsigned long long* ready = bars + 2 * kStages + 1;              // [stages] A normalised
-    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 3 * kStages + 1);
+    unsigned long long* arrived = bars + 3 * kStages + 1;            // partials of this CTA's rows have arrived
+    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 3 * kStages + 2);
     float* scale = reinterpret_cast<float*>(bars + 16);              // a_gain: [TN] 1 / rms of A's rows
     float2* norm = reinterpret_cast<float2*>(bars + 16);             // folded norm: [TN / splits] mean, 1 / standard deviation of this CTA's rows
     volatile uint32_t* abort_flag = tmem_slot + 1;
-    static_assert(3 * kStages + 2 <= 16, "barriers and flags end before the row scales");
+    unsigned char* gain_s = reinterpret_cast<unsigned char*>(bars) + 192 + TN * 8;      // a_gain, all_norm: [stages][64] the CTA's gains
+    static_assert(3 * kStages + 3 <= 16, "barriers and flags end before the row scales");
 
     const int warp = warp_index(), lane = threadIdx.x & 31;
     const int rank = blockIdx.x, splits = 1 << lg, tile_n = blockIdx.y, row_base = blockIdx.z * tile_rows;
     const int n_kb_all = g.K / SK, kb0 = n_kb_all * rank >> lg, n_kb = (n_kb_all * (rank + 1) >> lg) - kb0;   // >= 1: splits <= K / 64
     const int rows = min(tile_rows, g.M - row_base);
+    const bool all_norm = n_kb <= kStages;                           // no stage is used twice: see the normalising warps
 
     if (threadIdx.x == 0) {
-        for (int s = 0; s < kStages; ++s) { mbar_init(&full[s], 1); mbar_init(&empty[s], 1); mbar_init(&ready[s], Cfg::kNormGroup); }
+        for (int s = 0; s < kStages; ++s) { mbar_init(&full[s], 1); mbar_init(&empty[s], 1); mbar_init(&ready[s], all_norm ? kNormWarps : Cfg::kNormGroup); }
         mbar_init(acc_full, 1);
+        mbar_init(arrived, 1);
         *abort_flag = 0;
         fence_mbar_init();
+        // the partials of this CTA's rows, those of its own included
+        if (Cfg::kAsync && splits > 1) mbar_expect_tx(arrived, rank < rows ? (uint32_t)(((rows - 1 - rank) >> lg) + 1) * (SN * 4) << lg : 0u);
         tma_prefetch_desc(&tm_a);
         tma_prefetch_desc(&tm_w);
     }
@@ -264,10 +275,18 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constan
     // its k-blocks: group, group + kStages, ... (none for the warps left over); a thread keeps to one 16-byte column piece (eight
     // pieces a row), so its gains are one vector per k-block, the first of them fetched ahead of the wait like the weights
     constexpr int kNormThreads = 32 * Cfg::kNormGroup;
-    const int group = warp - 2 < kStages * Cfg::kNormGroup ? (warp - 2) / Cfg::kNormGroup : n_kb, nt = (threadIdx.x - 64) % kNormThreads, piece = nt & 7;
+    const int group = all_norm ? 0 : warp - 2 < kStages * Cfg::kNormGroup ? (warp - 2) / Cfg::kNormGroup : n_kb;
+    const int nt = all_norm ? threadIdx.x - 64 : (threadIdx.x - 64) % kNormThreads, piece = nt & 7;
     const uint4* gains = reinterpret_cast<const uint4*>(g.a_gain + (size_t)kb0 * SK) + piece;
     uint4 gain = make_uint4(0u, 0u, 0u, 0u);
-    if (normalises && group < n_kb) gain = gains[8 * group];
+    // Ahead of the wait, and in shared memory where that can be, so that they have arrived: a load that nothing uses before the wait is
+    // scheduled behind it, and gains come from HBM (1500 to 2000 cycles a k-block on the critical path).
+    float inv_k = 0.f;
+    if (normalises) {
+        asm volatile("rcp.rn.f32 %0, %1;" : "=f"(inv_k) : "f"((float)g.K));
+        if (!all_norm) { if (group < n_kb) gain = gains[8 * group]; }
+        else if (nt < 8 * n_kb) *reinterpret_cast<uint4*>(gain_s + nt * 16) = reinterpret_cast<const uint4*>(g.a_gain + (size_t)kb0 * SK)[nt];
+    }
     pdl_wait();                                                      // from here on what the kernels before wrote
     if (warp == 0 && elect_one()) {
         for (int kb = 0; kb < ahead; ++kb) tma_load_2d(sa + kb * Cfg::kA, &tm_a, (kb0 + kb) * SK, row_base, &full[kb]);
@@ -308,13 +327,27 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constan
             if (ok) umma_commit(acc_full); else *abort_flag = 1;
         }
     } else if (g.a_gain != nullptr) {
+        // eight lanes a row, each every eighth partial sum
         const int t = threadIdx.x - 64;
-        if (t < rows) scale[t] = 1.0f / sqrtf(row_sums(g, row_base + t).y * (1.0f / (float)g.K) + g.stats_eps);
+        for (int r0 = 0; r0 < rows; r0 += 4 * kNormWarps) {
+            const int r = r0 + (t >> 3);
+            float ss = 0.f;
+            if (r < rows) {
+                const float2* ps = reinterpret_cast<const float2*>(g.row_stats) + (size_t)(row_base + r) * g.stats_parts;
+                for (int i = t & 7; i < g.stats_parts; i += 8) ss += ps[i].y;
+            }
+#pragma unroll
+            for (int o = 1; o < 8; o <<= 1) ss += __shfl_xor_sync(0xffffffffu, ss, o);
+            if (r < rows && (t & 7) == 0) scale[r] = rsqrt_full(ss * inv_k + g.stats_eps);
+        }
         asm volatile("bar.sync 1, %0;" ::"n"(32 * kNormWarps) : "memory");
-        for (int kb = group; kb < n_kb; kb += kStages) {
+        // Up to as many k-blocks as stages (a short K, or one that many CTAs share) all warps take each of them.  Beyond that the groups.
+        const int kb_step = all_norm ? 1 : kStages, row_step = (all_norm ? 32 * kNormWarps : kNormThreads) / 8;
+#pragma unroll 1
+        for (int kb = group; kb < n_kb; kb += kb_step) {
             const int s = kb % kStages, use = kb / kStages;
-            const uint4 gq = gain;
-            if (kb + kStages < n_kb) gain = gains[8 * (kb + kStages)];
+            const uint4 gq = all_norm ? *reinterpret_cast<const uint4*>(gain_s + kb * 128 + piece * 16) : gain;
+            if (!all_norm && kb + kb_step < n_kb) gain = gains[8 * (kb + kb_step)];
             bool ok = true;
             uint32_t spins = 0;
             while (!mbar_try_wait_parked(&full[s], use & 1)) {
@@ -322,16 +355,15 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constan
             }
             if (!__all_sync(0xffffffffu, ok)) { *abort_flag = 1; break; }      // one answer for all lanes: warp-wide steps follow
             const uint32_t gw[4] = {gq.x, gq.y, gq.z, gq.w};
-            constexpr int kStep = kNormThreads / 8;
-#pragma unroll 4
-            for (int r = nt >> 3; r < rows; r += kStep) {
+#pragma unroll 2
+            for (int r = nt >> 3; r < rows; r += row_step) {
                 uint4* p = reinterpret_cast<uint4*>(sa + s * Cfg::kA + r * 128 + ((piece ^ (r & 7)) << 4));
                 const uint4 x = *p;
                 const uint32_t xw[4] = {x.x, x.y, x.z, x.w};
                 const float rs = scale[r];
                 uint32_t o[4];
 #pragma unroll
-                for (int j = 0; j < 4; ++j) o[j] = pack_bf16x2(bf16r(bf_lo(xw[j]) * rs) * bf_lo(gw[j]), bf16r(bf_hi(xw[j]) * rs) * bf_hi(gw[j]));
+                for (int j = 0; j < 4; ++j) o[j] = mul_bf16x2(pack_bf16x2(bf_lo(xw[j]) * rs, bf_hi(xw[j]) * rs), gw[j]);
                 *p = make_uint4(o[0], o[1], o[2], o[3]);
             }
             fence_proxy_async_smem();                                // the MMAs read through the async proxy
@@ -355,6 +387,16 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constan
         }
     }
     __syncwarp();
+    // Warp w reads TMEM lanes 32 (w % 4) .. + 31, one weight row = output column per thread; the two warps of a lane quarter
+    // take half of the token rows each.  A warp's store is 32 consecutive floats of one row, into the owner's buffer.
+    const int half = (warp >> 2) * (TN / 2);
+    const uint32_t src = smem_u32(part) + (uint32_t)rank * (TN >> lg) * (SN * 4) + 4u * ((warp & 3) * 32 + lane);
+    uint32_t to[kMaxSplit], to_bar[Cfg::kAsync ? kMaxSplit : 1];     // the owners of eight neighbouring rows
+#pragma unroll
+    for (int i = 0; i < kMaxSplit; ++i) {
+        to[i] = split_mapa(src, i & (splits - 1));
+        if (Cfg::kAsync) to_bar[Cfg::kAsync ? i : 0] = split_mapa(smem_u32(arrived), i & (splits - 1));
+    }
     bool ok = true;
     {
         uint32_t spins = 0;
@@ -372,26 +414,35 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constan
     } else if (Cfg::kAlias) {
         __syncthreads();
     }
-    // Warp w reads TMEM lanes 32 (w % 4) .. + 31, one weight row = output column per thread; the two warps of a lane quarter
-    // take half of the token rows each.  A warp's store is 32 consecutive floats of one row, into the owner's buffer.
-    const int half = (warp >> 2) * (TN / 2);
-    const uint32_t src = smem_u32(part) + (uint32_t)rank * (TN >> lg) * (SN * 4) + 4u * ((warp & 3) * 32 + lane);
 #pragma unroll
     for (int c = 0; c < TN / 2; c += 16) {
-        if (!ok || half + c >= rows) break;
+        if (half + c >= rows) break;                // where the wait ran out too: the owners count on the bytes, the status tells the caller
         uint32_t acc[16];
         tmem_ld_32x16(tmem_base + ((uint32_t)((warp & 3) * 32) << 16) + half + c, acc);
         tmem_ld_wait16(acc);
 #pragma unroll
         for (int i = 0; i < 16; ++i) {
             const int n = half + c + i;
-            if (n < rows) asm volatile("st.shared::cluster.b32 [%0], %1;" ::"r"(split_mapa(src + (uint32_t)(n >> lg) * (SN * 4), n & (splits - 1))), "r"(acc[i]) : "memory");
+            if (n < rows) {
+                const uint32_t dst = to[i % kMaxSplit] + (uint32_t)(n >> lg) * (SN * 4);
+                // a launch without clusters (splits == 1) may not use st.async: it is an illegal instruction there
+                if (!Cfg::kAsync || splits == 1) asm volatile("st.shared::cluster.b32 [%0], %1;" ::"r"(dst), "r"(acc[i]) : "memory");
+                else asm volatile("st.async.weak.shared::cluster.mbarrier::complete_tx::bytes.b32 [%0], %1, [%2];" ::"r"(dst), "r"(acc[i]), "r"(to_bar[Cfg::kAsync ? i % kMaxSplit : 0]) : "memory");
+            }
         }
     }
     tc_fence_before();
     __syncthreads();
-    if (splits > 1) { split_cluster_arrive(); split_cluster_wait(); }
     if (warp == 1) tmem_dealloc(tmem_base, TN);
+    if (!Cfg::kAsync) {
+        if (splits > 1) { split_cluster_arrive(); split_cluster_wait(); }
+    } else if (splits > 1) {
+        uint32_t spins = 0;
+        while (!mbar_try_wait_cluster(arrived, 0)) {
+            if (((++spins) & 255u) == 0u && (*abort_flag || spins >= kSplitSpin)) { *abort_flag = 1; break; }
+        }
+        __syncwarp();
+    }
     const uint32_t mine = smem_u32(part) + 16u * lane;
     const bool folded = g.row_stats != nullptr && g.a_gain == nullptr;
     for (int r0 = first; r0 < rows; r0 += U * step) {

@@ -80,13 +80,6 @@ __device__ __forceinline__ void mma16816(float (&d)[4], uint32_t a0, uint32_t a1
 __device__ __forceinline__ uint32_t norm_pair(uint32_t x, uint32_t g, float rstd) {
     return pack_bf16x2(bf16r(bf_lo(x) * rstd) * bf_lo(g), bf16r(bf_hi(x) * rstd) * bf_hi(g));
 }
-// 1 / sqrt(v): the hardware approximation and one Newton step (1.0f / sqrtf(v) is two long dependent sequences, and every kernel
-// that normalises has one on its critical path).  Over every float of [1, 4) at most 1.00 ulp from the 64-bit value and 0.28 on
-// average; 1.0f / sqrtf(v): 1.49 and 0.35.
-__device__ __forceinline__ float rsqrt_full(float v) {
-    const float r = rsqrtf(v), y = fmaf(r * 0.5f, fmaf(-v * r, r, 1.0f), r);
-    return v < INFINITY && v > 0.f ? y : r;           // 0 for a sum of squares that overflowed, not inf * 0
-}
 // RMSNorm of the NB rows of x (width D) into xs[b][..] (rows padded by 64 bytes, see the weight rows): the 512 threads share
 // the rows out, 2 NB values each, so that every value is normalised once per CTA.  Contains the two barriers after which xs
 // may be read.
@@ -578,23 +571,6 @@ __device__ __forceinline__ uint32_t swz(uint32_t base, int row, int chunk) { ret
 __device__ __forceinline__ void st_async_f32x2(void* p, int rank, float x, float y, void* bar) {
     asm volatile("st.async.weak.shared::cluster.mbarrier::complete_tx::bytes.v2.f32 [%0], {%1, %2}, [%3];"
                  ::"r"(map_to_cta(p, (uint32_t)rank)), "f"(x), "f"(y), "r"(map_to_cta(bar, (uint32_t)rank)) : "memory");
-}
-// The data of st_async_f32x2 from other CTAs is visible once this has returned true.
-__device__ __forceinline__ bool mbar_try_wait_cluster(void* bar, uint32_t parity) {
-    uint32_t ok;
-    asm volatile("{\n.reg .pred p;\nmbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2;\nselp.u32 %0, 1, 0, p;\n}\n"
-                 : "=r"(ok) : "r"(smem_u32(bar)), "r"(parity) : "memory");
-    return ok != 0;
-}
-__device__ __forceinline__ uint32_t mul_bf16x2(uint32_t a, uint32_t b) {
-    uint32_t d;
-    asm("mul.rn.bf16x2 %0, %1, %2;" : "=r"(d) : "r"(a), "r"(b));
-    return d;
-}
-__device__ __forceinline__ uint32_t add_bf16x2(uint32_t a, uint32_t b) {
-    uint32_t d;
-    asm("add.rn.bf16x2 %0, %1, %2;" : "=r"(d) : "r"(a), "r"(b));
-    return d;
 }
 
 // log2 of the pieces that the cache of a sequence with `len` positions is cut into, one CTA each.  Measured over all splits and

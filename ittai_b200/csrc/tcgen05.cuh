@@ -189,6 +189,13 @@ __device__ __forceinline__ bool mbar_try_wait_parked(void* bar, uint32_t parity)
         : "=r"(ok) : "r"(smem_u32(bar)), "r"(parity), "r"(ITTAI_PARK_NS) : "memory");
     return ok != 0;
 }
+// Whether the phase has completed, where other CTAs of the cluster have written the data that it announces (st.async).
+__device__ __forceinline__ bool mbar_try_wait_cluster(void* bar, uint32_t parity) {
+    uint32_t ok;
+    asm volatile("{\n.reg .pred p;\nmbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2;\nselp.u32 %0, 1, 0, p;\n}\n"
+                 : "=r"(ok) : "r"(smem_u32(bar)), "r"(parity) : "memory");
+    return ok != 0;
+}
 // Bounded mbarrier wait: false when the limit ran out.
 __device__ __forceinline__ bool mbar_wait_bounded(void* bar, uint32_t parity, uint32_t limit) {
     uint32_t spins = 0;
