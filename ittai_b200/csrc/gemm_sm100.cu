@@ -212,7 +212,10 @@ int gemm_args_from_abi(const IttaiGemm* a, GemmArgs* gp, CUtensorMap* tm_a, CUte
     rc = make_tmap_bf16(tm_b, a->w, a->n, a->k, ld_w, box_w);
     if (rc != ITTAI_OK) return rc;
     GemmArgs& g = *gp;
-    g.M = a->m; g.N = a->n; g.K = a->k; g.epi = epi;
+    g.M = a->m; g.N = a->n; g.epi = epi;
+    // A zero-padded A has nothing to add beyond its true width: whole k-blocks of zeros are left out (so400m, 1152 of 1280 columns: the
+    // QKV projection and fc1 take 18 k-blocks instead of 20).
+    g.K = a->row_stats != nullptr && a->stats_parts > 0 && a->stats_k > 0 ? (a->stats_k + GK - 1) / GK * GK : a->k;
     g.bias = reinterpret_cast<const float*>(a->bias);
     g.residual = reinterpret_cast<const bf16*>(a->residual);
     g.ld_res = ld_res;

@@ -326,3 +326,26 @@ def test_rotary_runs_cross_from_q_to_k(m):
     runs = _qk_runs(m, 148)
     assert [t for r in runs for t in r] == list(range((m + 255) // 256 * 16))
     assert sum(7 in [t % 16 for t in r[:-1]] for r in runs) >= m // 512
+
+
+@gpu
+@pytest.mark.parametrize("true,padded", [(1152, 1280), (1100, 1280), (64, 256)])
+@pytest.mark.parametrize("m", [40, 300, 2600])
+def test_zero_padded_columns_are_left_out(m, true, padded):
+    """A folded LayerNorm over the true width of a zero-padded A (split-K, one-SM and pair tiles): the bits of the same GEMM without
+    ``stats_k``, whose statistics are given ready-made, since zero products change no sum."""
+    from ittai_b200 import ops
+    n, width = 768, (true + 127) // 128
+    a = torch.zeros(m, padded, dtype=torch.bfloat16, device="cuda")
+    w = torch.zeros(n, padded, dtype=torch.bfloat16, device="cuda")
+    a[:, :true], w[:, :true] = _rand(m, true, seed=71), _rand(n, true, scale=0.05, seed=72)
+    x = a.float().view(m, padded // 128, 128)
+    parts = torch.stack([x.sum(-1), x.pow(2).sum(-1)], -1).contiguous()
+    cols, st = w.float().sum(1).contiguous(), ops.new_status("cuda")
+    mean = x.sum((1, 2)) / true
+    rstd = torch.rsqrt(x.pow(2).sum((1, 2)) / true - mean * mean + 1e-6)
+    got = ops.gemm(a, w, st, row_stats=parts, col_sums=cols, stats_eps=1e-6, stats_k=true, static_w=True)
+    ops.check_status(st)
+    acc = a.double() @ w.double().t()
+    _check(got, (rstd.double()[:, None] * (acc - mean.double()[:, None] * cols.double())).float(), f"{m}x{true} of {padded}")
+    assert width * 128 <= padded
