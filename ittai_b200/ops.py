@@ -99,6 +99,12 @@ def gemm_chain(descs, flags: torch.Tensor) -> None:
     _C.check(_C.lib().ittai_gemm_chain_launch(arr, n, flags.data_ptr(), _stream(flags)))
 
 
+def gemm_each(descs, like: torch.Tensor) -> None:
+    """The GEMMs of a chain as one launch each, on the stream of ``like``'s device: the same bits."""
+    for d in descs:
+        _C.check(_C.lib().ittai_gemm_bf16_launch(C.byref(d), _stream(like)))
+
+
 def row_stats(x: torch.Tensor, eps: float, out: torch.Tensor | None = None) -> torch.Tensor:
     """fp32 ``[rows, 2]``: mean and ``1/sqrt(var + eps)`` of every row of bf16 ``x``."""
     out = torch.empty(x.shape[0], 2, dtype=torch.float32, device=x.device) if out is None else out

@@ -66,6 +66,23 @@ def checked_shapes(inp, n: int, S: int) -> torch.Tensor:
     return shapes.to(torch.int32).contiguous()
 
 
+def chain_pays(rows: int, gemms, n_sms: int) -> bool:
+    """Whether the four GEMMs of a layer run faster as one chained launch than one by one (the same bits either way).  ``gemms``:
+    (N, K) of each, the QKV projection first; tiles of 256 x 256, one to a pair of SMs at a time.
+
+    A chain fills the rounds that single launches leave part-filled, but a tile of it waits for the row block of the GEMM before, and
+    with at most two rounds of QKV tiles there is not enough other work meanwhile.  us a forward, chain / one by one: ViT-B with
+    1568, 2156, 3136 rows 879 / 873, 945 / 927, 1066 / 1068, variable resolution with 2048 and 4096 902 / 876 and 1139 / 1089, so400m with
+    1458, 2187 2781 / 2736, 3011 / 2975; beyond the line 4704, 6272, 9408 rows 1195 / 1216, 1484 / 1704, 1991 / 2144, so400m with 2916,
+    5832 3638 / 3661, 6335 / 6549.  Where the single launches' rounds are full to 3 % (12 544 rows: 5.96, 1.99, 7.95 and 1.99 rounds) a chain
+    has nothing to fill: 2663 / 2642; with 16 384 rows, 8 % of the rounds empty, 3397 / 3485."""
+    pairs, blocks = n_sms // 2, -(-rows // 256)
+    tiles = [(blocks * (n // 256), k) for n, k in gemms]
+    if tiles[0][0] <= 2 * pairs:
+        return False
+    return sum(-(-t // pairs) * pairs * k for t, k in tiles) > 1.03 * sum(t * k for t, k in tiles)
+
+
 def part_size(n: int, B: int, S: int, chain: bool) -> int:
     """Images to run for a short batch of ``n``: at least the 1024 rows from which on the chained GEMMs are used where the full
     batch of ``B`` uses them: an image's result then does not depend on the batch it came in.  Without chains (fewer than 1024
@@ -170,7 +187,8 @@ class Engine:
         # produces it: one buffer for the stream after attention, one for the stream after the MLP
         self.stats_a = torch.zeros(M, D // 128, 2, dtype=torch.float32, device=dev)
         self.stats_m = torch.zeros(M, D // 128, 2, dtype=torch.float32, device=dev)
-        # ``chain``: the GEMMs between two attention kernels (out-proj, fc1, fc2, the next layer's QKV) run as ONE
+        self.n_sms = torch.cuda.get_device_properties(dev).multi_processor_count
+        # ``chain``: the GEMMs between two attention kernels (out-proj, fc1, fc2, the next layer's QKV) may run as ONE
         # persistent launch whose tiles wait on per-row-block counters, like the tasks of the reference's persistent kernel
         # (reference ``:197-333``); needs the folded LayerNorms (no kernel of another kind between the GEMMs) and M > 128
         self.chain = bool(chain) and self.fold_ln and M >= 1024      # a few row blocks only: nothing to overlap, one launch per GEMM is faster
@@ -202,12 +220,15 @@ class Engine:
                           o_strides=(D, hd), max_kv_len=kv_max, q_rows_total=self.M, kv_rows_total=self.M, status=st)
 
         if self.chain:
-            self.chain_flags.zero_()
+            chained = chain_pays(M, ((3 * D, D), (D, D), (self.F, D), (D, self.F)), self.n_sms)
+            if chained:
+                self.chain_flags.zero_()
             qkv = lambda w: ops.gemm_desc(x, w["qkv_f"][0], st, bias=w["qkv_f"][1], out=qkv_b, row_stats=stats_m,
                                           col_sums=w["qkv_f"][2], stats_eps=eps)[0]
             # patch embedding + the first QKV projection; then per layer out-proj, fc1, fc2 and the next layer's QKV (after
             # the last layer: the K/V projection of the pooling head)
-            ops.gemm_chain([ops.gemm_desc(patches, self.wpe, st, **embed)[0], qkv(self.layers[0])], self.chain_flags[len(self.layers)])
+            run = ops.gemm_chain if chained else lambda descs, flags: ops.gemm_each(descs, x)
+            run([ops.gemm_desc(patches, self.wpe, st, **embed)[0], qkv(self.layers[0])], self.chain_flags[len(self.layers)])
             for i, w in enumerate(self.layers):
                 attention()
                 descs = [ops.gemm_desc(attn, w["wo"], st, bias=w["bo"], residual=x, out=x, stats_out=stats_a)[0],
@@ -219,7 +240,7 @@ class Engine:
                 else:
                     descs.append(ops.gemm_desc(x, self.kv_f[0], st, bias=self.kv_f[1], out=kv, row_stats=stats_m,
                                                col_sums=self.kv_f[2], stats_eps=eps)[0])
-                ops.gemm_chain(descs, self.chain_flags[i])
+                run(descs, self.chain_flags[i])
         for w in (() if self.chain else self.layers):
             if fold:
                 ops.gemm(x, w["qkv_f"][0], st, static_w=True, bias=w["qkv_f"][1], out=qkv_b, row_stats=stats_m, col_sums=w["qkv_f"][2], stats_eps=eps)
@@ -309,7 +330,8 @@ class Engine:
     def launches_per_forward(self) -> int:
         """Kernels in one forward (all inside one CUDA graph)."""
         n_l = len(self.layers)
-        encoder = (n_l + 1) + n_l if self.chain else 1 + n_l * (5 if self.fold_ln else 7) + (1 if self.fold_ln else 2)
+        chained = self.chain and chain_pays(self.M, ((3 * self.D, self.D), (self.D, self.D), (self.F, self.D), (self.D, self.F)), self.n_sms)
+        encoder = (n_l + 1) + n_l if chained else 1 + n_l * (5 if self.fold_ln else 7) + (1 if self.fold_ln else 2)
         return (1 if self.conv else 0) + encoder + 5       # + pooling head: attention, projection, LayerNorm, two MLP GEMMs
 
     def check(self) -> None:

@@ -102,6 +102,7 @@ class PaddedEngine:
         # and the consuming epilogue finishes mean and rstd over the TRUE width (``stats_k``).
         self.fold_ln = bool(fold_ln) and M > 128
         self.chain = bool(chain) and self.fold_ln and M >= 1024
+        self.n_sms = torch.cuda.get_device_properties(dev).multi_processor_count
 
         def folded(w_bf16, bias, ln):
             g, beta = (F.pad(t, (0, Dp - D)) for t in ln)
@@ -135,6 +136,11 @@ class PaddedEngine:
         self.status = ops.new_status(dev)
         self._full, self._graphs, self._unread = Graphs(1 if graph else 0), Graphs(self.PARTS if graph else 0), False
 
+    def _chained(self, rows):
+        from .kernel import chain_pays
+        He, Dp, Fp = self.H * self.hde, self.Dp, self.Fp
+        return self.chain and chain_pays(rows, ((3 * He, Dp), (Dp, He), (Fp, Dp), (Dp, Fp)), self.n_sms)
+
     def _body(self, B):
         """Queue the forward of the first ``B`` images of the buffers."""
         D, S, H, hdp, eps, st = self.D, self.S0, self.H, self.hdp, self.eps, self.status
@@ -160,9 +166,9 @@ class PaddedEngine:
             embed = ops.gemm_desc(patches, self.wpe, st, **sw, bias=self.bpe, residual=pos, out=x, stats_out=stats_m)[0]
             qkv = lambda w: ops.gemm_desc(x, w["qkv_f"][0], st, bias=w["qkv_f"][1], out=qkv_b, row_stats=stats_m,
                                           col_sums=w["qkv_f"][2], **ln)[0]
-            run = (lambda descs, flags: ops.gemm_chain(descs, flags)) if self.chain else \
-                  (lambda descs, flags: [_C.check(_C.lib().ittai_gemm_bf16_launch(C.byref(d), ops._stream(x))) for d in descs])
-            if self.chain:
+            chained = self._chained(M)
+            run = ops.gemm_chain if chained else lambda descs, flags: ops.gemm_each(descs, x)
+            if chained:
                 self.chain_flags.zero_()
             run([embed, qkv(self.layers[0])], self.chain_flags[len(self.layers)])
             for i, w in enumerate(self.layers):
@@ -241,7 +247,7 @@ class PaddedEngine:
     def launches_per_forward(self) -> int:
         """Kernels in one forward (all inside one CUDA graph)."""
         n_l = len(self.layers)
-        encoder = (n_l + 1) + n_l if self.chain else 1 + n_l * (5 if self.fold_ln else 7) + (1 if self.fold_ln else 2)
+        encoder = (n_l + 1) + n_l if self._chained(self.M) else 1 + n_l * (5 if self.fold_ln else 7) + (1 if self.fold_ln else 2)
         return (1 if self.conv else 0) + encoder + 5
 
     def flops(self, formula: str = "reference") -> float:

@@ -84,3 +84,13 @@ def test_an_inputs_barrier_is_not_completed_again_before_it_was_looked_at(n_kb):
         with pytest.raises(RuntimeError, match="completed again"):
             for seed in range(200):
                 simulate_pair([n_kb] * 40, random.Random(seed), inputs=4)
+
+
+def test_chains_run_where_they_were_faster():
+    """Both sides of the two lines of the rule at the sizes that were measured."""
+    from ittai_b200.siglip.kernel import chain_pays
+    vit, so400m = ((2304, 768), (768, 768), (3072, 768), (768, 3072)), ((3840, 1280), (1280, 1280), (4352, 1280), (1280, 4352))
+    for rows, want in ((1024, False), (2156, False), (4096, False), (4097, True), (6272, True), (9408, True), (12544, False), (16384, True)):
+        assert chain_pays(rows, vit, 148) == want, rows
+    for rows, want in ((1458, False), (2187, False), (2304, False), (2305, True), (5832, True)):
+        assert chain_pays(rows, so400m, 148) == want, rows
