@@ -419,13 +419,17 @@ int cuda_fail(cudaError_t e, const char* what);
 bool attn_tc_supported(const IttaiAttention* p);          // attention_sm100.cu
 int attn_tc_launch(const IttaiAttention* p, cudaStream_t st);
 bool attn_fa_supported(const IttaiAttention* p);          // attention_fa_sm100.cu
-int attn_fa_launch(const IttaiAttention* p, cudaStream_t st);
+int attn_fa_launch(const IttaiAttention* p, bool disjoint, cudaStream_t st);
+int attention_launch(const IttaiAttention* p, bool disjoint, cudaStream_t st);
 
 }  // namespace ittai
 
 using namespace ittai;
 
-extern "C" int ittai_attention_launch(const IttaiAttention* p, void* stream) {
+extern "C" int ittai_attention_launch(const IttaiAttention* p, void* stream) { return attention_launch(p, false, (cudaStream_t)stream); }
+
+// `disjoint`: the caller vouches that no two sequences share a query row.
+int ittai::attention_launch(const IttaiAttention* p, bool disjoint, cudaStream_t stream) {
     if (!p || !p->q || !p->k || !p->v || !p->o || !p->seqs) { set_error("attention: null pointer"); return ITTAI_E_ARG; }
     if (p->head_dim != 64 && p->head_dim != 128 && !(p->head_dim == 80 && attn_fa_supported(p))) {
         set_error("attention: head_dim %d (64, 128, or 80 in the packed layout of the key-loop kernel)", p->head_dim);
@@ -434,15 +438,15 @@ extern "C" int ittai_attention_launch(const IttaiAttention* p, void* stream) {
     if (p->n_seqs < 1 || p->n_heads < 1 || p->group < 1 || p->max_q_len < 1) { set_error("attention: bad sizes"); return ITTAI_E_ARG; }
     const long long strides[] = {p->q_row, p->q_head, p->k_row, p->k_head, p->k_seq, p->v_row, p->v_head, p->v_seq, p->o_row};
     for (long long s : strides) if (s % 8) { set_error("attention: strides must be multiples of 8 elements"); return ITTAI_E_ARG; }
-    if (attn_tc_supported(p)) return attn_tc_launch(p, (cudaStream_t)stream);
-    if (attn_fa_supported(p)) return attn_fa_launch(p, (cudaStream_t)stream);
+    if (attn_tc_supported(p)) return attn_tc_launch(p, stream);
+    if (attn_fa_supported(p)) return attn_fa_launch(p, disjoint, stream);
     AttnArgs a;
     a.q = (const bf16*)p->q; a.k = (const bf16*)p->k; a.v = (const bf16*)p->v; a.o = (bf16*)p->o;
     a.q_row = p->q_row; a.q_head = p->q_head; a.k_row = p->k_row; a.k_head = p->k_head; a.k_seq = p->k_seq;
     a.v_row = p->v_row; a.v_head = p->v_head; a.v_seq = p->v_seq; a.o_row = p->o_row; a.o_head = p->o_head;
     a.seqs = (const int4*)p->seqs; a.group = p->group;
     a.scale_log2 = 1.4426950408889634f / sqrtf((float)p->head_dim);
-    cudaStream_t st = (cudaStream_t)stream;
+    cudaStream_t st = stream;
     const int ql = p->max_q_len, nh = p->n_heads, ns = p->n_seqs;
     int rc;
     if (p->head_dim == 64 && !p->causal && ql == 1) {

@@ -40,7 +40,16 @@ constexpr uint32_t kFaCols = 256, kFaOCol = 128;
 constexpr uint32_t kFaSpin = 1u << 22;
 constexpr uint32_t kFaQ = 0, kFaK = 32768, kFaV = 65536, kFaBar = 98304;
 constexpr uint32_t kFaX = kFaBar + 256;      // float [2 halves][128 rows]: what the two threads of a row tell each other
-constexpr uint32_t kFaSmem = kFaX + 1024 + 1024;
+constexpr int kFaListSeqs = 256, kFaListSteps = 64;
+// Ragged sequences: the non-empty (sequence, step of 128 rows) pairs in the order in which they are handed out, the last steps first.
+// order: sequences by their number of steps, descending; those that have step z are its first start[j + 1] - start[j], j = steps - 1 - z.
+struct FaList {
+    int total;
+    int start[kFaListSteps + 1];
+    unsigned short order[kFaListSeqs], steps[kFaListSeqs];
+};
+constexpr uint32_t kFaList = kFaX + 1024;
+constexpr uint32_t kFaSmem = kFaList + 1024, kFaSmemList = kFaSmem + ((sizeof(FaList) + 15) & ~15);
 constexpr float kFaRaise = 256.f;            // the reference is raised once sixteen neighbouring keys' P add up to more
 
 struct AttnFaArgs {
@@ -49,6 +58,7 @@ struct AttnFaArgs {
     long long o_row, o_head;
     int group, causal, seqs_ready;
     int k_seq_rows, k_head_rows;             // cache layout: strides in rows of 128 elements
+    int n_seqs, n_steps;                     // of a list
     int k_head_cols;                         // packed layout (heads side by side in a row, sequences by their row offsets): HDIM, else 0
     float scale_log2;
     uint32_t* status;
@@ -134,31 +144,62 @@ __device__ __forceinline__ float fa_half_max(uint32_t t_half, int lim) {
 }
 // One query tile: where it lies and how many key blocks it sees.
 struct FaTile { int head, r0, q_len, kv_len, n_blk, q_row, q_col, kv_row, kv_col; };
-template <int HDIM>
-__device__ __forceinline__ FaTile fa_tile(const AttnFaArgs& a, int x, int y, int z) {
-    const int4 sinfo = a.seqs[y];
+template <int HDIM, bool PAIR, bool LIST>
+__device__ __forceinline__ FaTile fa_tile(const AttnFaArgs& a, const FaList* list, int x, int y, int z) {
+    constexpr int kRows = PAIR ? kFaBlk / 2 : kFaBlk;        // query rows of a tile
     FaTile t;
-    t.head = x; t.r0 = ((int)gridDim.z - 1 - z) * kFaBlk; t.q_len = sinfo.y; t.kv_len = sinfo.w;
+    int step = (int)gridDim.z - 1 - z;
+    if constexpr (LIST) {
+        if (y >= list->total) { t = FaTile{}; return t; }      // no rows: passed over like the tiles of a sequence that is too short
+        int lo = 0, hi = a.n_steps - 1;                        // the last j with start[j] <= y
+        while (lo < hi) { const int m = (lo + hi + 1) >> 1; if (list->start[m] <= y) lo = m; else hi = m - 1; }
+        step = a.n_steps - 1 - lo;
+        y = list->order[y - list->start[lo]];
+    }
+    const int4 sinfo = a.seqs[y];
+    // PAIR: x is two times the key/value head and which 64 rows of a step of 128, the later ones first.  (With steps of 64 in z the tiles that
+    // share keys and values lie a whole layer of tiles apart: 64 texts of 512 tokens, whose keys and values exceed L2, 142 us instead of 126.)
+    t.head = PAIR ? x & ~1 : x; t.r0 = step * kFaBlk + (PAIR && (x & 1) == 0 ? kRows : 0); t.q_len = sinfo.y; t.kv_len = sinfo.w;
     // causal: query r sees keys <= r + (kv_len - q_len)
-    const int last_key = a.causal ? min(t.kv_len - 1, t.r0 + kFaBlk - 1 + t.kv_len - t.q_len) : t.kv_len - 1;
+    const int last_key = a.causal ? min(t.kv_len - 1, t.r0 + kRows - 1 + t.kv_len - t.q_len) : t.kv_len - 1;
     t.n_blk = last_key < 0 ? 0 : last_key / kFaBlk + 1;
-    const int kvh = x / a.group;
-    t.q_row = sinfo.x + t.r0; t.q_col = x * HDIM;
+    const int kvh = PAIR ? x >> 1 : x / a.group;
+    t.q_row = sinfo.x + t.r0; t.q_col = t.head * HDIM;
     t.kv_row = y * a.k_seq_rows + kvh * a.k_head_rows + sinfo.z; t.kv_col = kvh * a.k_head_cols;
     return t;
 }
-template <int HDIM>
-__device__ __forceinline__ FaTile fa_tile(const AttnFaArgs& a, int index) {
+template <int HDIM, bool PAIR, bool LIST>
+__device__ __forceinline__ FaTile fa_tile(const AttnFaArgs& a, const FaList* list, int index) {
     const int yz = index / (int)gridDim.x;
-    return fa_tile<HDIM>(a, index - yz * (int)gridDim.x, yz % (int)gridDim.y, yz / (int)gridDim.y);
+    return fa_tile<HDIM, PAIR, LIST>(a, list, index - yz * (int)gridDim.x, yz % (int)gridDim.y, yz / (int)gridDim.y);
 }
-template <int HDIM>
+template <int HDIM, bool PAIR>
 __device__ __forceinline__ void fa_zero_rows(const AttnFaArgs& a, const FaTile& t, int tid, int threads) {
     for (int i = tid; i < kFaBlk * 16; i += threads) {
-        const int row = i >> 4;
+        const int r = i >> 4, row = PAIR ? r & 63 : r, head = t.head + (PAIR ? r >> 6 : 0);
         if (t.r0 + row < t.q_len && (i & 15) < HDIM / 8)
-            *reinterpret_cast<uint4*>(a.o + (long long)(t.q_row + row) * a.o_row + (long long)t.head * a.o_head + (i & 15) * 8) = make_uint4(0, 0, 0, 0);
+            *reinterpret_cast<uint4*>(a.o + (long long)(t.q_row + row) * a.o_row + (long long)head * a.o_head + (i & 15) * 8) = make_uint4(0, 0, 0, 0);
     }
+}
+// Whole CTA.  A sequence takes part with the steps it has; ranks by counting (at most 256 x 256 comparisons, 55 texts 0.5 us, ahead of the wait
+// for the kernel in front).
+__device__ __forceinline__ void fa_build_list(const AttnFaArgs& a, FaList* list) {
+    for (int i = threadIdx.x; i < a.n_seqs; i += kFaThreads) list->steps[i] = (unsigned short)min(max(a.seqs[i].y + kFaBlk - 1, 0) / kFaBlk, a.n_steps);
+    __syncthreads();
+    for (int i = threadIdx.x; i < a.n_seqs; i += kFaThreads) {
+        const int mine = list->steps[i];
+        int rank = 0;
+        for (int u = 0; u < a.n_seqs; ++u) { const int s = list->steps[u]; rank += s > mine || (s == mine && u < i); }
+        list->order[rank] = (unsigned short)i;
+    }
+    // thread j: everything in front of step n_steps - 1 - j, all sequences' steps above it
+    for (int j = threadIdx.x; j <= a.n_steps; j += kFaThreads) {
+        int before = 0;
+        for (int u = 0; u < a.n_seqs; ++u) before += max((int)list->steps[u] - (a.n_steps - j), 0);
+        list->start[j] = before;
+        if (j == a.n_steps) list->total = before;
+    }
+    __syncthreads();
 }
 // Both 64-column atoms of a tile of 128 rows.
 __device__ __forceinline__ void fa_load(unsigned char* dst, const CUtensorMap* tm, int col, int row, void* bar) {
@@ -167,11 +208,28 @@ __device__ __forceinline__ void fa_load(unsigned char* dst, const CUtensorMap* t
     tma_load_2d(dst + 16384, tm, col + 64, row, bar);
 }
 
+// The query rows of a tile: 128 of one head, or with PAIR (boxes of 64 rows) 64 of each of two neighbouring heads.
+template <bool PAIR>
+__device__ __forceinline__ void fa_load_q(unsigned char* dst, const CUtensorMap* tm, const FaTile& t, void* bar) {
+    if constexpr (!PAIR) {
+        fa_load(dst, tm, t.q_col, t.q_row, bar);
+    } else {
+        mbar_expect_tx(bar, 32768);
+#pragma unroll
+        for (int i = 0; i < 4; ++i) tma_load_2d(dst + (i & 1) * 16384 + (i >> 1) * 8192, tm, t.q_col + 64 * i, t.q_row, bar);
+    }
+}
+
 // HDIM: 128, or 80 for heads packed 80 columns apart (a head_dim of 72, zero-padded to whole k-steps of 16): S then takes five
 // k-steps instead of eight and the projections around the kernel are 80/128 as wide.  The loads still fetch 128 columns (the
 // next head's, or zeros past the last one) and P V still computes 128: an MN-major operand comes in whole 64-column atoms.
 // The surplus columns of O are never read.
-template <int HDIM>
+// PAIR, where two query heads share a key/value head (HDIM 128): a tile is 64 query rows of both, rows 0..63 of the first and 64..127 of
+// the second.  The same keys and values serve both, and sequences are cut every 64 rows instead of 128: as many key blocks where the
+// lengths are multiples of 128, fewer otherwise (a text of 142 tokens: four per pair of heads instead of six, one of 30: one instead of two).
+// LIST: the tiles come from a list (see FaList).  A form of its own: with both ways in one kernel (53 -> 67 KB of code) the plain one took up to
+// 30 % longer (16 texts of 512 tokens 45 us instead of 35).
+template <int HDIM, bool PAIR, bool LIST>
 __global__ void __launch_bounds__(kFaThreads, 2)
 attn_fa_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUtensorMap tm_k,
                const __grid_constant__ CUtensorMap tm_v, const AttnFaArgs a) {
@@ -180,19 +238,21 @@ attn_fa_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
     // none of them writes it.  A kernel of the same run of dependent launches may (position rows of variable-resolution
     // images): every launch in between lets its successors start on entry, so nothing but the wait orders the two.
     if (!a.seqs_ready) pdl_wait();
+    extern __shared__ __align__(1024) unsigned char fa_raw[];
+    unsigned char* sm = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(fa_raw) + 1023) & ~(uintptr_t)1023);
+    FaList* list = reinterpret_cast<FaList*>(sm + kFaList);
+    if constexpr (LIST) fa_build_list(a, list);
     // Grid (heads, sequences, query tiles) with the tiles in descending order: CTAs are handed out in index order, so the
     // causal tiles that walk the most key blocks start first and the last ones are short.
-    const FaTile first = fa_tile<HDIM>(a, blockIdx.x, blockIdx.y, blockIdx.z);
+    const FaTile first = fa_tile<HDIM, PAIR, LIST>(a, list, blockIdx.x, blockIdx.y, blockIdx.z);
     if (first.r0 >= first.q_len) return;                   // the whole CTA: nothing allocated yet
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     if (first.n_blk == 0) {                                // no visible key: zero rows
         pdl_wait();
-        fa_zero_rows<HDIM>(a, first, threadIdx.x, kFaThreads);
+        fa_zero_rows<HDIM, PAIR>(a, first, threadIdx.x, kFaThreads);
         return;
     }
 
-    extern __shared__ __align__(1024) unsigned char fa_raw[];
-    unsigned char* sm = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(fa_raw) + 1023) & ~(uintptr_t)1023);
     unsigned long long* bars = reinterpret_cast<unsigned long long*>(sm + kFaBar);
     unsigned long long* bar_q = bars;             // Q landed
     unsigned long long* bar_k = bars + 1;         // K block landed (one phase per block)
@@ -214,7 +274,7 @@ attn_fa_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
         *abort_flag = 0;
         fence_mbar_init();
         pdl_wait();                                        // q, k, v come from the kernels before this one
-        fa_load(sm + kFaQ, &tm_q, first.q_col, first.q_row, bar_q);
+        fa_load_q<PAIR>(sm + kFaQ, &tm_q, first, bar_q);
         fa_load(sm + kFaK, &tm_k, first.kv_col, first.kv_row, bar_k);
         fa_load(sm + kFaV, &tm_v, first.kv_col, first.kv_row, bar_v);
     }
@@ -247,14 +307,14 @@ attn_fa_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
                     ++asked;
                     const int4 id = fa_answer(answer);
                     if (id.w == 0) { next = -1; return; }
-                    nt = fa_tile<HDIM>(a, id.x, id.y, id.z);
+                    nt = fa_tile<HDIM, PAIR, LIST>(a, list, id.x, id.y, id.z);
                     if (nt.r0 >= nt.q_len) ask();
                     else next = (id.z * (int)gridDim.y + id.y) * (int)gridDim.x + id.x;
                 }
             };
             auto load_next = [&]() {                         // Q and K are free once the last S of this tile is complete
                 if (nt.n_blk == 0) return;
-                fa_load(sm + kFaQ, &tm_q, nt.q_col, nt.q_row, bar_q);
+                fa_load_q<PAIR>(sm + kFaQ, &tm_q, nt, bar_q);
                 fa_load(sm + kFaK, &tm_k, nt.kv_col, nt.kv_row, bar_k);
             };
             for (int t = 0; ok; ++t) {
@@ -326,10 +386,10 @@ attn_fa_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
       uint32_t c = 0;                                        // key blocks before this tile
       for (int t = 0;; ++t) {
         const int q4 = warp & 3, half = (warp - 1) >> 2, r = q4 * 32 + lane;   // TMEM lane quarter; keys 64 half .. + 63 of a block; query row inside the tile
-        const FaTile tile = fa_tile<HDIM>(a, index);
+        const FaTile tile = fa_tile<HDIM, PAIR, LIST>(a, list, index);
         const int n_blk = tile.n_blk, kv_len = tile.kv_len;
         const uint32_t t_row = tmem_base + ((uint32_t)(q4 * 32) << 16), t_half = t_row + 64 * half;
-        const int row_limit = a.causal ? min(kv_len - 1, tile.r0 + r + kv_len - tile.q_len) : kv_len - 1;   // last key this row sees
+        const int row_limit = a.causal ? min(kv_len - 1, tile.r0 + (PAIR ? r & 63 : r) + kv_len - tile.q_len) : kv_len - 1;   // last key this row sees
         float* xrow = reinterpret_cast<float*>(sm + kFaX) + r;       // [2 halves], 128 floats apart
         float ref = 0.f;                                     // P = 2^(s * scale - ref); between blocks the same for both threads of a row
         float2 l2 = make_float2(0.f, 0.f);                   // this half's sum of P, even / odd keys
@@ -489,14 +549,14 @@ attn_fa_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
         }
         fa_vote(q4, false);
         const int sub = lane & 15;
-        const FaTile out = fa_tile<HDIM>(a, index);          // once more: kept across the key loop it would cost registers there
+        const FaTile out = fa_tile<HDIM, PAIR, LIST>(a, list, index);          // once more: kept across the key loop it would cost registers there
 #pragma unroll 4
         for (int it = 0; it < 8; ++it) {
-            const int rr = q4 * 32 + half * 16 + it * 2 + (lane >> 4), row = out.r0 + rr;
+            const int rr = q4 * 32 + half * 16 + it * 2 + (lane >> 4), tr = PAIR ? rr & 63 : rr, row = out.r0 + tr, head = out.head + (PAIR ? rr >> 6 : 0);
             const uint4 val = *reinterpret_cast<const uint4*>(stage + rr * 256 + ((sub ^ (rr & 15)) << 4));
-            if (row < out.q_len && sub < HDIM / 8) *reinterpret_cast<uint4*>(a.o + (long long)(out.q_row + rr) * a.o_row + (long long)out.head * a.o_head + 8 * sub) = val;
+            if (row < out.q_len && sub < HDIM / 8) *reinterpret_cast<uint4*>(a.o + (long long)(out.q_row + tr) * a.o_row + (long long)head * a.o_head + 8 * sub) = val;
         }
-        } else fa_zero_rows<HDIM>(a, tile, threadIdx.x - 32, 256);
+        } else fa_zero_rows<HDIM, PAIR>(a, tile, threadIdx.x - 32, 256);
         fence_proxy_async_smem();                            // the next V block is written through the async proxy
         tc_fence_before();
         __syncwarp();
@@ -535,10 +595,19 @@ bool attn_fa_supported(const IttaiAttention* p) {
            ((uintptr_t)p->o & 15) == 0 && p->o_row % 8 == 0 && p->o_head % 8 == 0;
 }
 
-template <int HDIM>
+static int fa_steps(const IttaiAttention* p) { return (p->max_q_len + kFaBlk - 1) / kFaBlk; }
+static int fa_list_bound(const IttaiAttention* p) { return p->q_rows_total / kFaBlk + p->n_seqs; }
+// A list of the non-empty tiles where the grid of all of them would be longer (sequences of different lengths): empty CTAs and answers that
+// name an empty tile cost more than the list.  55 texts of 16 to 512 tokens, us a layer: tiles of one head 51, of head pairs 47, from a list 39;
+// 200 texts of 16 to 80 56, 37 and 39 (one step each: no list).  Its length has a bound on the host only if the sequences' rows are
+// disjoint, which the prefill vouches for.
+static bool fa_list_pays(const IttaiAttention* p) {
+    return p->seqs_ready && p->n_seqs <= kFaListSeqs && fa_steps(p) <= kFaListSteps && (long long)fa_steps(p) * p->n_seqs > fa_list_bound(p);
+}
+template <int HDIM, bool PAIR, bool LIST>
 static int attn_fa_launch_t(const IttaiAttention* p, cudaStream_t st) {
     CUtensorMap tq, tk, tv;
-    int rc = make_tmap_bf16(&tq, p->q, p->q_rows_total, (long long)p->n_heads * HDIM, p->q_row, 128);
+    int rc = make_tmap_bf16(&tq, p->q, p->q_rows_total, (long long)p->n_heads * HDIM, p->q_row, PAIR ? 64 : 128);
     const bool packed = fa_packed_kv(p);
     const long long kv_cols = packed ? (long long)(p->n_heads / p->group) * HDIM : 128, kv_ld = packed ? p->k_row : 128;
     if (rc == ITTAI_OK) rc = make_tmap_bf16(&tk, p->k, p->kv_rows_total, kv_cols, kv_ld, 128);
@@ -548,7 +617,7 @@ static int attn_fa_launch_t(const IttaiAttention* p, cudaStream_t st) {
     int dev = 0;
     cudaGetDevice(&dev);
     if (attr_dev != dev) {
-        const cudaError_t e = cudaFuncSetAttribute(attn_fa_kernel<HDIM>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kFaSmem);
+        const cudaError_t e = cudaFuncSetAttribute(attn_fa_kernel<HDIM, PAIR, LIST>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(LIST ? kFaSmemList : kFaSmem));
         if (e != cudaSuccess) return cuda_fail(e, "cudaFuncSetAttribute(attn_fa_kernel)");
         attr_dev = dev;
     }
@@ -561,10 +630,18 @@ static int attn_fa_launch_t(const IttaiAttention* p, cudaStream_t st) {
     a.k_head_cols = packed ? HDIM : 0;
     a.scale_log2 = 1.4426950408889634f / sqrtf((float)HDIM);
     a.status = p->status;
-    const cudaError_t e = launch_pdl(attn_fa_kernel<HDIM>, dim3(p->n_heads, p->n_seqs, (p->max_q_len + 127) / 128), dim3(kFaThreads), kFaSmem, st, 1, tq, tk, tv, a);
+    a.n_seqs = p->n_seqs; a.n_steps = fa_steps(p);
+    // a list's grid is the bound on its length
+    const dim3 grid = LIST ? dim3(p->n_heads, fa_list_bound(p), 1) : dim3(p->n_heads, p->n_seqs, fa_steps(p));
+    const cudaError_t e = launch_pdl(attn_fa_kernel<HDIM, PAIR, LIST>, grid, dim3(kFaThreads), LIST ? kFaSmemList : kFaSmem, st, 1, tq, tk, tv, a);
     return e == cudaSuccess ? ITTAI_OK : cuda_fail(e, "launch attn_fa_kernel");
 }
 
-int attn_fa_launch(const IttaiAttention* p, cudaStream_t st) { return p->head_dim == 80 ? attn_fa_launch_t<80>(p, st) : attn_fa_launch_t<128>(p, st); }
+// `disjoint`: no two sequences share a query row.
+int attn_fa_launch(const IttaiAttention* p, bool disjoint, cudaStream_t st) {
+    if (p->head_dim == 80) return attn_fa_launch_t<80, false, false>(p, st);
+    if (p->group != 2 || p->n_heads % 2 != 0) return attn_fa_launch_t<128, false, false>(p, st);
+    return disjoint && fa_list_pays(p) ? attn_fa_launch_t<128, true, true>(p, st) : attn_fa_launch_t<128, true, false>(p, st);
+}
 
 }  // namespace ittai

@@ -103,3 +103,37 @@ def test_a_raise_in_every_chunk(step):
     ops.check_status(st)
     want = torch.softmax(q.double() @ kc[0, 0].double().t() / hd ** 0.5, -1) @ vc[0, 0].double()
     assert (out.double() - want).abs().max() <= 2.0 ** -7 * want.abs().max()
+
+
+@gpu
+@pytest.mark.parametrize("lens,prefix", [([0, 600, 1, 64, 129, 0, 128, 257, 511, 512, 65, 0] * 4, 0), ([2000, 0, 700], 33), ([7] * 255 + [300], 0), ([8192, 1], 0),
+                                         ([70, 3, 1030, 64, 63, 192], 0), ([30] * 300 + [400], 0)])
+def test_listed_tiles_match_the_grid(lens, prefix):
+    """Ragged sequences whose rows are disjoint: the tiles come from a list that each CTA builds (up to 256 sequences, 64 steps of 128 rows;
+    the last case has more).  The same bits as from the grid of all (sequence, step) pairs, and no row of another tile written."""
+    import ctypes as C
+    from ittai_b200 import _C, ops
+    H, KV, hd = 4, 2, 128
+    n, total = len(lens), sum(lens)
+    g = torch.Generator(device="cuda").manual_seed(total)
+    rn = lambda *s: torch.randn(*s, generator=g, device="cuda").to(torch.bfloat16)
+    rows = total + n * prefix
+    q, kc, vc = rn(total, H * hd), rn(KV, rows, hd), rn(KV, rows, hd)
+    seqs = torch.tensor([[sum(lens[:i]), m, sum(lens[:i]) + i * prefix, m + prefix if m else 0] for i, m in enumerate(lens)], dtype=torch.int32, device="cuda")
+    launch = getattr(_C.lib(), "_ZN5ittai16attention_launchEPK14IttaiAttentionbP11CUstream_st")      # used by the prefill, not exported
+    launch.argtypes = [C.c_void_p, C.c_bool, C.c_void_p]
+    st, outs = ops.new_status("cuda"), []
+    a = _C.Attention()
+    a.q, a.k, a.v, a.seqs, a.status = q.data_ptr(), kc.data_ptr(), vc.data_ptr(), seqs.data_ptr(), st.data_ptr()
+    a.q_row, a.q_head, a.o_row, a.o_head, a.k_row, a.v_row, a.k_head, a.v_head = H * hd, hd, H * hd, hd, hd, hd, rows * hd, rows * hd
+    a.n_seqs, a.n_heads, a.group, a.head_dim, a.causal, a.max_q_len = n, H, H // KV, hd, 1, max(lens)
+    a.q_rows_total, a.kv_rows_total, a.seqs_ready = total, KV * rows, 1
+    for listed in (False, True, True):
+        out = torch.full((total + 1, H * hd), 9.0, dtype=torch.bfloat16, device="cuda")
+        a.o = out.data_ptr()
+        torch.cuda.synchronize()
+        _C.check(launch(C.addressof(a), listed, ops._stream(q)))
+        ops.check_status(st)
+        outs.append(out)
+    assert torch.equal(outs[0], outs[1]) and torch.equal(outs[0], outs[2]) and (outs[0][-1] == 9.0).all()
+    assert total == 0 or not (outs[0][:total] == 9.0).all(1).any()
