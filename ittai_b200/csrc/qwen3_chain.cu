@@ -507,7 +507,7 @@ __global__ void __launch_bounds__(32 * NB) finish_kernel(const TokenArgs a) {
 
 // ---- attention ------------------------------------------------------------------------------------------------------------
 // One cluster of CS CTAs per (sequence, kv head); rank r takes the r-th piece of the cached positions (if the sequence is long
-// enough for so many, see split_log2), rank 0 also the new one (norm, rotation, append, and its own score).  Three groups of two
+// enough for so many, see pieces), rank 0 also the new one (norm, rotation, append, and its own score).  Three groups of two
 // compute warps take turns on 32-position tiles, a warp 16 positions of each with its own softmax; a seventh warp feeds a ring
 // of six 16 KB tiles (two CTAs per SM).  A warp's 16 positions are 16 MMAs: scores with the keys as A (M = positions) and the two query heads as N columns, P V with
 // V^T as A (ldmatrix.trans on the swizzled tile) and P as B, its middle, low and high parts in columns 0-1, 2-3 and 4-5.
@@ -573,29 +573,31 @@ __device__ __forceinline__ void st_async_f32x2(void* p, int rank, float x, float
                  ::"r"(map_to_cta(p, (uint32_t)rank)), "f"(x), "f"(y), "r"(map_to_cta(bar, (uint32_t)rank)) : "memory");
 }
 
-// log2 of the pieces that the cache of a sequence with `len` positions is cut into, one CTA each.  Measured over all splits and
-// lengths 30 to 8100 (us per step, best split first): 128 CTAs in all are best nearly everywhere (batch 4, 8100: 4 CTAs 1019,
-// 8 1095, 2 1346; batch 2, 8100: 8 CTAs 733, 16 852), because the next projection then still finds room.  Exceptions: a few
-// positions need no split (batch 1, 30: 425, else 428-443), clusters of 16 pay their barrier only from 1200 positions on
-// (batch 1, 800: 8 CTAs 445, 16 451; 3000: 501 and 478), and the longest caches at batch 8 want two CTAs per SM (8100: 4 CTAs
-// 1577, 2 1623; 500: 604 and 592).  Batch 4 is cut in four at every length, which below 48 positions is not the best (30: 471,
-// uncut 442, in two 465).
+// The pieces that the cache of a sequence with `len` positions is cut into, one CTA each.  What decides is whether every cluster of the
+// launch finds room while the projection in front still runs, one CTA per SM: seven clusters of 16 do, 8 of 12, 15 of 8, 16 of 7, 33 of 4.  The
+// eighth of 16 waited for the projection's SMs, and its CTAs asked for their keys when the others were half through.  us per step:
+// batch 1 in 8 / 12 / 16 pieces at 400 positions 384 / 389 / 401, 800 400 / 393 / 403, 2000 435 / 419 / 421, 4096 515 / 468 / 487, 8000 657 / 566
+// / 565 (10 pieces: 391 at 800, 478 at 4096; 14: 481 and, at 8000, 560); batch 2 in 4 / 7 / 8 at 60 402 / 396 / 400, 800 442 / 419 / 422, 4000
+// 669 / 544 / 554, 8000 869 / 700 / 694.  Few positions need no split (batch 1, 30: 425, else 428-443, with the kernels as they were then).  The
+// longest caches at batch 8 want two CTAs per SM (8100: 4 pieces 1577, 2 1623; 500: 604 and 592, likewise).  Batch 4 is cut in four at every
+// length, which below 48 positions was not the best (30: 471, uncut 442, in two 465).
 // A sequence's pieces follow from its OWN length, so that its sums are taken in the same order whatever the others of the
 // batch hold; the clusters of a launch have the size that the longest needs (the rule does not fall with `len`), and in those of
 // a shorter sequence the ranks past its pieces add exact zeros.
-__host__ __device__ constexpr int split_log2(int batch, int len) {
-    if (batch == 4) return 2;
-    if (len <= 48) return 0;
-    if (batch == 1) return len <= 1200 ? 3 : 4;
-    if (batch == 2) return len <= 400 ? 2 : 3;
-    return len <= 700 ? 1 : 2;
+constexpr int kPieces[] = {1, 2, 4, 7, 8, 12};             // cluster sizes, in the order of Plan::exec
+__host__ __device__ constexpr int pieces(int batch, int len) {
+    if (batch == 4) return 4;
+    if (len <= 48) return 1;
+    if (batch == 1) return len <= 400 ? 8 : 12;
+    if (batch == 2) return len <= 6000 ? 7 : 8;
+    return len <= 700 ? 2 : 4;
 }
 
 template <int CS>
 __global__ void __launch_bounds__(kAttnThreads, 2) attn_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constant__ CUtensorMap tm_v, const AttnChainArgs a) {
     extern __shared__ __align__(1024) unsigned char ring_raw[];
     unsigned char* ring = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(ring_raw) + 1023) & ~(uintptr_t)1023);
-    constexpr int NE = 2 * HD / CS;                             // outputs that a rank merges
+    constexpr int kMergers = CS >= 8 ? 8 : CS >= 4 ? 4 : CS, NE = 2 * HD / kMergers;      // the first ranks merge NE outputs each
     __shared__ unsigned long long full[kRing], empty[kRing], arrived;
     __shared__ __align__(16) uint32_t q_s[2][4][20];            // [head][t]: the 16 words that lane t of a quad holds as MMA operand
     __shared__ __align__(16) bf16 k_s[HD];
@@ -613,7 +615,7 @@ __global__ void __launch_bounds__(kAttnThreads, 2) attn_kernel(const __grid_cons
         failed = 0;
         mbar_init(&arrived, 1);
         fence_mbar_init();
-        if constexpr (CS > 1) mbar_expect_tx(&arrived, CS * (NE * 4 + 8));
+        if (CS > 1 && blockIdx.x % CS < kMergers) mbar_expect_tx(&arrived, CS * (NE * 4 + 8));
     }
     __syncthreads();
     // another CTA's shared memory may be written only once that CTA runs: every thread arrives here, waits before the merge
@@ -623,9 +625,8 @@ __global__ void __launch_bounds__(kAttnThreads, 2) attn_kernel(const __grid_cons
     // (late_trigger), so they may be read ahead of the wait.
     const int pos = (int)ld_relaxed(reinterpret_cast<const uint32_t*>(&a.st->cur_pos[b]));
     const int n_old = pos < 0 ? 0 : pos;
-    constexpr int kCsLog2 = CS == 16 ? 4 : CS == 8 ? 3 : CS == 4 ? 2 : CS == 2 ? 1 : 0;
-    const int own = split_log2(a.batch, n_old), lg = own < kCsLog2 ? own : kCsLog2;
-    const int chunk = (((n_old + (1 << lg) - 1) >> lg) + 15) & ~15;
+    const int own = pieces(a.batch, n_old), cut = own < CS ? own : CS;
+    const int chunk = ((n_old + cut - 1) / cut + 15) & ~15;
     const int p0 = rank * chunk < n_old ? rank * chunk : n_old, p1 = p0 + chunk < n_old ? p0 + chunk : n_old;
     const int n_tiles = (p1 - p0 + kTilePos - 1) / kTilePos;
     const int row_base = (int)(head_row * (size_t)a.kv_cap) + p0;
@@ -833,7 +834,7 @@ __global__ void __launch_bounds__(kAttnThreads, 2) attn_kernel(const __grid_cons
             }
         }
         if constexpr (CS > 1) {
-            if (tid < NE / 2) {
+            if (rank < kMergers && tid < NE / 2) {
                 uint32_t spins = 0;
                 while (!mbar_try_wait_cluster(&arrived, 0)) { if (++spins >= a.limit) { failed = 1; break; } }
                 float m = -1e30f, l = 0.f;
@@ -875,7 +876,7 @@ struct Plan {
     bool bound = false;
     cudaStream_t side = nullptr;
     cudaEvent_t last = nullptr;
-    cudaGraphExec_t exec[5][2] = {};      // by log2(CS) and whether the head runs
+    cudaGraphExec_t exec[sizeof(kPieces) / sizeof(int)][2] = {};      // by cluster size and whether the head runs
     std::mutex mu;
 };
 
@@ -909,9 +910,10 @@ static cudaError_t set_attributes() {
     if (e == cudaSuccess) e = prefer_shared(attn_kernel<1>, kAttnSmem);
     if (e == cudaSuccess) e = prefer_shared(attn_kernel<2>, kAttnSmem);
     if (e == cudaSuccess) e = prefer_shared(attn_kernel<4>, kAttnSmem);
+    if (e == cudaSuccess) e = prefer_shared(attn_kernel<7>, kAttnSmem);
     if (e == cudaSuccess) e = prefer_shared(attn_kernel<8>, kAttnSmem);
-    if (e == cudaSuccess) e = prefer_shared(attn_kernel<16>, kAttnSmem);
-    if (e == cudaSuccess) e = cudaFuncSetAttribute(attn_kernel<16>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
+    if (e == cudaSuccess) e = prefer_shared(attn_kernel<12>, kAttnSmem);
+    if (e == cudaSuccess) e = cudaFuncSetAttribute(attn_kernel<12>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
     if (e == cudaSuccess) attr_dev = dev;
     return e;
 }
@@ -941,8 +943,9 @@ static cudaError_t enqueue_token(const Plan& pl, int cs, bool head, cudaStream_t
             case 1: e = launch_attn<1>(pl, a, st); break;
             case 2: e = launch_attn<2>(pl, a, st); break;
             case 4: e = launch_attn<4>(pl, a, st); break;
+            case 7: e = launch_attn<7>(pl, a, st); break;
             case 8: e = launch_attn<8>(pl, a, st); break;
-            default: e = launch_attn<16>(pl, a, st); break;
+            default: e = launch_attn<12>(pl, a, st); break;
         }
         if (e != cudaSuccess) break;
         // gate/up finds no room on an SM while attention is there: its weights come as far as L2
@@ -1018,7 +1021,7 @@ static bool same_binding(const IttaiQwen3Decode& a, const IttaiQwen3Decode& b) {
            a.next_id == b.next_id && a.logits == b.logits && a.workspace == b.workspace && a.status == b.status;
 }
 
-static int capture(Plan* pl, int lg, bool head, cudaGraphExec_t* out) {
+static int capture(Plan* pl, int cs, bool head, cudaGraphExec_t* out) {
     if (pl->side == nullptr) {
         const cudaError_t e = cudaStreamCreateWithFlags(&pl->side, cudaStreamNonBlocking);
         if (e != cudaSuccess) return cuda_fail(e, "cudaStreamCreateWithFlags");
@@ -1026,7 +1029,7 @@ static int capture(Plan* pl, int lg, bool head, cudaGraphExec_t* out) {
     cudaGraph_t g = nullptr;
     cudaError_t e = cudaStreamBeginCapture(pl->side, cudaStreamCaptureModeThreadLocal);
     if (e != cudaSuccess) return cuda_fail(e, "cudaStreamBeginCapture");
-    const cudaError_t el = enqueue_token(*pl, 1 << lg, head, pl->side);
+    const cudaError_t el = enqueue_token(*pl, cs, head, pl->side);
     e = cudaStreamEndCapture(pl->side, &g);
     if (el != cudaSuccess || e != cudaSuccess) {
         if (g != nullptr) cudaGraphDestroy(g);
@@ -1044,14 +1047,16 @@ static int enqueue_call(Plan* pl, const IttaiQwen3Decode& p, int max_len, bool c
     enqueue_begin(*pl, p, st);
     for (int i = 0; i < p.n_steps; ++i) {
         const bool head = i >= p.n_forced - 1;
-        const int lg = split_log2(p.batch, max_len + i);
+        const int cs = pieces(p.batch, max_len + i);
+        int slot = 0;
+        while (kPieces[slot] != cs) ++slot;
         cudaError_t e;
         if (captured) {                                // a graph launch cannot be captured: the kernels themselves can
-            e = enqueue_token(*pl, 1 << lg, head, st);
+            e = enqueue_token(*pl, cs, head, st);
         } else {
-            cudaGraphExec_t& x = pl->exec[lg][head ? 1 : 0];
+            cudaGraphExec_t& x = pl->exec[slot][head ? 1 : 0];
             if (x == nullptr) {
-                const int rc = capture(pl, lg, head, &x);
+                const int rc = capture(pl, cs, head, &x);
                 if (rc != ITTAI_OK) return rc;
             }
             e = cudaGraphLaunch(x, st);

@@ -47,6 +47,13 @@ def test_step_at_length(tiny_hf, batch, length):
 
 
 @gpu
+@pytest.mark.parametrize("batch,length", [(1, 400), (1, 401), (1, 700), (2, 48), (2, 49), (2, 111), (2, 1000)])
+def test_step_at_pieces_that_are_no_power_of_two(tiny_hf, batch, length):
+    """Caches cut in 12 and in 7, of which 8 and 4 merge: both sides of the lines, last pieces that are short or empty."""
+    test_step_at_length(tiny_hf, batch, length)
+
+
+@gpu
 def test_a_captured_stream_gets_the_kernels(tiny_hf):
     """Inside a stream capture the chain enqueues its kernels instead of launching graphs of its own."""
     from ittai_b200.qwen3 import Qwen3Decoder
