@@ -134,7 +134,7 @@ struct GemvArgs {
     int ld_out;
     float eps;
     uint32_t* status;
-    const State* st;        // gate/up: the next layer's cache rows to bring into L2 (k_next [B * 8][kv_cap][128]); nullptr: none
+    const State* st;        // gate/up, or down at batch 1: the next layer's cache rows to bring into L2 (k_next [B * 8][kv_cap][128]); nullptr: none
     const bf16 *k_next, *v_next;
     int kv_cap;
     const unsigned char* ahead;      // O-proj: weights to bring into L2, eight pieces of ahead_bytes per CTA (nullptr: none)
@@ -175,9 +175,13 @@ __global__ void __launch_bounds__(kGemvThreads, 2) gemv_kernel(const GemvArgs a)
         for (int r = lane; r < ROWS; r += 32) bulk_g2s(w_s + r * LD, a.w + (size_t)(row0 + r) * K, K * 2, &landed);
     }
     if (!a.late_trigger) pdl_trigger();
-    if (EPI == kSwiglu && a.k_next != nullptr && warp == 1) {
+    // By gate/up, or at batch 1 by the down projection, which has more time before its wait (gate/up's last CTAs find room only when attention
+    // ends): batch 1 at 60 / 800 / 4096 / 6500 positions 381 / 377, 394 / 390, 469 / 462, 527 / 521; batch 2 at 1000 / 4000 423 / 419, 540 / 545;
+    // batch 4 at 1000 484 / 493.
+    if ((EPI == kSwiglu || (EPI == kResidual && NB == 1)) && a.k_next != nullptr && warp == 1) {
         // an even share of every sequence's cached rows; positions are stable here (see attn_kernel)
-        constexpr int kItems = NB * NKV, kParts = DGU / 48 / kItems;
+        constexpr int kItems = NB * NKV, kParts = DGU / 48 / kItems;                  // both have 128 CTAs
+        static_assert(DGU / 48 == D / 8, "an even share for every CTA");
         const int item = blockIdx.x % kItems, piece = blockIdx.x / kItems;
         int pos = (int)ld_relaxed(reinterpret_cast<const uint32_t*>(&a.st->cur_pos[item / NKV]));
         // More than L2 keeps until it is read.  us per step without / with it: batch 1 at 6500 / 8000 positions (27 / 33 MB a layer) 554 / 531
@@ -953,13 +957,14 @@ static cudaError_t enqueue_token(const Plan& pl, int cs, bool head, cudaStream_t
                    reinterpret_cast<const unsigned char*>(bp(p.wgu, (size_t)l * DGU * D)), DGU * D * 2 / (D / 8) / 8, 0, drop, limit_parked};
         e = launch_pdl(gemv_kernel<NB, DQ, 8, kResidual>, dim3(D / 8), dim3(kGemvThreads), gemv_smem<DQ, 8>(), st, 1, o);
         if (e != cudaSuccess) break;
-        const bool kv_ahead = l + 1 < p.n_layers;
         const size_t kv1 = kv + (size_t)NB * NKV * p.kv_cap * HD;
+        const bf16 *k1 = l + 1 < p.n_layers ? reinterpret_cast<const bf16*>(p.kcache) + kv1 : nullptr, *v1 = reinterpret_cast<const bf16*>(p.vcache) + kv1;
         GemvArgs gu{bp(p.wgu, (size_t)l * DGU * D), w.hmid, bp(p.ln2, (size_t)l * D), nullptr, w.act, FF, p.eps, p.status, w.st,
-                    kv_ahead ? reinterpret_cast<const bf16*>(p.kcache) + kv1 : nullptr, reinterpret_cast<const bf16*>(p.vcache) + kv1, p.kv_cap, nullptr, 0, 0, drop, limit_parked};
+                    NB > 1 ? k1 : nullptr, v1, p.kv_cap, nullptr, 0, 0, drop, limit_parked};
         e = launch_pdl(gemv_kernel<NB, D, 48, kSwiglu>, dim3(DGU / 48), dim3(kGemvThreads), gemv_smem<D, 48>(), st, 1, gu);
         if (e != cudaSuccess) break;
-        GemvArgs dn{bp(p.wd, (size_t)l * D * FF), w.act, nullptr, w.hmid, w.h, D, p.eps, p.status, nullptr, nullptr, nullptr, 0, nullptr, 0, 0, drop, limit_parked};
+        GemvArgs dn{bp(p.wd, (size_t)l * D * FF), w.act, nullptr, w.hmid, w.h, D, p.eps, p.status, w.st,
+                    NB == 1 ? k1 : nullptr, v1, p.kv_cap, nullptr, 0, 0, drop, limit_parked};
         e = launch_pdl(gemv_kernel<NB, FF, 8, kResidual>, dim3(D / 8), dim3(kGemvThreads), gemv_smem<FF, 8>(), st, 1, dn);
     }
     if (e != cudaSuccess) return e;
