@@ -22,7 +22,7 @@
 // Rounding points are the eager modules' (the same as in qwen3_decode.cu).
 //
 // Measured on a B200, us per step, the persistent kernel of qwen3_decode.cu -> this chain: batch 1 at 47 / 4096 / 8100 cached
-// positions 549 -> 376, 575 -> 459, 657 -> 565; batch 4 at 47 / 1000 / 8100 782 -> 423, 830 -> 482, 1419 -> 970; batch 8 at 1000 /
+// positions 549 -> 371, 575 -> 457, 657 -> 565; batch 4 at 47 / 1000 / 8100 782 -> 419, 830 -> 480, 1419 -> 970; batch 8 at 1000 /
 // 8100 1026 -> 612, 2211 -> 1544.  A layer takes 11.5 us at a short cache, from the last store of a kernel to that of the next: attention 3.3,
 // gate/up 2.7, QKV 2.0, down 2.0, O-proj 1.5, of each of which 0.6 to 0.8 are the boundary; the head 47 us at 6.6 TB/s.  What had
 // to go on the way (batch 1, 47 positions): weights through registers (800 us: a kernel's activation loads stand behind the
@@ -86,8 +86,8 @@ __device__ __forceinline__ uint32_t norm_pair(uint32_t x, uint32_t g, float rstd
 // may be read.
 constexpr int kXsLd = D + 32;             // bf16 per row of xs
 __device__ __forceinline__ void gemv_sync() { asm volatile("bar.sync 1, %0;" ::"n"(kGemvThreads) : "memory"); }   // not the head's feeding warp
-template <int NB>
-__device__ __forceinline__ void norm_rows(const bf16* x, const bf16* gain_s, bf16* xs, float* ss_s, int tid, float eps) {
+template <int NB, typename F>
+__device__ __forceinline__ void norm_rows(const bf16* x, const bf16* gain_s, bf16* xs, float* ss_s, int tid, float eps, F&& meanwhile) {
     constexpr int W = 16 / NB, E = 2 * NB;             // warps per row, values per thread
     const int warp = tid >> 5, b = warp / W, e0 = (tid - b * W * 32) * E;
     uint32_t u[NB];
@@ -101,6 +101,7 @@ __device__ __forceinline__ void norm_rows(const bf16* x, const bf16* gain_s, bf1
             u[4 * i] = q.x; u[4 * i + 1] = q.y; u[4 * i + 2] = q.z; u[4 * i + 3] = q.w;
         }
     }
+    meanwhile();
     float s = 0.f;
 #pragma unroll
     for (int i = 0; i < NB; ++i) s = fmaf(bf_lo(u[i]), bf_lo(u[i]), fmaf(bf_hi(u[i]), bf_hi(u[i]), s));
@@ -154,7 +155,7 @@ struct GemvArgs {
 template <int K, int ROWS>
 constexpr uint32_t gemv_smem() { return (uint32_t)ROWS * (K * 2 + 64); }
 
-template <int NB, int K, int ROWS, int EPI>
+template <int NB, int K, int ROWS, int EPI, int EARLY = 0>
 __global__ void __launch_bounds__(kGemvThreads, 2) gemv_kernel(const GemvArgs a) {
     constexpr int KC = ROWS == 32 ? 8 : 16, KW = K / KC, NJ = KW / 32, NR = ROWS == 8 ? 1 : 2, NT = ROWS == 48 ? 3 : 1;
     constexpr int LD = K * 2 + 64;                      // bytes per weight row in shared memory
@@ -203,26 +204,33 @@ __global__ void __launch_bounds__(kGemvThreads, 2) gemv_kernel(const GemvArgs a)
                                                        // left open here may be scheduled behind the wait
     // A warp's weights in registers ahead of the wait: 64 KB of a QKV slice take the shared memory 512 cycles, which stood between the
     // activations and the sums.  Gate/up would need 48 registers for it on top of its own and starts late (its last CTAs find room when
-    // attention ends): held there too, us per step 512 instead of 485 (batch 1, 4096), 499 instead of 482 (batch 4, 1000).  Waiting for the
+    // attention ends): held there too, us per step 512 instead of 485 (batch 1, 4096), 499 instead of 482 (batch 4, 1000); see hold_tiles for what it does.  Waiting for the
     // weights in front of the dependency costs nothing where they are late: asking once and loading the activations first
     // 413 instead of 400 (batch 1, 800).  None held -> this: batch 1 at 47 / 4096 391 -> 380, 498 -> 485, batch 4 and 8 at 1000 497 -> 482, 629 -> 614.
     constexpr bool kHeld = ROWS != 48;
-    uint4 wl[kHeld ? NT : 1][kHeld ? NJ : 1], wh[kHeld && NR == 2 ? NT : 1][kHeld && NR == 2 ? NJ : 1];
-    bool ok = true;
-    if constexpr (kHeld) {
-        ok = mbar_wait_bounded(&landed, 0, a.limit);
+    constexpr int kEarly = kHeld ? NT : EARLY, kRegs = kEarly > 0 ? kEarly : 1;
+    uint4 wl[kRegs][NJ], wh[NR == 2 ? kRegs : 1][NR == 2 ? NJ : 1];
+    auto hold = [&]() {
 #pragma unroll
-        for (int n = 0; n < NT; ++n)
+        for (int n = 0; n < kEarly; ++n)
 #pragma unroll
             for (int j = 0; j < NJ; ++j) {
                 wl[n][j] = lds128(wr + 16 * n * LD + 64 * j);
                 if constexpr (NR == 2) wh[n][j] = lds128(wr + (16 * n + 8) * LD + 64 * j);
             }
+    };
+    bool ok = true;
+    if constexpr (kHeld) {
+        ok = mbar_wait_bounded(&landed, 0, a.limit);
+        hold();
     }
     pdl_wait();
     if (a.late_trigger) pdl_trigger();
     uint4 x[NJ];
-    if constexpr (kNorm) norm_rows<NB>(a.x, gain_s, xs, ss_s, tid, a.eps);
+    // Gate/up, EARLY tiles: while the activations travel, if the weights are there
+    bool there = kHeld || EARLY == 0;
+    auto early = [&]() { if constexpr (!kHeld && EARLY > 0) { there = __all_sync(0xffffffffu, mbar_test(&landed, 0)); if (there) hold(); } };
+    if constexpr (kNorm) norm_rows<NB>(a.x, gain_s, xs, ss_s, tid, a.eps, early);
 #pragma unroll
     for (int j = 0; j < NJ; ++j) {
         if constexpr (kNorm) x[j] = g < NB ? *reinterpret_cast<const uint4*>(xs + g * kXsLd + col + 32 * j) : make_uint4(0u, 0u, 0u, 0u);
@@ -232,14 +240,17 @@ __global__ void __launch_bounds__(kGemvThreads, 2) gemv_kernel(const GemvArgs a)
     if constexpr (EPI == kResidual) {
         if (tid < 8 * NB) res = ldcg_bf16(a.res + (size_t)(tid >> 3) * D + row0 + (tid & 7));
     }
-    if constexpr (!kHeld) ok = mbar_wait_bounded(&landed, 0, a.limit);
+    if constexpr (!kHeld) {
+        ok = mbar_wait_bounded(&landed, 0, a.limit);
+        if (!there) hold();
+    }
 #pragma unroll
     for (int n = 0; n < NT; ++n) {
         float d0[4] = {0.f, 0.f, 0.f, 0.f}, d1[4] = {0.f, 0.f, 0.f, 0.f};
 #pragma unroll
         for (int j = 0; j < NJ; ++j) {
             uint4 lo, hi = make_uint4(0u, 0u, 0u, 0u);
-            if constexpr (kHeld) { lo = wl[n][j]; if constexpr (NR == 2) hi = wh[n][j]; }
+            if (n < kEarly) { lo = wl[n < kRegs ? n : 0][j]; if constexpr (NR == 2) hi = wh[n < kRegs ? n : 0][j]; }
             else { lo = lds128(wr + 16 * n * LD + 64 * j); if constexpr (NR == 2) hi = lds128(wr + (16 * n + 8) * LD + 64 * j); }
             mma16816(d0, lo.x, hi.x, lo.y, hi.y, x[j].x, x[j].y);
             mma16816(d1, lo.z, hi.z, lo.w, hi.w, x[j].z, x[j].w);
@@ -343,7 +354,7 @@ __global__ void __launch_bounds__(kGemvThreads + 32, 1) head_kernel(const HeadAr
     reinterpret_cast<uint32_t*>(gain_s)[tid] = reinterpret_cast<const uint32_t*>(a.gain)[tid];
     gemv_sync();                         // the gain has arrived (see gemv_kernel)
     pdl_wait();
-    norm_rows<NB>(a.x, gain_s, xs, ss_s, tid, a.eps);
+    norm_rows<NB>(a.x, gain_s, xs, ss_s, tid, a.eps, []() {});
     const int col = warp * KW + 8 * t;
     uint4 x[NJ];
 #pragma unroll
@@ -597,6 +608,12 @@ __host__ __device__ constexpr int pieces(int batch, int len) {
     if (batch == 2) return len <= 6000 ? 7 : 8;
     return len <= 700 ? 2 : 4;
 }
+
+// Whether gate/up takes two of its three tiles into registers while the activations travel (the same sums either way).  It pays while its
+// weights are there by then; beside long caches they arrive late, and a tile held then only comes between the wait and the sums.  us per
+// step without / with: batch 1 at 60 / 4096 / 6000 / 8000 positions 377 / 372, 460 / 457, 506 / 508, 559 / 564; batch 2 at 500 / 8000 404 / 400,
+// 702 / 709; batch 4 at 300 / 2000 433 / 430, 561 / 565; batch 8 at 500 / 2000 548 / 545, 748 / 752.  All three tiles spill: 409 at 60.
+__host__ __device__ constexpr bool hold_tiles(int batch, int len) { return batch * len <= 5000; }
 
 template <int CS>
 __global__ void __launch_bounds__(kAttnThreads, 2) attn_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constant__ CUtensorMap tm_v, const AttnChainArgs a) {
@@ -881,7 +898,7 @@ struct Plan {
     bool bound = false;
     cudaStream_t side = nullptr;
     cudaEvent_t last = nullptr;
-    cudaGraphExec_t exec[sizeof(kPieces) / sizeof(int)][2] = {};      // by cluster size and whether the head runs
+    cudaGraphExec_t exec[sizeof(kPieces) / sizeof(int)][2][2] = {};   // by cluster size, whether gate/up holds tiles and whether the head runs
     std::mutex mu;
 };
 
@@ -896,6 +913,7 @@ template <int NB>
 static cudaError_t set_attributes_nb() {
     cudaError_t e = prefer_shared(gemv_kernel<NB, D, 32, kPlain>, gemv_smem<D, 32>());
     if (e == cudaSuccess) e = prefer_shared(gemv_kernel<NB, D, 48, kSwiglu>, gemv_smem<D, 48>());
+    if (e == cudaSuccess) e = prefer_shared(gemv_kernel<NB, D, 48, kSwiglu, 2>, gemv_smem<D, 48>());
     if (e == cudaSuccess) e = prefer_shared(gemv_kernel<NB, DQ, 8, kResidual>, gemv_smem<DQ, 8>());
     if (e == cudaSuccess) e = prefer_shared(gemv_kernel<NB, FF, 8, kResidual>, gemv_smem<FF, 8>());
     if (e == cudaSuccess) e = prefer_shared(head_kernel<NB>, kHeadSmem);
@@ -930,7 +948,7 @@ static cudaError_t launch_attn(const Plan& pl, const AttnChainArgs& a, cudaStrea
 
 // The kernels of one token, in order, on `st` (captured into a graph, or launched as they are).
 template <int NB>
-static cudaError_t enqueue_token(const Plan& pl, int cs, bool head, cudaStream_t st) {
+static cudaError_t enqueue_token(const Plan& pl, int cs, bool held, bool head, cudaStream_t st) {
     const IttaiQwen3Decode& p = pl.p;
     const Buffers& w = pl.w;
     auto bp = [](const void* q, size_t off = 0) { return reinterpret_cast<const bf16*>(q) + off; };
@@ -962,7 +980,7 @@ static cudaError_t enqueue_token(const Plan& pl, int cs, bool head, cudaStream_t
         const bf16 *k1 = l + 1 < p.n_layers ? reinterpret_cast<const bf16*>(p.kcache) + kv1 : nullptr, *v1 = reinterpret_cast<const bf16*>(p.vcache) + kv1;
         GemvArgs gu{bp(p.wgu, (size_t)l * DGU * D), w.hmid, bp(p.ln2, (size_t)l * D), nullptr, w.act, FF, p.eps, p.status, w.st,
                     NB > 1 ? k1 : nullptr, v1, p.kv_cap, nullptr, 0, 0, drop, limit_parked};
-        e = launch_pdl(gemv_kernel<NB, D, 48, kSwiglu>, dim3(DGU / 48), dim3(kGemvThreads), gemv_smem<D, 48>(), st, 1, gu);
+        e = launch_pdl(held ? gemv_kernel<NB, D, 48, kSwiglu, 2> : gemv_kernel<NB, D, 48, kSwiglu>, dim3(DGU / 48), dim3(kGemvThreads), gemv_smem<D, 48>(), st, 1, gu);
         if (e != cudaSuccess) break;
         GemvArgs dn{bp(p.wd, (size_t)l * D * FF), w.act, nullptr, w.hmid, w.h, D, p.eps, p.status, w.st,
                     NB == 1 ? k1 : nullptr, v1, p.kv_cap, nullptr, 0, 0, drop, limit_parked};
@@ -976,12 +994,12 @@ static cudaError_t enqueue_token(const Plan& pl, int cs, bool head, cudaStream_t
     if (e != cudaSuccess) return e;
     return launch_pdl(finish_kernel<NB, true>, dim3(1), dim3(32 * NB), 0, st, 1, t);
 }
-static cudaError_t enqueue_token(const Plan& pl, int cs, bool head, cudaStream_t st) {
+static cudaError_t enqueue_token(const Plan& pl, int cs, bool held, bool head, cudaStream_t st) {
     switch (pl.p.batch) {
-        case 1: return enqueue_token<1>(pl, cs, head, st);
-        case 2: return enqueue_token<2>(pl, cs, head, st);
-        case 4: return enqueue_token<4>(pl, cs, head, st);
-        default: return enqueue_token<8>(pl, cs, head, st);
+        case 1: return enqueue_token<1>(pl, cs, held, head, st);
+        case 2: return enqueue_token<2>(pl, cs, held, head, st);
+        case 4: return enqueue_token<4>(pl, cs, held, head, st);
+        default: return enqueue_token<8>(pl, cs, held, head, st);
     }
 }
 static void enqueue_begin(const Plan& pl, const IttaiQwen3Decode& c, cudaStream_t st) {
@@ -996,9 +1014,10 @@ static void enqueue_begin(const Plan& pl, const IttaiQwen3Decode& c, cudaStream_
 }
 
 static void drop_graphs(Plan* pl) {
-    for (auto& row : pl->exec)
-        for (cudaGraphExec_t& x : row)
-            if (x != nullptr) { cudaGraphExecDestroy(x); x = nullptr; }
+    for (auto& size : pl->exec)
+        for (auto& row : size)
+            for (cudaGraphExec_t& x : row)
+                if (x != nullptr) { cudaGraphExecDestroy(x); x = nullptr; }
 }
 
 }  // namespace chain
@@ -1027,7 +1046,7 @@ static bool same_binding(const IttaiQwen3Decode& a, const IttaiQwen3Decode& b) {
            a.next_id == b.next_id && a.logits == b.logits && a.workspace == b.workspace && a.status == b.status;
 }
 
-static int capture(Plan* pl, int cs, bool head, cudaGraphExec_t* out) {
+static int capture(Plan* pl, int cs, bool held, bool head, cudaGraphExec_t* out) {
     if (pl->side == nullptr) {
         const cudaError_t e = cudaStreamCreateWithFlags(&pl->side, cudaStreamNonBlocking);
         if (e != cudaSuccess) return cuda_fail(e, "cudaStreamCreateWithFlags");
@@ -1035,7 +1054,7 @@ static int capture(Plan* pl, int cs, bool head, cudaGraphExec_t* out) {
     cudaGraph_t g = nullptr;
     cudaError_t e = cudaStreamBeginCapture(pl->side, cudaStreamCaptureModeThreadLocal);
     if (e != cudaSuccess) return cuda_fail(e, "cudaStreamBeginCapture");
-    const cudaError_t el = enqueue_token(*pl, cs, head, pl->side);
+    const cudaError_t el = enqueue_token(*pl, cs, held, head, pl->side);
     e = cudaStreamEndCapture(pl->side, &g);
     if (el != cudaSuccess || e != cudaSuccess) {
         if (g != nullptr) cudaGraphDestroy(g);
@@ -1054,15 +1073,16 @@ static int enqueue_call(Plan* pl, const IttaiQwen3Decode& p, int max_len, bool c
     for (int i = 0; i < p.n_steps; ++i) {
         const bool head = i >= p.n_forced - 1;
         const int cs = pieces(p.batch, max_len + i);
+        const bool held = hold_tiles(p.batch, max_len + i);
         int slot = 0;
         while (kPieces[slot] != cs) ++slot;
         cudaError_t e;
         if (captured) {                                // a graph launch cannot be captured: the kernels themselves can
-            e = enqueue_token(*pl, cs, head, st);
+            e = enqueue_token(*pl, cs, held, head, st);
         } else {
-            cudaGraphExec_t& x = pl->exec[slot][head ? 1 : 0];
+            cudaGraphExec_t& x = pl->exec[slot][held ? 1 : 0][head ? 1 : 0];
             if (x == nullptr) {
-                const int rc = capture(pl, cs, head, &x);
+                const int rc = capture(pl, cs, held, head, &x);
                 if (rc != ITTAI_OK) return rc;
             }
             e = cudaGraphLaunch(x, st);

@@ -113,3 +113,23 @@ def test_attention_keeps_fp32_probabilities(tiny_hf, batch, length):
         wrong = wrong[wrong <= 4]
         off, total = off + int(wrong.sum()), total + 128 * wrong.numel()
     assert total >= 0.9 * 64 * 2048 and off <= 8e-4 * total, off / total
+
+
+@gpu
+def test_tiles_held_by_gate_up_change_no_bit(tiny_hf):
+    """Both sides of the line up to which gate/up holds two of its three tiles in registers, crossed within one call: the logits of the step
+    at each length are those of a call of its own."""
+    from ittai_b200.qwen3 import Qwen3Decoder
+    model, dims = tiny_hf
+    d = Qwen3Decoder(model, max_batch=8, kv_capacity=640)                 # 8 x 625 positions
+    g = torch.Generator(device="cuda").manual_seed(3)
+    d.kcache.normal_(0.0, 1.0, generator=g)
+    d.vcache.normal_(0.0, 0.64, generator=g)
+    d.rewind(624)
+    d.next_id.copy_(torch.arange(8, dtype=torch.int32) + 5)
+    ids = d.decode(3).cpu()
+    last = d.logits.clone()
+    d.rewind(624)
+    d.next_id.copy_(torch.arange(8, dtype=torch.int32) + 5)
+    one = torch.cat([d.decode(1).cpu() for _ in range(3)], 1)
+    assert torch.equal(ids, one) and torch.equal(last, d.logits)
