@@ -475,6 +475,14 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constan
     }
     __syncthreads();
     if (*abort_flag) {
+        // A CTA that gave up may be ahead of others that have yet to write here, and must not leave before they have.  All send, also where
+        // their waits ran out, so the bytes come; should one take longer than this wait, the barrier holds this CTA until the others have left
+        // (threads that have exited count as arrived).  Only here: an arrival by everyone behind the sends costs each launch 0.5 us.
+        if (Cfg::kAsync && splits > 1) {
+            bool all = false;
+            for (uint32_t spins = 0; !all && spins < kSplitSpin; ++spins) all = mbar_try_wait_cluster(arrived, 0);
+            if (!__syncthreads_and(all)) { split_cluster_arrive(); split_cluster_wait(); }
+        }
         if (threadIdx.x == 0) {
             if (atomicCAS(&g.status[0], 0u, (uint32_t)ITTAI_ST_GEMM_TIMEOUT) == 0u) { g.status[1] = blockIdx.x; g.status[2] = (uint32_t)n_kb; }
             // let copies that may still be in flight land before the shared memory is handed back

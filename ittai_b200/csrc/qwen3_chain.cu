@@ -880,6 +880,17 @@ __global__ void __launch_bounds__(kAttnThreads, 2) attn_kernel(const __grid_cons
     }
     __syncthreads();
     if (failed) {
+        // A CTA that gave up may be ahead of ranks that have yet to write here, and must not leave before they have.  All send, also where
+        // their waits ran out, so the bytes come; should one take longer than this wait, the barrier holds this CTA until the others have left
+        // (threads that have exited count as arrived).  Only here: an arrival by everyone behind the sends costs a step 15 us.
+        if constexpr (CS > 1) {
+            bool all = rank >= kMergers;                       // nobody sends there
+            for (uint32_t spins = 0; !all && spins < kSpin; ++spins) all = mbar_try_wait_cluster(&arrived, 0);
+            if (!__syncthreads_and(all)) {
+                asm volatile("barrier.cluster.arrive.release;" ::: "memory");
+                asm volatile("barrier.cluster.wait.acquire;" ::: "memory");
+            }
+        }
         if (tid == 0) {
             if (atomicCAS(&a.status[0], 0u, (uint32_t)ITTAI_ST_STREAM_TIMEOUT) == 0u) { a.status[1] = (uint32_t)n_tiles; a.status[2] = blockIdx.x; }
             const long long t0 = clock64();                    // copies still in flight land before the shared memory is handed back
