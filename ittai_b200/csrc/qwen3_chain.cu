@@ -624,7 +624,7 @@ __global__ void __launch_bounds__(kAttnThreads, 2) attn_kernel(const __grid_cons
     __shared__ __align__(16) uint32_t q_s[2][4][20];            // [head][t]: the 16 words that lane t of a quad holds as MMA operand
     __shared__ __align__(16) bf16 k_s[HD];
     __shared__ __align__(8) float2 pml[2][kAttnWarps + 1];      // reference and sum of the warps' partials and of the new position
-    __shared__ __align__(8) float po[kAttnWarps + 1][2][HD];
+    __shared__ __align__(16) float po[kAttnWarps + 1][2][HD];
     __shared__ __align__(8) bf16 rot_s[4][HD];                  // q gain, k gain, cos | sin of the new position
     __shared__ __align__(8) float rv[CS][CS == 1 ? 2 : NE];     // partials of all ranks for this rank's outputs, which are of one head
     __shared__ __align__(8) float2 rml[CS];
