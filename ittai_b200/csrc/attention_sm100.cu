@@ -74,6 +74,10 @@ __device__ __forceinline__ bool mbar_wait_abortable(void* bar, uint32_t parity, 
     }
     return true;
 }
+// The same for a whole warp: one answer for all lanes, which go on with warp-wide steps (tcgen05.ld) or leave together.
+__device__ __forceinline__ bool mbar_wait_warp(void* bar, uint32_t parity, volatile uint32_t* abort_flag) {
+    return __all_sync(0xffffffffu, mbar_wait_abortable(bar, parity, abort_flag)) != 0;
+}
 __device__ __forceinline__ float ex2_fast(float x) {
     float y;
     asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
@@ -235,7 +239,7 @@ attn_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
                 const uint32_t ph = tcount & 1u;
                 const bool live = mt * 128 + q4 * 32 < q_len;    // a warp whose 32 rows are all padding skips the arithmetic
                 if (has) {
-                    ok = mbar_wait_abortable(bar_s + hf, ph, abort_flag);
+                    ok = mbar_wait_warp(bar_s + hf, ph, abort_flag);
                     if (!ok) break;
                     tc_fence_after();
                 }
@@ -329,7 +333,7 @@ attn_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
                 if (mt == mt0) {
                     // keys between the sequence's end and the MMA's K extent belong to a neighbour: zero those V rows so
                     // that 0 * V stays 0 whatever they hold (V landed long ago; the wait only orders the stores behind it)
-                    ok = mbar_wait_abortable(bar_v, icount & 1u, abort_flag);
+                    ok = mbar_wait_warp(bar_v, icount & 1u, abort_flag);
                     if (!ok) break;
                     const int t = tid - 32;
                     if (t < (n_keys - kv_len) * 8) {
@@ -342,7 +346,7 @@ attn_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
                 tc_fence_before();
                 mbar_arrive_cta(bar_p + hf);
                 // ---- epilogue: this warp's 32 output columns, (O_A 2^(ref_A - m) + O_B 2^(ref_B - m)) / l -> bf16 -> staging tile
-                ok = mbar_wait_abortable(bar_o, ph, abort_flag);      // O follows every arrival on bar_p, which follows the sums
+                ok = mbar_wait_warp(bar_o, ph, abort_flag);      // O follows every arrival on bar_p, which follows the sums
                 if (!ok) break;
                 tc_fence_after();
                 const float ra = xref[r], rb = xref[128 + r];
