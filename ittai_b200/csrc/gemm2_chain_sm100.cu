@@ -286,6 +286,7 @@ gemm2_chain_kernel(const __grid_constant__ ChainParams P) {
                     while (!mbar_try_wait_parked(&res_bar[b], (n >> 1) & 1)) {
                         if (((++spins) & 255u) == 0u && (*abort_flag || spins >= kSpin2)) { ok = false; break; }
                     }
+                    ok = __all_sync(0xffffffffu, ok);
                     if (!ok) { *abort_flag = 1; break; }
                     const unsigned char* rrow = so + 2048 + b * 2048 + lane * 64;
 #pragma unroll

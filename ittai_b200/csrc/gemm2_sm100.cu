@@ -365,10 +365,7 @@ gemm2_bf16_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constan
                 if (has_res) {
                     // out = bf16(residual + bf16(module output)); this thread's row piece of the TMA-filled buffer
                     const uint32_t b = cc & 1;
-                    uint32_t spins = 0;
-                    while (!mbar_try_wait_parked(&res_bar[b], (cc >> 1) & 1)) {
-                        if (((++spins) & 255u) == 0u && (*abort_flag || spins >= kSpin2)) { ok = false; break; }
-                    }
+                    ok = wait(&res_bar[b], (cc >> 1) & 1);
                     if (!ok) { *abort_flag = 1; break; }
                     const unsigned char* rrow = so + 2048 + b * 2048 + lane * 64;
 #pragma unroll

@@ -137,6 +137,7 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant
                     if (((++spins) & 255u) == 0u && (*abort_flag || spins >= kGemmSpin)) { ok = false; break; }
                 }
             }
+            ok = __all_sync(0xffffffffu, ok);                        // one answer for all lanes: what follows is warp-wide
             if (!ok) { *abort_flag = 1; break; }
             tc_fence_after();
             const int row = tile_m * GM + q * 32 + lane;
