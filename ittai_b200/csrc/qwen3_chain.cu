@@ -222,6 +222,7 @@ __global__ void __launch_bounds__(kGemvThreads, 2) gemv_kernel(const GemvArgs a)
     bool ok = true;
     if constexpr (kHeld) {
         ok = mbar_wait_bounded(&landed, 0, a.limit);
+        __syncwarp();                                  // the lanes left the wait one by one
         hold();
     }
     pdl_wait();
@@ -242,6 +243,7 @@ __global__ void __launch_bounds__(kGemvThreads, 2) gemv_kernel(const GemvArgs a)
     }
     if constexpr (!kHeld) {
         ok = mbar_wait_bounded(&landed, 0, a.limit);
+        __syncwarp();
         if (!there) hold();
     }
 #pragma unroll
@@ -343,7 +345,7 @@ __global__ void __launch_bounds__(kGemvThreads + 32, 1) head_kernel(const HeadAr
     if (warp == 16) {                    // the feeding warp: one row per lane
         for (int it = 0; it < n_it && !failed; ++it) {
             const int s = it % kHeadRing, r0 = r_lo + it * kHeadRows, n = r_hi - r0 < kHeadRows ? r_hi - r0 : kHeadRows;
-            if (it >= kHeadRing && !mbar_wait_bounded(&empty[s], ((it / kHeadRing) - 1) & 1, a.limit)) { failed = 1; break; }
+            if (it >= kHeadRing && !__all_sync(0xffffffffu, mbar_wait_bounded(&empty[s], ((it / kHeadRing) - 1) & 1, a.limit))) { failed = 1; break; }
             if (lane == 0) mbar_expect_tx(&full[s], (uint32_t)n * D * 2);
             __syncwarp();
             if (lane < n) bulk_g2s(w_s + (s * kHeadRows + lane) * kHeadLd, a.w + (size_t)(r0 + lane) * D, D * 2, &full[s]);
@@ -368,6 +370,7 @@ __global__ void __launch_bounds__(kGemvThreads + 32, 1) head_kernel(const HeadAr
         uint32_t spins = 0;
         while (!mbar_try_wait_parked(&full[s], (it / kHeadRing) & 1)) { if (++spins >= a.limit || failed) { ok = false; break; } }
         if (!ok) failed = 1;
+        __syncwarp();                    // the lanes left the wait one by one
         const unsigned char* wr = w_s + (s * kHeadRows + g) * kHeadLd + col * 2;
         float d0[4] = {0.f, 0.f, 0.f, 0.f}, d1[4] = {0.f, 0.f, 0.f, 0.f};
 #pragma unroll

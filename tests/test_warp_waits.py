@@ -52,10 +52,7 @@ def _lonely(text):
     return bad
 
 
-LATER = ("qwen3_chain.cu",)
-
-
-@pytest.mark.parametrize("source", sorted({os.path.basename(p) for p in glob.glob(os.path.join(CSRC, "*.cu*"))} - set(LATER)))
+@pytest.mark.parametrize("source", sorted(os.path.basename(p) for p in glob.glob(os.path.join(CSRC, "*.cu*"))))
 def test_lanes_wait_together(source):
     with open(os.path.join(CSRC, source)) as f:
         assert not _lonely(f.read())
