@@ -258,6 +258,9 @@ typedef struct IttaiGemm {
  * (src/ittai/qwen3/sm80.py:175-272, src/ittai/qwen3/sm90.py:256-316, src/ittai/siglip/kernel.py:197-333). */
 int ittai_gemm_bf16_launch(const IttaiGemm* g, void* stream);
 
+/* n calls of ittai_gemm_bf16_launch in order; the first one that fails ends them. */
+int ittai_gemm_each_launch(const IttaiGemm* gemms, int32_t n, void* stream);
+
 /* A chain of 1 to 4 GEMMs in ONE persistent launch: gemms[i + 1].a must be gemms[i].out (k = the previous n), every GEMM
  * has the same M > 128, epilogues ITTAI_EPI_NONE / ITTAI_EPI_GELU with bias, residual (also in place), a folded LayerNorm
  * and stats_out as in ittai_gemm_bf16_launch; the results are bit-identical to the same GEMMs launched one by one.  The tiles

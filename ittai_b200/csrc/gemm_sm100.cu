@@ -274,3 +274,12 @@ int gemm_normed_launch(const IttaiGemm* a, const void* gain, cudaStream_t st) { 
 extern "C" int ittai_gemm_bf16_launch(const IttaiGemm* a, void* stream) {
     return ittai::gemm_bf16_launch(a, reinterpret_cast<cudaStream_t>(stream), nullptr);
 }
+
+extern "C" int ittai_gemm_each_launch(const IttaiGemm* gemms, int32_t n, void* stream) {
+    if (!gemms || n < 1) { ittai::set_error("ittai_gemm_each_launch: no GEMMs"); return ITTAI_E_ARG; }
+    for (int i = 0; i < n; ++i) {
+        const int rc = ittai::gemm_bf16_launch(gemms + i, reinterpret_cast<cudaStream_t>(stream), nullptr);
+        if (rc != ITTAI_OK) return rc;
+    }
+    return ITTAI_OK;
+}

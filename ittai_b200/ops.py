@@ -100,9 +100,9 @@ def gemm_chain(descs, flags: torch.Tensor) -> None:
 
 
 def gemm_each(descs, like: torch.Tensor) -> None:
-    """The GEMMs of a chain as one launch each, on the stream of ``like``'s device: the same bits."""
-    for d in descs:
-        _C.check(_C.lib().ittai_gemm_bf16_launch(C.byref(d), _stream(like)))
+    """The GEMMs of a chain as one launch each, queued by one library call, on the stream of ``like``'s device: the same bits."""
+    n = len(descs)
+    _C.check(_C.lib().ittai_gemm_each_launch((_C.Gemm * n)(*descs), n, _stream(like)))
 
 
 def row_stats(x: torch.Tensor, eps: float, out: torch.Tensor | None = None) -> torch.Tensor:

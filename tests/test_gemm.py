@@ -349,3 +349,36 @@ def test_zero_padded_columns_are_left_out(m, true, padded):
     acc = a.double() @ w.double().t()
     _check(got, (rstd.double()[:, None] * (acc - mean.double()[:, None] * cols.double())).float(), f"{m}x{true} of {padded}")
     assert width * 128 <= padded
+
+
+def test_single_launches_of_a_run_are_queued_by_one_call(monkeypatch):
+    """Single launches in place of a chain (four GEMMs a layer) go through the binding once, as the chain does."""
+    from types import SimpleNamespace
+    from ittai_b200 import _C, ops
+    calls = []
+    count = lambda name: lambda *a: calls.append((name, a)) or 0
+    monkeypatch.setattr(_C, "lib", lambda: SimpleNamespace(ittai_gemm_each_launch=count("each"), ittai_gemm_bf16_launch=count("one")))
+    monkeypatch.setattr(ops, "_stream", lambda t: None)
+    descs = [_C.Gemm() for _ in range(4)]
+    for i, d in enumerate(descs):
+        d.m = 256 + i
+    ops.gemm_each(descs, None)
+    assert [name for name, _ in calls] == ["each"] and calls[0][1][1] == 4 and [d.m for d in calls[0][1][0]] == [256, 257, 258, 259]
+
+
+@gpu
+def test_a_run_of_single_launches(monkeypatch):
+    """The bits of the calls one by one; a record that is refused ends the run with its message, those before it have run."""
+    from ittai_b200 import _C, ops
+    a, w, st = _rand(300, 768, seed=81), _rand(768, 768, scale=0.05, seed=82), ops.new_status("cuda")
+    want = ops.gemm(ops.gemm(a, w, st), w, st, epi=_C.EPI_GELU)
+    d0, x = ops.gemm_desc(a, w, st)
+    d1, y = ops.gemm_desc(x, w, st, epi=_C.EPI_GELU)
+    ops.gemm_each([d0, d1], a)
+    assert torch.equal(y, want)
+    x.zero_()
+    d1.k = 100
+    with pytest.raises(_C.IttaiError, match="multiple"):
+        ops.gemm_each([d0, d1], a)
+    ops.check_status(st)
+    assert torch.equal(x, ops.gemm(a, w, st))
