@@ -301,6 +301,10 @@ typedef struct IttaiAttention {
     uint32_t* status;      /* [ITTAI_STATUS_WORDS] device words, or NULL */
 } IttaiAttention;
 int ittai_attention_launch(const IttaiAttention* a, void* stream);
+/* The same for sequences packed one behind the other: the caller vouches that no two records share a query row.  Where sequences differ in
+ * length the key-loop kernel then takes its tiles from a list instead of a grid of all sequences by the longest (seqs_ready = 1, two query
+ * heads to a key/value head). */
+int ittai_attention_packed_launch(const IttaiAttention* a, void* stream);
 
 /* ---- Qwen3 prefill ------------------------------------------------------------------------------------- */
 

@@ -420,16 +420,17 @@ bool attn_tc_supported(const IttaiAttention* p);          // attention_sm100.cu
 int attn_tc_launch(const IttaiAttention* p, cudaStream_t st);
 bool attn_fa_supported(const IttaiAttention* p);          // attention_fa_sm100.cu
 int attn_fa_launch(const IttaiAttention* p, bool disjoint, cudaStream_t st);
-int attention_launch(const IttaiAttention* p, bool disjoint, cudaStream_t st);
+static int attention_launch(const IttaiAttention* p, bool disjoint, cudaStream_t st);
 
 }  // namespace ittai
 
 using namespace ittai;
 
 extern "C" int ittai_attention_launch(const IttaiAttention* p, void* stream) { return attention_launch(p, false, (cudaStream_t)stream); }
+extern "C" int ittai_attention_packed_launch(const IttaiAttention* p, void* stream) { return attention_launch(p, true, (cudaStream_t)stream); }
 
 // `disjoint`: the caller vouches that no two sequences share a query row.
-int ittai::attention_launch(const IttaiAttention* p, bool disjoint, cudaStream_t stream) {
+static int ittai::attention_launch(const IttaiAttention* p, bool disjoint, cudaStream_t stream) {
     if (!p || !p->q || !p->k || !p->v || !p->o || !p->seqs) { set_error("attention: null pointer"); return ITTAI_E_ARG; }
     if (p->head_dim != 64 && p->head_dim != 128 && !(p->head_dim == 80 && attn_fa_supported(p))) {
         set_error("attention: head_dim %d (64, 128, or 80 in the packed layout of the key-loop kernel)", p->head_dim);

@@ -10,7 +10,6 @@
 namespace ittai {
 
 void set_error(const char* fmt, ...);
-int attention_launch(const IttaiAttention* p, bool disjoint, cudaStream_t st);                                              // attention.cu
 int embed_rows_launch(const int32_t* ids, const void* table, void* out, int rows, int vocab, float* stats, void* stream);   // rowwise.cu
 
 constexpr int D = ITTAI_Q3_D, DQ = ITTAI_Q3_DQ, DQKV = ITTAI_Q3_DQKV, DGU = ITTAI_Q3_DGU, FF = ITTAI_Q3_FF, HD = ITTAI_Q3_HD, NKV = ITTAI_Q3_NKV;
@@ -71,7 +70,7 @@ static int prefill_launch(const IttaiQwen3Prefill* p, void* st) {
         a.k_row = a.v_row = p->k_row; a.k_head = a.v_head = p->k_head; a.k_seq = a.v_seq = p->k_seq;
         a.seqs = p->seqs; a.n_seqs = p->n_seqs; a.n_heads = NH; a.group = NH / NKV; a.head_dim = HD; a.causal = 1; a.max_q_len = p->max_q_len;
         a.q_rows_total = T; a.kv_rows_total = (int32_t)p->kv_rows_total; a.status = p->status; a.seqs_ready = 1;
-        if (rc == ITTAI_OK) rc = attention_launch(&a, true, (cudaStream_t)st);
+        if (rc == ITTAI_OK) rc = ittai_attention_packed_launch(&a, st);
         gemm(p->attn, at(p->wo, (size_t)l * D * DQ), p->h, D, DQ, ITTAI_EPI_NONE, p->h, false, fold || normed, nullptr);
         if (!fold && !normed) norm(g2);
         gemm(fold || normed ? p->h : p->xn, at(fold ? p->wgu_f : p->wgu, (size_t)l * DGU * D), p->act, DGU, D, ITTAI_EPI_SWIGLU, nullptr, fold || normed, false, nullptr, normed ? g2 : nullptr);

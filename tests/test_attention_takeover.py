@@ -120,8 +120,6 @@ def test_listed_tiles_match_the_grid(lens, prefix):
     rows = total + n * prefix
     q, kc, vc = rn(total, H * hd), rn(KV, rows, hd), rn(KV, rows, hd)
     seqs = torch.tensor([[sum(lens[:i]), m, sum(lens[:i]) + i * prefix, m + prefix if m else 0] for i, m in enumerate(lens)], dtype=torch.int32, device="cuda")
-    launch = getattr(_C.lib(), "_ZN5ittai16attention_launchEPK14IttaiAttentionbP11CUstream_st")      # used by the prefill, not exported
-    launch.argtypes = [C.c_void_p, C.c_bool, C.c_void_p]
     st, outs = ops.new_status("cuda"), []
     a = _C.Attention()
     a.q, a.k, a.v, a.seqs, a.status = q.data_ptr(), kc.data_ptr(), vc.data_ptr(), seqs.data_ptr(), st.data_ptr()
@@ -132,7 +130,8 @@ def test_listed_tiles_match_the_grid(lens, prefix):
         out = torch.full((total + 1, H * hd), 9.0, dtype=torch.bfloat16, device="cuda")
         a.o = out.data_ptr()
         torch.cuda.synchronize()
-        _C.check(launch(C.addressof(a), listed, ops._stream(q)))
+        launch = _C.lib().ittai_attention_packed_launch if listed else _C.lib().ittai_attention_launch
+        _C.check(launch(C.byref(a), ops._stream(q)))
         ops.check_status(st)
         outs.append(out)
     assert torch.equal(outs[0], outs[1]) and torch.equal(outs[0], outs[2]) and (outs[0][-1] == 9.0).all()
