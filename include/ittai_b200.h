@@ -64,7 +64,8 @@ enum {
                                      status[2]=CTA, status[3]=tag seen, status[4]=tag expected */
     ITTAI_ST_BAD_TOKEN = 3,       /* status[1]=token id, status[2]=step, status[3]=position, status[4]=sequence */
     ITTAI_ST_STREAM_TIMEOUT = 4,  /* a weight-stream copy did not land: status[1]=entry, status[2]=CTA */
-    ITTAI_ST_GEMM_TIMEOUT = 5     /* a pipeline wait of a tensor-core kernel (GEMM, attention) ran out: status[1]=CTA */
+    ITTAI_ST_GEMM_TIMEOUT = 5,    /* a pipeline wait of a tensor-core kernel (GEMM, attention) ran out: status[1]=CTA */
+    ITTAI_ST_BAD_SEQS = 6         /* records of packed sequences share query rows: status[1]=tiles, status[2]=tiles that the rows can make */
 };
 
 /* Phases of one decoded token, in execution order inside a layer (ids used by ittai_qwen3_phase_launch). */
@@ -303,7 +304,7 @@ typedef struct IttaiAttention {
 int ittai_attention_launch(const IttaiAttention* a, void* stream);
 /* The same for sequences packed one behind the other: the caller vouches that no two records share a query row.  Where sequences differ in
  * length the key-loop kernel then takes its tiles from a list instead of a grid of all sequences by the longest (seqs_ready = 1, two query
- * heads to a key/value head). */
+ * heads to a key/value head); records that share rows, found out by tiles that the list has no room for, end in ITTAI_ST_BAD_SEQS. */
 int ittai_attention_packed_launch(const IttaiAttention* a, void* stream);
 
 /* ---- Qwen3 prefill ------------------------------------------------------------------------------------- */
@@ -328,7 +329,8 @@ typedef struct IttaiQwen3Prefill {
                               GEMMs from T > 128 on (layer 0's first norm reads the embedding rows and stays a pass) */
     const int32_t *ids, *pos, *seq, *slot;  /* [T] device */
     const int32_t* seqs;   /* [n_seqs][4] device, as in IttaiAttention with seqs_ready = 1: written by a copy, not by a kernel that
-                              this library queued just before */
+                              this library queued just before.  No two records share a query row, and all lie inside the T rows
+                              (as in ittai_attention_packed_launch) */
     void *kcache, *vcache; /* layer 0's store */
     int64_t kv_layer;      /* elements from one layer's store to the next (0: one store reused by every layer) */
     int64_t k_row, k_head, k_seq;  /* strides of the store, elements */

@@ -241,7 +241,13 @@ attn_fa_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
     extern __shared__ __align__(1024) unsigned char fa_raw[];
     unsigned char* sm = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(fa_raw) + 1023) & ~(uintptr_t)1023);
     FaList* list = reinterpret_cast<FaList*>(sm + kFaList);
-    if constexpr (LIST) fa_build_list(a, list);
+    if constexpr (LIST) {
+        fa_build_list(a, list);
+        // Records that share rows have more tiles than the grid, whose length the host takes from the rows: the surplus is not computed.
+        if (threadIdx.x == 0 && list->total > (int)gridDim.y && atomicCAS(&a.status[0], 0u, (uint32_t)ITTAI_ST_BAD_SEQS) == 0u) {
+            a.status[1] = (uint32_t)list->total; a.status[2] = gridDim.y;
+        }
+    }
     // Grid (heads, sequences, query tiles) with the tiles in descending order: CTAs are handed out in index order, so the
     // causal tiles that walk the most key blocks start first and the last ones are short.
     const FaTile first = fa_tile<HDIM, PAIR, LIST>(a, list, blockIdx.x, blockIdx.y, blockIdx.z);

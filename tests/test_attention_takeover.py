@@ -136,3 +136,26 @@ def test_listed_tiles_match_the_grid(lens, prefix):
         outs.append(out)
     assert torch.equal(outs[0], outs[1]) and torch.equal(outs[0], outs[2]) and (outs[0][-1] == 9.0).all()
     assert total == 0 or not (outs[0][:total] == 9.0).all(1).any()
+
+
+@gpu
+def test_packed_records_that_share_rows_are_reported():
+    """Nine records over the same 300 rows: more tiles than packed sequences of 300 rows can have.  The surplus used to be left out
+    without a word."""
+    import ctypes as C
+    from ittai_b200 import _C, ops
+    hd, n = 128, 300
+    q, kc, vc = (torch.ones(n, w, dtype=torch.bfloat16, device="cuda") for w in (2 * hd, hd, hd))
+    out, st = torch.zeros_like(q), ops.new_status("cuda")
+    seqs = torch.tensor([[0, n, 0, n]] * 9 + [[0, 1, 0, 1]], dtype=torch.int32, device="cuda")
+    a = _C.Attention()
+    a.q, a.k, a.v, a.o, a.seqs, a.status = q.data_ptr(), kc.data_ptr(), vc.data_ptr(), out.data_ptr(), seqs.data_ptr(), st.data_ptr()
+    a.q_row, a.q_head, a.o_row, a.o_head, a.k_row, a.v_row, a.k_head, a.v_head = 2 * hd, hd, 2 * hd, hd, hd, hd, n * hd, n * hd
+    a.n_seqs, a.n_heads, a.group, a.head_dim, a.causal, a.max_q_len, a.q_rows_total, a.kv_rows_total, a.seqs_ready = 10, 2, 2, hd, 1, n, n, n, 1
+    torch.cuda.synchronize()
+    _C.check(_C.lib().ittai_attention_packed_launch(C.byref(a), ops._stream(q)))
+    with pytest.raises(_C.IttaiError, match="share query rows"):
+        ops.check_status(st)
+    a.n_seqs, a.max_q_len = 1, n                                     # one record: no list, nothing to report
+    _C.check(_C.lib().ittai_attention_packed_launch(C.byref(a), ops._stream(q)))
+    ops.check_status(st)
