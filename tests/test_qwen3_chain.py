@@ -116,20 +116,55 @@ def test_attention_keeps_fp32_probabilities(tiny_hf, batch, length):
 
 
 @gpu
-def test_tiles_held_by_gate_up_change_no_bit(tiny_hf):
-    """Both sides of the line up to which gate/up holds two of its three tiles in registers, crossed within one call: the logits of the step
-    at each length are those of a call of its own."""
+@pytest.mark.parametrize("batch,length", [(1, 5000), (2, 2500), (4, 1250), (8, 625)])
+def test_tiles_held_by_gate_up_change_no_bit(tiny_hf, batch, length):
+    """The last length at which gate/up holds two of its three tiles in registers: ids, logits and cache rows of the step are the same,
+    bit for bit, where the bound on the positions that the caller gives (here one more) selects the kernel that holds none."""
+    import ctypes as C
+    from ittai_b200 import _C
     from ittai_b200.qwen3 import Qwen3Decoder
     model, dims = tiny_hf
-    d = Qwen3Decoder(model, max_batch=8, kv_capacity=640)                 # 8 x 625 positions
+    d = Qwen3Decoder(model, max_batch=batch, kv_capacity=length + 8)
     g = torch.Generator(device="cuda").manual_seed(3)
     d.kcache.normal_(0.0, 1.0, generator=g)
     d.vcache.normal_(0.0, 0.64, generator=g)
-    d.rewind(624)
-    d.next_id.copy_(torch.arange(8, dtype=torch.int32) + 5)
-    ids = d.decode(3).cpu()
-    last = d.logits.clone()
-    d.rewind(624)
-    d.next_id.copy_(torch.arange(8, dtype=torch.int32) + 5)
-    one = torch.cat([d.decode(1).cpu() for _ in range(3)], 1)
-    assert torch.equal(ids, one) and torch.equal(last, d.logits)
+    got = []
+    for bound in (length, length + 1):
+        d.rewind(length)
+        d.next_id.copy_(torch.arange(batch, dtype=torch.int32) + 5)
+        d.logits.zero_()
+        out = torch.full((1, batch), -7, dtype=torch.int32, device="cuda")
+        p = d._params(1, 0, None, out, None)
+        _C.check(d.lib.ittai_qwen3_chain_run(d._plan, C.byref(p), bound, d._stream()))
+        d.check_status()
+        got.append((out, d.logits.clone(), d.kcache[:, :, :, length].clone(), d.vcache[:, :, :, length].clone()))
+    assert (got[0][0] >= 0).all() and got[0][1].abs().max() > 0 and all(torch.equal(a, b) for a, b in zip(*got))
+
+
+@gpu
+@pytest.mark.parametrize("length", [6000, 6001])
+def test_step_at_clusters_of_eight_for_two_sequences(tiny_hf, length):
+    """Caches of two sequences cut in 7 up to 6000 positions and in 8 beyond: against the CPU restatement, and the first sequence's bits
+    beside a neighbour on either side of the line."""
+    from ittai_b200.qwen3 import Qwen3Decoder
+    model, dims = tiny_hf
+    cap = 6100
+    g = torch.Generator().manual_seed(length)
+    d = Qwen3Decoder(model, max_batch=2, kv_capacity=cap)
+    kv = [(torch.randn(dims.n_layers, 2, dims.n_kv_heads, cap, dims.head_dim, generator=g) * s).to(torch.bfloat16) for s in (1.0, 0.5)]
+    ids = torch.randint(0, dims.vocab, (2,), generator=g, dtype=torch.int32)
+    R = ref.Qwen3Ref(model.state_dict(), dims, cap)
+    R.k, R.v, R.len = kv[0][:, 0].float(), kv[1][:, 0].float(), length
+    want, first = R.forward(ids[:1].long()), None
+    for other in (40, 5999, 6050):
+        for c, t in zip((d.kcache, d.vcache), kv):
+            c.copy_(t)
+        d.set_length(0, length)
+        d.set_length(1, other)
+        d.next_id.copy_(ids)
+        got = d.decode(1)[0].item()
+        now = (got, d.logits[0].clone(), *(c[:, 0, :, length].clone() for c in (d.kcache, d.vcache)))
+        first = first or now
+        assert now[0] == first[0] and all(torch.equal(a, b) for a, b in zip(now[1:], first[1:])), other
+    logits = first[1].float().cpu()
+    assert (logits - want).abs().max() <= 3e-2 and F.cosine_similarity(logits, want, dim=0) >= 0.9995

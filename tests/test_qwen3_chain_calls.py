@@ -81,6 +81,33 @@ def test_a_wait_that_runs_out_ends_the_call(tiny_hf, batch):
 
 
 @gpu
+@pytest.mark.parametrize("batch,length", [(1, 60), (1, 500), (2, 60), (4, 30)])
+def test_a_wait_that_runs_out_beside_clusters(tiny_hf, batch, length):
+    """The same where the attention runs in clusters (of 8, 12, 7 and 4): the call ends with a report, the next one goes on."""
+    import ctypes as C
+    from ittai_b200 import _C
+    from ittai_b200.qwen3 import Qwen3Decoder
+    model, dims = tiny_hf
+    d = Qwen3Decoder(model, max_batch=batch, kv_capacity=600)
+    g = torch.Generator(device="cuda").manual_seed(length)
+    d.kcache.normal_(0.0, 1.0, generator=g)
+    d.vcache.normal_(0.0, 0.5, generator=g)
+    d.rewind(length)
+    d.next_id.fill_(7)
+    want = d.decode(3).cpu()
+    d.rewind(length)
+    d.next_id.fill_(7)
+    out = torch.full((2, batch), -7, dtype=torch.int32, device="cuda")
+    p = d._params(2, 0, None, out, None)
+    p.flags, p.spin_limit = _C.F_TEST_DROP_CTA, 64
+    _C.check(d.lib.ittai_qwen3_chain_run(d._plan, C.byref(p), length, d._stream()))
+    with pytest.raises(_C.IttaiError, match="stream"):
+        d.check_status()
+    assert (out == -7).all() and d.pos.tolist() == d.lengths == [length] * batch
+    assert torch.equal(d.decode(3).cpu(), want)
+
+
+@gpu
 def test_a_reported_failure_is_not_reported_again(tiny_hf):
     """After a failed decode, prefills that go well are accepted; so is what follows a second failure."""
     from ittai_b200._C import IttaiError
