@@ -332,10 +332,11 @@ def test_rotary_runs_cross_from_q_to_k(m):
 @pytest.mark.parametrize("true,padded", [(1152, 1280), (1100, 1280), (64, 256)])
 @pytest.mark.parametrize("m", [40, 300, 2600])
 def test_zero_padded_columns_are_left_out(m, true, padded):
-    """A folded LayerNorm over the true width of a zero-padded A (split-K, one-SM and pair tiles): the bits of the same GEMM without
-    ``stats_k``, whose statistics are given ready-made, since zero products change no sum."""
-    from ittai_b200 import ops
-    n, width = 768, (true + 127) // 128
+    """A folded LayerNorm over the true width of a zero-padded A (split-K, and above 128 rows pair tiles): the columns from the true width,
+    rounded up to a k-block, on are not read (NaNs in W there do not show), and the bits are those of the GEMM whose K ends there."""
+    import ctypes as C
+    from ittai_b200 import _C, ops
+    n, width = 768, -(-true // 64) * 64
     a = torch.zeros(m, padded, dtype=torch.bfloat16, device="cuda")
     w = torch.zeros(n, padded, dtype=torch.bfloat16, device="cuda")
     a[:, :true], w[:, :true] = _rand(m, true, seed=71), _rand(n, true, scale=0.05, seed=72)
@@ -344,11 +345,18 @@ def test_zero_padded_columns_are_left_out(m, true, padded):
     cols, st = w.float().sum(1).contiguous(), ops.new_status("cuda")
     mean = x.sum((1, 2)) / true
     rstd = torch.rsqrt(x.pow(2).sum((1, 2)) / true - mean * mean + 1e-6)
-    got = ops.gemm(a, w, st, row_stats=parts, col_sums=cols, stats_eps=1e-6, stats_k=true, static_w=True)
-    ops.check_status(st)
     acc = a.double() @ w.double().t()
-    _check(got, (rstd.double()[:, None] * (acc - mean.double()[:, None] * cols.double())).float(), f"{m}x{true} of {padded}")
-    assert width * 128 <= padded
+    want = (rstd.double()[:, None] * (acc - mean.double()[:, None] * cols.double())).float()
+    w[:, width:] = float("nan")
+    for static_w in (True,) if m <= 128 else (True, False):
+        kw = dict(row_stats=parts, col_sums=cols, stats_eps=1e-6, stats_k=true, static_w=static_w)
+        got = ops.gemm(a, w, st, **kw)
+        d, narrow = ops.gemm_desc(a, w, st, **kw)
+        d.k = width
+        _C.check(_C.lib().ittai_gemm_bf16_launch(C.byref(d), ops._stream(a)))
+        ops.check_status(st)
+        _check(got, want, f"{m}x{true} of {padded}")
+        assert torch.equal(got, narrow)
 
 
 def test_single_launches_of_a_run_are_queued_by_one_call(monkeypatch):
