@@ -75,7 +75,10 @@ def chain_pays(rows: int, gemms, n_sms: int) -> bool:
     1568, 2156, 3136 rows 879 / 873, 945 / 927, 1066 / 1068, variable resolution with 2048 and 4096 902 / 876 and 1139 / 1089, so400m with
     1458, 2187 2781 / 2736, 3011 / 2975; beyond the line 4704, 6272, 9408 rows 1195 / 1216, 1484 / 1704, 1991 / 2144, so400m with 2916,
     5832 3638 / 3661, 6335 / 6549.  Where the single launches' rounds are full to 3 % (12 544 rows: 5.96, 1.99, 7.95 and 1.99 rounds) a chain
-    has nothing to fill: 2663 / 2642; with 16 384 rows, 8 % of the rounds empty, 3397 / 3485."""
+    has nothing to fill.  ViT-B with 6076, 12 152, 12 544, 18 228, 18 816 rows 1424 / 1377, 2573 / 2581, 2676 / 2640, 3879 / 3800, 3922 / 3797, variable
+    resolution with 6144, 12 288, 18 432, 18 944 1362 / 1315, 2525 / 2523, 3817 / 3749, 3867 / 3741, so400m with 10 935, 18 225, 21 870, 26 244, 33 534, 43 740
+    10932 / 11034, 18808 / 18498, 22978 / 22539, 27237 / 26273, 34499 / 33268, 45352 / 44682; on the other side, 8 to 27 % of the rounds empty, 12 740,
+    15 680, 16 384 rows 2716 / 2891, 3312 / 3380, 3397 / 3485, so400m with 10 206, 11 664 10149 / 10679, 11802 / 12550."""
     pairs, blocks = n_sms // 2, -(-rows // 256)
     tiles = [(blocks * (n // 256), k) for n, k in gemms]
     if tiles[0][0] <= 2 * pairs:

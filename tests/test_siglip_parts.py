@@ -173,3 +173,30 @@ def test_a_new_staging_buffer_waits_for_the_block_s_last_user(slot):
     got = emb.embed(px)
     assert any(b.data_ptr() == ptr for b in emb._staged), "the block was not reused: the test does not test"
     assert torch.equal(seen, torch.arange(seen.numel(), dtype=torch.float32, device="cuda")) and torch.equal(got, want)
+
+
+@gpu
+@pytest.mark.parametrize("kind,batch", [("vit", 6), ("vit", 25), ("naflex", 5), ("so400m", 2), ("so400m", 5)])
+def test_chained_and_single_launches_give_the_same_bits(monkeypatch, kind, batch):
+    """Which of the two a forward takes follows from its rows; with the choice forced either way, on plain launches and from a graph."""
+    from ittai_b200.siglip import kernel
+    build = {"vit": hf.build_hf, "naflex": hf.build_hf_naflex, "so400m": hf.build_hf_so400m}[kind]
+    vm = build(n_layers=2, device="cuda")
+    if kind == "naflex":
+        inp = hf.naflex_inputs(SHAPES[:batch], seed=31)
+    else:
+        side = 224 if kind == "vit" else 384
+        inp = {"pixel_values": torch.randn(batch, 3, side, side, generator=torch.Generator().manual_seed(31))}
+    got, chains = {}, []
+    real = kernel.ops.gemm_chain
+    monkeypatch.setattr(kernel.ops, "gemm_chain", lambda *a: chains.append(1) or real(*a))
+    for chained in (True, False):
+        monkeypatch.setattr(kernel, "chain_pays", lambda *a: chained)
+        eng = kernel.Engine(vm, batch)
+        assert eng.chain
+        before = len(chains)
+        got[chained] = [eng.forward(inp).clone() for _ in range(3)]
+        eng.check()
+        assert (len(chains) > before) == chained
+        assert all(torch.equal(g, got[chained][0]) for g in got[chained])
+    assert torch.equal(got[True][0], got[False][0])
