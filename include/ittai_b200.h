@@ -175,11 +175,12 @@ int ittai_qwen3_phase_launch(const IttaiQwen3Decode* p, int phase, int layer, vo
 
 /* The same decode as a chain of small kernels, one CUDA graph per token, for callers that keep a plan: same struct, same
  * results (the arithmetic and its rounding points are those of ittai_qwen3_decode_launch; sums run in another order).
- * `plan` owns the graphs, which are captured at the first token that needs each of them (a graph per power-of-two split
- * of the attention, 2 ms each) and again when a pointer or size of *p other than n_steps, n_forced, forced, out_ids,
- * step_ns changes.  `max_len`: an upper bound of pos[b] over the sequences.  It picks the cluster size of a launch; a
- * sequence's results follow from its own length and `batch` alone, bit for bit.  p->phase_clk is not used.  An id or position out of range ends in ITTAI_ST_BAD_TOKEN, a wait that runs out in
- * ITTAI_ST_STREAM_TIMEOUT: the steps from there on store no id, `next_id` keeps the last good
+ * `plan` owns the graphs, which are captured at the first token that needs each of them (a graph per cluster size
+ * of the attention, with and without the head, with gate/up's tiles held in registers and not; 0.6 ms each where nothing
+ * hides it) and again when a pointer or size of *p other than n_steps, n_forced, forced, out_ids, step_ns changes.
+ * `max_len`: an upper bound of pos[b] over the sequences.  It picks the cluster size and the gate/up kernel of a launch; a
+ * sequence's results follow from its own length and `batch` alone, bit for bit.  p->phase_clk is not used.  An id or
+ * position out of range ends in ITTAI_ST_BAD_TOKEN, a wait that runs out in ITTAI_ST_STREAM_TIMEOUT: the steps from there on store no id, `next_id` keeps the last good
  * step's id and `pos` is what it was before the call.  A stream that is being captured gets the kernels themselves.  Calls on one plan are serialised,
  * on the host and on the device, whatever streams they are on; only a captured call's replays are the caller's to order. */
 int ittai_qwen3_chain_create(void** plan);

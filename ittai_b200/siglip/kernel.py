@@ -87,8 +87,8 @@ def chain_pays(rows: int, gemms, n_sms: int) -> bool:
 
 
 def part_size(n: int, B: int, S: int, chain: bool) -> int:
-    """Images to run for a short batch of ``n``: at least the 1024 rows from which on the chained GEMMs are used where the full
-    batch of ``B`` uses them: an image's result then does not depend on the batch it came in.  Without chains (fewer than 1024
+    """Images to run for a short batch of ``n``: where the full batch of ``B`` takes its sums over K in one piece (chained, or the same
+    GEMMs one by one, from 1024 rows on) at least that many rows: an image's result then does not depend on the batch it came in.  Without chains (fewer than 1024
     rows in the full batch) the GEMMs may split their sums over K by the number of rows, and it does in its last bits."""
     return max(n, min(B, -(-1024 // S))) if chain else n
 
