@@ -182,6 +182,128 @@ __global__ void __launch_bounds__(WARPS * 32) attn_fwd_kernel(const AttnArgs a) 
     }
 }
 
+// Few queries (at most 32 a sequence), causal, head_dim 128: a short prompt.  One CTA per (sequence, head), two warps per 16 queries that both
+// compute the scores and share the output's 128 columns out; 32 keys a step, the next step's on their way meanwhile.  It runs once per layer, so
+// what attn_fwd_kernel spends here, its 64-key steps unrolled for keys that do not exist, is code to be fetched (see the attention of
+// qwen3_chain.cu) and masks: a forward of 3 / 8 / 23 / 32 tokens 431 / 455 / 612 / 721 us with it, 375 / 401 / 557 / 664 with this one.
+constexpr int kFewRows = 32, kFewKeys = 32, kFewThreads = 128;
+__device__ __forceinline__ float ex2_ftz(float x) {
+    float y;
+    asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+    return y;
+}
+__global__ void __launch_bounds__(kFewThreads) attn_few_kernel(const AttnArgs a, int seqs_ready) {
+    constexpr int HD = 128;
+    extern __shared__ __align__(128) unsigned char attn_smem[];
+    bf16* sq = reinterpret_cast<bf16*>(attn_smem);
+    bf16* skv = sq + kFewRows * HD;                                   // [2][K | V][32 * HD]
+    const int tid = threadIdx.x, warp = warp_index(), lane = tid & 31, g = lane >> 2, t = lane & 3;
+    pdl_trigger();
+    int4 sinfo;
+    if (seqs_ready) sinfo = a.seqs[blockIdx.z];
+    pdl_wait();
+    if (!seqs_ready) sinfo = a.seqs[blockIdx.z];
+    const int q_len = sinfo.y, kv_len = sinfo.w, qb = blockIdx.x * kFewRows;
+    if (qb >= q_len) return;
+    const int head = blockIdx.y, kvh = head / a.group;
+    const bf16* qp = a.q + (long long)(sinfo.x + qb) * a.q_row + (long long)head * a.q_head;
+    const bf16* kp = a.k + (long long)blockIdx.z * a.k_seq + (long long)kvh * a.k_head + (long long)sinfo.z * a.k_row;
+    const bf16* vp = a.v + (long long)blockIdx.z * a.v_seq + (long long)kvh * a.v_head + (long long)sinfo.z * a.v_row;
+    const int q_rows = q_len - qb < kFewRows ? q_len - qb : kFewRows;
+    const int shift = kv_len - q_len + qb;                            // row i of the tile sees keys j <= i + shift
+    const int kv_end = q_rows + shift < kv_len ? q_rows + shift : kv_len;
+    // thread: 16-byte piece tid % 16 of rows tid / 16 + 8 i
+    const int lr = tid >> 4, lc = tid & 15;
+    auto load = [&](bf16* dst, const bf16* src, long long row_stride, int rows) {
+#pragma unroll
+        for (int i = 0; i < 4; ++i) cp_async16(dst + sw<HD>(lr + 8 * i, lc), src + (long long)(lr + 8 * i < rows ? lr + 8 * i : 0) * row_stride + lc * 8, lr + 8 * i < rows);
+    };
+    auto load_kv = [&](int kb, int buf) {
+        bf16* dst = skv + (size_t)buf * 2 * kFewKeys * HD;
+        load(dst, kp + (long long)kb * a.k_row, a.k_row, kv_end - kb);
+        load(dst + kFewKeys * HD, vp + (long long)kb * a.v_row, a.v_row, kv_end - kb);
+        asm volatile("cp.async.commit_group;" ::: "memory");
+    };
+    load(sq, qp, a.q_row, q_rows);
+    if (kv_end > 0) load_kv(0, 0); else asm volatile("cp.async.commit_group;" ::: "memory");
+    const int rt = 16 * (warp >> 1), half = warp & 1;                 // this warp's 16 queries, and half of the output columns
+    float o[8][4];
+#pragma unroll
+    for (int i = 0; i < 8; ++i) o[i][0] = o[i][1] = o[i][2] = o[i][3] = 0.f;
+    float m0 = -INFINITY, m1 = -INFINITY, l0 = 0.f, l1 = 0.f;         // rows g and g + 8
+    const int r0 = rt + g, r1 = r0 + 8;
+    int buf = 0;
+#pragma unroll 1
+    for (int kb = 0; kb < kv_end; kb += kFewKeys, buf ^= 1) {
+        asm volatile("cp.async.wait_group 0;" ::: "memory");
+        __syncthreads();                                              // this step's keys are there, and the other buffer has been read
+        if (kb + kFewKeys < kv_end) load_kv(kb + kFewKeys, buf ^ 1);
+        const bf16* sk = skv + (size_t)buf * 2 * kFewKeys * HD;
+        const bf16* sv = sk + kFewKeys * HD;
+        float s[4][4];
+#pragma unroll
+        for (int i = 0; i < 4; ++i) s[i][0] = s[i][1] = s[i][2] = s[i][3] = 0.f;
+#pragma unroll
+        for (int ks = 0; ks < HD / 16; ++ks) {
+            uint32_t qf[4], kf[4];
+            ldsm_x4(qf, sq + sw<HD>(rt + (lane & 15), ks * 2 + (lane >> 4)));
+#pragma unroll
+            for (int np = 0; np < 2; ++np) {
+                ldsm_x4(kf, sk + sw<HD>(np * 16 + (lane & 7) + (lane >> 4) * 8, ks * 2 + ((lane >> 3) & 1)));
+                mma16816(s[2 * np], qf, kf[0], kf[1]);
+                mma16816(s[2 * np + 1], qf, kf[2], kf[3]);
+            }
+        }
+        float x0 = -INFINITY, x1 = -INFINITY;
+#pragma unroll
+        for (int i = 0; i < 4; ++i)
+#pragma unroll
+            for (int e = 0; e < 2; ++e) {
+                const int j = kb + 8 * i + 2 * t + e;
+                s[i][e] = j < kv_len && j <= r0 + shift ? s[i][e] * a.scale_log2 : -INFINITY;
+                s[i][e + 2] = j < kv_len && j <= r1 + shift ? s[i][e + 2] * a.scale_log2 : -INFINITY;
+                x0 = fmaxf(x0, s[i][e]); x1 = fmaxf(x1, s[i][e + 2]);
+            }
+        x0 = fmaxf(x0, __shfl_xor_sync(0xffffffffu, x0, 1)); x1 = fmaxf(x1, __shfl_xor_sync(0xffffffffu, x1, 1));
+        x0 = fmaxf(x0, __shfl_xor_sync(0xffffffffu, x0, 2)); x1 = fmaxf(x1, __shfl_xor_sync(0xffffffffu, x1, 2));
+        const float n0 = fmaxf(m0, x0), n1 = fmaxf(m1, x1);
+        const float f0 = n0 == -INFINITY ? 0.f : n0, f1 = n1 == -INFINITY ? 0.f : n1;      // a row without keys so far
+        const float c0 = ex2_ftz(m0 - f0), c1 = ex2_ftz(m1 - f1);
+        m0 = n0; m1 = n1;
+        uint32_t pf[2][4];
+        float p0 = 0.f, p1 = 0.f;
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            const float e0 = ex2_ftz(s[i][0] - f0), e1 = ex2_ftz(s[i][1] - f0), e2 = ex2_ftz(s[i][2] - f1), e3 = ex2_ftz(s[i][3] - f1);
+            p0 += e0 + e1; p1 += e2 + e3;
+            pf[i / 2][(i & 1) * 2] = pack_bf16x2(e0, e1);
+            pf[i / 2][(i & 1) * 2 + 1] = pack_bf16x2(e2, e3);
+        }
+        l0 = l0 * c0 + p0; l1 = l1 * c1 + p1;
+#pragma unroll
+        for (int i = 0; i < 8; ++i) { o[i][0] *= c0; o[i][1] *= c0; o[i][2] *= c1; o[i][3] *= c1; }
+#pragma unroll
+        for (int ks = 0; ks < 2; ++ks)
+#pragma unroll
+            for (int dp = 0; dp < 4; ++dp) {
+                uint32_t vf[4];
+                ldsm_x4_t(vf, sv + sw<HD>(ks * 16 + (lane & 7) + ((lane >> 3) & 1) * 8, 8 * half + dp * 2 + (lane >> 4)));
+                mma16816(o[2 * dp], pf[ks], vf[0], vf[1]);
+                mma16816(o[2 * dp + 1], pf[ks], vf[2], vf[3]);
+            }
+    }
+    if (rt >= q_rows) return;
+    l0 += __shfl_xor_sync(0xffffffffu, l0, 1); l0 += __shfl_xor_sync(0xffffffffu, l0, 2);
+    l1 += __shfl_xor_sync(0xffffffffu, l1, 1); l1 += __shfl_xor_sync(0xffffffffu, l1, 2);
+    const float i0 = l0 > 0.f ? 1.0f / l0 : 0.f, i1 = l1 > 0.f ? 1.0f / l1 : 0.f;
+    bf16* op = a.o + (long long)(sinfo.x + qb) * a.o_row + (long long)head * a.o_head + 64 * half + 2 * t;
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+        if (r0 < q_rows) *reinterpret_cast<uint32_t*>(op + (long long)r0 * a.o_row + 8 * i) = pack_bf16x2(o[i][0] * i0, o[i][1] * i0);
+        if (r1 < q_rows) *reinterpret_cast<uint32_t*>(op + (long long)r1 * a.o_row + 8 * i) = pack_bf16x2(o[i][2] * i1, o[i][3] * i1);
+    }
+}
+
 // Short sequences (at most 256 keys, dense): one CTA per (sequence, head) keeps the whole K and V in shared memory,
 // loaded once, and every warp runs its 16 query rows against all keys with no CTA-wide barrier after the load: 13 warps
 // for SigLIP's 196 tokens, two CTAs per SM.  K and V are read from HBM once per head instead of once per query block.
@@ -453,6 +575,10 @@ static int ittai::attention_launch(const IttaiAttention* p, bool disjoint, cudaS
     if (p->head_dim == 64 && !p->causal && ql == 1) {
         const cudaError_t e1 = launch_pdl(attn_q1_kernel, dim3(nh, ns), dim3(32 * kQ1Warps), 0, st, 1, a);
         return e1 == cudaSuccess ? ITTAI_OK : cuda_fail(e1, "launch attn_q1_kernel");
+    }
+    if (p->head_dim == 128 && p->causal && ql <= kFewRows) {
+        const cudaError_t e1 = launch_pdl(attn_few_kernel, dim3(1, nh, ns), dim3(kFewThreads), (size_t)(kFewRows + 4 * kFewKeys) * 128 * 2, st, 1, a, p->seqs_ready);
+        return e1 == cudaSuccess ? ITTAI_OK : cuda_fail(e1, "launch attn_few_kernel");
     }
     if (p->head_dim == 128) rc = p->causal ? attn_launch<128, true, 4>(a, ql, nh, ns, st) : attn_launch<128, false, 4>(a, ql, nh, ns, st);
     else if (!p->causal && ql > 64 && ql <= 256 && p->max_kv_len > 0 && p->max_kv_len <= kShortKeys) rc = attn_short_launch(a, ql, nh, ns, st);

@@ -60,3 +60,20 @@ def test_more_shapes_than_graphs(tiny_hf):
             assert torch.equal(eng.forward([ids(n)]), w), n
         assert sorted(eng._graphs.graphs) == [(n, 1, n) for n in (2, 3, 4)]
     eng.check()
+
+
+@gpu
+def test_a_short_prompt_behind_a_cached_one(tiny_hf):
+    """The attention of few queries with cached keys in front of them, several steps of 32: a prompt appended in two pieces against the prompt
+    at once (keys and values of two layers; a
+    bf16 rounding is off by 1.1e-3 rms, eight in a row a layer: sqrt(2 * 16) * 1.1e-3 = 6.2e-3, half as much again for few tokens)."""
+    from ittai_b200.qwen3 import Qwen3Decoder
+    model, dims = tiny_hf
+    ids = hf.prompt_ids(150, seed=4, vocab=dims.vocab)
+    whole, pieces = (Qwen3Decoder(model, max_batch=1, kv_capacity=256) for _ in range(2))
+    whole.prefill_cache(ids)
+    for a, b in ((0, 97), (97, 98), (98, 128), (128, 150)):
+        pieces.prefill_cache(ids[a:b])
+    for a, b in ((whole.kcache, pieces.kcache), (whole.vcache, pieces.vcache)):
+        a, b = a[..., :150, :].float(), b[..., :150, :].float()
+        assert torch.linalg.vector_norm(a - b) <= 9.3e-3 * torch.linalg.vector_norm(b)
