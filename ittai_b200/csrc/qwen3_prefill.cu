@@ -6,11 +6,12 @@
 
 #include "../../include/ittai_b200.h"
 #include "gemm_split.h"
+#include "qwen3_short.h"
 
 namespace ittai {
 
 void set_error(const char* fmt, ...);
-int embed_rows_launch(const int32_t* ids, const void* table, void* out, int rows, int vocab, float* stats, void* stream);   // rowwise.cu
+int embed_rows_launch(const int32_t* ids, const void* table, void* out, int rows, int vocab, float* stats, float* squares, void* stream);   // rowwise.cu
 
 constexpr int D = ITTAI_Q3_D, DQ = ITTAI_Q3_DQ, DQKV = ITTAI_Q3_DQKV, DGU = ITTAI_Q3_DGU, FF = ITTAI_Q3_FF, HD = ITTAI_Q3_HD, NKV = ITTAI_Q3_NKV;
 constexpr int NH = DQ / HD;
@@ -33,7 +34,13 @@ static int prefill_launch(const IttaiQwen3Prefill* p, void* st) {
     cudaDeviceGetAttribute(&n_sms, cudaDevAttrMultiProcessorCount, dev);
     // a small forward: both normalised projections run as split-K GEMMs, which normalise their input themselves
     const bool normed = p->split_k && !fold && gemm_split_wins(T, DGU, n_sms) && gemm_split_wins(T, DQKV, n_sms);
-    int rc = embed_rows_launch(p->ids, p->embed, p->h, T, p->vocab, normed ? p->stats : nullptr, st);
+    // shorter still: projections of their own (figures in qwen3_short.cu; at 33 tokens a split-K forward takes 809 us, one of 32 took 749);
+    // the row statistics between them lie in xn, which nothing else uses then
+    const bool brief = p->split_k && fused && T <= kShortTokens;
+    float* squares = brief ? reinterpret_cast<float*>(p->xn) : nullptr;
+    ShortMaps maps;
+    int rc = brief ? short_maps(&maps, p) : ITTAI_OK;
+    if (rc == ITTAI_OK) rc = embed_rows_launch(p->ids, p->embed, p->h, T, p->vocab, normed && !brief ? p->stats : nullptr, squares, st);
     auto gemm = [&](const void* a, const void* w, void* out, int n, int k, int epi, const void* residual, bool norm, bool stats, const IttaiQkRope* rope,
                     const void* gain = nullptr) {
         if (rc != ITTAI_OK) return;
@@ -51,14 +58,16 @@ static int prefill_launch(const IttaiQwen3Prefill* p, void* st) {
         const void *qn = at(p->qn, (size_t)l * HD), *kn = at(p->kn, (size_t)l * HD);
         // layer 0 reads the embedding rows, which no GEMM epilogue produced: its first norm is a pass of its own
         const bool folded = fold && l > 0;
+        IttaiQkRope r = {};
+        r.qn = qn; r.kn = kn; r.rope = p->rope; r.pos = p->pos; r.seq = p->seq; r.slot = p->slot;
+        r.kcache_layer = kc; r.vcache_layer = vc; r.kv_cap = p->kv_cap; r.eps = p->eps;
         const void *g1 = at(p->ln1, (size_t)l * D), *g2 = at(p->ln2, (size_t)l * D);
-        if (!folded && !normed) norm(g1);
+        if (!folded && !normed && !brief) norm(g1);
         const void* x = folded || normed ? p->h : p->xn;
         const void* wq = at(folded ? p->wqkv_f : p->wqkv, (size_t)l * DQKV * D);
-        if (fused) {
-            IttaiQkRope r = {};
-            r.qn = qn; r.kn = kn; r.rope = p->rope; r.pos = p->pos; r.seq = p->seq; r.slot = p->slot;
-            r.kcache_layer = kc; r.vcache_layer = vc; r.kv_cap = p->kv_cap; r.eps = p->eps;
+        if (brief) {
+            rc = short_qkv(maps, p, l, r, g1, squares, (cudaStream_t)st);
+        } else if (fused) {
             gemm(x, wq, p->qkv, DQKV, D, ITTAI_EPI_QKROPE, nullptr, folded || normed, false, &r, normed ? g1 : nullptr);
         } else {
             gemm(x, wq, p->qkv, DQKV, D, ITTAI_EPI_NONE, nullptr, folded || normed, false, nullptr, normed ? g1 : nullptr);
@@ -71,6 +80,12 @@ static int prefill_launch(const IttaiQwen3Prefill* p, void* st) {
         a.seqs = p->seqs; a.n_seqs = p->n_seqs; a.n_heads = NH; a.group = NH / NKV; a.head_dim = HD; a.causal = 1; a.max_q_len = p->max_q_len;
         a.q_rows_total = T; a.kv_rows_total = (int32_t)p->kv_rows_total; a.status = p->status; a.seqs_ready = 1;
         if (rc == ITTAI_OK) rc = ittai_attention_packed_launch(&a, st);
+        if (brief) {
+            if (rc == ITTAI_OK) rc = short_o(maps, p, l, squares, (cudaStream_t)st);
+            if (rc == ITTAI_OK) rc = short_gate_up(maps, p, l, g2, squares, (cudaStream_t)st);
+            if (rc == ITTAI_OK) rc = short_down(maps, p, l, squares, (cudaStream_t)st);
+            continue;
+        }
         gemm(p->attn, at(p->wo, (size_t)l * D * DQ), p->h, D, DQ, ITTAI_EPI_NONE, p->h, false, fold || normed, nullptr);
         if (!fold && !normed) norm(g2);
         gemm(fold || normed ? p->h : p->xn, at(fold ? p->wgu_f : p->wgu, (size_t)l * DGU * D), p->act, DGU, D, ITTAI_EPI_SWIGLU, nullptr, fold || normed, false, nullptr, normed ? g2 : nullptr);

@@ -1,0 +1,380 @@
+// The four projections of a Qwen3 layer for forwards of at most 32 tokens (a search query, a short prompt).
+//
+// At this size a projection is its weights on their way and one chain of latencies.  As split-K GEMMs on tcgen05 (gemm_split_sm100.cu) the chain
+// was 9000 cycles for 23 tokens: activations through TMA, row statistics, a pass that normalises the landed tile in shared memory and
+// fences it for the async proxy, 16 MMAs that read the weights out of shared memory (40 cycles each), a commit, tensor memory back into
+// registers, partials in 4-byte stores.  Here everything between the activations and the output stays with the threads:
+//
+// * A cluster of four CTAs shares K out; a CTA has 128 (QKV: one head), 192 (gate/up) or 32 (O, down) weight rows of its quarter, 32 to 96 KB,
+//   on their way to shared memory ahead of griddepcontrol.wait, and holds them (gate/up: half of them) in registers as MMA operands by then.
+// * The activations of the quarter come by plain loads, whole rows of a warp, are normalised in registers on the way to shared memory with the
+//   rounding steps of rmsnorm_rows_kernel (1 / rms from 32 partial sums of squares, one a lane, that the kernel before left), and meet the
+//   weights in mma.sync m16n8k16: 32 rows x one K chunk x 8 NT tokens a warp.
+// * Chunks meet in shared memory, quarters through st.async, 16 bytes at a time, in the CTA that finishes the token (token n: rank n mod 4,
+//   where a warp or eight lanes hold a whole row piece for the head norm, the rotation or the statistics); sums in the order of chunks, then
+//   of ranks.
+//
+// Measured on a B200, a forward of 3 / 8 / 16 / 23 / 32 tokens, us, split-K GEMMs and attn_fwd_kernel -> this and attn_few_kernel:
+// 640 / 649 / 671 / 682 / 749 -> 365 / 400 / 473 / 534 / 620.  What grows with the tokens are the MMAs (legacy ones: 8 cycles each, 1150
+// of gate/up's 5800 cycles at 23 tokens), the sums' way through shared memory and the activations, which 32 CTAs read from the same lines of
+// L2.  Other forms, us at 3 / 23 / 32 tokens: weights from shared memory as the 128-row operand of tcgen05.mma, everything else alike 455 /
+// 582 / 618; tokens as the 128-row operand in tensor memory 603 / 692 / 744 (padded rows cost what real ones do: 54 cycles an MMA of 128
+// columns); one kernel for all four projections, its sizes arguments 528 / 654 / 697; QKV in 16 warps of 64 registers instead of 8 of 128
+// (their sums meet in four chunks instead of two) 369 / 554 / 666.
+#include <cuda.h>
+
+#include "gemm2_common.cuh"
+#include "qwen3_short.h"
+
+namespace ittai {
+namespace brief {
+
+constexpr int D = ITTAI_Q3_D, HD = ITTAI_Q3_HD, NKV = ITTAI_Q3_NKV, DQ = ITTAI_Q3_DQ, DQKV = ITTAI_Q3_DQKV, DGU = ITTAI_Q3_DGU, FF = ITTAI_Q3_FF;
+constexpr int kRanks = 4;                    // CTAs that share K out
+constexpr int kParts = D / 32;               // partial sums of squares of a row: one per 32-column tile of O and down
+constexpr uint32_t kSpin = 1u << 18;         // polls that park the warp for up to 2 us
+enum { kQkv = 0, kGateUp = 1, kResidual = 2 };
+
+template <int EPI, int K>
+struct Shape {
+    static constexpr int kSlice = K / kRanks;                                       // columns of a CTA
+    static constexpr int kRows = EPI == kQkv ? 128 : EPI == kGateUp ? 192 : 32;      // weight rows of a CTA
+    static constexpr int kChunk = EPI == kResidual ? 64 : 128;                         // columns of a warp
+    static constexpr int kChunks = kSlice / kChunk, kGroups = kRows / 32;            // warps: a chunk x 32 rows each
+    static constexpr int kWarps = kChunks * kGroups, kThreads = 32 * kWarps;
+    static constexpr int kSteps = kChunk / 16;                                       // MMAs along K
+    static constexpr int kHeld = EPI == kQkv ? 8 : 4;                                // of which as many have their weights in registers ahead of the wait
+    static constexpr int kXLd = kSlice * 2 + 16;                                     // bytes per token in shared memory: eight rows on different banks
+    static constexpr int kPartLd = kRows + 4;                                        // floats per token of a chunk's sums, likewise
+    static constexpr int kPieces = kSlice / 256;                                     // 16-byte pieces of a token row per lane
+    static_assert(kSlice % 256 == 0 && kSteps >= kHeld, "whole warps per token");
+    static_assert(EPI != kQkv || kWarps >= 8, "a warp for every token that a CTA finishes");
+};
+template <int NT, int EPI, int K>
+struct Plan {
+    using S = Shape<EPI, K>;
+    static constexpr uint32_t kW = S::kRows * S::kSlice * 2, kPart = S::kChunks * 8 * NT * S::kPartLd * 4;
+    static constexpr uint32_t kX = kW > kPart ? kW : kPart;                          // offset: the sums of the chunks take the place of the weights
+    static constexpr uint32_t kRecv = (kX + 8 * NT * S::kXLd + 127) / 128 * 128;     // offset: [ranks][2 NT tokens][rows] sums of the quarters
+    static constexpr uint32_t kSmem = kRecv + kRanks * 2 * NT * S::kRows * 4 + 1024;
+};
+
+struct Args {
+    const bf16* x;           // [T][K]
+    const bf16* gain;        // [D] norm in front of the projection (QKV, gate/up)
+    const float* stats_in;   // [T][kParts] sums of squares of x's rows (QKV, gate/up)
+    bf16* out;               // QKV: [T][DQKV], q heads; gate/up: [T][FF]; O, down: [T][D]
+    const bf16* res;         // O, down: [T][D]
+    float* stats_out;        // O, down: [T][kParts]
+    int tokens, w_row;       // first weight row of this layer in the map
+    float eps;
+    uint32_t* status;
+    IttaiQkRope rope;
+};
+
+__device__ __forceinline__ void ldsm4(uint32_t (&r)[4], uint32_t addr) {
+    asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0,%1,%2,%3}, [%4];" : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(addr) : "memory");
+}
+__device__ __forceinline__ void ldsm2(uint32_t& r0, uint32_t& r1, uint32_t addr) {
+    asm volatile("ldmatrix.sync.aligned.m8n8.x2.shared.b16 {%0,%1}, [%2];" : "=r"(r0), "=r"(r1) : "r"(addr) : "memory");
+}
+__device__ __forceinline__ void mma16816(float (&d)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1) {
+    asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, {%0, %1, %2, %3};"
+                 : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3]) : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
+}
+__device__ __forceinline__ float4 lds_f4(uint32_t addr) {
+    float4 v;
+    asm volatile("ld.shared.v4.f32 {%0,%1,%2,%3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "r"(addr) : "memory");
+    return v;
+}
+__device__ __forceinline__ void st_async_f32x4(uint32_t dst, float4 v, uint32_t bar) {
+    asm volatile("st.async.weak.shared::cluster.mbarrier::complete_tx::bytes.v4.f32 [%0], {%1, %2, %3, %4}, [%5];"
+                 ::"r"(dst), "f"(v.x), "f"(v.y), "f"(v.z), "f"(v.w), "r"(bar) : "memory");
+}
+__device__ __forceinline__ uint32_t map_addr(uint32_t addr, int rank) {
+    uint32_t a;
+    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(a) : "r"(addr), "r"(rank));
+    return a;
+}
+__device__ __forceinline__ float4 add4(float4 a, float4 b) { return make_float4(a.x + b.x, a.y + b.y, a.z + b.z, a.w + b.w); }
+
+template <int NT, int EPI, int K>
+__global__ void __launch_bounds__(Shape<EPI, K>::kThreads, 2) proj_kernel(const __grid_constant__ CUtensorMap tm_w, const Args a) {
+    using S = Shape<EPI, K>;
+    using P = Plan<NT, EPI, K>;
+    extern __shared__ __align__(1024) unsigned char smem_raw[];
+    unsigned char* sm = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
+    __shared__ unsigned long long landed, arrived;
+    const int warp = warp_index(), lane = threadIdx.x & 31;
+    const int rank = blockIdx.x % kRanks, tile = blockIdx.x / kRanks;
+    const int own = (a.tokens - rank + kRanks - 1) / kRanks;         // tokens that this CTA finishes (0 where there are fewer than ranks)
+    if (threadIdx.x == 0) {
+        mbar_init(&landed, 1);
+        mbar_init(&arrived, 1);
+        fence_mbar_init();
+        mbar_expect_tx(&landed, P::kW);
+        mbar_expect_tx(&arrived, (uint32_t)(own > 0 ? own : 0) * S::kRows * 4 * kRanks);
+#pragma unroll 1
+        for (int j = 0; j < S::kSlice / 64; ++j)
+            tma_load_2d(sm + j * S::kRows * 128, &tm_w, rank * S::kSlice + 64 * j, a.w_row + tile * S::kRows, &landed);
+    }
+    __syncthreads();
+    // another CTA's shared memory may be written only once that CTA runs; waited for ahead of the first write
+    asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
+    pdl_trigger();
+
+    const int chunk = warp / S::kGroups, group = warp % S::kGroups;
+    const uint32_t w0 = smem_u32(sm), x0 = w0 + P::kX;
+    // row of this lane in the ldmatrix of a 16 x 16 tile of weights: rows 0-7, 8-15, then the same with the upper eight columns
+    const int wrow = 32 * group + (lane & 15), whalf = lane >> 4;
+    auto load_w = [&](uint32_t (&f)[4], int mt, int ks) {
+        const int c = chunk * S::kChunk + 16 * ks;                    // column of the slice
+        const int row = wrow + 16 * mt;
+        ldsm4(f, w0 + (uint32_t)(c >> 6) * (S::kRows * 128) + (uint32_t)row * 128 + (uint32_t)((((c & 63) >> 3) + whalf) ^ (row & 7)) * 16);
+    };
+    uint4 gain = make_uint4(0u, 0u, 0u, 0u);
+    if constexpr (EPI != kResidual) gain = *reinterpret_cast<const uint4*>(a.gain + rank * S::kSlice + 8 * lane);
+    bool ok = mbar_wait_bounded(&landed, 0, kSpin);
+    __syncwarp();                                                     // the lanes left the wait one by one
+    uint32_t wf[S::kHeld][2][4];
+#pragma unroll
+    for (int ks = 0; ks < S::kHeld; ++ks) { load_w(wf[ks][0], 0, ks); load_w(wf[ks][1], 1, ks); }
+    if constexpr (EPI != kResidual) asm volatile("" : "+r"(gain.x), "+r"(gain.y), "+r"(gain.z), "+r"(gain.w));    // arrived: a load left open may be scheduled behind the wait
+    pdl_wait();
+
+    // ---- activations: a warp takes whole token rows of the slice
+    constexpr int kRounds = (8 * NT + S::kWarps - 1) / S::kWarps;
+    uint4 xv[kRounds][S::kPieces];
+    float ss[kRounds];
+#pragma unroll
+    for (int i = 0; i < kRounds; ++i) {
+        const int n = warp + i * S::kWarps;
+        ss[i] = 0.f;
+#pragma unroll
+        for (int p = 0; p < S::kPieces; ++p) xv[i][p] = make_uint4(0u, 0u, 0u, 0u);
+        if (n < a.tokens) {
+#pragma unroll
+            for (int p = 0; p < S::kPieces; ++p) xv[i][p] = ldcg128(a.x + (size_t)n * K + rank * S::kSlice + 256 * p + 8 * lane);
+            if constexpr (EPI != kResidual) ss[i] = ldcgf(a.stats_in + n * kParts + lane);
+        }
+    }
+    // what the epilogue reads, ahead of the main loop.  O, down: eight lanes a token, four columns each; QKV: a warp a token
+    const int quad = threadIdx.x & 7, slot8 = threadIdx.x >> 3;
+    uint2 res = make_uint2(0u, 0u), cosr = res, sinr = res, hgain = res;
+    bf16* dst = nullptr;
+    if constexpr (EPI == kResidual) {
+        if (slot8 < own) res = *reinterpret_cast<const uint2*>(a.res + (size_t)(kRanks * slot8 + rank) * D + tile * 32 + 4 * quad);
+    }
+    int pos = 0, seq = 0, row = 0;
+    const int n_own = kRanks * warp + rank;                           // QKV: the token of this warp
+    if constexpr (EPI == kQkv) {
+        if (warp < own) {
+            pos = a.rope.pos[n_own];
+            if (tile >= 16) { seq = a.rope.seq[n_own]; row = a.rope.slot[n_own]; }
+            if (tile < 24) hgain = *reinterpret_cast<const uint2*>(reinterpret_cast<const bf16*>(tile < 16 ? a.rope.qn : a.rope.kn) + 4 * lane);
+        }
+    }
+#pragma unroll
+    for (int i = 0; i < kRounds; ++i) {
+        const int n = warp + i * S::kWarps;
+        if (n < 8 * NT) {
+            if constexpr (EPI != kResidual) {
+                const float rstd = rsqrt_full(warp_sum(ss[i]) * (1.0f / D) + a.eps);
+                uint32_t* u = reinterpret_cast<uint32_t*>(&xv[i][0]);
+                const uint32_t gw[4] = {gain.x, gain.y, gain.z, gain.w};
+#pragma unroll
+                for (int j = 0; j < 4; ++j) u[j] = mul_bf16x2(pack_bf16x2(bf_lo(u[j]) * rstd, bf_hi(u[j]) * rstd), gw[j]);
+            }
+#pragma unroll
+            for (int p = 0; p < S::kPieces; ++p) *reinterpret_cast<uint4*>(sm + P::kX + n * S::kXLd + 512 * p + 16 * lane) = xv[i][p];
+        }
+    }
+    if constexpr (EPI == kQkv) {
+        if (warp < own) {
+            if (tile < 24) {
+                const bf16* rp = reinterpret_cast<const bf16*>(a.rope.rope) + (size_t)pos * HD + 4 * (lane & 15);
+                cosr = *reinterpret_cast<const uint2*>(rp); sinr = *reinterpret_cast<const uint2*>(rp + HD / 2);
+            }
+            dst = tile < 16 ? a.out + (size_t)n_own * DQKV + tile * HD + 4 * lane
+                            : reinterpret_cast<bf16*>(tile < 24 ? a.rope.kcache_layer : a.rope.vcache_layer) + (((size_t)seq * NKV + (tile & 7)) * a.rope.kv_cap + row) * HD + 4 * lane;
+        }
+    }
+    __syncthreads();
+
+    // ---- 32 rows x chunk x 8 NT tokens
+    float acc[2][NT][4];
+#pragma unroll
+    for (int m = 0; m < 2; ++m)
+#pragma unroll
+        for (int n = 0; n < NT; ++n) acc[m][n][0] = acc[m][n][1] = acc[m][n][2] = acc[m][n][3] = 0.f;
+    const uint32_t xl = x0 + (uint32_t)((lane & 7) + 8 * (lane >> 4)) * S::kXLd + chunk * S::kChunk * 2 + 16 * ((lane >> 3) & 1);
+#pragma unroll
+    for (int ks = 0; ks < S::kSteps; ++ks) {
+        uint32_t b[NT][2];
+#pragma unroll
+        for (int n = 0; n + 1 < NT; n += 2) {
+            uint32_t f[4];
+            ldsm4(f, xl + 8 * n * S::kXLd + 32 * ks);
+            b[n][0] = f[0]; b[n][1] = f[1]; b[n + 1][0] = f[2]; b[n + 1][1] = f[3];
+        }
+        if constexpr (NT & 1) ldsm2(b[NT - 1][0], b[NT - 1][1], x0 + (uint32_t)((lane & 7) + 8 * (NT - 1)) * S::kXLd + chunk * S::kChunk * 2 + 16 * ((lane >> 3) & 1) + 32 * ks);
+        if (ks >= S::kHeld) { load_w(wf[ks % S::kHeld][0], 0, ks); load_w(wf[ks % S::kHeld][1], 1, ks); }
+#pragma unroll
+        for (int n = 0; n < NT; ++n) {
+            mma16816(acc[0][n], wf[ks % S::kHeld][0], b[n][0], b[n][1]);
+            mma16816(acc[1][n], wf[ks % S::kHeld][1], b[n][0], b[n][1]);
+        }
+    }
+    if constexpr (S::kSteps > S::kHeld) __syncthreads();              // the weights in shared memory have been read by all
+    float* part = reinterpret_cast<float*>(sm) + (size_t)chunk * 8 * NT * S::kPartLd;
+    const int g = lane >> 2, t = lane & 3;
+#pragma unroll
+    for (int m = 0; m < 2; ++m)
+#pragma unroll
+        for (int n = 0; n < NT; ++n)
+#pragma unroll
+            for (int i = 0; i < 4; ++i) part[(8 * n + 2 * t + (i & 1)) * S::kPartLd + 32 * group + 16 * m + g + 8 * (i >> 1)] = acc[m][n][i];
+    __syncthreads();
+
+    // ---- sums of the chunks, four rows of a token at a time, to the rank that finishes the token
+    asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+    constexpr int kQuads = S::kRows / 4;
+    const uint32_t recv = w0 + P::kRecv;
+#pragma unroll 1
+    for (int i = threadIdx.x; i < a.tokens * kQuads; i += S::kThreads) {
+        const int n = i / kQuads, q = i % kQuads;
+        float4 v = lds_f4(w0 + (uint32_t)(n * S::kPartLd + 4 * q) * 4);
+#pragma unroll
+        for (int c = 1; c < S::kChunks; ++c) v = add4(v, lds_f4(w0 + (uint32_t)((c * 8 * NT + n) * S::kPartLd + 4 * q) * 4));
+        const int to = n % kRanks;
+        st_async_f32x4(map_addr(recv + (uint32_t)((rank * 2 * NT + n / kRanks) * S::kRows + 4 * q) * 4, to), v, map_addr(smem_u32(&arrived), to));
+    }
+    bool came = true;
+    {
+        uint32_t spins = 0;
+        while (!mbar_try_wait_cluster(&arrived, 0)) { if (++spins >= (kSpin << 4)) { came = false; break; } }
+    }
+    __syncwarp();
+    auto total = [&](int slot, int q) {                              // sums of the ranks, in their order
+        float4 v = lds_f4(recv + (uint32_t)(slot * S::kRows + 4 * q) * 4);
+#pragma unroll
+        for (int r = 1; r < kRanks; ++r) v = add4(v, lds_f4(recv + (uint32_t)((r * 2 * NT + slot) * S::kRows + 4 * q) * 4));
+        return v;
+    };
+    if constexpr (EPI == kQkv) {
+        if (warp < own) {
+            const float4 v = total(warp, lane);
+            uint32_t y0 = pack_bf16x2(v.x, v.y), y1 = pack_bf16x2(v.z, v.w);
+            if (tile < 24) {
+                // the rounding steps of qk_rope_scatter_kernel on packed pairs; the partner element 64 columns away is 16 lanes away
+                const float f0 = bf_lo(y0), f1 = bf_hi(y0), f2 = bf_lo(y1), f3 = bf_hi(y1);
+                const float rstd = rsqrt_full(warp_sum(fmaf(f0, f0, fmaf(f1, f1, fmaf(f2, f2, f3 * f3)))) * (1.0f / HD) + a.rope.eps);
+                const uint32_t n0 = mul_bf16x2(pack_bf16x2(f0 * rstd, f1 * rstd), hgain.x), n1 = mul_bf16x2(pack_bf16x2(f2 * rstd, f3 * rstd), hgain.y);
+                const uint32_t neg = lane < 16 ? 0x80008000u : 0u;
+                const uint32_t o0 = __shfl_xor_sync(0xffffffffu, n0, 16) ^ neg, o1 = __shfl_xor_sync(0xffffffffu, n1, 16) ^ neg;
+                y0 = add_bf16x2(mul_bf16x2(n0, cosr.x), mul_bf16x2(o0, sinr.x));
+                y1 = add_bf16x2(mul_bf16x2(n1, cosr.y), mul_bf16x2(o1, sinr.y));
+            }
+            *reinterpret_cast<uint2*>(dst) = make_uint2(y0, y1);
+        }
+    } else if constexpr (EPI == kGateUp) {
+#pragma unroll 1
+        for (int i = threadIdx.x; i < own * kQuads; i += S::kThreads) {
+            const int slot = i / kQuads, q = i % kQuads;
+            const float4 v = total(slot, q);
+            // adjacent rows are (gate, up): act = bf16(bf16(silu(bf16 gate)) * bf16 up)
+            const float g0 = bf16r(v.x), u0 = bf16r(v.y), g1 = bf16r(v.z), u1 = bf16r(v.w);
+            *reinterpret_cast<uint32_t*>(a.out + (size_t)(kRanks * slot + rank) * FF + tile * (S::kRows / 2) + 2 * q) =
+                pack_bf16x2(bf16r(g0 / (1.0f + expf(-g0))) * u0, bf16r(g1 / (1.0f + expf(-g1))) * u1);
+        }
+    } else {
+        if (warp < (own + 3) / 4) {                                   // whole warps: four tokens each
+            const float4 v = total(slot8 < own ? slot8 : 0, quad);
+            const uint2 o = make_uint2(pack_bf16x2(bf_lo(res.x) + bf16r(v.x), bf_hi(res.x) + bf16r(v.y)), pack_bf16x2(bf_lo(res.y) + bf16r(v.z), bf_hi(res.y) + bf16r(v.w)));
+            const float a0 = bf_lo(o.x), a1 = bf_hi(o.x), a2 = bf_lo(o.y), a3 = bf_hi(o.y);
+            float s = fmaf(a0, a0, fmaf(a1, a1, fmaf(a2, a2, a3 * a3)));
+#pragma unroll
+            for (int m = 1; m < 8; m <<= 1) s += __shfl_xor_sync(0xffffffffu, s, m);
+            if (slot8 < own) {
+                const int n = kRanks * slot8 + rank;
+                *reinterpret_cast<uint2*>(a.out + (size_t)n * D + tile * 32 + 4 * quad) = o;
+                if (quad == 0) a.stats_out[n * kParts + tile] = s;
+            }
+        }
+    }
+    if (!__syncthreads_and(ok && came)) {
+        // A CTA that gave up must not leave before what is owed to it has come: all send, also where their waits ran out.  Should a send take
+        // longer than this wait, the barrier holds the CTA until the others have left (threads that have exited count as arrived).
+        bool all = false;
+        for (uint32_t spins = 0; !all && spins < (kSpin << 4); ++spins) all = mbar_try_wait_cluster(&arrived, 0);
+        if (!__syncthreads_and(all)) {
+            asm volatile("barrier.cluster.arrive.release;" ::: "memory");
+            asm volatile("barrier.cluster.wait.acquire;" ::: "memory");
+        }
+        if (threadIdx.x == 0) {
+            if (atomicCAS(&a.status[0], 0u, (uint32_t)ITTAI_ST_GEMM_TIMEOUT) == 0u) { a.status[1] = blockIdx.x; a.status[2] = (uint32_t)K; }
+            const long long t0 = clock64();                           // copies still in flight land before the shared memory is handed back
+            while (clock64() - t0 < 2000000) {}
+        }
+        __syncthreads();
+    }
+}
+
+template <int NT, int EPI, int K>
+static cudaError_t launch(const CUtensorMap& tm, const Args& a, int n_rows, cudaStream_t st) {
+    using S = Shape<EPI, K>;
+    constexpr uint32_t kSmem = Plan<NT, EPI, K>::kSmem;
+    static thread_local int attr_dev = -1;
+    int dev = 0;
+    cudaGetDevice(&dev);
+    if (attr_dev != dev) {
+        const cudaError_t e = cudaFuncSetAttribute(proj_kernel<NT, EPI, K>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmem);
+        if (e != cudaSuccess) return e;
+        attr_dev = dev;
+    }
+    return launch_pdl(proj_kernel<NT, EPI, K>, dim3(kRanks * (n_rows / S::kRows)), dim3(S::kThreads), kSmem, st, kRanks, tm, a);
+}
+template <int EPI, int K>
+static cudaError_t launch_any(const CUtensorMap& tm, const Args& a, int n_rows, cudaStream_t st) {
+    switch ((a.tokens + 7) / 8) {
+        case 1: return launch<1, EPI, K>(tm, a, n_rows, st);
+        case 2: return launch<2, EPI, K>(tm, a, n_rows, st);
+        case 3: return launch<3, EPI, K>(tm, a, n_rows, st);
+        default: return launch<4, EPI, K>(tm, a, n_rows, st);
+    }
+}
+
+}  // namespace brief
+
+int cuda_fail(cudaError_t e, const char* what);
+
+int short_maps(ShortMaps* m, const IttaiQwen3Prefill* p) {
+    using namespace brief;
+    const long long L = p->n_layers;
+    int rc = make_tmap_bf16(&m->qkv, p->wqkv, L * DQKV, D, D, Shape<kQkv, D>::kRows);
+    if (rc == ITTAI_OK) rc = make_tmap_bf16(&m->o, p->wo, L * D, DQ, DQ, Shape<kResidual, DQ>::kRows);
+    if (rc == ITTAI_OK) rc = make_tmap_bf16(&m->gu, p->wgu, L * DGU, D, D, Shape<kGateUp, D>::kRows);
+    if (rc == ITTAI_OK) rc = make_tmap_bf16(&m->down, p->wd, L * D, FF, FF, Shape<kResidual, FF>::kRows);
+    return rc;
+}
+
+static int done(cudaError_t e) { return e == cudaSuccess ? ITTAI_OK : cuda_fail(e, "launch proj_kernel"); }
+
+int short_qkv(const ShortMaps& m, const IttaiQwen3Prefill* p, int layer, const IttaiQkRope& r, const void* gain, const float* stats, cudaStream_t st) {
+    brief::Args a{(const bf16*)p->h, (const bf16*)gain, stats, (bf16*)p->qkv, nullptr, nullptr, p->tokens, layer * brief::DQKV, p->eps, p->status, r};
+    return done(brief::launch_any<brief::kQkv, brief::D>(m.qkv, a, brief::DQKV, st));
+}
+int short_gate_up(const ShortMaps& m, const IttaiQwen3Prefill* p, int layer, const void* gain, const float* stats, cudaStream_t st) {
+    brief::Args a{(const bf16*)p->h, (const bf16*)gain, stats, (bf16*)p->act, nullptr, nullptr, p->tokens, layer * brief::DGU, p->eps, p->status, {}};
+    return done(brief::launch_any<brief::kGateUp, brief::D>(m.gu, a, brief::DGU, st));
+}
+int short_o(const ShortMaps& m, const IttaiQwen3Prefill* p, int layer, float* stats, cudaStream_t st) {
+    brief::Args a{(const bf16*)p->attn, nullptr, nullptr, (bf16*)p->h, (const bf16*)p->h, stats, p->tokens, layer * brief::D, p->eps, p->status, {}};
+    return done(brief::launch_any<brief::kResidual, brief::DQ>(m.o, a, brief::D, st));
+}
+int short_down(const ShortMaps& m, const IttaiQwen3Prefill* p, int layer, float* stats, cudaStream_t st) {
+    brief::Args a{(const bf16*)p->act, nullptr, nullptr, (bf16*)p->h, (const bf16*)p->h, stats, p->tokens, layer * brief::D, p->eps, p->status, {}};
+    return done(brief::launch_any<brief::kResidual, brief::FF>(m.down, a, brief::D, st));
+}
+
+}  // namespace ittai

@@ -286,9 +286,10 @@ __global__ void __launch_bounds__(kRowThreads) positions_kernel(const float* __r
 }
 
 // Embedding rows: out[t] = table[ids[t]], width 1024 (reference src/ittai/qwen3/base.py:147-162).  `stats` or null: [rows][8][2]
-// (sum, sum of squares) of every 128-column slice, as a GEMM's stats_out leaves them (16 lanes hold a slice).
+// (sum, sum of squares) of every 128-column slice, as a GEMM's stats_out leaves them (16 lanes hold a slice).  `squares` or null: [rows][32]
+// sums of squares of every 32-column slice, as the projections of short forwards leave them (4 lanes).
 __global__ void __launch_bounds__(kRowThreads) embed_rows_kernel(const int* __restrict__ ids, const bf16* __restrict__ table,
-                                                                   bf16* __restrict__ out, int rows, int vocab, float* __restrict__ stats) {
+                                                                   bf16* __restrict__ out, int rows, int vocab, float* __restrict__ stats, float* __restrict__ squares) {
     pdl_trigger();
     pdl_wait();
     const int row = blockIdx.x * (kRowThreads / 32) + (threadIdx.x >> 5), lane = threadIdx.x & 31;
@@ -299,8 +300,15 @@ __global__ void __launch_bounds__(kRowThreads) embed_rows_kernel(const int* __re
     for (int i = 0; i < 4; ++i) {
         const uint4 v = *reinterpret_cast<const uint4*>(table + (size_t)id * 1024 + (lane + 32 * i) * 8);
         *reinterpret_cast<uint4*>(out + (size_t)row * 1024 + (lane + 32 * i) * 8) = v;
+        const uint32_t w[4] = {v.x, v.y, v.z, v.w};
+        if (squares != nullptr) {
+            float s2 = 0.f;
+#pragma unroll
+            for (int j = 0; j < 4; ++j) s2 = fmaf(bf_lo(w[j]), bf_lo(w[j]), fmaf(bf_hi(w[j]), bf_hi(w[j]), s2));
+            s2 += __shfl_xor_sync(0xffffffffu, s2, 1); s2 += __shfl_xor_sync(0xffffffffu, s2, 2);
+            if ((lane & 3) == 0) squares[(size_t)row * 32 + 8 * i + (lane >> 2)] = s2;
+        }
         if (stats != nullptr) {
-            const uint32_t w[4] = {v.x, v.y, v.z, v.w};
             float s1 = 0.f, s2 = 0.f;
 #pragma unroll
             for (int j = 0; j < 4; ++j) { const float lo = bf_lo(w[j]), hi = bf_hi(w[j]); s1 += lo + hi; s2 = fmaf(lo, lo, fmaf(hi, hi, s2)); }
@@ -414,15 +422,15 @@ extern "C" int ittai_siglip_positions(const float* grid, int side, int width, co
 }
 
 namespace ittai {
-int embed_rows_launch(const int32_t* ids, const void* table, void* out, int rows, int vocab, float* stats, void* stream) {
+int embed_rows_launch(const int32_t* ids, const void* table, void* out, int rows, int vocab, float* stats, float* squares, void* stream) {
     if (!ids || !table || !out || rows < 1 || vocab < 1) { set_error("embed_rows: bad argument"); return ITTAI_E_ARG; }
-    launch_pdl(embed_rows_kernel, dim3(row_grid(rows)), dim3(kRowThreads), 0, (cudaStream_t)stream, 1, ids, (const bf16*)table, (bf16*)out, rows, vocab, stats);
+    launch_pdl(embed_rows_kernel, dim3(row_grid(rows)), dim3(kRowThreads), 0, (cudaStream_t)stream, 1, ids, (const bf16*)table, (bf16*)out, rows, vocab, stats, squares);
     return launched("embed_rows_kernel");
 }
 }  // namespace ittai
 
 extern "C" int ittai_embed_rows(const int32_t* ids, const void* table, void* out, int rows, int vocab, void* stream) {
-    return embed_rows_launch(ids, table, out, rows, vocab, nullptr, stream);
+    return embed_rows_launch(ids, table, out, rows, vocab, nullptr, nullptr, stream);
 }
 
 extern "C" int ittai_qwen3_final_pool(const void* h, const int32_t* rows, const void* gain, float* out, int n_seq, float eps, void* stream) {

@@ -66,7 +66,8 @@ def _block(text, start):
             return text[i:j + 1]
 
 
-@pytest.mark.parametrize("source,failure", [("gemm_split_sm100.cu", "if (*abort_flag) {"), ("qwen3_chain.cu", "if (failed) {")])
+@pytest.mark.parametrize("source,failure", [("gemm_split_sm100.cu", "if (*abort_flag) {"), ("qwen3_chain.cu", "if (failed) {"),
+                                            ("qwen3_short.cu", "if (!__syncthreads_and(ok && came)) {")])
 def test_the_kernels_follow_the_model(source, failure):
     """In the branch of a CTA that gave up: the wait for the bytes, the barrier behind it, and then the time for copies in flight."""
     with open(os.path.join(CSRC, source)) as f:

@@ -63,10 +63,33 @@ def test_more_shapes_than_graphs(tiny_hf):
 
 
 @gpu
+@pytest.mark.parametrize("lens", [[2], [7], [8], [9], [15, 1], [17], [24], [25], [31], [32], [33], [5, 9, 1, 17], [1] * 32])
+def test_short_forwards_match_the_split_gemms(tiny_hf, lens):
+    """Forwards of up to 32 tokens (their own projections and attention, tiles of 8 tokens, a token per rank of four) against the kernels of
+    longer ones with the same rounding points (``fused_rope=False``): embeddings and the last layer's keys and values.  Bound: a bf16
+    rounding is off by 1.1e-3 (rms), a layer has about eight in a row, so that two forwards of two layers whose roundings all fell
+    differently would be sqrt(2 * 16) * 1.1e-3 = 6.2e-3 apart; half as much again for few tokens."""
+    from ittai_b200.qwen3 import Engine
+    model, dims = tiny_hf
+    ids = [hf.prompt_ids(n, seed=90 + n + i, vocab=dims.vocab).tolist() for i, n in enumerate(lens)]
+    T, outs = sum(lens), []
+    for fused in (True, False):
+        eng = Engine(model.state_dict(), 128, 32, fused_rope=fused)
+        eng.kbuf.fill_(float("nan"))                      # rows behind the last token are not to be read
+        eng.vbuf.fill_(float("nan"))
+        out = eng.forward(ids).clone()
+        eng.check()
+        assert torch.equal(eng.forward(ids), out)
+        outs.append((out, eng.kbuf[0, :, :T].float(), eng.vbuf[0, :, :T].float()))
+        assert eng.kbuf[0, :, T:].isnan().all() and eng.vbuf[0, :, T:].isnan().all()
+    for a, b in zip(*outs):
+        assert torch.linalg.vector_norm(a - b) <= 9.3e-3 * torch.linalg.vector_norm(b), lens
+
+
+@gpu
 def test_a_short_prompt_behind_a_cached_one(tiny_hf):
     """The attention of few queries with cached keys in front of them, several steps of 32: a prompt appended in two pieces against the prompt
-    at once (keys and values of two layers; a
-    bf16 rounding is off by 1.1e-3 rms, eight in a row a layer: sqrt(2 * 16) * 1.1e-3 = 6.2e-3, half as much again for few tokens)."""
+    at once (keys and values of two layers: the bound above)."""
     from ittai_b200.qwen3 import Qwen3Decoder
     model, dims = tiny_hf
     ids = hf.prompt_ids(150, seed=4, vocab=dims.vocab)
