@@ -15,7 +15,7 @@
 //   of ranks.
 //
 // Measured on a B200, a forward of 3 / 8 / 16 / 23 / 32 tokens, us, split-K GEMMs and attn_fwd_kernel -> this and attn_few_kernel:
-// 640 / 649 / 671 / 682 / 749 -> 365 / 400 / 473 / 534 / 620.  What grows with the tokens are the MMAs (legacy ones: 8 cycles each, 1150
+// 640 / 649 / 671 / 682 / 749 -> 351 / 372 / 461 / 536 / 617.  What grows with the tokens are the MMAs (legacy ones: 8 cycles each, 1150
 // of gate/up's 5800 cycles at 23 tokens), the sums' way through shared memory and the activations, which 32 CTAs read from the same lines of
 // L2.  Other forms, us at 3 / 23 / 32 tokens: weights from shared memory as the 128-row operand of tcgen05.mma, everything else alike 455 /
 // 582 / 618; tokens as the 128-row operand in tensor memory 603 / 692 / 744 (padded rows cost what real ones do: 54 cycles an MMA of 128
@@ -134,11 +134,21 @@ __global__ void __launch_bounds__(Shape<EPI, K>::kThreads, 2) proj_kernel(const 
     };
     uint4 gain = make_uint4(0u, 0u, 0u, 0u);
     if constexpr (EPI != kResidual) gain = *reinterpret_cast<const uint4*>(a.gain + rank * S::kSlice + 8 * lane);
+    // The rotary arguments lie in a line of the kernel's parameters that nothing ahead of the wait has read: fetched behind it, they cost 500
+    // cycles: forwards of 3 / 8 / 23 / 32 tokens 365 / 390 / 534 / 621 -> 351 / 372 / 537 / 617 us.  The head norm's gain comes from HBM like the other one.
+    IttaiQkRope rope;
+    uint2 hgain = make_uint2(0u, 0u);
+    if constexpr (EPI == kQkv) {
+        rope = a.rope;
+        asm volatile("" : "+l"(rope.pos), "+l"(rope.seq), "+l"(rope.slot), "+l"(rope.rope));
+        if (tile < 24) hgain = *reinterpret_cast<const uint2*>(reinterpret_cast<const bf16*>(tile < 16 ? rope.qn : rope.kn) + 4 * lane);
+    }
     bool ok = mbar_wait_bounded(&landed, 0, kSpin);
     __syncwarp();                                                     // the lanes left the wait one by one
     uint32_t wf[S::kHeld][2][4];
 #pragma unroll
     for (int ks = 0; ks < S::kHeld; ++ks) { load_w(wf[ks][0], 0, ks); load_w(wf[ks][1], 1, ks); }
+    if constexpr (EPI == kQkv) asm volatile("" : "+r"(hgain.x), "+r"(hgain.y));
     if constexpr (EPI != kResidual) asm volatile("" : "+r"(gain.x), "+r"(gain.y), "+r"(gain.z), "+r"(gain.w));    // arrived: a load left open may be scheduled behind the wait
     pdl_wait();
 
@@ -160,7 +170,7 @@ __global__ void __launch_bounds__(Shape<EPI, K>::kThreads, 2) proj_kernel(const 
     }
     // what the epilogue reads, ahead of the main loop.  O, down: eight lanes a token, four columns each; QKV: a warp a token
     const int quad = threadIdx.x & 7, slot8 = threadIdx.x >> 3;
-    uint2 res = make_uint2(0u, 0u), cosr = res, sinr = res, hgain = res;
+    uint2 res = make_uint2(0u, 0u), cosr = res, sinr = res;
     bf16* dst = nullptr;
     if constexpr (EPI == kResidual) {
         if (slot8 < own) res = *reinterpret_cast<const uint2*>(a.res + (size_t)(kRanks * slot8 + rank) * D + tile * 32 + 4 * quad);
@@ -169,9 +179,8 @@ __global__ void __launch_bounds__(Shape<EPI, K>::kThreads, 2) proj_kernel(const 
     const int n_own = kRanks * warp + rank;                           // QKV: the token of this warp
     if constexpr (EPI == kQkv) {
         if (warp < own) {
-            pos = a.rope.pos[n_own];
-            if (tile >= 16) { seq = a.rope.seq[n_own]; row = a.rope.slot[n_own]; }
-            if (tile < 24) hgain = *reinterpret_cast<const uint2*>(reinterpret_cast<const bf16*>(tile < 16 ? a.rope.qn : a.rope.kn) + 4 * lane);
+            pos = rope.pos[n_own];
+            if (tile >= 16) { seq = rope.seq[n_own]; row = rope.slot[n_own]; }
         }
     }
 #pragma unroll
@@ -192,11 +201,11 @@ __global__ void __launch_bounds__(Shape<EPI, K>::kThreads, 2) proj_kernel(const 
     if constexpr (EPI == kQkv) {
         if (warp < own) {
             if (tile < 24) {
-                const bf16* rp = reinterpret_cast<const bf16*>(a.rope.rope) + (size_t)pos * HD + 4 * (lane & 15);
+                const bf16* rp = reinterpret_cast<const bf16*>(rope.rope) + (size_t)pos * HD + 4 * (lane & 15);
                 cosr = *reinterpret_cast<const uint2*>(rp); sinr = *reinterpret_cast<const uint2*>(rp + HD / 2);
             }
             dst = tile < 16 ? a.out + (size_t)n_own * DQKV + tile * HD + 4 * lane
-                            : reinterpret_cast<bf16*>(tile < 24 ? a.rope.kcache_layer : a.rope.vcache_layer) + (((size_t)seq * NKV + (tile & 7)) * a.rope.kv_cap + row) * HD + 4 * lane;
+                            : reinterpret_cast<bf16*>(tile < 24 ? rope.kcache_layer : rope.vcache_layer) + (((size_t)seq * NKV + (tile & 7)) * rope.kv_cap + row) * HD + 4 * lane;
         }
     }
     __syncthreads();
@@ -268,7 +277,7 @@ __global__ void __launch_bounds__(Shape<EPI, K>::kThreads, 2) proj_kernel(const 
             if (tile < 24) {
                 // the rounding steps of qk_rope_scatter_kernel on packed pairs; the partner element 64 columns away is 16 lanes away
                 const float f0 = bf_lo(y0), f1 = bf_hi(y0), f2 = bf_lo(y1), f3 = bf_hi(y1);
-                const float rstd = rsqrt_full(warp_sum(fmaf(f0, f0, fmaf(f1, f1, fmaf(f2, f2, f3 * f3)))) * (1.0f / HD) + a.rope.eps);
+                const float rstd = rsqrt_full(warp_sum(fmaf(f0, f0, fmaf(f1, f1, fmaf(f2, f2, f3 * f3)))) * (1.0f / HD) + rope.eps);
                 const uint32_t n0 = mul_bf16x2(pack_bf16x2(f0 * rstd, f1 * rstd), hgain.x), n1 = mul_bf16x2(pack_bf16x2(f2 * rstd, f3 * rstd), hgain.y);
                 const uint32_t neg = lane < 16 ? 0x80008000u : 0u;
                 const uint32_t o0 = __shfl_xor_sync(0xffffffffu, n0, 16) ^ neg, o1 = __shfl_xor_sync(0xffffffffu, n1, 16) ^ neg;
