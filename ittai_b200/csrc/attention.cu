@@ -182,11 +182,13 @@ __global__ void __launch_bounds__(WARPS * 32) attn_fwd_kernel(const AttnArgs a) 
     }
 }
 
-// Few queries (at most 32 a sequence), causal, head_dim 128: a short prompt.  One CTA per (sequence, head), two warps per 16 queries that both
-// compute the scores and share the output's 128 columns out; 32 keys a step, the next step's on their way meanwhile.  It runs once per layer, so
-// what attn_fwd_kernel spends here, its 64-key steps unrolled for keys that do not exist, is code to be fetched (see the attention of
-// qwen3_chain.cu) and masks: a forward of 3 / 8 / 23 / 32 tokens 431 / 455 / 612 / 721 us with it, 375 / 401 / 557 / 664 with this one.
-constexpr int kFewRows = 32, kFewKeys = 32, kFewThreads = 128;
+// Few queries (at most 64 a sequence), causal, head_dim 128: a short prompt.  One CTA per (sequence, head, 32 queries), two warps per 16 queries
+// that both compute the scores and share the output's 128 columns out; 32 keys a step, the next step's on their way meanwhile.  It runs once
+// per layer, so what attn_fwd_kernel spends here, its 64-key steps unrolled for keys that do not exist, is code to be fetched (see the
+// attention of qwen3_chain.cu) and masks.  Forwards of 3 / 8 / 23 / 32 / 33 / 48 / 64 tokens 431 / 455 / 612 / 721 / 729 / 787 / 953 us with it,
+// 375 / 401 / 557 / 664 / 695 / 759 / 923 with this one; 40 texts of 60 tokens 3136 and 3013, 130 of 40 5676 and 5612; 20 tokens behind 1000 / 8000
+// cached ones 1799 / 8477 and 1326 / 5835, 60 tokens 2339 / 10692 and 2221 / 10084.  (Above 64 the key-loop kernel on tcgen05 takes over.)
+constexpr int kFewMax = 64, kFewRows = 32, kFewKeys = 32, kFewThreads = 128;
 __device__ __forceinline__ float ex2_ftz(float x) {
     float y;
     asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
@@ -576,8 +578,8 @@ static int ittai::attention_launch(const IttaiAttention* p, bool disjoint, cudaS
         const cudaError_t e1 = launch_pdl(attn_q1_kernel, dim3(nh, ns), dim3(32 * kQ1Warps), 0, st, 1, a);
         return e1 == cudaSuccess ? ITTAI_OK : cuda_fail(e1, "launch attn_q1_kernel");
     }
-    if (p->head_dim == 128 && p->causal && ql <= kFewRows) {
-        const cudaError_t e1 = launch_pdl(attn_few_kernel, dim3(1, nh, ns), dim3(kFewThreads), (size_t)(kFewRows + 4 * kFewKeys) * 128 * 2, st, 1, a, p->seqs_ready);
+    if (p->head_dim == 128 && p->causal && ql <= kFewMax) {
+        const cudaError_t e1 = launch_pdl(attn_few_kernel, dim3((ql + kFewRows - 1) / kFewRows, nh, ns), dim3(kFewThreads), (size_t)(kFewRows + 4 * kFewKeys) * 128 * 2, st, 1, a, p->seqs_ready);
         return e1 == cudaSuccess ? ITTAI_OK : cuda_fail(e1, "launch attn_few_kernel");
     }
     if (p->head_dim == 128) rc = p->causal ? attn_launch<128, true, 4>(a, ql, nh, ns, st) : attn_launch<128, false, 4>(a, ql, nh, ns, st);

@@ -147,6 +147,35 @@ def test_attention_causal_gqa_cache_layout(q_len, prefix):
 
 
 @gpu
+@pytest.mark.parametrize("lens,prefix,group,ready", [([1], 0, 2, 0), ([5, 32, 17], 0, 2, 1), ([31], 1, 2, 1), ([33, 2], 0, 2, 1), ([40], 24, 1, 0), ([64, 63], 0, 2, 1),
+                                                     ([64], 64, 4, 1), ([16], 500, 2, 1), ([48, 0, 7], 31, 2, 1)])
+def test_attention_of_few_queries(lens, prefix, group, ready):
+    """At most 64 causal queries of head_dim 128: tiles of 32 queries, steps of 32 keys, and rows past each sequence that hold NaN.  Bound as for
+    the other kernels that round P to bf16."""
+    from ittai_b200 import ops
+    NH, hd, cap, B = 8, 128, 640, len(lens)
+    NKV, T = NH // group, sum(lens)
+    q = _rand(T, NH * hd, seed=12)
+    kc, vc = _rand(B, NKV, cap, hd, seed=13), _rand(B, NKV, cap, hd, seed=14)
+    out = torch.full((T, NH * hd), float("nan"), dtype=torch.bfloat16, device="cuda")
+    first = [sum(lens[:b]) for b in range(B)]
+    seqs = torch.tensor([[first[b], n, 0, prefix + n] for b, n in enumerate(lens)], dtype=torch.int32, device="cuda")
+    for b, n in enumerate(lens):
+        kc[b, :, prefix + n:] = float("nan")
+        vc[b, :, prefix + n:] = float("nan")
+    ops.attention(q, kc, vc, out, seqs, n_heads=NH, group=group, head_dim=hd, causal=True, max_q_len=max(lens), q_strides=(NH * hd, hd),
+                  k_strides=(hd, cap * hd, NKV * cap * hd), v_strides=(hd, cap * hd, NKV * cap * hd), o_strides=(NH * hd, hd), seqs_ready=bool(ready))
+    for b, n in enumerate(lens):
+        if n == 0:
+            continue
+        rows, kv = slice(first[b], first[b] + n), prefix + n
+        k, v = (c[b, :, :kv].float().repeat_interleave(group, 0) for c in (kc, vc))
+        mask = torch.arange(kv, device="cuda")[None, :] <= torch.arange(n, device="cuda")[:, None] + prefix
+        want = F.scaled_dot_product_attention(q[rows].float().view(n, NH, hd).transpose(0, 1), k, v, attn_mask=mask)
+        _check(out[rows], want.transpose(0, 1).reshape(n, NH * hd), f"few queries {n} behind {prefix}, group {group}")
+
+
+@gpu
 @pytest.mark.parametrize("q_len,prefix,causal", [(300, 0, True), (130, 70, True), (512, 0, True), (128, 1000, True), (65, 3, True), (200, 56, False)])
 def test_attention_key_loop_tensor_memory_kernel(q_len, prefix, causal):
     """The tcgen05 key-loop kernel (row totals + status words given) on the Qwen3 layout: q in a [T, 4096] qkv matrix, k/v in
