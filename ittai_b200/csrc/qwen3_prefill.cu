@@ -34,7 +34,7 @@ static int prefill_launch(const IttaiQwen3Prefill* p, void* st) {
     cudaDeviceGetAttribute(&n_sms, cudaDevAttrMultiProcessorCount, dev);
     // a small forward: both normalised projections run as split-K GEMMs, which normalise their input themselves
     const bool normed = p->split_k && !fold && gemm_split_wins(T, DGU, n_sms) && gemm_split_wins(T, DQKV, n_sms);
-    // shorter still: projections of their own (figures in qwen3_short.cu; at 33 tokens a split-K forward takes 809 us, one of 32 took 749);
+    // shorter still: projections of their own (figures in qwen3_short.cu);
     // the row statistics between them lie in xn, which nothing else uses then
     const bool brief = p->split_k && fused && T <= kShortTokens;
     float* squares = brief ? reinterpret_cast<float*>(p->xn) : nullptr;

@@ -1,4 +1,4 @@
-// The four projections of a Qwen3 layer for forwards of at most 32 tokens (a search query, a short prompt).
+// The four projections of a Qwen3 layer for forwards of at most 32 tokens (a search query, a short prompt), and below for 33 to 48.
 //
 // At this size a projection is its weights on their way and one chain of latencies.  As split-K GEMMs on tcgen05 (gemm_split_sm100.cu) the chain
 // was 9000 cycles for 23 tokens: activations through TMA, row statistics, a pass that normalises the landed tile in shared memory and
@@ -329,27 +329,304 @@ __global__ void __launch_bounds__(Shape<EPI, K>::kThreads, 2) proj_kernel(const 
     }
 }
 
-template <int NT, int EPI, int K>
-static cudaError_t launch(const CUtensorMap& tm, const Args& a, int n_rows, cudaStream_t st) {
-    using S = Shape<EPI, K>;
-    constexpr uint32_t kSmem = Plan<NT, EPI, K>::kSmem;
-    static thread_local int attr_dev = -1;
+// ---- 33 to 48 tokens ------------------------------------------------------------------------------------------------------
+// The same flow on tcgen05, whose MMA costs the same 40 cycles for 16 and for 64 tokens (it is the weights' 4 KB a step, read out of shared memory,
+// that take them): weights as the 128-row operand, activations normalised in registers on the way to where the MMA reads them, the
+// accumulator through shared memory, so that a token's sums lie side by side.  A cluster of eight shares the K of O and down (64 rows a CTA).
+// Forwards of 33 / 40 / 48 / 64 tokens, us: split-K GEMMs 816 / 821 / 860 / 957, this 729 / 755 / 787 / 986 (up to 32 tokens see the top of the
+// file).  Hence the line at 48: beyond, gate/up's shared memory leaves no room for its neighbours'.
+constexpr int kWideThreads = 256;
+template <int TN, int EPI, int K>
+struct WideShape {
+    static constexpr int kRanks = EPI == kResidual ? 8 : 4;                          // CTAs that share K out
+    static constexpr int kSlice = K / kRanks, kBlocks = kSlice / 64;                 // columns of a CTA
+    static constexpr int kRows = EPI == kQkv ? 128 : EPI == kGateUp ? 192 : 64;      // weight rows of a CTA
+    static constexpr int kAccs = kRows > 128 ? 2 : 1;                                // MMAs of 128 rows: the second one starts at row 64
+    static constexpr int kSlots = TN / kRanks;                                       // tokens that a CTA finishes at most
+    static constexpr int kPieces = kSlice / 8;                                       // 16-byte pieces of a token row
+    static constexpr int kRounds = TN * kPieces / kWideThreads;
+    static constexpr int kMine = (kSlots + kWideThreads / 32 - 1) / (kWideThreads / 32);       // QKV: tokens that a warp finishes
+    static constexpr int kPartLd = kRows + 4;                                        // floats per token on the way from the accumulator
+    static constexpr int kQuads = kRows / 4;
+    static constexpr uint32_t kW = kRows * kSlice * 2, kX = TN * kSlice * 2, kPart = TN * kPartLd * 4, kRecv = kRanks * kSlots * kRows * 4;
+    static constexpr uint32_t kSmem = kW + kX + kRecv + 1024;
+    static constexpr uint32_t kCols = TN * kAccs <= 64 ? 64 : 128;                      // of tensor memory: a power of two
+    static_assert(kPart <= kW, "the accumulator's way out takes the place of the weights");
+    static_assert(kRows >= 128 || kX >= 64 * 128, "an MMA reads 128 rows: those past the tile lie in the next block or in x");
+    static_assert(TN * kPieces % kWideThreads == 0 && TN % 16 == 0, "");
+};
+
+template <int TN, int EPI, int K>
+__global__ void __launch_bounds__(kWideThreads, 2) wide_kernel(const __grid_constant__ CUtensorMap tm_w, const Args a) {
+    using S = WideShape<TN, EPI, K>;
+    constexpr int kRanks = S::kRanks, kThreads = kWideThreads, kWarps = kThreads / 32;
+    extern __shared__ __align__(1024) unsigned char smem_raw[];
+    unsigned char* sm = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
+    unsigned char* sx = sm + S::kW;
+    __shared__ unsigned long long landed, acc_full, arrived;
+    __shared__ uint32_t tmem_slot;
+    __shared__ volatile uint32_t failed;
+    const int warp = warp_index(), lane = threadIdx.x & 31;
+    const int rank = blockIdx.x % kRanks, tile = blockIdx.x / kRanks;
+    const int own = (a.tokens - rank + kRanks - 1) / kRanks;         // tokens that this CTA finishes (0 where there are fewer than ranks)
+    if (threadIdx.x == 0) {
+        mbar_init(&landed, 1);
+        mbar_init(&acc_full, 1);
+        mbar_init(&arrived, 1);
+        failed = 0;
+        fence_mbar_init();
+        mbar_expect_tx(&landed, S::kW);
+        mbar_expect_tx(&arrived, (uint32_t)own * S::kRows * 4 * kRanks);
+#pragma unroll
+        for (int j = 0; j < S::kBlocks; ++j)
+            tma_load_2d(sm + j * S::kRows * 128, &tm_w, rank * S::kSlice + 64 * j, a.w_row + tile * S::kRows, &landed);
+    }
+    if (warp == 1) tmem_alloc(&tmem_slot, S::kCols);                  // ahead of the trigger: a later kernel on this SM cannot take them first
+    tc_fence_before();
+    __syncthreads();
+    tc_fence_after();
+    // another CTA's shared memory may be written only once that CTA runs; waited for ahead of the first write
+    asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
+    pdl_trigger();
+    const uint32_t tmem = tmem_slot;
+    uint4 gain = make_uint4(0u, 0u, 0u, 0u);
+    IttaiQkRope rope;
+    uint2 hgain = make_uint2(0u, 0u);
+    if constexpr (EPI == kQkv) {                                      // see proj_kernel
+        rope = a.rope;
+        asm volatile("" : "+l"(rope.pos), "+l"(rope.seq), "+l"(rope.slot), "+l"(rope.rope));
+        if (tile < 24) hgain = *reinterpret_cast<const uint2*>(reinterpret_cast<const bf16*>(tile < 16 ? rope.qn : rope.kn) + 4 * lane);
+        asm volatile("" : "+r"(hgain.x), "+r"(hgain.y));
+    }
+    if constexpr (EPI != kResidual) {
+        gain = *reinterpret_cast<const uint4*>(a.gain + rank * S::kSlice + 8 * lane);
+        asm volatile("" : "+r"(gain.x), "+r"(gain.y), "+r"(gain.z), "+r"(gain.w));     // arrived: a load left open may be scheduled behind the wait
+    }
+    pdl_wait();
+
+    // ---- activations: piece i of the slice is 16 bytes of token i / kPieces (with a norm a warp has a whole row)
+    uint4 xv[S::kRounds];
+    float ss[S::kRounds];
+#pragma unroll
+    for (int i = 0; i < S::kRounds; ++i) {
+        const int p = threadIdx.x + i * kThreads, n = p / S::kPieces;
+        xv[i] = make_uint4(0u, 0u, 0u, 0u);
+        ss[i] = 0.f;
+        if (n < a.tokens) {
+            xv[i] = ldcg128(a.x + (size_t)n * K + rank * S::kSlice + 8 * (p % S::kPieces));
+            if constexpr (EPI != kResidual) ss[i] = ldcgf(a.stats_in + n * kParts + lane);
+        }
+    }
+    // What the epilogue reads, ahead of the main loop.  O, down: 16 lanes a token, four columns each; QKV: a warp a token
+    const int quad = threadIdx.x & 15, slot16 = threadIdx.x >> 4;
+    uint2 res = make_uint2(0u, 0u), cosr[S::kMine], sinr[S::kMine];
+    bf16* dst[S::kMine];
+    if constexpr (EPI == kResidual) {
+        if (slot16 < own) res = *reinterpret_cast<const uint2*>(a.res + (size_t)(kRanks * slot16 + rank) * D + tile * 64 + 4 * quad);
+    }
+    int pos[S::kMine], seq[S::kMine], row[S::kMine];
+    if constexpr (EPI == kQkv) {
+#pragma unroll
+        for (int u = 0; u < S::kMine; ++u) {
+            const int n = kRanks * (warp + kWarps * u) + rank;        // the u-th token of this warp
+            pos[u] = seq[u] = row[u] = 0;
+            if (n < a.tokens) {
+                pos[u] = rope.pos[n];
+                if (tile >= 16) { seq[u] = rope.seq[n]; row[u] = rope.slot[n]; }
+            }
+        }
+    }
+#pragma unroll
+    for (int i = 0; i < S::kRounds; ++i) {
+        const int p = threadIdx.x + i * kThreads, n = p / S::kPieces, c = p % S::kPieces;
+        if (n < a.tokens) {                                           // rows past the last token: whatever lies there, their sums are not read
+            if constexpr (EPI != kResidual) {
+                const float rstd = rsqrt_full(warp_sum(ss[i]) * (1.0f / D) + a.eps);
+                uint32_t* u = reinterpret_cast<uint32_t*>(&xv[i]);
+                const uint32_t gw[4] = {gain.x, gain.y, gain.z, gain.w};
+#pragma unroll
+                for (int j = 0; j < 4; ++j) u[j] = mul_bf16x2(pack_bf16x2(bf_lo(u[j]) * rstd, bf_hi(u[j]) * rstd), gw[j]);
+            }
+            *reinterpret_cast<uint4*>(sx + (c >> 3) * (TN * 128) + n * 128 + (((c & 7) ^ (n & 7)) << 4)) = xv[i];
+        }
+    }
+    fence_proxy_async_smem();                                         // the MMAs read through the async proxy
+    if constexpr (EPI == kQkv) {
+#pragma unroll
+        for (int u = 0; u < S::kMine; ++u) {
+            const int n = kRanks * (warp + kWarps * u) + rank;
+            cosr[u] = sinr[u] = make_uint2(0u, 0u);
+            if (n < a.tokens && tile < 24) {
+                const bf16* rp = reinterpret_cast<const bf16*>(rope.rope) + (size_t)pos[u] * HD + 4 * (lane & 15);
+                cosr[u] = *reinterpret_cast<const uint2*>(rp); sinr[u] = *reinterpret_cast<const uint2*>(rp + HD / 2);
+            }
+            dst[u] = tile < 16 ? a.out + (size_t)n * DQKV + tile * HD + 4 * lane
+                               : reinterpret_cast<bf16*>(tile < 24 ? rope.kcache_layer : rope.vcache_layer) + (((size_t)seq[u] * NKV + (tile & 7)) * rope.kv_cap + row[u]) * HD + 4 * lane;
+        }
+    }
+    __syncthreads();
+    if (warp == 0) {
+        if (elect_one()) {
+            if (mbar_wait_bounded(&landed, 0, kSpin)) {
+                tc_fence_after();
+                constexpr uint32_t idesc = umma_idesc_bf16(128, TN);
+#pragma unroll
+                for (int kb = 0; kb < S::kBlocks; ++kb) {
+                    const uint64_t dw = umma_desc_sw128(sm + kb * S::kRows * 128), dx = umma_desc_sw128(sx + kb * TN * 128);
+#pragma unroll
+                    for (int k = 0; k < 4; ++k) {
+                        umma_bf16(tmem, dw + 2 * k, dx + 2 * k, idesc, kb > 0 || k > 0 ? 1u : 0u);
+                        if constexpr (S::kAccs == 2) umma_bf16(tmem + TN, dw + 2 * k + (64 * 128 >> 4), dx + 2 * k, idesc, kb > 0 || k > 0 ? 1u : 0u);
+                    }
+                }
+                umma_commit(&acc_full);
+            } else {
+                failed = 1;
+            }
+        }
+        __syncwarp();
+    }
+    {
+        bool ok = true;
+        uint32_t spins = 0;
+        while (!mbar_try_wait_parked(&acc_full, 0)) { if (failed || ++spins >= kSpin) { ok = false; break; } }
+        if (!__all_sync(0xffffffffu, ok)) failed = 1;
+        __syncwarp();
+    }
+    tc_fence_after();
+    // ---- accumulator: warp w may touch lanes 32 (w % 4) .. + 31, a weight row each; the two warps of a lane quarter share the tokens out
+    {
+        float* part = reinterpret_cast<float*>(sm);                   // in place of the weights: the MMAs have read them
+        const int q = warp & 3, half = (warp >> 2) * (TN / 2);
+#pragma unroll
+        for (int m = 0; m < S::kAccs; ++m) {
+            if ((S::kRows == 64 && q >= 2) || (m == 1 && q < 2)) continue;          // no rows of this tile, or the first MMA's
+#pragma unroll
+            for (int c = 0; c < TN / 2; c += 8) {
+                if (half + c < a.tokens) {
+                    uint32_t r[8];
+                    tmem_ld_32x8(tmem + ((uint32_t)(32 * q) << 16) + m * TN + half + c, r);
+                    tmem_ld_wait();
+#pragma unroll
+                    for (int i = 0; i < 8; ++i) part[(half + c + i) * S::kPartLd + 64 * m + 32 * q + lane] = __uint_as_float(r[i]);
+                }
+            }
+        }
+    }
+    tc_fence_before();
+    __syncthreads();
+    if (warp == 1) tmem_dealloc(tmem, S::kCols);
+    // ---- to the ranks that finish the tokens
+    asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+    const uint32_t w0 = smem_u32(sm), recv = smem_u32(sx) + S::kX;
+    for (int i = threadIdx.x; i < a.tokens * S::kQuads; i += kThreads) {
+        const int n = i / S::kQuads, q = i % S::kQuads, to = n % kRanks;
+        st_async_f32x4(map_addr(recv + (uint32_t)((rank * S::kSlots + n / kRanks) * S::kRows + 4 * q) * 4, to), lds_f4(w0 + (uint32_t)(n * S::kPartLd + 4 * q) * 4),
+                       map_addr(smem_u32(&arrived), to));
+    }
+    {
+        uint32_t spins = 0;
+        while (!mbar_try_wait_cluster(&arrived, 0)) { if (++spins >= (kSpin << 4)) { failed = 1; break; } }
+        __syncwarp();
+    }
+    auto total = [&](int slot, int q) {                              // sums of the ranks, in their order
+        float4 v = lds_f4(recv + (uint32_t)(slot * S::kRows + 4 * q) * 4);
+#pragma unroll
+        for (int r = 1; r < kRanks; ++r) v = add4(v, lds_f4(recv + (uint32_t)((r * S::kSlots + slot) * S::kRows + 4 * q) * 4));
+        return v;
+    };
+    if constexpr (EPI == kQkv) {
+#pragma unroll
+        for (int u = 0; u < S::kMine; ++u) {
+            if (warp + kWarps * u >= own) break;
+            const float4 v = total(warp + kWarps * u, lane);
+            uint32_t y0 = pack_bf16x2(v.x, v.y), y1 = pack_bf16x2(v.z, v.w);
+            if (tile < 24) {
+                // the rounding steps of qk_rope_scatter_kernel on packed pairs; the partner element 64 columns away is 16 lanes away
+                const float f0 = bf_lo(y0), f1 = bf_hi(y0), f2 = bf_lo(y1), f3 = bf_hi(y1);
+                const float rstd = rsqrt_full(warp_sum(fmaf(f0, f0, fmaf(f1, f1, fmaf(f2, f2, f3 * f3)))) * (1.0f / HD) + rope.eps);
+                const uint32_t n0 = mul_bf16x2(pack_bf16x2(f0 * rstd, f1 * rstd), hgain.x), n1 = mul_bf16x2(pack_bf16x2(f2 * rstd, f3 * rstd), hgain.y);
+                const uint32_t neg = lane < 16 ? 0x80008000u : 0u;
+                const uint32_t o0 = __shfl_xor_sync(0xffffffffu, n0, 16) ^ neg, o1 = __shfl_xor_sync(0xffffffffu, n1, 16) ^ neg;
+                y0 = add_bf16x2(mul_bf16x2(n0, cosr[u].x), mul_bf16x2(o0, sinr[u].x));
+                y1 = add_bf16x2(mul_bf16x2(n1, cosr[u].y), mul_bf16x2(o1, sinr[u].y));
+            }
+            *reinterpret_cast<uint2*>(dst[u]) = make_uint2(y0, y1);
+        }
+    } else if constexpr (EPI == kGateUp) {
+        for (int i = threadIdx.x; i < own * S::kQuads; i += kThreads) {
+            const int slot = i / S::kQuads, q = i % S::kQuads;
+            const float4 v = total(slot, q);
+            // adjacent rows are (gate, up): act = bf16(bf16(silu(bf16 gate)) * bf16 up)
+            const float g0 = bf16r(v.x), u0 = bf16r(v.y), g1 = bf16r(v.z), u1 = bf16r(v.w);
+            *reinterpret_cast<uint32_t*>(a.out + (size_t)(kRanks * slot + rank) * FF + tile * (S::kRows / 2) + 2 * q) =
+                pack_bf16x2(bf16r(g0 / (1.0f + expf(-g0))) * u0, bf16r(g1 / (1.0f + expf(-g1))) * u1);
+        }
+    } else {
+        if (2 * warp < own) {                                         // whole warps: two tokens each
+            const float4 v = total(slot16 < own ? slot16 : 0, quad);
+            const uint2 o = make_uint2(pack_bf16x2(bf_lo(res.x) + bf16r(v.x), bf_hi(res.x) + bf16r(v.y)), pack_bf16x2(bf_lo(res.y) + bf16r(v.z), bf_hi(res.y) + bf16r(v.w)));
+            const float a0 = bf_lo(o.x), a1 = bf_hi(o.x), a2 = bf_lo(o.y), a3 = bf_hi(o.y);
+            float s = fmaf(a0, a0, fmaf(a1, a1, fmaf(a2, a2, a3 * a3)));
+#pragma unroll
+            for (int m = 1; m < 8; m <<= 1) s += __shfl_xor_sync(0xffffffffu, s, m);
+            if (slot16 < own) {
+                const int n = kRanks * slot16 + rank;
+                *reinterpret_cast<uint2*>(a.out + (size_t)n * D + tile * 64 + 4 * quad) = o;
+                if ((quad & 7) == 0) a.stats_out[n * kParts + 2 * tile + (quad >> 3)] = s;
+            }
+        }
+    }
+    __syncthreads();
+    if (failed) {
+        // A CTA that gave up must not leave before what is owed to it has come: all send, also where their waits ran out.  Should a send take
+        // longer than this wait, the barrier holds the CTA until the others have left (threads that have exited count as arrived).
+        bool all = false;
+        for (uint32_t spins = 0; !all && spins < (kSpin << 4); ++spins) all = mbar_try_wait_cluster(&arrived, 0);
+        if (!__syncthreads_and(all)) {
+            asm volatile("barrier.cluster.arrive.release;" ::: "memory");
+            asm volatile("barrier.cluster.wait.acquire;" ::: "memory");
+        }
+        if (threadIdx.x == 0) {
+            if (atomicCAS(&a.status[0], 0u, (uint32_t)ITTAI_ST_GEMM_TIMEOUT) == 0u) { a.status[1] = blockIdx.x; a.status[2] = (uint32_t)K; }
+            const long long t0 = clock64();                           // copies still in flight land before the shared memory is handed back
+            while (clock64() - t0 < 2000000) {}
+        }
+        __syncthreads();
+    }
+}
+
+template <typename F>
+static cudaError_t start(F* kernel, int threads, uint32_t smem, int ranks, int rows, const CUtensorMap& tm, const Args& a, int n_rows, int* attr_dev, cudaStream_t st) {
     int dev = 0;
     cudaGetDevice(&dev);
-    if (attr_dev != dev) {
-        const cudaError_t e = cudaFuncSetAttribute(proj_kernel<NT, EPI, K>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmem);
+    if (*attr_dev != dev) {
+        const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
         if (e != cudaSuccess) return e;
-        attr_dev = dev;
+        *attr_dev = dev;
     }
-    return launch_pdl(proj_kernel<NT, EPI, K>, dim3(kRanks * (n_rows / S::kRows)), dim3(S::kThreads), kSmem, st, kRanks, tm, a);
+    return launch_pdl(kernel, dim3(ranks * (n_rows / rows)), dim3(threads), smem, st, ranks, tm, a);
+}
+template <int NT, int EPI, int K>
+static cudaError_t launch_narrow(const CUtensorMap& tm, const Args& a, int n_rows, cudaStream_t st) {
+    using S = Shape<EPI, K>;
+    static thread_local int attr_dev = -1;
+    return start(proj_kernel<NT, EPI, K>, S::kThreads, Plan<NT, EPI, K>::kSmem, kRanks, S::kRows, tm, a, n_rows, &attr_dev, st);
+}
+template <int TN, int EPI, int K>
+static cudaError_t launch_wide(const CUtensorMap& tm, const Args& a, int n_rows, cudaStream_t st) {
+    using S = WideShape<TN, EPI, K>;
+    static thread_local int attr_dev = -1;
+    return start(wide_kernel<TN, EPI, K>, kWideThreads, S::kSmem, S::kRanks, S::kRows, tm, a, n_rows, &attr_dev, st);
 }
 template <int EPI, int K>
 static cudaError_t launch_any(const CUtensorMap& tm, const Args& a, int n_rows, cudaStream_t st) {
+    if (a.tokens > kNarrowTokens) return launch_wide<48, EPI, K>(tm, a, n_rows, st);
     switch ((a.tokens + 7) / 8) {
-        case 1: return launch<1, EPI, K>(tm, a, n_rows, st);
-        case 2: return launch<2, EPI, K>(tm, a, n_rows, st);
-        case 3: return launch<3, EPI, K>(tm, a, n_rows, st);
-        default: return launch<4, EPI, K>(tm, a, n_rows, st);
+        case 1: return launch_narrow<1, EPI, K>(tm, a, n_rows, st);
+        case 2: return launch_narrow<2, EPI, K>(tm, a, n_rows, st);
+        case 3: return launch_narrow<3, EPI, K>(tm, a, n_rows, st);
+        default: return launch_narrow<4, EPI, K>(tm, a, n_rows, st);
     }
 }
 
@@ -360,10 +637,11 @@ int cuda_fail(cudaError_t e, const char* what);
 int short_maps(ShortMaps* m, const IttaiQwen3Prefill* p) {
     using namespace brief;
     const long long L = p->n_layers;
+    const bool wide = p->tokens > kNarrowTokens;
     int rc = make_tmap_bf16(&m->qkv, p->wqkv, L * DQKV, D, D, Shape<kQkv, D>::kRows);
-    if (rc == ITTAI_OK) rc = make_tmap_bf16(&m->o, p->wo, L * D, DQ, DQ, Shape<kResidual, DQ>::kRows);
+    if (rc == ITTAI_OK) rc = make_tmap_bf16(&m->o, p->wo, L * D, DQ, DQ, wide ? WideShape<48, kResidual, DQ>::kRows : Shape<kResidual, DQ>::kRows);
     if (rc == ITTAI_OK) rc = make_tmap_bf16(&m->gu, p->wgu, L * DGU, D, D, Shape<kGateUp, D>::kRows);
-    if (rc == ITTAI_OK) rc = make_tmap_bf16(&m->down, p->wd, L * D, FF, FF, Shape<kResidual, FF>::kRows);
+    if (rc == ITTAI_OK) rc = make_tmap_bf16(&m->down, p->wd, L * D, FF, FF, wide ? WideShape<48, kResidual, FF>::kRows : Shape<kResidual, FF>::kRows);
     return rc;
 }
 

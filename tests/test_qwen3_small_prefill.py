@@ -63,9 +63,9 @@ def test_more_shapes_than_graphs(tiny_hf):
 
 
 @gpu
-@pytest.mark.parametrize("lens", [[2], [7], [8], [9], [15, 1], [17], [24], [25], [31], [32], [33], [5, 9, 1, 17], [1] * 32])
+@pytest.mark.parametrize("lens", [[2], [7], [8], [9], [15, 1], [17], [24], [25], [31], [32], [33], [40], [47], [48], [49], [5, 9, 1, 17], [1] * 32, [16, 1, 31]])
 def test_short_forwards_match_the_split_gemms(tiny_hf, lens):
-    """Forwards of up to 32 tokens (their own projections and attention, tiles of 8 tokens, a token per rank of four) against the kernels of
+    """Forwards of up to 48 tokens (their own projections, tiles of 8 or of 48 tokens, a token per rank of four or eight) against the kernels of
     longer ones with the same rounding points (``fused_rope=False``): embeddings and the last layer's keys and values.  Bound: a bf16
     rounding is off by 1.1e-3 (rms), a layer has about eight in a row, so that two forwards of two layers whose roundings all fell
     differently would be sqrt(2 * 16) * 1.1e-3 = 6.2e-3 apart; half as much again for few tokens."""
@@ -88,14 +88,14 @@ def test_short_forwards_match_the_split_gemms(tiny_hf, lens):
 
 @gpu
 def test_a_short_prompt_behind_a_cached_one(tiny_hf):
-    """The attention of few queries with cached keys in front of them, several steps of 32: a prompt appended in two pieces against the prompt
+    """The attention of few queries, one tile of 32 or two, with cached keys in front of them: a prompt appended in pieces against the prompt
     at once (keys and values of two layers: the bound above)."""
     from ittai_b200.qwen3 import Qwen3Decoder
     model, dims = tiny_hf
     ids = hf.prompt_ids(150, seed=4, vocab=dims.vocab)
     whole, pieces = (Qwen3Decoder(model, max_batch=1, kv_capacity=256) for _ in range(2))
     whole.prefill_cache(ids)
-    for a, b in ((0, 97), (97, 98), (98, 128), (128, 150)):
+    for a, b in ((0, 64), (64, 97), (97, 98), (98, 128), (128, 150)):
         pieces.prefill_cache(ids[a:b])
     for a, b in ((whole.kcache, pieces.kcache), (whole.vcache, pieces.vcache)):
         a, b = a[..., :150, :].float(), b[..., :150, :].float()
