@@ -15,6 +15,11 @@ __device__ __forceinline__ void tma_load_2d(void* dst, const void* tmap, int x, 
     asm volatile("cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];"
                  ::"r"(smem_u32(dst)), "l"(tmap), "r"(x), "r"(y), "r"(smem_u32(bar)) : "memory");
 }
+// The same tile as far as L2.  A hint that nothing waits for and that hands no data over: unlike a load it may be given for an operand that
+// kernels still running write.
+__device__ __forceinline__ void tma_prefetch_2d(const void* tmap, int x, int y) {
+    asm volatile("cp.async.bulk.prefetch.tensor.2d.L2.global.tile [%0, {%1, %2}];" ::"l"(tmap), "r"(x), "r"(y) : "memory");
+}
 // 2-D tiled store shared -> global (rows and columns outside the tensor are dropped); completion is tracked per thread in
 // bulk groups: tma_store_commit() closes a group, tma_store_wait_read<N>() returns once all but the N newest groups have
 // finished READING shared memory.
