@@ -12,7 +12,9 @@
 //   weights in mma.sync m16n8k16: 32 rows x one K chunk x 8 NT tokens a warp.
 // * Chunks meet in shared memory, quarters through st.async, 16 bytes at a time, in the CTA that finishes the token (token n: rank n mod 4,
 //   where a warp or eight lanes hold a whole row piece for the head norm, the rotation or the statistics); sums in the order of chunks, then
-//   of ranks.
+//   of ranks from the last one on (as good as any: against the eager module's 64 tokens behind a prompt of 32, which near-ties decide, the orders
+//   0 1 2 3 / 3 2 1 0 / chunks in pairs agree in 60 / 62 / 62, at an rms distance of 9.5e-3 / 9.5e-3 / 9.4e-3, the split-K GEMMs in 62 at 10.0e-3;
+//   pairs cost 4 % at 17 to 24 tokens).
 //
 // Measured on a B200, a forward of 3 / 8 / 16 / 23 / 32 tokens, us, split-K GEMMs and attn_fwd_kernel -> this and attn_few_kernel:
 // 640 / 649 / 671 / 682 / 749 -> 351 / 372 / 461 / 536 / 617.  What grows with the tokens are the MMAs (legacy ones: 8 cycles each, 1150
@@ -264,10 +266,10 @@ __global__ void __launch_bounds__(Shape<EPI, K>::kThreads, 2) proj_kernel(const 
         while (!mbar_try_wait_cluster(&arrived, 0)) { if (++spins >= (kSpin << 4)) { came = false; break; } }
     }
     __syncwarp();
-    auto total = [&](int slot, int q) {                              // sums of the ranks, in their order
-        float4 v = lds_f4(recv + (uint32_t)(slot * S::kRows + 4 * q) * 4);
+    auto total = [&](int slot, int q) {                              // sums of the ranks, the last one's first
+        float4 v = lds_f4(recv + (uint32_t)(((kRanks - 1) * 2 * NT + slot) * S::kRows + 4 * q) * 4);
 #pragma unroll
-        for (int r = 1; r < kRanks; ++r) v = add4(v, lds_f4(recv + (uint32_t)((r * 2 * NT + slot) * S::kRows + 4 * q) * 4));
+        for (int r = kRanks - 2; r >= 0; --r) v = add4(v, lds_f4(recv + (uint32_t)((r * 2 * NT + slot) * S::kRows + 4 * q) * 4));
         return v;
     };
     if constexpr (EPI == kQkv) {
