@@ -39,7 +39,7 @@ constexpr uint32_t kTmemCols = 512;
 
 template <int TN, int STAGES>
 __global__ void __launch_bounds__(kGemmThreads, 1)
-gemm_bf16_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant__ CUtensorMap tm_b, const GemmArgs g) {
+gemm_bf16_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant__ CUtensorMap tm_b, const GemmArgs g, const int box_a) {
     extern __shared__ __align__(1024) unsigned char gsm_raw[];
     unsigned char* gsm = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(gsm_raw) + 1023) & ~(uintptr_t)1023);
     unsigned char* sa = gsm;                                         // [stages][128 rows][128 B]
@@ -93,7 +93,7 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant
                         if (*abort_flag) break;
                     }
                     free = it + 1 < STAGES || mbar_test(&empty[(it + 1) % STAGES], ((it + 1) / STAGES - 1) & 1);
-                    mbar_expect_tx(&full[s], kStageBytesA + GemmCfg<TN, STAGES>::kStageBytesB);
+                    mbar_expect_tx(&full[s], box_a * GK * 2 + GemmCfg<TN, STAGES>::kStageBytesB);
                     tma_load_2d(sa + s * kStageBytesA, &tm_a, kb * GK, tile_m * GM, &full[s]);
                     tma_load_2d(sb + s * GemmCfg<TN, STAGES>::kStageBytesB, &tm_b, kb * GK, tile_n * TN, &full[s]);
                 }
@@ -253,7 +253,9 @@ int gemm_bf16_launch(const IttaiGemm* a, cudaStream_t st, const void* a_gain) {
     // value: 256 x 256 pair tiles leave most of the GPU idle then.  M 200 to 1152, N 1024: K 2048 14.7 -> 8.5 us, K 3072 19.3 -> 10.9.
     const bool narrow = a != nullptr && a->epi == ITTAI_EPI_NONE && !a->row_stats && !a->stats_out && (long long)((a->m + GM - 1) / GM) * (a->n / 64) <= n_sms;
     const bool pair = !split && a != nullptr && a->m > GM && !narrow;
-    const int box_a = split ? gemm_split_rows(a->m, a->n, a->k, n_sms) : GM;
+    // One-SM tiles of fewer rows than 128 load no others: rows past M would be written as zeros all the same, 16 KB a k-block beside the weights' 8.
+    // Their accumulator rows come from whatever the stage holds, and are not stored.  Prefill of 17 / 58 tokens 1442 / 1407 -> 1253 / 1359 us.
+    const int box_a = split ? gemm_split_rows(a->m, a->n, a->k, n_sms) : !pair && a != nullptr && a->m < GM ? (a->m + 7) / 8 * 8 : GM;
     CUtensorMap tm_a, tm_b;
     GemmArgs g;
     const int rc = gemm_args_from_abi(a, &g, &tm_a, &tm_b, a ? a->epi & ~ITTAI_GEMM_STATIC_W : 0, split, split || pair ? 128 : 64, box_a);
@@ -270,7 +272,7 @@ int gemm_bf16_launch(const IttaiGemm* a, cudaStream_t st, const void* a_gain) {
         attr_dev = dev;
     }
     const int tiles = ((a->m + GM - 1) / GM) * (a->n / 64);
-    const cudaError_t e = launch_pdl(gemm_bf16_kernel<64, 8>, dim3(tiles < n_sms ? tiles : n_sms), dim3(kGemmThreads), GemmCfg<64, 8>::kSmem, st, 1, tm_a, tm_b, g);
+    const cudaError_t e = launch_pdl(gemm_bf16_kernel<64, 8>, dim3(tiles < n_sms ? tiles : n_sms), dim3(kGemmThreads), GemmCfg<64, 8>::kSmem, st, 1, tm_a, tm_b, g, box_a);
     return e == cudaSuccess ? ITTAI_OK : cuda_fail(e, "launch gemm_bf16_kernel");
 }
 

@@ -56,6 +56,22 @@ def test_one_sm_and_two_sm_kernels_agree_bit_for_bit(n, k):
 
 
 @gpu
+@pytest.mark.parametrize("m", [2, 7, 8, 9, 16, 57, 120, 121, 127])
+def test_short_tiles_load_only_their_rows(m):
+    """The one-SM kernel's tile of fewer than 128 rows (boxes of A rounded up to eight rows), behind a launch that leaves NaNs in the stages: the
+    bits of the same rows in a tile of 128, several times round the ring of stages, and no row past the last."""
+    from ittai_b200 import ops
+    a, w, res = _rand(128, 2048, seed=61), _rand(1024, 2048, scale=0.05, seed=62), _rand(128, 1024, seed=63)
+    st = ops.new_status("cuda")
+    want = ops.gemm(a, w, st, residual=res)
+    ops.gemm(torch.full_like(a, float("nan")), w, st)
+    guard = torch.full((m + 1, 1024), 3.0, dtype=torch.bfloat16, device="cuda")
+    got = ops.gemm(a[:m], w, st, residual=res[:m], out=guard[:m])
+    ops.check_status(st)
+    assert torch.equal(got, want[:m]) and (guard[m] == 3.0).all()
+
+
+@gpu
 def test_gemm_row_identity():
     """A = rows of the identity picks out columns of W: catches a wrong swizzle or K-step in the operand descriptors."""
     from ittai_b200 import ops
