@@ -162,3 +162,29 @@ def test_calls_on_two_streams_follow_one_another(tiny_hf):
     torch.cuda.synchronize()
     d.check_status()
     assert torch.equal(torch.cat([t.cpu() for t in parts], 1), want) and d.pos.tolist() == d.lengths == [90, 90]
+
+
+@gpu
+@pytest.mark.parametrize("batch,length,steps", [(1, 380, 45), (2, 20, 50), (4, 10, 21), (8, 600, 47)])
+def test_several_tokens_a_graph_are_the_tokens_one_by_one(tiny_hf, batch, length, steps):
+    """A long call queues several tokens as one graph from its 17th on, with single ones where the rest is shorter or a line of the rules
+    (clusters: 400, 48 and 700 positions; tiles held: 625 of eight) falls among them: ids, logits and cache rows are those of calls of one
+    step, in the first call and, with the graphs there, in the next."""
+    from ittai_b200.qwen3 import Qwen3Decoder
+    model, dims = tiny_hf
+    g = torch.Generator().manual_seed(7 * batch)
+    d = Qwen3Decoder(model, max_batch=batch, kv_capacity=1024)
+    kv = [(torch.randn(d.kcache.shape, generator=g) * s).to(torch.bfloat16) for s in (1.0, 0.5)]
+    ids = torch.randint(0, dims.vocab, (batch,), generator=g, dtype=torch.int32)
+
+    def run(call):
+        for c, t in zip((d.kcache, d.vcache), kv):
+            c.copy_(t)
+        d.rewind(length)
+        d.next_id.copy_(ids)
+        return torch.cat([d.decode(n).clone() for n in call], 1), d.logits.clone(), d.pos.clone(), d.kcache[:, :, :, :length + steps].clone(), d.vcache[:, :, :, :length + steps].clone()
+
+    want = run([1] * steps)
+    for call in ([steps], [steps], [17, steps - 17], [steps - 2, 2]):
+        for got, ref in zip(run(call), want):
+            assert torch.equal(got, ref), call
