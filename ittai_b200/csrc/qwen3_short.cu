@@ -17,7 +17,7 @@
 //   pairs cost 4 % at 17 to 24 tokens).
 //
 // Measured on a B200, a forward of 3 / 8 / 16 / 23 / 32 tokens, us, split-K GEMMs and attn_fwd_kernel -> this and attn_few_kernel:
-// 640 / 649 / 671 / 682 / 749 -> 351 / 372 / 461 / 536 / 617.  What grows with the tokens are the MMAs (legacy ones: 8 cycles each, 1150
+// 640 / 649 / 671 / 682 / 749 -> 345 / 357 / 438 / 515 / 604.  What grows with the tokens are the MMAs (legacy ones: 8 cycles each, 1150
 // of gate/up's 5800 cycles at 23 tokens), the sums' way through shared memory and the activations, which 32 CTAs read from the same lines of
 // L2.  Other forms, us at 3 / 23 / 32 tokens: weights from shared memory as the 128-row operand of tcgen05.mma, everything else alike 455 /
 // 582 / 618; tokens as the 128-row operand in tensor memory 603 / 692 / 744 (padded rows cost what real ones do: 54 cycles an MMA of 128
@@ -58,7 +58,13 @@ struct Plan {
     static constexpr uint32_t kW = S::kRows * S::kSlice * 2, kPart = S::kChunks * 8 * NT * S::kPartLd * 4;
     static constexpr uint32_t kX = kW > kPart ? kW : kPart;                          // offset: the sums of the chunks take the place of the weights
     static constexpr uint32_t kRecv = (kX + 8 * NT * S::kXLd + 127) / 128 * 128;     // offset: [ranks][2 NT tokens][rows] sums of the quarters
-    static constexpr uint32_t kSmem = kRecv + kRanks * 2 * NT * S::kRows * 4 + 1024;
+    static constexpr uint32_t kNeed = kRecv + kRanks * 2 * NT * S::kRows * 4 + 1024;
+    // Asked for, whether needed or not.  A kernel starts while the one in front holds 128 of the 148 SMs: what fits three times on an SM goes to
+    // the empty ones by threes, and the slowest CTA is what the next kernel waits for.  O-proj with room for one or two: forwards of 9 / 16 / 23 /
+    // 32 tokens, us, as little as needed 422 / 455 / 553 / 611, 76 KB 424 / 447 / 526 / 613, this 416 / 438 / 515 / 604 (of which for 32 tokens the QKV
+    // projection's one a SM); one a SM throughout 428 / 491 / 566 / 641, gate/up then finds no room beside it.  Up to 8 tokens every form lost 2 to 10 %.
+    static constexpr uint32_t kAtLeast = NT == 1 ? 0 : EPI == kQkv ? (NT == 4 ? 114 << 10 : 0) : EPI == kResidual && K == DQ ? (NT == 2 ? 106 << 10 : NT == 3 ? 98 << 10 : 86 << 10) : 0;
+    static constexpr uint32_t kSmem = kNeed > kAtLeast ? kNeed : kAtLeast;
 };
 
 struct Args {
@@ -152,6 +158,10 @@ __global__ void __launch_bounds__(Shape<EPI, K>::kThreads, 2) proj_kernel(const 
     for (int ks = 0; ks < S::kHeld; ++ks) { load_w(wf[ks][0], 0, ks); load_w(wf[ks][1], 1, ks); }
     if constexpr (EPI == kQkv) asm volatile("" : "+r"(hgain.x), "+r"(hgain.y));
     if constexpr (EPI != kResidual) asm volatile("" : "+r"(gain.x), "+r"(gain.y), "+r"(gain.z), "+r"(gain.w));    // arrived: a load left open may be scheduled behind the wait
+    // addresses ahead of the wait: behind it only requests with constant offsets
+    const bf16* xp = a.x + (size_t)warp * K + rank * S::kSlice + 8 * lane;
+    const float* sp = EPI != kResidual ? a.stats_in + warp * kParts + lane : nullptr;
+    asm volatile("" : "+l"(xp), "+l"(sp));
     pdl_wait();
 
     // ---- activations: a warp takes whole token rows of the slice
@@ -166,8 +176,8 @@ __global__ void __launch_bounds__(Shape<EPI, K>::kThreads, 2) proj_kernel(const 
         for (int p = 0; p < S::kPieces; ++p) xv[i][p] = make_uint4(0u, 0u, 0u, 0u);
         if (n < a.tokens) {
 #pragma unroll
-            for (int p = 0; p < S::kPieces; ++p) xv[i][p] = ldcg128(a.x + (size_t)n * K + rank * S::kSlice + 256 * p + 8 * lane);
-            if constexpr (EPI != kResidual) ss[i] = ldcgf(a.stats_in + n * kParts + lane);
+            for (int p = 0; p < S::kPieces; ++p) xv[i][p] = ldcg128(xp + (size_t)i * S::kWarps * K + 256 * p);
+            if constexpr (EPI != kResidual) ss[i] = ldcgf(sp + i * S::kWarps * kParts);
         }
     }
     // what the epilogue reads, ahead of the main loop.  O, down: eight lanes a token, four columns each; QKV: a warp a token
