@@ -533,17 +533,23 @@ int gemm_split_rows(int m, int n, int k, int n_sms) {
 
 template <int TN, int EPI>
 static cudaError_t split_launch(const CUtensorMap& tm_a, const CUtensorMap& tm_w, const GemmArgs& g, int n_sms, cudaStream_t st) {
+    constexpr uint32_t kLone = SplitCfg<TN>::kSmem > 115u * 1024 ? SplitCfg<TN>::kSmem : 115u * 1024;      // one CTA per SM
     static thread_local int attr_dev = -1;
     int dev = 0;
     cudaGetDevice(&dev);
     if (attr_dev != dev) {
-        const cudaError_t e = cudaFuncSetAttribute(gemm_split_kernel<TN, EPI>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SplitCfg<TN>::kSmem);
+        const cudaError_t e = cudaFuncSetAttribute(gemm_split_kernel<TN, EPI>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kLone);
         if (e != cudaSuccess) return e;
         attr_dev = dev;
     }
     const int tiles_m = (g.M + TN - 1) / TN, tiles_n = g.N / SN, lg = split_log2(tiles_m * tiles_n, g.K / SK, n_sms);
+    // A tower's QKV projection whose CTAs all find an SM of their own gets it, by shared memory that it does not need; otherwise SMs that the kernel in
+    // front leaves empty take two.  One image of ViT-B/16 403.5 -> 391.2 us, of the variable-resolution tower 445 -> 429.  Not the others: two such
+    // kernels in a row share no SM, and the second one's weights then come only when the first has ended (language, O-proj or down this way
+    // 880 -> 980 us at 64 tokens; its QKV projection 805 -> 813 at 49, 876 -> 866 at 64, 1159 -> 1164 at 128).
+    const bool lone = EPI == ITTAI_EPI_NONE && g.row_stats != nullptr && g.a_gain == nullptr && (tiles_m * tiles_n) << lg <= n_sms;
     // even row tiles: 196 rows are 98 and 98, not 128 and 68
-    return launch_pdl(gemm_split_kernel<TN, EPI>, dim3(1 << lg, tiles_n, tiles_m), dim3(kSplitThreads), SplitCfg<TN>::kSmem, st, 1 << lg, tm_a, tm_w, g,
+    return launch_pdl(gemm_split_kernel<TN, EPI>, dim3(1 << lg, tiles_n, tiles_m), dim3(kSplitThreads), lone ? kLone : SplitCfg<TN>::kSmem, st, 1 << lg, tm_a, tm_w, g,
                       (g.M + tiles_m - 1) / tiles_m, lg);
 }
 template <int TN>
