@@ -920,9 +920,9 @@ struct Plan {
 // Tokens of a kind in one graph.  Between the kernels of a graph a launch overlaps its predecessor's tail, and the first projection's weights come
 // while the last kernel of the token before runs; between graphs neither.  us per step with 1 / 2 / 4 / 8 / 16 tokens a graph: batch 1 at 60
 // 374.8 / 373.5 / 371.9 / 371.3 / 370.8, at 4096 460 / 458.2 / 456.7 / 456.6 / 456, batch 4 at 300 434 / 430.4 / 429.4 / 429.2 / 428.2, batch 8 at 1000
-// 615.8 / 613 / 611.6 / 610.9 / 610.  Capturing four takes the host 2.4 ms: it is done where the GPU has 16 tokens of this call to work on
-// meanwhile, or after 512 tokens of short calls.
-constexpr int kSeveral = 4, kSeveralInCall = 16, kSeveralAfter = 512;
+// 615.8 / 613 / 611.6 / 610.9 / 610.  Capturing four takes the host 2.4 to 3.3 ms: it is done while the GPU has work of the call, behind the 16th token
+// of a long one, or behind the last of a call of eight or more once 64 have been queued one by one (the request loop's).
+constexpr int kSeveral = 4, kSeveralInCall = 16, kSeveralAfter = 64, kSeveralBehind = 8;
 
 template <typename F>
 static cudaError_t prefer_shared(F* fn, int dynamic = 0) {
@@ -1112,7 +1112,7 @@ static int enqueue_call(Plan* pl, const IttaiQwen3Decode& p, int max_len, bool c
             const bool same = head && last < p.n_steps && pieces(p.batch, len) == cs && hold_tiles(p.batch, len) == held;
             cudaGraphExec_t& s = pl->several[slot][held ? 1 : 0];
             int& queued = pl->queued[slot][held ? 1 : 0];
-            const bool several = same && (s != nullptr || i >= kSeveralInCall || queued >= kSeveralAfter);
+            const bool several = same && (s != nullptr || i >= kSeveralInCall);
             cudaGraphExec_t& x = several ? s : pl->exec[slot][held ? 1 : 0][head ? 1 : 0];
             if (x == nullptr) {
                 const int rc = capture(pl, cs, held, head, several ? kSeveral : 1, &x);
@@ -1120,7 +1120,11 @@ static int enqueue_call(Plan* pl, const IttaiQwen3Decode& p, int max_len, bool c
             }
             e = cudaGraphLaunch(x, st);
             if (several) i = last;
-            else if (queued < kSeveralAfter) ++queued;
+            else if (head && queued < kSeveralAfter) ++queued;
+            if (i + 1 >= p.n_steps && i + 1 >= kSeveralBehind && head && queued >= kSeveralAfter && s == nullptr && e == cudaSuccess) {
+                const int rc = capture(pl, cs, held, true, kSeveral, &s);
+                if (rc != ITTAI_OK) return rc;
+            }
         }
         if (e != cudaSuccess) return cuda_fail(e, "launch of a decode step");
     }
