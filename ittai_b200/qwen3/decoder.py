@@ -199,6 +199,11 @@ class Qwen3Decoder:
         its ids forced (lm_head only on the final one), which also yields the logits and the first generated id.
         ``tensor_cores`` forces one path (default: tensor cores from 32 prompt tokens on).
         """
+        return self._prefill_and_decode(ids, 1, tensor_cores)[-1]
+
+    def _prefill_and_decode(self, ids, n_steps: int, tensor_cores: bool | None = None) -> torch.Tensor:
+        """``prefill``, and ``n_steps - 1`` further greedy steps in the same call of the decode chain: int32 ``[n_steps, B]`` on the device.  (As two
+        calls the first one's status was waited for while the GPU stood still: a prompt of 47 and 32 tokens 12.97 -> 12.87 ms.)"""
         ids = torch.as_tensor(ids, dtype=torch.int32)
         if ids.dim() == 1:
             ids = ids[None]
@@ -210,8 +215,8 @@ class Qwen3Decoder:
             self._prefill_dense(ids[:, :T - 1], check=False)     # the launch below reads both verdicts
             ids = ids[:, T - 1:]
         forced = ids.t().contiguous().to(self.dev, non_blocking=True)       # [T, B]
-        out, _ = self._launch(forced.shape[0], forced=forced)
-        return out[-1]
+        out, _ = self._launch(forced.shape[0] + n_steps - 1, forced=forced)
+        return out[forced.shape[0] - 1:]
 
     def prefill_slots(self, prompts: dict) -> None:
         """Append token ids to the caches of SOME sequences of the batch, each with its own length: ``prompts`` maps a
@@ -382,7 +387,4 @@ class Qwen3Decoder:
     def generate(self, prompt_host: torch.Tensor, n_steps: int) -> torch.Tensor:
         """End to end from host memory: copy the prompt ids in, prefill, decode, copy the ids out (host tensor [B, n_steps])."""
         self.reset()
-        first = self.prefill(prompt_host)
-        rest = self.decode(n_steps - 1) if n_steps > 1 else None
-        out = first[:, None] if rest is None else torch.cat([first[:, None], rest], 1)
-        return out.cpu()
+        return self._prefill_and_decode(prompt_host, max(n_steps, 1)).t().contiguous().cpu()
