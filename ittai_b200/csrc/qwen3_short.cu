@@ -646,8 +646,13 @@ static cudaError_t launch_any(const CUtensorMap& tm, const Args& a, int n_rows, 
 
 int cuda_fail(cudaError_t e, const char* what);
 
+void set_error(const char* fmt, ...);
+
 int short_maps(ShortMaps* m, const IttaiQwen3Prefill* p) {
     using namespace brief;
+    // what the GEMMs of longer forwards ask of their operands: rows are read 16 bytes at a time
+    const void* rows[] = {p->wqkv, p->wo, p->wgu, p->wd, p->ln1, p->ln2, p->h, p->xn, p->qkv, p->attn, p->act};
+    for (const void* r : rows) if ((uintptr_t)r & 15) { set_error("prefill: weights, gains and activations must be 16-byte aligned"); return ITTAI_E_ARG; }
     const long long L = p->n_layers;
     const bool wide = p->tokens > kNarrowTokens;
     int rc = make_tmap_bf16(&m->qkv, p->wqkv, L * DQKV, D, D, Shape<kQkv, D>::kRows);

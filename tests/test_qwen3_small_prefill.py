@@ -100,3 +100,20 @@ def test_a_short_prompt_behind_a_cached_one(tiny_hf):
     for a, b in ((whole.kcache, pieces.kcache), (whole.vcache, pieces.vcache)):
         a, b = a[..., :150, :].float(), b[..., :150, :].float()
         assert torch.linalg.vector_norm(a - b) <= 9.3e-3 * torch.linalg.vector_norm(b)
+
+
+@pytest.mark.parametrize("tokens", [1, 32, 48])
+def test_short_forwards_refuse_misaligned_rows(tokens):
+    """Before anything is launched (CPU): an operand that the kernels read or write 16 bytes at a time lies eight bytes off."""
+    import ctypes as C
+    from ittai_b200 import _C
+    names = ("wqkv", "wo", "wgu", "wd", "ln1", "ln2", "h", "xn", "qkv", "attn", "act")
+    others = ("qn", "kn", "embed", "rope", "ids", "pos", "seq", "slot", "seqs", "kcache", "vcache", "stats", "zeros", "status")
+    for off in names:
+        p = _C.Qwen3Prefill()
+        p.n_layers, p.vocab, p.tokens, p.n_seqs, p.max_q_len, p.kv_cap, p.fused_rope, p.split_k = 1, 8, tokens, 1, tokens, 64, 1, 1
+        for i, name in enumerate(names + others):
+            setattr(p, name, 4096 * (i + 1) + (8 if name == off else 0))
+        assert _C.lib().ittai_qwen3_prefill_launch(C.byref(p), None) == -1, off
+        with pytest.raises(_C.IttaiError, match="16-byte"):
+            _C.check(-1)
