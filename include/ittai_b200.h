@@ -173,11 +173,11 @@ int ittai_qwen3_decode_launch_static(const IttaiQwen3Decode* p, void* stream);
  * read, not advanced. */
 int ittai_qwen3_phase_launch(const IttaiQwen3Decode* p, int phase, int layer, void* stream);
 
-/* The same decode as a chain of small kernels, one CUDA graph per token, for callers that keep a plan: same struct, same
+/* The same decode as a chain of small kernels, one CUDA graph per token or per four, for callers that keep a plan: same struct, same
  * results (the arithmetic and its rounding points are those of ittai_qwen3_decode_launch; sums run in another order).
  * `plan` owns the graphs, which are captured at the first token that needs each of them (a graph per cluster size
  * of the attention, with and without the head, with gate/up's tiles held in registers and not; 0.6 ms each where nothing
- * hides it) and again when a pointer or size of *p other than n_steps, n_forced, forced, out_ids, step_ns changes.
+ * hides it; those of four tokens, 2.4 to 3.3 ms, behind launches that keep the GPU busy meanwhile) and again when a pointer or size of *p other than n_steps, n_forced, forced, out_ids, step_ns changes.
  * `max_len`: an upper bound of pos[b] over the sequences.  It picks the cluster size and the gate/up kernel of a launch; a
  * sequence's results follow from its own length and `batch` alone, bit for bit.  p->phase_clk is not used.  An id or
  * position out of range ends in ITTAI_ST_BAD_TOKEN, a wait that runs out in ITTAI_ST_STREAM_TIMEOUT: the steps from there on store no id, `next_id` keeps the last good
@@ -337,7 +337,7 @@ typedef struct IttaiQwen3Prefill {
     int64_t kv_layer;      /* elements from one layer's store to the next (0: one store reused by every layer) */
     int64_t k_row, k_head, k_seq;  /* strides of the store, elements */
     int64_t kv_rows_total; /* rows of one layer's store */
-    void *h, *xn, *qkv, *attn, *act;  /* bf16 [T, 1024], [T, 1024], [T, 4096], [T, 2048], [T, 3072] */
+    void *h, *xn, *qkv, *attn, *act;  /* bf16 [T, 1024], [T, 1024], [T, 4096], [T, 2048], [T, 3072], 16-byte aligned */
     float* stats;          /* [T][8][2], used with folded norms and with split_k */
     const float* zeros;    /* [6144] zeros (the column sums of a folded RMSNorm), likewise */
     uint32_t* status;      /* as in IttaiGemm */
