@@ -205,7 +205,11 @@ __global__ void __launch_bounds__(kFewThreads) attn_few_kernel(const AttnArgs a,
     if (!seqs_ready) pdl_wait();
     const int4 sinfo = a.seqs[blockIdx.z];
     const int q_len = sinfo.y, kv_len = sinfo.w, qb = blockIdx.x * kFewRows;
-    if (qb >= q_len) return;
+    // an empty tile; a first one waits even so: behind a grid without any wait the next one would start ahead of what runs in front of this
+    if (qb >= q_len) {
+        if (seqs_ready && blockIdx.x == 0) pdl_wait();
+        return;
+    }
     const int head = blockIdx.y, kvh = head / a.group;
     const bf16* qp = a.q + (long long)(sinfo.x + qb) * a.q_row + (long long)head * a.q_head;
     const bf16* kp = a.k + (long long)blockIdx.z * a.k_seq + (long long)kvh * a.k_head + (long long)sinfo.z * a.k_row;

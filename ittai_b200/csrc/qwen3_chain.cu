@@ -1122,8 +1122,8 @@ static int enqueue_call(Plan* pl, const IttaiQwen3Decode& p, int max_len, bool c
             if (several) i = last;
             else if (head && queued < kSeveralAfter) ++queued;
             if (i + 1 >= p.n_steps && i + 1 >= kSeveralBehind && head && queued >= kSeveralAfter && s == nullptr && e == cudaSuccess) {
-                const int rc = capture(pl, cs, held, true, kSeveral, &s);
-                if (rc != ITTAI_OK) return rc;
+                // the call's work is queued: without this graph the next calls go on one by one, and it is tried again 64 tokens later
+                if (capture(pl, cs, held, true, kSeveral, &s) != ITTAI_OK) { cudaGetLastError(); queued = 0; }
             }
         }
         if (e != cudaSuccess) return cuda_fail(e, "launch of a decode step");
