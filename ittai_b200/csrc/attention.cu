@@ -4,6 +4,8 @@
 // K/V blocks streamed, scores and softmax in fp32 in the log2 domain, P rounded to bf16 for the PV product.
 // Tensor-core path: warp-level mma.sync m16n8k16 (bf16 in, fp32 accumulate) on ldmatrix fragments from swizzled
 // shared memory.  Attention is a few percent of SigLIP's FLOPs and a third of a 4k prefill's.
+#include <type_traits>
+
 #include "common.cuh"
 #include "launch.h"
 
@@ -182,29 +184,32 @@ __global__ void __launch_bounds__(WARPS * 32) attn_fwd_kernel(const AttnArgs a) 
     }
 }
 
-// Few queries (at most 64 a sequence), causal, head_dim 128: a short prompt.  One CTA per (sequence, head, 32 queries), two warps per 16 queries
-// that both compute the scores and share the output's 128 columns out; 32 keys a step, the next step's on their way meanwhile.  It runs once
-// per layer, so what attn_fwd_kernel spends here, its 64-key steps unrolled for keys that do not exist, is code to be fetched (see the
-// attention of qwen3_chain.cu) and masks.  Forwards of 3 / 8 / 23 / 32 / 33 / 48 / 64 tokens 431 / 455 / 612 / 721 / 729 / 787 / 953 us with it,
-// 375 / 401 / 557 / 664 / 695 / 759 / 923 with this one; 40 texts of 60 tokens 3136 and 3013, 130 of 40 5676 and 5612; 20 tokens behind 1000 / 8000
-// cached ones 1799 / 8477 and 1326 / 5835, 60 tokens 2339 / 10692 and 2221 / 10084.  (Above 64 the key-loop kernel on tcgen05 takes over.)
-constexpr int kFewMax = 64, kFewRows = 32, kFewKeys = 32, kFewThreads = 128;
+// Few queries (at most 64 a sequence), causal, head_dim 128: a short prompt.  One CTA per (sequence, head, ROWS queries), 32 keys a step, the next
+// step's on their way meanwhile.  It runs once per layer, so what attn_fwd_kernel spends here, its 64-key steps unrolled for keys that do not
+// exist, is code to be fetched (see the attention of qwen3_chain.cu) and masks.  ROWS = 32: two warps per 16 queries that both compute the scores
+// and share the output's 128 columns out, the shorter chain; ROWS = 64: a warp per 16 queries, half the loads and two thirds of the MMAs, where
+// there are more tiles than SMs.  A query's values are the same bits in both.  How the CTAs are spread over the SMs: attn_few_launch_rows.
+// Texts of 3 / 8 / 23 / 32 / 48 / 64 tokens through the embedder, us, attn_fwd_kernel and split-K GEMMs -> this and qwen3_short.cu's projections (the
+// latter up to 48 tokens): 693 / 702 / 737 / 803 / 898 / 996 -> 393 / 438 / 568 / 660 / 766 / 924.  (Above 64 the key-loop kernel on tcgen05 takes over.)
+constexpr int kFewMax = 64, kFewKeys = 32, kFewThreads = 128;
 __device__ __forceinline__ float ex2_ftz(float x) {
     float y;
     asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
     return y;
 }
+template <int ROWS>
 __global__ void __launch_bounds__(kFewThreads) attn_few_kernel(const AttnArgs a, int seqs_ready) {
-    constexpr int HD = 128;
+    constexpr int HD = 128, kShare = ROWS / 16 * 32 == kFewThreads ? 1 : 2, kCols = HD / kShare;   // warps that share 16 queries' columns out
+    static_assert(ROWS / 16 * kShare * 32 == kFewThreads, "");
     extern __shared__ __align__(128) unsigned char attn_smem[];
     bf16* sq = reinterpret_cast<bf16*>(attn_smem);
-    bf16* skv = sq + kFewRows * HD;                                   // [2][K | V][32 * HD]
+    bf16* skv = sq + ROWS * HD;                                   // [2][K | V][32 * HD]
     const int tid = threadIdx.x, warp = warp_index(), lane = tid & 31, g = lane >> 2, t = lane & 3;
     pdl_trigger();
     // With records that may be read ahead of the wait the addresses are there behind it: 400 of the kernel's 3200 cycles at 23 tokens.
     if (!seqs_ready) pdl_wait();
     const int4 sinfo = a.seqs[blockIdx.z];
-    const int q_len = sinfo.y, kv_len = sinfo.w, qb = blockIdx.x * kFewRows;
+    const int q_len = sinfo.y, kv_len = sinfo.w, qb = blockIdx.x * ROWS;
     // an empty tile; a first one waits even so: behind a grid without any wait the next one would start ahead of what runs in front of this
     if (qb >= q_len) {
         if (seqs_ready && blockIdx.x == 0) pdl_wait();
@@ -214,7 +219,7 @@ __global__ void __launch_bounds__(kFewThreads) attn_few_kernel(const AttnArgs a,
     const bf16* qp = a.q + (long long)(sinfo.x + qb) * a.q_row + (long long)head * a.q_head;
     const bf16* kp = a.k + (long long)blockIdx.z * a.k_seq + (long long)kvh * a.k_head + (long long)sinfo.z * a.k_row;
     const bf16* vp = a.v + (long long)blockIdx.z * a.v_seq + (long long)kvh * a.v_head + (long long)sinfo.z * a.v_row;
-    const int q_rows = q_len - qb < kFewRows ? q_len - qb : kFewRows;
+    const int q_rows = q_len - qb < ROWS ? q_len - qb : ROWS;
     const int shift = kv_len - q_len + qb;                            // row i of the tile sees keys j <= i + shift
     const int kv_end = q_rows + shift < kv_len ? q_rows + shift : kv_len;
     // thread: 16-byte piece tid % 16 of rows tid / 16 + 8 i
@@ -223,24 +228,24 @@ __global__ void __launch_bounds__(kFewThreads) attn_few_kernel(const AttnArgs a,
     long long q8 = 8 * a.q_row, k8 = 8 * a.k_row, v8 = 8 * a.v_row;
     asm volatile("" : "+l"(qt), "+l"(kt), "+l"(vt), "+l"(q8), "+l"(k8), "+l"(v8));
     // rows past the end: the first one's address, nothing read
-    auto load = [&](bf16* dst, const bf16* src, long long step, int rows) {
+    auto load = [&](bf16* dst, const bf16* src, long long step, int rows, auto pieces) {
 #pragma unroll
-        for (int i = 0; i < 4; ++i) cp_async16(dst + sw<HD>(lr + 8 * i, lc), lr + 8 * i < rows ? src + i * step : a.q, lr + 8 * i < rows);
+        for (int i = 0; i < decltype(pieces)::value; ++i) cp_async16(dst + sw<HD>(lr + 8 * i, lc), lr + 8 * i < rows ? src + i * step : a.q, lr + 8 * i < rows);
     };
     auto load_kv = [&](int kb, int buf) {
         bf16* dst = skv + (size_t)buf * 2 * kFewKeys * HD;
-        load(dst, kt, k8, kv_end - kb);
-        load(dst + kFewKeys * HD, vt, v8, kv_end - kb);
+        load(dst, kt, k8, kv_end - kb, std::integral_constant<int, kFewKeys / 8>());
+        load(dst + kFewKeys * HD, vt, v8, kv_end - kb, std::integral_constant<int, kFewKeys / 8>());
         kt += 4 * k8; vt += 4 * v8;
         asm volatile("cp.async.commit_group;" ::: "memory");
     };
     if (seqs_ready) pdl_wait();
-    load(sq, qt, q8, q_rows);
+    load(sq, qt, q8, q_rows, std::integral_constant<int, ROWS / 8>());
     if (kv_end > 0) load_kv(0, 0); else asm volatile("cp.async.commit_group;" ::: "memory");
-    const int rt = 16 * (warp >> 1), half = warp & 1;                 // this warp's 16 queries, and half of the output columns
-    float o[8][4];
+    const int rt = 16 * (warp / kShare), part = warp % kShare;        // this warp's 16 queries, and its share of the output columns
+    float o[kCols / 8][4];
 #pragma unroll
-    for (int i = 0; i < 8; ++i) o[i][0] = o[i][1] = o[i][2] = o[i][3] = 0.f;
+    for (int i = 0; i < kCols / 8; ++i) o[i][0] = o[i][1] = o[i][2] = o[i][3] = 0.f;
     float m0 = -INFINITY, m1 = -INFINITY, l0 = 0.f, l1 = 0.f;         // rows g and g + 8
     const int r0 = rt + g, r1 = r0 + 8;
     int buf = 0;
@@ -292,13 +297,13 @@ __global__ void __launch_bounds__(kFewThreads) attn_few_kernel(const AttnArgs a,
         }
         l0 = l0 * c0 + p0; l1 = l1 * c1 + p1;
 #pragma unroll
-        for (int i = 0; i < 8; ++i) { o[i][0] *= c0; o[i][1] *= c0; o[i][2] *= c1; o[i][3] *= c1; }
+        for (int i = 0; i < kCols / 8; ++i) { o[i][0] *= c0; o[i][1] *= c0; o[i][2] *= c1; o[i][3] *= c1; }
 #pragma unroll
         for (int ks = 0; ks < 2; ++ks)
 #pragma unroll
-            for (int dp = 0; dp < 4; ++dp) {
+            for (int dp = 0; dp < kCols / 16; ++dp) {
                 uint32_t vf[4];
-                ldsm_x4_t(vf, sv + sw<HD>(ks * 16 + (lane & 7) + ((lane >> 3) & 1) * 8, 8 * half + dp * 2 + (lane >> 4)));
+                ldsm_x4_t(vf, sv + sw<HD>(ks * 16 + (lane & 7) + ((lane >> 3) & 1) * 8, kCols / 8 * part + dp * 2 + (lane >> 4)));
                 mma16816(o[2 * dp], pf[ks], vf[0], vf[1]);
                 mma16816(o[2 * dp + 1], pf[ks], vf[2], vf[3]);
             }
@@ -307,9 +312,9 @@ __global__ void __launch_bounds__(kFewThreads) attn_few_kernel(const AttnArgs a,
     l0 += __shfl_xor_sync(0xffffffffu, l0, 1); l0 += __shfl_xor_sync(0xffffffffu, l0, 2);
     l1 += __shfl_xor_sync(0xffffffffu, l1, 1); l1 += __shfl_xor_sync(0xffffffffu, l1, 2);
     const float i0 = l0 > 0.f ? 1.0f / l0 : 0.f, i1 = l1 > 0.f ? 1.0f / l1 : 0.f;
-    bf16* op = a.o + (long long)(sinfo.x + qb) * a.o_row + (long long)head * a.o_head + 64 * half + 2 * t;
+    bf16* op = a.o + (long long)(sinfo.x + qb) * a.o_row + (long long)head * a.o_head + kCols * part + 2 * t;
 #pragma unroll
-    for (int i = 0; i < 8; ++i) {
+    for (int i = 0; i < kCols / 8; ++i) {
         if (r0 < q_rows) *reinterpret_cast<uint32_t*>(op + (long long)r0 * a.o_row + 8 * i) = pack_bf16x2(o[i][0] * i0, o[i][1] * i0);
         if (r1 < q_rows) *reinterpret_cast<uint32_t*>(op + (long long)r1 * a.o_row + 8 * i) = pack_bf16x2(o[i][2] * i1, o[i][3] * i1);
     }
@@ -547,6 +552,43 @@ static int attn_launch(const AttnArgs& a, int max_q_len, int n_heads, int n_seqs
     return 0;
 }
 
+// A CTA asks for so much shared memory that an SM takes no more of them than its even share: they start while the kernel in front holds most SMs, and
+// without that the empty ones filled up (five on an SM), which a long cache then paid for.  16 heads, one layer, us, attn_fwd_kernel / packed / spread:
+// 16 sequences of 16 queries behind 1000 cached keys 39 / 51 / 31, four of 64 45 / 36 / 24.  Forwards of 28 layers, us: 4 x 2 tokens behind 7900 cached
+// ones 8640 / 11 340 / 5650, 8 x 5 behind 1000 2010 / 2270 / 1570; texts of 40 and 64 tokens 874 / 756 / 732 and 996 / 940 / 921.
+template <int ROWS>
+static cudaError_t attn_few_launch_rows(const AttnArgs& a, int max_q_len, int n_heads, int n_seqs, int seqs_ready, int n_sms, cudaStream_t st) {
+    constexpr int kNeed = (ROWS + 4 * kFewKeys) * 128 * 2, kSm = 228 * 1024, kLone = kSm / 2 + 128;
+    static thread_local int attr_dev = -1;
+    int dev = 0;
+    cudaGetDevice(&dev);
+    if (attr_dev != dev) {
+        const cudaError_t e = cudaFuncSetAttribute(attn_few_kernel<ROWS>, cudaFuncAttributeMaxDynamicSharedMemorySize, kLone);
+        if (e != cudaSuccess) return e;
+        attr_dev = dev;
+    }
+    const dim3 grid((max_q_len + ROWS - 1) / ROWS, n_heads, n_seqs);
+    const long long per_sm = ((long long)grid.x * grid.y * grid.z + n_sms - 1) / n_sms;
+    const int room = kSm / (int)(per_sm < 8 ? per_sm + 1 : 9) - 1024 + 128;        // per_sm + 1 of them, with 1 KB each for the system, do not fit
+    return launch_pdl(attn_few_kernel<ROWS>, grid, dim3(kFewThreads), (size_t)(room > kNeed ? room : kNeed), st, 1, a, seqs_ready);
+}
+static cudaError_t attn_few_launch(const AttnArgs& a, int max_q_len, int n_heads, int n_seqs, int seqs_ready, cudaStream_t st) {
+    static thread_local int sm_dev = -1, n_sms = 0;
+    int dev = 0;
+    cudaGetDevice(&dev);
+    if (sm_dev != dev) {
+        const cudaError_t e = cudaDeviceGetAttribute(&n_sms, cudaDevAttrMultiProcessorCount, dev);
+        if (e != cudaSuccess) return e;
+        sm_dev = dev;
+    }
+    // More tiles of 32 queries than SMs: tiles of 64, if there are so many queries.  One layer, us, attn_fwd_kernel / tiles of 32 / of 64: 64 sequences of
+    // 33 queries behind 1000 keys 180 / 187 / 121, of 64 behind 100 42 / 41 / 29, five (160 tiles of 32) of 33 behind 1000 44 / 32 / 25; but four (128)
+    // 44 / 23.6 / 24.5.
+    const bool whole = max_q_len > 32 && 2ll * n_heads * n_seqs > n_sms;
+    return whole ? attn_few_launch_rows<64>(a, max_q_len, n_heads, n_seqs, seqs_ready, n_sms, st)
+                 : attn_few_launch_rows<32>(a, max_q_len, n_heads, n_seqs, seqs_ready, n_sms, st);
+}
+
 void set_error(const char* fmt, ...);
 int cuda_fail(cudaError_t e, const char* what);
 bool attn_tc_supported(const IttaiAttention* p);          // attention_sm100.cu
@@ -588,7 +630,7 @@ static int ittai::attention_launch(const IttaiAttention* p, bool disjoint, cudaS
         return e1 == cudaSuccess ? ITTAI_OK : cuda_fail(e1, "launch attn_q1_kernel");
     }
     if (p->head_dim == 128 && p->causal && ql <= kFewMax) {
-        const cudaError_t e1 = launch_pdl(attn_few_kernel, dim3((ql + kFewRows - 1) / kFewRows, nh, ns), dim3(kFewThreads), (size_t)(kFewRows + 4 * kFewKeys) * 128 * 2, st, 1, a, p->seqs_ready);
+        const cudaError_t e1 = attn_few_launch(a, ql, nh, ns, p->seqs_ready, st);
         return e1 == cudaSuccess ? ITTAI_OK : cuda_fail(e1, "launch attn_few_kernel");
     }
     if (p->head_dim == 128) rc = p->causal ? attn_launch<128, true, 4>(a, ql, nh, ns, st) : attn_launch<128, false, 4>(a, ql, nh, ns, st);
