@@ -39,7 +39,7 @@ constexpr uint32_t kTmemCols = 512;
 
 template <int TN, int STAGES>
 __global__ void __launch_bounds__(kGemmThreads, 1)
-gemm_bf16_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant__ CUtensorMap tm_b, const GemmArgs g, const int box_a) {
+gemm_bf16_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant__ CUtensorMap tm_b, const GemmArgs g, const int box_a, const int ahead) {
     extern __shared__ __align__(1024) unsigned char gsm_raw[];
     unsigned char* gsm = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(gsm_raw) + 1023) & ~(uintptr_t)1023);
     unsigned char* sa = gsm;                                         // [stages][128 rows][128 B]
@@ -69,11 +69,11 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
-    // W as far as L2, an even share for every CTA, in the order of use: 16 CTAs that read 400 KB of weights each from HBM in 64 KB pieces wait for
-    // its latency.  Prefill of 17 / 58 / 120 / 139 / 442 tokens in one order of sums 1490 / 1490 / 1547 / 1955 / 2077 -> 1442 / 1407 / 1453 / 1912 / 2049 us.
-    // (In the pair and the split-K kernel: no change.)
+    // W as far as L2 (`ahead` boxes of it, none or all), an even share for every CTA, in the order of use: 16 CTAs that read 400 KB of weights each from
+    // HBM in 64 KB pieces wait for its latency.  Prefill of 17 / 58 / 120 / 139 / 442 tokens in one order of sums 1490 / 1490 / 1547 / 1955 / 2077 ->
+    // 1442 / 1407 / 1453 / 1912 / 2049 us.  (In the pair and the split-K kernel: no change.)
     if (warp == 0 && elect_one()) {
-        for (int i = blockIdx.x; i < tiles_n * n_kb; i += gridDim.x) tma_prefetch_2d(&tm_b, i / tiles_n * GK, i % tiles_n * TN);
+        for (int i = blockIdx.x; i < ahead; i += gridDim.x) tma_prefetch_2d(&tm_b, i / tiles_n * GK, i % tiles_n * TN);
     }
     __syncwarp();
     pdl_wait();                                                      // operands come from the kernels before this one
@@ -272,7 +272,13 @@ int gemm_bf16_launch(const IttaiGemm* a, cudaStream_t st, const void* a_gain) {
         attr_dev = dev;
     }
     const int tiles = ((a->m + GM - 1) / GM) * (a->n / 64);
-    const cudaError_t e = launch_pdl(gemm_bf16_kernel<64, 8>, dim3(tiles < n_sms ? tiles : n_sms), dim3(kGemmThreads), GemmCfg<64, 8>::kSmem, st, 1, tm_a, tm_b, g, box_a);
+    // W is brought into L2 ahead of the wait where it is at most 16 MiB and K at most 3072: a longer one keeps HBM busy by itself and then waits behind
+    // its own requests, and one beyond L2 is read twice.  M 128, W from HBM, us, without / with: N 1024 K 2048 8.1 / 7.4, N 4096 K 1024 5.9 / 5.2 and K 2048
+    // (on the line) 8.5 / 7.6, N 1024 K 3072 10.6 / 10.3 (M 442 10.4 / 9.6); beyond it N 2048 K 4096 13.2 / 13.8, N 4096 K 4096 14.2 / 15.7, N 8192 K 1536 and
+    // 2048 8.1 / 8.1 and 9.8 / 10.3, N 16384 K 4096 31.8 / 38.3, N 151808 K 1024 71.7 / 83.6 (N 12288 K 1024, 10.8 / 9.4, would gain).
+    const bool prefetch = g.K <= 3072 && (long long)g.N * g.K <= 8 << 20;
+    const cudaError_t e = launch_pdl(gemm_bf16_kernel<64, 8>, dim3(tiles < n_sms ? tiles : n_sms), dim3(kGemmThreads), GemmCfg<64, 8>::kSmem, st, 1, tm_a, tm_b, g, box_a,
+                                     prefetch ? g.N / 64 * (g.K / GK) : 0);
     return e == cudaSuccess ? ITTAI_OK : cuda_fail(e, "launch gemm_bf16_kernel");
 }
 

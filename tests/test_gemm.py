@@ -72,6 +72,44 @@ def test_short_tiles_load_only_their_rows(m):
 
 
 @gpu
+@pytest.mark.parametrize("n,k", [(4096, 2048), (4352, 2048), (256, 3072), (256, 3136), (16384, 512), (151808, 64)])
+def test_weights_ahead_of_the_wait_and_not(n, k):
+    """Both sides of the lines up to which the one-SM kernel brings W into L2 first (16 MiB, K 3072), behind a launch that writes nothing of it."""
+    from ittai_b200 import ops
+    a, w = _rand(70, k, seed=64), _rand(n, k, scale=0.05, seed=65)
+    st = ops.new_status("cuda")
+    for m in (70, 5):
+        _check(ops.gemm(a[:m], w, st), a[:m].float() @ w.float().T, f"W {n} x {k}, {m} rows")
+    ops.check_status(st)
+
+
+@gpu
+def test_a_weight_beyond_l2_streams_at_the_rate_of_memory():
+    """537 MB of weights for 64 rows: 1.2 times as long as a copy that moves as many bytes.  (Requested as a whole ahead of its use, 1.5 times.)"""
+    from ittai_b200 import ops
+    a, w = _rand(64, 4096, seed=66), torch.zeros(65536, 4096, dtype=torch.bfloat16, device="cuda")
+    half = w.numel() // 2
+    src, dst = torch.zeros(2, half, dtype=torch.bfloat16, device="cuda")
+    st, out = ops.new_status("cuda"), torch.empty(64, 65536, dtype=torch.bfloat16, device="cuda")
+
+    def us(call):
+        times = []
+        for _ in range(9):
+            e = [torch.cuda.Event(enable_timing=True) for _ in range(2)]
+            e[0].record()
+            for _ in range(5):
+                call()
+            e[1].record()
+            torch.cuda.synchronize()
+            times.append(e[0].elapsed_time(e[1]) * 200)
+        return sorted(times)[4]
+
+    copy = us(lambda: dst.copy_(src))
+    assert us(lambda: ops.gemm(a, w, st, out=out)) < 1.38 * copy, copy
+    ops.check_status(st)
+
+
+@gpu
 def test_gemm_row_identity():
     """A = rows of the identity picks out columns of W: catches a wrong swizzle or K-step in the operand descriptors."""
     from ittai_b200 import ops
