@@ -209,6 +209,8 @@ class Qwen3Decoder:
             ids = ids[None]
         assert ids.shape[0] == self.B, "one prompt per sequence of the batch"
         T = ids.shape[1]
+        if T < 1:                                                # ahead of the launch: further steps alone would go on from the id of an earlier call
+            raise _C.IttaiError("an empty prompt")
         if tensor_cores is None:
             tensor_cores = T >= 32
         if tensor_cores and T > 1:

@@ -54,3 +54,22 @@ def test_embedder_batches_respect_both_limits():
     assert list(e._batches([])) == []
     with pytest.raises(ValueError):
         list(e._batches([3, 11]))
+
+
+def test_an_empty_prompt_is_refused_ahead_of_any_launch():
+    """``prefill`` and ``generate`` of no tokens, on a decoder that has served a prompt before and still holds its last id."""
+    import pytest
+    from ittai_b200 import _C
+    from ittai_b200.qwen3.decoder import Qwen3Decoder
+    for batch in (1, 2):
+        d = Qwen3Decoder.__new__(Qwen3Decoder)
+        d.B, d.cap, d.dev = batch, 64, torch.device("cpu")
+        d.pos, d.next_id, d.lengths, d._unchecked = torch.full((batch,), 9), torch.full((batch,), 5), [9] * batch, 0
+        launched = []
+        d._launch = lambda n, **kw: launched.append(n) or (torch.zeros(n, batch, dtype=torch.int32), None)
+        empty = torch.zeros(batch, 0, dtype=torch.int32)
+        for call in (lambda: d.generate(empty, 8), lambda: d.generate(empty, 1), lambda: d.prefill(empty), lambda: d.prefill(empty, tensor_cores=True)):
+            with pytest.raises(_C.IttaiError):
+                call()
+        assert launched == []
+        assert d.generate(torch.zeros(batch, 3, dtype=torch.int32), 4).shape == (batch, 4) and launched == [6]
