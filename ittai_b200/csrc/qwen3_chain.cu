@@ -1098,6 +1098,7 @@ static int capture(Plan* pl, int cs, bool held, bool head, int tokens, cudaGraph
 // Everything one call queues on `st`.
 static int enqueue_call(Plan* pl, const IttaiQwen3Decode& p, int max_len, bool captured, cudaStream_t st) {
     enqueue_begin(*pl, p, st);
+    bool refused = false;                              // a graph of several tokens could not be had in this call: it goes on with those of one
     for (int i = 0; i < p.n_steps; ++i) {
         const bool head = i >= p.n_forced - 1;
         const int cs = pieces(p.batch, max_len + i);
@@ -1112,16 +1113,17 @@ static int enqueue_call(Plan* pl, const IttaiQwen3Decode& p, int max_len, bool c
             const bool same = head && last < p.n_steps && pieces(p.batch, len) == cs && hold_tiles(p.batch, len) == held;
             cudaGraphExec_t& s = pl->several[slot][held ? 1 : 0];
             int& queued = pl->queued[slot][held ? 1 : 0];
-            const bool several = same && (s != nullptr || i >= kSeveralInCall);
+            if (same && s == nullptr && i >= kSeveralInCall && !refused && capture(pl, cs, held, head, kSeveral, &s) != ITTAI_OK) { cudaGetLastError(); refused = true; }
+            const bool several = same && s != nullptr;
             cudaGraphExec_t& x = several ? s : pl->exec[slot][held ? 1 : 0][head ? 1 : 0];
             if (x == nullptr) {
-                const int rc = capture(pl, cs, held, head, several ? kSeveral : 1, &x);
+                const int rc = capture(pl, cs, held, head, 1, &x);
                 if (rc != ITTAI_OK) return rc;
             }
             e = cudaGraphLaunch(x, st);
             if (several) i = last;
             else if (head && queued < kSeveralAfter) ++queued;
-            if (i + 1 >= p.n_steps && i + 1 >= kSeveralBehind && head && queued >= kSeveralAfter && s == nullptr && e == cudaSuccess) {
+            if (i + 1 >= p.n_steps && i + 1 >= kSeveralBehind && head && queued >= kSeveralAfter && s == nullptr && !refused && e == cudaSuccess) {
                 // the call's work is queued: without this graph the next calls go on one by one, and it is tried again 64 tokens later
                 if (capture(pl, cs, held, true, kSeveral, &s) != ITTAI_OK) { cudaGetLastError(); queued = 0; }
             }
