@@ -189,8 +189,8 @@ __global__ void __launch_bounds__(WARPS * 32) attn_fwd_kernel(const AttnArgs a) 
 // exist, is code to be fetched (see the attention of qwen3_chain.cu) and masks.  ROWS = 32: two warps per 16 queries that both compute the scores
 // and share the output's 128 columns out, the shorter chain; ROWS = 64: a warp per 16 queries, half the loads and two thirds of the MMAs, where
 // there are more tiles than SMs.  A query's values are the same bits in both.  How the CTAs are spread over the SMs: attn_few_launch_rows.
-// Texts of 3 / 8 / 23 / 32 / 48 / 64 tokens through the embedder, us, attn_fwd_kernel and split-K GEMMs -> this and qwen3_short.cu's projections (the
-// latter up to 48 tokens): 693 / 702 / 737 / 803 / 898 / 996 -> 393 / 438 / 568 / 660 / 766 / 924.  (Above 64 the key-loop kernel on tcgen05 takes over.)
+// Forwards of 3 / 8 / 23 / 32 / 48 / 64 tokens with split-K projections, us, attn_fwd_kernel -> this: 627 / 637 / 669 / 737 / 834 / 927 -> 555 / 568 /
+// 602 / 671 / 769 / 852; 40 texts of 60 tokens 3086 -> 2937, 130 of 40 5574 -> 5440.  (Above 64 the key-loop kernel on tcgen05 takes over.)
 constexpr int kFewMax = 64, kFewKeys = 32, kFewThreads = 128;
 __device__ __forceinline__ float ex2_ftz(float x) {
     float y;

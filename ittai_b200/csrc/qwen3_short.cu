@@ -12,17 +12,18 @@
 //   weights in mma.sync m16n8k16: 32 rows x one K chunk x 8 NT tokens a warp.
 // * Chunks meet in shared memory, quarters through st.async, 16 bytes at a time, in the CTA that finishes the token (token n: rank n mod 4,
 //   where a warp or eight lanes hold a whole row piece for the head norm, the rotation or the statistics); sums in the order of chunks, then
-//   of ranks from the last one on (as good as any: against the eager module's 64 tokens behind a prompt of 32, which near-ties decide, the orders
-//   0 1 2 3 / 3 2 1 0 / chunks in pairs agree in 60 / 62 / 62, at an rms distance of 9.5e-3 / 9.5e-3 / 9.4e-3, the split-K GEMMs in 62 at 10.0e-3;
-//   pairs cost 4 % at 17 to 24 tokens).
+//   of ranks from the last one on.  No order is the better one: against the eager module's 64 tokens behind a prompt of 32, which near-ties decide,
+//   0 1 2 3 / 3 2 1 0 / chunks in pairs agree in 60 / 62 / 62, at an rms distance of 9.5e-3 / 9.5e-3 / 9.4e-3, the split-K GEMMs in 62 at 10.0e-3; the
+//   test of that fixture asks for 61, which the ascending order misses and this one does not (pairs cost 4 % at 17 to 24 tokens).  Over many
+//   prompts, against 64 bits, the error is that of the kernels before (700 prompts of 47 and 31 more tokens: logits +0.01 +- 0.15 %).
 //
-// Measured on a B200, a forward of 3 / 8 / 16 / 23 / 32 tokens, us, split-K GEMMs and attn_fwd_kernel -> this and attn_few_kernel:
-// 640 / 649 / 671 / 682 / 749 -> 345 / 357 / 438 / 515 / 604.  What grows with the tokens are the MMAs (legacy ones: 8 cycles each, 1150
+// Measured on a B200, a forward of 3 / 8 / 16 / 23 / 32 tokens with attn_few_kernel, us, split-K GEMMs -> this: 555 / 568 / 587 / 602 / 671 ->
+// 328 / 345 / 420 / 504 / 584.  What grows with the tokens are the MMAs (legacy ones: 8 cycles each, 1150
 // of gate/up's 5800 cycles at 23 tokens), the sums' way through shared memory and the activations, which 32 CTAs read from the same lines of
-// L2.  Other forms, us at 3 / 23 / 32 tokens: weights from shared memory as the 128-row operand of tcgen05.mma, everything else alike 455 /
-// 582 / 618; tokens as the 128-row operand in tensor memory 603 / 692 / 744 (padded rows cost what real ones do: 54 cycles an MMA of 128
-// columns); one kernel for all four projections, its sizes arguments 528 / 654 / 697; QKV in 16 warps of 64 registers instead of 8 of 128
-// (their sums meet in four chunks instead of two) 369 / 554 / 666.
+// L2.  Other forms while they were built, us at 3 / 23 / 32 tokens, when this took 365 / 534 / 620: weights from shared memory as the 128-row operand of
+// tcgen05.mma, everything else alike 455 / 582 / 618; tokens as the 128-row operand in tensor memory 603 / 692 / 744 (padded rows cost what real
+// ones do: 54 cycles an MMA of 128 columns); one kernel for all four projections, its sizes arguments 528 / 654 / 697; QKV in 16 warps of 64
+// registers instead of 8 of 128 (their sums meet in four chunks instead of two) 369 / 554 / 666.
 #include <cuda.h>
 
 #include "gemm2_common.cuh"
@@ -59,11 +60,13 @@ struct Plan {
     static constexpr uint32_t kX = kW > kPart ? kW : kPart;                          // offset: the sums of the chunks take the place of the weights
     static constexpr uint32_t kRecv = (kX + 8 * NT * S::kXLd + 127) / 128 * 128;     // offset: [ranks][2 NT tokens][rows] sums of the quarters
     static constexpr uint32_t kNeed = kRecv + kRanks * 2 * NT * S::kRows * 4 + 1024;
-    // Asked for, whether needed or not.  A kernel starts while the one in front holds 128 of the 148 SMs: what fits three times on an SM goes to
-    // the empty ones by threes, and the slowest CTA is what the next kernel waits for.  O-proj with room for one or two: forwards of 9 / 16 / 23 /
-    // 32 tokens, us, as little as needed 422 / 455 / 553 / 611, 76 KB 424 / 447 / 526 / 613, this 416 / 438 / 515 / 604 (of which for 32 tokens the QKV
-    // projection's one a SM); one a SM throughout 428 / 491 / 566 / 641, gate/up then finds no room beside it.  Up to 8 tokens every form lost 2 to 10 %.
-    static constexpr uint32_t kAtLeast = NT == 1 ? 0 : EPI == kQkv ? (NT == 4 ? 114 << 10 : 0) : EPI == kResidual && K == DQ ? (NT == 2 ? 106 << 10 : NT == 3 ? 98 << 10 : 86 << 10) : 0;
+    // Asked for, whether needed or not, from 9 tokens on: O-proj so much that an SM takes two of its CTAs and nothing beside them, QKV (25 to 32 tokens)
+    // so much that it takes one.  A kernel starts while the one in front holds 128 of the 148 SMs: what fits three times on an SM goes to the empty
+    // ones by threes, and the slowest CTA is what the next kernel waits for.  Texts of 12 / 16 / 23 / 32 tokens through the embedder, us, O-proj as
+    // little as needed 484 / 496 / 605 / 657, two and 74 KB (76 KB each) beside them 485 / 498 / 576 / 659, this and 106 KB 474 / 487 / 566 / 655, one a SM
+    // 533 / 545 / 616 / 672: gate/up then finds no room beside it.  QKV as little as needed, 32 tokens in one and three texts 666 and 661, this 657 and
+    // 639; at 9 and 16 tokens 3 and 1 % slower.  Up to 8 tokens every form lost 2 to 10 %.
+    static constexpr uint32_t kAtLeast = EPI == kQkv && NT == 4 ? 114 << 10 : EPI == kResidual && K == DQ && NT > 1 ? 98 << 10 : 0;
     static constexpr uint32_t kSmem = kNeed > kAtLeast ? kNeed : kAtLeast;
 };
 
@@ -345,8 +348,9 @@ __global__ void __launch_bounds__(Shape<EPI, K>::kThreads, 2) proj_kernel(const 
 // The same flow on tcgen05, whose MMA costs the same 40 cycles for 16 and for 64 tokens (it is the weights' 4 KB a step, read out of shared memory,
 // that take them): weights as the 128-row operand, activations normalised in registers on the way to where the MMA reads them, the
 // accumulator through shared memory, so that a token's sums lie side by side.  A cluster of eight shares the K of O and down (64 rows a CTA).
-// Forwards of 33 / 40 / 48 / 64 tokens, us: split-K GEMMs 816 / 821 / 860 / 957, this 729 / 755 / 787 / 986 (up to 32 tokens see the top of the
-// file).  Hence the line at 48: beyond, gate/up's shared memory leaves no room for its neighbours'.
+// Forwards of 33 / 40 / 48 tokens with attn_few_kernel, us: split-K GEMMs 725 / 742 / 769, this 649 / 679 / 710 (up to 32 tokens see the top of the
+// file).  The line at 48: an instantiation for 64 tokens, whose gate/up leaves no room in shared memory for its neighbours, took 986 against 957
+// when it was tried.  Sums of the ranks in ascending order.
 constexpr int kWideThreads = 256;
 template <int TN, int EPI, int K>
 struct WideShape {
@@ -662,7 +666,7 @@ int short_maps(ShortMaps* m, const IttaiQwen3Prefill* p) {
     return rc;
 }
 
-static int done(cudaError_t e) { return e == cudaSuccess ? ITTAI_OK : cuda_fail(e, "launch proj_kernel"); }
+static int done(cudaError_t e) { return e == cudaSuccess ? ITTAI_OK : cuda_fail(e, "launch of a short projection"); }
 
 int short_qkv(const ShortMaps& m, const IttaiQwen3Prefill* p, int layer, const IttaiQkRope& r, const void* gain, const float* stats, cudaStream_t st) {
     brief::Args a{(const bf16*)p->h, (const bf16*)gain, stats, (bf16*)p->qkv, nullptr, nullptr, p->tokens, layer * brief::DQKV, p->eps, p->status, r};

@@ -1,5 +1,5 @@
-"""CTAs of a cluster that send partials into one another's shared memory (``csrc/gemm_split_sm100.cu``, ``csrc/qwen3_chain.cu``): none may
-leave while another can still write to it, also where waits run out.  A host model of the roles; no wait is made to run out on a GPU
+"""CTAs of a cluster that send partials into one another's shared memory (``csrc/gemm_split_sm100.cu``, ``csrc/qwen3_chain.cu`` and both kernels of
+``csrc/qwen3_short.cu``): none may leave while another can still write to it, also where waits run out.  A host model of the roles; no wait is made to run out on a GPU
 for it (CPU)."""
 import os
 import random
@@ -67,7 +67,7 @@ def _block(text, start):
 
 
 @pytest.mark.parametrize("source,failure", [("gemm_split_sm100.cu", "if (*abort_flag) {"), ("qwen3_chain.cu", "if (failed) {"),
-                                            ("qwen3_short.cu", "if (!__syncthreads_and(ok && came)) {")])
+                                            ("qwen3_short.cu", "if (!__syncthreads_and(ok && came)) {"), ("qwen3_short.cu", "if (failed) {")])
 def test_the_kernels_follow_the_model(source, failure):
     """In the branch of a CTA that gave up: the wait for the bytes, the barrier behind it, and then the time for copies in flight."""
     with open(os.path.join(CSRC, source)) as f:

@@ -188,3 +188,26 @@ def test_several_tokens_a_graph_are_the_tokens_one_by_one(tiny_hf, batch, length
     for call in ([steps], [steps], [17, steps - 17], [steps - 2, 2]):
         for got, ref in zip(run(call), want):
             assert torch.equal(got, ref), call
+
+
+@gpu
+@pytest.mark.parametrize("batch,length", [(1, 20), (8, 500)])
+def test_the_graph_captured_behind_short_calls_is_the_tokens_one_by_one(tiny_hf, batch, length):
+    """A request loop's calls of eight steps: single tokens until 64 of a kind are queued, then a graph of four, captured behind a call (the host
+    side: test_qwen3_chain_host.py).  Ids, logits and cache rows are those of calls of one step."""
+    from ittai_b200.qwen3 import Qwen3Decoder
+    model, dims = tiny_hf
+    g = torch.Generator().manual_seed(11 * batch)
+    steps, kv, got = 96, None, []
+    ids = torch.randint(0, dims.vocab, (batch,), generator=g, dtype=torch.int32)
+    for call in (8, 1):
+        d = Qwen3Decoder(model, max_batch=batch, kv_capacity=640)
+        kv = kv or [(torch.randn(d.kcache.shape, generator=g) * s).to(torch.bfloat16) for s in (1.0, 0.5)]
+        for c, t in zip((d.kcache, d.vcache), kv):
+            c.copy_(t)
+        d.rewind(length)
+        d.next_id.copy_(ids)
+        out = torch.cat([d.decode(call).clone() for _ in range(steps // call)], 1)
+        got.append((out, d.logits.clone(), d.pos.clone(), d.kcache[:, :, :, :length + steps].clone(), d.vcache[:, :, :, :length + steps].clone()))
+    for a, b in zip(*got):
+        assert torch.equal(a, b)

@@ -247,6 +247,34 @@ def test_full_model_config1(full_hf, golden_dir):
 
 
 @gpu
+def test_short_prompts_against_wide_arithmetic(full_hf):
+    """Twenty prompts whose first 1 to 48 tokens take the projections of short forwards, at full depth, against the eager module in 64 bits (norms and
+    softmax in 32).  Judged is the distance of the logits, which near-ties do not decide: at most what 28 layers of eight bf16 roundings
+    amount to, sqrt(28 * 8) * 1.1e-3 = 1.7e-2 of the logits' norm, and half as much again for one prompt; over all of them no more than the
+    prompts fed through the decode steps (the paired difference scatters by 4 % a prompt, 1 % over twenty: 5 %).  The choice may differ
+    only where the two best are a tie."""
+    import copy
+    from ittai_b200.qwen3 import Qwen3Decoder
+    wide = copy.deepcopy(full_hf).to("cuda", torch.float64)
+    d = Qwen3Decoder(full_hf, max_batch=1, kv_capacity=64)
+    err = {True: [], False: []}
+    for i, n in enumerate((2, 3, 4, 6, 8, 9, 12, 16, 17, 20, 23, 25, 28, 32, 33, 34, 37, 41, 45, 49)):
+        ids = hf.prompt_ids(n, seed=500 + i)
+        with torch.no_grad():
+            want = wide(ids[None].long().cuda()).logits[0, -1].double()
+        gap = float(want.topk(2).values.diff().abs())
+        for dense in err:
+            d.reset()
+            first = int(d.prefill(ids, tensor_cores=dense)[0])
+            got = d.logits[0].double()
+            err[dense].append(float((got - want).norm() / want.norm()))
+            assert first == int(got.argmax()) and (first == int(want.argmax()) or gap <= TIE_GAP), (n, dense, gap)
+    mean = {k: sum(v) / len(v) for k, v in err.items()}
+    print({k: (round(mean[k], 6), round(max(v), 6)) for k, v in err.items()})
+    assert max(err[True]) <= 1.5 * 1.7e-2 and mean[True] <= 1.05 * mean[False], (mean, err)
+
+
+@gpu
 def test_long_context_against_eager_on_device(full_hf, golden_dir):
     """BASELINE config 2 shape: 4096-id prompt (seed 1), capacity 8192, then teacher-forced steps; the checker is the
     eager model run on the same GPU.  The max-abs gate is the distance between the eager model's own variants recorded

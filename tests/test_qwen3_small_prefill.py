@@ -87,6 +87,21 @@ def test_short_forwards_match_the_split_gemms(tiny_hf, lens):
 
 
 @gpu
+def test_a_short_text_does_not_depend_on_the_others(tiny_hf):
+    """Up to 32 tokens: the order of every sum is the same whatever tile a token lies in, so a text's embedding is the same bits alone and
+    packed with others (tiles of 8 to 32 tokens; attention of its own rows)."""
+    from ittai_b200.qwen3 import Engine
+    model, dims = tiny_hf
+    eng = Engine(model.state_dict(), 128, 32)
+    for lens in ([3, 5], [7, 9, 1], [8, 16], [9, 23], [31, 1], [2, 30], [1] * 32, [16, 15, 1]):
+        ids = [hf.prompt_ids(n, seed=40 + n + i, vocab=dims.vocab).tolist() for i, n in enumerate(lens)]
+        together = eng.forward(ids).clone()
+        for i, text in enumerate(ids):
+            assert torch.equal(eng.forward([text])[0], together[i]), (lens, i)
+    eng.check()
+
+
+@gpu
 def test_a_short_prompt_behind_a_cached_one(tiny_hf):
     """The attention of few queries, one tile of 32 or two, with cached keys in front of them: a prompt appended in pieces against the prompt
     at once (keys and values of two layers: the bound above)."""
