@@ -337,7 +337,8 @@ typedef struct IttaiQwen3Prefill {
     int64_t kv_layer;      /* elements from one layer's store to the next (0: one store reused by every layer) */
     int64_t k_row, k_head, k_seq;  /* strides of the store, elements */
     int64_t kv_rows_total; /* rows of one layer's store */
-    void *h, *xn, *qkv, *attn, *act;  /* bf16 [T, 1024], [T, 1024], [T, 4096], [T, 2048], [T, 3072], 16-byte aligned */
+    void *h, *xn, *qkv, *attn, *act;  /* bf16 [T, 1024], [T, 1024], [T, 4096], [T, 2048], [T, 3072], 16-byte aligned; all scratch but h
+                              (xn holds normalised rows or, in short forwards, fp32 sums of squares) */
     float* stats;          /* [T][8][2], used with folded norms and with split_k */
     const float* zeros;    /* [6144] zeros (the column sums of a folded RMSNorm), likewise */
     uint32_t* status;      /* as in IttaiGemm */

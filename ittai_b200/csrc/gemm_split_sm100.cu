@@ -510,8 +510,9 @@ static int split_log2(int tiles, int n_kb, int n_sms) {
 // Up to half as many tiles of 128 x 128 as SMs.  Measured on a B200 with weights from HBM inside a CUDA graph, us, the kernel that
 // would run otherwise -> this one.  Pair kernel: N 1024 K 3072 at M 196 / 512 / 1024 / 1152 19.1 -> 7.3, 19.0 -> 8.9, 19.3 -> 11.9,
 // 19.5 -> 14.2, beyond the line at 1536 19.1 -> 15.9; N 768 K 768 at M 196 / 1024 / 1536 8.7 -> 3.7, 8.7 -> 5.7, 8.8 -> 7.6, beyond it at
-// 2048 8.8 -> 7.9; N 2304 K 768 at M 512 8.9 -> 7.7, beyond it at 784 9.0 -> 8.1.  128 x 64 tiles of one CTA each (M <= 128): N 1024
-// K 3072 at M 32 / 128 10.0 -> 4.6, 10.4 -> 6.5; N 768 K 768 4.5 -> 3.1, 5.2 -> 3.5; N 4096 K 1024 at M 128 5.8 -> 6.4, N 6144 6.7 -> 7.0.
+// 2048 8.8 -> 7.9; N 2304 K 768 at M 512 8.9 -> 7.7, beyond it at 784 9.0 -> 8.1.  128 x 64 tiles of one CTA each (M <= 128, which bring W into L2
+// first): N 1024 K 3072 at M 32 / 128 9.7 -> 4.3, 10.3 -> 6.6; N 768 K 768 3.8 -> 2.9, 4.6 -> 3.3; N 4096 K 1024 at M 32 / 64 / 128 4.7 -> 3.9, 4.9 -> 5.5,
+// 5.2 -> 6.3, N 6144 5.4 -> 4.5, 5.7 -> 5.8, 6.2 -> 6.7 (where this one is the slower it still spares a norm's pass, or the rotation's).
 // The line dates from an earlier form of both kernels and lies on the safe side of today's crossing with the pair kernel.  The
 // one-CTA tiles, which only unsplit GEMMs reach above 128 rows, are the fastest of the three where they fill most of one round of the
 // SMs: 5.1 us for N 768 K 768 at M 1536, 10.3 for N 1024 K 3072 at M 1152, 5.4 for N 2304 K 768 at M 512.

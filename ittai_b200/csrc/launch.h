@@ -4,9 +4,10 @@
 // that it shares with its successors are its own.  So a kernel may be resident while several kernels in front of it still run
 // (each of them triggers before it waits): what it reads ahead of its wait has to be complete before the FIRST of them starts.
 // Ahead of the wait run barrier initialisation, tensor-memory allocation and descriptor prefetch, and in some kernels loads of
-// such data: weights in the split-K GEMM and the decode chain; in the chain also positions and older cache rows, which the
-// late trigger of a token's first kernel makes safe; sequence records in the key-loop attention, where the caller vouches for
-// them.  ITTAI_PDL=0 in the environment turns the attribute off (plain stream order).
+// such data: weights in the split-K GEMM, the decode chain and the projections of short forwards (there the norms' gains, too); in the
+// chain also positions and older cache rows, which the late trigger of a token's first kernel makes safe; sequence records in the
+// key-loop attention and the one for few queries, where the caller vouches for them.  (The one-SM GEMM only asks for weights to be
+// brought into L2, which hands no data over.)  ITTAI_PDL=0 in the environment turns the attribute off (plain stream order).
 #pragma once
 #include <cuda_runtime.h>
 
