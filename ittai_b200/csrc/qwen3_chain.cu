@@ -22,8 +22,8 @@
 // Rounding points are the eager modules' (the same as in qwen3_decode.cu).
 //
 // Measured on a B200, us per step, the persistent kernel of qwen3_decode.cu -> this chain: batch 1 at 47 / 4096 / 8100 cached
-// positions 549 -> 369, 575 -> 453, 657 -> 565; batch 4 at 47 / 1000 / 8100 782 -> 418, 830 -> 476, 1419 -> 976; batch 8 at 1000
-// 1026 -> 612.  A layer takes 11.5 us at a short cache, from the last store of a kernel to that of the next: attention 3.3,
+// positions 549 -> 370, 575 -> 455, 657 -> 568; batch 4 at 47 / 1000 / 8100 782 -> 419, 830 -> 478, 1419 -> 982; batch 8 at 1000 /
+// 8100 1026 -> 611, 2211 -> 1545.  A layer takes 11.5 us at a short cache, from the last store of a kernel to that of the next: attention 3.3,
 // gate/up 2.7, QKV 2.0, down 2.0, O-proj 1.5, of each of which 0.6 to 0.8 are the boundary; the head 47 us at 6.6 TB/s.  What had
 // to go on the way (batch 1, 47 positions): weights through registers (800 us: a kernel's activation loads stand behind the
 // next kernel's weight loads in the load pipe), normalisation in every warp's fragments (509: issue-bound), constants
