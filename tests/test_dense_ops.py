@@ -210,6 +210,52 @@ def test_attention_of_few_queries_in_tiles_of_32_and_of_64(lens, prefix):
 
 
 @gpu
+@pytest.mark.parametrize("seed", range(16))
+def test_attention_of_few_queries_over_the_forms_it_takes(seed):
+    """Random forms against fp32: keys and values side by side in packed rows or in a cache with odd strides, key rows from an offset on, fewer keys
+    than queries (rows that see none give zeros), gaps between the sequences' rows, bounds above the longest, tiles of 32 and of 64."""
+    import random
+    from ittai_b200 import ops
+    rng, hd = random.Random(seed), 128
+    NKV, group, B = rng.choice([1, 2, 8]), rng.choice([1, 2, 4]), rng.choice([1, 3, 12, 20])
+    lens = [rng.choice([0, 1, 2, 15, 16, 17, 31, 32, 33, 48, 63, 64]) for _ in range(B)]
+    keys = [max(0, n + rng.choice([0, 0, 1, 31, 32, 200, -3, -40])) for n in lens]
+    first, rows = [0] * B, 3
+    for b in rng.sample(range(B), B):
+        first[b], rows = rows, rows + lens[b] + rng.choice([0, 2])
+    NH = NKV * group
+    q_head, o_row = hd + rng.choice([0, 8]), NH * hd + rng.choice([0, 8])
+    q_row = NH * q_head + 8
+    q = _rand(rows * q_row, seed=seed)
+    if seed % 2:
+        k_row, k_head, k_seq = 2 * NKV * hd, hd, 0
+        row0 = [sum(keys[:b]) + b for b in range(B)]
+        k = _rand((sum(keys) + B) * k_row, seed=seed + 100)
+        v = k[NKV * hd:]
+    else:
+        row0 = [rng.choice([0, 5, 32]) for _ in range(B)]
+        k_row = hd + rng.choice([0, 8])
+        k_head = (max(a + n for a, n in zip(row0, keys)) + 1) * k_row
+        k_seq = NKV * k_head + 8
+        k, v = _rand(B * k_seq, seed=seed + 100), _rand(B * k_seq, seed=seed + 200)
+    out = torch.full((rows, o_row), 3.0, dtype=torch.bfloat16, device="cuda")
+    seqs = torch.tensor([[first[b], lens[b], row0[b], keys[b]] for b in range(B)], dtype=torch.int32, device="cuda")
+    ops.attention(q, k, v, out, seqs, n_heads=NH, group=group, head_dim=hd, causal=True, max_q_len=rng.choice([max(lens + [1]), 64]), q_strides=(q_row, q_head),
+                  k_strides=(k_row, k_head, k_seq), v_strides=(k_row, k_head, k_seq), o_strides=(o_row, hd))
+    untouched = torch.ones(rows, dtype=torch.bool)
+    for b, (n, m) in enumerate(zip(lens, keys)):
+        untouched[first[b]:first[b] + n] = False
+        if n == 0:
+            continue
+        Q = q.as_strided((NH, n, hd), (q_head, q_row, 1), first[b] * q_row).float()
+        K, V = (t.as_strided((NKV, m, hd), (k_head, k_row, 1), t.storage_offset() + b * k_seq + row0[b] * k_row).float().repeat_interleave(group, 0) for t in (k, v))
+        seen = torch.arange(m, device="cuda")[None, :] <= torch.arange(n, device="cuda")[:, None] + m - n
+        w = (Q @ K.transpose(1, 2) * hd ** -0.5).masked_fill(~seen, float("-inf")).softmax(-1).nan_to_num(0.0)
+        _check(out[first[b]:first[b] + n, :NH * hd], (w @ V).transpose(0, 1).reshape(n, NH * hd), f"sequence {b}: {n} queries, {m} keys")
+    assert (out[untouched.cuda()] == 3.0).all() and (out[:, NH * hd:] == 3.0).all()
+
+
+@gpu
 def test_attention_of_few_queries_is_spread_over_the_sms():
     """128 tiles find an SM each: four sequences behind a long cache take about as long as one.  (Packed onto fewer SMs 1.7 times as
     long: a kernel starts while the one before it holds SMs, and fills the ones that it finds empty.)"""
